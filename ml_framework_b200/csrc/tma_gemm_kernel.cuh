@@ -274,7 +274,8 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
     __shared__ uint32_t tmem_base_slot;
     __shared__ int abort_flag;
 
-    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const int t = threadIdx.x, lane = t & 31;
+    const int warp = __shfl_sync(0xffffffffu, t >> 5, 0);       // the same in all lanes, and known to be
     const int bn = p.bn, stages = p.stages;
     // PAIR: the two CTAs of a cluster work on one tile of 256 rows; `rank` 0 (the even CTA) issues its MMAs
     constexpr int TM = PAIR ? 2 * TC_BM : TC_BM;
@@ -321,8 +322,9 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
         ktiles = (kend - kbeg + TC_BK - 1) / TC_BK;
     };
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
         // ---------------- TMA producer ----------------
+        const bool leader = elect_one();
         const CUtensorMap *mA[3] = {&mapA0, &mapA1, &mapA2};
         const CUtensorMap *mB[3] = {&mapB0, &mapB1, &mapB2};
         auto ld2d = [&](uint32_t dst, const CUtensorMap *m, int x, int y, uint32_t bar) {
@@ -373,6 +375,7 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
                     if (++s == stages) { s = 0; ph ^= 1u; }
                     continue;
                 }
+                if (leader) {
                 if (rank == 0) mbar_expect_tx(full0 + 8 * s, tx_bytes);
                 int bk = k0;                                  // B's coordinate along the contraction
                 if (p.a_mode == TMA_A_ROWS) {
@@ -404,6 +407,7 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
 #pragma unroll
                     for (int i = 0; i < NS; i++) ld2d(b_tile(s, i), mB[i], bk, nb0, bar);
                 }
+                }
                 if (++s == stages) { s = 0; ph ^= 1u; }
             }
         }
@@ -416,8 +420,9 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
                 while (!mbar_try_wait(full0 + 8 * (k % stages), (uint32_t)(k / stages) & 1u) && clock64() - t0 < p.wait_clocks) {}
             }
         }
-    } else if (warp >= 1 && warp <= issuers && lane == 0 && rank == 0) {
+    } else if (warp >= 1 && warp <= issuers && rank == 0) {
         // ---------------- MMA issuers (in the even CTA of a pair) ----------------
+        const bool leader = elect_one();
         const int me = warp - 1;
         uint32_t idesc = umma_idesc_16bit(bn, p.a_fp16, p.b_fp16) | ((uint32_t)(a_mn ? 1 : 0) << 15) | ((uint32_t)p.b_mn << 16);
         if (PAIR) idesc = (idesc & ~(31u << 24)) | ((uint32_t)(TM >> 4) << 24);          // M = 256 over the two CTAs
@@ -452,27 +457,32 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
                 const uint64_t das = da0 + (uint32_t)s * stage16, dbs = db0 + (uint32_t)s * stage16;
                 // the K = 16 slices of this thread (da0 / db0 already point at its first one), fully unrolled either way: the
                 // issuing thread's own instruction stream is what limits the MMA rate
-                auto slice = [&](uint64_t dsa, uint64_t dsb) {
+                auto slice = [&](uint64_t dsa, uint64_t dsb, bool first) {
                     uint64_t da[NS], db[NS];
 #pragma unroll
                     for (int i = 0; i < NS; i++) { da[i] = dsa + (uint32_t)i * a_copy16; db[i] = dsb + (uint32_t)i * b_copy16; }
 #pragma unroll
                     for (int q = 0; q < NPROD; q++) {
-                        if (PAIR) umma2_bf16(d_tmem, da[pa[q]], db[pb[q]], idesc, acc); else umma_bf16(d_tmem, da[pa[q]], db[pb[q]], idesc, acc);
-                        acc = 1;
+                        const bool open = first && q == 0;        // only the k-step's first product can start the accumulator
+                        if (PAIR) umma2_bf16(d_tmem, da[pa[q]], db[pb[q]], idesc, open ? acc : 1u);
+                        else if (open) umma_bf16(d_tmem, da[pa[q]], db[pb[q]], idesc, acc);
+                        else umma_bf16_add(d_tmem, da[pa[q]], db[pb[q]], idesc);
                     }
                 };
+                if (leader) {
                 if (issuers == 2) {
 #pragma unroll
-                    for (int jj = 0; jj < TC_BK / 32; jj++) slice(das + (uint32_t)(2 * jj) * a_step16, dbs + (uint32_t)(2 * jj) * b_step16);
+                    for (int jj = 0; jj < TC_BK / 32; jj++) slice(das + (uint32_t)(2 * jj) * a_step16, dbs + (uint32_t)(2 * jj) * b_step16, jj == 0);
                 } else {
 #pragma unroll
-                    for (int jj = 0; jj < TC_BK / 16; jj++) slice(das + (uint32_t)jj * a_step16, dbs + (uint32_t)jj * b_step16);
+                    for (int jj = 0; jj < TC_BK / 16; jj++) slice(das + (uint32_t)jj * a_step16, dbs + (uint32_t)jj * b_step16, jj == 0);
                 }
                 if (PAIR) umma2_commit_both(empty0 + 8 * s); else umma_commit(empty0 + 8 * s);
+                }
+                acc = 1;
                 if (++s == stages) { s = 0; ph ^= 1u; }
             }
-            if (alive) { if (PAIR) umma2_commit_both(tfull0 + 8 * buf); else umma_commit(tfull0 + 8 * buf); }   // accumulator complete
+            if (alive && leader) { if (PAIR) umma2_commit_both(tfull0 + 8 * buf); else umma_commit(tfull0 + 8 * buf); }   // accumulator complete
         }
     } else if (warp >= TG_EPI_WARP0) {
         // ---------------- epilogue: warp w drains TMEM lane quarter w % 4 ----------------
