@@ -169,7 +169,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) tc_contraction_kernel(AL al, BL
                 // every MMA has completed, so the operand stages are free: reuse them as per-warp staging
                 float *stage = reinterpret_cast<float *>(smem + (size_t)warp * EPI_WARP_SMEM);
                 int cb = half * cols_per_half;
-                drain_accumulator(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)cb, m0 + q * 32, n0, cb, cb + cols_per_half,
+                drain_accumulator(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)cb, m0 + q * 32, n0, cb, cb + cols_per_half, 32,
                                   p.M, p.N, cs, p.partial, (long long)blockIdx.z * p.M * p.N, stage);
             }
         }

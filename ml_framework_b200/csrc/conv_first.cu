@@ -505,9 +505,9 @@ first_tc_fwd_kernel(const float *__restrict__ X, const float *__restrict__ Wt, S
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * bn + c0);
             if (c0 >= bn) {}
             else if (pool_on)
-                drain_accumulator_pooled(taddr, tile * TC_BM + q * 32, c0, c1 - c0, (int)pixels, g.F, bias, act, po, stage);
+                drain_accumulator_pooled(taddr, tile * TC_BM + q * 32, 0, c0, c1, 32, (int)pixels, g.F, bias, act, po, stage);
             else
-                drain_accumulator(taddr, tile * TC_BM + q * 32, 0, c0, c1, (int)pixels, g.F, cs, nullptr, 0, stage, bias, act);
+                drain_accumulator(taddr, tile * TC_BM + q * 32, 0, c0, c1, 32, (int)pixels, g.F, cs, nullptr, 0, stage, bias, act);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(tempty0 + 8 * buf);

@@ -34,11 +34,17 @@ struct StoreDenseCopies {
     static constexpr bool kMContiguous = false;
     float *C; long long ld;
     __nv_bfloat16 *cp[3]; int cld, ns; Enc enc;
-    __device__ void copy_out(int m, int n, float v) const {
+    __device__ void copy_out4(int m, int n, const float4 &x) const {       // n a multiple of 4, as is the pitch
+        const float v[4] = {x.x, x.y, x.z, x.w};
+        const long long o = (long long)m * cld + n;
+#pragma unroll
+        for (int j = 0; j < 4; j++) store_split1(v[j], ns, enc, cp[0] + o + j, cp[1] + o + j, cp[2] + o + j);
+    }
+    __device__ void operator()(int m, int n, float v) const {
+        C[(long long)m * ld + n] = v;
         const long long o = (long long)m * cld + n;
         store_split1(v, ns, enc, cp[0] + o, cp[1] + o, cp[2] + o);
     }
-    __device__ void operator()(int m, int n, float v) const { C[(long long)m * ld + n] = v; copy_out(m, n, v); }
     __device__ float *row(int m) const { return C + (long long)m * ld; }
     __device__ long long nstride() const { return 1; }
 };

@@ -93,7 +93,8 @@ __device__ __forceinline__ void umma_bf16_add(uint32_t d_tmem, uint64_t adesc, u
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float *v) {
+// 32 columns of this warp's 32 lanes, requested; the values may be used after tmem_ld_wait on them.
+__device__ __forceinline__ void tmem_ld32_issue(uint32_t taddr, float *v) {
     uint32_t *r = reinterpret_cast<uint32_t *>(v);
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
                  "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
@@ -102,17 +103,32 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float *v) {
                    "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
                    "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
                  : "r"(taddr) : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
-// The same over `nacc` accumulators that sit `acc_stride` columns apart and hold partial sums of one tile (one per MMA-issuing
-// thread): their sum, added in index order.
+__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// keeps every use of the values behind the wait
+__device__ __forceinline__ void tmem_ld_pin(float *v) {
+#pragma unroll
+    for (int i = 0; i < 32; i++) asm volatile("" : "+f"(v[i]));
+}
+__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float *v) {
+    tmem_ld32_issue(taddr, v);
+    tmem_ld_wait();
+    tmem_ld_pin(v);
+}
+// The same over one or two accumulators that sit `acc_stride` columns apart and hold partial sums of one tile (one per
+// MMA-issuing thread): their sum, in index order.  Both loads are in flight together.
 __device__ __forceinline__ void tmem_ld32_sum(uint32_t taddr, float *v, int nacc, uint32_t acc_stride) {
-    tmem_ld32(taddr, v);
-    for (int i = 1; i < nacc; i++) {
+    if (nacc == 2) {
         float w[32];
-        tmem_ld32(taddr + (uint32_t)i * acc_stride, w);
+        tmem_ld32_issue(taddr, v);
+        tmem_ld32_issue(taddr + acc_stride, w);
+        tmem_ld_wait();
+        tmem_ld_pin(v);
+        tmem_ld_pin(w);
 #pragma unroll
         for (int j = 0; j < 32; j++) v[j] += w[j];
+    } else {
+        tmem_ld32(taddr, v);
     }
 }
 
@@ -201,6 +217,12 @@ __device__ __forceinline__ void store_split8(float *v, const Enc &e, void *d0, v
         if (NS >= 2) *reinterpret_cast<uint4 *>(d1) = split_chunk(v);
         if (NS >= 3) *reinterpret_cast<uint4 *>(d2) = split_chunk(v);
     }
+}
+// The same with the number of copies known at run time (8 consecutive values, 16-byte chunks).
+__device__ __forceinline__ void store_split8_n(float *v, int ns, const Enc &e, __nv_bfloat16 *d0, __nv_bfloat16 *d1, __nv_bfloat16 *d2) {
+    if (ns == 1) store_split8<1>(v, e, d0, d1, d2);
+    else if (ns == 2) store_split8<2>(v, e, d0, d1, d2);
+    else store_split8<3>(v, e, d0, d1, d2);
 }
 // The same for one value (ns known at run time).
 __device__ __forceinline__ void store_split1(float v, int ns, const Enc &e, __nv_bfloat16 *d0, __nv_bfloat16 *d1, __nv_bfloat16 *d2) {

@@ -249,9 +249,10 @@ struct TmaGemmParams {
     FastDiv by_mtiles, by_ntiles, by_OHW, by_OW, by_S, by_cchunks;      // filled by launch_tma_gemm
 };
 
-// warp 0: TMA producer; warps 1-2: MMA issuers (the first p.issuers of them); warp 3 allocates TMEM; warps 4-7: epilogue.
-// (Eight warps: with a ninth the register file would be shared out as for twelve, 168 registers per thread, and the epilogue spills.)
-constexpr int TG_THREADS = 256, TG_EPI_WARP0 = 4;
+// warp 0: TMA producer; warps 1-2: MMA issuers (the first p.issuers of them); warp 3 allocates TMEM; warps 4-11: epilogue, two warps
+// per TMEM lane quarter, which take its 32-column chunks alternately.  One warp per quarter drained a 128 x 128 tile in about the
+// time of twice its main loop (VGG, 128 filters at 16 x 16: launch 80 us, main loop alone 37 us).
+constexpr int TG_THREADS = 384, TG_EPI_WARP0 = 4, TG_EPI_WARPS = 8;
 
 // Persistent kernel: each CTA walks tiles  id = blockIdx.x, blockIdx.x + gridDim.x, ...  (m-tile fastest, then n-tile,
 // then K split).  The operand ring keeps streaming across tile boundaries and the accumulator is double-buffered in
@@ -292,7 +293,7 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
     const uint32_t smem0 = smem_u32(smem);
     auto a_tile = [&](int s, int i) { return smem0 + (uint32_t)s * stage_bytes + (uint32_t)i * a_bytes; };
     auto b_tile = [&](int s, int i) { return smem0 + (uint32_t)s * stage_bytes + (uint32_t)NS * a_bytes + (uint32_t)i * b_bytes; };
-    unsigned char *epi_smem = smem + (size_t)stages * stage_bytes;   // 4 x EPI_WARP_SMEM after the ring
+    unsigned char *epi_smem = smem + (size_t)stages * stage_bytes;   // one EPI_WARP_SMEM per epilogue warp after the ring
     const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[8]), tfull0 = smem_u32(&bars[16]), tempty0 = smem_u32(&bars[18]);
     const int issuers = PAIR ? 1 : p.issuers;
     const uint32_t tmem_cols = (uint32_t)(2 * issuers * bn < 32 ? 32 : 2 * issuers * bn);
@@ -300,7 +301,7 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
     if (t == 0) {
         abort_flag = 0;
         for (int s = 0; s < stages; s++) { mbar_init(full0 + 8 * s, 1); mbar_init(empty0 + 8 * s, issuers); }
-        for (int b = 0; b < 2; b++) { mbar_init(tfull0 + 8 * b, issuers); mbar_init(tempty0 + 8 * b, PAIR ? 8 : 4); }
+        for (int b = 0; b < 2; b++) { mbar_init(tfull0 + 8 * b, issuers); mbar_init(tempty0 + 8 * b, PAIR ? 2 * TG_EPI_WARPS : TG_EPI_WARPS); }
         fence_mbar_init();
         fence_async_smem();
     }
@@ -485,8 +486,8 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
             if (alive && leader) { if (PAIR) umma2_commit_both(tfull0 + 8 * buf); else umma_commit(tfull0 + 8 * buf); }   // accumulator complete
         }
     } else if (warp >= TG_EPI_WARP0) {
-        // ---------------- epilogue: warp w drains TMEM lane quarter w % 4 ----------------
-        const int q = warp & 3;
+        // ---------------- epilogue: warp w drains TMEM lane quarter w % 4, every second 32-column chunk ----------------
+        const int q = warp & 3, c_first = ((warp - TG_EPI_WARP0) >> 2) * 32;
         float *stage = reinterpret_cast<float *>(epi_smem + (size_t)(warp - TG_EPI_WARP0) * EPI_WARP_SMEM);
         const float out_scale = p.dinv ? p.out_scale * __ldg(p.dinv) : p.out_scale;
         int local = 0;
@@ -495,17 +496,24 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
             int m0, n0, kbeg, ktiles, z;
             tile_origin(id, m0, n0, kbeg, ktiles, z);
             const int buf = local & 1;
-            if (!mbar_wait(tfull0 + 8 * buf, ((uint32_t)local >> 1) & 1u, abortp, p.status, 3, p.wait_clocks)) break;
+            // (a longer budget than the issuers', so that a stage that never fills is reported by the role that waits for it)
+            if (!mbar_wait(tfull0 + 8 * buf, ((uint32_t)local >> 1) & 1u, abortp, p.status, 3, p.wait_clocks + (p.wait_clocks >> 2))) break;
             tc_fence_after();
-            if (p.pool_on)
-                drain_accumulator_pooled(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * issuers * bn), m0 + q * 32, n0, bn, p.M, p.N,
-                                         p.bias, p.act, p.pool, stage, out_scale, issuers, (uint32_t)bn);
+            // the accumulator goes back to the issuers as soon as its last chunk is in registers
+            auto release = [&]() {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) { if (PAIR) mbar_arrive_cluster(tempty_at + 8 * buf); else mbar_arrive(tempty0 + 8 * buf); }
+            };
+            const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * issuers * bn + c_first);
+            if (c_first >= bn)                                     // a 32-column tile has one chunk
+                release();
+            else if (p.pool_on)
+                drain_accumulator_pooled(taddr, m0 + q * 32, n0, c_first, bn, 64, p.M, p.N, p.bias, p.act, p.pool, stage, out_scale, issuers,
+                                         (uint32_t)bn, release);
             else
-                drain_accumulator(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * issuers * bn), m0 + q * 32, n0, 0, bn, p.M, p.N, cs,
-                                  p.partial, (long long)z * p.M * p.N, stage, p.bias, p.act, out_scale, issuers, (uint32_t)bn);
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) { if (PAIR) mbar_arrive_cluster(tempty_at + 8 * buf); else mbar_arrive(tempty0 + 8 * buf); }
+                drain_accumulator(taddr, m0 + q * 32, n0, c_first, bn, 64, p.M, p.N, cs, p.partial, (long long)z * p.M * p.N, stage, p.bias,
+                                  p.act, out_scale, issuers, (uint32_t)bn, release);
         }
     }
     tc_fence_before();
@@ -543,7 +551,7 @@ inline int tma_pick_bn(int N, int ns, int b_mn) {
     if (ns == 2 && bn > rt().tile_n_cap2) bn = rt().tile_n_cap2;
     if (ns >= 3 && bn > rt().tile_n_cap3) bn = rt().tile_n_cap3;
     // at least two stages of ns * (128 + bn) * 128 bytes must fit beside the epilogue staging
-    while (bn > 32 && 2 * (size_t)ns * (TC_BM + bn) * 128 > 225 * 1024 - 4 * EPI_WARP_SMEM - 1024) bn >>= 1;
+    while (bn > 32 && 2 * (size_t)ns * (TC_BM + bn) * 128 > 225 * 1024 - TG_EPI_WARPS * EPI_WARP_SMEM - 1024) bn >>= 1;
     return bn;
 }
 
@@ -575,10 +583,10 @@ int launch_tma_gemm(const TmaMaps &maps, TmaGemmParams p, const CS &cs, int ns, 
     const int tm = p.pair ? 2 * TC_BM : TC_BM;
     size_t stage = (size_t)ns * (TC_BM * 128 + (size_t)(p.pair ? p.bn / 2 : p.bn) * 128);
     // 227 KB per CTA on sm_100a; keep 2 KB for the kernel's static shared memory and alignment slack
-    int stages = (int)((225 * 1024 - 4 * EPI_WARP_SMEM - 1024) / stage);
+    int stages = (int)((225 * 1024 - TG_EPI_WARPS * EPI_WARP_SMEM - 1024) / stage);
     if (stages > 8) stages = 8;
     if (stages < 2) return fail(SEERA_E_LIMIT, "%s: tile does not fit shared memory", name);
-    size_t smem = stage * stages + 4 * EPI_WARP_SMEM + 1024;
+    size_t smem = stage * stages + TG_EPI_WARPS * EPI_WARP_SMEM + 1024;
     long long tiles = (long long)((p.M + tm - 1) / tm) * ((p.N + p.bn - 1) / p.bn);
     // Split of the contraction: every (tile, split) item is one pass of a persistent CTA, so the launch takes
     // ceil(items / SMs) rounds of ceil(ksteps / splits) k-steps each, plus a fixed cost per item (pipeline fill, the
