@@ -18,6 +18,8 @@ What is different underneath:
 """
 from __future__ import annotations
 
+import math
+
 import numpy as np
 
 from . import seera_cuda
@@ -26,36 +28,34 @@ _UPLOAD = {"float32": seera_cuda.to_device_f32, "int32": seera_cuda.to_device_i3
 _NP = {"float32": np.float32, "int32": np.int32, "int16": np.int16}
 
 
-def _numel(shape):
-    n = 1
-    for d in shape:
-        n *= d
-    return n
+_numel = math.prod
+_bare = object.__new__
 
 
 class cuten:
     supported_types = ["float32", "int32", "int16"]
 
+    # What an instance starts from; a step makes dozens of these objects, so only what differs is stored on one.
+    dtype = "float32"
+    shape = size = None
+    _ptr = None
+    _const = None                 # pending fill value of a lazy constant
+    _base = None                  # owner of the memory this tensor views
+    _owns_memory = True           # an empty shell: the caller assigns a fresh address it owns
+
     def __init__(self, data=None, dtype="float32"):
         if dtype not in self.supported_types:
+            self._owns_memory = False
             raise ValueError("[cuTen]:Not Supported by cuTen, try in CPU")
-        self.dtype = dtype
-        self._ptr = None
-        self._const = None            # pending fill value of a lazy constant
-        self._base = None             # owner of the memory this tensor views
-        self._owns_memory = False
+        if dtype != "float32":
+            self.dtype = dtype
         if isinstance(data, (list, tuple)):
             data = np.array(data, dtype=dtype)
         if isinstance(data, np.ndarray):
-            arr = np.ascontiguousarray(data.astype(dtype))
+            arr = np.ascontiguousarray(data, dtype=dtype)
             self._ptr = _UPLOAD[dtype](arr)
             self.shape = arr.shape
             self.size = arr.size
-            self._owns_memory = True
-        else:
-            self.shape = None
-            self.size = None
-            self._owns_memory = True     # an empty shell: the caller assigns a fresh address it owns
 
     # ---- the device address: plain attribute for callers, lazy for constants ----------------
     @property
@@ -81,10 +81,9 @@ class cuten:
         return self._const if self._ptr is None else None
 
     def __del__(self):
-        ptr = getattr(self, "_ptr", None)
-        if getattr(self, "_owns_memory", False) and ptr is not None and getattr(self, "_base", None) is None:
+        if self._owns_memory and self._ptr is not None and self._base is None:
             try:
-                seera_cuda.cuda_free(ptr)
+                seera_cuda.cuda_free(self._ptr)
             except Exception:
                 pass
             self._ptr = None
@@ -92,17 +91,20 @@ class cuten:
     # ---- construction helpers -------------------------------------------------------------------
     @classmethod
     def _wrap(cls, ptr, shape, dtype="float32"):
-        t = cls(None, dtype)
+        t = _bare(cls)
         t._ptr = ptr
-        t.shape = tuple(shape)
+        t.shape = shape = tuple(shape)
         t.size = _numel(shape)
+        if dtype != "float32":
+            if dtype not in cls.supported_types:
+                t._owns_memory = False
+                raise ValueError("[cuTen]:Not Supported by cuTen, try in CPU")
+            t.dtype = dtype
         return t
 
     @classmethod
     def _constant(cls, shape, value, dtype="float32"):
-        t = cls(None, dtype)
-        t.shape = tuple(shape)
-        t.size = _numel(shape)
+        t = cls._wrap(None, shape, dtype)
         t._const = float(value)
         return t
 

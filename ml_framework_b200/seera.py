@@ -21,6 +21,7 @@ There is no CPU path here: `device` must be "cuda" and the compiled engine must 
 """
 from __future__ import annotations
 
+import math
 import pickle
 
 import numpy as np
@@ -33,34 +34,51 @@ _ACTIVATIONS = ("relu", "sigmoid", "softmax", "tanh")
 f32 = np.float32
 
 
-def _numel(shape):
-    n = 1
-    for d in shape:
-        n *= d
-    return n
+_numel = math.prod
+_wrap = cuten._wrap
+_malloc = sc.cuda_malloc_f32
+_bare = object.__new__
 
 
 def _new(shape):
-    return cuten._wrap(sc.cuda_malloc_f32(_numel(shape)), shape)
+    return _wrap(_malloc(_numel(shape)), shape)
 
 
 # ─────────────────────────────────────────────────────────────────────────────────────────────
 # Tensor: a device value, its gradient, and the closure that propagates the gradient
 # ─────────────────────────────────────────────────────────────────────────────────────────────
 class Tensor:
+    # What an instance starts from.  The eager path makes one of these per layer and call, so only what differs is stored on one.
+    dtype = "float32"
+    is_leaf = False
+    grad = None                      # cuten, set by backward
+    _parents = ()
+    _backward = None                 # fn(grad: cuten) -> None, deposits into parents via _accumulate
+    _softmax_logits = None           # for a softmax output: the Tensor of logits it came from
+    _grad_slot = None                # for a parameter: its view into the model's gradient arena
+    _takes_pooled = False            # its backward takes the gradient of a 2x2 max-pool of it in pooled form
+    _copies = None                   # channels-last copies of the value, made by its producer for a convolution
+    _rows = None                     # row-major copies of the value, made by its producer for a Dense layer
+
     def __init__(self, value, dtype="float32", is_leaf=False, device="cuda"):
         if isinstance(value, Tensor):
             value = value.value
         if not isinstance(value, cuten):
             value = cuten(np.ascontiguousarray(np.asarray(value, dtype=np.float32)))
         self.value = value
-        self.dtype = dtype
-        self.is_leaf = is_leaf
-        self.grad = None                 # cuten, set by backward
-        self._parents = ()
-        self._backward = None            # fn(grad: cuten) -> None, deposits into parents via _accumulate
-        self._softmax_logits = None      # for a softmax output: the Tensor of logits it came from
-        self._grad_slot = None           # for a parameter: its view into the model's gradient arena
+        if dtype != "float32":
+            self.dtype = dtype
+        if is_leaf:
+            self.is_leaf = is_leaf
+
+    @classmethod
+    def _of(cls, value, parents, backward):
+        """The output of an operation on the device."""
+        t = _bare(cls)
+        t.value = value
+        t._parents = parents
+        t._backward = backward
+        return t
 
     # the reference reads gradients as `t.node.cp` (Seera_init.py:53-55)
     @property
@@ -164,8 +182,8 @@ class _KeptCopies:
     """Owner of the channels-last copies a forward call kept for its backward call (0: none kept)."""
     __slots__ = ("h",)
 
-    def __init__(self):
-        self.h = 0
+    def __init__(self, h=0):
+        self.h = h
 
     def release(self):
         if self.h:
@@ -179,8 +197,8 @@ class _KeptRows:
     """Owner of row-major operand copies a Dense forward call kept or handed on (0: none)."""
     __slots__ = ("h",)
 
-    def __init__(self):
-        self.h = 0
+    def __init__(self, h=0):
+        self.h = h
 
     def release(self):
         if self.h:
@@ -199,33 +217,42 @@ class autograd4nn:
 
     def backward(self):
         order, seen = [], set()
-        stack = [(self.hook, False)]
+        stack = [self.hook]
         while stack:                                   # iterative DFS: no recursion limit on deep nets
-            t, done = stack.pop()
-            if done:
-                order.append(t)
+            t = stack.pop()
+            if t is None:                              # everything above its tensor has been placed
+                order.append(stack.pop())
                 continue
-            if id(t) in seen:
+            if t in seen:
                 continue
-            seen.add(id(t))
-            stack.append((t, True))
+            seen.add(t)
+            stack.append(t)
+            stack.append(None)
             for p in t._parents:
-                stack.append((p, False))
+                if not p.is_leaf:                      # a leaf keeps its gradient and passes nothing on
+                    stack.append(p)
         for t in order:
             if not t.is_leaf:
                 t.grad = None
         self.hook.grad = cuten.ones_like(self.hook.value)
         for t in reversed(order):
-            if t._backward is not None and t.grad is not None:
-                if isinstance(t.grad, _PooledGrad) and not getattr(t, "_takes_pooled", False):
-                    t.grad = t.grad.materialize()
-                t._backward(t.grad)
+            back, g = t._backward, t.grad
+            if back is not None and g is not None:
+                if g.__class__ is _PooledGrad and not t._takes_pooled:
+                    t.grad = g = g.materialize()
+                back(g)
 
 
 # ─────────────────────────────────────────────────────────────────────────────────────────────
 # Layers
 # ─────────────────────────────────────────────────────────────────────────────────────────────
 class Layer:
+    # which layers read this one's output (set while a model is put together): a producer can then hand on more than its values
+    _pool_consumer = None
+    _feeds_conv = _feeds_dense = False
+    _fused = None                    # a pool that the layer folded into its own launch: (pooled, mask, copies)
+    _model = None
+
     def __init__(self):
         self.inputs = []
         self.outputs = []
@@ -309,66 +336,34 @@ class _ParamLayer(Layer):
             neg = v * (-1)
             sc.cuda_elemadd(t.value.main_ptr, neg.main_ptr, t.value.main_ptr, t.value.size)
 
-    # fused epilogue / prologue shared by Dense, Conv2D, ConvTranspose2D
-    def _finish_forward(self, x, z, channels, inner, product, contraction_backward, fused_backward=None, takes_pooled=False):
-        """product(bias_ptr, act_code) fills z with act(contraction + bias) in one call; this wraps z as the layer's
-        output Tensor and attaches the backward closure."""
-        act = self.layeract
-        W, b = self.weights, self.bais
-        if act == "softmax":
-            if len(z.shape) != 2:
-                raise ValueError("[Engine]: Softmax VJP requires at least 2D")
-            product(b.value.main_ptr, 0)
-            logits = Tensor(z)
-            y = _new(z.shape)
-            sc.cuda_softmax_fwd(z.main_ptr, y.main_ptr, z.shape[0], z.shape[1])
-            out = Tensor(y)
-            out._softmax_logits = logits
-            out._parents = (logits,)
+    # shared by Dense, Conv2D, ConvTranspose2D
+    def _output(self, x, z, node_backward, takes_pooled=False):
+        """The layer's output Tensor around `z`, which holds act(contraction + bias), or the logits of a softmax."""
+        node = Tensor._of(z, (x, self.weights, self.bais), node_backward)
+        if takes_pooled:
+            node._takes_pooled = True
+        if self.layeract != "softmax":
+            return node
+        y = _new(z.shape)
+        sc.cuda_softmax_fwd(z._ptr, y._ptr, z.shape[0], z.shape[1])
 
-            def softmax_backward(g, y=y, logits=logits):
-                dz = _new(y.shape)
-                sc.cuda_softmax_vjp(y.main_ptr, g.main_ptr, dz.main_ptr, y.shape[0], y.shape[1])
-                logits._accumulate(dz)
-            out._backward = softmax_backward
-            node, code = logits, 0
-        else:
-            code = _ACT[act]
-            product(b.value.main_ptr, code)
-            out = Tensor(z)
-            node = out
-        node._parents = (x, W, b)
-
-        node._takes_pooled = takes_pooled and fused_backward is not None
-
-        def layer_backward(g, y=node.value, code=code):
-            db = b._grad_target()
-            if fused_backward is not None:          # activation, bias and contraction gradients in one call
-                dx, dw = fused_backward(g, y, code, db)
-                b._accumulate(db)
-                W._accumulate(dw)
-                hook = getattr(getattr(self, "_model", None), "_on_grad_ready", None)
-                if hook is not None and W.grad is W._grad_slot and b.grad is b._grad_slot:
-                    hook(W)
-                if dx is not None:
-                    x._accumulate(dx)
-                return
-            if code == 0:
-                dz = g
-                sc.act_bias_bwd(g.main_ptr, 0, g.main_ptr, db.main_ptr, y.size, channels, inner, 0)
-            else:
-                dz = _new(y.shape)
-                sc.act_bias_bwd(g.main_ptr, y.main_ptr, dz.main_ptr, db.main_ptr, y.size, channels, inner, code)
-            b._accumulate(db)
-            dx, dw = contraction_backward(dz)
-            W._accumulate(dw)
-            hook = getattr(getattr(self, "_model", None), "_on_grad_ready", None)
-            if hook is not None and W.grad is W._grad_slot and b.grad is b._grad_slot:
-                hook(W)                      # this layer's gradients sit in the arena: a bucket may go out
-            if dx is not None:
-                x._accumulate(dx)
-        node._backward = layer_backward
+        def softmax_backward(g):
+            dz = _new(y.shape)
+            sc.cuda_softmax_vjp(y._ptr, g.main_ptr, dz._ptr, y.shape[0], y.shape[1])
+            node._accumulate(dz)
+        out = Tensor._of(y, (node,), softmax_backward)
+        out._softmax_logits = node
         return out
+
+    def _deliver(self, x, W, b, dx, dw, db):
+        """Gradients of one backward call to the input and the parameters."""
+        b._accumulate(db)
+        W._accumulate(dw)
+        model = self._model
+        if model is not None and model._on_grad_ready is not None and W.grad is W._grad_slot and b.grad is b._grad_slot:
+            model._on_grad_ready(W)          # this layer's gradients sit in the arena: a bucket may go out
+        if dx is not None:
+            x._accumulate(dx)
 
 
 class Dense(_ParamLayer):
@@ -390,40 +385,35 @@ class Dense(_ParamLayer):
 
     def forward(self):
         x = self.inputs = self.inpobj.outputs
-        xv, W = x.value, self.weights.value
-        if len(xv.shape) != 2 or xv.shape[1] != self.in_units:
-            raise ValueError(f"[cuTen]: matmul: inner dimensions must agree, got {xv.shape} @ {W.shape}")
-        M, K, N = xv.shape[0], self.in_units, self.out_units
+        W, b = self.weights, self.bais
+        xv, wv = x.value, W.value
+        shape = xv.shape
+        if len(shape) != 2 or shape[1] != self.in_units:
+            raise ValueError(f"[cuTen]: matmul: inner dimensions must agree, got {xv.shape} @ {wv.shape}")
+        M, K, N = shape[0], self.in_units, self.out_units
         z = _new((M, N))
-        kept = {"a": _KeptRows(), "w": _KeptRows()}
-        given = getattr(x, "_rows", None) if x.value is xv else None        # copies written by the Dense layer before
-        out_rows = _KeptRows()
-        want_out = DENSE_EPILOGUE_COPIES and bool(getattr(self, "_feeds_dense", False)) and self.layeract != "softmax"
+        code = _ACT.get(self.layeract, 0)                    # a softmax follows the product as a pass of its own
+        given = x._rows                                      # copies written by the Dense layer before
+        want_out = DENSE_EPILOGUE_COPIES and self._feeds_dense and self.layeract != "softmax"
+        ha, hw, ho = sc.matmul_bias_act_fwd_s(xv.main_ptr, wv.main_ptr, b.value.main_ptr, z._ptr, M, N, K, code, given.h if given else 0, want_out)
+        kept_a, kept_w = _KeptRows(ha) if ha else None, _KeptRows(hw) if hw else None
+        need_dx = not x.is_leaf
 
-        def product(bias, code):
-            kept["a"].h, kept["w"].h, out_rows.h = sc.matmul_bias_act_fwd_s(xv.main_ptr, W.main_ptr, bias, z.main_ptr, M, N, K, code,
-                                                                             given.h if given else 0, want_out)
-
-        def fused_backward(g, y, code, db, need_dx=not x.is_leaf):
+        def backward(g):
             # activation slope, bias gradient, dA and dB in one call; it reads the copies the forward call kept
-            dw = self.weights._grad_target()
-            dx = _new(xv.shape) if need_dx else None
-            sc.matmul_act_bwd(xv.main_ptr, W.main_ptr, y.main_ptr if code else 0, g.main_ptr, dx.main_ptr if need_dx else 0, dw.main_ptr,
-                              db.main_ptr, M, N, K, code, kept["a"].h or (given.h if given else 0), kept["w"].h)
-            kept["a"].release(); kept["w"].release()
-            if given:
-                given.release()
-            return dx, dw
-
-        def contraction_backward(dz, need_dx=not x.is_leaf):
-            dw = self.weights._grad_target()
-            dx = _new(xv.shape) if need_dx else None
-            sc.cuda_matmul_bwd(xv.main_ptr, W.main_ptr, dz.main_ptr, dx.main_ptr if need_dx else 0, dw.main_ptr, M, N, K, 1)
-            return dx, dw
-        self.outputs = self._finish_forward(x, z, N, 1, product, contraction_backward, fused_backward)
+            db, dw = b._grad_target(), W._grad_target()
+            dx = _new(shape) if need_dx else None
+            a = kept_a or given
+            sc.matmul_act_bwd(xv._ptr, wv._ptr, z._ptr if code else 0, g.main_ptr, dx._ptr if need_dx else 0, dw._ptr, db._ptr, M, N, K, code,
+                              a.h if a else 0, kept_w.h if kept_w else 0)
+            for k in (kept_a, kept_w, given):
+                if k:
+                    k.release()
+            self._deliver(x, W, b, dx, dw, db)
+        self.outputs = out = self._output(x, z, backward)
         if want_out:
-            self.outputs._rows = out_rows
-        return self.outputs
+            out._rows = _KeptRows(ho)
+        return out
 
     def __repr__(self):
         return f"Dense({self.in_units}→{self.out_units}, act={self.layeract}, params={self.in_units * self.out_units + self.out_units})"
@@ -450,60 +440,56 @@ class Conv2D(_ParamLayer):
 
     def forward(self):
         x = self.inputs = self.inpobj.outputs
-        xv, W = x.value, self.weights.value
+        W, b = self.weights, self.bais
+        xv, wv = x.value, W.value
+        given = x._copies                                    # copies made by the producer of x
         if len(xv.shape) == 3:
-            xv = xv.reshape((1,) + tuple(xv.shape))
-        if len(xv.shape) != 4:
+            xv, given = xv.reshape((1,) + tuple(xv.shape)), None
+        shape = xv.shape
+        if len(shape) != 4:
             raise ValueError("[cuTen]: conv2d expects 4-D tensors (N,C,H,W) and (F,C,KH,KW)")
-        N, C, H, Wd = xv.shape
+        if self.layeract == "softmax":
+            raise ValueError("[Engine]: Softmax VJP requires at least 2D")
+        N, C, H, Wd = shape
         F, (KH, KW), (sh, sw), (ph, pw) = self.out_channels, self.kernel_size, self.stride, self.zero_padding
         OH, OW = (H + 2 * ph - KH) // sh + 1, (Wd + 2 * pw - KW) // sw + 1
-        kept = _KeptCopies()
-        given = getattr(x, "_copies", None) if x.value is xv else None       # copies made by the producer of x
-        pool = getattr(self, "_pool_consumer", None)
+        code = _ACT[self.layeract]
+        pool = self._pool_consumer
         self._fused = None
-        if (FUSE_POOL and pool is not None and self.layeract != "softmax"
-                and sc.conv2d_pool_fusable(N, C, H, Wd, F, KH, KW, sh, sw, ph, pw)):
+        if FUSE_POOL and pool is not None and sc.conv2d_pool_fusable(N, C, H, Wd, F, KH, KW, sh, sw, ph, pw):
             # the pool is folded into this layer's epilogue: z stays a shape without memory
-            z = cuten._wrap(0, (N, F, OH, OW))
+            z = _wrap(0, (N, F, OH, OW))
             z._owns_memory = False
-            pooled = _new((N, F, OH // 2, OW // 2))
-            pmask = cuten._wrap(sc.cuda_malloc_i32(N * F * (OH // 2) * (OW // 2)), (N, F, OH // 2, OW // 2), "int32")
-            pcopies = _KeptCopies()
-
-            def product(bias, code):
-                kept.h, pcopies.h = sc.conv2d_bias_act_pool_fwd_s(xv.main_ptr, W.main_ptr, bias, pooled.main_ptr, pmask.main_ptr, N, C, H,
-                                                                  Wd, F, KH, KW, ph, pw, sh, sw, code, given.h if given else 0,
-                                                                  bool(getattr(pool, "_feeds_conv", False)))
-            self._fused = (pooled, pmask, pcopies)
+            half = (N, F, OH // 2, OW // 2)
+            pooled = _new(half)
+            pmask = _wrap(sc.cuda_malloc_i32(pooled.size), half, "int32")
+            h, hp = sc.conv2d_bias_act_pool_fwd_s(xv.main_ptr, wv.main_ptr, b.value.main_ptr, pooled._ptr, pmask._ptr, N, C, H, Wd, F, KH, KW,
+                                                  ph, pw, sh, sw, code, given.h if given else 0, pool._feeds_conv)
+            self._fused = (pooled, pmask, _KeptCopies(hp) if hp else None)
         else:
             z = _new((N, F, OH, OW))
+            h = sc.conv2d_bias_act_fwd_s(xv.main_ptr, wv.main_ptr, b.value.main_ptr, z._ptr, N, C, H, Wd, F, KH, KW, ph, pw, sh, sw, code,
+                                         given.h if given else 0)
+        kept = _KeptCopies(h) if h else None
+        need_dx = not x.is_leaf
 
-            def product(bias, code):
-                kept.h = sc.conv2d_bias_act_fwd_s(xv.main_ptr, W.main_ptr, bias, z.main_ptr, N, C, H, Wd, F, KH, KW, ph, pw, sh, sw,
-                                                  code, given.h if given else 0)
-
-        def fused_backward(g, y, code, db, need_dx=not x.is_leaf):
-            dw = self.weights._grad_target()
-            dx = _new(xv.shape) if need_dx else None
-            if isinstance(g, _PooledGrad):
-                gptr, gpptr, mptr, ypptr = 0, g.gp.main_ptr, g.mask.main_ptr, g.pooled.main_ptr if g.pooled is not None else 0
+        def backward(g):
+            # pool routing, activation slope, bias gradient, dX and dW in one call
+            db, dw = b._grad_target(), W._grad_target()
+            dx = _new(shape) if need_dx else None
+            if g.__class__ is _PooledGrad:
+                gptr, gpptr, mptr, ypptr = 0, g.gp.main_ptr, g.mask._ptr, g.pooled.main_ptr if g.pooled is not None else 0
             else:
                 gptr, gpptr, mptr, ypptr = g.main_ptr, 0, 0, 0
-            sc.conv2d_act_bwd(W.main_ptr, xv.main_ptr, y.main_ptr, gptr, gpptr, mptr, ypptr, dx.main_ptr if need_dx else 0, dw.main_ptr,
-                              db.main_ptr, N, C, H, Wd, F, KH, KW, sh, sw, ph, pw, code, kept.h or (given.h if given else 0))
-            kept.release()
+            k = kept or given
+            sc.conv2d_act_bwd(wv._ptr, xv._ptr, z._ptr, gptr, gpptr, mptr, ypptr, dx._ptr if need_dx else 0, dw._ptr, db._ptr,
+                              N, C, H, Wd, F, KH, KW, sh, sw, ph, pw, code, k.h if k else 0)
+            if kept:
+                kept.release()
             if given:
                 given.release()
-            return dx, dw
-
-        def contraction_backward(dz, need_dx=not x.is_leaf):
-            dw = self.weights._grad_target()
-            dx = _new(xv.shape) if need_dx else None
-            sc.cuda_conv2d_bwd(W.main_ptr, xv.main_ptr, dz.main_ptr, dx.main_ptr if need_dx else 0, dw.main_ptr,
-                               N, C, H, Wd, F, KH, KW, sh, sw, ph, pw)
-            return dx, dw
-        self.outputs = self._finish_forward(x, z, F, OH * OW, product, contraction_backward, fused_backward, takes_pooled=True)
+            self._deliver(x, W, b, dx, dw, db)
+        self.outputs = self._output(x, z, backward, takes_pooled=True)
         return self.outputs
 
     def __repr__(self):
@@ -528,24 +514,34 @@ class ConvTranspose2D(_ParamLayer):
 
     def forward(self):
         x = self.inputs = self.inpobj.outputs
-        xv, W = x.value, self.weights.value
-        if len(xv.shape) != 4:
+        W, b = self.weights, self.bais
+        xv, wv = x.value, W.value
+        shape = xv.shape
+        if len(shape) != 4:
             raise ValueError("[cuTen]: conv2d_transpose expects 4-D tensors (N,Cin,H,W) and (Cin,Cout,KH,KW)")
-        N, Cin, H, Wd = xv.shape
+        if self.layeract == "softmax":
+            raise ValueError("[Engine]: Softmax VJP requires at least 2D")
+        N, Cin, H, Wd = shape
         Cout, (KH, KW), (sh, sw), (ph, pw) = self.out_channels, self.kernel_size, self.stride, self.zero_padding
         Ho, Wo = (H - 1) * sh - 2 * ph + KH, (Wd - 1) * sw - 2 * pw + KW
+        code = _ACT[self.layeract]
         z = _new((N, Cout, Ho, Wo))
+        sc.conv2DTranspose_bias_act_fwd(xv.main_ptr, wv.main_ptr, b.value.main_ptr, z._ptr, N, Cin, H, Wd, Cout, KH, KW, sh, sw, ph, pw, code)
+        need_dx = not x.is_leaf
 
-        def product(bias, code):
-            sc.conv2DTranspose_bias_act_fwd(xv.main_ptr, W.main_ptr, bias, z.main_ptr, N, Cin, H, Wd, Cout, KH, KW, sh, sw, ph, pw, code)
-
-        def contraction_backward(dz, need_dx=not x.is_leaf):
-            dw = self.weights._grad_target()
-            dx = _new(xv.shape) if need_dx else None
-            sc.cuda_conv2DTranspose_bwd(W.main_ptr, xv.main_ptr, dz.main_ptr, dx.main_ptr if need_dx else 0, dw.main_ptr,
-                                        N, Cin, H, Wd, Cout, KH, KW, sh, sw, ph, pw)
-            return dx, dw
-        self.outputs = self._finish_forward(x, z, Cout, Ho * Wo, product, contraction_backward)
+        def backward(g):
+            db, dw = b._grad_target(), W._grad_target()
+            dz = g
+            if code:
+                dz = _new(z.shape)
+                sc.act_bias_bwd(g.main_ptr, z._ptr, dz._ptr, db._ptr, z.size, Cout, Ho * Wo, code)
+            else:
+                sc.act_bias_bwd(g.main_ptr, 0, g.main_ptr, db._ptr, z.size, Cout, Ho * Wo, 0)
+            dx = _new(shape) if need_dx else None
+            sc.cuda_conv2DTranspose_bwd(wv._ptr, xv._ptr, dz.main_ptr, dx._ptr if need_dx else 0, dw._ptr, N, Cin, H, Wd, Cout, KH, KW,
+                                       sh, sw, ph, pw)
+            self._deliver(x, W, b, dx, dw, db)
+        self.outputs = self._output(x, z, backward)
         return self.outputs
 
     def __repr__(self):
@@ -597,32 +593,29 @@ class _BatchNorm(_ParamLayer):
     def forward(self):
         x = self.inputs = self.inpobj.outputs
         xv = x.value
-        self._shape_ok(xv.shape)
-        N, C = xv.shape[0], xv.shape[1]
-        S = 1
-        for d in xv.shape[2:]:
-            S *= d
+        shape = xv.shape
+        self._shape_ok(shape)
+        N, C = shape[0], shape[1]
+        S = _numel(shape[2:])
         g, b = self.weights, self.bais
-        y, mean, si = _new(xv.shape), _new((C,)), _new((C,))
+        y, mean, si = _new(shape), _new((C,)), _new((C,))
         fwd, bwd = (sc.batchnorm_fwd_sync, sc.batchnorm_bwd_sync) if self.sync else (sc.batchnorm_fwd, sc.batchnorm_bwd)
-        fwd(xv.main_ptr, g.value.main_ptr, b.value.main_ptr, self._rm.main_ptr, self._rv.main_ptr, y.main_ptr,
-                         mean.main_ptr, si.main_ptr, N, C, S, float(self.momentum), float(self.eps), bool(self.training))
-        out = Tensor(y)
-        out._parents = (x, g, b)
+        fwd(xv.main_ptr, g.value.main_ptr, b.value.main_ptr, self._rm.main_ptr, self._rv.main_ptr, y._ptr, mean._ptr, si._ptr, N, C, S,
+            float(self.momentum), float(self.eps), bool(self.training))
+        need_dx = not x.is_leaf
 
-        def backward(dy, need_dx=not x.is_leaf):
+        def backward(dy):
             dg, db = g._grad_target(), b._grad_target()
-            dx = _new(xv.shape)
-            bwd(dy.main_ptr, xv.main_ptr, mean.main_ptr, si.main_ptr, g.value.main_ptr, dx.main_ptr, dg.main_ptr, db.main_ptr, N, C, S)
+            dx = _new(shape)
+            bwd(dy.main_ptr, xv._ptr, mean._ptr, si._ptr, g.value._ptr, dx._ptr, dg._ptr, db._ptr, N, C, S)
             g._accumulate(dg)
             b._accumulate(db)
-            hook = getattr(getattr(self, "_model", None), "_on_grad_ready", None)
-            if hook is not None and g.grad is g._grad_slot and b.grad is b._grad_slot:
-                hook(g)
+            model = self._model
+            if model is not None and model._on_grad_ready is not None and g.grad is g._grad_slot and b.grad is b._grad_slot:
+                model._on_grad_ready(g)
             if need_dx:
                 x._accumulate(dx)
-        out._backward = backward
-        self.outputs = out
+        self.outputs = out = Tensor._of(y, (x, g, b), backward)
         return out
 
 
@@ -668,15 +661,12 @@ class Concatenate(Layer):
         a, b = self.inputs = [l.outputs for l in self.input_layers]
         av, bv = a.value, b.value
         y = av.concatenate2D(bv) if len(av.shape) >= 4 else av.concatenate1D(bv)
-        out = Tensor(y)
-        out._parents = (a, b)
 
         def backward(g):
             da, db = cuten._concat_backward(g, av, bv)
             a._accumulate(da)
             b._accumulate(db)
-        out._backward = backward
-        self.outputs = out
+        self.outputs = out = Tensor._of(y, (a, b), backward)
         return out
 
     def __repr__(self):
@@ -703,40 +693,37 @@ class MaxPool2D(Layer):
         xv = x.value
         if len(xv.shape) != 4:
             raise ValueError("[cuTen]: maxpool2d expects 4-D tensor (N,C,H,W)")
-        N, C, H, W = xv.shape
+        N, C, H, W = shape = xv.shape
         (KH, KW), (sh, sw), (ph, pw) = self.pool_size, self.stride, self.padding
         OH, OW = (H + 2 * ph - KH) // sh + 1, (W + 2 * pw - KW) // sw + 1
         if OH * OW > H * W:
             raise ValueError("[cuTen]: maxpool2d with more outputs than inputs is not supported")
         tiles_exactly = (KH, KW, sh, sw, ph, pw) == (2, 2, 2, 2, 0, 0) and H % 2 == 0 and W % 2 == 0
-        fused = getattr(self.inpobj, "_fused", None)
+        fused = self.inpobj._fused
         if fused is not None:                     # the producing convolution already pooled its output
             y, mask, copies = fused
             self.inpobj._fused = None
         else:
             y = _new((N, C, OH, OW))
-            mask = cuten._wrap(sc.cuda_malloc_i32(N * C * OH * OW), (N, C, OH, OW), "int32")
-            copies = _KeptCopies()
-        if fused is not None:
-            pass
-        elif tiles_exactly and getattr(self, "_feeds_conv", False):   # also leaves the channels-last copies of y for that convolution
-            copies.h = sc.maxpool2x2_fwd_s(xv.main_ptr, y.main_ptr, mask.main_ptr, N, C, H, W)
-        else:
-            sc.cuda_maxpool_fwd(xv.main_ptr, y.main_ptr, mask.main_ptr, N, C, H, W, KH, KW, ph, pw, sh, sw)
-        out = Tensor(y)
-        out._parents = (x,)
-        out._copies = copies
+            mask = _wrap(sc.cuda_malloc_i32(y.size), y.shape, "int32")
+            copies = None
+            if tiles_exactly and self._feeds_conv:   # also leaves the channels-last copies of y for that convolution
+                h = sc.maxpool2x2_fwd_s(xv.main_ptr, y._ptr, mask._ptr, N, C, H, W)
+                copies = _KeptCopies(h) if h else None
+            else:
+                sc.cuda_maxpool_fwd(xv.main_ptr, y._ptr, mask._ptr, N, C, H, W, KH, KW, ph, pw, sh, sw)
         self.mask = mask
 
         def backward(g):
-            if tiles_exactly and getattr(x, "_takes_pooled", False):
-                x._accumulate(_PooledGrad(g, mask, xv.shape, y))   # the producer routes it through the mask itself
+            if tiles_exactly and x._takes_pooled:
+                x._accumulate(_PooledGrad(g, mask, shape, y))   # the producer routes it through the mask itself
                 return
-            dx = _new(xv.shape)
-            sc.cuda_maxpool_bwd(g.main_ptr, mask.main_ptr, dx.main_ptr, N, C, H, W, KH, KW, ph, pw, sh, sw)
+            dx = _new(shape)
+            sc.cuda_maxpool_bwd(g.main_ptr, mask._ptr, dx._ptr, N, C, H, W, KH, KW, ph, pw, sh, sw)
             x._accumulate(dx)
-        out._backward = backward
-        self.outputs = out
+        self.outputs = out = Tensor._of(y, (x,), backward)
+        if copies is not None:
+            out._copies = copies
         return out
 
     def __repr__(self):
@@ -762,16 +749,13 @@ class Unpool2D_Nearest(Layer):
         sw, sh = self.size                       # the reference unpacks (sw, sh) (Seera_init.py:793)
         N, C, H, W = xv.shape
         y = _new((N, C, H * sh, W * sw))
-        sc.cuda_unpooling_fwd(xv.main_ptr, y.main_ptr, N, C, H, W, sh, sw)
-        out = Tensor(y)
-        out._parents = (x,)
+        sc.cuda_unpooling_fwd(xv.main_ptr, y._ptr, N, C, H, W, sh, sw)
 
         def backward(g):
             dx = _new(xv.shape)
-            sc.cuda_unpooling_bwd(g.main_ptr, dx.main_ptr, N, C, H, W, sh, sw)
+            sc.cuda_unpooling_bwd(g.main_ptr, dx._ptr, N, C, H, W, sh, sw)
             x._accumulate(dx)
-        out._backward = backward
-        self.outputs = out
+        self.outputs = out = Tensor._of(y, (x,), backward)
         return out
 
     def __repr__(self):
@@ -787,10 +771,8 @@ class Flatten(Layer):
 
     def forward(self):
         x = self.inputs = self.inpobj.outputs
-        out = Tensor(x.value.flatten())
-        out._parents = (x,)
-        out._backward = lambda g: x._accumulate(g.reshape(x.value.shape))
-        self.outputs = out
+        shape = x.value.shape
+        self.outputs = out = Tensor._of(x.value.flatten(), (x,), lambda g: x._accumulate(g.reshape(shape)))
         return out
 
     def __repr__(self):
@@ -811,6 +793,7 @@ class Sequential:
         self.device = device
         self.model = [layers[0]] + [layer(layers[i]) for i, layer in enumerate(layers[1:])]
         self.world, self._allreduce, self._on_grad_ready = 1, None, None
+        self._modal = [l for l in self.model if hasattr(l, "training")]       # layers that behave differently in evaluation
         self._build_arena()
         for l in self.param_layers:
             l._model = self
@@ -880,14 +863,13 @@ class Sequential:
             self._set_mode(True)
 
     def _set_mode(self, training=True):
-        for l in self.model:
-            if hasattr(l, "training"):
-                l.training = training
+        for l in self._modal:
+            l.training = training
 
     def zero_grad(self):
         """Parameter gradients restart from zero: the next backward writes them instead of adding."""
-        for t in self.parameters():
-            t.grad = None
+        for l in self.param_layers:
+            l.weights.grad = l.bais.grad = None
 
     def get_params(self):
         for l in self.param_layers:
@@ -903,6 +885,8 @@ class Sequential:
         """Copy every parameter gradient into its slot of the gradient arena (no-op for slots already there)."""
         for t in self.parameters():
             g = t.grad
+            if g is t._grad_slot and g is not None:
+                continue
             dst = self.grads.main_ptr + 4 * t._arena_off
             if g is None:
                 sc.cuda_memset(dst, 0, 4 * t._arena_n)
@@ -1109,12 +1093,11 @@ class Loss:
         if tuple(yv.shape) != (N, C):
             raise ValueError(f"[cuTen]: Shapes {tuple(yv.shape)} and {(N, C)} not broadcastable")
         rows, loss, dz = _new((N,)), _new((1,)), _new((N, C))
-        sc.softmax_cce_fwd_bwd(z.main_ptr, yv.main_ptr, y_pred.value.main_ptr, rows.main_ptr, loss.main_ptr, dz.main_ptr,
+        sc.softmax_cce_fwd_bwd(z.main_ptr, yv.main_ptr, y_pred.value.main_ptr, rows._ptr, loss._ptr, dz._ptr,
                                N, C, float(epsilon), float(f32(1.0 / N)))
-        out = Tensor(loss)
-        out._parents = (logits,)
+        # the gradient arrives as the all-ones seed of a scalar loss
+        out = Tensor._of(loss, (logits,), lambda g: (_scale_gradients(dz), logits._accumulate(dz)))
         out._keep = (rows, yv)
-        out._backward = lambda g: (_scale_gradients(dz), logits._accumulate(dz))       # g is the all-ones seed of a scalar loss
         return out
 
     def _elementwise(self, kernel, y_pred, y, *extra):
@@ -1124,10 +1107,8 @@ class Loss:
         part, loss, dp = _new((sc.mse_partials(p.size),)), _new((1,)), _new(p.shape)
         kernel(p.main_ptr, yv.main_ptr, part.main_ptr, loss.main_ptr, dp.main_ptr, p.size,
                float(f32(1.0 / p.size)), *extra)
-        out = Tensor(loss)
-        out._parents = (y_pred,)
+        out = Tensor._of(loss, (y_pred,), lambda g: (_scale_gradients(dp), y_pred._accumulate(dp)))
         out._keep = (part, yv)
-        out._backward = lambda g: (_scale_gradients(dp), y_pred._accumulate(dp))
         return out
 
     def mse(self, y_pred, y):
@@ -1156,6 +1137,7 @@ class _Optimizer:
         self.model = model
         self.use_gpu = True
         self._hyper = cuten(np.zeros(16, np.float32))
+        self._hyper_host = np.zeros(16, np.float32)
         # data parallel: the bucket hooks apply the update range by range behind each bucket's sum (dp.update_in_buckets);
         # step() then only completes the sums
         self.updates_by_bucket = False
@@ -1175,9 +1157,9 @@ class _Optimizer:
         return 1.0 / self.model.world if self.model._allreduce is not None else 1.0
 
     def _upload(self, values):
-        h = np.zeros(16, np.float32)
-        h[:len(values)] = np.asarray(values, np.float32)
-        sc.upload_f32(self._hyper.main_ptr, h)
+        h = self._hyper_host                      # pageable memory: the copy has left it when upload_f32 returns
+        h[:len(values)] = values
+        sc.upload_f32(self._hyper._ptr, h)
 
     @staticmethod
     def from_state(model, state):
