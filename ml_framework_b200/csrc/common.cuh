@@ -103,8 +103,29 @@ struct ProfBytes {
     ~ProfBytes() { profile_end_bytes(bytes, tag); }
 };
 
+// An optimizer launch, described so that a recorded one can be given other scalars (runtime.cu, fused.cu).
+struct OptLaunch {
+    static constexpr int MAX_ARGS = 16;
+    int kind;                      // 0 Adam, 1 SGD
+    float *w; const float *g; float *m, *v;
+    long long n; bool vec; int grid;
+    float scalars[9]; int n_scalars;
+};
+void graph_note_optimizer(const OptLaunch &launch);
+// kernel, grid, block and argument pointers of the launch (the pointers point into `launch`)
+void optimizer_node_params(const OptLaunch &launch, cudaKernelNodeParams &kp, void **args);
+
 // Device float[2]: {dynamic factor of the fp16 gradient copies, its inverse}; both 1 until a loss head sets them (fused.cu).
 float *grad_scale_words();
+
+// runtime.cu: hands the launches of an open seera_batch_begin to the device; the rest of that batch is launched one by one.  Called
+// before whatever a recording cannot hold: a wait, a copy from or to host memory, an event, another recording.
+int batch_flush();
+// RAII bracket over the launches of one entry (no-op inside a batch that is open already).
+struct Batch {
+    Batch(uint64_t tag) { seera_batch_begin(tag); }
+    ~Batch() { seera_batch_end(); }
+};
 
 // Pool-backed scratch for internal use (split-K partials, operand shadows).
 void graph_note_collective();              // runtime.cu: the open capture records a collective

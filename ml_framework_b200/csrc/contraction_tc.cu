@@ -359,6 +359,7 @@ int seera_tc_convT_bwd(const float *Wt, const float *X, const float *dY, float *
 
 // Reads and clears the device status word of the tensor-core kernels (0 = every wait completed).
 int seera_tc_device_status(void) {
+    if (batch_flush()) return -1;
     int *w = tc_status_word();
     if (!w) return -1;
     int v = 0;

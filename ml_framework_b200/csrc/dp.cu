@@ -133,6 +133,7 @@ int seera_dp_unique_id(void *out, int size) {
 }
 
 int seera_dp_init(int rank, int world, const void *unique_id, int size) {
+    if (int s = batch_flush()) return s;
     SEERA_ENSURE();
     Dp &d = dp();
     if (d.comm) return fail(SEERA_E_ARG, "dp_init: already initialised (rank %d of %d)", d.rank, d.world);
@@ -161,6 +162,7 @@ int seera_dp_nccl_version(void) { return dp().version; }
 
 /* Device memory the collectives can use in place: ncclMemAlloc + registration with the communicator. */
 void *seera_dp_alloc(size_t bytes) {
+    if (batch_flush()) return nullptr;
     if (ensure_init() || need_comm("dp_alloc")) return nullptr;
     Dp &d = dp();
     void *p = nullptr;
@@ -185,6 +187,7 @@ void *seera_dp_alloc(size_t bytes) {
 }
 
 int seera_dp_free(void *p) {
+    if (int s = batch_flush()) return s;
     if (!p) return SEERA_OK;
     Dp &d = dp();
     auto it = d.regs.find(p);
@@ -213,6 +216,7 @@ static int red_op(int op, ncclRedOp_t *out) {
 
 /* In-place reduction of n floats over the ranks, enqueued on the COMPUTE stream (ordered with the kernels around it). */
 int seera_dp_allreduce(float *buf, long long n, int op) {
+    if (int s = batch_flush()) return s;
     SEERA_ENSURE();
     if (int s = need_comm("dp_allreduce")) return s;
     if (!buf || n < 0) return fail(SEERA_E_ARG, "dp_allreduce: bad argument");
@@ -227,6 +231,7 @@ int seera_dp_allreduce(float *buf, long long n, int op) {
 }
 
 int seera_dp_broadcast(float *buf, long long n, int root) {
+    if (int s = batch_flush()) return s;
     SEERA_ENSURE();
     if (int s = need_comm("dp_broadcast")) return s;
     if (!buf || n < 0 || root < 0 || root >= dp().world) return fail(SEERA_E_ARG, "dp_broadcast: bad argument");
@@ -241,6 +246,7 @@ int seera_dp_broadcast(float *buf, long long n, int root) {
 /* Sum of floats [begin, end) of `arena` over the ranks on the communication stream, after everything the compute stream
  * holds so far; returns at once. */
 int seera_dp_reduce_range(float *arena, long long begin, long long end) {
+    if (int s = batch_flush()) return s;
     SEERA_ENSURE();
     if (int s = need_comm("dp_reduce_range")) return s;
     if (!arena || begin < 0 || end < begin) return fail(SEERA_E_ARG, "dp_reduce_range: bad range");
@@ -261,6 +267,7 @@ int seera_dp_reduce_range(float *arena, long long begin, long long end) {
  * Only for entries that take no scratch memory from the pool (the optimizer steps): the pool recycles blocks in the order
  * of ONE stream. */
 int seera_dp_side_begin(void) {
+    if (int s = batch_flush()) return s;
     SEERA_ENSURE();
     if (int s = need_comm("dp_side_begin")) return s;
     Dp &d = dp();
@@ -274,6 +281,7 @@ int seera_dp_side_begin(void) {
     return SEERA_OK;
 }
 int seera_dp_side_end(void) {
+    if (int s = batch_flush()) return s;
     Dp &d = dp();
     if (!d.side) return SEERA_OK;
     rt().stream = d.main_stream;
@@ -283,6 +291,7 @@ int seera_dp_side_end(void) {
 
 /* The compute stream waits for every range enqueued since the last join. */
 int seera_dp_join(void) {
+    if (int s = batch_flush()) return s;
     SEERA_ENSURE();
     Dp &d = dp();
     if (d.side) seera_dp_side_end();
@@ -308,6 +317,7 @@ int seera_dp_poll(void) {
  * or on an asynchronous NCCL error the communicator is aborted, so that the process can go on without it, and an error
  * status is returned.  Not allowed during a capture. */
 int seera_dp_wait_host(int timeout_ms) {
+    if (int s = batch_flush()) return s;
     SEERA_ENSURE();
     if (rt().capturing) return fail(SEERA_E_ARG, "dp_wait_host: not allowed while a graph is being captured");
     Dp &d = dp();
@@ -349,6 +359,7 @@ int seera_dp_wait_host(int timeout_ms) {
 /* Drops the communicator without talking to the peers (ncclCommAbort): the way out when one of them is known to be gone.
  * Blocks seera_dp_alloc handed out stay allocated until the process ends. */
 int seera_dp_abort(void) {
+    if (int s = batch_flush()) return s;
     Dp &d = dp();
     seera_dp_side_end();
     if (!d.comm) return SEERA_OK;
@@ -362,6 +373,7 @@ int seera_dp_abort(void) {
 }
 
 int seera_dp_finalize(void) {
+    if (int s = batch_flush()) return s;
     Dp &d = dp();
     seera_dp_side_end();
     if (!d.comm) return SEERA_OK;

@@ -330,6 +330,18 @@ __global__ void __launch_bounds__(256) sgd_kernel(float *__restrict__ w, const f
     sgd_range(w, g, vel, n, vec, lr, mu, gs);
 }
 
+void optimizer_node_params(const OptLaunch &l, cudaKernelNodeParams &kp, void **args) {
+    OptLaunch *o = const_cast<OptLaunch *>(&l);
+    int i = 0;
+    args[i++] = &o->w; args[i++] = &o->g; args[i++] = &o->m;
+    if (l.kind == 0) args[i++] = &o->v;
+    args[i++] = &o->n; args[i++] = &o->vec;
+    if (l.kind == 0) { static_assert(sizeof(AdamArgs) == 9 * sizeof(float), "nine scalars in declaration order"); args[i++] = o->scalars; }
+    else for (int k = 0; k < 3; k++) args[i++] = &o->scalars[k];
+    kp.func = l.kind == 0 ? (void *)adam_kernel : (void *)sgd_kernel;
+    kp.gridDim = dim3(l.grid); kp.blockDim = dim3(256); kp.sharedMemBytes = 0; kp.kernelParams = args; kp.extra = nullptr;
+}
+
 // ---- dynamic factor of the fp16 gradient copies -------------------------------------------------------------------
 __global__ void grad_scale_reset_kernel(float *w) {
     if (threadIdx.x == 0) { w[0] = 1.f; w[1] = 1.f; reinterpret_cast<unsigned *>(w)[2] = 0u; w[3] = 0.f; }
@@ -586,8 +598,10 @@ int seera_adam_step(float *w, const float *g, float *m, float *v, int n, float l
     bool vec = aligned16(w) && aligned16(g) && aligned16(m) && aligned16(v);
     AdamArgs a{lr, beta1, omb1, beta2, omb2, eps, c1, c2, grad_scale};
     ProfBytes pb(28.0 * n, "adam");
-    adam_kernel<<<stride_grid(vec ? (n + 3) / 4 : n), 256, 0, rt().stream>>>(w, g, m, v, n, vec, a);
+    const int grid = stride_grid(vec ? (n + 3) / 4 : n);
+    adam_kernel<<<grid, 256, 0, rt().stream>>>(w, g, m, v, n, vec, a);
     SEERA_LAUNCH_CHECK("adam_step");
+    if (rt().capturing) graph_note_optimizer({0, w, g, m, v, n, vec, grid, {lr, beta1, omb1, beta2, omb2, eps, c1, c2, grad_scale}, 9});
     return SEERA_OK;
 }
 
@@ -618,8 +632,10 @@ int seera_sgd_step(float *w, const float *g, float *vel, int n, float lr, float 
     if (n == 0) return SEERA_OK;
     bool vec = aligned16(w) && aligned16(g) && aligned16(vel);
     ProfBytes pb(20.0 * n, "sgd");
-    sgd_kernel<<<stride_grid(vec ? (n + 3) / 4 : n), 256, 0, rt().stream>>>(w, g, vel, n, vec, lr, momentum, grad_scale);
+    const int grid = stride_grid(vec ? (n + 3) / 4 : n);
+    sgd_kernel<<<grid, 256, 0, rt().stream>>>(w, g, vel, n, vec, lr, momentum, grad_scale);
     SEERA_LAUNCH_CHECK("sgd_step");
+    if (rt().capturing) graph_note_optimizer({1, w, g, vel, nullptr, n, vec, grid, {lr, momentum, grad_scale}, 3});
     return SEERA_OK;
 }
 

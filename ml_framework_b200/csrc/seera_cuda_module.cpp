@@ -178,6 +178,9 @@ PYBIND11_MODULE(seera_cuda, m) {
     m.def("graph_end", []() { return ckp(seera_graph_end()); });
     m.def("graph_launch", [](uptr g) { ck(seera_graph_launch(P<void>(g))); });
     m.def("graph_destroy", [](uptr g) { ck(seera_graph_destroy(P<void>(g))); });
+    m.def("batch_begin", [](uint64_t tag) { ck(seera_batch_begin(tag)); });
+    m.def("batch_end", []() { ck(seera_batch_end()); });
+    m.def("graph_set_scalars", [](uptr g, const std::vector<float> &v) { ck(seera_graph_set_scalars(P<void>(g), v.data(), (int)v.size())); });
     m.def("is_capturing", []() { return seera_is_capturing() != 0; });
     m.def("cuda_adam_step_dev", [](uptr w, uptr g, uptr mm, uptr v, int n, uptr h) {
         ck(seera_adam_step_dev(P<F>(w), P<const F>(g), P<F>(mm), P<F>(v), n, P<const F>(h))); });

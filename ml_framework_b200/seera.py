@@ -44,6 +44,31 @@ def _new(shape):
     return _wrap(_malloc(_numel(shape)), shape)
 
 
+# One submission for the launches of a phase (seera_batch_begin / _end): inside, the engine records its launches, and the end hands
+# them over as one graph - a third of the host time per launch and no gaps between them on the device.  A tag names what decides
+# which launches follow: the layers, the input's shape, the precision.  The first pass under a tag runs launch by launch, so that
+# whatever is set up on first use is set up outside a recording.
+_batch_begin, _batch_end = getattr(sc, "batch_begin", None), getattr(sc, "batch_end", None)
+_tags_seen = set()
+
+
+def _open_batch(tag):
+    """True if a batch was opened; the caller then owes a _batch_end()."""
+    if tag is None or _batch_begin is None:
+        return False
+    if tag not in _tags_seen:
+        if len(_tags_seen) > 4096:
+            _tags_seen.clear()
+        _tags_seen.add(tag)
+        return False
+    _batch_begin(tag)
+    return True
+
+
+def _make_tag(*what):
+    return hash(what) & 0x7fffffffffffffff
+
+
 # ─────────────────────────────────────────────────────────────────────────────────────────────
 # Tensor: a device value, its gradient, and the closure that propagates the gradient
 # ─────────────────────────────────────────────────────────────────────────────────────────────
@@ -59,6 +84,7 @@ class Tensor:
     _takes_pooled = False            # its backward takes the gradient of a 2x2 max-pool of it in pooled form
     _copies = None                   # channels-last copies of the value, made by its producer for a convolution
     _rows = None                     # row-major copies of the value, made by its producer for a Dense layer
+    _tag = None                      # batch tag of the model pass it came from
 
     def __init__(self, value, dtype="float32", is_leaf=False, device="cuda"):
         if isinstance(value, Tensor):
@@ -216,6 +242,15 @@ class autograd4nn:
         self.backward()
 
     def backward(self):
+        tag = self.hook._tag
+        opened = _open_batch(None if tag is None else _make_tag(tag, "backward"))
+        try:
+            self._run()
+        finally:
+            if opened:
+                _batch_end()
+
+    def _run(self):
         order, seen = [], set()
         stack = [self.hook]
         while stack:                                   # iterative DFS: no recursion limit on deep nets
@@ -782,6 +817,11 @@ class Flatten(Layer):
 # ─────────────────────────────────────────────────────────────────────────────────────────────
 # Sequential
 # ─────────────────────────────────────────────────────────────────────────────────────────────
+# what of a layer decides which launches it makes
+_STRUCTURE = ("in_units", "out_units", "layeract", "in_channels", "out_channels", "kernel_size", "stride", "zero_padding", "pool_size",
+              "padding", "size", "_num")
+
+
 class Sequential:
     def __init__(self, layers, device="cuda"):
         if not isinstance(layers, list):
@@ -794,6 +834,7 @@ class Sequential:
         self.model = [layers[0]] + [layer(layers[i]) for i, layer in enumerate(layers[1:])]
         self.world, self._allreduce, self._on_grad_ready = 1, None, None
         self._modal = [l for l in self.model if hasattr(l, "training")]       # layers that behave differently in evaluation
+        self._structure = hash(tuple((l.__class__.__name__,) + tuple(getattr(l, k, None) for k in _STRUCTURE) for l in self.model))
         self._build_arena()
         for l in self.param_layers:
             l._model = self
@@ -849,10 +890,26 @@ class Sequential:
             if not isinstance(X, Tensor):
                 raise TypeError("Input must be a Tensor or numpy array.")
             self.model[0].inputs = X
-        out = None
-        for layer in self.model:
-            out = layer.forward()
+        tag = self._tag("forward")
+        opened = _open_batch(tag)
+        try:
+            out = None
+            for layer in self.model:
+                out = layer.forward()
+        finally:
+            if opened:
+                _batch_end()
+        if tag is not None:
+            out._tag = tag
         return out
+
+    def _tag(self, *phase):
+        """Tag of a pass over the current input, or None where it does not run as one batch: with gradients exchanged between
+        ranks during backward, other streams take part in it."""
+        X = self.model[0].inputs
+        if self._allreduce is not None or self._on_grad_ready is not None or not isinstance(X, Tensor):
+            return None
+        return _make_tag(self._structure, X.value.shape, sc.get_precision(), FUSE_POOL, DENSE_EPILOGUE_COPIES, *phase)
 
     def predict(self, X):
         """Forward in evaluation mode: BatchNorm layers normalise with their running statistics (Seera.py:690-700)."""
@@ -945,10 +1002,16 @@ class Sequential:
                     else:
                         yv = cuten._wrap(st["dy"].main_ptr, (m,) + y.shape[1:])
                         yv._owns_memory = False
-                    loss = Loss(self.forward(xb), Tensor(yv, is_leaf=True))
-                    self.zero_grad()
-                    autograd4nn(loss)
-                    Optimizer.step()
+                    self.model[0].inputs = xb
+                    opened = _open_batch(self._tag("fit", yv.shape, Optimizer.__class__.__name__))
+                    try:
+                        loss = Loss(self.forward(), Tensor(yv, is_leaf=True))
+                        self.zero_grad()
+                        autograd4nn(loss)
+                        Optimizer.step()
+                    finally:
+                        if opened:
+                            _batch_end()
                     if pending is not None:         # the device is already busy with step k
                         sc.copy_synchronize()
                         total += float(slots[(k - 1) & 1])
@@ -1098,6 +1161,7 @@ class Loss:
         # the gradient arrives as the all-ones seed of a scalar loss
         out = Tensor._of(loss, (logits,), lambda g: (_scale_gradients(dz), logits._accumulate(dz)))
         out._keep = (rows, yv)
+        out._tag = y_pred._tag
         return out
 
     def _elementwise(self, kernel, y_pred, y, *extra):
@@ -1109,6 +1173,7 @@ class Loss:
                float(f32(1.0 / p.size)), *extra)
         out = Tensor._of(loss, (y_pred,), lambda g: (_scale_gradients(dp), y_pred._accumulate(dp)))
         out._keep = (part, yv)
+        out._tag = y_pred._tag
         return out
 
     def mse(self, y_pred, y):
@@ -1142,6 +1207,9 @@ class _Optimizer:
         # step() then only completes the sums
         self.updates_by_bucket = False
         self._advanced = False
+        # a recording whose replays replace the scalars in the graph itself (Trainer.capture), instead of reading them from the
+        # device buffer
+        self._scalars_in_graph = False
 
     def _state(self):
         n = max(self.model.n_arena, 1)
@@ -1192,14 +1260,24 @@ class _Optimizer:
         if end > begin:
             self._enqueue(begin, end)
 
+    def advance(self):
+        """Puts the scalars of the next update on the device and counts it."""
+        self._upload(self._scalars())
+
     def step(self):
-        """One update.  Outside a capture this also refreshes the device scalars and advances the step count."""
-        if not sc.is_capturing() and not self._advanced:
-            self.advance()
+        """One update; outside a capture this also advances the step count."""
+        by_bucket = self.updates_by_bucket and self.model._allreduce is not None
+        capturing = sc.is_capturing()
+        scalars = None
+        if by_bucket:
+            if not capturing and not self._advanced:
+                self.advance()
+        elif not capturing or self._scalars_in_graph:
+            scalars = self._scalars(count=not capturing)      # by value with the launch: nothing to upload
         self._advanced = False
         self._grads_ready()
-        if not (self.updates_by_bucket and self.model._allreduce is not None):
-            self._enqueue()
+        if not by_bucket:
+            self._enqueue(scalars=scalars)
 
 
 class SGD(_Optimizer):
@@ -1210,17 +1288,21 @@ class SGD(_Optimizer):
         self.lr, self.momentum = lr, momentum
         self.velocity = self._state()
 
-    def advance(self):
-        self._upload([self.lr, self.momentum, self._grad_scale()])
+    def _scalars(self, count=True):
+        return [self.lr, self.momentum, self._grad_scale()]
 
     def state_dict(self):
         return {"kind": "sgd", "lr": self.lr, "momentum": self.momentum, "velocity": self.velocity.to_host_f32().copy()}
 
-    def _enqueue(self, begin=0, end=None):
+    def _enqueue(self, begin=0, end=None, scalars=None):
         m = self.model
         end = m.n_arena if end is None else end
         o = 4 * begin
-        sc.cuda_sgd_step_dev(m.params.main_ptr + o, m.grads.main_ptr + o, self.velocity.main_ptr + o, end - begin, self._hyper.main_ptr)
+        at = (m.params.main_ptr + o, m.grads.main_ptr + o, self.velocity.main_ptr + o, end - begin)
+        if scalars is None:
+            sc.cuda_sgd_step_dev(*at, self._hyper.main_ptr)
+        else:
+            sc.cuda_sgd_step(*at, *scalars)
 
 
 class Adam(_Optimizer):
@@ -1231,18 +1313,23 @@ class Adam(_Optimizer):
         self.lr, self.beta1, self.beta2, self.eps, self.t = lr, beta1, beta2, eps, 1
         self.m, self.v = self._state(), self._state()
 
-    def advance(self):
-        b1, b2 = self.beta1, self.beta2
-        self._upload([self.lr, b1, 1 - b1, b2, 1 - b2, self.eps, 1 - b1 ** self.t, 1 - b2 ** self.t, self._grad_scale()])
-        self.t += 1
+    def _scalars(self, count=True):
+        """The update's scalars at the current step; `count` moves on to the next step."""
+        b1, b2, t = self.beta1, self.beta2, self.t
+        if count:
+            self.t = t + 1
+        return [self.lr, b1, 1 - b1, b2, 1 - b2, self.eps, 1 - b1 ** t, 1 - b2 ** t, self._grad_scale()]
 
     def state_dict(self):
         return {"kind": "adam", "lr": self.lr, "beta1": self.beta1, "beta2": self.beta2, "eps": self.eps, "t": self.t,
                 "m": self.m.to_host_f32().copy(), "v": self.v.to_host_f32().copy()}
 
-    def _enqueue(self, begin=0, end=None):
+    def _enqueue(self, begin=0, end=None, scalars=None):
         md = self.model
         end = md.n_arena if end is None else end
         o = 4 * begin
-        sc.cuda_adam_step_dev(md.params.main_ptr + o, md.grads.main_ptr + o, self.m.main_ptr + o, self.v.main_ptr + o, end - begin,
-                              self._hyper.main_ptr)
+        at = (md.params.main_ptr + o, md.grads.main_ptr + o, self.m.main_ptr + o, self.v.main_ptr + o, end - begin)
+        if scalars is None:
+            sc.cuda_adam_step_dev(*at, self._hyper.main_ptr)
+        else:
+            sc.cuda_adam_step(*at, *scalars)

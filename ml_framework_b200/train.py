@@ -82,9 +82,17 @@ class Trainer:
         return loss
 
     def step(self, X, Y):
+        X = X if isinstance(X, S.Tensor) else S.Tensor(X, is_leaf=True)
+        Y = Y if isinstance(Y, S.Tensor) else S.Tensor(Y, is_leaf=True)
         self.opt.begin_step()
-        loss = self.forward_backward(X, Y)
-        self.opt.step()
+        self.model.model[0].inputs = X
+        opened = S._open_batch(self.model._tag("step", self.precision, self.work.loss, self.work.opt["kind"]))
+        try:
+            loss = self.forward_backward(X, Y)
+            self.opt.step()
+        finally:
+            if opened:
+                S._batch_end()
         return loss
 
     # ---- whole-step CUDA graph -------------------------------------------------------------------
@@ -99,6 +107,8 @@ class Trainer:
         if self.model._allreduce is not None and not getattr(self.model, "_collectives_capturable", False):
             raise RuntimeError("capture needs collectives that can be recorded (dp.attach_nccl); with other collectives use "
                                "capture_data_parallel")
+        # the update's scalars travel with the recorded launch and are replaced in it before each replay
+        self.opt._scalars_in_graph = self._scalars_in_graph = not self.opt.updates_by_bucket and hasattr(sc, "graph_set_scalars")
         sc.graph_begin()
         try:
             loss = self.step(X, Y)
@@ -108,12 +118,17 @@ class Trainer:
             except Exception:
                 pass
             raise
+        finally:
+            self.opt._scalars_in_graph = False
         self._graph = sc.graph_end()
         self._graph_keep = (X, Y, loss, self.pred)
         return loss
 
     def replay(self):
-        self.opt.advance()
+        if self._scalars_in_graph:
+            sc.graph_set_scalars(self._graph, self.opt._scalars())
+        else:
+            self.opt.advance()
         sc.graph_launch(self._graph)
         return self._graph_keep[2]
 
