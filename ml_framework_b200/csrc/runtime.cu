@@ -12,6 +12,7 @@
 #include <cstring>
 #include <string>
 #include <map>
+#include <mutex>
 #include <unordered_map>
 #include <vector>
 
@@ -243,6 +244,9 @@ void graphs_with_collectives_release() {
 
 using namespace seera;
 
+static void pinned_trim();
+static void pinned_other_streams();
+
 extern "C" {
 
 int seera_init(int device) {
@@ -282,6 +286,7 @@ int seera_synchronize(void) {
 int seera_set_stream(void *s) {
     SEERA_ENSURE();
     if (int e = batch_flush()) return e;
+    pinned_other_streams();
     rt().stream = s ? reinterpret_cast<cudaStream_t>(s) : rt().own_stream;
     return SEERA_OK;
 }
@@ -434,6 +439,7 @@ int seera_pool_trim(void) {
         for (void *b : kv.second) { cudaFree(b); p.reserved -= kv.first; }
         kv.second.clear();
     }
+    pinned_trim();
     return SEERA_OK;
 }
 size_t seera_pool_bytes_reserved(void) { return pool().reserved; }
@@ -536,13 +542,91 @@ int seera_batch_end(void) {
     return --b.depth ? SEERA_OK : batch_flush();
 }
 
+// Page-locked host blocks.  The driver takes milliseconds to pin and unpin a block (3 ms for 200 KB measured; a training loop of
+// eight steps took 1 to 7 ms for its five blocks and 0.9 ms for the steps), so freed blocks are kept for the next request of
+// their rounded size, up to PINNED_KEPT_MAX bytes; seera_pool_trim gives them back.  A kept block is handed out again once the work that
+// was queued when it was freed has passed, since a copy may still be reading it.
+}  // extern "C"
+static cudaStream_t copy_stream(int *status);
+namespace {
+constexpr size_t PINNED_KEPT_MAX = size_t(256) << 20;
+struct PinnedBlock { void *p; cudaEvent_t compute, copy; };
+struct Pinned {
+    std::mutex mu;
+    std::unordered_map<void *, size_t> live;
+    std::map<size_t, std::vector<PinnedBlock>> kept;
+    size_t kept_bytes = 0;
+    bool other_streams = false;                         // seera_set_stream was used: a copy may be queued on a stream not watched here
+};
+Pinned &pinned() { static Pinned p; return p; }
+size_t pinned_round(size_t n) {                       // powers of two from a page up to 1 MiB, then 2 MiB granules
+    if (n > (size_t(1) << 20)) return (n + (size_t(2) << 20) - 1) & ~((size_t(2) << 20) - 1);
+    size_t r = 4096;
+    while (r < n) r <<= 1;
+    return r;
+}
+void pinned_drop(PinnedBlock &b) {
+    cudaEventDestroy(b.compute); cudaEventDestroy(b.copy);
+    cudaFreeHost(b.p);
+}
+}  // namespace
+static void pinned_other_streams() { pinned().other_streams = true; }
+static void pinned_trim() {
+    Pinned &k = pinned();
+    std::lock_guard<std::mutex> lock(k.mu);
+    for (auto &kv : k.kept) for (PinnedBlock &b : kv.second) pinned_drop(b);
+    k.kept.clear();
+    k.kept_bytes = 0;
+}
+extern "C" {
 void *seera_host_alloc_pinned(size_t n) {
     if (ensure_init()) return nullptr;
+    Pinned &k = pinned();
+    const size_t sz = pinned_round(n);
+    std::lock_guard<std::mutex> lock(k.mu);
+    auto it = k.kept.find(sz);
+    if (it != k.kept.end())
+        for (size_t i = 0; i < it->second.size(); i++) {
+            PinnedBlock b = it->second[i];
+            if (cudaEventQuery(b.compute) != cudaSuccess || cudaEventQuery(b.copy) != cudaSuccess) { cudaGetLastError(); continue; }
+            it->second.erase(it->second.begin() + (long)i);
+            k.kept_bytes -= sz;
+            cudaEventDestroy(b.compute); cudaEventDestroy(b.copy);
+            k.live[b.p] = sz;
+            return b.p;
+        }
     void *p = nullptr;
-    if (cudaMallocHost(&p, n ? n : 1) != cudaSuccess) { cudaGetLastError(); fail(SEERA_E_OOM, "cudaMallocHost(%zu)", n); return nullptr; }
+    if (cudaMallocHost(&p, sz) != cudaSuccess) { cudaGetLastError(); fail(SEERA_E_OOM, "cudaMallocHost(%zu)", n); return nullptr; }
+    k.live[p] = sz;
     return p;
 }
-int seera_host_free_pinned(void *p) { return p ? check_cuda(cudaFreeHost(p), "cudaFreeHost") : SEERA_OK; }
+int seera_host_free_pinned(void *p) {
+    if (!p) return SEERA_OK;
+    if (int s = batch_flush()) return s;
+    Pinned &k = pinned();
+    std::lock_guard<std::mutex> lock(k.mu);
+    auto it = k.live.find(p);
+    const size_t sz = it == k.live.end() ? 0 : it->second;
+    if (sz) k.live.erase(it);
+    int st = SEERA_OK;
+    cudaStream_t cs = nullptr;
+    if (sz && !k.other_streams && !rt().capturing && rt().stream && k.kept_bytes + sz <= PINNED_KEPT_MAX && (cs = copy_stream(&st))) {
+        PinnedBlock b{p, nullptr, nullptr};
+        bool ok = cudaEventCreateWithFlags(&b.compute, cudaEventDisableTiming) == cudaSuccess;
+        if (ok && cudaEventCreateWithFlags(&b.copy, cudaEventDisableTiming) != cudaSuccess) { cudaEventDestroy(b.compute); ok = false; }
+        if (ok && (cudaEventRecord(b.compute, rt().stream) != cudaSuccess || cudaEventRecord(b.copy, cs) != cudaSuccess)) {
+            cudaEventDestroy(b.compute); cudaEventDestroy(b.copy);
+            ok = false;
+        }
+        if (ok) {
+            k.kept[sz].push_back(b);
+            k.kept_bytes += sz;
+            return SEERA_OK;
+        }
+        cudaGetLastError();
+    }
+    return check_cuda(cudaFreeHost(p), "cudaFreeHost");
+}
 
 int seera_cuda_memcopy_devicetodevice(void *dst, const void *src, int num_elem) {
     SEERA_ENSURE();
@@ -591,6 +675,7 @@ int seera_stream_delay(int microseconds) {
 // ---- copy stream: host<->device transfers that overlap the compute stream -----------------------------------
 // One extra non-blocking stream per process.  Ordering against the compute stream is explicit: each fence records an
 // event at the current tail of one stream and makes the other wait for it, so "everything queued so far" is the unit.
+}  // extern "C"
 static cudaStream_t copy_stream(int *status) {
     static cudaStream_t cs[64] = {nullptr};
     const int dev = rt().device & 63;
@@ -600,6 +685,7 @@ static cudaStream_t copy_stream(int *status) {
     }
     return cs[dev];
 }
+extern "C" {
 static int fence(cudaStream_t from, cudaStream_t to, const char *what) {
     cudaEvent_t ev;
     if (int s = check_cuda(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming), what)) return s;
