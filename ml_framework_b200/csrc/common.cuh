@@ -88,6 +88,20 @@ inline void launch_sum_splits(const float *partial, float *out, int n, int split
         if (_e != cudaSuccess) return seera::check_cuda(_e, name);                 \
     } while (0)
 
+// Two fp32 multiply-adds per instruction (each half rounded as fmaf rounds): the way to the full fp32 rate on sm_100.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 ffma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float &lo, float &hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // Contraction profile (seera_profile_enable): bracket a launch sequence with events and book its FLOPs.

@@ -278,80 +278,163 @@ int conv_few_fwd(const float *X, const float *Wt, const float *bias, float *Y, i
 // per channel come from shared memory as broadcast 16-byte reads.  The layer output is never stored: pooled values, the
 // window-local argmax (scan order (0,0), (0,1), (1,0), (1,1), strict comparison: the first maximum wins, as in
 // cuda_maxpool_fwd) and the channels-last bf16 copies of the pooled tensor for the next convolution are.  Exact fp32.
-__global__ void __launch_bounds__(256, 3) conv3x3_pool_kernel(const float *__restrict__ x, const float *__restrict__ Wt,
+//
+// A warp works on 32 windows x FW filters; FW = 16 wherever the filter count allows, so that an input value is fetched and duplicated
+// for the packed multiply-adds once per 16 filters and a lane writes 32 contiguous bytes of each channels-last copy, a whole sector.
+// STAGED: the block copies a band of window rows with its border of zeros into shared memory while it computes on the band before,
+// and lanes read their patches from there, 8 bytes at a time and with nothing to test; else (an image too wide for a band) from
+// global memory with the border tested per value, which costs a third of all instructions and leaves the loads' latency exposed.
+// VGG's first layer (3 -> 64 channels, 32 x 32), 777 images: 117 us with 8 filters per warp, scalar multiply-adds and unstaged
+// loads; the multiply-adds alone need 38 us of the fp32 pipe.
+struct PoolBand {
+    int rows, pitch;           // padded input rows of a band and floats per row (even)
+    int window_rows, per_image;    // window rows of a band, bands per image
+    int buffers;
+    FastDiv by_bands, by_pitch, by_rows;
+};
+__device__ __forceinline__ void cp_async4(uint32_t dst, const float *src, bool take) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(take ? 4 : 0) : "memory");
+}
+template <int FW, bool RELU, bool STAGED>
+__global__ void __launch_bounds__(256, 2) conv3x3_pool_kernel(const float *__restrict__ x, const float *__restrict__ Wt,
                                                            const float *__restrict__ bias, PoolOut po, int NB, int C, int H, int W,
                                                            int F, int OH, int OW, int ph, int pw, int act, FastDiv by_Pq,
-                                                           FastDiv by_OWq) {
-    extern __shared__ float wk[];                         // [C][9][F], then [F] biases
+                                                           FastDiv by_OWq, FastDiv by_groups, PoolBand band) {
+    extern __shared__ __align__(16) float wk[];           // [C][9][F], [F] biases, then the bands
     for (int e = threadIdx.x; e < C * 9 * F; e += blockDim.x) {
         const int f = e % F, k = e / F;                   // k = c * 9 + t
         wk[e] = __ldg(Wt + (long long)f * C * 9 + k);
     }
     for (int e = threadIdx.x; e < F; e += blockDim.x) wk[C * 9 * F + e] = bias ? __ldg(bias + e) : 0.f;
-    __syncthreads();
+    float *bands = wk + (C * 9 + 1) * F;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int OWq = OW >> 1, Pq = (OH >> 1) * OWq;
-    const long long windows = (long long)NB * Pq;
-    const long long tiles = (windows + 31) / 32;
-    for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-        const long long wl = tile * 32 + lane;
-        if (wl >= windows) continue;
-        const int wi = (int)wl, n = by_Pq.div(wi), wrem = wi - n * Pq, ohq = by_OWq.div(wrem), owq = wrem - ohq * OWq;
-        const int ih0 = 2 * ohq - ph, iw0 = 2 * owq - pw;
-        bool rowok[4], colok[4];
+    const int OWq = OW >> 1, OHq = OH >> 1, Pq = OHq * OWq, plane = H * W;
+    const int groups = by_groups.d, bplane = band.rows * band.pitch, bsize = C * bplane;
+
+    // one warp: 32 windows x FW filters; the patch of channel c is fetched by fetch(c, v)
+    auto compute = [&](int n, int wrem, int f0, bool live, auto fetch) {
+        f32x2 acc[4][FW / 2];                             // [pixel of the window][pair of filters]
 #pragma unroll
-        for (int i = 0; i < 4; i++) { rowok[i] = (unsigned)(ih0 + i) < (unsigned)H; colok[i] = (unsigned)(iw0 + i) < (unsigned)W; }
-        const float *xn = x + (long long)n * C * H * W + (long long)ih0 * W + iw0;
-        for (int fg = warp; fg * 8 < F; fg += 8) {
-            const int f0 = fg * 8;
-            float acc[4][8];
+        for (int p = 0; p < 4; p++)
 #pragma unroll
-            for (int p = 0; p < 4; p++)
+            for (int f = 0; f < FW / 2; f++) acc[p][f] = 0ull;
+        const float *wc = wk + f0;
+        for (int c = 0; c < C; c++, wc += 9 * F) {
+            f32x2 v[4][4];
+            fetch(c, v);
 #pragma unroll
-                for (int f = 0; f < 8; f++) acc[p][f] = 0.f;
-            for (int c = 0; c < C; c++) {
-                const float *xc = xn + (long long)c * H * W;
-                float v[4][4];
+            for (int t = 0; t < 9; t++) {
+                const int r = t / 3, s = t - r * 3;
 #pragma unroll
-                for (int i = 0; i < 4; i++)
-#pragma unroll
-                    for (int j = 0; j < 4; j++) v[i][j] = (rowok[i] && colok[j]) ? __ldg(xc + i * W + j) : 0.f;
-#pragma unroll
-                for (int t = 0; t < 9; t++) {
-                    const float4 wa = *reinterpret_cast<const float4 *>(wk + (c * 9 + t) * F + f0);
-                    const float4 wb = *reinterpret_cast<const float4 *>(wk + (c * 9 + t) * F + f0 + 4);
-                    const float w8[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
-                    const int r = t / 3, s = t - r * 3;
+                for (int f = 0; f < FW / 4; f++) {
+                    const ulonglong2 w2 = *reinterpret_cast<const ulonglong2 *>(wc + t * F + 4 * f);
 #pragma unroll
                     for (int p = 0; p < 4; p++) {
-                        const float a = v[(p >> 1) + r][(p & 1) + s];
-#pragma unroll
-                        for (int f = 0; f < 8; f++) acc[p][f] = fmaf(a, w8[f], acc[p][f]);
+                        acc[p][2 * f] = ffma2(v[(p >> 1) + r][(p & 1) + s], w2.x, acc[p][2 * f]);
+                        acc[p][2 * f + 1] = ffma2(v[(p >> 1) + r][(p & 1) + s], w2.y, acc[p][2 * f + 1]);
                     }
                 }
             }
+        }
+        if (!live) return;
+        const float *bk = wk + C * 9 * F + f0;
+        const long long o0 = ((long long)n * F + f0) * Pq + wrem, c0 = ((long long)n * Pq + wrem) * po.Cp + f0;
+        float *op = po.pooled + o0;
+        int *om = po.mask + o0;
+#pragma unroll
+        for (int h = 0; h < FW / 8; h++) {
             float mx[8];
 #pragma unroll
             for (int f = 0; f < 8; f++) {
-                const float b = wk[C * 9 * F + f0 + f];
+                const float b = bk[8 * h + f];
                 float m = -3.402823466e+38f;
                 int id = 0;
 #pragma unroll
                 for (int p = 0; p < 4; p++) {
-                    const float z = epilogue_act(acc[p][f] + b, act);
+                    float lo, hi;
+                    unpack2(acc[p][4 * h + (f >> 1)], lo, hi);
+                    float z = ((f & 1) ? hi : lo) + b;
+                    if (!RELU) z = epilogue_act(z, act);
                     if (z > m) { m = z; id = p; }
                 }
-                const long long q = ((long long)n * F + f0 + f) * Pq + wrem;
-                po.pooled[q] = m;
-                po.mask[q] = id;
+                // relu after the maximum: the same value and, since a window without a positive entry is all zeros, the same index
+                if (RELU && !(m > 0.f)) { m = 0.f; id = 0; }
+                op[(unsigned)((8 * h + f) * Pq)] = m;
+                om[(unsigned)((8 * h + f) * Pq)] = id;
                 mx[f] = m;
             }
             if (po.copy[0]) {
-                const long long o = ((long long)n * Pq + wrem) * po.Cp + f0;
-                if (po.ns == 1) store_split8<1>(mx, po.enc, po.copy[0] + o, nullptr, nullptr);
-                else if (po.ns == 2) store_split8<2>(mx, po.enc, po.copy[0] + o, po.copy[1] + o, nullptr);
-                else store_split8<3>(mx, po.enc, po.copy[0] + o, po.copy[1] + o, po.copy[2] + o);
+                const long long o = c0 + 8 * h;
+                store_split8_n(mx, po.ns, po.enc, po.copy[0] + o, po.copy[1] + o, po.copy[2] + o);
             }
+        }
+    };
+
+    if (STAGED) {
+        const int total = NB * band.per_image;
+        auto stage = [&](int id, float *dst) {
+            const int n = band.by_bands.div(id), b = id - n * band.per_image, ih0 = 2 * b * band.window_rows - ph;
+            const float *xn = x + (long long)n * C * plane;
+            const uint32_t d0 = (uint32_t)__cvta_generic_to_shared(dst);
+            for (int e = threadIdx.x; e < bsize; e += blockDim.x) {
+                const int rr = band.by_pitch.div(e), j = e - rr * band.pitch, c = band.by_rows.div(rr), i = rr - c * band.rows;
+                const int ih = ih0 + i, iw = j - pw;
+                const bool in = (unsigned)ih < (unsigned)H && (unsigned)iw < (unsigned)W;
+                cp_async4(d0 + 4u * (uint32_t)e, in ? xn + c * plane + ih * W + iw : x, in);
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        int buf = 0;
+        if (band.buffers == 2 && (int)blockIdx.x < total) stage(blockIdx.x, bands);
+        for (int id = blockIdx.x; id < total; id += gridDim.x) {
+            if (band.buffers == 2) {
+                if (id + (int)gridDim.x < total) stage(id + gridDim.x, bands + (buf ^ 1) * bsize);
+                else asm volatile("cp.async.commit_group;" ::: "memory");
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
+            } else {
+                stage(id, bands);
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+            }
+            __syncthreads();
+            const float *src = bands + buf * bsize;
+            const int n = band.by_bands.div(id), b = id - n * band.per_image, q0 = b * band.window_rows;
+            const int windows = min(band.window_rows, OHq - q0) * OWq, items = ((windows + 31) >> 5) * groups;
+            for (int item = warp; item < items; item += 8) {
+                const int tile = by_groups.div(item), f0 = (item - tile * groups) * FW;
+                const int w = tile * 32 + lane, wl = min(w, windows - 1), qr = by_OWq.div(wl), qc = wl - qr * OWq;
+                const float *patch = src + 2 * qr * band.pitch + 2 * qc;
+                compute(n, (q0 + qr) * OWq + qc, f0, w < windows, [&](int c, f32x2 (*v)[4]) {
+#pragma unroll
+                    for (int i = 0; i < 4; i++) {
+                        const float2 u = *reinterpret_cast<const float2 *>(patch + c * bplane + i * band.pitch);
+                        const float2 t = *reinterpret_cast<const float2 *>(patch + c * bplane + i * band.pitch + 2);
+                        v[i][0] = pack2(u.x, u.x); v[i][1] = pack2(u.y, u.y); v[i][2] = pack2(t.x, t.x); v[i][3] = pack2(t.y, t.y);
+                    }
+                });
+            }
+            __syncthreads();                              // the band has been read: the copy after next may overwrite it
+            if (band.buffers == 2) buf ^= 1;
+        }
+    } else {
+        __syncthreads();
+        const int windows = NB * Pq, items = ((windows + 31) >> 5) * groups;
+        // neighbouring warps take the filter groups of one tile of windows, so that its input lines are found in L1
+        for (int item = blockIdx.x * 8 + warp; item < items; item += gridDim.x * 8) {
+            const int tile = by_groups.div(item), f0 = (item - tile * groups) * FW;
+            const int w = tile * 32 + lane, wi = min(w, windows - 1);
+            const int n = by_Pq.div(wi), wrem = wi - n * Pq, ohq = by_OWq.div(wrem), owq = wrem - ohq * OWq;
+            const int ih0 = 2 * ohq - ph, iw0 = 2 * owq - pw;
+            const float *xn = x + (long long)n * C * plane + ih0 * W + iw0;
+            compute(n, wrem, f0, w < windows, [&](int c, f32x2 (*v)[4]) {
+#pragma unroll
+                for (int i = 0; i < 4; i++)
+#pragma unroll
+                    for (int j = 0; j < 4; j++) {
+                        const bool in = (unsigned)(ih0 + i) < (unsigned)H && (unsigned)(iw0 + j) < (unsigned)W;
+                        const float e = in ? __ldg(xn + c * plane + i * W + j) : 0.f;
+                        v[i][j] = pack2(e, e);
+                    }
+            });
         }
     }
 }
@@ -365,12 +448,47 @@ bool conv_pool_simt_applies(int NB, int C, int H, int W, int F, int R, int S, in
 int conv_pool_simt(const float *X, const float *Wt, const float *bias, const PoolOut &pool, int NB, int C, int H, int W, int F, int ph, int pw,
                    int act, const char *name) {
     const int OH = H + 2 * ph - 2, OW = W + 2 * pw - 2, Pq = (OH / 2) * (OW / 2);
-    const long long tiles = ((long long)NB * Pq + 31) / 32;
-    const int grid = (int)(tiles < (long long)rt().sm_count * 8 ? tiles : (long long)rt().sm_count * 8);
+    const bool wide = (F & 15) == 0;
+    const int groups = F / (wide ? 16 : 8);
+    if (((long long)NB * Pq + 31) / 32 * groups > 0x7fffffff) return fail(SEERA_E_LIMIT, "%s: too many windows", name);
+    // Bands: as many window rows as fit 16 KB, at least one; two buffers while they leave room for two blocks on an SM, one up to
+    // 150 KB, and beyond that (a row of 4 x C x W values) no staging at all.
+    PoolBand band{};
+    band.pitch = (OW + 2 + 1) & ~1;
+    const size_t row = (size_t)C * band.pitch * sizeof(float), wbytes = (size_t)(C * 9 + 1) * F * sizeof(float);
+    int wr = (int)((16 * 1024 / row - 2) / 2);
+    if (16 * 1024 < 4 * row) wr = 1;
+    if (wr > OH / 2) wr = OH / 2;
+    // ... and shorter ones while a block would get fewer than eight of them (the last round of bands leaves blocks idle) and a band
+    // still holds work for its eight warps
+    while (wr > 1 && (long long)NB * ((OH / 2 + wr - 1) / wr) < 8ll * 2 * rt().sm_count && (wr / 2) * (OW / 2) * groups >= 8 * 32) wr /= 2;
+    band.window_rows = wr; band.rows = 2 * wr + 2; band.per_image = (OH / 2 + wr - 1) / wr;
+    const size_t bytes = band.rows * row;
+    band.buffers = bytes <= 32 * 1024 ? 2 : 1;
+    const bool staged = bytes <= 150 * 1024;
+    band.by_bands = fast_div(band.per_image); band.by_pitch = fast_div(band.pitch); band.by_rows = fast_div(band.rows);
+    const long long need = staged ? (long long)NB * band.per_image : (((long long)NB * Pq + 31) / 32 * groups + 7) / 8;
+    const long long cap = (long long)rt().sm_count * 2;       // two resident blocks per SM
+    const int grid = (int)(need < cap ? need : cap);
+    const size_t smem = wbytes + (staged ? band.buffers * bytes : 0);
     cudaStream_t st = rt().stream;
+    cudaError_t attr = cudaSuccess;
+    auto launch = [&](auto kern) {
+        if (smem > 48 * 1024) attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (attr == cudaSuccess)
+            kern<<<grid, 256, smem, st>>>(X, Wt, bias, pool, NB, C, H, W, F, OH, OW, ph, pw, act, fast_div(Pq), fast_div(OW / 2),
+                                          fast_div(groups), band);
+    };
     profile_begin();
-    conv3x3_pool_kernel<<<grid, 256, (size_t)(C * 9 + 1) * F * sizeof(float), st>>>(X, Wt, bias, pool, NB, C, H, W, F, OH, OW, ph, pw, act,
-                                                                               fast_div(Pq), fast_div(OW / 2));
+    const bool relu = act == SEERA_ACT_RELU;
+    if (staged) {
+        if (wide) { if (relu) launch(conv3x3_pool_kernel<16, true, true>); else launch(conv3x3_pool_kernel<16, false, true>); }
+        else { if (relu) launch(conv3x3_pool_kernel<8, true, true>); else launch(conv3x3_pool_kernel<8, false, true>); }
+    } else {
+        if (wide) { if (relu) launch(conv3x3_pool_kernel<16, true, false>); else launch(conv3x3_pool_kernel<16, false, false>); }
+        else { if (relu) launch(conv3x3_pool_kernel<8, true, false>); else launch(conv3x3_pool_kernel<8, false, false>); }
+    }
+    if (attr != cudaSuccess) return check_cuda(attr, name);
     count_launch();
     cudaError_t e = cudaGetLastError();
     profile_end(2.0 * NB * OH * OW * (double)F * C * 9, name);
