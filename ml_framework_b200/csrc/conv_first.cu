@@ -15,16 +15,12 @@
 // (engine_cuda/src/conv_fwd.cu, conv_bwd.cu: im2col + WMMA GEMM there).
 #include "common.cuh"
 #include "contraction_functors.cuh"
+#include "conv_first.cuh"
 #include "internal.h"
 #include "tc_epilogue.cuh"
 #include "tma_gemm_kernel.cuh"
 
 namespace seera {
-
-struct FirstGeom {
-    int NB, C, H, W, F, R, S, sh, sw, ph, pw, OH, OW, K;
-    FastDiv by_P, by_OW, by_Pq, by_OWq;      // pixels per image, output width, and the same counted in 2x2 windows
-};
 
 __device__ __forceinline__ float first_act(float z, int act) {
     switch (act) {
@@ -45,28 +41,6 @@ __device__ __forceinline__ void fill_patch_table(int *koff, int *krs, const Firs
         krs[k] = k < g.K ? ((r << 16) | s) : ((ones_col && k == g.K) ? -2 : -1);
     }
 }
-
-// Where the weight gradient takes the output gradient dz[img][f][pixel] from: a stored fp32 tensor, or computed on the
-// fly as dy * act'(y) with dy either a full-resolution gradient g or the gradient gp of a 2x2 / stride-2 max-pool of
-// y routed through the pool's window-local argmax indices.
-struct DzSource {
-    const float *dz;            // stored gradient, or null
-    const float *g, *gp;        // exactly one of these when dz is null
-    const int *mask;
-    const float *y;
-    int act;
-    const float *yp;            // with gp: the pool's output (y at each window's argmax), or null
-};
-__device__ __forceinline__ float first_slope(float y, int act) {
-    switch (act) {
-        case SEERA_ACT_RELU: return y > 0.f ? 1.f : 0.f;
-        case SEERA_ACT_SIGMOID: return y * (1.f - y);
-        case SEERA_ACT_TANH: return 1.f - y * y;
-        default: return 1.f;
-    }
-}
-
-constexpr int FIRST_FC = 64;        // filters per block pass
 
 // ---- forward ----------------------------------------------------------------------------------------------------
 template <int KP, int PIX>
@@ -914,7 +888,13 @@ int conv_first_fwd(const float *X, const float *Wt, const float *bias, float *Y,
     return e == cudaSuccess ? SEERA_OK : check_cuda(e, name);
 }
 
+void first_wgrad_reduce(const float *partial, float *dW, float *dbias, int F, int K, int KP, int nblocks, cudaStream_t st) {
+    conv_first_wgrad_reduce_kernel<<<(F + FIRST_FC - 1) / FIRST_FC * FIRST_FC * KP / 32, 256, 0, st>>>(partial, dW, dbias, F, K, KP, nblocks);
+    count_launch();
+}
+
 static int first_wgrad_run(const float *X, const DzSource &src, float *dW, float *dbias, const FirstGeom &g, const char *name) {
+    if (first_dw_applies(g, src)) return first_dw(X, src, dW, dbias, g, name);
     if (first_tc_wgrad_ok(g, dbias != nullptr)) return first_tc_wgrad(X, src, dW, dbias, g, name);
     long long pixels = (long long)g.NB * g.OH * g.OW;
     int ntiles = (int)((pixels + FIRST_TP - 1) / FIRST_TP);
@@ -972,7 +952,7 @@ int conv_first_act_wgrad(const float *X, const float *y, const float *g, const f
     FirstGeom geo;
     if (!first_geom(geo, NB, C, H, W, F, R, S, sh, sw, ph, pw)) return fail(SEERA_E_LIMIT, "%s: shape outside the short-patch kernel", name);
     if ((g == nullptr) == (gp == nullptr) || (gp && (!mask || (geo.OH & 1) || (geo.OW & 1))) ||
-        (act != SEERA_ACT_NONE && !y && !(gp && y_pooled && first_tc_wgrad_ok(geo, dbias != nullptr))))
+        (act != SEERA_ACT_NONE && !y && !(gp && y_pooled)))
         return fail(SEERA_E_ARG, "%s: bad argument", name);
     return first_wgrad_run(X, DzSource{nullptr, g, gp, mask, y, act, y_pooled}, dW, dbias, geo, name);
 }
