@@ -312,6 +312,13 @@ int seera_conv2d_bias_act_fwd(const float *image, const float *kernel, const flo
                               int F, int R, int S, int pad_h, int pad_w, int stride_h, int stride_w, int act);
 int seera_conv2DTranspose_bias_act_fwd(const float *X, const float *W, const float *bias, float *out, int batch, int Cin, int Hin,
                                        int Win, int Cout, int KH, int KW, int strideh, int stridew, int padh, int padw, int act);
+/* Nearest 2x2 unpooling and a 3x3 unit-stride transposed convolution with padding 1 onto one channel, as one operation on the
+ * low-resolution tensor x[N,Cin,H,W] (the unpooled tensor is never formed): y[N,1,2H,2W] = act(convT(unpool(x), w) + bias[0]), and its
+ * gradients from the gradient g of y (dx may be NULL). */
+int   seera_unpool2_convT_fusable(int N, int Cin, int H, int W, int Cout, int KH, int KW, int sh, int sw, int ph, int pw);
+int   seera_unpool2_convT_bias_act_fwd(const float *x, const float *w, const float *bias, float *y, int N, int Cin, int H, int W, int act);
+int   seera_unpool2_convT_act_bwd(const float *w, const float *x, const float *y, const float *g, float *dx, float *dw, float *db, int N,
+                                  int Cin, int H, int W, int act);
 /* Channels-last bf16 copies of one NCHW activation tensor, as the tensor-core convolutions read them.  A forward call
  * can hand the copies of its input to the matching backward call instead of producing them twice.  Opaque; owned
  * by the caller once returned; release with seera_shadow_free (stream-ordered, NULL allowed).

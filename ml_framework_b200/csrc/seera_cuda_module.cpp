@@ -232,6 +232,13 @@ PYBIND11_MODULE(seera_cuda, m) {
                                              int sh, int sw, int ph, int pw, int act) {
         ck(seera_conv2DTranspose_bias_act_fwd(P<const F>(x), P<const F>(w), P<const F>(b), P<F>(o), N, Ci, H, W, Co, KH, KW, sh, sw, ph,
                                               pw, act)); });
+    m.def("unpool2_convT_fusable", [](int N, int Ci, int H, int W, int Co, int KH, int KW, int sh, int sw, int ph, int pw) {
+        return seera_unpool2_convT_fusable(N, Ci, H, W, Co, KH, KW, sh, sw, ph, pw) != 0; });
+    m.def("unpool2_convT_bias_act_fwd", [](uptr x, uptr w, uptr b, uptr y, int N, int Ci, int H, int W, int act) {
+        ck(seera_unpool2_convT_bias_act_fwd(P<const F>(x), P<const F>(w), P<const F>(b), P<F>(y), N, Ci, H, W, act)); });
+    m.def("unpool2_convT_act_bwd", [](uptr w, uptr x, uptr y, uptr g, uptr dx, uptr dw, uptr db, int N, int Ci, int H, int W, int act) {
+        ck(seera_unpool2_convT_act_bwd(P<const F>(w), P<const F>(x), P<const F>(y), P<const F>(g), P<F>(dx), P<F>(dw), P<F>(db), N, Ci, H, W,
+                                       act)); });
     m.def("conv2d_bias_act_fwd_s", [](uptr x, uptr w, uptr b, uptr o, int N, int C, int H, int W, int Fo, int R, int S, int ph, int pw,
                                       int sh, int sw, int act, uptr x_in) {
         seera_shadow_t *keep = nullptr;

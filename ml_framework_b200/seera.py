@@ -180,6 +180,8 @@ tensor = Tensor
 # can do it; the convolution's own full-resolution output is then never materialised.  Set to False to keep every
 # layer's output in memory.
 FUSE_POOL = True
+# A 2x2 unpooling that feeds a ConvTranspose2D leaves its output unmade until somebody reads it (see _Unpooled).
+_LAZY_UNPOOL = hasattr(sc, "unpool2_convT_fusable")
 # A Dense layer that feeds another Dense layer can have its GEMM epilogue write the 16-bit copies of its output that the next
 # layer's GEMM reads (seera_matmul_bias_act_fwd_s, c_copies).  Off: at the sizes measured (4096 x 1024 outputs, one tile per
 # CTA) the two-byte stores lengthen an epilogue that nothing overlaps by more than the next layer's vectorised conversion
@@ -202,6 +204,30 @@ class _PooledGrad:
         dx = _new(self.shape)
         sc.cuda_maxpool_bwd(self.gp.main_ptr, self.mask.main_ptr, dx.main_ptr, N, C, H, W, 2, 2, 0, 0, 2, 2)
         return dx
+
+
+class _Unpooled(cuten):
+    """The 2x2 nearest unpooling of `low` as a tensor whose memory is made when its address is asked for.  The transposed convolution that
+    reads it can work from `low` directly, and then it never is."""
+    low = None
+
+    @classmethod
+    def of(cls, low):
+        N, C, H, W = low.shape
+        t = cls._wrap(None, (N, C, 2 * H, 2 * W))
+        t.low = low
+        return t
+
+    @property
+    def main_ptr(self):
+        if self._ptr is None:
+            self._ptr = _malloc(self.size)
+            sc.cuda_unpooling_fwd(self.low.main_ptr, self._ptr, *self.low.shape, 2, 2)
+        return self._ptr
+
+    @main_ptr.setter
+    def main_ptr(self, value):
+        self._ptr = value
 
 
 class _KeptCopies:
@@ -284,7 +310,7 @@ class autograd4nn:
 class Layer:
     # which layers read this one's output (set while a model is put together): a producer can then hand on more than its values
     _pool_consumer = None
-    _feeds_conv = _feeds_dense = False
+    _feeds_conv = _feeds_dense = _feeds_convT = False
     _fused = None                    # a pool that the layer folded into its own launch: (pooled, mask, copies)
     _model = None
 
@@ -547,6 +573,11 @@ class ConvTranspose2D(_ParamLayer):
         self.weights = Tensor(self._w_init, is_leaf=True)
         self.bais = Tensor(self._b_init, is_leaf=True)
 
+    def __call__(self, input_layer):
+        super().__call__(input_layer)
+        input_layer._feeds_convT = True       # an unpooling producer then leaves its output to be read at the low resolution
+        return self
+
     def forward(self):
         x = self.inputs = self.inpobj.outputs
         W, b = self.weights, self.bais
@@ -561,6 +592,9 @@ class ConvTranspose2D(_ParamLayer):
         Ho, Wo = (H - 1) * sh - 2 * ph + KH, (Wd - 1) * sw - 2 * pw + KW
         code = _ACT[self.layeract]
         z = _new((N, Cout, Ho, Wo))
+        if (xv.__class__ is _Unpooled and xv._ptr is None and H % 2 == 0 and Wd % 2 == 0
+                and sc.unpool2_convT_fusable(N, Cin, H // 2, Wd // 2, Cout, KH, KW, sh, sw, ph, pw)):
+            return self._forward_unpooled(x, xv.low, z, code)
         sc.conv2DTranspose_bias_act_fwd(xv.main_ptr, wv.main_ptr, b.value.main_ptr, z._ptr, N, Cin, H, Wd, Cout, KH, KW, sh, sw, ph, pw, code)
         need_dx = not x.is_leaf
 
@@ -576,6 +610,23 @@ class ConvTranspose2D(_ParamLayer):
             sc.cuda_conv2DTranspose_bwd(wv._ptr, xv._ptr, dz.main_ptr, dx._ptr if need_dx else 0, dw._ptr, N, Cin, H, Wd, Cout, KH, KW,
                                        sh, sw, ph, pw)
             self._deliver(x, W, b, dx, dw, db)
+        self.outputs = self._output(x, z, backward)
+        return self.outputs
+
+    def _forward_unpooled(self, x, low, z, code):
+        """The unpooling before this layer and the layer in one, from the low-resolution tensor and with its gradient as result."""
+        W, b = self.weights, self.bais
+        N, Cin, H, Wd = low.shape
+        sc.unpool2_convT_bias_act_fwd(low.main_ptr, W.value.main_ptr, b.value.main_ptr, z._ptr, N, Cin, H, Wd, code)
+        source = x._parents[0]                    # what was unpooled: its gradient goes to it directly
+        need_dx = not source.is_leaf
+
+        def backward(g):
+            db, dw = b._grad_target(), W._grad_target()
+            dlow = _new(low.shape) if need_dx else None
+            sc.unpool2_convT_act_bwd(W.value._ptr, low._ptr, z._ptr if code else 0, g.main_ptr, dlow._ptr if need_dx else 0, dw._ptr, db._ptr,
+                                     N, Cin, H, Wd, code)
+            self._deliver(source, W, b, dlow, dw, db)
         self.outputs = self._output(x, z, backward)
         return self.outputs
 
@@ -782,12 +833,15 @@ class Unpool2D_Nearest(Layer):
         if len(xv.shape) != 4:
             raise ValueError("[cuTen]:unpool expects 4-D tensor (N,C,H,W)")
         sw, sh = self.size                       # the reference unpacks (sw, sh) (Seera_init.py:793)
-        N, C, H, W = xv.shape
-        y = _new((N, C, H * sh, W * sw))
-        sc.cuda_unpooling_fwd(xv.main_ptr, y._ptr, N, C, H, W, sh, sw)
+        N, C, H, W = shape = xv.shape
+        if self._feeds_convT and (sw, sh) == (2, 2) and _LAZY_UNPOOL:
+            y = _Unpooled.of(xv)
+        else:
+            y = _new((N, C, H * sh, W * sw))
+            sc.cuda_unpooling_fwd(xv.main_ptr, y._ptr, N, C, H, W, sh, sw)
 
         def backward(g):
-            dx = _new(xv.shape)
+            dx = _new(shape)
             sc.cuda_unpooling_bwd(g.main_ptr, dx._ptr, N, C, H, W, sh, sw)
             x._accumulate(dx)
         self.outputs = out = Tensor._of(y, (x,), backward)
