@@ -26,6 +26,10 @@ struct Runtime {
     int mma_issuers = 0;                // cap on the MMA-issuing threads of the TMA-fed GEMM kernel (0: none; 1 or 2)
     bool pair_tiles = false;            // TMA-fed GEMMs as clusters of two CTAs on 256-row tiles where the plan finds it pays
     bool conv_tma = true;               // convolutions in modes 1-3: TMA im2col kernel (false: in-kernel gather kernel)
+    // the loss gradient whose largest entry the loss head has already turned into the dynamic factor (grad_scale_update then has
+    // nothing left to do for it)
+    const float *scaled_grad = nullptr;
+    long long scaled_n = 0;
     bool capturing = false;             // a stream capture (seera_graph_begin) is open
     bool tc_used = false;               // a tensor-core kernel ran since the status word was last read
     int status = 0;
@@ -49,29 +53,34 @@ inline int stride_grid(long long work_items, int threads = 256) {
 inline void count_launch(int n = 1) { rt().launches += n; }
 
 // out[c] = sum over s < splits of partial[s * n + c], added in a fixed order (the same bits on every run).  A block owns 32
-// consecutive columns; its eight warps take the splits w, w + 8, ... (128-byte coalesced reads, splits / 8 dependent loads
-// instead of `splits`), then the eight sums are added in warp order.  Columns at or beyond n_first go to out2 (may be null).
-static __global__ void __launch_bounds__(256) sum_splits_kernel(const float *__restrict__ partial, float *__restrict__ out,
-                                                                float *__restrict__ out2, int n_first, int n, int splits) {
-    __shared__ float sm[8][33];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = blockIdx.x * 32 + lane;
+// consecutive columns; its warps take the splits w, w + warps, ... (128-byte coalesced reads), then their sums are added in warp
+// order.  Columns at or beyond n_first go to out2 (may be null).  What such a launch waits for is the chain of reads of one warp: up to
+// 32 warps keep it at a few reads however many splits there are (288 columns of 296 splits: 8 us with 8 warps).
+static __global__ void __launch_bounds__(1024) sum_splits_kernel(const float *__restrict__ partial, float *__restrict__ out,
+                                                                 float *__restrict__ out2, int n_first, int n, int splits) {
+    __shared__ float sm[32][33];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5, c = blockIdx.x * 32 + lane;
     float t = 0.f;
-    if (c < n) {
-#pragma unroll 4
-        for (int s = warp; s < splits; s += 8) t += __ldg(partial + (long long)s * n + c);
-    }
+    if (c < n)
+        for (int s = warp; s < splits; s += 8 * warps) {
+            float v[8];                                       // all of them requested before the first is added
+#pragma unroll
+            for (int k = 0; k < 8; k++) v[k] = s + k * warps < splits ? __ldg(partial + (long long)(s + k * warps) * n + c) : 0.f;
+#pragma unroll
+            for (int k = 0; k < 8; k++) t += v[k];
+        }
     sm[warp][lane] = t;
     __syncthreads();
     if (warp == 0 && c < n) {
         float r = sm[0][lane];
-#pragma unroll
-        for (int w = 1; w < 8; w++) r += sm[w][lane];
+        for (int w = 1; w < warps; w++) r += sm[w][lane];
         if (c < n_first) out[c] = r;
         else if (out2) out2[c - n_first] = r;
     }
 }
 inline void launch_sum_splits(const float *partial, float *out, int n, int splits, cudaStream_t st, float *out2 = nullptr, int n_first = -1) {
-    sum_splits_kernel<<<(n + 31) / 32, 256, 0, st>>>(partial, out, out2, n_first < 0 ? n : n_first, n, splits);
+    const int threads = splits <= 64 ? 256 : (splits <= 128 ? 512 : 1024);
+    sum_splits_kernel<<<(n + 31) / 32, threads, 0, st>>>(partial, out, out2, n_first < 0 ? n : n_first, n, splits);
     count_launch();
 }
 

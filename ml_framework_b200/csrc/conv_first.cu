@@ -261,29 +261,31 @@ __global__ void __launch_bounds__(256) conv_first_wgrad_kernel(const float *__re
 
 // dW[f][k] = sum over blocks of partial[chunk][block][f - f0][k].  A block of 8 warps owns 32 outputs (one per lane);
 // warp w adds blocks w, w + 8, ... in order and the eight sums meet in shared memory in warp order: a fixed order.
-__global__ void __launch_bounds__(256) conv_first_wgrad_reduce_kernel(const float *__restrict__ partial, float *__restrict__ dW,
-                                                                      float *__restrict__ dbias, int F, int K, int KP, int nblocks) {
-    __shared__ float part[8][32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+__global__ void __launch_bounds__(1024) conv_first_wgrad_reduce_kernel(const float *__restrict__ partial, float *__restrict__ dW,
+                                                                       float *__restrict__ dbias, int F, int K, int KP, int nblocks) {
+    __shared__ float part[32][33];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const int e = blockIdx.x * 32 + lane;                  // index into the padded [F rounded to 64][KP] grid
     const int f = e / KP, k = e - f * KP;
     const int chunk = f / FIRST_FC, fl = f - chunk * FIRST_FC;
+    const bool wanted = f < F && (k < K || (dbias && k == K));
     const float *p = partial + (long long)chunk * nblocks * (FIRST_FC * KP) + fl * KP + k;
-    float s0 = 0.f, s1 = 0.f;
-    int b = warp;
-    for (; b + 8 < nblocks; b += 16) {
-        s0 += p[(long long)b * (FIRST_FC * KP)];
-        s1 += p[(long long)(b + 8) * (FIRST_FC * KP)];
-    }
-    if (b < nblocks) s0 += p[(long long)b * (FIRST_FC * KP)];
-    part[warp][lane] = s0 + s1;
-    __syncthreads();
-    if (warp == 0 && f < F && (k < K || (dbias && k == K))) {
-        float s = 0.f;
+    float s = 0.f;
+    if (wanted)
+        for (int b = warp; b < nblocks; b += 8 * warps) {
+            float v[8];                                       // all of them requested before the first is added
 #pragma unroll
-        for (int w = 0; w < 8; w++) s += part[w][lane];
-        if (k < K) dW[(long long)f * K + k] = s;
-        else dbias[f] = s;                       // the column of ones: sum of the output gradient per filter
+            for (int j = 0; j < 8; j++) v[j] = b + j * warps < nblocks ? __ldg(p + (long long)(b + j * warps) * (FIRST_FC * KP)) : 0.f;
+#pragma unroll
+            for (int j = 0; j < 8; j++) s += v[j];
+        }
+    part[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0 && wanted) {
+        float t = part[0][lane];
+        for (int w = 1; w < warps; w++) t += part[w][lane];
+        if (k < K) dW[(long long)f * K + k] = t;
+        else dbias[f] = t;                       // the column of ones: sum of the output gradient per filter
     }
 }
 
@@ -748,6 +750,12 @@ first_tc_wgrad_kernel(const float *__restrict__ X, DzSource src, float *__restri
     if (warp == MMA_WARP) tmem_dealloc(tmem_base, 64);
 }
 
+void first_wgrad_reduce(const float *partial, float *dW, float *dbias, int F, int K, int KP, int nblocks, cudaStream_t st) {
+    conv_first_wgrad_reduce_kernel<<<(F + FIRST_FC - 1) / FIRST_FC * FIRST_FC * KP / 32, nblocks <= 64 ? 256 : (nblocks <= 128 ? 512 : 1024), 0, st>>>(
+        partial, dW, dbias, F, K, KP, nblocks);
+    count_launch();
+}
+
 // Dynamic shared memory limit raised once per kernel instantiation and device.
 template <class K>
 static cudaError_t raise_smem_limit(K kernel, int *done_flags) {
@@ -819,8 +827,7 @@ static int first_tc_wgrad(const float *X, const DzSource &src, float *dW, float 
     count_launch();
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e == cudaSuccess) {
-        conv_first_wgrad_reduce_kernel<<<boxes * 64 * 64 / 32, 256, 0, st>>>(partial, dW, dbias, g.F, g.K, 64, nblocks);
-        count_launch();
+        first_wgrad_reduce(partial, dW, dbias, g.F, g.K, 64, nblocks, st);
         e = cudaGetLastError();
     }
     profile_end(2.0 * pixels * (double)g.F * g.K, name);
@@ -888,11 +895,6 @@ int conv_first_fwd(const float *X, const float *Wt, const float *bias, float *Y,
     return e == cudaSuccess ? SEERA_OK : check_cuda(e, name);
 }
 
-void first_wgrad_reduce(const float *partial, float *dW, float *dbias, int F, int K, int KP, int nblocks, cudaStream_t st) {
-    conv_first_wgrad_reduce_kernel<<<(F + FIRST_FC - 1) / FIRST_FC * FIRST_FC * KP / 32, 256, 0, st>>>(partial, dW, dbias, F, K, KP, nblocks);
-    count_launch();
-}
-
 static int first_wgrad_run(const float *X, const DzSource &src, float *dW, float *dbias, const FirstGeom &g, const char *name) {
     if (first_dw_applies(g, src)) return first_dw(X, src, dW, dbias, g, name);
     if (first_tc_wgrad_ok(g, dbias != nullptr)) return first_tc_wgrad(X, src, dW, dbias, g, name);
@@ -920,8 +922,7 @@ static int first_wgrad_run(const float *X, const DzSource &src, float *dW, float
     count_launch();
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) {
-        conv_first_wgrad_reduce_kernel<<<chunks * FIRST_FC * KP / 32, 256, 0, st>>>(partial, dW, dbias, g.F, g.K, KP, nblocks);
-        count_launch();
+        first_wgrad_reduce(partial, dW, dbias, g.F, g.K, KP, nblocks, st);
         e = cudaGetLastError();
     }
     profile_end(2.0 * pixels * (double)g.F * g.K, name);

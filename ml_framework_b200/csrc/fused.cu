@@ -188,9 +188,71 @@ __global__ void __launch_bounds__(256) softmax_vjp_kernel(const float *__restric
 }
 
 // softmax -> clip -> log -> -y* -> sum(-1), and the gradient of inv_count * sum_rows w.r.t. z
+// factor = 2^(-4 - e) with amax = m * 2^e, m in [0.5, 1): together with the static 2^12 of the gradient class the largest
+// entry of the loss gradient lands in [128, 256) - eight binades of headroom below fp16's maximum for gradients that grow
+// on the way down the network, twenty-one binades of normal range below it for those that shrink.
+__device__ __forceinline__ void grad_scale_finalize(float *w) {
+    const float amax = __uint_as_float(atomicExch(reinterpret_cast<unsigned *>(w) + 2, 0u));
+    int e = 0;
+    if (amax > 0.f) frexpf(amax, &e);
+    e = max(-100, min(30, e));
+    w[0] = amax > 0.f ? ldexpf(1.f, -4 - e) : 1.f;
+    w[1] = amax > 0.f ? ldexpf(1.f, 4 + e) : 1.f;
+}
+// infinities and NaNs do not steer the scale
+__device__ __forceinline__ float scale_entry(float g) { const float a = fabsf(g); return a < 3.0e38f ? a : 0.f; }
+
+// True in the block that finishes last; everything the others wrote before is then visible to it.  The counter (one of a
+// few that the launches use in turn) is back at zero afterwards.
+__device__ unsigned int g_finish_counters[64];
+__device__ __forceinline__ bool last_block_done(int counter) {
+    __shared__ int last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicInc(&g_finish_counters[counter], gridDim.x - 1) == gridDim.x - 1;
+    __syncthreads();
+    if (last) __threadfence();
+    return last != 0;
+}
+// The last block of a loss launch: the mean from what the blocks left in v[0..n), in a fixed order, and (scale != null) the dynamic
+// factor of the fp16 gradient copies from the largest entry.
+__device__ __forceinline__ void finish_loss(const float *v, int n, float factor, float *out, float *scale, float *sm) {
+    float acc = 0.f;
+    for (int i = threadIdx.x; i < n; i += 16 * blockDim.x) {
+        float q[16];                                   // all of them requested before the first is added
+#pragma unroll
+        for (int k = 0; k < 16; k++) q[k] = i + k * (int)blockDim.x < n ? __ldcg(v + i + k * blockDim.x) : 0.f;
+#pragma unroll
+        for (int k = 0; k < 16; k++) acc += q[k];
+    }
+    const float t = block_sum_256(acc, sm);
+    if (threadIdx.x == 0) {
+        *out = t * factor;
+        if (scale) grad_scale_finalize(scale);
+    }
+}
+__device__ __forceinline__ void note_largest(float m, float *scale) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0 && m > 0.f) atomicMax(reinterpret_cast<unsigned *>(scale) + 2, __float_as_uint(m));
+}
+inline int next_finish_counter() { static int k = 0; k = (k + 1) & 63; return k; }
+// Where a loss launch in the present precision mode leaves the factor (null: the copies of this mode have none), and the note that
+// it has done so for gradient `dz`.
+inline float *loss_scale(const float *dz, long long n) {
+    if (rt().precision != 4 && rt().precision != 5) return nullptr;
+    float *w = grad_scale_words();
+    rt().scaled_grad = w ? dz : nullptr;
+    rt().scaled_n = n;
+    return w;
+}
+
 __global__ void __launch_bounds__(256) softmax_cce_kernel(const float *__restrict__ z, const float *__restrict__ yhot,
                                                           float *__restrict__ p, float *__restrict__ loss_rows,
-                                                          float *__restrict__ dz, int N, int C, float eps, float inv_count) {
+                                                          float *__restrict__ dz, int N, int C, float eps, float inv_count,
+                                                          float *__restrict__ loss_mean, float *__restrict__ scale, int counter) {
+    __shared__ float sm[8];
+    float largest = 0.f;
     int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     int nwarp = gridDim.x * (blockDim.x >> 5);
     float hi = 1.0f - eps;
@@ -216,48 +278,64 @@ __global__ void __launch_bounds__(256) softmax_cce_kernel(const float *__restric
         }
         loss = warp_sum(loss);
         dot = warp_sum(dot);
-        for (int c = lane; c < C; c += 32) dr[c] = pr[c] * (dr[c] - dot);
+        for (int c = lane; c < C; c += 32) {
+            const float d = pr[c] * (dr[c] - dot);
+            dr[c] = d;
+            largest = fmaxf(largest, scale_entry(d));
+        }
         if (lane == 0) loss_rows[row] = loss;
     }
+    if (scale) note_largest(largest, scale);
+    if (last_block_done(counter)) finish_loss(loss_rows, N, inv_count, loss_mean, scale, sm);
 }
 
 // Deterministic single-block sum of n floats times scale.
-__global__ void __launch_bounds__(1024) scaled_sum_kernel(const float *__restrict__ v, float *__restrict__ out, int n, float scale) {
-    __shared__ float sm[32];
-    float acc = 0.f;
-#pragma unroll 4
-    for (int i = threadIdx.x; i < n; i += blockDim.x) acc += v[i];
-    float t = block_sum_256(acc, sm);
-    if (threadIdx.x == 0) *out = t * scale;
-}
-
 // Element-wise losses with their gradient in the same pass.  KIND 0: (p-y)^2 (Seera.py:943-945); 1: |p-y| with the sign
 // convention of abs_fwd, 0 at 0 (Seera.py:947-949, engine/src/activation_ops.cpp:50-56); 2: binary cross-entropy
 // -y log(p+eps) - (1-y) log(1-p+eps) (Seera.py:951-953).  dp = dloss/dp * inv_count; per-block sums go to `partials`.
 template <int KIND>
 __global__ void __launch_bounds__(256) elem_loss_kernel(const float *__restrict__ p, const float *__restrict__ y,
                                                         float *__restrict__ partials, float *__restrict__ dp,
-                                                        long long n, float inv_count, float eps) {
+                                                        long long n, float inv_count, float eps, float *__restrict__ loss_mean,
+                                                        float *__restrict__ scale, int counter, bool vec) {
     __shared__ float sm[8];
+    float largest = 0.f;
     long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x, nthr = (long long)gridDim.x * blockDim.x;
     float acc = 0.f;
-    for (long long i = tid; i < n; i += nthr) {
+    auto one = [&](float pv, float yv) {
+        float g;
         if (KIND == 0) {
-            float d = p[i] + y[i] * -1.0f;
+            const float d = pv + yv * -1.0f;
             acc += d * d;
-            dp[i] = (2.0f * d) * inv_count;
+            g = (2.0f * d) * inv_count;
         } else if (KIND == 1) {
-            float d = p[i] + y[i] * -1.0f;
+            const float d = pv + yv * -1.0f;
             acc += fabsf(d);
-            dp[i] = (d > 0.f ? 1.f : (d < 0.f ? -1.f : 0.f)) * inv_count;
+            g = (d > 0.f ? 1.f : (d < 0.f ? -1.f : 0.f)) * inv_count;
         } else {
-            const float pv = p[i], yv = y[i], a = pv + eps, b = (1.f - pv) + eps;
+            const float a = pv + eps, b = (1.f - pv) + eps;
             acc += -yv * logf(a) - (1.f - yv) * logf(b);
-            dp[i] = (-yv / a + (1.f - yv) / b) * inv_count;
+            g = (-yv / a + (1.f - yv) / b) * inv_count;
         }
+        largest = fmaxf(largest, scale_entry(g));
+        return g;
+    };
+    long long done = 0;
+    if (vec) {
+        const long long n4 = n >> 2;
+        for (long long i = tid; i < n4; i += nthr) {
+            const float4 a = __ldg(reinterpret_cast<const float4 *>(p) + i), b = __ldg(reinterpret_cast<const float4 *>(y) + i);
+            float4 g;
+            g.x = one(a.x, b.x); g.y = one(a.y, b.y); g.z = one(a.z, b.z); g.w = one(a.w, b.w);
+            reinterpret_cast<float4 *>(dp)[i] = g;
+        }
+        done = n4 << 2;
     }
+    for (long long i = done + tid; i < n; i += nthr) dp[i] = one(p[i], y[i]);
     float t = block_sum_256(acc, sm);
     if (threadIdx.x == 0) partials[blockIdx.x] = t;
+    if (scale) note_largest(largest, scale);
+    if (last_block_done(counter)) finish_loss(partials, gridDim.x, inv_count, loss_mean, scale, sm);
 }
 
 // ---- optimizers -------------------------------------------------------------------------------------------
@@ -357,19 +435,8 @@ __global__ void __launch_bounds__(256) grad_amax_kernel(const float *__restrict_
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     if ((threadIdx.x & 31) == 0 && m > 0.f) atomicMax(amax_bits, __float_as_uint(m));
 }
-// factor = 2^(-4 - e) with amax = m * 2^e, m in [0.5, 1): together with the static 2^12 of the gradient class the largest
-// entry of the loss gradient lands in [128, 256) - eight binades of headroom below fp16's maximum for gradients that grow
-// on the way down the network, twenty-one binades of normal range below it for those that shrink.
 __global__ void grad_scale_finalize_kernel(float *w) {
-    if (threadIdx.x != 0) return;
-    unsigned *bits = reinterpret_cast<unsigned *>(w) + 2;
-    const float amax = __uint_as_float(*bits);
-    *bits = 0u;
-    int e = 0;
-    if (amax > 0.f) frexpf(amax, &e);
-    e = max(-100, min(30, e));
-    w[0] = amax > 0.f ? ldexpf(1.f, -4 - e) : 1.f;
-    w[1] = amax > 0.f ? ldexpf(1.f, 4 + e) : 1.f;
+    if (threadIdx.x == 0) grad_scale_finalize(w);
 }
 
 float *grad_scale_words() {
@@ -536,10 +603,11 @@ int seera_softmax_cce_fwd_bwd(const float *z, const float *onehot, float *p, flo
     if (N < 1 || C < 1 || !z || !onehot || !p || !loss_rows || !loss_mean || !dz)
         return fail(SEERA_E_ARG, "softmax_cce_fwd_bwd: bad argument");
     ProfBytes pb(16.0 * N * C, "softmax_cce");
-    softmax_cce_kernel<<<stride_grid((long long)N * 32), 256, 0, rt().stream>>>(z, onehot, p, loss_rows, dz, N, C, eps, inv_count);
+    // at most two blocks per SM: every block pays for its turn at the finish counter
+    const int grid = (int)((N + 7) / 8 < 2 * rt().sm_count ? (N + 7) / 8 : 2 * rt().sm_count);
+    softmax_cce_kernel<<<grid, 256, 0, rt().stream>>>(z, onehot, p, loss_rows, dz, N, C, eps, inv_count, loss_mean,
+                                                                                loss_scale(dz, (long long)N * C), next_finish_counter());
     SEERA_LAUNCH_CHECK("softmax_cce");
-    scaled_sum_kernel<<<1, N > 1024 ? 1024 : 256, 0, rt().stream>>>(loss_rows, loss_mean, N, inv_count);
-    SEERA_LAUNCH_CHECK("softmax_cce(sum)");
     return SEERA_OK;
 }
 
@@ -552,14 +620,16 @@ static int elem_loss(int kind, const float *p, const float *y, float *partials, 
                      float inv_count, float eps, const char *name) {
     SEERA_ENSURE();
     if (size < 1 || !p || !y || !partials || !loss_mean || !dp) return fail(SEERA_E_ARG, "%s: bad argument", name);
-    int g = stride_grid(size);
+    const bool vec = aligned16(p) && aligned16(y) && aligned16(dp);
+    int g = stride_grid(vec ? (size + 3) / 4 : size);
+    if (g > 2 * rt().sm_count) g = 2 * rt().sm_count;        // every block pays for its turn at the finish counter
     cudaStream_t st = rt().stream;
+    float *scale = loss_scale(dp, size);
+    const int counter = next_finish_counter();
     ProfBytes pb(12.0 * size, name);
-    if (kind == 0) elem_loss_kernel<0><<<g, 256, 0, st>>>(p, y, partials, dp, size, inv_count, eps);
-    else if (kind == 1) elem_loss_kernel<1><<<g, 256, 0, st>>>(p, y, partials, dp, size, inv_count, eps);
-    else elem_loss_kernel<2><<<g, 256, 0, st>>>(p, y, partials, dp, size, inv_count, eps);
-    SEERA_LAUNCH_CHECK(name);
-    scaled_sum_kernel<<<1, g > 1024 ? 1024 : 256, 0, st>>>(partials, loss_mean, g, inv_count);
+    if (kind == 0) elem_loss_kernel<0><<<g, 256, 0, st>>>(p, y, partials, dp, size, inv_count, eps, loss_mean, scale, counter, vec);
+    else if (kind == 1) elem_loss_kernel<1><<<g, 256, 0, st>>>(p, y, partials, dp, size, inv_count, eps, loss_mean, scale, counter, vec);
+    else elem_loss_kernel<2><<<g, 256, 0, st>>>(p, y, partials, dp, size, inv_count, eps, loss_mean, scale, counter, vec);
     SEERA_LAUNCH_CHECK(name);
     return SEERA_OK;
 }
@@ -583,6 +653,8 @@ int seera_grad_scale_update(const float *g, long long n) {
     float *w = grad_scale_words();
     if (!w) return fail(SEERA_E_OOM, "grad_scale_update: no device memory for the scale words");
     if (n == 0) return SEERA_OK;
+    if (g == rt().scaled_grad && n == rt().scaled_n) { rt().scaled_grad = nullptr; return SEERA_OK; }     // the loss head has done it
+    rt().scaled_grad = nullptr;                   // the factor is about to be another gradient's
     grad_amax_kernel<<<stride_grid(n), 256, 0, rt().stream>>>(g, n, reinterpret_cast<unsigned *>(w) + 2);
     SEERA_LAUNCH_CHECK("grad_scale_update(amax)");
     grad_scale_finalize_kernel<<<1, 32, 0, rt().stream>>>(w);

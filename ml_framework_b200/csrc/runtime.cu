@@ -420,6 +420,7 @@ int seera_cuda_free(void *ptr) {
     Pool &p = pool();
     auto it = p.live.find(ptr);
     if (it == p.live.end()) return fail(SEERA_E_ARG, "cuda_free(%p): not a live block of this pool", ptr);
+    if (ptr == rt().scaled_grad) rt().scaled_grad = nullptr;
     auto ow = p.owner.find(ptr);
     if (ow != p.owner.end()) {
         // a block a captured graph writes on every replay: reusable inside that capture, otherwise kept aside
@@ -450,6 +451,7 @@ int seera_graph_begin(void) {
     if (p.capturing) return fail(SEERA_E_ARG, "graph_begin: a capture is already open");
     if (int s = batch_flush()) return s;
     if (int s = check_cuda(cudaStreamBeginCapture(rt().stream, cudaStreamCaptureModeRelaxed), "cudaStreamBeginCapture")) return s;
+    rt().scaled_grad = nullptr;
     p.cur = new GraphRec();
     p.cur->launches_at_begin = rt().launches;
     p.cap_free.clear();
@@ -463,6 +465,7 @@ void *seera_graph_end(void) {
     if (!p.capturing) { fail(SEERA_E_ARG, "graph_end: no capture is open"); return nullptr; }
     p.capturing = false;
     rt().capturing = false;
+    rt().scaled_grad = nullptr;
     p.cap_free.clear();
     GraphRec *g = p.cur;
     p.cur = nullptr;
