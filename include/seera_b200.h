@@ -366,6 +366,26 @@ int seera_conv2d_bias_act_pool_fwd_s(const float *image, const float *kernel, co
 int seera_conv2d_act_bwd(const float *W, const float *X, const float *y, const float *g, const float *gp, const int *pool_mask,
                          const float *y_pooled, float *dX, float *dW, float *dbias, int batch, int C, int H, int W_in, int F, int R, int S,
                          int strideh, int stridew, int padh, int padw, int act, seera_shadow_t *x_shadow);
+/* The same with more handed from call to call, for a host that keeps it (every handle may be NULL):
+ *   *w_keep    receives the 16-bit copies of the filters a unit-stride forward made; given back as w_keep they serve the data gradient
+ *   *y_copies  receives channels-last copies of the OUTPUT for the convolution that reads it (its x_in), written by the same launch
+ * and for transposed convolutions x_in / x_keep as above, and a backward from the gradient g of the activated output y that applies
+ * the slope and sums the bias gradient while it makes the products' operands. */
+int seera_conv2d_bias_act_fwd_k(const float *image, const float *kernel, const float *bias, float *out, int batchN, int C, int H, int W, int F,
+                                int R, int S, int pad_h, int pad_w, int stride_h, int stride_w, int act, seera_shadow_t *x_in,
+                                seera_shadow_t **x_keep, seera_rows_t **w_keep, seera_shadow_t **y_copies);
+int seera_conv2d_bias_act_pool_fwd_k(const float *image, const float *kernel, const float *bias, float *pooled, int *mask, int batchN, int C,
+                                     int H, int W, int F, int R, int S, int pad_h, int pad_w, int stride_h, int stride_w, int act,
+                                     seera_shadow_t *x_in, seera_shadow_t **x_keep, seera_rows_t **w_keep, seera_shadow_t **pooled_copies);
+int seera_conv2d_act_bwd_k(const float *kernel, const float *image, const float *y, const float *g, const float *gp, const int *pool_mask,
+                           const float *y_pooled, float *dX, float *dW, float *dbias, int batchN, int C, int H, int W, int F, int R, int S,
+                           int stride_h, int stride_w, int pad_h, int pad_w, int act, seera_shadow_t *x_shadow, seera_rows_t *w_keep);
+int seera_conv2DTranspose_bias_act_fwd_k(const float *X, const float *W, const float *bias, float *out, int batch, int Cin, int Hin, int Win,
+                                         int Cout, int KH, int KW, int sh, int sw, int ph, int pw, int act, seera_shadow_t *x_in,
+                                         seera_shadow_t **x_keep);
+int seera_conv2DTranspose_act_bwd_k(const float *W, const float *X, const float *y, const float *g, float *dX, float *dW, float *dbias,
+                                    int batch, int Cin, int Hin, int Win, int Cout, int KH, int KW, int sh, int sw, int ph, int pw, int act,
+                                    seera_shadow_t *x_shadow);
 /* dz = dy * act'(y), with the derivative written in terms of the OUTPUT y (relu: y > 0; sigmoid:
  * y(1-y); tanh: 1-y^2), and dbias[c] = sum of dz over that channel.  Replaces cuda_elemmult with the
  * stored local gradient plus broadcast_mul_4d + three cuda_sum_fwd (Seera_Engine.py:571-583, :43-65). */

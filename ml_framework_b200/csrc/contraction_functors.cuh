@@ -7,6 +7,7 @@
 // convolution input, the col2im gather of a data gradient and the per-tap view of a weight gradient.
 #pragma once
 #include "common.cuh"
+#include "tc_ptx.cuh"
 
 namespace seera {
 
@@ -137,12 +138,30 @@ struct StoreDenseT {       // C[n*ld + m]
 struct StorePixelRows {    // m = (img, p): out[(img*Nch + n)*P + p]
     static constexpr bool kMContiguous = true;
     float *out; int Nch, P;
+    // optional channels-last 16-bit copies of the same values, for the layer that reads them (pitch Cp, a multiple of 8)
+    __nv_bfloat16 *cp[3] = {nullptr, nullptr, nullptr};
+    int Cp = 0, ns = 0;
+    Enc enc{0, 1.f, nullptr};
     __device__ void operator()(int m, int n, float v) const {
         int img = m / P, p = m - img * P;
         out[((long long)img * Nch + n) * P + p] = v;
     }
     __device__ float *row(int m) const { int img = m / P, p = m - img * P; return out + (long long)img * Nch * P + p; }
     __device__ long long nstride() const { return P; }
+    // 32 consecutive channels of pixel m: a lane's own row, 64 contiguous bytes of each copy
+    __device__ void copy_row(int m, int n0, const float *v) const {
+        if (!cp[0]) return;
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const int n = n0 + 8 * c;
+            if (n >= Cp) return;
+            float o8[8];
+#pragma unroll
+            for (int i = 0; i < 8; i++) o8[i] = n + i < Nch ? v[8 * c + i] : 0.f;
+            const long long o = (long long)m * Cp + n;
+            store_split8_n(o8, ns, enc, cp[0] + o, cp[1] + o, cp[2] + o);
+        }
+    }
 };
 
 }  // namespace seera

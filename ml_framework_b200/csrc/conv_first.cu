@@ -772,7 +772,7 @@ static bool first_tc_wgrad_ok(const FirstGeom &g, bool want_bias) {
 }
 
 static int first_tc_fwd(const float *X, const float *Wt, const float *bias, float *Y, const FirstGeom &g, int act, const char *name,
-                        const PoolOut *pool = nullptr) {
+                        const PoolOut *pool = nullptr, const StorePixelRows *with_copies = nullptr) {
     const int ns = rt().precision == 5 ? 2 : precision_copies();   // these kernels split into bf16 themselves: the fp16 modes 4 and 5 run as bf16x3
     const int bn = g.F <= 32 ? 32 : (g.F <= 64 ? 64 : 128);
     const int nslices = (g.K + 15) / 16;
@@ -785,6 +785,7 @@ static int first_tc_fwd(const float *X, const float *Wt, const float *bias, floa
     const size_t smem = fixed + (size_t)stages * ns * TC_BM * 128;
     const dim3 grid((unsigned)(tiles < rt().sm_count ? tiles : rt().sm_count));
     StorePixelRows cs{Y, g.F, g.OH * g.OW};
+    if (with_copies) cs = *with_copies;
     PoolOut po{};
     const int pool_on = pool ? 1 : 0;
     if (pool) { po = *pool; pool_out_geometry(po, g.OH * g.OW, g.OW, 1); }
@@ -861,10 +862,16 @@ int conv_first_pool_fwd(const float *X, const float *Wt, const float *bias, cons
     return first_tc_fwd(X, Wt, bias, nullptr, g, act, name, &pool);
 }
 
+bool conv_first_copies_ok(const float *X, const float *Y, int NB, int C, int H, int W, int F, int R, int S, int sh, int sw, int ph, int pw) {
+    FirstGeom g;
+    return first_geom(g, NB, C, H, W, F, R, S, sh, sw, ph, pw) && first_tc_fwd_ok(g) &&
+           !conv_c1_fwd_applies(X, Y, NB, C, H, W, F, R, S, sh, sw, ph, pw);
+}
 int conv_first_fwd(const float *X, const float *Wt, const float *bias, float *Y, int NB, int C, int H, int W, int F, int R, int S,
-                   int ph, int pw, int sh, int sw, int act, const char *name) {
+                   int ph, int pw, int sh, int sw, int act, const char *name, const StorePixelRows *with_copies) {
     FirstGeom g;
     if (!first_geom(g, NB, C, H, W, F, R, S, sh, sw, ph, pw)) return fail(SEERA_E_LIMIT, "%s: shape outside the short-patch kernel", name);
+    if (with_copies) return first_tc_fwd(X, Wt, bias, Y, g, act, name, nullptr, with_copies);
     if (conv_c1_fwd_applies(X, Y, NB, C, H, W, F, R, S, sh, sw, ph, pw))       // one input channel, "same" 3 x 3: output-bound stencil
         return conv_c1_fwd(X, Wt, bias, Y, NB, H, W, F, ph, act, name);
     if (first_tc_fwd_ok(g)) return first_tc_fwd(X, Wt, bias, Y, g, act, name);

@@ -270,7 +270,8 @@ struct StoreWgrad {
 
 // Y[NB, F, OH, OW] = conv(X_nhwc, weights Wk[F][tap][Cp]) with window R x S, stride, lower padding.
 static int tma_fprop(const NhwcShadow &x, const Shadow &wk, float *Y, int F, int R, int S, int sh, int sw, int ph, int pw,
-                     int OH, int OW, int ns, const char *name, const float *bias = nullptr, int act = 0, const PoolOut *pool = nullptr) {
+                     int OH, int OW, int ns, const char *name, const float *bias = nullptr, int act = 0, const PoolOut *pool = nullptr,
+                     const NhwcShadow *ycopies = nullptr) {
     TmaGemmParams p{};
     p.bias = bias; p.act = act;
     if (pool) { p.pool_on = 1; p.pool = *pool; pool_out_geometry(p.pool, OH * OW, OW, 0); }
@@ -288,7 +289,34 @@ static int tma_fprop(const NhwcShadow &x, const Shadow &wk, float *Y, int F, int
         if (int s = make_map_2d(&maps.b[i], wk.p[j], wk.rows, wk.cols, wk.ld, 64, p.pair ? p.bn / 2 : p.bn)) return s;
     }
     double flops = 2.0 * p.M * (double)F * x.C * R * S;
-    return launch_tma_gemm(maps, p, StorePixelRows{Y, F, OH * OW}, ns, false, flops, name);
+    StorePixelRows cs{Y, F, OH * OW};
+    if (ycopies) {
+        for (int i = 0; i < 3; i++) cs.cp[i] = ycopies->p[i];
+        cs.Cp = ycopies->Cp; cs.ns = ns; cs.enc = ycopies->enc;
+    }
+    return launch_tma_gemm(maps, p, cs, ns, false, flops, name);
+}
+
+// Unit-stride data gradient from the forward's filter copies w[F][tap][Cp] as they are: the contraction runs over (tap, filter), so
+// for a tap they are a [filter, channel] matrix read along its columns, taps in reverse order.
+static int tma_dgrad_kept(const NhwcShadow &dy, const Shadow &w, float *dX, int C, int R, int S, int ph, int pw, int H, int W, int ns,
+                          const char *name) {
+    TmaGemmParams p{};
+    p.a_mode = TMA_A_IM2COL; p.b_mn = 1;
+    p.a_fp16 = dy.enc.fmt; p.b_fp16 = w.enc.fmt; p.out_scale = 1.f / (dy.enc.scale * w.enc.scale); p.dinv = enc_dinv(dy.enc, w.enc);
+    p.M = dy.NB * H * W; p.N = C;
+    p.cchunks = (dy.Cp + 63) / 64; p.cpad = dy.Cp; p.taps = R * S; p.S = S;
+    p.wflip = w.cols / (R * S);
+    p.K = p.taps * p.cchunks * 64;
+    p.OW = W; p.OHW = H * W; p.sw = 1; p.sh = 1; p.pw = S - 1 - pw; p.ph = R - 1 - ph;
+    tma_plan(p, ns, false);
+    TmaMaps maps;
+    for (int i = 0; i < 3; i++) {
+        int j = i < ns ? i : 0;
+        if (int s = make_map_im2col(&maps.a[i], dy.p[j], dy.NB, dy.H, dy.W, dy.Cp, R, S, 1, 1, p.ph, p.pw, 64, TC_BM)) return s;
+        if (int s = make_map_2d(&maps.b[i], w.p[j], w.rows, w.cols, w.ld, 64, 64)) return s;
+    }
+    return launch_tma_gemm(maps, p, StorePixelRows{dX, C, H * W}, ns, false, 2.0 * p.M * (double)C * dy.C * R * S, name);
 }
 
 // dW[Fo][C][R][S] = sum over output pixels of dY_nhwc[pix, f] * X_nhwc[window(pix)+tap, c]
@@ -727,8 +755,11 @@ static const NhwcShadow *usable(const seera_shadow *h, int ns, int NB, int C, in
 
 // Convolution backward; xk / dyk are optional kept shadows of X / dY (dY itself may then be null unless the short-patch
 // weight gradient or a fallback needs the fp32 tensor).
+static int convT_bwd_products(const float *Wt, const float *X, const NhwcShadow &dys, float *dX, float *dW, int NB, int Cin, int H, int W, int Cout,
+                              int KH, int KW, int sh, int sw, int ph, int pw, const seera_shadow *x_shadow);
 static int tma_conv2d_bwd_kept(const float *Wt, const float *X, const float *dY, float *dX, float *dW, int NB, int C, int H, int W,
-                               int F, int R, int S, int sh, int sw, int ph, int pw, const seera_shadow *xk, const seera_shadow *dyk) {
+                               int F, int R, int S, int sh, int sw, int ph, int pw, const seera_shadow *xk, const seera_shadow *dyk,
+                               const seera_rows *wk = nullptr) {
     SEERA_ENSURE();
     if (!conv_ok(NB, C, H, W, F, R, S, sh, sw, ph, pw) || !X || !Wt || (!dY && !dyk)) return fail(SEERA_E_ARG, "cuda_conv2d_bwd: bad argument");
     int OH = (H + 2 * ph - R) / sh + 1, OW = (W + 2 * pw - S) / sw + 1;
@@ -749,8 +780,10 @@ static int tma_conv2d_bwd_kept(const float *Wt, const float *X, const float *dY,
     }
     if (!s && dX) {
         if (sh == 1 && sw == 1) {     // dX = forward convolution of dY with flipped taps and swapped channel roles, pad' = K-1-pad
-            s = make_weight_shadow(Wt, C, F, R * S, R * S, (long long)C * R * S, 1, ns, wd);
-            if (!s) s = tma_fprop(*dys, wd, dX, C, R, S, 1, 1, R - 1 - ph, S - 1 - pw, H, W, ns, "cuda_conv2d_bwd(dX)");
+            const Shadow *kept = rows_usable(wk, ns, F, R * S * ((C + 7) / 8 * 8), CLS_WEIGHT);
+            if (kept) s = tma_dgrad_kept(*dys, *kept, dX, C, R, S, ph, pw, H, W, ns, "cuda_conv2d_bwd(dX)");
+            else s = make_weight_shadow(Wt, C, F, R * S, R * S, (long long)C * R * S, 1, ns, wd);
+            if (!s && !kept) s = tma_fprop(*dys, wd, dX, C, R, S, 1, 1, R - 1 - ph, S - 1 - pw, H, W, ns, "cuda_conv2d_bwd(dX)");
         } else if (phases) {
             s = tma_dgrad_phases(*dys, Wt, R * S, (long long)C * R * S, dX, C, H, W, R, S, sh, sw, ph, pw, ns, "cuda_conv2d_bwd(dX)");
         } else {
@@ -769,9 +802,31 @@ static int tma_conv2d_bwd_kept(const float *Wt, const float *X, const float *dY,
     return s;
 }
 
+// Both products of a transposed convolution's backward from the copies of its output gradient.
+static int convT_bwd_products(const float *Wt, const float *X, const NhwcShadow &dys, float *dX, float *dW, int NB, int Cin, int H, int W, int Cout,
+                              int KH, int KW, int sh, int sw, int ph, int pw, const seera_shadow *x_shadow) {
+    const int ns = precision_copies(), taps = KH * KW;
+    NhwcShadow local; Shadow wk;
+    int s = SEERA_OK;
+    if (dX) {            // dX[NB,Cin,H,W] = convolution of dY with Wt read as [F = Cin][C = Cout][KH][KW]
+        s = make_weight_shadow(Wt, Cin, Cout, taps, (long long)Cout * taps, taps, 0, ns, wk);
+        if (!s) s = tma_fprop(dys, wk, dX, Cin, KH, KW, sh, sw, ph, pw, H, W, ns, "cuda_conv2DTranspose_bwd(dX)");
+    }
+    if (!s && dW) {      // dW[Cin][Cout][KH][KW]: weight gradient of that convolution with dY as its input and X as its output gradient
+        const NhwcShadow *xs = usable(x_shadow, wgrad_copies(ns), NB, Cin, H, W, CLS_ACT);
+        if (!xs) { s = make_nhwc(X, NB, Cin, H, W, ns, local, CLS_ACT); xs = &local; }
+        if (!s) s = tma_wgrad(dys, *xs, dW, KH, KW, sh, sw, ph, pw, wgrad_copies(ns), "cuda_conv2DTranspose_bwd(dW)");
+    }
+    free_nhwc(local); free_shadow(wk);
+    return s;
+}
+
 }  // namespace seera
 
 using namespace seera;
+
+static int convT_fwd_kept(const float *X, const float *Wt, const float *bias, float *out, int NB, int Cin, int H, int W, int Cout, int KH,
+                          int KW, int sh, int sw, int ph, int pw, int act, const seera_shadow *x_in, seera_shadow **x_keep);
 
 extern "C" {
 
@@ -824,29 +879,62 @@ void seera_shadow_free(seera_shadow_t *h) {
 
 int seera_conv2d_bias_act_fwd_s(const float *X, const float *Wt, const float *bias, float *Y, int NB, int C, int H, int W, int F,
                                 int R, int S, int ph, int pw, int sh, int sw, int act, seera_shadow_t *x_in, seera_shadow_t **x_keep) {
+    return seera_conv2d_bias_act_fwd_k(X, Wt, bias, Y, NB, C, H, W, F, R, S, ph, pw, sh, sw, act, x_in, x_keep, nullptr, nullptr);
+}
+
+int seera_conv2d_bias_act_fwd_k(const float *X, const float *Wt, const float *bias, float *Y, int NB, int C, int H, int W, int F,
+                                int R, int S, int ph, int pw, int sh, int sw, int act, seera_shadow_t *x_in, seera_shadow_t **x_keep,
+                                seera_rows_t **w_keep, seera_shadow_t **y_copies) {
     SEERA_ENSURE();
     if (x_keep) *x_keep = nullptr;
-    if (!keeps_shadows(NB, C, H, W, F, R, S, sh, sw, ph, pw))
+    if (w_keep) *w_keep = nullptr;
+    if (y_copies) *y_copies = nullptr;
+    int OH = (H + 2 * ph - R) / (sh > 0 ? sh : 1) + 1, OW = (W + 2 * pw - S) / (sw > 0 ? sw : 1) + 1;
+    const int ns = precision_copies();
+    // the copies of the output, where the layer that writes it can write them on the way
+    NhwcShadow yc;
+    auto want_copies = [&]() -> int {
+        if (!y_copies) return SEERA_OK;
+        yc.NB = NB; yc.H = OH; yc.W = OW; yc.C = F; yc.Cp = (F + 7) / 8 * 8;
+        yc.enc = enc_for(CLS_ACT);
+        const size_t bytes = (size_t)NB * OH * OW * yc.Cp * 2;
+        for (int i = 0; i < ns; i++) { yc.p[i] = (__nv_bfloat16 *)scratch_alloc(bytes); if (!yc.p[i]) { free_nhwc(yc); return SEERA_E_OOM; } }
+        return SEERA_OK;
+    };
+    auto hand_copies = [&](int s) {
+        if (!s && y_copies && yc.p[0]) *y_copies = new seera_shadow{yc, ns};
+        else free_nhwc(yc);
+        return s;
+    };
+    if (!keeps_shadows(NB, C, H, W, F, R, S, sh, sw, ph, pw)) {
+        if (y_copies && rt().precision && rt().conv_tma && X && Wt && Y && conv_ok(NB, C, H, W, F, R, S, sh, sw, ph, pw) && OH >= 1 && OW >= 1 &&
+            conv_first_copies_ok(X, Y, NB, C, H, W, F, R, S, sh, sw, ph, pw)) {
+            if (int s = want_copies()) return s;
+            StorePixelRows cs{Y, F, OH * OW};
+            for (int i = 0; i < 3; i++) cs.cp[i] = yc.p[i];
+            cs.Cp = yc.Cp; cs.ns = ns; cs.enc = yc.enc;
+            return hand_copies(conv_first_fwd(X, Wt, bias, Y, NB, C, H, W, F, R, S, ph, pw, sh, sw, act, "cuda_conv2d_fwd", &cs));
+        }
         return seera_conv2d_bias_act_fwd(X, Wt, bias, Y, NB, C, H, W, F, R, S, ph, pw, sh, sw, act);
+    }
     if (!X || !Wt || !Y) return fail(SEERA_E_ARG, "cuda_conv2d_fwd: bad argument");
-    int OH = (H + 2 * ph - R) / sh + 1, OW = (W + 2 * pw - S) / sw + 1;
     if (OH < 1 || OW < 1) return fail(SEERA_E_ARG, "cuda_conv2d_fwd: kernel larger than padded input");
     if (sh == 1 && sw == 1 && conv_few_applies(NB, C, F, R, S, OH, OW))       // reads X in place: no copies made, none kept
         return conv_few_fwd(X, Wt, bias, Y, NB, C, H, W, F, R, S, ph, pw, OH, OW, act, 0, "cuda_conv2d_fwd");
-    int ns = precision_copies();
     NhwcShadow local; Shadow wk;
     const NhwcShadow *xs = usable(x_in, ns, NB, C, H, W, CLS_ACT);
     int s = SEERA_OK;
     if (!xs) { s = make_nhwc(X, NB, C, H, W, ns, local, CLS_ACT); xs = &local; }
     if (!s) s = make_weight_shadow(Wt, F, C, R * S, (long long)C * R * S, R * S, 0, ns, wk);
-    if (!s) s = tma_fprop(*xs, wk, Y, F, R, S, sh, sw, ph, pw, OH, OW, ns, "cuda_conv2d_fwd", bias, act);
-    free_shadow(wk);
+    if (!s) s = want_copies();
+    if (!s) s = tma_fprop(*xs, wk, Y, F, R, S, sh, sw, ph, pw, OH, OW, ns, "cuda_conv2d_fwd", bias, act, nullptr, y_copies ? &yc : nullptr);
+    if (!s && w_keep && sh == 1 && sw == 1) *w_keep = new seera_rows{wk, ns}; else free_shadow(wk);
     if (!s && x_keep && xs == &local) {
         *x_keep = new seera_shadow{local, ns};          // ownership of the device copies moves to the handle
     } else {
         free_nhwc(local);
     }
-    return s;
+    return hand_copies(s);
 }
 
 int seera_maxpool2x2_fwd_s(const float *X, float *out, int *mask, int N, int C, int H, int W, seera_shadow_t **out_shadow) {
@@ -899,8 +987,15 @@ int seera_conv2d_pool_fusable(int NB, int C, int H, int W, int F, int R, int S, 
 int seera_conv2d_bias_act_pool_fwd_s(const float *X, const float *Wt, const float *bias, float *pooled, int *mask, int NB, int C, int H,
                                      int W, int F, int R, int S, int ph, int pw, int sh, int sw, int act, seera_shadow_t *x_in,
                                      seera_shadow_t **x_keep, seera_shadow_t **pooled_copies) {
+    return seera_conv2d_bias_act_pool_fwd_k(X, Wt, bias, pooled, mask, NB, C, H, W, F, R, S, ph, pw, sh, sw, act, x_in, x_keep, nullptr,
+                                            pooled_copies);
+}
+int seera_conv2d_bias_act_pool_fwd_k(const float *X, const float *Wt, const float *bias, float *pooled, int *mask, int NB, int C, int H,
+                                     int W, int F, int R, int S, int ph, int pw, int sh, int sw, int act, seera_shadow_t *x_in,
+                                     seera_shadow_t **x_keep, seera_rows_t **w_keep, seera_shadow_t **pooled_copies) {
     SEERA_ENSURE();
     if (x_keep) *x_keep = nullptr;
+    if (w_keep) *w_keep = nullptr;
     if (pooled_copies) *pooled_copies = nullptr;
     if (!X || !Wt || !pooled || !mask) return fail(SEERA_E_ARG, "conv2d_pool_fwd: bad argument");
     if (!pool_in_epilogue_ok(NB, C, H, W, F, R, S, sh, sw, ph, pw))
@@ -928,7 +1023,7 @@ int seera_conv2d_bias_act_pool_fwd_s(const float *X, const float *Wt, const floa
         if (!xs) { s = make_nhwc(X, NB, C, H, W, ns, local, CLS_ACT); xs = &local; }
         if (!s) s = make_weight_shadow(Wt, F, C, R * S, (long long)C * R * S, R * S, 0, ns, wk);
         if (!s) s = tma_fprop(*xs, wk, nullptr, F, R, S, sh, sw, ph, pw, OH, OW, ns, "conv2d_pool_fwd", bias, act, &po);
-        free_shadow(wk);
+        if (!s && w_keep && sh == 1 && sw == 1) *w_keep = new seera_rows{wk, ns}; else free_shadow(wk);
         if (!s && x_keep && xs == &local) *x_keep = new seera_shadow{local, ns};
         else free_nhwc(local);
     }
@@ -989,6 +1084,11 @@ static int make_dz_shadow(const float *g, const float *gp, const int *mask, cons
 int seera_conv2d_act_bwd(const float *Wt, const float *X, const float *y, const float *g, const float *gp, const int *pool_mask,
                          const float *y_pooled, float *dX, float *dW, float *dbias, int NB, int C, int H, int W, int F, int R, int S, int sh, int sw,
                          int ph, int pw, int act, seera_shadow_t *x_shadow) {
+    return seera_conv2d_act_bwd_k(Wt, X, y, g, gp, pool_mask, y_pooled, dX, dW, dbias, NB, C, H, W, F, R, S, sh, sw, ph, pw, act, x_shadow, nullptr);
+}
+int seera_conv2d_act_bwd_k(const float *Wt, const float *X, const float *y, const float *g, const float *gp, const int *pool_mask,
+                           const float *y_pooled, float *dX, float *dW, float *dbias, int NB, int C, int H, int W, int F, int R, int S, int sh,
+                           int sw, int ph, int pw, int act, seera_shadow_t *x_shadow, seera_rows_t *w_keep) {
     SEERA_ENSURE();
     if (!conv_ok(NB, C, H, W, F, R, S, sh, sw, ph, pw) || !X || !Wt || (g == nullptr) == (gp == nullptr) || (gp && !pool_mask) ||
         (act != SEERA_ACT_NONE && !y && !(gp && y_pooled)))
@@ -1001,7 +1101,7 @@ int seera_conv2d_act_bwd(const float *Wt, const float *X, const float *y, const 
         (sh == 1 && sw == 1 ? true : phases_supported(H, W, OH, OW, R, S, sh, sw, ph, pw) || !dX)) {
         seera_shadow dz{NhwcShadow{}, precision_copies()};
         int s = make_dz_shadow(g, gp, pool_mask, y, gp ? y_pooled : nullptr, dbias, NB, F, OH, OW, act, dz.ns, dz.s);
-        if (!s) s = tma_conv2d_bwd_kept(Wt, X, nullptr, dX, dW, NB, C, H, W, F, R, S, sh, sw, ph, pw, x_shadow, &dz);
+        if (!s) s = tma_conv2d_bwd_kept(Wt, X, nullptr, dX, dW, NB, C, H, W, F, R, S, sh, sw, ph, pw, x_shadow, &dz, w_keep);
         free_nhwc(dz.s);
         return s;
     }
@@ -1046,6 +1146,11 @@ int seera_tma_convT_fwd(const float *X, const float *Wt, float *out, int NB, int
 // out = act(convT(X, Wt) + bias[cout]); bias may be null.
 int seera_tma_convT_bias_act_fwd(const float *X, const float *Wt, const float *bias, float *out, int NB, int Cin, int H, int W,
                                  int Cout, int KH, int KW, int sh, int sw, int ph, int pw, int act) {
+    return convT_fwd_kept(X, Wt, bias, out, NB, Cin, H, W, Cout, KH, KW, sh, sw, ph, pw, act, nullptr, nullptr);
+}
+}  // extern "C"
+static int convT_fwd_kept(const float *X, const float *Wt, const float *bias, float *out, int NB, int Cin, int H, int W, int Cout, int KH,
+                          int KW, int sh, int sw, int ph, int pw, int act, const seera_shadow *x_in, seera_shadow **x_keep) {
     SEERA_ENSURE();
     int Ho = (H - 1) * sh - 2 * ph + KH, Wo = (W - 1) * sw - 2 * pw + KW;
     if (!conv_ok(NB, Cin, H, W, Cout, KH, KW, sh, sw, ph, pw) || Ho < 1 || Wo < 1 || !X || !Wt || !out)
@@ -1060,9 +1165,11 @@ int seera_tma_convT_bias_act_fwd(const float *X, const float *Wt, const float *b
         return s;
     }
     int ns = precision_copies();
-    NhwcShadow xs; Shadow wd;
-    int taps = KH * KW;
-    int s = make_nhwc(X, NB, Cin, H, W, ns, xs, CLS_ACT);
+    NhwcShadow local; Shadow wd;
+    int taps = KH * KW, s = SEERA_OK;
+    const NhwcShadow *given = usable(x_in, ns, NB, Cin, H, W, CLS_ACT);
+    if (!given) s = make_nhwc(X, NB, Cin, H, W, ns, local, CLS_ACT);
+    const NhwcShadow &xs = given ? *given : local;
     if (!s && unit) {
         s = make_weight_shadow(Wt, Cout, Cin, taps, taps, (long long)Cout * taps, 1, ns, wd);
         if (!s) s = tma_fprop(xs, wd, out, Cout, KH, KW, 1, 1, KH - 1 - ph, KW - 1 - pw, Ho, Wo, ns, "cuda_conv2DTranpose_fwd", bias, act);
@@ -1070,8 +1177,18 @@ int seera_tma_convT_bias_act_fwd(const float *X, const float *Wt, const float *b
         s = tma_dgrad_phases(xs, Wt, taps, (long long)Cout * taps, out, Cout, Ho, Wo, KH, KW, sh, sw, ph, pw, ns, "cuda_conv2DTranpose_fwd",
                              bias, act);
     }
-    free_nhwc(xs); free_shadow(wd);
+    if (!s && x_keep && !given) *x_keep = new seera_shadow{local, ns}; else free_nhwc(local);
+    free_shadow(wd);
     return s;
+}
+extern "C" {
+int seera_conv2DTranspose_bias_act_fwd_k(const float *X, const float *W, const float *bias, float *out, int batch, int Cin, int Hin, int Win,
+                                         int Cout, int KH, int KW, int sh, int sw, int ph, int pw, int act, seera_shadow_t *x_in,
+                                         seera_shadow_t **x_keep) {
+    if (x_keep) *x_keep = nullptr;
+    if (rt().precision && rt().conv_tma)
+        return convT_fwd_kept(X, W, bias, out, batch, Cin, Hin, Win, Cout, KH, KW, sh, sw, ph, pw, act, x_in, x_keep);
+    return seera_conv2DTranspose_bias_act_fwd(X, W, bias, out, batch, Cin, Hin, Win, Cout, KH, KW, sh, sw, ph, pw, act);
 }
 
 int seera_tma_convT_bwd(const float *Wt, const float *X, const float *dY, float *dX, float *dW, int NB, int Cin, int H, int W,
@@ -1089,19 +1206,35 @@ int seera_tma_convT_bwd(const float *Wt, const float *X, const float *dY, float 
         if (!s && dW) s = conv_first_wgrad(dY, X, dW, NB, Cout, Ho, Wo, Cin, KH, KW, sh, sw, ph, pw, "cuda_conv2DTranspose_bwd(dW)");
         return s;
     }
-    int ns = precision_copies();
-    int taps = KH * KW;
-    NhwcShadow dys, xs; Shadow wk;
-    int s = make_nhwc(dY, NB, Cout, Ho, Wo, ns, dys, CLS_GRAD);
-    if (!s && dX) {      // dX[NB,Cin,H,W] = convolution of dY with Wt read as [F = Cin][C = Cout][KH][KW]
-        s = make_weight_shadow(Wt, Cin, Cout, taps, (long long)Cout * taps, taps, 0, ns, wk);
-        if (!s) s = tma_fprop(dys, wk, dX, Cin, KH, KW, sh, sw, ph, pw, H, W, ns, "cuda_conv2DTranspose_bwd(dX)");
+    NhwcShadow dys;
+    int s = make_nhwc(dY, NB, Cout, Ho, Wo, precision_copies(), dys, CLS_GRAD);
+    if (!s) s = convT_bwd_products(Wt, X, dys, dX, dW, NB, Cin, H, W, Cout, KH, KW, sh, sw, ph, pw, nullptr);
+    free_nhwc(dys);
+    return s;
+}
+
+// Backward of y = act(convT(X, Wt) + bias) from the gradient g of y: slope, bias gradient and the products' operand copies in one pass.
+int seera_conv2DTranspose_act_bwd_k(const float *Wt, const float *X, const float *y, const float *g, float *dX, float *dW, float *dbias,
+                                    int NB, int Cin, int H, int W, int Cout, int KH, int KW, int sh, int sw, int ph, int pw, int act,
+                                    seera_shadow_t *x_shadow) {
+    SEERA_ENSURE();
+    int Ho = (H - 1) * sh - 2 * ph + KH, Wo = (W - 1) * sw - 2 * pw + KW;
+    if (!conv_ok(NB, Cin, H, W, Cout, KH, KW, sh, sw, ph, pw) || Ho < 1 || Wo < 1 || !X || !Wt || !g || !dW || !dbias || (act != SEERA_ACT_NONE && !y) ||
+        (Ho + 2 * ph - KH) / sh + 1 != H || (Wo + 2 * pw - KW) / sw + 1 != W)
+        return fail(SEERA_E_ARG, "conv2DTranspose_act_bwd: bad argument");
+    if (rt().precision && rt().conv_tma && tma_conv_supported(NB, KH, KW, sh, sw, ph, pw) && !conv_first_applies(Cout, KH, KW)) {
+        NhwcShadow dys;
+        int s = make_dz_shadow(g, nullptr, nullptr, y, nullptr, dbias, NB, Cout, Ho, Wo, act, precision_copies(), dys);
+        if (!s) s = convT_bwd_products(Wt, X, dys, dX, dW, NB, Cin, H, W, Cout, KH, KW, sh, sw, ph, pw, x_shadow);
+        free_nhwc(dys);
+        return s;
     }
-    if (!s && dW) {      // dW[Cin][Cout][KH][KW]: weight gradient of that convolution with dY as its input and X as its output gradient
-        s = make_nhwc(X, NB, Cin, H, W, ns, xs, CLS_ACT);
-        if (!s) s = tma_wgrad(dys, xs, dW, KH, KW, sh, sw, ph, pw, wgrad_copies(ns), "cuda_conv2DTranspose_bwd(dW)");
-    }
-    free_nhwc(dys); free_nhwc(xs); free_shadow(wk);
+    const int n = NB * Cout * Ho * Wo;
+    float *dz = act ? (float *)scratch_alloc((size_t)n * sizeof(float)) : nullptr;
+    if (act && !dz) return SEERA_E_OOM;
+    int s = seera_act_bias_bwd(g, act ? y : nullptr, act ? dz : const_cast<float *>(g), dbias, n, Cout, Ho * Wo, act);
+    if (!s) s = seera_cuda_conv2DTranspose_bwd(Wt, X, act ? dz : g, dX, dW, NB, Cin, H, W, Cout, KH, KW, sh, sw, ph, pw);
+    if (dz) scratch_free(dz);
     return s;
 }
 

@@ -19,14 +19,6 @@
 #include "tma_gemm_kernel.cuh"
 
 
-// ---- Dense layers that hand their 16-bit operand copies from call to call ------------------------------------------------
-// Row-major copies of one [rows, cols] matrix (activations of a Dense layer, or its weight matrix), kept by the caller
-// between the forward and the backward call of a layer, or written by one layer's epilogue for the next layer's forward.
-struct seera_rows {
-    seera::Shadow s;
-    int ns;
-};
-
 namespace seera {
 
 // C[m*ld + n] plus the 16-bit copies of the same values: the output of a Dense layer that feeds another Dense layer.
@@ -114,7 +106,7 @@ __global__ void __launch_bounds__(256) dz_rows_kernel(const float *__restrict__ 
         }
     }
 }
-static const Shadow *rows_usable(const seera_rows *h, int ns, int rows, int cols, int cls) {
+const Shadow *rows_usable(const seera_rows *h, int ns, int rows, int cols, int cls) {
     const Enc want = enc_for(cls);
     if (!h || h->ns < ns || h->s.rows != rows || h->s.cols != cols || h->s.enc.fmt != want.fmt || h->s.enc.scale != want.scale ||
         h->s.enc.dscale != want.dscale) return nullptr;

@@ -65,8 +65,11 @@ int wgrad_c1(const float *A, const float *dY, float *dW, int NB, int H, int W, i
              const char *name);
 // Direct fp32 kernels for convolutions with C*R*S <= 64 (conv_first.cu); bias may be null.
 bool conv_first_applies(int C, int R, int S);
+// `cs` (may be null): where the output goes, with its channels-last copies; only where conv_first_copies_ok says so.
+struct StorePixelRows;
 int conv_first_fwd(const float *X, const float *Wt, const float *bias, float *Y, int NB, int C, int H, int W, int F, int R, int S,
-                   int ph, int pw, int sh, int sw, int act, const char *name);
+                   int ph, int pw, int sh, int sw, int act, const char *name, const StorePixelRows *cs = nullptr);
+bool conv_first_copies_ok(const float *X, const float *Y, int NB, int C, int H, int W, int F, int R, int S, int sh, int sw, int ph, int pw);
 bool conv_first_fuses_bias(int C, int R, int S);
 int conv_first_act_wgrad(const float *X, const float *y, const float *g, const float *gp, const int *mask, const float *y_pooled,
                          float *dW, float *dbias, int NB, int C, int H, int W, int F, int R, int S, int sh, int sw, int ph, int pw,

@@ -257,6 +257,36 @@ PYBIND11_MODULE(seera_cuda, m) {
         ck(seera_conv2d_bias_act_pool_fwd_s(P<const F>(x), P<const F>(w), P<const F>(b), P<F>(pooled), P<int>(mask), N, C, H, W, Fo, R, S,
                                             ph, pw, sh, sw, act, P<seera_shadow_t>(x_in), &keep, want_copies ? &pc : nullptr));
         return std::make_pair(reinterpret_cast<uptr>(keep), reinterpret_cast<uptr>(pc)); });
+    // forms that hand more from call to call: (x_keep, w_keep, y_copies), (x_keep, w_keep, pooled_copies), x_keep; 0 where there is none
+    m.def("conv2d_bias_act_fwd_k", [](uptr x, uptr w, uptr b, uptr o, int N, int C, int H, int W, int Fo, int R, int S, int ph, int pw, int sh,
+                                      int sw, int act, uptr x_in, bool want_y) {
+        seera_shadow_t *xk = nullptr, *yc = nullptr;
+        seera_rows_t *wk = nullptr;
+        ck(seera_conv2d_bias_act_fwd_k(P<const F>(x), P<const F>(w), P<const F>(b), P<F>(o), N, C, H, W, Fo, R, S, ph, pw, sh, sw, act,
+                                       P<seera_shadow_t>(x_in), &xk, &wk, want_y ? &yc : nullptr));
+        return py::make_tuple(reinterpret_cast<uptr>(xk), reinterpret_cast<uptr>(wk), reinterpret_cast<uptr>(yc)); });
+    m.def("conv2d_bias_act_pool_fwd_k", [](uptr x, uptr w, uptr b, uptr pooled, uptr mask, int N, int C, int H, int W, int Fo, int R, int S, int ph,
+                                           int pw, int sh, int sw, int act, uptr x_in, bool want_copies) {
+        seera_shadow_t *xk = nullptr, *pc = nullptr;
+        seera_rows_t *wk = nullptr;
+        ck(seera_conv2d_bias_act_pool_fwd_k(P<const F>(x), P<const F>(w), P<const F>(b), P<F>(pooled), P<int>(mask), N, C, H, W, Fo, R, S, ph, pw,
+                                            sh, sw, act, P<seera_shadow_t>(x_in), &xk, &wk, want_copies ? &pc : nullptr));
+        return py::make_tuple(reinterpret_cast<uptr>(xk), reinterpret_cast<uptr>(wk), reinterpret_cast<uptr>(pc)); });
+    m.def("conv2d_act_bwd_k", [](uptr w, uptr x, uptr y, uptr g, uptr gp, uptr mask, uptr yp, uptr dx, uptr dw, uptr db, int N, int C, int H,
+                                 int W, int Fo, int R, int S, int sh, int sw, int ph, int pw, int act, uptr x_shadow, uptr w_keep) {
+        ck(seera_conv2d_act_bwd_k(P<const F>(w), P<const F>(x), P<const F>(y), P<const F>(g), P<const F>(gp), P<const int>(mask), P<const F>(yp),
+                                  P<F>(dx), P<F>(dw), P<F>(db), N, C, H, W, Fo, R, S, sh, sw, ph, pw, act, P<seera_shadow_t>(x_shadow),
+                                  P<seera_rows_t>(w_keep))); });
+    m.def("conv2DTranspose_bias_act_fwd_k", [](uptr x, uptr w, uptr b, uptr o, int N, int Ci, int H, int W, int Co, int KH, int KW, int sh, int sw,
+                                               int ph, int pw, int act, uptr x_in) {
+        seera_shadow_t *xk = nullptr;
+        ck(seera_conv2DTranspose_bias_act_fwd_k(P<const F>(x), P<const F>(w), P<const F>(b), P<F>(o), N, Ci, H, W, Co, KH, KW, sh, sw, ph, pw, act,
+                                                P<seera_shadow_t>(x_in), &xk));
+        return reinterpret_cast<uptr>(xk); });
+    m.def("conv2DTranspose_act_bwd_k", [](uptr w, uptr x, uptr y, uptr g, uptr dx, uptr dw, uptr db, int N, int Ci, int H, int W, int Co, int KH,
+                                          int KW, int sh, int sw, int ph, int pw, int act, uptr x_shadow) {
+        ck(seera_conv2DTranspose_act_bwd_k(P<const F>(w), P<const F>(x), P<const F>(y), P<const F>(g), P<F>(dx), P<F>(dw), P<F>(db), N, Ci, H, W,
+                                           Co, KH, KW, sh, sw, ph, pw, act, P<seera_shadow_t>(x_shadow))); });
     m.def("shadow_free", [](uptr h) { seera_shadow_free(P<seera_shadow_t>(h)); });
     m.def("rows_free", [](uptr h) { seera_rows_free(P<seera_rows_t>(h)); });
     // Dense forward that keeps / hands on its operand copies: returns (a_keep, w_keep, c_copies) handles (0: none)

@@ -42,6 +42,14 @@ __device__ __forceinline__ auto maybe_copy_out4(const CS &cs, int m, int n, cons
 template <class CS>
 __device__ __forceinline__ void maybe_copy_out4(const CS &, int, int, const float4 &, long) {}
 
+// ... or copy_row(m, n0, 32 values) where lanes hold rows.
+template <class CS>
+__device__ __forceinline__ auto maybe_copy_row(const CS &cs, int m, int n0, const float *v, int) -> decltype(cs.copy_row(m, n0, v), void()) {
+    cs.copy_row(m, n0, v);
+}
+template <class CS>
+__device__ __forceinline__ void maybe_copy_row(const CS &, int, int, const float *, long) {}
+
 struct NoRelease { __device__ void operator()() const {} };
 
 template <class CS, class Release = NoRelease>
@@ -104,6 +112,7 @@ __device__ __forceinline__ void drain_accumulator(uint32_t taddr, int row_base, 
                         q += sn;
                     }
                 }
+                maybe_copy_row(cs, m_own, col_base + c, v, 0);
             }
         }
     } else {

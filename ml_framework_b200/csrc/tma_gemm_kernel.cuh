@@ -55,6 +55,19 @@ struct Shadow {
     Enc enc{0, 1.f, nullptr};
 };
 
+}  // namespace seera
+// ---- layers that hand their 16-bit operand copies from call to call --------------------------------------------------------
+// Row-major copies of one [rows, cols] matrix (activations of a Dense layer, its weight matrix, a convolution's filters as
+// [F][tap][channel]), kept by the caller between the forward and the backward call of a layer, or written by one layer's epilogue
+// for the next layer's forward.
+struct seera_rows {
+    seera::Shadow s;
+    int ns;
+};
+namespace seera {
+// The copies if they serve a product of `ns` copies of a [rows, cols] matrix of this class in the present encoding, else null.
+const Shadow *rows_usable(const seera_rows *h, int ns, int rows, int cols, int cls);
+
 // Classes of tensor, for the scale of an fp16 encoding: activations are O(1) after He / Glorot initialisation, weights a
 // few hundredths, gradients of a batch-mean loss 1e-6 .. 1e-2.  With the factors 2^4 / 2^8 / 2^12 the second copy of a
 // value stays a normal fp16 number down to a magnitude of 2^-7 / 2^-11 / 2^-15 (below that its absolute error is
@@ -234,6 +247,8 @@ struct TmaGemmParams {
     int sw, sh, pw, ph;      // window stride and lower padding
     int S, taps;             // filter width and R*S
     int cpad, cchunks;       // channel pitch of the weight rows / channels rounded up to 64, in chunks of 64
+    int wflip;               // TMA_A_IM2COL with b_mn: B is [channel of A][tap][wflip columns], its taps in reverse order (a data
+                             // gradient that reads the forward's filter copies as they are)
     float *partial;
     int *status;
     unsigned long long wait_clocks;   // budget of every bounded wait in the kernel
@@ -378,7 +393,7 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
                 }
                 if (leader) {
                 if (rank == 0) mbar_expect_tx(full0 + 8 * s, tx_bytes);
-                int bk = k0;                                  // B's coordinate along the contraction
+                int bk = k0, bx = 0;                          // B's coordinate along the contraction, and where its columns begin
                 if (p.a_mode == TMA_A_ROWS) {
 #pragma unroll
                     for (int i = 0; i < NS; i++) ld2d(a_tile(s, i), mA[i], k0, m0, bar);
@@ -391,7 +406,8 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
                     int r = p.by_S.div(tap), sx = tap - r * p.S;
 #pragma unroll
                     for (int i = 0; i < NS; i++) ldim(a_tile(s, i), mA[i], c0, pix_w, pix_h, pix_img, sx, r, bar);
-                    bk = tap * p.cpad + c0;
+                    if (p.b_mn) { bk = c0; bx = (p.taps - 1 - tap) * p.wflip; }
+                    else bk = tap * p.cpad + c0;
                 } else {
                     int img = p.by_OHW.div(k0), rem = k0 - img * p.OHW, oh = p.by_OW.div(rem), ow = rem - oh * p.OW;
                     int w = ow * p.sw - p.pw, h = oh * p.sh - p.ph;
@@ -403,7 +419,7 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
                 if (p.b_mn) {
 #pragma unroll
                     for (int i = 0; i < NS; i++)
-                        for (int b = 0; b < bh / 64; b++) ld2d(b_tile(s, i) + b * 8192, mB[i], nb0 + 64 * b, bk, bar);
+                        for (int b = 0; b < bh / 64; b++) ld2d(b_tile(s, i) + b * 8192, mB[i], bx + nb0 + 64 * b, bk, bar);
                 } else {
 #pragma unroll
                     for (int i = 0; i < NS; i++) ld2d(b_tile(s, i), mB[i], bk, nb0, bar);

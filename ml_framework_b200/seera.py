@@ -182,6 +182,8 @@ tensor = Tensor
 FUSE_POOL = True
 # A 2x2 unpooling that feeds a ConvTranspose2D leaves its output unmade until somebody reads it (see _Unpooled).
 _LAZY_UNPOOL = hasattr(sc, "unpool2_convT_fusable")
+# The engine's forms that hand operand copies on from call to call (filters to the data gradient, outputs to the next convolution).
+_KEEPS = hasattr(sc, "conv2d_act_bwd_k")
 # A Dense layer that feeds another Dense layer can have its GEMM epilogue write the 16-bit copies of its output that the next
 # layer's GEMM reads (seera_matmul_bias_act_fwd_s, c_copies).  Off: at the sizes measured (4096 x 1024 outputs, one tile per
 # CTA) the two-byte stores lengthen an epilogue that nothing overlaps by more than the next layer's vectorised conversion
@@ -310,7 +312,7 @@ class autograd4nn:
 class Layer:
     # which layers read this one's output (set while a model is put together): a producer can then hand on more than its values
     _pool_consumer = None
-    _feeds_conv = _feeds_dense = _feeds_convT = False
+    _feeds_conv = _feeds_dense = _feeds_convT = _feeds_copies = False
     _fused = None                    # a pool that the layer folded into its own launch: (pooled, mask, copies)
     _model = None
 
@@ -497,6 +499,8 @@ class Conv2D(_ParamLayer):
     def __call__(self, input_layer):
         super().__call__(input_layer)
         input_layer._feeds_conv = True        # a pooling producer then also emits the channels-last copies this layer reads
+        if self.out_channels not in (1, 2, 4):        # those few read their input in place
+            input_layer._feeds_copies = True
         return self
 
     def forward(self):
@@ -524,14 +528,22 @@ class Conv2D(_ParamLayer):
             half = (N, F, OH // 2, OW // 2)
             pooled = _new(half)
             pmask = _wrap(sc.cuda_malloc_i32(pooled.size), half, "int32")
-            h, hp = sc.conv2d_bias_act_pool_fwd_s(xv.main_ptr, wv.main_ptr, b.value.main_ptr, pooled._ptr, pmask._ptr, N, C, H, Wd, F, KH, KW,
-                                                  ph, pw, sh, sw, code, given.h if given else 0, pool._feeds_conv)
+            args = (xv.main_ptr, wv.main_ptr, b.value.main_ptr, pooled._ptr, pmask._ptr, N, C, H, Wd, F, KH, KW, ph, pw, sh, sw, code,
+                    given.h if given else 0, pool._feeds_conv)
+            if _KEEPS:
+                h, hw, hp = sc.conv2d_bias_act_pool_fwd_k(*args)
+            else:
+                (h, hp), hw = sc.conv2d_bias_act_pool_fwd_s(*args), 0
             self._fused = (pooled, pmask, _KeptCopies(hp) if hp else None)
+            hy = 0
         else:
             z = _new((N, F, OH, OW))
-            h = sc.conv2d_bias_act_fwd_s(xv.main_ptr, wv.main_ptr, b.value.main_ptr, z._ptr, N, C, H, Wd, F, KH, KW, ph, pw, sh, sw, code,
-                                         given.h if given else 0)
-        kept = _KeptCopies(h) if h else None
+            args = (xv.main_ptr, wv.main_ptr, b.value.main_ptr, z._ptr, N, C, H, Wd, F, KH, KW, ph, pw, sh, sw, code, given.h if given else 0)
+            if _KEEPS:
+                h, hw, hy = sc.conv2d_bias_act_fwd_k(*args, self._feeds_copies)
+            else:
+                h, hw, hy = sc.conv2d_bias_act_fwd_s(*args), 0, 0
+        kept, kept_w = _KeptCopies(h) if h else None, _KeptRows(hw) if hw else None
         need_dx = not x.is_leaf
 
         def backward(g):
@@ -543,15 +555,20 @@ class Conv2D(_ParamLayer):
             else:
                 gptr, gpptr, mptr, ypptr = g.main_ptr, 0, 0, 0
             k = kept or given
-            sc.conv2d_act_bwd(wv._ptr, xv._ptr, z._ptr, gptr, gpptr, mptr, ypptr, dx._ptr if need_dx else 0, dw._ptr, db._ptr,
-                              N, C, H, Wd, F, KH, KW, sh, sw, ph, pw, code, k.h if k else 0)
-            if kept:
-                kept.release()
-            if given:
-                given.release()
+            args = (wv._ptr, xv._ptr, z._ptr, gptr, gpptr, mptr, ypptr, dx._ptr if need_dx else 0, dw._ptr, db._ptr,
+                    N, C, H, Wd, F, KH, KW, sh, sw, ph, pw, code, k.h if k else 0)
+            if _KEEPS:
+                sc.conv2d_act_bwd_k(*args, kept_w.h if kept_w else 0)
+            else:
+                sc.conv2d_act_bwd(*args)
+            for k in (kept, kept_w, given):
+                if k:
+                    k.release()
             self._deliver(x, W, b, dx, dw, db)
-        self.outputs = self._output(x, z, backward, takes_pooled=True)
-        return self.outputs
+        self.outputs = out = self._output(x, z, backward, takes_pooled=True)
+        if hy:
+            out._copies = _KeptCopies(hy)
+        return out
 
     def __repr__(self):
         return f"Conv2D({self.in_channels}→{self.out_channels}, kernel={self.kernel_size}, act={self.layeract})"
@@ -576,6 +593,8 @@ class ConvTranspose2D(_ParamLayer):
     def __call__(self, input_layer):
         super().__call__(input_layer)
         input_layer._feeds_convT = True       # an unpooling producer then leaves its output to be read at the low resolution
+        if self.out_channels * self.kernel_size[0] * self.kernel_size[1] > 64:        # shorter patches read their input in place
+            input_layer._feeds_copies = True
         return self
 
     def forward(self):
@@ -595,8 +614,27 @@ class ConvTranspose2D(_ParamLayer):
         if (xv.__class__ is _Unpooled and xv._ptr is None and H % 2 == 0 and Wd % 2 == 0
                 and sc.unpool2_convT_fusable(N, Cin, H // 2, Wd // 2, Cout, KH, KW, sh, sw, ph, pw)):
             return self._forward_unpooled(x, xv.low, z, code)
-        sc.conv2DTranspose_bias_act_fwd(xv.main_ptr, wv.main_ptr, b.value.main_ptr, z._ptr, N, Cin, H, Wd, Cout, KH, KW, sh, sw, ph, pw, code)
         need_dx = not x.is_leaf
+        if _KEEPS:
+            given = x._copies
+            h = sc.conv2DTranspose_bias_act_fwd_k(xv.main_ptr, wv.main_ptr, b.value.main_ptr, z._ptr, N, Cin, H, Wd, Cout, KH, KW, sh, sw, ph, pw,
+                                                  code, given.h if given else 0)
+            kept = _KeptCopies(h) if h else None
+
+            def backward(g):
+                # activation slope, bias gradient and both products in one call
+                db, dw = b._grad_target(), W._grad_target()
+                dx = _new(shape) if need_dx else None
+                k = kept or given
+                sc.conv2DTranspose_act_bwd_k(wv._ptr, xv._ptr, z._ptr, g.main_ptr, dx._ptr if need_dx else 0, dw._ptr, db._ptr, N, Cin, H, Wd, Cout,
+                                             KH, KW, sh, sw, ph, pw, code, k.h if k else 0)
+                for k in (kept, given):
+                    if k:
+                        k.release()
+                self._deliver(x, W, b, dx, dw, db)
+            self.outputs = self._output(x, z, backward)
+            return self.outputs
+        sc.conv2DTranspose_bias_act_fwd(xv.main_ptr, wv.main_ptr, b.value.main_ptr, z._ptr, N, Cin, H, Wd, Cout, KH, KW, sh, sw, ph, pw, code)
 
         def backward(g):
             db, dw = b._grad_target(), W._grad_target()
