@@ -301,9 +301,16 @@ __global__ void __launch_bounds__(256, 2) conv3x3_pool_kernel(const float *__res
                                                            int F, int OH, int OW, int ph, int pw, int act, FastDiv by_Pq,
                                                            FastDiv by_OWq, FastDiv by_groups, PoolBand band) {
     extern __shared__ __align__(16) float wk[];           // [C][9][F], [F] biases, then the bands
-    for (int e = threadIdx.x; e < C * 9 * F; e += blockDim.x) {
-        const int f = e % F, k = e / F;                   // k = c * 9 + t
-        wk[e] = __ldg(Wt + (long long)f * C * 9 + k);
+    for (int e0 = threadIdx.x; e0 < C * 9 * F; e0 += 8 * 256) {      // eight in flight: one at a time, this was a quarter of a small launch
+        float w[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const int e = e0 + j * 256, k = e / F, f = e - k * F;    // k = c * 9 + t
+            w[j] = e < C * 9 * F ? __ldg(Wt + f * C * 9 + k) : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+            if (e0 + j * 256 < C * 9 * F) wk[e0 + j * 256] = w[j];
     }
     for (int e = threadIdx.x; e < F; e += blockDim.x) wk[C * 9 * F + e] = bias ? __ldg(bias + e) : 0.f;
     float *bands = wk + (C * 9 + 1) * F;
@@ -441,14 +448,15 @@ __global__ void __launch_bounds__(256, 2) conv3x3_pool_kernel(const float *__res
 
 bool conv_pool_simt_applies(int NB, int C, int H, int W, int F, int R, int S, int sh, int sw, int ph, int pw) {
     const int OH = H + 2 * ph - 2, OW = W + 2 * pw - 2;
-    return R == 3 && S == 3 && sh == 1 && sw == 1 && C >= 1 && C <= 7 && (F & 7) == 0 && F <= 512 && OH >= 2 && OW >= 2 && !(OH & 1) && !(OW & 1) &&
+    return R == 3 && S == 3 && sh == 1 && sw == 1 && C >= 1 && (C <= 7 || conv_small_applies(NB, C, H, W, F, R, S, sh, sw, ph, pw)) && (F & 7) == 0 && F <= 512 && OH >= 2 && OW >= 2 && !(OH & 1) && !(OW & 1) &&
            (long long)NB * OH * OW < (1ll << 31) && (size_t)(C * 9 + 1) * F * sizeof(float) <= 40 * 1024;
 }
 
 int conv_pool_simt(const float *X, const float *Wt, const float *bias, const PoolOut &pool, int NB, int C, int H, int W, int F, int ph, int pw,
                    int act, const char *name) {
     const int OH = H + 2 * ph - 2, OW = W + 2 * pw - 2, Pq = (OH / 2) * (OW / 2);
-    const bool wide = (F & 15) == 0;
+    // (16 filters per warp unless the layer is so small that the warps would not go round the schedulers)
+    const bool wide = (F & 15) == 0 && ((long long)NB * Pq + 31) / 32 * (F / 16) >= 4ll * rt().sm_count;
     const int groups = F / (wide ? 16 : 8);
     if (((long long)NB * Pq + 31) / 32 * groups > 0x7fffffff) return fail(SEERA_E_LIMIT, "%s: too many windows", name);
     // Bands: as many window rows as fit 16 KB, at least one; two buffers while they leave room for two blocks on an SM, one up to

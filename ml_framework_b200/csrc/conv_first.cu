@@ -262,14 +262,15 @@ __global__ void __launch_bounds__(256) conv_first_wgrad_kernel(const float *__re
 // dW[f][k] = sum over blocks of partial[chunk][block][f - f0][k].  A block of 8 warps owns 32 outputs (one per lane);
 // warp w adds blocks w, w + 8, ... in order and the eight sums meet in shared memory in warp order: a fixed order.
 __global__ void __launch_bounds__(1024) conv_first_wgrad_reduce_kernel(const float *__restrict__ partial, float *__restrict__ dW,
-                                                                       float *__restrict__ dbias, int F, int K, int KP, int nblocks) {
+                                                                       float *__restrict__ dbias, int F, int K, int Kg, int KP, int nblocks) {
     __shared__ float part[32][33];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const int e = blockIdx.x * 32 + lane;                  // index into the padded [F rounded to 64][KP] grid
     const int f = e / KP, k = e - f * KP;
     const int chunk = f / FIRST_FC, fl = f - chunk * FIRST_FC;
-    const bool wanted = f < F && (k < K || (dbias && k == K));
-    const float *p = partial + (long long)chunk * nblocks * (FIRST_FC * KP) + fl * KP + k;
+    const int k0 = blockIdx.y * Kg;                        // the group's first column of dW
+    const bool tap = k < Kg && k0 + k < K, wanted = f < F && (tap || (dbias && k == Kg && blockIdx.y == 0));
+    const float *p = partial + ((long long)blockIdx.y * ((F + FIRST_FC - 1) / FIRST_FC) + chunk) * nblocks * (FIRST_FC * KP) + fl * KP + k;
     float s = 0.f;
     if (wanted)
         for (int b = warp; b < nblocks; b += 8 * warps) {
@@ -284,7 +285,7 @@ __global__ void __launch_bounds__(1024) conv_first_wgrad_reduce_kernel(const flo
     if (warp == 0 && wanted) {
         float t = part[0][lane];
         for (int w = 1; w < warps; w++) t += part[w][lane];
-        if (k < K) dW[(long long)f * K + k] = t;
+        if (tap) dW[(long long)f * K + k0 + k] = t;
         else dbias[f] = t;                       // the column of ones: sum of the output gradient per filter
     }
 }
@@ -750,9 +751,10 @@ first_tc_wgrad_kernel(const float *__restrict__ X, DzSource src, float *__restri
     if (warp == MMA_WARP) tmem_dealloc(tmem_base, 64);
 }
 
-void first_wgrad_reduce(const float *partial, float *dW, float *dbias, int F, int K, int KP, int nblocks, cudaStream_t st) {
-    conv_first_wgrad_reduce_kernel<<<(F + FIRST_FC - 1) / FIRST_FC * FIRST_FC * KP / 32, nblocks <= 64 ? 256 : (nblocks <= 128 ? 512 : 1024), 0, st>>>(
-        partial, dW, dbias, F, K, KP, nblocks);
+void first_wgrad_reduce(const float *partial, float *dW, float *dbias, int F, int K, int Kg, int KP, int nblocks, cudaStream_t st) {
+    const dim3 grid((unsigned)((F + FIRST_FC - 1) / FIRST_FC * FIRST_FC * KP / 32), (unsigned)((K + Kg - 1) / Kg));
+    conv_first_wgrad_reduce_kernel<<<grid, nblocks <= 64 ? 256 : (nblocks <= 128 ? 512 : 1024), 0, st>>>(
+        partial, dW, dbias, F, K, Kg, KP, nblocks);
     count_launch();
 }
 
@@ -828,7 +830,7 @@ static int first_tc_wgrad(const float *X, const DzSource &src, float *dW, float 
     count_launch();
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e == cudaSuccess) {
-        first_wgrad_reduce(partial, dW, dbias, g.F, g.K, 64, nblocks, st);
+        first_wgrad_reduce(partial, dW, dbias, g.F, g.K, g.K, 64, nblocks, st);
         e = cudaGetLastError();
     }
     profile_end(2.0 * pixels * (double)g.F * g.K, name);
@@ -849,14 +851,11 @@ bool conv_first_applies(int C, int R, int S) { return C * R * S <= 64; }
 // The forward with the 2x2 max-pool of its output folded into the epilogue (tensor-core variant only).
 bool conv_first_pool_ok(int NB, int C, int H, int W, int F, int R, int S, int sh, int sw, int ph, int pw) {
     FirstGeom g;
-    if (conv_pool_simt_applies(NB, C, H, W, F, R, S, sh, sw, ph, pw)) return true;
     return first_geom(g, NB, C, H, W, F, R, S, sh, sw, ph, pw) && first_tc_fwd_ok(g) && g.OH >= 2 && g.OW >= 2 && !(g.OH & 1) && !(g.OW & 1);
 }
 int conv_first_pool_fwd(const float *X, const float *Wt, const float *bias, const PoolOut &pool, int NB, int C, int H, int W, int F, int R,
                         int S, int ph, int pw, int sh, int sw, int act, const char *name) {
     if (!conv_first_pool_ok(NB, C, H, W, F, R, S, sh, sw, ph, pw)) return fail(SEERA_E_LIMIT, "%s: shape outside the fused pool path", name);
-    if (conv_pool_simt_applies(NB, C, H, W, F, R, S, sh, sw, ph, pw))       // 3 x 3, unit stride: fp32 stencil with the pool folded in
-        return conv_pool_simt(X, Wt, bias, pool, NB, C, H, W, F, ph, pw, act, name);
     FirstGeom g;
     first_geom(g, NB, C, H, W, F, R, S, sh, sw, ph, pw);
     return first_tc_fwd(X, Wt, bias, nullptr, g, act, name, &pool);
@@ -929,7 +928,7 @@ static int first_wgrad_run(const float *X, const DzSource &src, float *dW, float
     count_launch();
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) {
-        first_wgrad_reduce(partial, dW, dbias, g.F, g.K, KP, nblocks, st);
+        first_wgrad_reduce(partial, dW, dbias, g.F, g.K, g.K, KP, nblocks, st);
         e = cudaGetLastError();
     }
     profile_end(2.0 * pixels * (double)g.F * g.K, name);

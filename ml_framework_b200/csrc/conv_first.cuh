@@ -35,7 +35,7 @@ constexpr int FIRST_FC = 64;        // filters per block pass
 // dW (and dbias, if not null) of a 3 x 3 layer on CUDA cores in exact fp32 (conv_first_dw.cu)
 bool first_dw_applies(const FirstGeom &g, const DzSource &src);
 int first_dw(const float *X, const DzSource &src, float *dW, float *dbias, const FirstGeom &g, const char *name);
-// Adds the blocks' partial sums [chunk of 64 filters][block][64][KP] in block order; column K holds the bias gradient.
-void first_wgrad_reduce(const float *partial, float *dW, float *dbias, int F, int K, int KP, int nblocks, cudaStream_t st);
+// Adds the blocks' partial sums [group of Kg taps][chunk of 64 filters][block][64][KP] in block order; column Kg holds the bias gradient.
+void first_wgrad_reduce(const float *partial, float *dW, float *dbias, int F, int K, int Kg, int KP, int nblocks, cudaStream_t st);
 
 }  // namespace seera

@@ -1,5 +1,5 @@
 // Weight and bias gradient of a 3 x 3 convolution with one to four input channels (the first layer of an image network, the last
-// of an autoencoder), exact fp32 on the CUDA cores.
+// of an autoencoder), exact fp32 on the CUDA cores; a layer of little work with more channels goes in groups of four (conv_small.cu).
 //
 // The gradient arrives through a 2x2 / stride-2 max-pool (pooled gradient, argmax index, pooled output) or at full resolution (with
 // the layer output); activation slope and pool routing are applied on the way in.  A UNIT is a 2 x 2 block of output pixels with the
@@ -53,10 +53,12 @@ struct DwShape {
 template <int C, int ST, int FL, bool POOLED>
 __global__ void __launch_bounds__(256, 2) first_dw_kernel(const float *__restrict__ X, DzSource src, float *__restrict__ partial, FirstGeom g,
                                                           int units, int ntiles, int stages, int vf, FastDiv by_units, FastDiv by_cols) {
+    // blockIdx.z: group of C of the g.C input channels
     using Sh = DwShape<C, ST, FL, POOLED>;
     constexpr int KP = Sh::KP, K = Sh::K, VROW = Sh::VROW, ROWS = Sh::ROWS, COLS = Sh::COLS, SUB = 32 / FL;
     extern __shared__ __align__(16) float sm[];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int c_first = blockIdx.z * C, c_here = min(C, g.C - c_first);
     const int f0 = blockIdx.y * FIRST_FC, FC = min(vf, g.F - f0), STAGE = Sh::stage(vf);
     const int plane = g.H * g.W, P = g.OH * g.OW, Pq = P >> 2, ucols = by_cols.d;
     const bool sloped = src.act != SEERA_ACT_NONE;
@@ -73,7 +75,7 @@ __global__ void __launch_bounds__(256, 2) first_dw_kernel(const float *__restric
         const bool live = u < units;
         const int ul = live ? u : 0, n = by_units.div(ul), rem = ul - n * by_units.d, ur = by_cols.div(rem), uc = rem - ur * ucols;
         const int oh = 2 * ur, ow = 2 * uc, ih0 = oh * ST - g.ph, iw0 = ow * ST - g.pw;
-        const float *xn = X + (long long)n * C * plane;
+        const float *xn = X + ((long long)n * g.C + c_first) * plane;
         float *stage = sm + s * STAGE;
         const uint32_t d0 = (uint32_t)__cvta_generic_to_shared(stage + (lane >> 1) * Sh::PAIR + (lane & 1));
         bool colok[3 + ST];
@@ -83,7 +85,7 @@ __global__ void __launch_bounds__(256, 2) first_dw_kernel(const float *__restric
         for (int r0 = 0; r0 < C * ROWS; r0 += 8) {
             const int rr = r0 + warp, c = rr / ROWS, i = rr - c * ROWS;
             if (rr < C * ROWS) {
-                const bool rowok = live && (unsigned)(ih0 + i) < (unsigned)g.H;
+                const bool rowok = live && c < c_here && (unsigned)(ih0 + i) < (unsigned)g.H;
                 const int off = c * plane + (ih0 + i) * g.W + iw0;
 #pragma unroll
                 for (int j = 0; j < 3 + ST; j++) {
@@ -244,7 +246,7 @@ __global__ void __launch_bounds__(256, 2) first_dw_kernel(const float *__restric
         red[k * 32 + lane] = lo;                   // [column][lane]
     }
     __syncthreads();
-    float *out = partial + ((long long)blockIdx.y * gridDim.x + blockIdx.x) * (FIRST_FC * KP);
+    float *out = partial + (((long long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x) * (FIRST_FC * KP);
     for (int e = t; e < FC * KP; e += 256) {
         const int f = e / KP, k = e - f * KP;
         float s = 0.f;
@@ -278,23 +280,24 @@ static int dw_launch(const DwCall &a) {
     if (stages < 2) stages = 2;
     const size_t smem = stages * stage_bytes > red_bytes ? stages * stage_bytes : red_bytes;
     const int per_sm = smem <= 112 * 1024 ? 2 : 1;
-    int nblocks = rt().sm_count * per_sm / chunks;
+    const int cgroups = (g.C + C - 1) / C;
+    int nblocks = rt().sm_count * per_sm / (chunks * cgroups);
     if (nblocks > (ntiles + 1) / 2) nblocks = (ntiles + 1) / 2;      // a block with one tile is all start and end
     if (nblocks < 1) nblocks = 1;
-    float *partial = (float *)scratch_alloc((size_t)chunks * nblocks * FIRST_FC * Sh::KP * sizeof(float));
+    float *partial = (float *)scratch_alloc((size_t)cgroups * chunks * nblocks * FIRST_FC * Sh::KP * sizeof(float));
     if (!partial) return SEERA_E_OOM;
     cudaStream_t st = rt().stream;
     profile_begin();
     auto kern = first_dw_kernel<C, ST, FL, POOLED>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess) {
-        kern<<<dim3((unsigned)nblocks, (unsigned)chunks), 256, smem, st>>>(a.X, *a.src, partial, g, units, ntiles, stages, vf, fast_div(per_image),
+        kern<<<dim3((unsigned)nblocks, (unsigned)chunks, (unsigned)cgroups), 256, smem, st>>>(a.X, *a.src, partial, g, units, ntiles, stages, vf, fast_div(per_image),
                                                                          fast_div(ucols));
         count_launch();
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) {
-        first_wgrad_reduce(partial, a.dW, a.dbias, g.F, g.K, Sh::KP, nblocks, st);
+        first_wgrad_reduce(partial, a.dW, a.dbias, g.F, g.K, Sh::K, Sh::KP, nblocks, st);
         e = cudaGetLastError();
     }
     profile_end(2.0 * g.NB * g.OH * g.OW * (double)g.F * g.K, a.name);
@@ -310,7 +313,7 @@ static int dw_pick(const DwCall &a) {
 
 int first_dw(const float *X, const DzSource &src, float *dW, float *dbias, const FirstGeom &g, const char *name) {
     const DwCall a{X, &src, dW, dbias, &g, name};
-    if (g.sh == 1) return g.C == 1 ? dw_pick<1, 1>(a) : g.C == 2 ? dw_pick<2, 1>(a) : g.C == 3 ? dw_pick<3, 1>(a) : dw_pick<4, 1>(a);
+    if (g.sh == 1) return g.C == 1 ? dw_pick<1, 1>(a) : g.C == 2 ? dw_pick<2, 1>(a) : g.C == 3 ? dw_pick<3, 1>(a) : dw_pick<4, 1>(a);        // more in groups of four
     return g.C == 1 ? dw_pick<1, 2>(a) : g.C == 2 ? dw_pick<2, 2>(a) : g.C == 3 ? dw_pick<3, 2>(a) : dw_pick<4, 2>(a);
 }
 

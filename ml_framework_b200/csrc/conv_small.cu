@@ -1,0 +1,244 @@
+// 3 x 3 unit-stride convolutions of little work (a few tens of million multiply-adds: the inner layers of a small network, or of any
+// network at a small batch), exact fp32 on the CUDA cores.
+//
+// On the tensor-core path such a layer is all start-up: its filters are converted by one launch, the GEMM walks nine k-steps of 64
+// channels of which it has eight or sixteen, and its gradient needs channels-last copies first - 12 us forward and 29 us backward for
+// work of a microsecond (8 -> 16 channels, 64 images of 14 x 14; here 5 and 16 us).  Here a block takes a band of one image, stages it
+// with its border of zeros, the filters as [input channel][tap][output channel], and a warp forms 32 blocks of 2 x 2 outputs for FW output channels:
+// per input channel 8 reads of its own 4 x 4 patch and 9 broadcasts of FW weights for 36 FW / 2 packed multiply-adds.  The data
+// gradient is the same convolution of dz with the taps reversed; dz - activation slope, and the routing through a 2x2 max-pool - is
+// formed while the band is staged.  The weight gradient goes to first_dw in groups of four input channels, and a layer with its pool to
+// conv_pool_simt.
+#include "conv_first.cuh"
+#include "internal.h"
+
+namespace seera {
+
+// Where the lines lie, forward with pool + backward, microseconds against the tensor-core path in fp16x3 / bf16x6 (which pads the
+// channels of both operands to 64, so that its cost does not fall with C * F): 8 -> 16 channels 19 against 38 / 44 at 2 million
+// multiply-adds, 38 against 101 / 132 at 64, 64 against 168 / 233 at 128; 16 -> 32 channels 34 against 35 / 43 at 2, 35 against 39 / 46
+// at 32, 45 against 43 / 52 at 64; 32 -> 32 channels 42 against 33 / 40 at 2.
+bool conv_small_applies(int NB, int C, int H, int W, int F, int R, int S, int sh, int sw, int ph, int pw) {
+    // not in the modes of a single rounded product, whose results are those of rounded operands
+    if (rt().precision < 2 || rt().precision > 4 || !rt().conv_tma) return false;
+    if (R != 3 || S != 3 || sh != 1 || sw != 1 || ph < 0 || pw < 0 || ph > 2 || pw > 2 || NB < 1 || C * 9 <= 64 || C > 64 || F < 1 || F > 64 || C * F > 512)
+        return false;
+    const long long OH = (long long)H + 2 * ph - 2, OW = (long long)W + 2 * pw - 2, h = OH > H ? OH : H, w = OW > W ? OW : W;
+    if (OH < 1 || OW < 1 || w * (C > F ? C : F) > 6144) return false;        // four rows of every channel fit a block's shared memory
+    return NB * h * w < (1ll << 26) && NB * h * w * 9 * (C * F) * (C * F) <= 1ll << 35;
+}
+
+// What a band is made from: a tensor, its product with the slope of the activation whose output is y, or a pooled gradient.
+struct SmallSource {
+    const float *v, *y;        // y null: no slope
+    const int *mask;           // v (and y) of a 2x2 / stride-2 max-pool; null: full resolution
+    int act;
+};
+struct SmallGeom {
+    int I, IH, IW, O, OH, OW, ph, pw;        // input / output channels and planes, lower padding
+    int window_rows, per_image, rows, pitch, OP, groups;
+    FastDiv by_bands, by_pitch, by_rows, by_cols, by_groups;
+};
+
+template <int FW>
+__global__ void __launch_bounds__(256) conv3x3_small_kernel(SmallSource src, const float *__restrict__ Wt, const float *__restrict__ bias,
+                                                            float *__restrict__ Y, SmallGeom g, int total, int reversed, int act) {
+    extern __shared__ __align__(16) float sm[];          // [I][9][OP] weights, [OP] biases, [8][4 FW][32] sums, [I][rows][pitch] band
+    float *bk = sm + g.I * 9 * g.OP, *red = bk + g.OP, *band = red + 8 * 4 * FW * 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = g.I * 9 * g.OP;
+    // Wt[o][i][t], or for the data gradient Wt[i][o][8 - t]
+    for (int e0 = threadIdx.x; e0 < nw; e0 += 8 * 256) {
+        float w[8];
+#pragma unroll
+        for (int j = 0; j < 8; j++) {
+            const int e = e0 + j * 256, k = e / g.OP, o = e - k * g.OP, i = k / 9, t = k - i * 9;
+            w[j] = e < nw && o < g.O ? __ldg(Wt + (reversed ? ((long long)i * g.O + o) * 9 + 8 - t : ((long long)o * g.I + i) * 9 + t)) : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < 8; j++)
+            if (e0 + j * 256 < nw) sm[e0 + j * 256] = w[j];
+    }
+    for (int e = threadIdx.x; e < g.OP; e += 256) bk[e] = bias && e < g.O ? __ldg(bias + e) : 0.f;
+    const int bplane = g.rows * g.pitch, bsize = g.I * bplane, cols = (g.OW + 1) >> 1;
+    const long long iplane = (long long)g.IH * g.IW, oplane = (long long)g.OH * g.OW;
+    const bool pairs = (g.OW & 1) == 0 && (reinterpret_cast<uintptr_t>(Y) & 7) == 0;
+
+    for (int id = blockIdx.x; id < total; id += gridDim.x) {
+        const int n = g.by_bands.div(id), q0 = (id - n * g.per_image) * g.window_rows, ih0 = 2 * q0 - g.ph;
+        if (src.mask) {                                   // every pixel from its window's gradient, index and output
+            const int Wq = g.IW >> 1;
+            const long long qplane = iplane >> 2, base = (long long)n * g.I * qplane;
+            for (int e0 = threadIdx.x; e0 < bsize; e0 += 8 * 256) {
+                float v[8], y[8];
+                int m[8], pos[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const int e = e0 + j * 256, rr = g.by_pitch.div(e), x = e - rr * g.pitch, i = g.by_rows.div(rr);
+                    const int ih = ih0 + rr - i * g.rows, iw = x - g.pw;
+                    const bool in = e < bsize && (unsigned)ih < (unsigned)g.IH && (unsigned)iw < (unsigned)g.IW;
+                    const long long o = in ? base + i * qplane + (long long)(ih >> 1) * Wq + (iw >> 1) : 0;
+                    pos[j] = in ? ((ih & 1) << 1) | (iw & 1) : -1;
+                    v[j] = __ldg(src.v + o); m[j] = __ldg(src.mask + o); y[j] = src.y ? __ldg(src.y + o) : 0.f;
+                }
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    if (e0 + j * 256 < bsize)
+                        band[e0 + j * 256] = m[j] == pos[j] ? v[j] * (src.y ? first_slope(y[j], src.act) : 1.f) : 0.f;
+            }
+        } else {
+            const long long base = (long long)n * g.I * iplane;
+            for (int e0 = threadIdx.x; e0 < bsize; e0 += 8 * 256) {
+                float v[8], y[8];
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const int e = e0 + j * 256, rr = g.by_pitch.div(e), x = e - rr * g.pitch, i = g.by_rows.div(rr);
+                    const int ih = ih0 + rr - i * g.rows, iw = x - g.pw;
+                    const bool in = e < bsize && (unsigned)ih < (unsigned)g.IH && (unsigned)iw < (unsigned)g.IW;
+                    const long long o = base + i * iplane + (long long)ih * g.IW + iw;
+                    v[j] = in ? __ldg(src.v + o) : 0.f;
+                    y[j] = in && src.y ? __ldg(src.y + o) : 0.f;
+                }
+#pragma unroll
+                for (int j = 0; j < 8; j++)
+                    if (e0 + j * 256 < bsize) band[e0 + j * 256] = src.y ? v[j] * first_slope(y[j], src.act) : v[j];
+            }
+        }
+        __syncthreads();
+        const int windows = min(g.window_rows, ((g.OH + 1) >> 1) - q0) * cols, items = ((windows + 31) >> 5) * g.groups;
+        // at most half as many items as warps: several warps share an item, each with its part of the input
+        // channels (not in the forward, which gives the same bits as conv_pool_simt)
+        const int lg = items > 4 || !reversed ? 0 : (items > 2 ? 1 : (items > 1 ? 2 : 3)), part = warp & ((1 << lg) - 1), ipart = (g.I + (1 << lg) - 1) >> lg;
+        const int i0 = part * ipart, i1 = min(g.I, i0 + ipart);
+        for (int base = 0; base < items; base += 8 >> lg) {
+            const int at = base + (warp >> lg), item = min(at, items - 1);
+            const bool mine = at < items;
+            const int tile = g.by_groups.div(item), o0 = (item - tile * g.groups) * FW;
+            const int w = tile * 32 + lane, wl = min(w, windows - 1), qr = g.by_cols.div(wl), qc = wl - qr * cols;
+            const float *patch = band + i0 * bplane + 2 * qr * g.pitch + 2 * qc, *wc = sm + i0 * 9 * g.OP + o0;
+            f32x2 acc[4][FW / 2];                         // [pixel of the 2 x 2 block][pair of output channels]
+#pragma unroll
+            for (int p = 0; p < 4; p++)
+#pragma unroll
+                for (int f = 0; f < FW / 2; f++) acc[p][f] = 0ull;
+            for (int i = i0; i < i1; i++, wc += 9 * g.OP, patch += bplane) {
+                f32x2 v[4][4];
+#pragma unroll
+                for (int r = 0; r < 4; r++) {
+                    const float2 u = *reinterpret_cast<const float2 *>(patch + r * g.pitch), t = *reinterpret_cast<const float2 *>(patch + r * g.pitch + 2);
+                    v[r][0] = pack2(u.x, u.x); v[r][1] = pack2(u.y, u.y); v[r][2] = pack2(t.x, t.x); v[r][3] = pack2(t.y, t.y);
+                }
+#pragma unroll
+                for (int t = 0; t < 9; t++)
+#pragma unroll
+                    for (int f = 0; f < FW / 4; f++) {
+                        const ulonglong2 w2 = *reinterpret_cast<const ulonglong2 *>(wc + t * g.OP + 4 * f);
+#pragma unroll
+                        for (int p = 0; p < 4; p++) {
+                            acc[p][2 * f] = ffma2(v[(p >> 1) + t / 3][(p & 1) + t % 3], w2.x, acc[p][2 * f]);
+                            acc[p][2 * f + 1] = ffma2(v[(p >> 1) + t / 3][(p & 1) + t % 3], w2.y, acc[p][2 * f + 1]);
+                        }
+                    }
+            }
+            if (lg) {                                     // the parts are added in order
+                float *mine_at = red + warp * (4 * FW * 32) + lane;
+                if (part)
+#pragma unroll
+                    for (int k = 0; k < 2 * FW; k++) {
+                        float lo, hi;
+                        unpack2(acc[k / (FW / 2)][k % (FW / 2)], lo, hi);
+                        mine_at[(2 * k) * 32] = lo; mine_at[(2 * k + 1) * 32] = hi;
+                    }
+                __syncthreads();
+                if (!part)
+                    for (int q = 1; q < 1 << lg; q++)
+#pragma unroll
+                        for (int k = 0; k < 2 * FW; k++) {
+                            const float *o = mine_at + q * (4 * FW * 32) + 2 * k * 32;
+                            acc[k / (FW / 2)][k % (FW / 2)] = add2(acc[k / (FW / 2)][k % (FW / 2)], pack2(o[0], o[32]));
+                        }
+            }
+            if (w < windows && mine && !part) {
+                const int oh = 2 * (q0 + qr), ow = 2 * qc;
+                float *yo = Y + ((long long)n * g.O + o0) * oplane + (long long)oh * g.OW + ow;
+#pragma unroll
+                for (int f = 0; f < FW; f++, yo += oplane) {
+                    if (o0 + f >= g.O) break;
+                    float z[4];
+#pragma unroll
+                    for (int p = 0; p < 4; p++) {
+                        float lo, hi;
+                        unpack2(acc[p][f >> 1], lo, hi);
+                        z[p] = epilogue_act(((f & 1) ? hi : lo) + bk[o0 + f], act);
+                    }
+                    if (pairs) {
+                        *reinterpret_cast<float2 *>(yo) = make_float2(z[0], z[1]);
+                        if (oh + 1 < g.OH) *reinterpret_cast<float2 *>(yo + g.OW) = make_float2(z[2], z[3]);
+                    } else {
+                        yo[0] = z[0];
+                        if (ow + 1 < g.OW) yo[1] = z[1];
+                        if (oh + 1 < g.OH) { yo[g.OW] = z[2]; if (ow + 1 < g.OW) yo[g.OW + 1] = z[3]; }
+                    }
+                }
+            }
+        }
+        __syncthreads();                                  // the band has been read
+    }
+}
+
+static int small_run(const SmallSource &src, const float *Wt, const float *bias, float *Y, int NB, int I, int IH, int IW, int O, int OH, int OW,
+                     int ph, int pw, int reversed, int act, const char *name) {
+    SmallGeom g{};
+    g.I = I; g.IH = IH; g.IW = IW; g.O = O; g.OH = OH; g.OW = OW; g.ph = ph; g.pw = pw;
+    const int wrows = (OH + 1) / 2, cols = (OW + 1) / 2;
+    // four output channels per warp: a small layer has too few 32-window tiles to fill the chip with more
+    constexpr int FW = 4;
+    g.OP = (O + FW - 1) / FW * FW; g.groups = g.OP / FW;
+    g.pitch = 2 * cols + 2;
+    // bands of as many window rows as fit 24 KB (at least one), fewer while the blocks would not go round the SMs
+    const size_t row = (size_t)I * g.pitch * sizeof(float);
+    int wr = 24 * 1024 > 4 * row ? (int)((24 * 1024 / row - 2) / 2) : 1;
+    if (wr > wrows) wr = wrows;
+    while (wr > 1 && (long long)NB * ((wrows + wr - 1) / wr) < rt().sm_count) wr = (wr + 1) / 2;
+    g.window_rows = wr; g.rows = 2 * wr + 2; g.per_image = (wrows + wr - 1) / wr;
+    g.by_bands = fast_div(g.per_image); g.by_pitch = fast_div(g.pitch); g.by_rows = fast_div(g.rows);
+    g.by_cols = fast_div(cols); g.by_groups = fast_div(g.groups);
+    const size_t smem = ((size_t)(I * 9 + 1) * g.OP + 8 * 4 * FW * 32) * sizeof(float) + g.rows * row;
+    const int total = NB * g.per_image;
+    int grid = rt().sm_count * 4;
+    if (grid > total) grid = total;
+    profile_begin();
+    cudaError_t e = cudaSuccess;
+    if (smem > 48 * 1024) e = cudaFuncSetAttribute(conv3x3_small_kernel<FW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess) {
+        conv3x3_small_kernel<FW><<<grid, 256, smem, rt().stream>>>(src, Wt, bias, Y, g, total, reversed, act);
+        count_launch();
+        e = cudaGetLastError();
+    }
+    profile_end(2.0 * NB * OH * OW * (double)O * I * 9, name);
+    return e == cudaSuccess ? SEERA_OK : check_cuda(e, name);
+}
+
+int conv_small_fwd(const float *X, const float *Wt, const float *bias, float *Y, int NB, int C, int H, int W, int F, int ph, int pw, int act,
+                   const char *name) {
+    return small_run(SmallSource{X, nullptr, nullptr, 0}, Wt, bias, Y, NB, C, H, W, F, H + 2 * ph - 2, W + 2 * pw - 2, ph, pw, 0, act, name);
+}
+bool conv_small_bwd_applies(const float *y, const float *gp, const float *y_pooled, int act) {
+    return !gp || act == SEERA_ACT_NONE || y_pooled;       // with the layer output alone a pooled gradient's slope would need a gather
+}
+int conv_small_bwd(const float *Wt, const float *X, const float *y, const float *g, const float *gp, const int *mask, const float *y_pooled,
+                   float *dX, float *dW, float *dbias, int NB, int C, int H, int W, int F, int ph, int pw, int act, const char *name) {
+    const int OH = H + 2 * ph - 2, OW = W + 2 * pw - 2;
+    const bool sloped = act != SEERA_ACT_NONE;
+    int s = SEERA_OK;
+    if (dX) {
+        const SmallSource src{gp ? gp : g, sloped ? (gp ? y_pooled : y) : nullptr, gp ? mask : nullptr, act};
+        s = small_run(src, Wt, nullptr, dX, NB, F, OH, OW, C, H, W, 2 - ph, 2 - pw, 1, SEERA_ACT_NONE, name);
+    }
+    if (!s && dW) {
+        FirstGeom geo{NB, C, H, W, F, 3, 3, 1, 1, ph, pw, OH, OW, C * 9};
+        s = first_dw(X, DzSource{nullptr, g, gp, mask, y, act, y_pooled}, dW, dbias, geo, name);
+    }
+    return s;
+}
+
+}  // namespace seera

@@ -762,6 +762,8 @@ static int tma_conv2d_bwd_kept(const float *Wt, const float *X, const float *dY,
                                const seera_rows *wk = nullptr) {
     SEERA_ENSURE();
     if (!conv_ok(NB, C, H, W, F, R, S, sh, sw, ph, pw) || !X || !Wt || (!dY && !dyk)) return fail(SEERA_E_ARG, "cuda_conv2d_bwd: bad argument");
+    if (dY && !dyk && conv_small_applies(NB, C, H, W, F, R, S, sh, sw, ph, pw))
+        return conv_small_bwd(Wt, X, nullptr, dY, nullptr, nullptr, nullptr, dX, dW, nullptr, NB, C, H, W, F, ph, pw, SEERA_ACT_NONE, "cuda_conv2d_bwd");
     int OH = (H + 2 * ph - R) / sh + 1, OW = (W + 2 * pw - S) / sw + 1;
     if (OH < 1 || OW < 1) return fail(SEERA_E_ARG, "cuda_conv2d_bwd: kernel larger than padded input");
     const bool first = conv_first_applies(C, R, S);
@@ -827,6 +829,9 @@ using namespace seera;
 
 static int convT_fwd_kept(const float *X, const float *Wt, const float *bias, float *out, int NB, int Cin, int H, int W, int Cout, int KH,
                           int KW, int sh, int sw, int ph, int pw, int act, const seera_shadow *x_in, seera_shadow **x_keep);
+static int conv_fwd_kept(const float *X, const float *Wt, const float *bias, float *Y, int NB, int C, int H, int W, int F, int R, int S, int ph,
+                         int pw, int sh, int sw, int act, seera_shadow_t *x_in, seera_shadow_t **x_keep, seera_rows_t **w_keep,
+                         seera_shadow_t **y_copies, bool direct);
 
 extern "C" {
 
@@ -846,6 +851,8 @@ int seera_tma_conv2d_bias_act_fwd(const float *X, const float *Wt, const float *
         return conv_first_fwd(X, Wt, bias, Y, NB, C, H, W, F, R, S, ph, pw, sh, sw, act, "cuda_conv2d_fwd");
     if (sh == 1 && sw == 1 && conv_few_applies(NB, C, F, R, S, OH, OW))       // a few filters: a stencil, not a GEMM
         return conv_few_fwd(X, Wt, bias, Y, NB, C, H, W, F, R, S, ph, pw, OH, OW, act, 0, "cuda_conv2d_fwd");
+    if (conv_small_applies(NB, C, H, W, F, R, S, sh, sw, ph, pw))             // little work: start-up would be all of it
+        return conv_small_fwd(X, Wt, bias, Y, NB, C, H, W, F, ph, pw, act, "cuda_conv2d_fwd");
     if (!tma_conv_supported(NB, R, S, sh, sw, ph, pw)) {
         int s = seera_tc_conv2d_fwd(X, Wt, Y, NB, C, H, W, F, R, S, ph, pw, sh, sw);
         if (!s && (bias || act)) s = seera_bias_act_fwd(Y, bias, Y, NB * F * OH * OW, F, OH * OW, act);
@@ -879,12 +886,19 @@ void seera_shadow_free(seera_shadow_t *h) {
 
 int seera_conv2d_bias_act_fwd_s(const float *X, const float *Wt, const float *bias, float *Y, int NB, int C, int H, int W, int F,
                                 int R, int S, int ph, int pw, int sh, int sw, int act, seera_shadow_t *x_in, seera_shadow_t **x_keep) {
-    return seera_conv2d_bias_act_fwd_k(X, Wt, bias, Y, NB, C, H, W, F, R, S, ph, pw, sh, sw, act, x_in, x_keep, nullptr, nullptr);
+    return conv_fwd_kept(X, Wt, bias, Y, NB, C, H, W, F, R, S, ph, pw, sh, sw, act, x_in, x_keep, nullptr, nullptr, false);
 }
 
 int seera_conv2d_bias_act_fwd_k(const float *X, const float *Wt, const float *bias, float *Y, int NB, int C, int H, int W, int F,
                                 int R, int S, int ph, int pw, int sh, int sw, int act, seera_shadow_t *x_in, seera_shadow_t **x_keep,
                                 seera_rows_t **w_keep, seera_shadow_t **y_copies) {
+    return conv_fwd_kept(X, Wt, bias, Y, NB, C, H, W, F, R, S, ph, pw, sh, sw, act, x_in, x_keep, w_keep, y_copies, true);
+}
+}  // extern "C"
+// `direct`: a layer of little work, whose gradients will not read copies either, may do without any
+static int conv_fwd_kept(const float *X, const float *Wt, const float *bias, float *Y, int NB, int C, int H, int W, int F, int R, int S, int ph,
+                         int pw, int sh, int sw, int act, seera_shadow_t *x_in, seera_shadow_t **x_keep, seera_rows_t **w_keep,
+                         seera_shadow_t **y_copies, bool direct) {
     SEERA_ENSURE();
     if (x_keep) *x_keep = nullptr;
     if (w_keep) *w_keep = nullptr;
@@ -906,7 +920,7 @@ int seera_conv2d_bias_act_fwd_k(const float *X, const float *Wt, const float *bi
         else free_nhwc(yc);
         return s;
     };
-    if (!keeps_shadows(NB, C, H, W, F, R, S, sh, sw, ph, pw)) {
+    if (!keeps_shadows(NB, C, H, W, F, R, S, sh, sw, ph, pw) || (direct && conv_small_applies(NB, C, H, W, F, R, S, sh, sw, ph, pw))) {
         if (y_copies && rt().precision && rt().conv_tma && X && Wt && Y && conv_ok(NB, C, H, W, F, R, S, sh, sw, ph, pw) && OH >= 1 && OW >= 1 &&
             conv_first_copies_ok(X, Y, NB, C, H, W, F, R, S, sh, sw, ph, pw)) {
             if (int s = want_copies()) return s;
@@ -936,6 +950,7 @@ int seera_conv2d_bias_act_fwd_k(const float *X, const float *Wt, const float *bi
     }
     return hand_copies(s);
 }
+extern "C" {
 
 int seera_maxpool2x2_fwd_s(const float *X, float *out, int *mask, int N, int C, int H, int W, seera_shadow_t **out_shadow) {
     SEERA_ENSURE();
@@ -973,8 +988,9 @@ int seera_maxpool2x2_fwd_s(const float *X, float *out, int *mask, int N, int C, 
 // In raster row order a 2x2 window must lie inside one epilogue warp's 32 rows: OW a power of two <= 16 and an even OH.
 static bool pool_in_epilogue_ok(int NB, int C, int H, int W, int F, int R, int S, int sh, int sw, int ph, int pw) {
     if (!rt().precision || !rt().conv_tma || !conv_ok(NB, C, H, W, F, R, S, sh, sw, ph, pw)) return false;
-    if (conv_first_applies(C, R, S))       // the fp32 stencil kernel always; the tensor-core short-patch kernel's pooled epilogue only on request
-        return conv_pool_simt_applies(NB, C, H, W, F, R, S, sh, sw, ph, pw) || (rt().pool_short_patch && conv_first_pool_ok(NB, C, H, W, F, R, S, sh, sw, ph, pw));
+    if (conv_pool_simt_applies(NB, C, H, W, F, R, S, sh, sw, ph, pw)) return true;
+    if (conv_first_applies(C, R, S))       // the tensor-core short-patch kernel's pooled epilogue only on request
+        return (rt().pool_short_patch && conv_first_pool_ok(NB, C, H, W, F, R, S, sh, sw, ph, pw));
     if (!tma_conv_supported(NB, R, S, sh, sw, ph, pw)) return false;
     const int OH = (H + 2 * ph - R) / sh + 1, OW = (W + 2 * pw - S) / sw + 1;
     return OH >= 2 && !(OH & 1) && (OW == 2 || OW == 4 || OW == 8 || OW == 16);
@@ -1014,7 +1030,9 @@ int seera_conv2d_bias_act_pool_fwd_k(const float *X, const float *Wt, const floa
         po.ns = ns; po.Cp = pc.Cp; po.enc = pc.enc;
     }
     int s;
-    if (conv_first_applies(C, R, S)) {
+    if (conv_pool_simt_applies(NB, C, H, W, F, R, S, sh, sw, ph, pw)) {
+        s = conv_pool_simt(X, Wt, bias, po, NB, C, H, W, F, ph, pw, act, "conv2d_pool_fwd");
+    } else if (conv_first_applies(C, R, S)) {
         s = conv_first_pool_fwd(X, Wt, bias, po, NB, C, H, W, F, R, S, ph, pw, sh, sw, act, "conv2d_pool_fwd");
     } else {
         NhwcShadow local; Shadow wk;
@@ -1096,6 +1114,8 @@ int seera_conv2d_act_bwd_k(const float *Wt, const float *X, const float *y, cons
     int OH = (H + 2 * ph - R) / sh + 1, OW = (W + 2 * pw - S) / sw + 1;
     if (OH < 1 || OW < 1) return fail(SEERA_E_ARG, "conv2d_act_bwd: kernel larger than padded input");
     if (gp && ((OH & 1) || (OW & 1))) return fail(SEERA_E_ARG, "conv2d_act_bwd: pooled gradient needs even output height and width");
+    if (dW && conv_small_applies(NB, C, H, W, F, R, S, sh, sw, ph, pw) && conv_small_bwd_applies(y, gp, y_pooled, act))
+        return conv_small_bwd(Wt, X, y, g, gp, pool_mask, gp ? y_pooled : nullptr, dX, dW, dbias, NB, C, H, W, F, ph, pw, act, "conv2d_act_bwd");
     const long long out_elems = (long long)NB * F * OH * OW;
     if (keeps_shadows(NB, C, H, W, F, R, S, sh, sw, ph, pw) &&
         (sh == 1 && sw == 1 ? true : phases_supported(H, W, OH, OW, R, S, sh, sw, ph, pw) || !dX)) {

@@ -52,10 +52,18 @@ int skinny_bwd(const float *A, const float *B, const float *dC, float *dA, float
 bool conv_few_applies(int NB, int C, int F, int R, int S, int OH, int OW);
 int conv_few_fwd(const float *X, const float *Wt, const float *bias, float *Y, int NB, int C, int H, int W, int F, int R, int S, int PH,
                  int PW, int OH, int OW, int act, int transposed, const char *name);
-// 3 x 3 unit-stride convolution with at most seven input channels + bias + activation + 2x2 max-pool, direct fp32 (conv_few.cu).
+// 3 x 3 unit-stride convolution of a layer with at most seven input channels or little work + bias + activation + 2x2 max-pool, direct fp32 (conv_few.cu).
 bool conv_pool_simt_applies(int NB, int C, int H, int W, int F, int R, int S, int sh, int sw, int ph, int pw);
 int conv_pool_simt(const float *X, const float *Wt, const float *bias, const PoolOut &pool, int NB, int C, int H, int W, int F, int ph, int pw,
                    int act, const char *name);
+// 3 x 3 unit-stride convolutions of little work, exact fp32 on the CUDA cores (conv_small.cu); bias, y, dX, dW and dbias may be null.
+// The gradient is g at full resolution or gp through a 2x2 max-pool.
+bool conv_small_applies(int NB, int C, int H, int W, int F, int R, int S, int sh, int sw, int ph, int pw);
+int conv_small_fwd(const float *X, const float *Wt, const float *bias, float *Y, int NB, int C, int H, int W, int F, int ph, int pw, int act,
+                   const char *name);
+bool conv_small_bwd_applies(const float *y, const float *gp, const float *y_pooled, int act);
+int conv_small_bwd(const float *Wt, const float *X, const float *y, const float *g, const float *gp, const int *mask, const float *y_pooled,
+                   float *dX, float *dW, float *dbias, int NB, int C, int H, int W, int F, int ph, int pw, int act, const char *name);
 // Forward of a "same" 3 x 3 unit-stride convolution with one input channel, direct fp32 (conv_few.cu); bias may be null.
 bool conv_c1_fwd_applies(const float *X, const float *Y, int NB, int C, int H, int W, int F, int R, int S, int sh, int sw, int ph, int pw);
 int conv_c1_fwd(const float *X, const float *Wt, const float *bias, float *Y, int NB, int H, int W, int F, int ph, int act, const char *name);

@@ -49,11 +49,11 @@ def test_convolution_with_everything_kept(sc, shape, mode, tol):
     y = activated(co.conv2d_forward(x, w, st, st, pad, pad) + b.reshape(1, F, 1, 1), act)
     assert rel_l2(sc.to_host_f32(yd, y.shape), y) < tol
     # the copies of y are what a convolution would have made of y
-    w2 = rs.standard_normal((5, F, 3, 3)).astype(np.float32)
+    w2 = rs.standard_normal((5, F, 5, 5)).astype(np.float32)
     w2d, outs = sc.to_device_f32(w2.ravel()), [sc.cuda_malloc_f32(N * 5 * OH * OW) for _ in range(2)]
     assert hy
     for o, given in zip(outs, (hy, 0)):
-        k = sc.conv2d_bias_act_fwd_s(yd, w2d, 0, o, N, F, OH, OW, 5, 3, 3, 1, 1, 1, 1, 0, given)
+        k = sc.conv2d_bias_act_fwd_s(yd, w2d, 0, o, N, F, OH, OW, 5, 5, 5, 2, 2, 1, 1, 0, given)
         assert bool(k) != bool(given)
         sc.shadow_free(k)
     assert np.array_equal(*(sc.to_host_f32(o, (N, 5, OH, OW)) for o in outs))
