@@ -10,6 +10,8 @@
 //   Adam / SGD              ~30 cuten operator launches per parameter tensor       (Seera.py:1038-1063, :992-1001)
 // Arithmetic follows the CPU engine, the parity oracle (engine/src/activation_ops.cpp:84-115,
 // Seera.py:1069-1084, :1006-1008).
+#include <atomic>
+
 #include "common.cuh"
 
 namespace seera {
@@ -236,7 +238,7 @@ __device__ __forceinline__ void note_largest(float m, float *scale) {
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     if ((threadIdx.x & 31) == 0 && m > 0.f) atomicMax(reinterpret_cast<unsigned *>(scale) + 2, __float_as_uint(m));
 }
-inline int next_finish_counter() { static int k = 0; k = (k + 1) & 63; return k; }
+inline int next_finish_counter() { static std::atomic<unsigned> k{0}; return (int)(++k & 63u); }
 // Where a loss launch in the present precision mode leaves the factor (null: the copies of this mode have none), and the note that
 // it has done so for gradient `dz`.
 inline float *loss_scale(const float *dz, long long n) {
@@ -284,6 +286,69 @@ __global__ void __launch_bounds__(256) softmax_cce_kernel(const float *__restric
             largest = fmaxf(largest, scale_entry(d));
         }
         if (lane == 0) loss_rows[row] = loss;
+    }
+    if (scale) note_largest(largest, scale);
+    if (last_block_done(counter)) finish_loss(loss_rows, N, inv_count, loss_mean, scale, sm);
+}
+// The same with a row's values in the registers of L lanes, V each (C <= L * V): nothing is stored to be read again, and where 16 lanes
+// hold a row a warp takes two.  4096 rows of 10: 8.0 -> 5.8 us.
+template <int L, int V>
+__global__ void __launch_bounds__(256) softmax_cce_row_kernel(const float *__restrict__ z, const float *__restrict__ yhot,
+                                                              float *__restrict__ p, float *__restrict__ loss_rows,
+                                                              float *__restrict__ dz, int N, int C, float eps, float inv_count,
+                                                              float *__restrict__ loss_mean, float *__restrict__ scale, int counter) {
+    __shared__ float sm[8];
+    const int lane = threadIdx.x % L, per_block = 256 / L;
+    const float hi = 1.0f - eps;
+    auto across = [](float v, auto op) {
+#pragma unroll
+        for (int o = L / 2; o > 0; o >>= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, o));
+        return v;
+    };
+    auto add = [](float a, float b) { return a + b; };
+    float largest = 0.f;
+    // rows beyond the last are walked with the others of their warp and write nothing
+    for (int r0 = blockIdx.x * per_block; r0 < N; r0 += gridDim.x * per_block) {
+        const int row = r0 + threadIdx.x / L;
+        const long long at = (long long)row * C;
+        float x[V], y[V], g[V], mx = -INFINITY, sum = 0.f, loss = 0.f, dot = 0.f;
+#pragma unroll
+        for (int j = 0; j < V; j++) {
+            const bool in = row < N && lane + j * L < C;
+            x[j] = in ? __ldg(z + at + lane + j * L) : -INFINITY;
+            y[j] = in ? __ldg(yhot + at + lane + j * L) : 0.f;
+        }
+#pragma unroll
+        for (int j = 0; j < V; j++) mx = fmaxf(mx, x[j]);
+        mx = across(mx, [](float a, float b) { return fmaxf(a, b); });
+#pragma unroll
+        for (int j = 0; j < V; j++) {
+            x[j] = lane + j * L < C ? expf(x[j] - mx) : 0.f;
+            sum += x[j];
+        }
+        const float inv = 1.f / across(sum, add);
+#pragma unroll
+        for (int j = 0; j < V; j++) {
+            const float pv = x[j] * inv, pc = pv < eps ? eps : (pv > hi ? hi : pv), negy = y[j] * -1.0f;
+            x[j] = pv;
+            g[j] = 0.f;
+            if (lane + j * L < C) {
+                loss += negy * logf(pc);
+                g[j] = (pv >= eps && pv <= hi) ? (1.0f / pc) * (negy * inv_count) : 0.f;   // d loss / d p
+                dot += g[j] * pv;
+            }
+        }
+        loss = across(loss, add);
+        dot = across(dot, add);
+#pragma unroll
+        for (int j = 0; j < V; j++)
+            if (row < N && lane + j * L < C) {
+                const float d = x[j] * (g[j] - dot);
+                p[at + lane + j * L] = x[j];
+                dz[at + lane + j * L] = d;
+                largest = fmaxf(largest, scale_entry(d));
+            }
+        if (lane == 0 && row < N) loss_rows[row] = loss;
     }
     if (scale) note_largest(largest, scale);
     if (last_block_done(counter)) finish_loss(loss_rows, N, inv_count, loss_mean, scale, sm);
@@ -604,9 +669,15 @@ int seera_softmax_cce_fwd_bwd(const float *z, const float *onehot, float *p, flo
         return fail(SEERA_E_ARG, "softmax_cce_fwd_bwd: bad argument");
     ProfBytes pb(16.0 * N * C, "softmax_cce");
     // at most two blocks per SM: every block pays for its turn at the finish counter
-    const int grid = (int)((N + 7) / 8 < 2 * rt().sm_count ? (N + 7) / 8 : 2 * rt().sm_count);
-    softmax_cce_kernel<<<grid, 256, 0, rt().stream>>>(z, onehot, p, loss_rows, dz, N, C, eps, inv_count, loss_mean,
-                                                                                loss_scale(dz, (long long)N * C), next_finish_counter());
+    const int per_block = C <= 16 ? 16 : 8, need = (N + per_block - 1) / per_block, grid = need < 2 * rt().sm_count ? need : 2 * rt().sm_count;
+    auto launch = [&](auto kern) {
+        kern<<<grid, 256, 0, rt().stream>>>(z, onehot, p, loss_rows, dz, N, C, eps, inv_count, loss_mean, loss_scale(dz, (long long)N * C),
+                                            next_finish_counter());
+    };
+    if (C <= 16) launch(softmax_cce_row_kernel<16, 1>);
+    else if (C <= 32) launch(softmax_cce_row_kernel<32, 1>);
+    else if (C <= 128) launch(softmax_cce_row_kernel<32, 4>);
+    else launch(softmax_cce_kernel);
     SEERA_LAUNCH_CHECK("softmax_cce");
     return SEERA_OK;
 }

@@ -10,6 +10,9 @@
 //   dA = dC B^T            one thread per element of dA, N multiply-adds
 //   dB = A^T dC (+ dbias)  one thread per row of dB walks its share of the M rows; the shares are summed in a fixed order by a
 //                          second small kernel, so the result does not depend on scheduling
+// All three are bound by how many reads they keep in flight and by what the two narrow operands cost on the way (a row of B per lane
+// touches a line per lane, so B and dB pass through shared memory where that pays).  4096 x 1024 x 10: forward 11.1 -> 8.5 us,
+// dA 6.1 -> 5.3, dB 10.2 -> 6.0; 1000 x 1024 x 10: 6.0 -> 5.2, 3.0, 8.2 -> 3.3.
 #include "common.cuh"
 #include "internal.h"
 #include "tc_epilogue.cuh"
@@ -18,8 +21,10 @@ namespace seera {
 
 constexpr int SK_MAXN = 16;
 
-// k-extent of the slice of B a block keeps in shared memory: N * sk_kc(N) floats, at most 48 KB
-__host__ __device__ constexpr int sk_kc(int n) { return n <= 12 ? 1024 : 768; }
+// k-extent of the slice of B a block keeps in shared memory, N rows of sk_pitch(N) floats, at most 48 KB; the pitch keeps the copies of
+// one k (N of them, a pitch apart) in different banks
+__host__ __device__ constexpr int sk_kc(int n) { return n <= 11 ? 1024 : 704; }
+__host__ __device__ constexpr int sk_pitch(int n) { return sk_kc(n) + 4; }
 constexpr int SK_ROWS = 64;          // most rows of dC a block stages at a time in the two backward kernels
 
 // C = act(A B + bias).  A block keeps B^T (slice by slice when K exceeds it) in shared memory as bt[n][k], so that lane = k reads
@@ -29,33 +34,59 @@ constexpr int SK_ROWS = 64;          // most rows of dC a block stages at a time
 template <int N>
 __global__ void __launch_bounds__(256) skinny_fwd_kernel(const float *__restrict__ A, const float *__restrict__ B, const float *__restrict__ bias,
                                                          float *__restrict__ C, int rows, int K, int act) {
-    constexpr int SK_KC = sk_kc(N);
-    extern __shared__ float bt[];                                        // [N][SK_KC]
+    constexpr int SK_KC = sk_kc(N), PITCH = sk_pitch(N);
+    extern __shared__ float bt[];                                        // [N][PITCH]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int k0 = 0; k0 < K; k0 += SK_KC) {
         const int kc = min(SK_KC, K - k0);
         __syncthreads();
-        for (int e = threadIdx.x; e < kc * N; e += 256) {                 // e = k * N + n: consecutive floats of B
+        // e = k * N + n: consecutive floats of B, every copy in flight at once
+        for (int e = threadIdx.x; e < kc * N; e += 256) {
             const int k = e / N, n = e - k * N;
-            bt[n * SK_KC + k] = __ldg(B + (long long)k0 * N + e);
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(bt + n * PITCH + k)),
+                         "l"(B + (long long)k0 * N + e) : "memory");
         }
-        __syncthreads();
+        asm volatile("cp.async.commit_group;" ::: "memory");
         const bool first = k0 == 0, last = k0 + kc == K;
-        for (int m = (blockIdx.x * 8 + warp) * 2; m < rows; m += gridDim.x * 16) {
-            const bool two = m + 1 < rows;
-            const float *a0 = A + (long long)m * K + k0, *a1 = a0 + (two ? K : 0);
-            float acc0[N], acc1[N];
+        bool landed = false;
+        for (int mb = blockIdx.x * 16; mb < rows; mb += gridDim.x * 16) {
+            const int m = mb + warp * 2;
+            const bool one = m < rows, two = m + 1 < rows;
+            const float *a0 = A + (one ? (long long)m * K : 0) + k0, *a1 = a0 + (two ? K : 0);
+            float acc0[N], acc1[N], x0[8], x1[8];
 #pragma unroll
             for (int n = 0; n < N; n++) { acc0[n] = 0.f; acc1[n] = 0.f; }
-#pragma unroll 8
-            for (int k = lane; k < kc; k += 32) {
-                const float x0 = __ldg(a0 + k), x1 = __ldg(a1 + k);
+            // eight steps of both rows are fetched while the eight before are used, the first of them while B lands
+            auto fetch = [&](int kb, float (&u)[8], float (&v)[8]) {
 #pragma unroll
-                for (int n = 0; n < N; n++) {
-                    const float b = bt[n * SK_KC + k];
-                    acc0[n] = fmaf(x0, b, acc0[n]);
-                    acc1[n] = fmaf(x1, b, acc1[n]);
+                for (int j = 0; j < 8; j++) {
+                    const int k = kb + 32 * j + lane;
+                    u[j] = k < kc ? __ldg(a0 + k) : 0.f;
+                    v[j] = k < kc ? __ldg(a1 + k) : 0.f;
                 }
+            };
+            fetch(0, x0, x1);
+            if (!landed) {
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+                __syncthreads();
+                landed = true;
+            }
+            for (int kb = 0; kb < kc; kb += 256) {
+                float y0[8], y1[8];
+                fetch(kb + 256, y0, y1);
+#pragma unroll
+                for (int j = 0; j < 8; j++) {
+                    const int k = kb + 32 * j + lane;
+                    if (kb + 32 * j >= kc) break;
+                    const float *b = bt + min(k, kc - 1);
+#pragma unroll
+                    for (int n = 0; n < N; n++) {
+                        acc0[n] = fmaf(x0[j], b[n * PITCH], acc0[n]);
+                        acc1[n] = fmaf(x1[j], b[n * PITCH], acc1[n]);
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 8; j++) { x0[j] = y0[j]; x1[j] = y1[j]; }
             }
             float v0 = 0.f, v1 = 0.f;
 #pragma unroll
@@ -68,7 +99,7 @@ __global__ void __launch_bounds__(256) skinny_fwd_kernel(const float *__restrict
                 }
                 if (lane == n) { v0 = t0; v1 = t1; }
             }
-            if (lane < N) {
+            if (lane < N && one) {
                 float *c0 = C + (long long)m * N + lane;
                 if (!first) { v0 += *c0; if (two) v1 += c0[N]; }
                 if (last) {
@@ -83,46 +114,56 @@ __global__ void __launch_bounds__(256) skinny_fwd_kernel(const float *__restrict
     }
 }
 
-// The same for few rows (at most a few blocks' worth per SM): one block per pair of rows, its eight warps take interleaved
+// The same for few rows (at most a few blocks' worth per SM): one block per ROWS rows (two, or four once that still leaves a block for
+// every SM: what bounds it then is the reads of B), its eight warps take interleaved
 // 32-wide pieces of k, B read in place (a warp's reads of B cover 32 * N consecutive floats over its n loop, served by L1), the
 // warps' sums added in warp order through shared memory.  No staging of B, and a long contraction (a flattened feature map into
 // ten classes) is spread over eight warps instead of walked by one.
-template <int N>
+template <int N, int ROWS>
 __global__ void __launch_bounds__(256) skinny_fwd_small_kernel(const float *__restrict__ A, const float *__restrict__ B,
                                                                const float *__restrict__ bias, float *__restrict__ C, int rows, int K, int act) {
-    __shared__ float red[8][2][N];
+    __shared__ float red[8][ROWS][N];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int m = blockIdx.x * 2;
-    const bool two = m + 1 < rows;
-    const float *a0 = A + (long long)m * K, *a1 = a0 + (two ? K : 0);
-    float acc0[N], acc1[N];
+    const int m = blockIdx.x * ROWS;
+    const float *a[ROWS];
+    float acc[ROWS][N];
 #pragma unroll
-    for (int n = 0; n < N; n++) { acc0[n] = 0.f; acc1[n] = 0.f; }
+    for (int r = 0; r < ROWS; r++) {
+        a[r] = A + (long long)min(m + r, rows - 1) * K;
+#pragma unroll
+        for (int n = 0; n < N; n++) acc[r][n] = 0.f;
+    }
+    constexpr int W = N % 2 == 0 ? 2 : 1;                 // floats of a row of B per read (its alignment: see skinny_fwd)
 #pragma unroll 2
     for (int k = warp * 32 + lane; k < K; k += 256) {
-        const float x0 = __ldg(a0 + k), x1 = __ldg(a1 + k);
-        const float *b = B + (long long)k * N;
+        float x[ROWS], b[N];
+#pragma unroll
+        for (int r = 0; r < ROWS; r++) x[r] = __ldg(a[r] + k);
+#pragma unroll
+        for (int n = 0; n < N; n += W) {
+            if (W == 2) {
+                const float2 t = __ldg(reinterpret_cast<const float2 *>(B + (long long)k * N + n));
+                b[n] = t.x; b[n + W - 1] = t.y;
+            } else b[n] = __ldg(B + (long long)k * N + n);
+        }
+#pragma unroll
+        for (int n = 0; n < N; n++)
+#pragma unroll
+            for (int r = 0; r < ROWS; r++) acc[r][n] = fmaf(x[r], b[n], acc[r][n]);
+    }
+#pragma unroll
+    for (int r = 0; r < ROWS; r++)
 #pragma unroll
         for (int n = 0; n < N; n++) {
-            const float bv = __ldg(b + n);
-            acc0[n] = fmaf(x0, bv, acc0[n]);
-            acc1[n] = fmaf(x1, bv, acc1[n]);
-        }
-    }
+            float t = acc[r][n];
 #pragma unroll
-    for (int n = 0; n < N; n++) {
-        float t0 = acc0[n], t1 = acc1[n];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            t0 += __shfl_xor_sync(0xffffffffu, t0, o);
-            t1 += __shfl_xor_sync(0xffffffffu, t1, o);
+            for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+            if (lane == 0) red[warp][r][n] = t;
         }
-        if (lane == 0) { red[warp][0][n] = t0; red[warp][1][n] = t1; }
-    }
     __syncthreads();
-    if (threadIdx.x < 2 * N) {
+    if (threadIdx.x < ROWS * N) {
         const int r = threadIdx.x / N, n = threadIdx.x - r * N;
-        if (r == 0 || two) {
+        if (m + r < rows) {
             float v = 0.f;
 #pragma unroll
             for (int w = 0; w < 8; w++) v += red[w][r][n];
@@ -152,17 +193,34 @@ struct SkinnyRows {
     }
 };
 
-// dA = dC B^T.  Grid (ceil(K / 256), row groups); thread = one column k of dA with its row of B in registers, walking the rows
-// of its group: N multiply-adds per element against broadcast reads of the staged dC rows, stores coalesced over k.
-template <int N>
+// dA = dC B^T.  Grid (ceil(K / 256 V), row groups); thread = V neighbouring columns k of dA (V = 4 where K and the addresses allow) with
+// their rows of B in registers, walking the rows of its group: V N multiply-adds against broadcast reads of a staged dC row, which one
+// column per thread would be bound by; stores coalesced over k.
+template <int N, int V>
 __global__ void __launch_bounds__(256) skinny_dA_kernel(const float *__restrict__ dC, const float *__restrict__ B, float *__restrict__ dA,
                                                         int rows, int K, int chunk_rows) {
     __shared__ __align__(16) SkinnyRows<N> sd;
+    extern __shared__ __align__(16) float sb[];           // V = 4: the block's 1024 rows of B
     constexpr int NP = SkinnyRows<N>::NP;
-    const int k = blockIdx.x * 256 + threadIdx.x;
-    float b[N];
+    const int k = (blockIdx.x * 256 + threadIdx.x) * V;
+    float b[V][N];
+    if (V == 4) {
+        const int k0 = blockIdx.x * 1024, n4 = min(1024, K - k0) * N / 4;
+        for (int e = threadIdx.x; e < n4; e += 256)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(sb + 4 * e)),
+                         "l"(B + (long long)k0 * N + 4 * e) : "memory");
+        asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+        __syncthreads();
+        if (k < K)
 #pragma unroll
-    for (int n = 0; n < N; n++) b[n] = k < K ? __ldg(B + (long long)k * N + n) : 0.f;
+            for (int j = 0; j < V * N; j += 4) {
+                const float4 t = *reinterpret_cast<const float4 *>(sb + threadIdx.x * (V * N) + j);
+                b[j / N][j % N] = t.x; b[(j + 1) / N][(j + 1) % N] = t.y; b[(j + 2) / N][(j + 2) % N] = t.z; b[(j + 3) / N][(j + 3) % N] = t.w;
+            }
+    } else {
+#pragma unroll
+        for (int n = 0; n < N; n++) b[0][n] = k < K ? __ldg(B + (long long)k * N + n) : 0.f;
+    }
     for (int m0 = blockIdx.y * chunk_rows; m0 < rows; m0 += gridDim.y * chunk_rows) {
         const int nrows = min(chunk_rows, rows - m0);
         __syncthreads();
@@ -171,68 +229,83 @@ __global__ void __launch_bounds__(256) skinny_dA_kernel(const float *__restrict_
         if (k < K) {
 #pragma unroll 4
             for (int r = 0; r < nrows; r++) {
-                float d[NP];
+                float d[NP], s[V];
                 sd.row(r, d);
-                float s = 0.f;
 #pragma unroll
-                for (int n = 0; n < N; n++) s = fmaf(d[n], b[n], s);
-                dA[(long long)(m0 + r) * K + k] = s;
+                for (int v = 0; v < V; v++) {
+                    s[v] = 0.f;
+#pragma unroll
+                    for (int n = 0; n < N; n++) s[v] = fmaf(d[n], b[v][n], s[v]);
+                }
+                float *o = dA + (long long)(m0 + r) * K + k;
+                if (V == 4) *reinterpret_cast<float4 *>(o) = make_float4(s[0], s[V > 1 ? 1 : 0], s[V > 2 ? 2 : 0], s[V > 3 ? 3 : 0]);
+                else *o = s[0];
             }
         }
     }
 }
 
-// dB = A^T dC, dbias = column sums of dC.  Grid (ceil(K / 256), splits); thread = one row k of dB walking its split's rows of A
-// (coalesced over k, eight loads in flight) against the staged dC rows.  The splits' sums are added up in index order by a second
-// small kernel, so the result is the same on every run.
-template <int N>
+// dB = A^T dC, dbias = column sums of dC.  Grid (ceil(K / 256 V), splits); thread = V neighbouring rows k of dB (V = 2 where K and the
+// address allow) walking its split's rows of A (coalesced over k, sixteen loads in flight, those past the end predicated off) against
+// the staged dC rows.  The splits' sums are added up in index order by a second small kernel, so the result is the same on every run.
+template <int N, int V>
 __global__ void __launch_bounds__(256) skinny_dB_kernel(const float *__restrict__ A, const float *__restrict__ dC, float *__restrict__ dB,
                                                         float *__restrict__ dbias, float *__restrict__ partial, int rows, int K, int chunk_rows) {
     __shared__ __align__(16) SkinnyRows<N> sd;
+    __shared__ float so[256 * V * N];
     constexpr int NP = SkinnyRows<N>::NP;
-    const int k = blockIdx.x * 256 + threadIdx.x, s = blockIdx.y, splits = gridDim.y;
+    const int k = (blockIdx.x * 256 + threadIdx.x) * V, s = blockIdx.y, splits = gridDim.y;
     const int chunks = (rows + chunk_rows - 1) / chunk_rows, per = (chunks + splits - 1) / splits;
     const int m_begin = (int)min((long long)rows, (long long)s * per * chunk_rows), m_end = (int)min((long long)rows, (long long)(s + 1) * per * chunk_rows);
-    float acc[N], colsum = 0.f;
+    float acc[V][N], colsum = 0.f;
 #pragma unroll
-    for (int n = 0; n < N; n++) acc[n] = 0.f;
+    for (int v = 0; v < V; v++)
+#pragma unroll
+        for (int n = 0; n < N; n++) acc[v][n] = 0.f;
     for (int m0 = m_begin; m0 < m_end; m0 += chunk_rows) {
         const int nrows = min(chunk_rows, m_end - m0);
+        float x[16][V];
+        auto fetch = [&](int r0) {
+            const float *a = A + (long long)m0 * K + k;
+#pragma unroll
+            for (int j = 0; j < 16; j++) {
+                const bool in = k < K && r0 + j < nrows;
+                if (V == 2) {
+                    const float2 t = in ? __ldg(reinterpret_cast<const float2 *>(a + (long long)(r0 + j) * K)) : make_float2(0.f, 0.f);
+                    x[j][0] = t.x; x[j][V - 1] = t.y;
+                } else x[j][0] = in ? __ldg(a + (long long)(r0 + j) * K) : 0.f;
+            }
+        };
+        fetch(0);                                         // on their way while the rows of dC are staged
         __syncthreads();
         sd.stage(dC, m0, nrows);
         __syncthreads();
         if (blockIdx.x == 0 && threadIdx.x < N)
             for (int r = 0; r < nrows; r++) colsum += sd.v[r][threadIdx.x];
-        if (k < K) {
-            const float *a = A + (long long)m0 * K + k;
-            int r = 0;
-            for (; r + 8 <= nrows; r += 8) {
-                float x[8];
+        for (int r = 0; r < nrows; r += 16) {
+            if (r) fetch(r);
 #pragma unroll
-                for (int j = 0; j < 8; j++) x[j] = __ldg(a + (long long)(r + j) * K);
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    float d[NP];
-                    sd.row(r + j, d);
-#pragma unroll
-                    for (int n = 0; n < N; n++) acc[n] = fmaf(x[j], d[n], acc[n]);
-                }
-            }
-            for (; r < nrows; r++) {
-                const float x = __ldg(a + (long long)r * K);
+            for (int j = 0; j < 16; j++) {
+                if (r + j >= nrows) break;
                 float d[NP];
-                sd.row(r, d);
+                sd.row(r + j, d);
 #pragma unroll
-                for (int n = 0; n < N; n++) acc[n] = fmaf(x, d[n], acc[n]);
+                for (int v = 0; v < V; v++)
+#pragma unroll
+                    for (int n = 0; n < N; n++) acc[v][n] = fmaf(x[j][v], d[n], acc[v][n]);
             }
         }
     }
-    // one split: the sums are the result; several: partial[split][k][n] (row K = the column sums), added up in index order below
-    if (k < K) {
-        float *p = splits == 1 ? dB + (long long)k * N : partial + ((long long)s * (K + 1) + k) * N;
+    // one split: the sums are the result; several: partial[split][k][n] (row K = the column sums), added up in index order below.  They
+    // leave through shared memory: N V floats per thread, side by side, would touch a line per lane and store.
 #pragma unroll
-        for (int n = 0; n < N; n++) p[n] = acc[n];
-    }
+    for (int v = 0; v < V; v++)
+#pragma unroll
+        for (int n = 0; n < N; n++) so[threadIdx.x * (V * N) + v * N + n] = acc[v][n];
+    __syncthreads();
+    const int k0 = blockIdx.x * (256 * V), count = min(256 * V, K - k0) * N;
+    float *p = (splits == 1 ? dB : partial + (long long)s * (K + 1) * N) + (long long)k0 * N;
+    for (int e = threadIdx.x; e < count; e += 256) p[e] = so[e];
     if (blockIdx.x == 0 && threadIdx.x < N) {
         if (splits > 1) partial[((long long)s * (K + 1) + K) * N + threadIdx.x] = colsum;
         else if (dbias) dbias[threadIdx.x] = colsum;
@@ -260,11 +333,13 @@ int skinny_fwd(const float *A, const float *B, const float *bias, float *C, int 
     cudaStream_t st = rt().stream;
     int grid = (rows + 15) / 16;
     if (grid > rt().sm_count * 2) grid = rt().sm_count * 2;
-    const size_t smem = (size_t)N * sk_kc(N) * sizeof(float);
+    const size_t smem = (size_t)N * sk_pitch(N) * sizeof(float);
     const bool small = (rows + 1) / 2 <= rt().sm_count * 4;             // a block per pair of rows still fits a wave or so
     profile_begin();
-    if (small) { SK_DISPATCH(N, (skinny_fwd_small_kernel<NN><<<(rows + 1) / 2, 256, 0, st>>>(A, B, bias, C, rows, K, act))) }
-    else
+    if (small && (reinterpret_cast<uintptr_t>(B) & 7) == 0) {
+        if ((rows + 3) / 4 >= rt().sm_count) { SK_DISPATCH(N, (skinny_fwd_small_kernel<NN, 4><<<(rows + 3) / 4, 256, 0, st>>>(A, B, bias, C, rows, K, act))) }
+        else { SK_DISPATCH(N, (skinny_fwd_small_kernel<NN, 2><<<(rows + 1) / 2, 256, 0, st>>>(A, B, bias, C, rows, K, act))) }
+    } else
     SK_DISPATCH(N, (skinny_fwd_kernel<NN><<<grid, 256, smem, st>>>(A, B, bias, C, rows, K, act)))
     count_launch();
     profile_end(2.0 * rows * N * (double)K, name);
@@ -275,22 +350,40 @@ int skinny_fwd(const float *A, const float *B, const float *bias, float *C, int 
 int skinny_bwd(const float *A, const float *B, const float *dC, float *dA, float *dB, float *dbias, int rows, int N, int K) {
     cudaStream_t st = rt().stream;
     cudaError_t e = cudaSuccess;
-    const int kblocks = (K + 255) / 256;
-    int groups = (rt().sm_count * 4 + kblocks - 1) / kblocks;            // about four blocks per SM
-    // rows staged at a time: few where the rows are few, so that a small problem still spreads over many blocks (8 ... SK_ROWS)
-    int chunk_rows = ((rows + groups - 1) / groups + 7) / 8 * 8;
-    if (chunk_rows > SK_ROWS) chunk_rows = SK_ROWS;
-    const int chunks = (rows + chunk_rows - 1) / chunk_rows;
-    if (groups > chunks) groups = chunks;
-    if (groups > 65535) groups = 65535;
+    auto aligned = [&](const void *p, int v) { return K % v == 0 && (reinterpret_cast<uintptr_t>(p) & (4 * v - 1)) == 0; };
+    // rows staged at a time and row groups for `kblocks` blocks of columns: about `per_sm` blocks per SM; few rows where the rows are few,
+    // so that a small problem still spreads over many blocks (at least `least`, at most SK_ROWS)
+    int chunk_rows = 0, groups = 0;
+    auto split = [&](int kblocks, int per_sm, int least) {
+        groups = (rt().sm_count * per_sm + kblocks - 1) / kblocks;
+        chunk_rows = ((rows + groups - 1) / groups + least - 1) / least * least;
+        if (chunk_rows > SK_ROWS) chunk_rows = SK_ROWS;
+        const int chunks = (rows + chunk_rows - 1) / chunk_rows;
+        if (groups > chunks) groups = chunks;
+        if (groups > 65535) groups = 65535;
+    };
     if (dA) {
         profile_begin();
-        SK_DISPATCH(N, (skinny_dA_kernel<NN><<<dim3(kblocks, groups), 256, 0, st>>>(dC, B, dA, rows, K, chunk_rows)))
+        // (the copy of B per block pays from a few rows per block on)
+        if (aligned(dA, 4) && aligned(B, 4) && (long long)rows * K >= 1 << 19) {
+            const int kb = (K / 4 + 255) / 256;
+            const size_t smem = (size_t)1024 * N * sizeof(float);
+            split(kb, 2, 8);
+            if (smem > 44 * 1024) SK_DISPATCH(N, e = cudaFuncSetAttribute(skinny_dA_kernel<NN, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem))
+            if (e == cudaSuccess) SK_DISPATCH(N, (skinny_dA_kernel<NN, 4><<<dim3(kb, groups), 256, smem, st>>>(dC, B, dA, rows, K, chunk_rows)))
+        } else {
+            const int kb = (K + 255) / 256;
+            split(kb, 4, 8);
+            SK_DISPATCH(N, (skinny_dA_kernel<NN, 1><<<dim3(kb, groups), 256, 0, st>>>(dC, B, dA, rows, K, chunk_rows)))
+        }
         count_launch();
         profile_end(2.0 * rows * N * (double)K, "cuda_matmul_bwd(dA)");
-        e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaGetLastError();
     }
     if (e == cudaSuccess && (dB || dbias)) {
+        const bool two = aligned(A, 2);
+        const int kb = ((two ? K / 2 : K) + 255) / 256;
+        split(kb, 2, (long long)rows * K >= 1 << 19 ? 16 : 8);        // few splits: what each of them leaves is written and read again
         const int splits = groups;
         float *partial = (float *)scratch_alloc((size_t)splits * (K + 1) * N * sizeof(float));
         float *db_out = dB;
@@ -298,7 +391,8 @@ int skinny_bwd(const float *A, const float *B, const float *dC, float *dA, float
         if (!partial) return SEERA_E_OOM;
         if (!dB) { tmp = (float *)scratch_alloc((size_t)K * N * sizeof(float)); if (!tmp) { scratch_free(partial); return SEERA_E_OOM; } db_out = tmp; }
         profile_begin();
-        SK_DISPATCH(N, (skinny_dB_kernel<NN><<<dim3(kblocks, splits), 256, 0, st>>>(A, dC, db_out, dbias, partial, rows, K, chunk_rows)))
+        if (two) { SK_DISPATCH(N, (skinny_dB_kernel<NN, 2><<<dim3(kb, splits), 256, 0, st>>>(A, dC, db_out, dbias, partial, rows, K, chunk_rows))) }
+        else { SK_DISPATCH(N, (skinny_dB_kernel<NN, 1><<<dim3(kb, splits), 256, 0, st>>>(A, dC, db_out, dbias, partial, rows, K, chunk_rows))) }
         count_launch();
         if (splits > 1) {
             launch_sum_splits(partial, db_out, (K + 1) * N, splits, st, dbias, K * N);

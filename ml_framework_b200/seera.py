@@ -232,6 +232,35 @@ class _Unpooled(cuten):
         self._ptr = value
 
 
+class _Softmax(cuten):
+    """The row softmax of the logits `z` as a tensor whose values are made when its address is asked for.  The cross-entropy, which has to
+    form them anyway, writes them on its way (claim), and a training step then needs no pass for them."""
+    z = None
+
+    @classmethod
+    def of(cls, z):
+        t = cls._wrap(None, z.shape)
+        t.z = z
+        return t
+
+    def claim(self):
+        """Address for a caller that writes the values itself."""
+        if self._ptr is None:
+            self._ptr = _malloc(self.size)
+        return self._ptr
+
+    @property
+    def main_ptr(self):
+        if self._ptr is None:
+            self._ptr = _malloc(self.size)
+            sc.cuda_softmax_fwd(self.z.main_ptr, self._ptr, *self.shape)
+        return self._ptr
+
+    @main_ptr.setter
+    def main_ptr(self, value):
+        self._ptr = value
+
+
 class _KeptCopies:
     """Owner of the channels-last copies a forward call kept for its backward call (0: none kept)."""
     __slots__ = ("h",)
@@ -407,12 +436,11 @@ class _ParamLayer(Layer):
             node._takes_pooled = True
         if self.layeract != "softmax":
             return node
-        y = _new(z.shape)
-        sc.cuda_softmax_fwd(z._ptr, y._ptr, z.shape[0], z.shape[1])
+        y = _Softmax.of(z)
 
         def softmax_backward(g):
             dz = _new(y.shape)
-            sc.cuda_softmax_vjp(y._ptr, g.main_ptr, dz._ptr, y.shape[0], y.shape[1])
+            sc.cuda_softmax_vjp(y.main_ptr, g.main_ptr, dz._ptr, y.shape[0], y.shape[1])
             node._accumulate(dz)
         out = Tensor._of(y, (node,), softmax_backward)
         out._softmax_logits = node
@@ -1248,7 +1276,8 @@ class Loss:
         if tuple(yv.shape) != (N, C):
             raise ValueError(f"[cuTen]: Shapes {tuple(yv.shape)} and {(N, C)} not broadcastable")
         rows, loss, dz = _new((N,)), _new((1,)), _new((N, C))
-        sc.softmax_cce_fwd_bwd(z.main_ptr, yv.main_ptr, y_pred.value.main_ptr, rows._ptr, loss._ptr, dz._ptr,
+        p = y_pred.value
+        sc.softmax_cce_fwd_bwd(z.main_ptr, yv.main_ptr, p.claim() if p.__class__ is _Softmax else p.main_ptr, rows._ptr, loss._ptr, dz._ptr,
                                N, C, float(epsilon), float(f32(1.0 / N)))
         # the gradient arrives as the all-ones seed of a scalar loss
         out = Tensor._of(loss, (logits,), lambda g: (_scale_gradients(dz), logits._accumulate(dz)))

@@ -1,0 +1,70 @@
+"""Classifier heads: dense products of few output columns (exact fp32) and the softmax cross-entropy, at the edges of their variants."""
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture
+def sc():
+    from ml_framework_b200 import seera_cuda as sc
+    sc.init(0)
+    sc.set_precision(3)
+    yield sc
+    sc.set_precision(0)
+
+
+#         rows  K    N
+SHAPES = [(1, 1, 1), (3, 5, 7), (64, 784, 10), (593, 256, 16), (1000, 1024, 10), (1185, 1030, 10), (2500, 1500, 3), (601, 1026, 13), (1300, 2050, 16)]
+
+
+@pytest.mark.parametrize("shape", SHAPES)
+def test_products_of_few_columns(sc, shape):
+    M, K, N = shape
+    rs = np.random.RandomState(sum(shape))
+    a, b, g, bias = (rs.standard_normal(s).astype(np.float32) for s in ((M, K), (K, N), (M, N), (N,)))
+    ad, bd, gd, biasd = (sc.to_device_f32(t.ravel()) for t in (a, b, g, bias))
+    cd, da, db = (sc.cuda_malloc_f32(t.size) for t in (g, a, b))
+    sc.matmul_bias_act_fwd(ad, bd, biasd, cd, M, N, K, 1)
+    a64, b64, g64 = (t.astype(np.float64) for t in (a, b, g))
+    assert rel_l2(sc.to_host_f32(cd, (M, N)), np.maximum(a64 @ b64 + bias, 0)) < 2e-6
+    sc.cuda_matmul_bwd(ad, bd, gd, da, db, M, N, K, 1)
+    assert rel_l2(sc.to_host_f32(da, (M, K)), g64 @ b64.T) < 2e-6 and rel_l2(sc.to_host_f32(db, (K, N)), a64.T @ g64) < 2e-6
+    for p in (ad, bd, gd, biasd, cd, da, db):
+        sc.cuda_free(p)
+
+
+@pytest.mark.parametrize("shape", [(1, 1), (1, 10), (64, 10), (4097, 10), (5000, 16), (37, 17), (300, 32), (33, 33), (9, 128), (7, 129)])
+def test_softmax_cross_entropy(sc, shape):
+    N, C = shape
+    rs = np.random.RandomState(N + C)
+    z, y = (rs.standard_normal(shape) * 3).astype(np.float32), np.eye(C, dtype=np.float32)[rs.randint(0, C, N)]
+    zd, yd = sc.to_device_f32(z.ravel()), sc.to_device_f32(y.ravel())
+    p, rows, loss, dz = (sc.cuda_malloc_f32(k) for k in (N * C, N, 1, N * C))
+    eps = 1e-7
+    for _ in range(2):                          # the finish counter starts from zero again
+        sc.softmax_cce_fwd_bwd(zd, yd, p, rows, loss, dz, N, C, eps, 1.0 / N)
+    e = np.exp(z.astype(np.float64) - z.max(1, keepdims=True))
+    want = e / e.sum(1, keepdims=True)
+    clipped = np.clip(want, eps, 1 - eps)
+    per_row = -(y * np.log(clipped)).sum(1)
+    g = np.where((want >= eps) & (want <= 1 - eps), -y / clipped / N, 0)
+    assert rel_l2(sc.to_host_f32(p, shape), want) < 1e-6
+    assert np.allclose(sc.to_host_f32(rows, (N,)), per_row, rtol=2e-5, atol=2e-7)
+    assert np.allclose(sc.to_host_f32(loss, (1,)), per_row.mean(), rtol=2e-5, atol=2e-7)
+    assert np.abs(sc.to_host_f32(dz, shape) - want * (g - (g * want).sum(1, keepdims=True))).max() < 2e-6 / N
+    for q in (zd, yd, p, rows, loss, dz):
+        sc.cuda_free(q)
+
+
+def test_the_predictions_are_there_for_whoever_reads_them(sc):
+    from ml_framework_b200 import seera as S
+    rs = np.random.RandomState(1)
+    x, y = rs.standard_normal((6, 5)).astype(np.float32), np.eye(3, dtype=np.float32)[[0, 1, 2, 0, 1, 2]]
+    model = S.Sequential([S.Input((5,)), S.Dense(5, 3, "softmax")])
+    before = model.forward(x).to_numpy()        # read before any loss
+    pred = model.forward(x)
+    S.Loss().categorical_cross_entropy(pred, S.Tensor(y, is_leaf=True))
+    assert np.allclose(pred.to_numpy(), before, rtol=1e-6) and np.allclose(before.sum(1), 1, rtol=1e-5)
