@@ -988,7 +988,7 @@ int seera_maxpool2x2_fwd_s(const float *X, float *out, int *mask, int N, int C, 
 // In raster row order a 2x2 window must lie inside one epilogue warp's 32 rows: OW a power of two <= 16 and an even OH.
 static bool pool_in_epilogue_ok(int NB, int C, int H, int W, int F, int R, int S, int sh, int sw, int ph, int pw) {
     if (!rt().precision || !rt().conv_tma || !conv_ok(NB, C, H, W, F, R, S, sh, sw, ph, pw)) return false;
-    if (conv_pool_simt_applies(NB, C, H, W, F, R, S, sh, sw, ph, pw)) return true;
+    if (conv_pool_tc_applies(NB, C, H, W, F, R, S, sh, sw, ph, pw) || conv_pool_simt_applies(NB, C, H, W, F, R, S, sh, sw, ph, pw)) return true;
     if (conv_first_applies(C, R, S))       // the tensor-core short-patch kernel's pooled epilogue only on request
         return (rt().pool_short_patch && conv_first_pool_ok(NB, C, H, W, F, R, S, sh, sw, ph, pw));
     if (!tma_conv_supported(NB, R, S, sh, sw, ph, pw)) return false;
@@ -1030,7 +1030,9 @@ int seera_conv2d_bias_act_pool_fwd_k(const float *X, const float *Wt, const floa
         po.ns = ns; po.Cp = pc.Cp; po.enc = pc.enc;
     }
     int s;
-    if (conv_pool_simt_applies(NB, C, H, W, F, R, S, sh, sw, ph, pw)) {
+    if (conv_pool_tc_applies(NB, C, H, W, F, R, S, sh, sw, ph, pw)) {
+        s = conv_pool_tc(X, Wt, bias, po, NB, C, H, W, F, ph, pw, act, "conv2d_pool_fwd");
+    } else if (conv_pool_simt_applies(NB, C, H, W, F, R, S, sh, sw, ph, pw)) {
         s = conv_pool_simt(X, Wt, bias, po, NB, C, H, W, F, ph, pw, act, "conv2d_pool_fwd");
     } else if (conv_first_applies(C, R, S)) {
         s = conv_first_pool_fwd(X, Wt, bias, po, NB, C, H, W, F, R, S, ph, pw, sh, sw, act, "conv2d_pool_fwd");

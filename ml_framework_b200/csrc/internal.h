@@ -56,6 +56,10 @@ int conv_few_fwd(const float *X, const float *Wt, const float *bias, float *Y, i
 bool conv_pool_simt_applies(int NB, int C, int H, int W, int F, int R, int S, int sh, int sw, int ph, int pw);
 int conv_pool_simt(const float *X, const float *Wt, const float *bias, const PoolOut &pool, int NB, int C, int H, int W, int F, int ph, int pw,
                    int act, const char *name);
+// The same on the tensor cores for one to three input channels and a batch that fills the chip, fp32-class (conv_pool_tc.cu).
+bool conv_pool_tc_applies(int NB, int C, int H, int W, int F, int R, int S, int sh, int sw, int ph, int pw);
+int conv_pool_tc(const float *X, const float *Wt, const float *bias, const PoolOut &pool, int NB, int C, int H, int W, int F, int ph, int pw,
+                 int act, const char *name);
 // 3 x 3 unit-stride convolutions of little work, exact fp32 on the CUDA cores (conv_small.cu); bias, y, dX, dW and dbias may be null.
 // The gradient is g at full resolution or gp through a 2x2 max-pool.
 bool conv_small_applies(int NB, int C, int H, int W, int F, int R, int S, int sh, int sw, int ph, int pw);

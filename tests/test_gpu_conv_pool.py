@@ -14,7 +14,10 @@ pytestmark = pytest.mark.gpu
 SHAPES = [(1, 1, 2, 2, 8, 1), (5, 1, 28, 28, 8, 1), (3, 3, 32, 32, 64, 1), (2, 2, 30, 18, 24, 0), (9, 7, 6, 10, 16, 2),
           (1, 3, 70, 90, 16, 1),          # several bands, the last one partial
           (2, 3, 6, 900, 8, 1),           # one window row per band, one buffer
-          (1, 7, 4, 1500, 16, 1)]         # not staged
+          (1, 7, 4, 1500, 16, 1),         # not staged
+          # on the tensor cores: one to three channels, a ragged last tile, filters in one chunk of 16s or several of 64, images across tiles
+          (77, 3, 32, 32, 64, 1), (18, 1, 70, 62, 32, 1), (19, 2, 66, 66, 48, 0), (13, 3, 60, 54, 128, 2), (2401, 1, 6, 10, 64, 0),
+          (701, 2, 18, 18, 32, 1)]        # several tiles per CTA
 
 
 @pytest.mark.parametrize("mode,act", [(3, 1), (4, 1), (1, 2), (3, 0)])
