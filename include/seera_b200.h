@@ -66,6 +66,7 @@ int         seera_event_destroy(void *event);
  * algorithmic bytes of a bandwidth-bound pass), and leaves the table alone.  Nothing is recorded during a
  * stream capture.  No counterpart in the reference. */
 int         seera_profile_enable(int on);
+int         seera_profile_enabled(void);
 int         seera_profile_read(uint64_t *launches, double *ms, double *flops);
 int         seera_profile_read_kinds(uint64_t *launches3, double *ms3, double *flops3);
 int         seera_profile_report(char *buf, size_t size);

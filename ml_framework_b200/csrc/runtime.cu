@@ -7,6 +7,7 @@
 // rounded size.  All work runs on one stream, so a block returned by cuda_free may be reused
 // by the next allocation without waiting: every kernel that still reads it was enqueued earlier.
 #include "common.cuh"
+#include <algorithm>
 #include <cstdarg>
 #include <cstdlib>
 #include <cstring>
@@ -74,6 +75,7 @@ struct GraphRec {
     uint64_t launches_at_begin = 0;
     bool collectives = false;                           // the recording holds launches of the data-parallel communicator
     std::vector<OptNode> optimizers;                    // recorded optimizer updates, whose scalars change from replay to replay
+    size_t chain = 0;                                   // number of nodes if each follows the one before it, else 0
 };
 static std::vector<GraphRec *> &live_graphs() { static std::vector<GraphRec *> v; return v; }
 struct Pool {
@@ -218,6 +220,67 @@ void graph_note_optimizer(const OptLaunch &launch) {
         cudaGetLastError();
 }
 
+// Executable graphs of recordings that have been destroyed, for the next recording of as many launches in a row: updating one takes
+// 8 us where making one takes 125 and destroying it 110 (14 launches; a short training run records its step once).  At most
+// SPARES_MAX; seera_pool_trim gives them back.  Nodes are named by the graph an executable was made from, which stays with it.
+namespace {
+constexpr size_t SPARES_MAX = 4;
+struct Spare {
+    cudaGraph_t graph;
+    cudaGraphExec_t exec;
+    std::vector<OptNode> optimizers;
+    size_t chain;
+};
+std::vector<Spare> &spares() { static std::vector<Spare> v; return v; }
+}  // namespace
+static size_t chain_length(cudaGraph_t g) {
+    size_t nodes = 0, edges = 0, roots = 0;
+    if (cudaGraphGetNodes(g, nullptr, &nodes) != cudaSuccess || cudaGraphGetEdges(g, nullptr, nullptr, &edges) != cudaSuccess ||
+        cudaGraphGetRootNodes(g, nullptr, &roots) != cudaSuccess || !nodes || roots != 1 || edges != nodes - 1) {
+        cudaGetLastError();
+        return 0;
+    }
+    std::vector<cudaGraphNode_t> from(edges), to(edges);
+    if (edges && cudaGraphGetEdges(g, from.data(), to.data(), &edges) != cudaSuccess) { cudaGetLastError(); return 0; }
+    std::sort(from.begin(), from.end());
+    return std::adjacent_find(from.begin(), from.end()) == from.end() ? nodes : 0;       // nothing has two successors
+}
+static void spares_trim(size_t keep) {
+    auto &v = spares();
+    while (v.size() > keep) {
+        cudaGraphExecDestroy(v.front().exec);
+        cudaGraphDestroy(v.front().graph);
+        v.erase(v.begin());
+    }
+}
+static void take_spare(GraphRec *g) {
+    auto &v = spares();
+    for (size_t i = v.size(); i-- > 0;) {
+        if (v[i].chain != g->chain || v[i].optimizers.size() != g->optimizers.size()) continue;
+        Spare sp = v[i];
+        v.erase(v.begin() + (long)i);
+        cudaGraphExecUpdateResultInfo info;
+        if (cudaGraphExecUpdate(sp.exec, g->graph, &info) == cudaSuccess) {
+            cudaGraphDestroy(g->graph);
+            g->graph = sp.graph;
+            g->exec = sp.exec;
+            for (size_t k = 0; k < sp.optimizers.size(); k++) g->optimizers[k].node = sp.optimizers[k].node;
+            return;
+        }
+        cudaGetLastError();                             // other launches: not for this recording, nor known to be for any other
+        cudaGraphExecDestroy(sp.exec);
+        cudaGraphDestroy(sp.graph);
+    }
+}
+// The caller has waited for the graph's last launch.
+static void keep_spare(GraphRec *g) {
+    if (!g->exec || !g->graph || !g->chain) return;
+    spares_trim(SPARES_MAX - 1);
+    spares().push_back({g->graph, g->exec, g->optimizers, g->chain});
+    g->graph = nullptr;
+    g->exec = nullptr;
+}
+
 void *scratch_alloc(size_t bytes) { return seera_cuda_malloc(bytes); }
 void scratch_free(void *p) { seera_cuda_free(p); }
 
@@ -317,6 +380,7 @@ float seera_event_elapsed_ms(void *a, void *b) {
 }
 int seera_event_destroy(void *ev) { return ev ? check_cuda(cudaEventDestroy((cudaEvent_t)ev), "cudaEventDestroy") : SEERA_OK; }
 
+int seera_profile_enabled(void) { return seera::prof().on ? 1 : 0; }
 int seera_profile_enable(int on) {
     auto &p = seera::prof();
     if (int s = batch_flush()) return s;
@@ -440,6 +504,7 @@ int seera_pool_trim(void) {
         for (void *b : kv.second) { cudaFree(b); p.reserved -= kv.first; }
         kv.second.clear();
     }
+    spares_trim(0);
     pinned_trim();
     return SEERA_OK;
 }
@@ -472,7 +537,11 @@ void *seera_graph_end(void) {
     g->kernels = rt().launches - g->launches_at_begin;
     rt().launches = g->launches_at_begin;               // recorded, not executed
     cudaError_t e = cudaStreamEndCapture(rt().stream, &g->graph);
-    if (e == cudaSuccess) e = cudaGraphInstantiate(&g->exec, g->graph, 0);
+    if (e == cudaSuccess && !g->collectives) {
+        g->chain = chain_length(g->graph);
+        if (g->chain) take_spare(g);
+    }
+    if (e == cudaSuccess && !g->exec) e = cudaGraphInstantiate(&g->exec, g->graph, 0);
     if (e != cudaSuccess) {
         check_cuda(e, "graph_end");
         cudaGetLastError();
@@ -498,6 +567,7 @@ int seera_graph_destroy(void *graph) {
     Pool &p = pool();
     batch_flush();
     if (rt().stream) cudaStreamSynchronize(rt().stream);
+    keep_spare(g);
     if (g->exec) cudaGraphExecDestroy(g->exec);
     if (g->graph) cudaGraphDestroy(g->graph);
     for (auto &b : g->blocks) {

@@ -148,6 +148,7 @@ PYBIND11_MODULE(seera_cuda, m) {
     m.def("event_record", [](uptr e) { ck(seera_event_record(P<void>(e))); });
     m.def("event_elapsed_ms", [](uptr a, uptr b) { return seera_event_elapsed_ms(P<void>(a), P<void>(b)); });
     m.def("event_destroy", [](uptr e) { ck(seera_event_destroy(P<void>(e))); });
+    m.def("profile_enabled", []() { return seera_profile_enabled() != 0; });
     m.def("profile_enable", [](int on) { ck(seera_profile_enable(on)); });
     m.def("profile_read_kinds", []() {
         uint64_t n[3]; double ms[3], fl[3];

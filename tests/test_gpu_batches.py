@@ -98,3 +98,59 @@ def test_page_locked_blocks_are_used_again_only_when_their_copies_have_passed(sc
         assert np.all(sc.to_host_f32(d, (n,)) == k)
         sc.host_free_pinned(q)
     sc.cuda_free(d)
+
+
+@pytest.mark.parametrize("labels", [False, True])
+def test_a_recorded_fit_equals_an_eager_one(monkeypatch, labels):
+    """Ragged last batches between replays, BatchNorm's running statistics, history, weights and what the layers hold afterwards."""
+    from ml_framework_b200 import seera as S, seera_cuda as sc
+    sc.init(0)
+    sc.set_precision(3)
+    rs = np.random.RandomState(4)
+    X, lab = rs.standard_normal((75, 1, 8, 8)).astype(np.float32), rs.randint(0, 5, 75).astype(np.int32)
+    runs = []
+    for first in (10 ** 9, 1):
+        monkeypatch.setattr(S, "_RECORD_FROM", first)
+        np.random.seed(2)
+        m = S.Sequential([S.Input((1, 8, 8)), S.Conv2D(8, 1, (3, 3), "relu", stride=1, zero_padding=1), S.BatchNorm2d(8),
+                          S.MaxPool2D((2, 2), stride=2), S.Flatten(), S.Dense(128, 5, activation="softmax")])
+        opt = S.Adam(m, lr=1e-2)
+        h = m.fit(X, lab if labels else np.eye(5, dtype=np.float32)[lab], opt, S.Loss().categorical_cross_entropy, Epochs=3, batch_size=16,
+                  Loss_interval=100, num_classes=5 if labels else None)
+        bn = m.model[2]
+        runs.append([h, opt.t, bn._rm.to_host_f32(), bn._rv.to_host_f32(), m.model[-1].outputs.to_numpy(),
+                     *(t.to_numpy() for t in m.parameters()), *(t.grad.to_host_f32() for t in m.parameters())])
+    for a, b in zip(*runs):
+        assert np.array_equal(a, b)
+    sc.set_precision(0)
+
+
+def test_recordings_made_from_one_another():
+    """A recording destroyed leaves its executable to the next of as many launches: other operators, addresses and optimizer scalars."""
+    from ml_framework_b200 import seera_cuda as sc
+    sc.init(0)
+    n = 1000
+    rs = np.random.RandomState(0)
+    host = [rs.standard_normal(n).astype(np.float32) for _ in range(3)]
+    for round_ in range(8):
+        d = [sc.to_device_f32(a) for a in host]
+        out, vel = sc.cuda_malloc_f32(n), sc.cuda_zeros_f(n)
+        other = round_ % 3
+        sc.graph_begin()
+        (sc.cuda_elemadd, sc.cuda_elemmult, sc.cuda_elemadd)[other](d[0], d[1], out, n)
+        sc.cuda_sgd_step(d[2], out, vel, n, 0.1, 0.0, 1.0)
+        if other == 2:
+            sc.cuda_elemadd(d[0], d[0], out, n)
+        g = sc.graph_end()
+        w = host[2].copy()
+        base = host[0] * host[1] if other == 1 else host[0] + host[1]
+        for lr in (0.5, 0.25):
+            sc.graph_set_scalars(g, [lr, 0.0, 1.0])
+            sc.graph_launch(g)
+            w = w - np.float32(lr) * base
+        assert np.allclose(sc.to_host_f32(d[2], (n,)), w, rtol=1e-6, atol=1e-6)
+        sc.graph_destroy(g)
+        if round_ == 5:
+            sc.pool_trim()
+        for p in d + [out, vel]:
+            sc.cuda_free(p)
