@@ -863,6 +863,7 @@ int conv_first_pool_fwd(const float *X, const float *Wt, const float *bias, cons
 
 bool conv_first_copies_ok(const float *X, const float *Y, int NB, int C, int H, int W, int F, int R, int S, int sh, int sw, int ph, int pw) {
     FirstGeom g;
+    if (conv_direct_applies(NB, C, H, W, F, R, S, sh, sw, ph, pw, true)) return true;
     return first_geom(g, NB, C, H, W, F, R, S, sh, sw, ph, pw) && first_tc_fwd_ok(g) &&
            !conv_c1_fwd_applies(X, Y, NB, C, H, W, F, R, S, sh, sw, ph, pw);
 }
@@ -870,9 +871,13 @@ int conv_first_fwd(const float *X, const float *Wt, const float *bias, float *Y,
                    int ph, int pw, int sh, int sw, int act, const char *name, const StorePixelRows *with_copies) {
     FirstGeom g;
     if (!first_geom(g, NB, C, H, W, F, R, S, sh, sw, ph, pw)) return fail(SEERA_E_LIMIT, "%s: shape outside the short-patch kernel", name);
+    if (with_copies && conv_direct_applies(NB, C, H, W, F, R, S, sh, sw, ph, pw, true))
+        return conv_direct_fwd(X, Wt, bias, Y, NB, C, H, W, F, sh, ph, pw, act, with_copies, name);
     if (with_copies) return first_tc_fwd(X, Wt, bias, Y, g, act, name, nullptr, with_copies);
     if (conv_c1_fwd_applies(X, Y, NB, C, H, W, F, R, S, sh, sw, ph, pw))       // one input channel, "same" 3 x 3: output-bound stencil
         return conv_c1_fwd(X, Wt, bias, Y, NB, H, W, F, ph, act, name);
+    if (conv_direct_applies(NB, C, H, W, F, R, S, sh, sw, ph, pw, false))
+        return conv_direct_fwd(X, Wt, bias, Y, NB, C, H, W, F, sh, ph, pw, act, nullptr, name);
     if (first_tc_fwd_ok(g)) return first_tc_fwd(X, Wt, bias, Y, g, act, name);
     long long pixels = (long long)NB * g.OH * g.OW;
     unsigned chunks = (unsigned)((F + FIRST_FC - 1) / FIRST_FC);

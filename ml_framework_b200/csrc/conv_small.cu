@@ -9,7 +9,14 @@
 // gradient is the same convolution of dz with the taps reversed; dz - activation slope, and the routing through a 2x2 max-pool - is
 // formed while the band is staged.  The weight gradient goes to first_dw in groups of four input channels, and a layer with its pool to
 // conv_pool_simt.
+//
+// The forward of a layer with up to four input channels (stride 1 or 2) takes the same kernel at any size: it is bound by its stores - the
+// output and, for the convolution that reads it, the channels-last copies - of which a lane with 16 filters writes whole sectors, where
+// the tensor-core form is bound by the warps that gather and split patches.  1 -> 32 channels, stride 2, 256 images of 64 x 64 with copies
+// (67 MB): 35 -> 28 us, a third of it waiting for instructions (the straight-line code runs twice per warp); passing the outputs through
+// shared memory to shorten it gave 26 there and cost 2 us where no copies are made.  3 -> 32 channels, 128 images of 32 x 32: 14.6 -> 10.9.
 #include "conv_first.cuh"
+#include "contraction_functors.cuh"
 #include "internal.h"
 
 namespace seera {
@@ -34,17 +41,25 @@ struct SmallSource {
     const int *mask;           // v (and y) of a 2x2 / stride-2 max-pool; null: full resolution
     int act;
 };
+// Channels-last copies of the output ([pixel][Cp], Cp = O); p[0] null: none.
+struct SmallCopies {
+    __nv_bfloat16 *p[3];
+    int Cp, ns;
+    Enc enc;
+};
 struct SmallGeom {
     int I, IH, IW, O, OH, OW, ph, pw;        // input / output channels and planes, lower padding
     int window_rows, per_image, rows, pitch, OP, groups;
     FastDiv by_bands, by_pitch, by_rows, by_cols, by_groups;
 };
 
-template <int FW>
-__global__ void __launch_bounds__(256) conv3x3_small_kernel(SmallSource src, const float *__restrict__ Wt, const float *__restrict__ bias,
-                                                            float *__restrict__ Y, SmallGeom g, int total, int reversed, int act) {
-    extern __shared__ __align__(16) float sm[];          // [I][9][OP] weights, [OP] biases, [8][4 FW][32] sums, [I][rows][pitch] band
-    float *bk = sm + g.I * 9 * g.OP, *red = bk + g.OP, *band = red + 8 * 4 * FW * 32;
+template <int FW, int ST>
+__global__ void __launch_bounds__(256, FW >= 8 ? 2 : 1) conv3x3_small_kernel(SmallSource src, const float *__restrict__ Wt,
+                                                                              const float *__restrict__ bias, float *__restrict__ Y,
+                                                                              SmallCopies cc, SmallGeom g, int total, int reversed, int act) {
+    constexpr int PR = 3 + ST, PC = (PR + 1) / 2 * 2;     // rows of a patch, and columns read of it
+    extern __shared__ __align__(16) float sm[];          // [I][9][OP] weights, [OP] biases, [8][4 FW][32] sums (data gradient), [I][rows][pitch] band
+    float *bk = sm + g.I * 9 * g.OP, *red = bk + g.OP, *band = red + (reversed ? 8 * 4 * FW * 32 : 0);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = g.I * 9 * g.OP;
     // Wt[o][i][t], or for the data gradient Wt[i][o][8 - t]
     for (int e0 = threadIdx.x; e0 < nw; e0 += 8 * 256) {
@@ -64,7 +79,7 @@ __global__ void __launch_bounds__(256) conv3x3_small_kernel(SmallSource src, con
     const bool pairs = (g.OW & 1) == 0 && (reinterpret_cast<uintptr_t>(Y) & 7) == 0;
 
     for (int id = blockIdx.x; id < total; id += gridDim.x) {
-        const int n = g.by_bands.div(id), q0 = (id - n * g.per_image) * g.window_rows, ih0 = 2 * q0 - g.ph;
+        const int n = g.by_bands.div(id), q0 = (id - n * g.per_image) * g.window_rows, ih0 = 2 * ST * q0 - g.ph;
         if (src.mask) {                                   // every pixel from its window's gradient, index and output
             const int Wq = g.IW >> 1;
             const long long qplane = iplane >> 2, base = (long long)n * g.I * qplane;
@@ -114,19 +129,21 @@ __global__ void __launch_bounds__(256) conv3x3_small_kernel(SmallSource src, con
             const bool mine = at < items;
             const int tile = g.by_groups.div(item), o0 = (item - tile * g.groups) * FW;
             const int w = tile * 32 + lane, wl = min(w, windows - 1), qr = g.by_cols.div(wl), qc = wl - qr * cols;
-            const float *patch = band + i0 * bplane + 2 * qr * g.pitch + 2 * qc, *wc = sm + i0 * 9 * g.OP + o0;
+            const float *patch = band + i0 * bplane + 2 * ST * qr * g.pitch + 2 * ST * qc, *wc = sm + i0 * 9 * g.OP + o0;
             f32x2 acc[4][FW / 2];                         // [pixel of the 2 x 2 block][pair of output channels]
 #pragma unroll
             for (int p = 0; p < 4; p++)
 #pragma unroll
                 for (int f = 0; f < FW / 2; f++) acc[p][f] = 0ull;
             for (int i = i0; i < i1; i++, wc += 9 * g.OP, patch += bplane) {
-                f32x2 v[4][4];
+                f32x2 v[PR][PC];
 #pragma unroll
-                for (int r = 0; r < 4; r++) {
-                    const float2 u = *reinterpret_cast<const float2 *>(patch + r * g.pitch), t = *reinterpret_cast<const float2 *>(patch + r * g.pitch + 2);
-                    v[r][0] = pack2(u.x, u.x); v[r][1] = pack2(u.y, u.y); v[r][2] = pack2(t.x, t.x); v[r][3] = pack2(t.y, t.y);
-                }
+                for (int r = 0; r < PR; r++)
+#pragma unroll
+                    for (int j = 0; j < PC; j += 2) {
+                        const float2 u = *reinterpret_cast<const float2 *>(patch + r * g.pitch + j);
+                        v[r][j] = pack2(u.x, u.x); v[r][j + 1] = pack2(u.y, u.y);
+                    }
 #pragma unroll
                 for (int t = 0; t < 9; t++)
 #pragma unroll
@@ -134,8 +151,8 @@ __global__ void __launch_bounds__(256) conv3x3_small_kernel(SmallSource src, con
                         const ulonglong2 w2 = *reinterpret_cast<const ulonglong2 *>(wc + t * g.OP + 4 * f);
 #pragma unroll
                         for (int p = 0; p < 4; p++) {
-                            acc[p][2 * f] = ffma2(v[(p >> 1) + t / 3][(p & 1) + t % 3], w2.x, acc[p][2 * f]);
-                            acc[p][2 * f + 1] = ffma2(v[(p >> 1) + t / 3][(p & 1) + t % 3], w2.y, acc[p][2 * f + 1]);
+                            acc[p][2 * f] = ffma2(v[(p >> 1) * ST + t / 3][(p & 1) * ST + t % 3], w2.x, acc[p][2 * f]);
+                            acc[p][2 * f + 1] = ffma2(v[(p >> 1) * ST + t / 3][(p & 1) * ST + t % 3], w2.y, acc[p][2 * f + 1]);
                         }
                     }
             }
@@ -160,23 +177,34 @@ __global__ void __launch_bounds__(256) conv3x3_small_kernel(SmallSource src, con
             if (w < windows && mine && !part) {
                 const int oh = 2 * (q0 + qr), ow = 2 * qc;
                 float *yo = Y + ((long long)n * g.O + o0) * oplane + (long long)oh * g.OW + ow;
+                float z[4][FW];
+#pragma unroll
+                for (int p = 0; p < 4; p++)
+#pragma unroll
+                    for (int f = 0; f < FW; f += 2) {
+                        unpack2(acc[p][f >> 1], z[p][f], z[p][f + 1]);
+                        z[p][f] = epilogue_act(z[p][f] + bk[o0 + f], act);
+                        z[p][f + 1] = epilogue_act(z[p][f + 1] + bk[o0 + f + 1], act);
+                    }
 #pragma unroll
                 for (int f = 0; f < FW; f++, yo += oplane) {
                     if (o0 + f >= g.O) break;
-                    float z[4];
+                    if (pairs) {
+                        *reinterpret_cast<float2 *>(yo) = make_float2(z[0][f], z[1][f]);
+                        if (oh + 1 < g.OH) *reinterpret_cast<float2 *>(yo + g.OW) = make_float2(z[2][f], z[3][f]);
+                    } else {
+                        yo[0] = z[0][f];
+                        if (ow + 1 < g.OW) yo[1] = z[1][f];
+                        if (oh + 1 < g.OH) { yo[g.OW] = z[2][f]; if (ow + 1 < g.OW) yo[g.OW + 1] = z[3][f]; }
+                    }
+                }
+                if (FW >= 8 && cc.p[0]) {
 #pragma unroll
                     for (int p = 0; p < 4; p++) {
-                        float lo, hi;
-                        unpack2(acc[p][f >> 1], lo, hi);
-                        z[p] = epilogue_act(((f & 1) ? hi : lo) + bk[o0 + f], act);
-                    }
-                    if (pairs) {
-                        *reinterpret_cast<float2 *>(yo) = make_float2(z[0], z[1]);
-                        if (oh + 1 < g.OH) *reinterpret_cast<float2 *>(yo + g.OW) = make_float2(z[2], z[3]);
-                    } else {
-                        yo[0] = z[0];
-                        if (ow + 1 < g.OW) yo[1] = z[1];
-                        if (oh + 1 < g.OH) { yo[g.OW] = z[2]; if (ow + 1 < g.OW) yo[g.OW + 1] = z[3]; }
+                        if (oh + (p >> 1) >= g.OH || ow + (p & 1) >= g.OW) continue;
+                        const long long c = ((long long)n * oplane + (long long)(oh + (p >> 1)) * g.OW + ow + (p & 1)) * cc.Cp + o0;
+#pragma unroll
+                        for (int h = 0; h + 8 <= FW; h += 8) store_split8_n(z[p] + h, cc.ns, cc.enc, cc.p[0] + c + h, cc.p[1] + c + h, cc.p[2] + c + h);
                     }
                 }
             }
@@ -185,37 +213,69 @@ __global__ void __launch_bounds__(256) conv3x3_small_kernel(SmallSource src, con
     }
 }
 
-static int small_run(const SmallSource &src, const float *Wt, const float *bias, float *Y, int NB, int I, int IH, int IW, int O, int OH, int OW,
-                     int ph, int pw, int reversed, int act, const char *name) {
+template <int FW, int ST>
+static int small_launch(const SmallSource &src, const float *Wt, const float *bias, float *Y, int NB, int I, int IH, int IW, int O, int OH, int OW,
+                        int ph, int pw, int reversed, int act, const SmallCopies &cc, const char *name) {
     SmallGeom g{};
     g.I = I; g.IH = IH; g.IW = IW; g.O = O; g.OH = OH; g.OW = OW; g.ph = ph; g.pw = pw;
     const int wrows = (OH + 1) / 2, cols = (OW + 1) / 2;
-    // four output channels per warp: a small layer has too few 32-window tiles to fill the chip with more
-    constexpr int FW = 4;
     g.OP = (O + FW - 1) / FW * FW; g.groups = g.OP / FW;
-    g.pitch = 2 * cols + 2;
+    g.pitch = 2 * ST * cols + 2;
     // bands of as many window rows as fit 24 KB (at least one), fewer while the blocks would not go round the SMs
     const size_t row = (size_t)I * g.pitch * sizeof(float);
-    int wr = 24 * 1024 > 4 * row ? (int)((24 * 1024 / row - 2) / 2) : 1;
-    if (wr > wrows) wr = wrows;
+    auto rows = [](int wr) { return 2 * ST * wr + 3 - ST; };
+    int wr = 1;
+    while (wr < wrows && rows(wr + 1) * row <= 24 * 1024) wr++;
     while (wr > 1 && (long long)NB * ((wrows + wr - 1) / wr) < rt().sm_count) wr = (wr + 1) / 2;
-    g.window_rows = wr; g.rows = 2 * wr + 2; g.per_image = (wrows + wr - 1) / wr;
+    g.window_rows = wr; g.rows = rows(wr); g.per_image = (wrows + wr - 1) / wr;
     g.by_bands = fast_div(g.per_image); g.by_pitch = fast_div(g.pitch); g.by_rows = fast_div(g.rows);
     g.by_cols = fast_div(cols); g.by_groups = fast_div(g.groups);
-    const size_t smem = ((size_t)(I * 9 + 1) * g.OP + 8 * 4 * FW * 32) * sizeof(float) + g.rows * row;
+    const size_t smem = ((size_t)(I * 9 + 1) * g.OP + (reversed ? 8 * 4 * FW * 32 : 0)) * sizeof(float) + g.rows * row;
     const int total = NB * g.per_image;
     int grid = rt().sm_count * 4;
     if (grid > total) grid = total;
     profile_begin();
     cudaError_t e = cudaSuccess;
-    if (smem > 48 * 1024) e = cudaFuncSetAttribute(conv3x3_small_kernel<FW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem > 48 * 1024) e = cudaFuncSetAttribute(conv3x3_small_kernel<FW, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess) {
-        conv3x3_small_kernel<FW><<<grid, 256, smem, rt().stream>>>(src, Wt, bias, Y, g, total, reversed, act);
+        conv3x3_small_kernel<FW, ST><<<grid, 256, smem, rt().stream>>>(src, Wt, bias, Y, cc, g, total, reversed, act);
         count_launch();
         e = cudaGetLastError();
     }
     profile_end(2.0 * NB * OH * OW * (double)O * I * 9, name);
     return e == cudaSuccess ? SEERA_OK : check_cuda(e, name);
+}
+// four output channels per warp: a small layer has too few 32-window tiles to fill the chip with more
+static int small_run(const SmallSource &src, const float *Wt, const float *bias, float *Y, int NB, int I, int IH, int IW, int O, int OH, int OW,
+                     int ph, int pw, int reversed, int act, const char *name) {
+    return small_launch<4, 1>(src, Wt, bias, Y, NB, I, IH, IW, O, OH, OW, ph, pw, reversed, act, SmallCopies{}, name);
+}
+
+bool conv_direct_applies(int NB, int C, int H, int W, int F, int R, int S, int sh, int sw, int ph, int pw, bool copies) {
+    // not in the mode of a single bf16 product, whose results are those of rounded operands
+    if (rt().precision < 2 || !rt().conv_tma || R != 3 || S != 3 || sh != sw || sh < 1 || sh > 2 || ph < 0 || pw < 0 || ph > 2 || pw > 2) return false;
+    const long long OH = ((long long)H + 2 * ph - 3) / sh + 1, OW = ((long long)W + 2 * pw - 3) / sw + 1;
+    return NB >= 1 && C >= 1 && C <= 4 && F >= 1 && (size_t)(C * 9 + 1) * (F + 15) * sizeof(float) <= 64 * 1024 && (!copies || F % 8 == 0) &&
+           H + 2 * ph >= 3 && W + 2 * pw >= 3 && (long long)W * C <= 4096 && NB * OH * OW < (1ll << 31) - 64 && (long long)C * H * W < (1ll << 30);
+}
+int conv_direct_fwd(const float *X, const float *Wt, const float *bias, float *Y, int NB, int C, int H, int W, int F, int st, int ph, int pw, int act,
+                    const StorePixelRows *copies, const char *name) {
+    const int OH = (H + 2 * ph - 3) / st + 1, OW = (W + 2 * pw - 3) / st + 1;
+    SmallCopies cc{};
+    if (copies) {
+        for (int i = 0; i < 3; i++) cc.p[i] = copies->cp[i];
+        cc.Cp = copies->Cp; cc.ns = copies->ns; cc.enc = copies->enc;
+    }
+    const SmallSource src{X, nullptr, nullptr, 0};
+    // 16 filters per warp (one read of a value per 16 of them, whole sectors of the copies) where that leaves every scheduler a warp
+    const long long tiles = (long long)NB * ((OH + 1) / 2) * ((OW + 1) / 2) / 32;
+#define SEERA_DIRECT(FW) \
+    (st == 1 ? small_launch<FW, 1>(src, Wt, bias, Y, NB, C, H, W, F, OH, OW, ph, pw, 0, act, cc, name) \
+             : small_launch<FW, 2>(src, Wt, bias, Y, NB, C, H, W, F, OH, OW, ph, pw, 0, act, cc, name))
+    if (F > 8 && (!copies || F % 16 == 0) && tiles * ((F + 15) / 16) >= 4ll * rt().sm_count) return SEERA_DIRECT(16);
+    if (F > 4) return SEERA_DIRECT(8);
+    return SEERA_DIRECT(4);
+#undef SEERA_DIRECT
 }
 
 int conv_small_fwd(const float *X, const float *Wt, const float *bias, float *Y, int NB, int C, int H, int W, int F, int ph, int pw, int act,

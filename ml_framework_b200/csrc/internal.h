@@ -68,6 +68,12 @@ int conv_small_fwd(const float *X, const float *Wt, const float *bias, float *Y,
 bool conv_small_bwd_applies(const float *y, const float *gp, const float *y_pooled, int act);
 int conv_small_bwd(const float *Wt, const float *X, const float *y, const float *g, const float *gp, const int *mask, const float *y_pooled,
                    float *dX, float *dW, float *dbias, int NB, int C, int H, int W, int F, int ph, int pw, int act, const char *name);
+// Forward of a 3 x 3 convolution of stride 1 or 2 with at most four input channels, exact fp32 on the CUDA cores, with channels-last
+// copies of the output on request (conv_small.cu); bias and copies may be null.
+struct StorePixelRows;
+bool conv_direct_applies(int NB, int C, int H, int W, int F, int R, int S, int sh, int sw, int ph, int pw, bool copies);
+int conv_direct_fwd(const float *X, const float *Wt, const float *bias, float *Y, int NB, int C, int H, int W, int F, int st, int ph, int pw, int act,
+                    const StorePixelRows *copies, const char *name);
 // Forward of a "same" 3 x 3 unit-stride convolution with one input channel, direct fp32 (conv_few.cu); bias may be null.
 bool conv_c1_fwd_applies(const float *X, const float *Y, int NB, int C, int H, int W, int F, int R, int S, int sh, int sw, int ph, int pw);
 int conv_c1_fwd(const float *X, const float *Wt, const float *bias, float *Y, int NB, int H, int W, int F, int ph, int act, const char *name);

@@ -71,3 +71,40 @@ def test_small_convolution(shape, mode):
         sc.cuda_free(p)
     sc.set_precision(0)
     assert capi.load().seera_tc_device_status() == 0
+
+
+#         N  C  H   W   F  pad stride
+DIRECT = [(1, 1, 3, 3, 1, 0, 1), (3, 3, 9, 11, 7, 1, 1), (40, 3, 32, 32, 32, 1, 1), (64, 1, 64, 62, 32, 1, 2), (2, 4, 17, 13, 24, 2, 2),
+          (1, 2, 5, 900, 16, 1, 2), (30, 1, 63, 65, 48, 0, 1), (5, 3, 6, 1300, 8, 2, 1)]
+
+
+@pytest.mark.parametrize("mode", [3, 4])
+@pytest.mark.parametrize("shape", DIRECT)
+def test_forward_of_a_layer_with_few_channels(shape, mode):
+    from ml_framework_b200 import capi, seera_cuda as sc
+    sc.init(0)
+    sc.set_precision(mode)
+    N, C, H, W, F, pad, st = shape
+    act = sum(shape) % 3
+    OH, OW = (H + 2 * pad - 3) // st + 1, (W + 2 * pad - 3) // st + 1
+    rs = np.random.RandomState(sum(shape))
+    x, w, b = (rs.standard_normal(s).astype(np.float32) for s in ((N, C, H, W), (F, C, 3, 3), (F,)))
+    xd, wd, bd = (sc.to_device_f32(a.ravel()) for a in (x, w, b))
+    yd = sc.cuda_malloc_f32(N * F * OH * OW)
+    want = activated(co.conv2d_forward(x, w, st, st, pad, pad) + b.reshape(1, F, 1, 1), act)
+    w2d = sc.to_device_f32(rs.standard_normal(5 * F * 25).astype(np.float32))
+    outs = [sc.cuda_malloc_f32(N * 5 * OH * OW) for _ in range(2)]
+    for copies in (True, False):
+        hx, hw, hy = sc.conv2d_bias_act_fwd_k(xd, wd, bd, yd, N, C, H, W, F, 3, 3, pad, pad, st, st, act, 0, copies)
+        # (copies of a number of filters that is no multiple of 8 are the tensor-core kernel's)
+        assert rel_l2(sc.to_host_f32(yd, want.shape), want) < (2e-5 if copies and F % 8 else 2e-6) and not hx and not hw
+        if hy:                      # what a convolution makes of the copies is what it makes of the output itself
+            for o, given in zip(outs, (hy, 0)):
+                sc.shadow_free(sc.conv2d_bias_act_fwd_s(yd, w2d, 0, o, N, F, OH, OW, 5, 5, 5, 2, 2, 1, 1, 0, given))
+            assert np.array_equal(*(sc.to_host_f32(o, (N, 5, OH, OW)) for o in outs))
+            sc.shadow_free(hy)
+        assert bool(hy) == copies or F % 8
+    for p in (xd, wd, bd, yd, w2d, *outs):
+        sc.cuda_free(p)
+    sc.set_precision(0)
+    assert capi.load().seera_tc_device_status() == 0
