@@ -224,23 +224,34 @@ static int make_weight_shadow(const float *Wt, int O, int I, int taps, long long
     return e == cudaSuccess ? SEERA_OK : check_cuda(e, "shadow_weight");
 }
 
-// Filter shadow of one output phase of a strided data gradient: out[o][(t',u')][ip] = W[o*so + i*si + r*S + s] with
-// r = r0 + sh*(Ta-1-t'), s = s0 + sw*(Ub-1-u')  (the taps that reach this phase, flipped), zero for i >= I.
+// Filter copies of all output phases of a strided data gradient, blockIdx.y = phase (a, b) = (y / sw, y % sw), one after the other:
+// out[o][(t',u')][ip] = W[o*so + i*si + r*S + s] with r = r0 + sh*(Ta-1-t'), s = s0 + sw*(Ub-1-u')  (the taps that reach this
+// phase, flipped), zero for i >= I.  A phase holds Ta * Ub of the R * S taps, and starts after those of the phases before it.
+struct PhaseTaps { int r0, Ta, s0, Ub, first; };
+__host__ __device__ inline PhaseTaps phase_taps(int a, int b, int R, int S, int sh, int sw, int ph, int pw) {
+    auto start = [](int x, int pad, int stride) { return (x + pad) % stride; };
+    auto count = [&](int x, int pad, int stride, int K) { const int r = start(x, pad, stride); return r < K ? (K - r + stride - 1) / stride : 0; };
+    PhaseTaps t{start(a, ph, sh), count(a, ph, sh, R), start(b, pw, sw), count(b, pw, sw, S), 0};
+    for (int x = 0; x < a; x++) t.first += count(x, ph, sh, R) * S;          // a row of phases holds every column tap
+    for (int x = 0; x < b; x++) t.first += t.Ta * count(x, pw, sw, S);
+    return t;
+}
 template <int NS>
 __global__ void __launch_bounds__(256) shadow_weight_phase_kernel(const float *__restrict__ Wt, int O, int I, int Ip, long long so, long long si,
-                                                                  int S, int r0, int sh, int Ta, int s0, int sw, int Ub,
+                                                                  int R, int S, int sh, int sw, int ph, int pw,
                                                                   __nv_bfloat16 *__restrict__ d0, __nv_bfloat16 *__restrict__ d1,
                                                                   __nv_bfloat16 *__restrict__ d2, Enc enc) {
-    const int taps = Ta * Ub;
-    long long total = (long long)O * taps * Ip;
+    const PhaseTaps t = phase_taps(blockIdx.y / sw, blockIdx.y % sw, R, S, sh, sw, ph, pw);
+    const int taps = t.Ta * t.Ub;
+    const long long total = (long long)O * taps * Ip, at = (long long)O * t.first * Ip;
     long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x, nthr = (long long)gridDim.x * blockDim.x;
     for (long long e = tid; e < total; e += nthr) {
         int i = (int)(e % Ip); long long t2 = e / Ip;
         int tap = (int)(t2 % taps); int o = (int)(t2 / taps);
-        int tp = tap / Ub, up = tap - tp * Ub;
-        int r = r0 + sh * (Ta - 1 - tp), sx = s0 + sw * (Ub - 1 - up);
+        int tp = tap / t.Ub, up = tap - tp * t.Ub;
+        int r = t.r0 + sh * (t.Ta - 1 - tp), sx = t.s0 + sw * (t.Ub - 1 - up);
         float v = i < I ? __ldg(Wt + o * so + i * si + r * S + sx) : 0.f;
-        store_split1(v, NS, enc, d0 + e, d1 + e, d2 + e);
+        store_split1(v, NS, enc, d0 + at + e, d1 + at + e, d2 + at + e);
     }
 }
 
@@ -383,24 +394,28 @@ static int tma_dgrad_phases(const NhwcShadow &g, const float *Wt, long long so, 
         if (e != cudaSuccess) return check_cuda(e, name);
     }
     const int Ip = g.Cp;
+    Shadow all;                                            // the phases' filters, made in one launch
+    if (int e = alloc_shadow(all, Nch, R * S * Ip, ns)) return e;
+    all.enc = enc_for(CLS_WEIGHT);
+    const int pieces = stride_grid((long long)Nch * R * S * Ip / (sh * sw) + 1);
+    const dim3 wgrid((unsigned)pieces, (unsigned)(sh * sw));
+    if (ns == 1) shadow_weight_phase_kernel<1><<<wgrid, 256, 0, st>>>(Wt, Nch, g.C, Ip, so, si, R, S, sh, sw, ph, pw, all.p[0], all.p[1], all.p[2], all.enc);
+    else if (ns == 2) shadow_weight_phase_kernel<2><<<wgrid, 256, 0, st>>>(Wt, Nch, g.C, Ip, so, si, R, S, sh, sw, ph, pw, all.p[0], all.p[1], all.p[2], all.enc);
+    else shadow_weight_phase_kernel<3><<<wgrid, 256, 0, st>>>(Wt, Nch, g.C, Ip, so, si, R, S, sh, sw, ph, pw, all.p[0], all.p[1], all.p[2], all.enc);
+    count_launch();
+    cudaError_t ce = cudaGetLastError();
+    if (ce != cudaSuccess) { free_shadow(all); return check_cuda(ce, "shadow_weight_phase"); }
     for (int a = 0; a < sh; a++) {
         PhaseAxis y = phase_axis(a, ph, sh, R, H, g.H);
         if (!y.T || !y.G) continue;
         for (int b = 0; b < sw; b++) {
             PhaseAxis x = phase_axis(b, pw, sw, S, W, g.W);
             if (!x.T || !x.G) continue;
-            Shadow wk;
             const int taps = y.T * x.T;
-            if (int e = alloc_shadow(wk, Nch, taps * Ip, ns)) return e;
-            wk.enc = enc_for(CLS_WEIGHT);
-            long long total = (long long)Nch * taps * Ip;
-            int grid = stride_grid(total);
-            if (ns == 1) shadow_weight_phase_kernel<1><<<grid, 256, 0, st>>>(Wt, Nch, g.C, Ip, so, si, S, y.r0, sh, y.T, x.r0, sw, x.T, wk.p[0], wk.p[1], wk.p[2], wk.enc);
-            else if (ns == 2) shadow_weight_phase_kernel<2><<<grid, 256, 0, st>>>(Wt, Nch, g.C, Ip, so, si, S, y.r0, sh, y.T, x.r0, sw, x.T, wk.p[0], wk.p[1], wk.p[2], wk.enc);
-            else shadow_weight_phase_kernel<3><<<grid, 256, 0, st>>>(Wt, Nch, g.C, Ip, so, si, S, y.r0, sh, y.T, x.r0, sw, x.T, wk.p[0], wk.p[1], wk.p[2], wk.enc);
-            count_launch();
-            cudaError_t ce = cudaGetLastError();
-            if (ce != cudaSuccess) { free_shadow(wk); return check_cuda(ce, "shadow_weight_phase"); }
+            Shadow wk = all;
+            wk.cols = wk.ld = taps * Ip;
+            const long long first = (long long)Nch * phase_taps(a, b, R, S, sh, sw, ph, pw).first * Ip;
+            for (int i = 0; i < ns; i++) wk.p[i] = all.p[i] + first;
 
             TmaGemmParams p{};
             p.bias = bias; p.act = act;
@@ -420,10 +435,10 @@ static int tma_dgrad_phases(const NhwcShadow &g, const float *Wt, long long so, 
             }
             double flops = 2.0 * p.M * (double)Nch * g.C * taps;
             if (!e) e = launch_tma_gemm(maps, p, StorePhaseRows{out, Nch, H, W, y.G, x.G, a, b, sh, sw}, ns, false, flops, name);
-            free_shadow(wk);
-            if (e) return e;
+            if (e) { free_shadow(all); return e; }
         }
     }
+    free_shadow(all);
     return SEERA_OK;
 }
 
