@@ -14,7 +14,7 @@
 // output and, for the convolution that reads it, the channels-last copies - of which a lane with 16 filters writes whole sectors, where
 // the tensor-core form is bound by the warps that gather and split patches.  1 -> 32 channels, stride 2, 256 images of 64 x 64 with copies
 // (67 MB): 35 -> 28 us, a third of it waiting for instructions (the straight-line code runs twice per warp); passing the outputs through
-// shared memory to shorten it gave 26 there and cost 2 us where no copies are made.  3 -> 32 channels, 128 images of 32 x 32: 14.6 -> 10.9.
+// shared memory to shorten it gave 26 there and cost 2 us where no copies are made.
 #include "conv_first.cuh"
 #include "contraction_functors.cuh"
 #include "internal.h"
@@ -252,8 +252,10 @@ static int small_run(const SmallSource &src, const float *Wt, const float *bias,
 }
 
 bool conv_direct_applies(int NB, int C, int H, int W, int F, int R, int S, int sh, int sw, int ph, int pw, bool copies) {
-    // not in the mode of a single bf16 product, whose results are those of rounded operands
-    if (rt().precision < 2 || !rt().conv_tma || R != 3 || S != 3 || sh != sw || sh < 1 || sh > 2 || ph < 0 || pw < 0 || ph > 2 || pw > 2) return false;
+    // Not in the mode of a single bf16 product, whose results are those of rounded operands, nor in that of three copies: there the
+    // tensor-core kernel rounds as little as this one, and another order of the sums would move ties of the pools behind the layer (1e-3 of a
+    // first layer's gradient behind a batch normalisation) for 4 us of a step of 300.
+    if (rt().precision < 2 || rt().precision == 3 || !rt().conv_tma || R != 3 || S != 3 || sh != sw || sh < 1 || sh > 2 || ph < 0 || pw < 0 || ph > 2 || pw > 2) return false;
     const long long OH = ((long long)H + 2 * ph - 3) / sh + 1, OW = ((long long)W + 2 * pw - 3) / sw + 1;
     return NB >= 1 && C >= 1 && C <= 4 && F >= 1 && (size_t)(C * 9 + 1) * (F + 15) * sizeof(float) <= 64 * 1024 && (!copies || F % 8 == 0) &&
            H + 2 * ph >= 3 && W + 2 * pw >= 3 && (long long)W * C <= 4096 && NB * OH * OW < (1ll << 31) - 64 && (long long)C * H * W < (1ll << 30);
