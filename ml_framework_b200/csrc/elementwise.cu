@@ -52,6 +52,27 @@ int launch_unary(const float *x, float *out, float *grad, int size, Op op, const
     return SEERA_OK;
 }
 
+// Two copies in one launch.  As two memcpys of 3.1 MB and 40 KB between replays of a graph they took 5.7 + 1.8 us and 15 us of gaps.
+__global__ void __launch_bounds__(256) copy_two_kernel(const float *__restrict__ s0, float *__restrict__ d0, int n0, int vec0,
+                                                       const float *__restrict__ s1, float *__restrict__ d1, int n1, int vec1) {
+    const int tid = blockIdx.x * 256 + threadIdx.x, nthr = gridDim.x * 256;
+    for (int half = 0; half < 2; half++) {
+        const float *s = half ? s1 : s0;
+        float *d = half ? d1 : d0;
+        const int n = half ? n1 : n0, n4 = (half ? vec1 : vec0) ? n >> 2 : 0;
+        const float4 *s4 = reinterpret_cast<const float4 *>(s);
+        float4 *d4 = reinterpret_cast<float4 *>(d);
+        for (long long i = tid; i < n4; i += 4ll * nthr) {
+            float4 v[4];
+#pragma unroll
+            for (int k = 0; k < 4; k++) if (i + (long long)k * nthr < n4) v[k] = __ldg(s4 + i + (long long)k * nthr);
+#pragma unroll
+            for (int k = 0; k < 4; k++) if (i + (long long)k * nthr < n4) d4[i + (long long)k * nthr] = v[k];
+        }
+        for (long long i = 4ll * n4 + tid; i < n; i += nthr) d[i] = s[i];
+    }
+}
+
 // ---- flat binary ---------------------------------------------------------------------------
 struct BAdd { __device__ float operator()(float a, float b) const { return a + b; } };
 struct BSub { __device__ float operator()(float a, float b) const { return a - b; } };
@@ -187,6 +208,18 @@ __global__ void __launch_bounds__(256) concat_kernel(const float *a_, const floa
 }
 
 extern "C" {
+
+int seera_copy_two(void *dst0, const void *src0, int n0, void *dst1, const void *src1, int n1) {
+    SEERA_ENSURE();
+    if (n0 < 0 || n1 < 0 || (n0 && (!dst0 || !src0)) || (n1 && (!dst1 || !src1))) return fail(SEERA_E_ARG, "copy_two: bad argument");
+    if (!n0 && !n1) return SEERA_OK;
+    const int largest = n0 > n1 ? n0 : n1, grid = stride_grid((largest + 15) / 16);
+    copy_two_kernel<<<grid, 256, 0, rt().stream>>>(static_cast<const float *>(src0), static_cast<float *>(dst0), n0, aligned16(src0) && aligned16(dst0),
+                                                   static_cast<const float *>(src1), static_cast<float *>(dst1), n1, aligned16(src1) && aligned16(dst1));
+    SEERA_LAUNCH_CHECK("copy_two");
+    return SEERA_OK;
+}
+
 int seera_cuda_relu_fwd(const float *x, float *o, float *g, int n)    { return launch_unary(x, o, g, n, OpRelu{}, "cuda_relu_fwd"); }
 int seera_cuda_sigmoid_fwd(const float *x, float *o, float *g, int n) { return launch_unary(x, o, g, n, OpSigmoid{}, "cuda_sigmoid_fwd"); }
 int seera_cuda_tanh_fwd(const float *x, float *o, float *g, int n)    { return launch_unary(x, o, g, n, OpTanh{}, "cuda_tanh_fwd"); }

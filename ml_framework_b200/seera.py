@@ -986,8 +986,7 @@ class _RecordedStep:
             self.graph = sc.graph_end()
 
     def load(self, x, y):
-        sc.cuda_memcopy_devicetodevice(self.x.main_ptr, x.main_ptr, self.x.size)
-        sc.cuda_memcopy_devicetodevice(self.y.main_ptr, y.main_ptr, self.y.size)
+        sc.copy_two(self.x.main_ptr, x.main_ptr, self.x.size, self.y.main_ptr, y.main_ptr, self.y.size)
 
     def replay(self):
         sc.graph_set_scalars(self.graph, self.optimizer._scalars())

@@ -222,8 +222,7 @@ class Trainer:
             upload(batch)
         while batch is not None:
             sc.compute_wait_copy()                   # batch i has landed in the staging buffers
-            sc.cuda_memcopy_devicetodevice(X.value.main_ptr, sx.main_ptr, X.value.size)
-            sc.cuda_memcopy_devicetodevice(Y.value.main_ptr, sy.main_ptr, Y.value.size)
+            sc.copy_two(X.value.main_ptr, sx.main_ptr, X.value.size, Y.value.main_ptr, sy.main_ptr, Y.value.size)
             sc.copy_wait_compute()                   # the staging buffers are free again after those two copies
             replay()
             if i:                                    # loss of step i-1: the device is already busy with step i
