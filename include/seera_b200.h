@@ -135,8 +135,9 @@ void *seera_cuda_malloc_i32(int n_elements);        /* :44 */
 void *seera_cuda_malloc_i16(int n_elements);        /* :51 */
 int   seera_cuda_free(void *ptr);                   /* :58  returns the block to the pool           */
 int   seera_cuda_memcopy_devicetodevice(void *dst, const void *src, int num_elem); /* :61 counts FLOAT elements */
-/* two such copies in one launch: a step's inputs and targets into the buffers its recording reads */
-int   seera_copy_two(void *dst0, const void *src0, int n0, void *dst1, const void *src1, int n1);
+/* three such copies in one launch: a step's inputs and targets into the buffers its recording reads, and the loss of the step before out
+ * of the recording's way */
+int   seera_copy_three(void *dst0, const void *src0, int n0, void *dst1, const void *src1, int n1, void *dst2, const void *src2, int n2);
 int   seera_cuda_memset(void *ptr, int value, size_t n_bytes);                     /* :65 */
 int   seera_pool_trim(void);                        /* releases cached blocks to the driver         */
 size_t seera_pool_bytes_reserved(void);

@@ -52,10 +52,12 @@ int launch_unary(const float *x, float *out, float *grad, int size, Op op, const
     return SEERA_OK;
 }
 
-// Two copies in one launch.  As two memcpys of 3.1 MB and 40 KB between replays of a graph they took 5.7 + 1.8 us and 15 us of gaps.
-__global__ void __launch_bounds__(256) copy_two_kernel(const float *__restrict__ s0, float *__restrict__ d0, int n0, int vec0,
-                                                       const float *__restrict__ s1, float *__restrict__ d1, int n1, int vec1) {
+// Three copies in one launch, the last a short one.  As two memcpys of 3.1 MB and 40 KB between replays of a graph they took 5.7 + 1.8 us and 15 us of gaps.
+__global__ void __launch_bounds__(256) copy_three_kernel(const float *__restrict__ s0, float *__restrict__ d0, int n0, int vec0,
+                                                       const float *__restrict__ s1, float *__restrict__ d1, int n1, int vec1,
+                                                       const float *__restrict__ s2, float *__restrict__ d2, int n2) {
     const int tid = blockIdx.x * 256 + threadIdx.x, nthr = gridDim.x * 256;
+    for (int i = tid; i < n2; i += nthr) d2[i] = s2[i];
     for (int half = 0; half < 2; half++) {
         const float *s = half ? s1 : s0;
         float *d = half ? d1 : d0;
@@ -209,14 +211,15 @@ __global__ void __launch_bounds__(256) concat_kernel(const float *a_, const floa
 
 extern "C" {
 
-int seera_copy_two(void *dst0, const void *src0, int n0, void *dst1, const void *src1, int n1) {
+int seera_copy_three(void *dst0, const void *src0, int n0, void *dst1, const void *src1, int n1, void *dst2, const void *src2, int n2) {
     SEERA_ENSURE();
-    if (n0 < 0 || n1 < 0 || (n0 && (!dst0 || !src0)) || (n1 && (!dst1 || !src1))) return fail(SEERA_E_ARG, "copy_two: bad argument");
-    if (!n0 && !n1) return SEERA_OK;
-    const int largest = n0 > n1 ? n0 : n1, grid = stride_grid((largest + 15) / 16);
-    copy_two_kernel<<<grid, 256, 0, rt().stream>>>(static_cast<const float *>(src0), static_cast<float *>(dst0), n0, aligned16(src0) && aligned16(dst0),
-                                                   static_cast<const float *>(src1), static_cast<float *>(dst1), n1, aligned16(src1) && aligned16(dst1));
-    SEERA_LAUNCH_CHECK("copy_two");
+    if (n0 < 0 || n1 < 0 || n2 < 0 || (n0 && (!dst0 || !src0)) || (n1 && (!dst1 || !src1)) || (n2 && (!dst2 || !src2))) return fail(SEERA_E_ARG, "copy_three: bad argument");
+    if (!n0 && !n1 && !n2) return SEERA_OK;
+    const int two = n0 > n1 ? n0 : n1, largest = two > n2 ? two : n2, grid = stride_grid((largest + 15) / 16);
+    copy_three_kernel<<<grid, 256, 0, rt().stream>>>(static_cast<const float *>(src0), static_cast<float *>(dst0), n0, aligned16(src0) && aligned16(dst0),
+                                                   static_cast<const float *>(src1), static_cast<float *>(dst1), n1, aligned16(src1) && aligned16(dst1),
+                                                   static_cast<const float *>(src2), static_cast<float *>(dst2), n2);
+    SEERA_LAUNCH_CHECK("copy_three");
     return SEERA_OK;
 }
 

@@ -53,8 +53,8 @@ PYBIND11_MODULE(seera_cuda, m) {
     m.def("cuda_malloc_i32", [](int n) { return ckp(seera_cuda_malloc_i32(n)); });
     m.def("cuda_malloc_i16", [](int n) { return ckp(seera_cuda_malloc_i16(n)); });
     m.def("cuda_free", [](uptr p) { seera_cuda_free(P<void>(p)); });
-    m.def("copy_two", [](uptr d0, uptr s0, int n0, uptr d1, uptr s1, int n1) {
-        ck(seera_copy_two(P<void>(d0), P<const void>(s0), n0, P<void>(d1), P<const void>(s1), n1)); });
+    m.def("copy_three", [](uptr d0, uptr s0, int n0, uptr d1, uptr s1, int n1, uptr d2, uptr s2, int n2) {
+        ck(seera_copy_three(P<void>(d0), P<const void>(s0), n0, P<void>(d1), P<const void>(s1), n1, P<void>(d2), P<const void>(s2), n2)); });
     m.def("cuda_memcopy_devicetodevice", [](uptr d, uptr s, int n) { ck(seera_cuda_memcopy_devicetodevice(P<void>(d), P<const void>(s), n)); });
     m.def("cuda_memset", [](uptr p, int v, size_t n) { ck(seera_cuda_memset(P<void>(p), v, n)); });
 

@@ -985,8 +985,10 @@ class _RecordedStep:
             optimizer._scalars_in_graph = False
             self.graph = sc.graph_end()
 
-    def load(self, x, y):
-        sc.copy_two(self.x.main_ptr, x.main_ptr, self.x.size, self.y.main_ptr, y.main_ptr, self.y.size)
+    def load(self, x, y, last_loss, kept):
+        """Inputs and targets of the next replay; the loss of the step before goes to the address `kept`, which no replay overwrites."""
+        sc.copy_three(self.x.main_ptr, x.main_ptr, self.x.size, self.y.main_ptr, y.main_ptr, self.y.size,
+                      kept, last_loss.value.main_ptr if last_loss is not None else 0, 0 if last_loss is None else 1)
 
     def replay(self):
         sc.graph_set_scalars(self.graph, self.optimizer._scalars())
@@ -1152,6 +1154,7 @@ class Sequential:
                           "dl": cuten._wrap(sc.cuda_malloc_i32(bs), (bs,), "int32") if labels else None})
         hl = sc.host_alloc_pinned(8)
         slots = sc.host_view(hl, 8).view(np.float32)
+        kept = _new((2,))                       # the losses of two steps, where no replay overwrites them
         history = []
 
         def eager_step(st, m):
@@ -1197,9 +1200,13 @@ class Sequential:
                             recorded = _RecordedStep(self, Optimizer, Loss, (m,) + X_train.shape[1:],
                                                      (m,) if labels else (m,) + y.shape[1:], int(num_classes) if labels else 0)
                         ran_one = True
+                    at, source = 4 * ((k - 1) & 1), None if pending is None else pending.value.main_ptr
                     if m == bs and recorded is not None:
-                        recorded.load(st["dx"], st["dl"] if labels else st["dy"])
-                    sc.copy_wait_compute()          # set (k + 1) % 2 is free once step k - 1 has run
+                        recorded.load(st["dx"], st["dl"] if labels else st["dy"], pending, kept.main_ptr + at)
+                        source = kept.main_ptr + at
+                    sc.copy_wait_compute()          # once step k - 1 has run, set (k + 1) % 2 is free and its loss final
+                    if pending is not None:
+                        sc.copy_download(hl + at, source, 4)
                     if m == bs and recorded is not None:
                         loss = recorded.replay()
                     else:
@@ -1209,9 +1216,9 @@ class Sequential:
                         total += float(slots[(k - 1) & 1])
                     if k + 1 < len(starts):
                         sizes[k + 1] = upload(k + 1)
-                    sc.copy_wait_compute()          # the loss is final once step k has run
-                    sc.copy_download(hl + 4 * (k & 1), loss.value.main_ptr, 4)
                     pending = loss
+                sc.copy_wait_compute()
+                sc.copy_download(hl + 4 * ((len(starts) - 1) & 1), pending.value.main_ptr, 4)
                 sc.copy_synchronize()
                 total += float(slots[(len(starts) - 1) & 1])
                 history.append(total / len(starts))

@@ -207,8 +207,8 @@ class Trainer:
         X, Y, loss = self._graph_keep[:3]
         replay = self.replay_data_parallel if data_parallel else self.replay
         if getattr(self, "_stage", None) is None:
-            self._stage = (S._new(X.value.shape), S._new(Y.value.shape), sc.host_alloc_pinned(8))
-        sx, sy, hl = self._stage
+            self._stage = (S._new(X.value.shape), S._new(Y.value.shape), sc.host_alloc_pinned(8), S._new((2,)))
+        sx, sy, hl, kept = self._stage                 # kept: the losses of two steps, where no replay overwrites them
         slots = (ctypes.c_float * 2).from_address(hl)
         nbx, nby = X.value.size * 4, Y.value.size * 4
 
@@ -222,8 +222,12 @@ class Trainer:
             upload(batch)
         while batch is not None:
             sc.compute_wait_copy()                   # batch i has landed in the staging buffers
-            sc.copy_two(X.value.main_ptr, sx.main_ptr, X.value.size, Y.value.main_ptr, sy.main_ptr, Y.value.size)
-            sc.copy_wait_compute()                   # the staging buffers are free again after those two copies
+            at = 4 * ((i - 1) & 1)
+            sc.copy_three(X.value.main_ptr, sx.main_ptr, X.value.size, Y.value.main_ptr, sy.main_ptr, Y.value.size,
+                          kept.main_ptr + at, loss.value.main_ptr, 1 if i else 0)
+            sc.copy_wait_compute()                   # the staging buffers are free again after those copies, the loss of step i-1 is kept
+            if i:
+                sc.copy_download(hl + at, kept.main_ptr + at, 4)
             replay()
             if i:                                    # loss of step i-1: the device is already busy with step i
                 sc.copy_synchronize()
@@ -231,10 +235,10 @@ class Trainer:
             batch = next(it, None)
             if batch is not None:
                 upload(batch)
-            sc.copy_wait_compute()                   # the loss is final once step i has run
-            sc.copy_download(hl + 4 * (i & 1), loss.value.main_ptr, 4)
             i += 1
         if i:
+            sc.copy_wait_compute()                   # the last loss is final once its step has run
+            sc.copy_download(hl + 4 * ((i - 1) & 1), loss.value.main_ptr, 4)
             sc.copy_synchronize()
             losses.append(float(slots[(i - 1) & 1]))
         return losses

@@ -157,16 +157,17 @@ def test_recordings_made_from_one_another():
 
 
 @pytest.mark.parametrize("n0,n1,shift", [(1, 0, 0), (0, 5, 0), (3, 17, 1), (4096, 10, 0), (1000003, 640, 2), (70, 2000000, 4)])
-def test_two_copies_in_one_launch(n0, n1, shift):
+def test_three_copies_in_one_launch(n0, n1, shift):
     from ml_framework_b200 import seera_cuda as sc
     sc.init(0)
     rs = np.random.RandomState(n0 + n1)
     a, b = (rs.standard_normal(n + shift).astype(np.float32) for n in (n0, n1))
     src = [sc.to_device_f32(t) for t in (np.append(a, 0.0).astype(np.float32), np.append(b, 0.0).astype(np.float32))]
-    dst = [sc.cuda_zeros_f(n + 1) for n in (n0, n1)]
-    sc.copy_two(dst[0], src[0] + 4 * shift, n0, dst[1], src[1] + 4 * shift, n1)
+    dst, last = [sc.cuda_zeros_f(n + 1) for n in (n0, n1)], sc.cuda_zeros_f(2)
+    sc.copy_three(dst[0], src[0] + 4 * shift, n0, dst[1], src[1] + 4 * shift, n1, last, src[0], 1)
     for d, t, n in ((dst[0], a, n0), (dst[1], b, n1)):
         got = sc.to_host_f32(d, (n + 1,))
         assert np.array_equal(got[:n], t[shift:]) and got[n] == 0
-    for p in src + dst:
+    assert np.array_equal(sc.to_host_f32(last, (2,)), [np.append(a, 0.0).astype(np.float32)[0], 0])
+    for p in src + dst + [last]:
         sc.cuda_free(p)
