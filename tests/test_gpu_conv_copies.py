@@ -28,7 +28,7 @@ def slope(y, act):
 
 
 #         N  C  H  W   F  R  S  pad stride
-CONVS = [(1, 8, 5, 6, 8, 1, 1, 0, 1), (2, 72, 9, 7, 66, 3, 3, 1, 1), (3, 17, 12, 13, 130, 3, 3, 0, 1), (2, 64, 11, 9, 40, 5, 3, 2, 1),
+CONVS = [(1, 8, 5, 6, 8, 1, 1, 0, 1), (3, 70, 4, 4, 40, 3, 3, 1, 1), (2, 72, 9, 7, 66, 3, 3, 1, 1), (3, 17, 12, 13, 130, 3, 3, 0, 1), (2, 64, 11, 9, 40, 5, 3, 2, 1),
          (2, 24, 12, 12, 33, 3, 3, 1, 2),        # strided: no filters kept
          (4, 3, 20, 16, 24, 3, 3, 1, 1), (2, 1, 12, 15, 17, 5, 5, 2, 1)]        # short patches: the copies of y by the first-layer kernel
 
