@@ -171,3 +171,30 @@ def test_three_copies_in_one_launch(n0, n1, shift):
     assert np.array_equal(sc.to_host_f32(last, (2,)), [np.append(a, 0.0).astype(np.float32)[0], 0])
     for p in src + dst + [last]:
         sc.cuda_free(p)
+
+
+@pytest.mark.parametrize("transposed", [False, True])
+def test_gradient_entries_submitted_as_one_batch(transposed):
+    """The first call of a shape launches one by one, later ones as a batch: the same bits, other addresses, other operands, no data gradient."""
+    from ml_framework_b200 import seera_cuda as sc
+    sc.init(0)
+    for mode in (1, 3, 4):
+        sc.set_precision(mode)
+        N, C, H, W, F = 3, 20, 9, 11, 24
+        call = sc.cuda_conv2DTranspose_bwd if transposed else sc.cuda_conv2d_bwd
+        got = []
+        for k in range(5):
+            rs = np.random.RandomState(7 + k % 2)
+            ci, co = (C, F)
+            x, g = (rs.standard_normal((N, c, H, W)).astype(np.float32) for c in (ci, co))
+            w = rs.standard_normal((C, F, 3, 3) if transposed else (F, C, 3, 3)).astype(np.float32)
+            hold = sc.cuda_malloc_f32(1000 * (k + 1))                    # other addresses than the call before
+            d = [sc.to_device_f32(a.ravel()) for a in (w, x, g)]
+            dx, dw = sc.cuda_malloc_f32(x.size), sc.cuda_malloc_f32(w.size)
+            call(d[0], d[1], d[2], dx if k < 4 else 0, dw, N, C, H, W, F, 3, 3, 1, 1, 1, 1)
+            got.append((sc.to_host_f32(dx, x.shape) if k < 4 else None, sc.to_host_f32(dw, w.shape)))
+            for p in d + [dx, dw, hold]:
+                sc.cuda_free(p)
+        assert np.array_equal(got[0][0], got[2][0]) and np.array_equal(got[1][0], got[3][0])
+        assert all(np.array_equal(got[k][1], got[k + 2][1]) for k in range(3)) and not np.array_equal(got[0][1], got[1][1])
+    sc.set_precision(0)
