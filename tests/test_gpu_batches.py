@@ -60,6 +60,8 @@ def test_a_tag_may_bring_other_launches(sc):
         assert np.array_equal(sc.to_host_f32(o, (256,)), 2 * (np.maximum(h, 0) if k % 2 else np.abs(h)))
     with pytest.raises(RuntimeError):
         sc.batch_end()                                       # none is open
+    from ml_framework_b200 import capi
+    capi.load().seera_clear_status()
 
 
 @pytest.mark.parametrize("name,n", [("c1", 5), ("c2", 33), ("c4", 3)])
