@@ -152,13 +152,15 @@ int   seera_graph_destroy(void *graph);
 int   seera_is_capturing(void);
 /* One submission for many launches.  Between batch_begin and batch_end the library's launches are recorded, and batch_end hands
  * them to the device as one graph: about 0.9 us of host time per launch instead of 2.8, and no gaps between them on the device.
- * Everything has been enqueued when batch_end returns, in the order of the calls; the executable graph is kept under `tag` (a
- * hash of whatever decides which launches follow) and updated in place by the next batch of that tag, or built anew where the
- * launches turn out to be others.  Calls that wait, read or write host memory, record events or use another stream first submit
- * what has been recorded; the rest of the batch is then launched call by call, as it is inside a seera_graph_begin recording and
- * while the profile is on.  Batches nest: the outermost one counts. */
+ * Everything has been enqueued when batch_end returns, in the order of the calls.  The executable graph is kept under `tag` and the
+ * number and kinds of the launches, and updated in place by the next such batch: a tag names a kind of pass, whose sizes, kernels and
+ * addresses may differ from time to time.  A limited number is kept; a batch that finds no room is launched call by call.  Calls that
+ * wait, read or write host memory, record events or use another stream first submit what has been recorded; the rest of the batch is
+ * then launched call by call, as it is inside a seera_graph_begin recording and while the profile is on.  Batches nest: the
+ * outermost one counts. */
 int   seera_batch_begin(uint64_t tag);
 int   seera_batch_end(void);
+int   seera_batches_kept(void);                     /* executable graphs kept for further batches */
 /* The scalars of the optimizer updates (seera_adam_step, seera_sgd_step) recorded in a graph: 9 floats lr, beta1, 1 - beta1, beta2,
  * 1 - beta2, eps, c1, c2, grad_scale for Adam, 3 floats lr, momentum, grad_scale for SGD.  Takes effect with the next launch. */
 int   seera_graph_set_scalars(void *graph, const float *values, int n);

@@ -151,6 +151,11 @@ static void profile_collect() {
 // A launch costs the host about 2.8 us here; recorded into a stream capture it costs 0.25, and bringing a kept executable graph
 // up to date with the recording another 0.45 per kernel (50 kernels: 47 us against 121 launched one by one, and the device runs
 // them without the 1-2 us between separate launches).
+//
+// An update can change grids, arguments and kernels, but not how many nodes there are or what kind each is: executables are kept by the
+// caller's tag and that.  A recording for which there is none is given one while there is room; from then on it replaces one that
+// BATCH_STALE batches have passed over, and where there is no such it is launched node by node, at what its launches would have cost
+// without a batch.  Nothing here waits for the device: an executable graph that is destroyed while it runs is freed when it ends.
 namespace {
 struct BatchState {
     int depth = 0;
@@ -158,54 +163,146 @@ struct BatchState {
     uint64_t tag = 0;
     cudaStream_t stream = nullptr;
     struct Exec { cudaGraphExec_t exec; uint64_t used; };
-    std::unordered_map<uint64_t, Exec> kept;            // by tag and number of nodes
+    std::unordered_map<uint64_t, Exec> kept;            // by tag and kinds of nodes
     uint64_t clock = 0;
 };
-constexpr size_t BATCH_KEPT_MAX = 64;                   // executable graphs kept; the one unused for longest goes first
+constexpr size_t BATCH_KEPT_MAX = 64;
+constexpr uint64_t BATCH_STALE = 1024;                  // making and destroying an executable (125 + 110 us for 14 launches) per so many batches
 BatchState &batch() { static BatchState b; return b; }
-}  // namespace
 
-int batch_flush() {
+// The nodes of a graph in order, if each follows the one before it; else nothing.
+std::vector<cudaGraphNode_t> chain_of(cudaGraph_t g) {
+    std::vector<cudaGraphNode_t> order;
+    size_t nodes = 0, edges = 0, roots = 1;
+    cudaGraphNode_t at = nullptr;
+    if (cudaGraphGetNodes(g, nullptr, &nodes) != cudaSuccess || cudaGraphGetEdges(g, nullptr, nullptr, &edges) != cudaSuccess ||
+        !nodes || edges != nodes - 1 || cudaGraphGetRootNodes(g, nullptr, &roots) != cudaSuccess || roots != 1 ||
+        cudaGraphGetRootNodes(g, &at, &roots) != cudaSuccess) {
+        cudaGetLastError();
+        return order;
+    }
+    std::vector<cudaGraphNode_t> from(edges), to(edges);
+    if (edges && cudaGraphGetEdges(g, from.data(), to.data(), &edges) != cudaSuccess) { cudaGetLastError(); return order; }
+    std::vector<std::pair<cudaGraphNode_t, cudaGraphNode_t>> next(edges);
+    for (size_t i = 0; i < edges; i++) next[i] = {from[i], to[i]};
+    std::sort(next.begin(), next.end());
+    while (at) {
+        order.push_back(at);
+        auto it = std::lower_bound(next.begin(), next.end(), std::make_pair(at, cudaGraphNode_t(nullptr)));
+        at = it != next.end() && it->first == at && order.size() < nodes ? it->second : nullptr;
+    }
+    if (order.size() != nodes) order.clear();           // something has two successors
+    return order;
+}
+
+// One node as a launch of its own.
+cudaError_t launch_node(cudaGraphNode_t node, cudaStream_t st) {
+    cudaGraphNodeType type;
+    cudaError_t e = cudaGraphNodeGetType(node, &type);
+    if (e != cudaSuccess || type == cudaGraphNodeTypeEmpty) return e;
+    if (type == cudaGraphNodeTypeKernel) {
+        cudaKernelNodeParams kp = {};
+        cudaKernelNodeAttrValue v = {};
+        if ((e = cudaGraphKernelNodeGetParams(node, &kp)) != cudaSuccess) return e;
+        if ((e = cudaGraphKernelNodeGetAttribute(node, cudaLaunchAttributeClusterDimension, &v)) != cudaSuccess) return e;
+        cudaLaunchConfig_t cfg = {};
+        cudaLaunchAttribute attr[1];
+        cfg.gridDim = kp.gridDim; cfg.blockDim = kp.blockDim; cfg.dynamicSmemBytes = kp.sharedMemBytes; cfg.stream = st;
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val = v;
+        cfg.attrs = attr; cfg.numAttrs = v.clusterDim.x > 1 ? 1 : 0;
+        return cudaLaunchKernelExC(&cfg, kp.func, kp.kernelParams);
+    }
+    if (type == cudaGraphNodeTypeMemset) {
+        cudaMemsetParams mp = {};
+        if ((e = cudaGraphMemsetNodeGetParams(node, &mp)) != cudaSuccess) return e;
+        return mp.height > 1 ? cudaMemset2DAsync(mp.dst, mp.pitch, (int)(mp.value & 255), mp.width * mp.elementSize, mp.height, st)
+                             : cudaMemsetAsync(mp.dst, (int)(mp.value & 255), mp.width * mp.elementSize, st);
+    }
+    cudaMemcpy3DParms cp = {};
+    if ((e = cudaGraphMemcpyNodeGetParams(node, &cp)) != cudaSuccess) return e;
+    return cudaMemcpy3DAsync(&cp, st);
+}
+// Whether launch_node can: kernels, copies, and fills with one byte.
+bool launches_alone(cudaGraphNode_t node) {
+    cudaGraphNodeType type;
+    if (cudaGraphNodeGetType(node, &type) != cudaSuccess) { cudaGetLastError(); return false; }
+    if (type != cudaGraphNodeTypeMemset) return type == cudaGraphNodeTypeKernel || type == cudaGraphNodeTypeMemcpy || type == cudaGraphNodeTypeEmpty;
+    cudaMemsetParams mp = {};
+    if (cudaGraphMemsetNodeGetParams(node, &mp) != cudaSuccess) { cudaGetLastError(); return false; }
+    const unsigned byte = mp.value & 255u;
+    return mp.value == (mp.elementSize == 4 ? byte * 0x01010101u : (mp.elementSize == 2 ? byte * 0x0101u : byte));
+}
+}  // namespace
+static std::vector<cudaGraphNode_t> nodes_of(cudaGraph_t g) {
+    size_t n = 0;
+    std::vector<cudaGraphNode_t> v;
+    if (cudaGraphGetNodes(g, nullptr, &n) == cudaSuccess && n) {
+        v.resize(n);
+        if (cudaGraphGetNodes(g, v.data(), &n) != cudaSuccess) v.clear();
+    }
+    return v;
+}
+
+// Hands over what an open batch has recorded.  `keep`: a recording of a whole batch, whose executable is worth keeping.
+static int batch_submit(bool keep) {
     BatchState &b = batch();
     if (!b.open) return SEERA_OK;
     b.open = false;
     cudaGraph_t g = nullptr;
     if (int s = check_cuda(cudaStreamEndCapture(b.stream, &g), "batch: cudaStreamEndCapture")) { cudaGetLastError(); return s; }
-    size_t n = 0;
-    cudaError_t e = cudaGraphGetNodes(g, nullptr, &n);
-    if (e == cudaSuccess && n) {
-        const uint64_t key = b.tag ^ (0x9E3779B97F4A7C15ull * (uint64_t)n);
+    cudaError_t e = cudaSuccess;
+    const std::vector<cudaGraphNode_t> nodes = nodes_of(g);
+    if (!nodes.empty()) {
+        uint64_t key = b.tag ^ (0x9E3779B97F4A7C15ull * (uint64_t)nodes.size());
+        for (size_t i = 0; i < nodes.size(); i++) {
+            cudaGraphNodeType type = cudaGraphNodeTypeKernel;
+            cudaGraphNodeGetType(nodes[i], &type);
+            if (type != cudaGraphNodeTypeKernel) key = (key ^ (i * 16 + (uint64_t)type)) * 1099511628211ull;
+        }
+        ++b.clock;
         auto it = b.kept.find(key);
         if (it != b.kept.end()) {
             cudaGraphExecUpdateResultInfo info;
-            if (cudaGraphExecUpdate(it->second.exec, g, &info) != cudaSuccess) {      // other launches under the same tag
+            if (cudaGraphExecUpdate(it->second.exec, g, &info) != cudaSuccess) {
                 cudaGetLastError();
-                cudaStreamSynchronize(b.stream);
                 cudaGraphExecDestroy(it->second.exec);
                 b.kept.erase(it);
                 it = b.kept.end();
+                keep = false;
             }
         }
-        if (it == b.kept.end()) {
-            if (b.kept.size() >= BATCH_KEPT_MAX) {
+        if (it != b.kept.end()) {
+            it->second.used = b.clock;
+            e = cudaGraphLaunch(it->second.exec, b.stream);
+        } else {
+            const std::vector<cudaGraphNode_t> chain = chain_of(g);
+            if (chain.empty()) keep = false;
+            if (keep && b.kept.size() >= BATCH_KEPT_MAX) {
                 auto old = b.kept.begin();
                 for (auto i = b.kept.begin(); i != b.kept.end(); ++i) if (i->second.used < old->second.used) old = i;
-                cudaStreamSynchronize(b.stream);
-                cudaGraphExecDestroy(old->second.exec);
-                b.kept.erase(old);
+                if (b.clock - old->second.used > BATCH_STALE) {
+                    cudaGraphExecDestroy(old->second.exec);
+                    b.kept.erase(old);
+                } else {
+                    keep = false;
+                }
             }
-            cudaGraphExec_t x = nullptr;
-            e = cudaGraphInstantiate(&x, g, 0);
-            if (e == cudaSuccess) it = b.kept.emplace(key, BatchState::Exec{x, 0}).first;
-        }
-        if (e == cudaSuccess) {
-            it->second.used = ++b.clock;
-            e = cudaGraphLaunch(it->second.exec, b.stream);
+            if (!keep && !chain.empty() && std::all_of(chain.begin(), chain.end(), launches_alone)) {
+                for (size_t i = 0; i < chain.size() && e == cudaSuccess; i++) e = launch_node(chain[i], b.stream);
+            } else {
+                cudaGraphExec_t x = nullptr;
+                e = cudaGraphInstantiate(&x, g, 0);
+                if (e == cudaSuccess) e = cudaGraphLaunch(x, b.stream);
+                if (x && keep) b.kept.emplace(key, BatchState::Exec{x, b.clock});
+                else if (x) cudaGraphExecDestroy(x);
+            }
         }
     }
     cudaGraphDestroy(g);
     return e == cudaSuccess ? SEERA_OK : check_cuda(e, "batch");
 }
+int batch_flush() { return batch_submit(false); }
 
 // An optimizer update is being recorded into the open capture: its node is the one the stream's next work will depend on.
 void graph_note_optimizer(const OptLaunch &launch) {
@@ -233,18 +330,6 @@ struct Spare {
 };
 std::vector<Spare> &spares() { static std::vector<Spare> v; return v; }
 }  // namespace
-static size_t chain_length(cudaGraph_t g) {
-    size_t nodes = 0, edges = 0, roots = 0;
-    if (cudaGraphGetNodes(g, nullptr, &nodes) != cudaSuccess || cudaGraphGetEdges(g, nullptr, nullptr, &edges) != cudaSuccess ||
-        cudaGraphGetRootNodes(g, nullptr, &roots) != cudaSuccess || !nodes || roots != 1 || edges != nodes - 1) {
-        cudaGetLastError();
-        return 0;
-    }
-    std::vector<cudaGraphNode_t> from(edges), to(edges);
-    if (edges && cudaGraphGetEdges(g, from.data(), to.data(), &edges) != cudaSuccess) { cudaGetLastError(); return 0; }
-    std::sort(from.begin(), from.end());
-    return std::adjacent_find(from.begin(), from.end()) == from.end() ? nodes : 0;       // nothing has two successors
-}
 static void spares_trim(size_t keep) {
     auto &v = spares();
     while (v.size() > keep) {
@@ -538,7 +623,7 @@ void *seera_graph_end(void) {
     rt().launches = g->launches_at_begin;               // recorded, not executed
     cudaError_t e = cudaStreamEndCapture(rt().stream, &g->graph);
     if (e == cudaSuccess && !g->collectives) {
-        g->chain = chain_length(g->graph);
+        g->chain = chain_of(g->graph).size();
         if (g->chain) take_spare(g);
     }
     if (e == cudaSuccess && !g->exec) e = cudaGraphInstantiate(&g->exec, g->graph, 0);
@@ -609,10 +694,11 @@ int seera_batch_begin(uint64_t tag) {
     b.stream = rt().stream;
     return SEERA_OK;
 }
+int seera_batches_kept(void) { return (int)batch().kept.size(); }
 int seera_batch_end(void) {
     BatchState &b = batch();
     if (b.depth == 0) return fail(SEERA_E_ARG, "batch_end: no batch is open");
-    return --b.depth ? SEERA_OK : batch_flush();
+    return --b.depth ? SEERA_OK : batch_submit(true);
 }
 
 // Page-locked host blocks.  The driver takes milliseconds to pin and unpin a block (3 ms for 200 KB measured; a training loop of

@@ -183,6 +183,7 @@ PYBIND11_MODULE(seera_cuda, m) {
     m.def("graph_destroy", [](uptr g) { ck(seera_graph_destroy(P<void>(g))); });
     m.def("batch_begin", [](uint64_t tag) { ck(seera_batch_begin(tag)); });
     m.def("batch_end", []() { ck(seera_batch_end()); });
+    m.def("batches_kept", []() { return seera_batches_kept(); });
     m.def("graph_set_scalars", [](uptr g, const std::vector<float> &v) { ck(seera_graph_set_scalars(P<void>(g), v.data(), (int)v.size())); });
     m.def("is_capturing", []() { return seera_is_capturing() != 0; });
     m.def("cuda_adam_step_dev", [](uptr w, uptr g, uptr mm, uptr v, int n, uptr h) {

@@ -200,3 +200,65 @@ def test_gradient_entries_submitted_as_one_batch(transposed):
         assert np.array_equal(got[0][0], got[2][0]) and np.array_equal(got[1][0], got[3][0])
         assert all(np.array_equal(got[k][1], got[k + 2][1]) for k in range(3)) and not np.array_equal(got[0][1], got[1][1])
     sc.set_precision(0)
+
+
+def test_more_kinds_of_batches_than_are_kept(sc):
+    """Beyond the executables that are kept a batch is launched node by node: kernels (some of them clusters), fills and copies."""
+    n, m = 1000, 256
+    rs = np.random.RandomState(3)
+    a, b = (rs.standard_normal((m, m)).astype(np.float32) for _ in range(2))
+    da, db, dc = sc.to_device_f32(a), sc.to_device_f32(b), sc.cuda_malloc_f32(m * m)
+    sc.set_precision(1)
+    try:
+        for pair in (0, 1):
+            sc.set_option("pair_tiles", pair)
+            sc.cuda_matmul(da, db, dc, m, m, m, 1)
+            want = sc.to_host_f32(dc, (m, m))
+            for rep in range(2):
+                for tag in range(100):
+                    p, q = sc.cuda_ones_f(n), sc.cuda_malloc_f32(n)
+                    sc.cuda_memset(dc, 255, 4 * m * m)
+                    sc.batch_begin((1000 << 8) + tag)
+                    sc.cuda_memset(q, 0, 4 * n)
+                    sc.cuda_scaler_add_f(p, float(tag), n)
+                    sc.cuda_memcopy_devicetodevice(q, p, n // 2)
+                    sc.cuda_scaler_multiply_f(q, 2.0, n)
+                    sc.cuda_matmul(da, db, dc, m, m, m, 1)
+                    sc.batch_end()
+                    assert sc.batches_kept() <= 64
+                    got = sc.to_host_f32(q, (n,))
+                    assert np.all(got[:n // 2] == 2 * (tag + 1)) and np.all(got[n // 2:] == 0)
+                    assert np.array_equal(sc.to_host_f32(dc, (m, m)), want)
+                    sc.cuda_free(p)
+                    sc.cuda_free(q)
+    finally:
+        sc.set_option("pair_tiles", 0)
+        sc.set_precision(0)
+        for p in (da, db, dc):
+            sc.cuda_free(p)
+
+
+def test_predictions_over_more_sizes_than_executables_are_kept(sc, monkeypatch):
+    """A server's batches: no size waits for another's executable.  The time allows a quarter over launches made one by one."""
+    import time
+    from ml_framework_b200 import seera as S, train, workloads as wl
+    sc.set_precision(3)
+    work = wl.WORKLOADS["c1"]()
+    model = train.build_model(work, work.params(1))
+    xs = [S.Tensor(work.batch(n, n)[0], is_leaf=True) for n in range(1, 121)]
+    before, took, got = sc.batches_kept(), [], []
+    for batched in (False, True):
+        monkeypatch.setattr(S, "_batch_begin", sc.batch_begin if batched else None)
+        best = 1e9
+        for rep in range(4):
+            sc.stream_synchronize()
+            t = time.perf_counter()
+            out = [model.predict(x) for x in xs]
+            sc.stream_synchronize()
+            if rep:
+                best = min(best, time.perf_counter() - t)
+        took.append(best)
+        got.append([o.to_numpy() for o in out])
+    assert all(np.array_equal(a, b) for a, b in zip(*got))
+    assert sc.batches_kept() - before <= 12
+    assert took[1] <= 1.25 * took[0], took
