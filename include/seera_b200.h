@@ -139,7 +139,9 @@ int   seera_cuda_memcopy_devicetodevice(void *dst, const void *src, int num_elem
  * of the recording's way */
 int   seera_copy_three(void *dst0, const void *src0, int n0, void *dst1, const void *src1, int n1, void *dst2, const void *src2, int n2);
 int   seera_cuda_memset(void *ptr, int value, size_t n_bytes);                     /* :65 */
-int   seera_pool_trim(void);                        /* releases cached blocks to the driver         */
+/* Releases to the driver what is cached for later calls: device and page-locked blocks, executable graphs of batches and of
+ * destroyed recordings.  Waits for the stream. */
+int   seera_pool_trim(void);
 size_t seera_pool_bytes_reserved(void);
 /* Stream capture of a whole step into a CUDA graph.  Between graph_begin and graph_end every call of this
  * library is recorded instead of executed; blocks the recorded work allocates stay reserved for the graph

@@ -589,6 +589,8 @@ int seera_pool_trim(void) {
         for (void *b : kv.second) { cudaFree(b); p.reserved -= kv.first; }
         kv.second.clear();
     }
+    for (auto &kv : batch().kept) cudaGraphExecDestroy(kv.second.exec);
+    batch().kept.clear();
     spares_trim(0);
     pinned_trim();
     return SEERA_OK;

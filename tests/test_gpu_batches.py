@@ -262,3 +262,18 @@ def test_predictions_over_more_sizes_than_executables_are_kept(sc, monkeypatch):
     assert all(np.array_equal(a, b) for a, b in zip(*got))
     assert sc.batches_kept() - before <= 12
     assert took[1] <= 1.25 * took[0], took
+
+
+def test_trimming_gives_back_the_executables_of_batches(sc):
+    for rep in range(3):
+        p = sc.cuda_ones_f(100)
+        for k in (2, 3):
+            sc.batch_begin(21)
+            for i in range(k):
+                sc.cuda_scaler_add_f(p, 1.0, 100)
+            sc.batch_end()
+        assert sc.batches_kept() >= 2
+        sc.pool_trim()                                       # the last batch may still be running
+        assert sc.batches_kept() == 0
+        assert np.all(sc.to_host_f32(p, (100,)) == 6)
+        sc.cuda_free(p)
