@@ -543,6 +543,9 @@ void *seera_cuda_malloc(size_t n_bytes) {
         if (p.capturing) { p.owner[b] = p.cur; p.cur->blocks.push_back({b, sz}); }
         return b;
     }
+    // A pass that has to grow the pool (a new model's first) runs launch by launch from here: held back, its launches would wait out
+    // every cudaMalloc of the pass, where the device can work through them meanwhile.
+    if (batch_flush()) return nullptr;
     void *b = nullptr;
     cudaError_t e = cudaMalloc(&b, sz);
     if (e != cudaSuccess) {            // give cached blocks back to the driver and retry once

@@ -277,3 +277,29 @@ def test_trimming_gives_back_the_executables_of_batches(sc):
         assert sc.batches_kept() == 0
         assert np.all(sc.to_host_f32(p, (100,)) == 6)
         sc.cuda_free(p)
+
+
+def _is_recording(stream):
+    import ctypes
+    status = ctypes.c_int(-1)
+    assert ctypes.CDLL("libcuda.so.1").cuStreamIsCapturing(ctypes.c_void_p(stream), ctypes.byref(status)) == 0
+    return status.value != 0
+
+
+def test_a_batch_that_grows_the_pool_goes_on_launch_by_launch(sc):
+    """The device works through what came before while the driver looks for memory; blocks at hand leave the batch together."""
+    stream, n = sc.get_stream(), (37 << 20) // 4
+    sc.pool_trim()
+    for rep in range(2):
+        p = sc.cuda_ones_f(100)
+        sc.batch_begin(22)
+        sc.cuda_scaler_add_f(p, 1.0, 100)
+        assert _is_recording(stream)
+        q = sc.cuda_malloc_f32(n)                            # from the driver the first time, from the pool the second
+        assert _is_recording(stream) == (rep == 1)
+        sc.cuda_memset(q, 0, 4 * n)
+        sc.cuda_scaler_add_f(p, 1.0, 100)
+        sc.batch_end()
+        assert np.all(sc.to_host_f32(p, (100,)) == 3) and not sc.to_host_f32(q, (n,)).any()
+        sc.cuda_free(p)
+        sc.cuda_free(q)
