@@ -159,7 +159,7 @@ int   seera_is_capturing(void);
  * addresses may differ from time to time.  A limited number is kept; a batch that finds no room is launched call by call.  Calls that
  * wait, read or write host memory, record events or use another stream first submit what has been recorded; the rest of the batch is
  * then launched call by call, as it is inside a seera_graph_begin recording and while the profile is on.  Batches nest: the
- * outermost one counts. */
+ * outermost one counts, and where it found the device idle a longer inner one is submitted at its own end. */
 int   seera_batch_begin(uint64_t tag);
 int   seera_batch_end(void);
 int   seera_batches_kept(void);                     /* executable graphs kept for further batches */

@@ -303,3 +303,23 @@ def test_a_batch_that_grows_the_pool_goes_on_launch_by_launch(sc):
         assert np.all(sc.to_host_f32(p, (100,)) == 3) and not sc.to_host_f32(q, (n,)).any()
         sc.cuda_free(p)
         sc.cuda_free(q)
+
+
+@pytest.mark.parametrize("k,parts", [(11, 1), (12, 2), (40, 2)])
+def test_an_idle_device_gets_a_long_inner_batch_at_its_end(sc, k, parts):
+    for rep in range(3):
+        p = sc.cuda_ones_f(100)
+        sc.stream_synchronize()
+        sc.pool_trim()
+        sc.batch_begin(23)
+        for inner in range(2):                               # after the first part the device has work: the rest goes together
+            sc.batch_begin(24)
+            for i in range(k):
+                sc.cuda_scaler_add_f(p, 1.0, 100)
+            sc.batch_end()
+            assert sc.batches_kept() == parts - 1
+        sc.cuda_scaler_multiply_f(p, 2.0, 100)
+        sc.batch_end()
+        assert sc.batches_kept() == parts
+        assert np.all(sc.to_host_f32(p, (100,)) == 2 * (1 + 2 * k))
+        sc.cuda_free(p)
