@@ -152,27 +152,34 @@ static void profile_collect() {
 // up to date with the recording another 0.45 per kernel (50 kernels: 47 us against 121 launched one by one, and the device runs
 // them without the 1-2 us between separate launches).
 //
-// An update can change grids, arguments and kernels, but not how many nodes there are or what kind each is: executables are kept by the
-// caller's tag and that.  A recording for which there is none is given one while there is room; from then on it replaces one that
-// BATCH_STALE batches have passed over, and where there is no such it is launched node by node, at what its launches would have cost
-// without a batch.  Nothing here waits for the device: an executable graph that is destroyed while it runs is freed when it ends.
+// An update can change grids, arguments and kernels, but not how many nodes there are or what kind each is.  It is not free, though, where it
+// changes kernels: an executable runs its nodes fastest as those it was made of (an autoencoder step of 64 images 236 us, 251 with the
+// executable of a step of 8).  So a batch has one by its tag and number of nodes, while BATCH_KEPT_MAX leave room or one of them has been
+// passed over by BATCH_STALE batches; beyond that, batches of the same kinds of nodes share one, and where those are full as well the batch
+// is launched node by node, at what its launches would have cost without one.  Predictions of a small CNN over 200 batch sizes: 154 us
+// a call when every miss made an executable in place of another, 31 here as launched one by one (VGG 298, 141, 160).  Nothing here waits:
+// an executable graph that is destroyed while it runs is freed when it ends.
 namespace {
 struct BatchState {
     int depth = 0;
     bool open = false;                                  // the stream is being captured
-    bool starved = false;                               // the device had nothing to do when the batch was opened
-    uint64_t tag = 0, launches_at_open = 0;
+    cudaEvent_t last = nullptr;                         // behind the last batch
+    bool parted = false;                                // a first part of it has been submitted
+    uint64_t tag = 0, inner_at = 0;                     // ... and the launch count where the batch directly inside began
     cudaStream_t stream = nullptr;
     struct Exec { cudaGraphExec_t exec; uint64_t used; };
-    std::unordered_map<uint64_t, Exec> kept;            // by tag and kinds of nodes
-    uint64_t clock = 0;
+    std::unordered_map<uint64_t, Exec> kept;            // by tag and number of nodes
+    std::unordered_map<uint64_t, Exec> shared;          // by kinds of nodes
+    uint64_t clock = 0, replaced = 0;                   // batches submitted; when an executable last made room for another
 };
 constexpr size_t BATCH_KEPT_MAX = 64;
-// A pass inside a batch that leaves this many launches behind is submitted at its end if the device was idle when the batch was opened:
-// a step that is waited for would else run host and device one after the other (VGG at 100 images: 557 -> 474 us).  Below that the
+// The first pass inside a batch that makes this many launches is submitted at its end if the device has finished the batch before: a
+// step that is waited for would else run host and device one after the other (VGG at 100 images: 557 -> 474 us).  Below that the
 // second submission (6 us) costs a small network more than the device's head start gives.
 constexpr uint64_t BATCH_PART = 12;
-constexpr uint64_t BATCH_STALE = 1024;                  // making and destroying an executable (125 + 110 us for 14 launches) per so many batches
+// An executable takes 125 us to make and 110 to destroy (14 launches): one in BATCH_TURN batches may go for another.
+constexpr uint64_t BATCH_STALE = 1024, BATCH_TURN = 64;
+constexpr size_t BATCH_SHARED_MAX = 32;
 BatchState &batch() { static BatchState b; return b; }
 
 // The nodes of a graph in order, if each follows the one before it; else nothing.
@@ -238,16 +245,17 @@ bool launches_alone(cudaGraphNode_t node) {
     const unsigned byte = mp.value & 255u;
     return mp.value == (mp.elementSize == 4 ? byte * 0x01010101u : (mp.elementSize == 2 ? byte * 0x0101u : byte));
 }
-}  // namespace
-static std::vector<cudaGraphNode_t> nodes_of(cudaGraph_t g) {
-    size_t n = 0;
-    std::vector<cudaGraphNode_t> v;
-    if (cudaGraphGetNodes(g, nullptr, &n) == cudaSuccess && n) {
-        v.resize(n);
-        if (cudaGraphGetNodes(g, v.data(), &n) != cudaSuccess) v.clear();
+// Number and kinds of the nodes of a chain.
+uint64_t kinds_of(const std::vector<cudaGraphNode_t> &chain) {
+    uint64_t h = chain.size();
+    for (size_t i = 0; i < chain.size(); i++) {
+        cudaGraphNodeType type = cudaGraphNodeTypeKernel;
+        cudaGraphNodeGetType(chain[i], &type);
+        if (type != cudaGraphNodeTypeKernel) h = (h ^ (i * 16 + (uint64_t)type)) * 1099511628211ull;
     }
-    return v;
+    return h;
 }
+}  // namespace
 
 // Hands over what an open batch has recorded.  `keep`: a recording of a whole batch, whose executable is worth keeping.
 static int batch_submit(bool keep) {
@@ -257,54 +265,54 @@ static int batch_submit(bool keep) {
     cudaGraph_t g = nullptr;
     if (int s = check_cuda(cudaStreamEndCapture(b.stream, &g), "batch: cudaStreamEndCapture")) { cudaGetLastError(); return s; }
     cudaError_t e = cudaSuccess;
-    const std::vector<cudaGraphNode_t> nodes = nodes_of(g);
-    if (!nodes.empty()) {
-        uint64_t key = b.tag ^ (0x9E3779B97F4A7C15ull * (uint64_t)nodes.size());
-        for (size_t i = 0; i < nodes.size(); i++) {
-            cudaGraphNodeType type = cudaGraphNodeTypeKernel;
-            cudaGraphNodeGetType(nodes[i], &type);
-            if (type != cudaGraphNodeTypeKernel) key = (key ^ (i * 16 + (uint64_t)type)) * 1099511628211ull;
-        }
+    size_t n = 0;
+    e = cudaGraphGetNodes(g, nullptr, &n);
+    if (e == cudaSuccess && n) {
         ++b.clock;
-        auto it = b.kept.find(key);
-        if (it != b.kept.end()) {
+        // The executable under `key`, brought up to date, or null.
+        auto updated = [&](std::unordered_map<uint64_t, BatchState::Exec> &m, uint64_t key) -> cudaGraphExec_t {
+            auto it = m.find(key);
+            if (it == m.end()) return nullptr;
             cudaGraphExecUpdateResultInfo info;
             if (cudaGraphExecUpdate(it->second.exec, g, &info) != cudaSuccess) {
                 cudaGetLastError();
                 cudaGraphExecDestroy(it->second.exec);
-                b.kept.erase(it);
-                it = b.kept.end();
-                keep = false;
+                m.erase(it);
+                return nullptr;
+            }
+            it->second.used = b.clock;
+            return it->second.exec;
+        };
+        uint64_t key = b.tag ^ (0x9E3779B97F4A7C15ull * (uint64_t)n);
+        cudaGraphExec_t x = updated(b.kept, key);
+        const std::vector<cudaGraphNode_t> chain = x ? std::vector<cudaGraphNode_t>() : chain_of(g);
+        auto *into = &b.kept;
+        if (!x && keep && !chain.empty() && b.kept.size() >= BATCH_KEPT_MAX) {
+            auto old = b.kept.begin();
+            for (auto i = b.kept.begin(); i != b.kept.end(); ++i) if (i->second.used < old->second.used) old = i;
+            if (b.clock - old->second.used > BATCH_STALE && b.clock - b.replaced >= BATCH_TURN) {
+                b.replaced = b.clock;
+                cudaGraphExecDestroy(old->second.exec);
+                b.kept.erase(old);
+            } else {
+                key = kinds_of(chain);
+                x = updated(b.shared, key);
+                into = b.shared.size() < BATCH_SHARED_MAX ? &b.shared : nullptr;
             }
         }
-        if (it != b.kept.end()) {
-            it->second.used = b.clock;
-            e = cudaGraphLaunch(it->second.exec, b.stream);
+        if (x) {
+            e = cudaGraphLaunch(x, b.stream);
+        } else if (!chain.empty() && (!keep || !into) && std::all_of(chain.begin(), chain.end(), launches_alone)) {
+            for (size_t i = 0; i < chain.size() && e == cudaSuccess; i++) e = launch_node(chain[i], b.stream);
         } else {
-            const std::vector<cudaGraphNode_t> chain = chain_of(g);
-            if (chain.empty()) keep = false;
-            if (keep && b.kept.size() >= BATCH_KEPT_MAX) {
-                auto old = b.kept.begin();
-                for (auto i = b.kept.begin(); i != b.kept.end(); ++i) if (i->second.used < old->second.used) old = i;
-                if (b.clock - old->second.used > BATCH_STALE) {
-                    cudaGraphExecDestroy(old->second.exec);
-                    b.kept.erase(old);
-                } else {
-                    keep = false;
-                }
-            }
-            if (!keep && !chain.empty() && std::all_of(chain.begin(), chain.end(), launches_alone)) {
-                for (size_t i = 0; i < chain.size() && e == cudaSuccess; i++) e = launch_node(chain[i], b.stream);
-            } else {
-                cudaGraphExec_t x = nullptr;
-                e = cudaGraphInstantiate(&x, g, 0);
-                if (e == cudaSuccess) e = cudaGraphLaunch(x, b.stream);
-                if (x && keep) b.kept.emplace(key, BatchState::Exec{x, b.clock});
-                else if (x) cudaGraphExecDestroy(x);
-            }
+            e = cudaGraphInstantiate(&x, g, 0);
+            if (e == cudaSuccess) e = cudaGraphLaunch(x, b.stream);
+            if (x && keep && into && !chain.empty()) (*into)[key] = BatchState::Exec{x, b.clock};
+            else if (x) cudaGraphExecDestroy(x);
         }
     }
     cudaGraphDestroy(g);
+    if (e == cudaSuccess && (b.last || cudaEventCreateWithFlags(&b.last, cudaEventDisableTiming) == cudaSuccess)) e = cudaEventRecord(b.last, b.stream);
     return e == cudaSuccess ? SEERA_OK : check_cuda(e, "batch");
 }
 int batch_flush() { return batch_submit(false); }
@@ -597,8 +605,10 @@ int seera_pool_trim(void) {
         for (void *b : kv.second) { cudaFree(b); p.reserved -= kv.first; }
         kv.second.clear();
     }
-    for (auto &kv : batch().kept) cudaGraphExecDestroy(kv.second.exec);
-    batch().kept.clear();
+    for (auto *m : {&batch().kept, &batch().shared}) {
+        for (auto &kv : *m) cudaGraphExecDestroy(kv.second.exec);
+        m->clear();
+    }
     spares_trim(0);
     pinned_trim();
     return SEERA_OK;
@@ -697,28 +707,30 @@ static int batch_open(uint64_t tag) {
     b.open = true;
     b.tag = tag;
     b.stream = rt().stream;
-    b.launches_at_open = rt().launches;
     return SEERA_OK;
 }
 int seera_batch_begin(uint64_t tag) {
     SEERA_ENSURE();
     BatchState &b = batch();
-    if (b.depth++ > 0) return SEERA_OK;
+    if (b.depth++ > 0) {
+        if (b.depth == 2) b.inner_at = rt().launches;
+        return SEERA_OK;
+    }
+    b.parted = false;
     if (rt().capturing || prof().on || rt().stream == nullptr) return SEERA_OK;
     cudaStreamCaptureStatus st;
     if (cudaStreamIsCapturing(rt().stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) { cudaGetLastError(); return SEERA_OK; }
-    b.starved = cudaStreamQuery(rt().stream) == cudaSuccess;
-    if (!b.starved) cudaGetLastError();
     return batch_open(tag);
 }
-int seera_batches_kept(void) { return (int)batch().kept.size(); }
+int seera_batches_kept(void) { return (int)(batch().kept.size() + batch().shared.size()); }
 int seera_batch_end(void) {
     BatchState &b = batch();
     if (b.depth == 0) return fail(SEERA_E_ARG, "batch_end: no batch is open");
     if (--b.depth == 0) return batch_submit(true);
-    if (!b.open || !b.starved || rt().launches - b.launches_at_open < BATCH_PART) return SEERA_OK;
+    if (!b.open || b.parted || b.depth > 1 || rt().launches - b.inner_at < BATCH_PART) return SEERA_OK;
+    if (b.last && cudaEventQuery(b.last) != cudaSuccess) { cudaGetLastError(); return SEERA_OK; }
+    b.parted = true;
     if (int s = batch_submit(true)) return s;
-    b.starved = false;                                  // from here on the device has work ahead
     return batch_open(b.tag);
 }
 

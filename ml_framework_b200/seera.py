@@ -45,22 +45,21 @@ def _new(shape):
 
 
 # One submission for the launches of a phase (seera_batch_begin / _end): inside, the engine records its launches, and the end hands
-# them over as one graph - a third of the host time per launch and no gaps between them on the device.  A tag names the kind of pass:
-# the layers and the precision.  The engine brings one executable graph per tag and number of launches up to date with sizes and
-# addresses; the first pass at a size runs launch by launch, so that whatever is set up on first use is set up outside a recording.
+# them over as one graph - a third of the host time per launch and no gaps between them on the device.  A tag names what decides
+# which launches follow: the layers, the input's shape, the precision.  The first pass under a tag runs launch by launch, so that
+# whatever is set up on first use is set up outside a recording.
 _batch_begin, _batch_end = getattr(sc, "batch_begin", None), getattr(sc, "batch_end", None)
-_passes_seen = set()
+_tags_seen = set()
 
 
-def _open_batch(tag, size):
+def _open_batch(tag):
     """True if a batch was opened; the caller then owes a _batch_end()."""
     if tag is None or _batch_begin is None:
         return False
-    key = (tag, size)
-    if key not in _passes_seen:
-        if len(_passes_seen) > 4096:
-            _passes_seen.clear()
-        _passes_seen.add(key)
+    if tag not in _tags_seen:
+        if len(_tags_seen) > 4096:
+            _tags_seen.clear()
+        _tags_seen.add(tag)
         return False
     _batch_begin(tag)
     return True
@@ -85,7 +84,7 @@ class Tensor:
     _takes_pooled = False            # its backward takes the gradient of a 2x2 max-pool of it in pooled form
     _copies = None                   # channels-last copies of the value, made by its producer for a convolution
     _rows = None                     # row-major copies of the value, made by its producer for a Dense layer
-    _pass = None                     # batch tag and input shape of the model pass it came from
+    _tag = None                      # batch tag of the model pass it came from
 
     def __init__(self, value, dtype="float32", is_leaf=False, device="cuda"):
         if isinstance(value, Tensor):
@@ -300,8 +299,8 @@ class autograd4nn:
         self.backward()
 
     def backward(self):
-        tag, size = self.hook._pass or (None, None)
-        opened = _open_batch(None if tag is None else _make_tag(tag, "backward"), size)
+        tag = self.hook._tag
+        opened = _open_batch(None if tag is None else _make_tag(tag, "backward"))
         try:
             self._run()
         finally:
@@ -1070,8 +1069,8 @@ class Sequential:
             if not isinstance(X, Tensor):
                 raise TypeError("Input must be a Tensor or numpy array.")
             self.model[0].inputs = X
-        tag, size = self._tag("forward"), self._input_shape()
-        opened = _open_batch(tag, size)
+        tag = self._tag("forward")
+        opened = _open_batch(tag)
         try:
             out = None
             for layer in self.model:
@@ -1080,19 +1079,16 @@ class Sequential:
             if opened:
                 _batch_end()
         if tag is not None:
-            out._pass = tag, size
+            out._tag = tag
         return out
-
-    def _input_shape(self):
-        X = self.model[0].inputs
-        return X.value.shape if isinstance(X, Tensor) else None
 
     def _tag(self, *phase):
         """Tag of a pass over the current input, or None where it does not run as one batch: with gradients exchanged between
         ranks during backward, other streams take part in it."""
-        if self._allreduce is not None or self._on_grad_ready is not None or not isinstance(self.model[0].inputs, Tensor):
+        X = self.model[0].inputs
+        if self._allreduce is not None or self._on_grad_ready is not None or not isinstance(X, Tensor):
             return None
-        return _make_tag(self._structure, sc.get_precision(), FUSE_POOL, DENSE_EPILOGUE_COPIES, *phase)
+        return _make_tag(self._structure, X.value.shape, sc.get_precision(), FUSE_POOL, DENSE_EPILOGUE_COPIES, *phase)
 
     def predict(self, X):
         """Forward in evaluation mode: BatchNorm layers normalise with their running statistics (Seera.py:690-700)."""
@@ -1171,7 +1167,7 @@ class Sequential:
                 yv = cuten._wrap(st["dy"].main_ptr, (m,) + y.shape[1:])
                 yv._owns_memory = False
             self.model[0].inputs = xb
-            opened = _open_batch(self._tag("fit", Optimizer.__class__.__name__), (xb.value.shape, yv.shape))
+            opened = _open_batch(self._tag("fit", yv.shape, Optimizer.__class__.__name__))
             try:
                 return _train_step(self, Optimizer, Loss, Tensor(yv, is_leaf=True))
             finally:
@@ -1367,7 +1363,7 @@ class Loss:
         # the gradient arrives as the all-ones seed of a scalar loss
         out = Tensor._of(loss, (logits,), lambda g: (_scale_gradients(dz), logits._accumulate(dz)))
         out._keep = (rows, yv)
-        out._pass = y_pred._pass
+        out._tag = y_pred._tag
         return out
 
     def _elementwise(self, kernel, y_pred, y, *extra):
@@ -1379,7 +1375,7 @@ class Loss:
                float(f32(1.0 / p.size)), *extra)
         out = Tensor._of(loss, (y_pred,), lambda g: (_scale_gradients(dp), y_pred._accumulate(dp)))
         out._keep = (part, yv)
-        out._pass = y_pred._pass
+        out._tag = y_pred._tag
         return out
 
     def mse(self, y_pred, y):

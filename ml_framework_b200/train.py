@@ -86,7 +86,7 @@ class Trainer:
         Y = Y if isinstance(Y, S.Tensor) else S.Tensor(Y, is_leaf=True)
         self.opt.begin_step()
         self.model.model[0].inputs = X
-        opened = S._open_batch(self.model._tag("step", self.precision, self.work.loss, self.work.opt["kind"]), X.value.shape)
+        opened = S._open_batch(self.model._tag("step", self.precision, self.work.loss, self.work.opt["kind"]))
         try:
             loss = self.forward_backward(X, Y)
             self.opt.step()
