@@ -47,13 +47,16 @@ def _new(shape):
 # One submission for the launches of a phase (seera_batch_begin / _end): inside, the engine records its launches, and the end hands
 # them over as one graph - a third of the host time per launch and no gaps between them on the device.  A tag names what decides
 # which launches follow: the layers, the input's shape, the precision.  The first pass under a tag runs launch by launch, so that
-# whatever is set up on first use is set up outside a recording.
+# whatever is set up on first use is set up outside a recording.  Only what is this module's own runs inside one: a caller's layer,
+# loss, optimizer or gradient function may launch, wait or record events on the stream by itself.
 _batch_begin, _batch_end = getattr(sc, "batch_begin", None), getattr(sc, "batch_end", None)
 _tags_seen = set()
+_inside = 0                          # batches open: what runs inside one has been looked over
 
 
 def _open_batch(tag):
-    """True if a batch was opened; the caller then owes a _batch_end()."""
+    """True if a batch was opened; the caller then owes a _close_batch()."""
+    global _inside
     if tag is None or _batch_begin is None:
         return False
     if tag not in _tags_seen:
@@ -62,7 +65,14 @@ def _open_batch(tag):
         _tags_seen.add(tag)
         return False
     _batch_begin(tag)
+    _inside += 1
     return True
+
+
+def _close_batch():
+    global _inside
+    _inside -= 1
+    _batch_end()
 
 
 def _make_tag(*what):
@@ -84,7 +94,7 @@ class Tensor:
     _takes_pooled = False            # its backward takes the gradient of a 2x2 max-pool of it in pooled form
     _copies = None                   # channels-last copies of the value, made by its producer for a convolution
     _rows = None                     # row-major copies of the value, made by its producer for a Dense layer
-    _tag = None                      # batch tag of the model pass it came from
+    _tag = None                      # (batch tag, model) of the pass it came from
 
     def __init__(self, value, dtype="float32", is_leaf=False, device="cuda"):
         if isinstance(value, Tensor):
@@ -291,6 +301,9 @@ class _KeptRows:
     __del__ = release
 
 
+_Function = type(lambda: None)
+
+
 class autograd4nn:
     """Reverse pass from a scalar loss: `autograd4nn(loss)` (same call shape as Seera_Engine.py:24-26)."""
 
@@ -299,16 +312,20 @@ class autograd4nn:
         self.backward()
 
     def backward(self):
-        tag = self.hook._tag
-        opened = _open_batch(None if tag is None else _make_tag(tag, "backward"))
+        order, own = self._order()
+        opened = False
+        if own and self.hook._tag is not None:
+            tag, model = self.hook._tag
+            opened = model._exchanges_nothing() and _open_batch(_make_tag(tag, "backward"))
         try:
-            self._run()
+            self._run(order)
         finally:
             if opened:
-                _batch_end()
+                _close_batch()
 
-    def _run(self):
-        order, seen = [], set()
+    def _order(self):
+        """Every tensor that the gradient passes, parents first, and whether all of it is this module's own."""
+        order, seen, own = [], set(), True
         stack = [self.hook]
         while stack:                                   # iterative DFS: no recursion limit on deep nets
             t = stack.pop()
@@ -318,11 +335,17 @@ class autograd4nn:
             if t in seen:
                 continue
             seen.add(t)
+            back = t._backward
+            if back is not None and (back.__class__ is not _Function or back.__module__ != __name__):
+                own = False
             stack.append(t)
             stack.append(None)
             for p in t._parents:
                 if not p.is_leaf:                      # a leaf keeps its gradient and passes nothing on
                     stack.append(p)
+        return order, own
+
+    def _run(self, order):
         for t in order:
             if not t.is_leaf:
                 t.grad = None
@@ -934,6 +957,10 @@ class Flatten(Layer):
         return "Flatten Layer"
 
 
+_OWN_LAYERS = {c: c.forward for c in (Input, Dense, Conv2D, ConvTranspose2D, BatchNorm1d, BatchNorm2d, Concatenate, MaxPool2D, Unpool2D_Nearest,
+                                       Flatten)}
+
+
 # ─────────────────────────────────────────────────────────────────────────────────────────────
 # Sequential
 # ─────────────────────────────────────────────────────────────────────────────────────────────
@@ -951,6 +978,10 @@ def _train_step(model, optimizer, lossf, y):
     return loss
 
 
+def _own_step(optimizer, lossf):
+    return optimizer.__class__ in (SGD, Adam) and getattr(lossf, "__func__", None) in _LOSSES
+
+
 # Full batches left to run from which recording the step pays: recording costs the host an eager step, a replay half of one (small CNN
 # at batch 64: 130 and 70 us a step, of which the device works 50).  500 samples by 64: 1160 -> 905 us, 2048: 4430 -> 2390 us.
 _RECORD_FROM = 3
@@ -963,9 +994,8 @@ class _RecordedStep:
     def fits(model, optimizer, lossf):
         """Steps whose every part is this module's own: what a caller's layer, loss or optimizer does on the host would not be repeated."""
         return (hasattr(sc, "graph_set_scalars") and not sc.is_capturing() and not sc.profile_enabled()
-                and model._allreduce is None and model._on_grad_ready is None
-                and optimizer.__class__ in (SGD, Adam) and optimizer.model is model and not optimizer.updates_by_bucket
-                and getattr(lossf, "__func__", None) in _LOSSES and all(l.__class__.__module__ == __name__ for l in model.model))
+                and model._exchanges_nothing() and _own_step(optimizer, lossf) and optimizer.model is model
+                and not optimizer.updates_by_bucket and model._own_passes())
 
     def __init__(self, model, optimizer, lossf, xshape, yshape, classes):
         self.model, self.optimizer = model, optimizer
@@ -1069,26 +1099,40 @@ class Sequential:
             if not isinstance(X, Tensor):
                 raise TypeError("Input must be a Tensor or numpy array.")
             self.model[0].inputs = X
-        tag = self._tag("forward")
-        opened = _open_batch(tag)
+        tag = None if _inside else self._tag("forward")
+        opened = _open_batch(0 if _inside else tag)        # (inside a training step's: its first part ends with the forward)
         try:
             out = None
             for layer in self.model:
                 out = layer.forward()
         finally:
             if opened:
-                _batch_end()
+                _close_batch()
         if tag is not None:
-            out._tag = tag
+            out._tag = tag, self
         return out
 
     def _tag(self, *phase):
         """Tag of a pass over the current input, or None where it does not run as one batch: with gradients exchanged between
         ranks during backward, other streams take part in it."""
         X = self.model[0].inputs
-        if self._allreduce is not None or self._on_grad_ready is not None or not isinstance(X, Tensor):
+        if self._allreduce is not None or self._on_grad_ready is not None or X.__class__ is not Tensor or not self._own_passes():
             return None
         return _make_tag(self._structure, X.value.shape, sc.get_precision(), FUSE_POOL, DENSE_EPILOGUE_COPIES, *phase)
+
+    def _exchanges_nothing(self):
+        return self._allreduce is None and self._on_grad_ready is None
+
+    def _own_passes(self):
+        if self.__class__ is not Sequential and self.__class__.forward is not Sequential.forward:
+            return False
+        try:
+            for l in self.model:
+                if l.forward.__func__ is not _OWN_LAYERS.get(l.__class__):
+                    return False
+        except AttributeError:                        # a function in the place of the method
+            return False
+        return True
 
     def predict(self, X):
         """Forward in evaluation mode: BatchNorm layers normalise with their running statistics (Seera.py:690-700)."""
@@ -1167,12 +1211,12 @@ class Sequential:
                 yv = cuten._wrap(st["dy"].main_ptr, (m,) + y.shape[1:])
                 yv._owns_memory = False
             self.model[0].inputs = xb
-            opened = _open_batch(self._tag("fit", yv.shape, Optimizer.__class__.__name__))
+            opened = _own_step(Optimizer, Loss) and _open_batch(self._tag("fit", yv.shape, Optimizer.__class__.__name__))
             try:
                 return _train_step(self, Optimizer, Loss, Tensor(yv, is_leaf=True))
             finally:
                 if opened:
-                    _batch_end()
+                    _close_batch()
         full_left = (n // bs) * Epochs          # full batches still to run
         recorded, recordable, ran_one = None, _RecordedStep.fits(self, Optimizer, Loss), False
         try:

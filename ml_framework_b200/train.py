@@ -86,13 +86,14 @@ class Trainer:
         Y = Y if isinstance(Y, S.Tensor) else S.Tensor(Y, is_leaf=True)
         self.opt.begin_step()
         self.model.model[0].inputs = X
-        opened = S._open_batch(self.model._tag("step", self.precision, self.work.loss, self.work.opt["kind"]))
+        opened = (self.__class__ is Trainer and X._backward is None and S._own_step(self.opt, self.lossf)
+                  and S._open_batch(self.model._tag("step", self.precision, self.work.loss, self.work.opt["kind"])))
         try:
             loss = self.forward_backward(X, Y)
             self.opt.step()
         finally:
             if opened:
-                S._batch_end()
+                S._close_batch()
         return loss
 
     # ---- whole-step CUDA graph -------------------------------------------------------------------

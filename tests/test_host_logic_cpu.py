@@ -413,3 +413,66 @@ def test_unmodified_reference_python_layer_runs_on_this_cuten(host, golden_dir):
             sys.modules.pop(k, None)
             if v is not None:
                 sys.modules[k] = v
+
+
+@pytest.mark.parametrize("foreign", ["nothing", "layer", "forward of one layer", "gradient", "loss", "optimizer", "model"])
+def test_batches_hold_nothing_of_the_callers(host, monkeypatch, foreign):
+    """What a caller's own code does on the stream is neither recorded nor held back: no batch is open while it runs."""
+    S, state = host.seera, {"open": 0, "opened": 0, "ran": 0}
+
+    def begin(tag):
+        state["open"] += 1
+        state["opened"] += 1
+
+    def end():
+        state["open"] -= 1
+
+    def mine(*_):
+        assert not state["open"]
+        state["ran"] += 1
+    monkeypatch.setattr(S, "_batch_begin", begin)
+    monkeypatch.setattr(S, "_batch_end", end)
+
+    class Mine(S.Dense):
+        def forward(self):
+            mine()
+            return super().forward()
+
+    class MineOpt(S.SGD):
+        def step(self):
+            mine()
+            super().step()
+
+    class MineModel(S.Sequential):
+        def forward(self, X=None):
+            mine()
+            return super().forward(X)
+    np.random.seed(0)
+    model = (MineModel if foreign == "model" else S.Sequential)(
+        [S.Input((6,)), S.Dense(6, 8, activation="relu"), (Mine if foreign == "layer" else S.Dense)(8, 8, activation="relu"),
+         S.Dense(8, 3, activation="softmax")])
+    if foreign == "forward of one layer":
+        own = model.model[2].forward
+        model.model[2].forward = lambda: (mine(), own())[1]
+    opt, cce = (MineOpt if foreign == "optimizer" else S.SGD)(model, lr=0.1), S.Loss().categorical_cross_entropy
+    if foreign == "loss":
+        loss = lambda p, y: (mine(), cce(p, y))[1]                       # noqa: E731
+    elif foreign == "gradient":
+        def loss(p, y):
+            out = cce(p, y)
+            back = out._backward
+            out._backward = lambda g: (mine(), back(g))
+            return out
+    else:
+        loss = cce
+    rs = np.random.RandomState(1)
+    X, Y = rs.standard_normal((20, 6)).astype(np.float32), np.eye(3, dtype=np.float32)[rs.randint(0, 3, 20)]
+    model.fit(X, Y, opt, loss, Epochs=2, batch_size=5, Loss_interval=100)
+    assert state["open"] == 0 and (state["ran"] > 0) == (foreign != "nothing")
+    trainer = host.train.Trainer.__new__(host.train.Trainer)
+    trainer.model, trainer.opt, trainer.lossf, trainer.precision = model, opt, loss, None
+    trainer.work = types.SimpleNamespace(loss="cce", opt={"kind": "sgd"})
+    state["opened"] = 0
+    for _ in range(3):
+        trainer.step(X, Y)
+    assert state["open"] == 0 and (state["opened"] > 0) == (foreign in ("nothing", "gradient", "loss", "optimizer"))        # the forward is one
