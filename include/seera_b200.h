@@ -152,14 +152,15 @@ void *seera_graph_end(void);                        /* NULL on failure */
 int   seera_graph_launch(void *graph);
 int   seera_graph_destroy(void *graph);
 int   seera_is_capturing(void);
-/* One submission for many launches.  Between batch_begin and batch_end the library's launches are recorded, and batch_end hands
- * them to the device as one graph: about 0.9 us of host time per launch instead of 2.8, and no gaps between them on the device.
- * Everything has been enqueued when batch_end returns, in the order of the calls.  The executable graph is kept under `tag` (a hash of
- * whatever decides which launches follow) and updated in place by the next batch of that tag.  A limited number is kept; batches beyond
- * share executables of as many launches, or are launched call by call. Calls that
- * wait, read or write host memory, record events or use another stream first submit what has been recorded; the rest of the batch is
- * then launched call by call, as it is inside a seera_graph_begin recording and while the profile is on.  Batches nest: the
- * outermost one counts, and the first long one inside it is submitted at its own end if the device waits for work. */
+/* One submission for many launches.  Between batch_begin and batch_end the library's launches are noted down, and batch_end hands
+ * them to the device as one graph: 0.1 to 0.4 us of host time per launch instead of 2.8, and no gaps between them on the device.
+ * Everything has been enqueued when batch_end returns, in the order of the calls.  The executable graph of a row of kernels and grids
+ * is kept under `tag` (a name for the kind of pass) and given the arguments of the next such batch; a limited number is kept, and a
+ * batch without one is launched call by call.  Calls that wait, read or write host memory, record events or use another stream first
+ * submit what there is, and so does an allocation that the driver has to serve; the rest of the batch is then launched call by call, as
+ * it is inside a seera_graph_begin recording and while the profile is on.  The stream is not captured: other threads may do what they
+ * like, but what a caller enqueues on the stream by itself comes before the launches that are held back (seera_get_stream submits them).
+ * Batches nest: the outermost one counts, and the first long one inside it is submitted at its own end if the device waits for work. */
 int   seera_batch_begin(uint64_t tag);
 int   seera_batch_end(void);
 int   seera_batches_kept(void);                     /* executable graphs kept for further batches */

@@ -24,6 +24,8 @@ EXT = os.path.join(PKG, "seera_cuda" + sysconfig.get_config_var("EXT_SUFFIX"))
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-I" + os.path.join(ROOT, "include"), "-I" + CSRC]
+# the launches of this library pass through csrc/batch.cu
+WRAPPED = ["-Xlinker", ",".join("--wrap=" + f for f in ("cudaLaunchKernel", "cudaLaunchKernelExC", "cudaMemsetAsync", "cudaMemcpyAsync"))]
 
 
 def _newer(target, deps):
@@ -56,8 +58,8 @@ def build(force=False, verbose=False, ptxas_info=False):
             jobs.append([NVCC] + NVCC_FLAGS + (["-Xptxas", "-v"] if ptxas_info else []) + ["-c", src, "-o", o])
     with cf.ThreadPoolExecutor(max_workers=min(8, max(1, len(jobs)))) as ex:
         list(ex.map(lambda c: _run(c, verbose or ptxas_info), jobs))
-    if force or jobs or _newer(LIB, objs):
-        _run([NVCC, "-shared", "-o", LIB] + objs + ["-lcudart"], verbose)
+    if force or jobs or _newer(LIB, objs + [os.path.join(PKG, "build.py")]):
+        _run([NVCC, "-shared", "-o", LIB] + objs + ["-lcudart"] + WRAPPED, verbose)
     shim = os.path.join(CSRC, "seera_cuda_module.cpp")
     if force or _newer(EXT, [shim, LIB] + headers):
         import pybind11

@@ -146,9 +146,13 @@ void optimizer_node_params(const OptLaunch &launch, cudaKernelNodeParams &kp, vo
 // Device float[2]: {dynamic factor of the fp16 gradient copies, its inverse}; both 1 until a loss head sets them (fused.cu).
 float *grad_scale_words();
 
-// runtime.cu: hands the launches of an open seera_batch_begin to the device; the rest of that batch is launched one by one.  Called
-// before whatever a recording cannot hold: a wait, a copy from or to host memory, an event, another recording.
+// batch.cu: hands the launches of an open seera_batch_begin to the device; the rest of that batch is launched one by one.  Called
+// before whatever has to come behind them: a wait, a copy from or to host memory, an event, another recording.
 int batch_flush();
+void batch_trim();                          // gives back the executable graphs kept for further batches
+// Lets a kernel be launched with up to `bytes` of dynamic shared memory.  The limit is the kernel's and not a launch's: it is only ever
+// raised, since a launch that has been noted down comes after this call.
+cudaError_t allow_smem(const void *kernel, size_t bytes);
 // RAII bracket over the launches of one entry (no-op inside a batch that is open already).
 struct Batch {
     Batch(uint64_t tag) { seera_batch_begin(tag); }

@@ -234,11 +234,11 @@ int run_tc(const AL &al, const BL &bl, const CS &cs, int M, int N, int K, bool a
     profile_begin();
     if (split3) {
         auto kern = tc_contraction_kernel<true, A_KFAST, B_KFAST, AL, BL, CS>;
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = allow_smem((const void *)kern, smem);
         if (e == cudaSuccess) { kern<<<grid, TC_THREADS, smem, st>>>(al, bl, cs, p); e = cudaGetLastError(); }
     } else {
         auto kern = tc_contraction_kernel<false, A_KFAST, B_KFAST, AL, BL, CS>;
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        e = allow_smem((const void *)kern, smem);
         if (e == cudaSuccess) { kern<<<grid, TC_THREADS, smem, st>>>(al, bl, cs, p); e = cudaGetLastError(); }
     }
     count_launch();

@@ -482,7 +482,7 @@ int conv_pool_simt(const float *X, const float *Wt, const float *bias, const Poo
     cudaStream_t st = rt().stream;
     cudaError_t attr = cudaSuccess;
     auto launch = [&](auto kern) {
-        if (smem > 48 * 1024) attr = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        attr = allow_smem((const void *)kern, smem);
         if (attr == cudaSuccess)
             kern<<<grid, 256, smem, st>>>(X, Wt, bias, pool, NB, C, H, W, F, OH, OW, ph, pw, act, fast_div(Pq), fast_div(OW / 2),
                                           fast_div(groups), band);

@@ -758,15 +758,8 @@ void first_wgrad_reduce(const float *partial, float *dW, float *dbias, int F, in
     count_launch();
 }
 
-// Dynamic shared memory limit raised once per kernel instantiation and device.
 template <class K>
-static cudaError_t raise_smem_limit(K kernel, int *done_flags) {
-    const int dev = rt().device & 63;
-    if (done_flags[dev]) return cudaSuccess;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);
-    if (e == cudaSuccess) done_flags[dev] = 1;
-    return e;
-}
+static cudaError_t raise_smem_limit(K kernel) { return allow_smem((const void *)kernel, 225 * 1024); }
 
 static bool first_tc_fwd_ok(const FirstGeom &g) { return rt().precision >= 1 && g.F <= 128 && (long long)g.NB * g.OH * g.OW < (1LL << 31) - 256; }
 static bool first_tc_wgrad_ok(const FirstGeom &g, bool want_bias) {
@@ -793,11 +786,10 @@ static int first_tc_fwd(const float *X, const float *Wt, const float *bias, floa
     if (pool) { po = *pool; pool_out_geometry(po, g.OH * g.OW, g.OW, 1); }
     cudaStream_t st = rt().stream;
     cudaError_t e;
-    static int f1[64], f2[64], f3[64];
     profile_begin();
-    if (ns == 1) { e = raise_smem_limit(first_tc_fwd_kernel<1>, f1); if (e == cudaSuccess) first_tc_fwd_kernel<1><<<grid, FTC_THREADS, smem, st>>>(X, Wt, cs, g, bias, act, bn, stages, nslices, pool_on, po, tc_status_word()); }
-    else if (ns == 2) { e = raise_smem_limit(first_tc_fwd_kernel<2>, f2); if (e == cudaSuccess) first_tc_fwd_kernel<2><<<grid, FTC_THREADS, smem, st>>>(X, Wt, cs, g, bias, act, bn, stages, nslices, pool_on, po, tc_status_word()); }
-    else { e = raise_smem_limit(first_tc_fwd_kernel<3>, f3); if (e == cudaSuccess) first_tc_fwd_kernel<3><<<grid, FTC_THREADS, smem, st>>>(X, Wt, cs, g, bias, act, bn, stages, nslices, pool_on, po, tc_status_word()); }
+    if (ns == 1) { e = raise_smem_limit(first_tc_fwd_kernel<1>); if (e == cudaSuccess) first_tc_fwd_kernel<1><<<grid, FTC_THREADS, smem, st>>>(X, Wt, cs, g, bias, act, bn, stages, nslices, pool_on, po, tc_status_word()); }
+    else if (ns == 2) { e = raise_smem_limit(first_tc_fwd_kernel<2>); if (e == cudaSuccess) first_tc_fwd_kernel<2><<<grid, FTC_THREADS, smem, st>>>(X, Wt, cs, g, bias, act, bn, stages, nslices, pool_on, po, tc_status_word()); }
+    else { e = raise_smem_limit(first_tc_fwd_kernel<3>); if (e == cudaSuccess) first_tc_fwd_kernel<3><<<grid, FTC_THREADS, smem, st>>>(X, Wt, cs, g, bias, act, bn, stages, nslices, pool_on, po, tc_status_word()); }
     count_launch();
     if (e == cudaSuccess) e = cudaGetLastError();
     profile_end(2.0 * pixels * (double)g.F * g.K, name);
@@ -821,12 +813,11 @@ static int first_tc_wgrad(const float *X, const DzSource &src, float *dW, float 
     if (!partial) return SEERA_E_OOM;
     cudaStream_t st = rt().stream;
     cudaError_t e;
-    static int f1[64], f2[64], f3[64];
     const int ones = dbias ? 1 : 0;
     profile_begin();
-    if (ns == 1) { e = raise_smem_limit(first_tc_wgrad_kernel<1>, f1); if (e == cudaSuccess) first_tc_wgrad_kernel<1><<<nblocks, FTW_THREADS, smem, st>>>(X, src, partial, g, nsteps, stages, ones, by_window, tc_status_word()); }
-    else if (ns == 2) { e = raise_smem_limit(first_tc_wgrad_kernel<2>, f2); if (e == cudaSuccess) first_tc_wgrad_kernel<2><<<nblocks, FTW_THREADS, smem, st>>>(X, src, partial, g, nsteps, stages, ones, by_window, tc_status_word()); }
-    else { e = raise_smem_limit(first_tc_wgrad_kernel<3>, f3); if (e == cudaSuccess) first_tc_wgrad_kernel<3><<<nblocks, FTW_THREADS, smem, st>>>(X, src, partial, g, nsteps, stages, ones, by_window, tc_status_word()); }
+    if (ns == 1) { e = raise_smem_limit(first_tc_wgrad_kernel<1>); if (e == cudaSuccess) first_tc_wgrad_kernel<1><<<nblocks, FTW_THREADS, smem, st>>>(X, src, partial, g, nsteps, stages, ones, by_window, tc_status_word()); }
+    else if (ns == 2) { e = raise_smem_limit(first_tc_wgrad_kernel<2>); if (e == cudaSuccess) first_tc_wgrad_kernel<2><<<nblocks, FTW_THREADS, smem, st>>>(X, src, partial, g, nsteps, stages, ones, by_window, tc_status_word()); }
+    else { e = raise_smem_limit(first_tc_wgrad_kernel<3>); if (e == cudaSuccess) first_tc_wgrad_kernel<3><<<nblocks, FTW_THREADS, smem, st>>>(X, src, partial, g, nsteps, stages, ones, by_window, tc_status_word()); }
     count_launch();
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e == cudaSuccess) {

@@ -289,7 +289,7 @@ static int dw_launch(const DwCall &a) {
     cudaStream_t st = rt().stream;
     profile_begin();
     auto kern = first_dw_kernel<C, ST, FL, POOLED>;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem((const void *)kern, smem);
     if (e == cudaSuccess) {
         kern<<<dim3((unsigned)nblocks, (unsigned)chunks, (unsigned)cgroups), 256, smem, st>>>(a.X, *a.src, partial, g, units, ntiles, stages, vf, fast_div(per_image),
                                                                          fast_div(ucols));

@@ -253,7 +253,7 @@ int conv_pool_tc(const float *X, const float *Wt, const float *bias, const PoolO
     profile_begin();
     cudaError_t e = cudaSuccess;
     auto launch = [&](auto kern) {
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PT_SMEM);
+        e = allow_smem((const void *)kern, PT_SMEM);
         if (e == cudaSuccess) kern<<<dim3((unsigned)gx, (unsigned)chunks), PT_THREADS, PT_SMEM, rt().stream>>>(X, Wt, bias, pool, g, tc_status_word());
     };
 #define SEERA_PT(CV) \

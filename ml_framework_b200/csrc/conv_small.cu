@@ -235,8 +235,7 @@ static int small_launch(const SmallSource &src, const float *Wt, const float *bi
     int grid = rt().sm_count * 4;
     if (grid > total) grid = total;
     profile_begin();
-    cudaError_t e = cudaSuccess;
-    if (smem > 48 * 1024) e = cudaFuncSetAttribute(conv3x3_small_kernel<FW, ST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem((const void *)conv3x3_small_kernel<FW, ST>, smem);
     if (e == cudaSuccess) {
         conv3x3_small_kernel<FW, ST><<<grid, 256, smem, rt().stream>>>(src, Wt, bias, Y, cc, g, total, reversed, act);
         count_launch();

@@ -31,9 +31,9 @@ bool seen_before(uint64_t tag) {
     return !seen.insert(tag).second;
 }
 template <class Call>
-int as_batch(uint64_t tag, Call call) {
-    if (seera::ensure_init() || seera::rt().precision == 0 || !seen_before(tag)) return call();
-    if (int s = seera_batch_begin(tag)) return s;
+int as_batch(uint64_t entry, uint64_t call_tag, Call call) {
+    if (seera::ensure_init() || seera::rt().precision == 0 || !seen_before(call_tag)) return call();
+    if (int s = seera_batch_begin(entry)) return s;
     const int s = call(), e = seera_batch_end();
     return s ? s : e;
 }
@@ -91,7 +91,7 @@ int seera_cuda_conv2d_fwd(const float *image, const float *kernel, float *out, i
 }
 int seera_cuda_conv2d_bwd(const float *W, const float *X, const float *dY, float *dX, float *dW, int batch, int C, int H, int W_in,
                           int F, int R, int S, int strideh, int stridew, int padh, int padw) {
-    return as_batch(entry_tag({1, rt().precision, rt().conv_tma, dX != nullptr, dW != nullptr, batch, C, H, W_in, F, R, S, strideh, stridew, padh, padw}), [&] {
+    return as_batch(1, entry_tag({1, rt().precision, rt().conv_tma, dX != nullptr, dW != nullptr, batch, C, H, W_in, F, R, S, strideh, stridew, padh, padw}), [&] {
         return rt().precision ? (rt().conv_tma ? seera_tma_conv2d_bwd(W, X, dY, dX, dW, batch, C, H, W_in, F, R, S, strideh, stridew, padh, padw) : seera_tc_conv2d_bwd(W, X, dY, dX, dW, batch, C, H, W_in, F, R, S, strideh, stridew, padh, padw)) : seera_simt_conv2d_bwd(W, X, dY, dX, dW, batch, C, H, W_in, F, R, S, strideh, stridew, padh, padw);
     });
 }
@@ -101,7 +101,7 @@ int seera_cuda_conv2DTranpose_fwd(const float *X, const float *W, float *out, in
 }
 int seera_cuda_conv2DTranspose_bwd(const float *W, const float *X, const float *dY, float *dX, float *dW, int batch, int Cin, int Hin,
                                    int Win, int Cout, int KH, int KW, int strideh, int stridew, int padh, int padw) {
-    return as_batch(entry_tag({2, rt().precision, rt().conv_tma, dX != nullptr, dW != nullptr, batch, Cin, Hin, Win, Cout, KH, KW, strideh, stridew, padh, padw}), [&] {
+    return as_batch(2, entry_tag({2, rt().precision, rt().conv_tma, dX != nullptr, dW != nullptr, batch, Cin, Hin, Win, Cout, KH, KW, strideh, stridew, padh, padw}), [&] {
         return rt().precision ? (rt().conv_tma ? seera_tma_convT_bwd(W, X, dY, dX, dW, batch, Cin, Hin, Win, Cout, KH, KW, strideh, stridew, padh, padw) : seera_tc_convT_bwd(W, X, dY, dX, dW, batch, Cin, Hin, Win, Cout, KH, KW, strideh, stridew, padh, padw)) : seera_simt_convT_bwd(W, X, dY, dX, dW, batch, Cin, Hin, Win, Cout, KH, KW, strideh, stridew, padh, padw);
     });
 }

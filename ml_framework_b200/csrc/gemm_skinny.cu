@@ -369,7 +369,7 @@ int skinny_bwd(const float *A, const float *B, const float *dC, float *dA, float
             const int kb = (K / 4 + 255) / 256;
             const size_t smem = (size_t)1024 * N * sizeof(float);
             split(kb, 2, 8);
-            if (smem > 44 * 1024) SK_DISPATCH(N, e = cudaFuncSetAttribute(skinny_dA_kernel<NN, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem))
+            SK_DISPATCH(N, e = allow_smem((const void *)skinny_dA_kernel<NN, 4>, smem))
             if (e == cudaSuccess) SK_DISPATCH(N, (skinny_dA_kernel<NN, 4><<<dim3(kb, groups), 256, smem, st>>>(dC, B, dA, rows, K, chunk_rows)))
         } else {
             const int kb = (K + 255) / 256;

@@ -147,176 +147,6 @@ static void profile_collect() {
     p.recs.clear();
 }
 
-// ---- batches: many launches, one submission ------------------------------------------------------------------------------
-// A launch costs the host about 2.8 us here; recorded into a stream capture it costs 0.25, and bringing a kept executable graph
-// up to date with the recording another 0.45 per kernel (50 kernels: 47 us against 121 launched one by one, and the device runs
-// them without the 1-2 us between separate launches).
-//
-// An update can change grids, arguments and kernels, but not how many nodes there are or what kind each is.  It is not free, though, where it
-// changes kernels: an executable runs its nodes fastest as those it was made of (an autoencoder step of 64 images 236 us, 251 with the
-// executable of a step of 8).  So a batch has one by its tag and number of nodes, while BATCH_KEPT_MAX leave room or one of them has been
-// passed over by BATCH_STALE batches; beyond that, batches of the same kinds of nodes share one, and where those are full as well the batch
-// is launched node by node, at what its launches would have cost without one.  Predictions of a small CNN over 200 batch sizes: 154 us
-// a call when every miss made an executable in place of another, 31 here as launched one by one (VGG 298, 141, 160).  Nothing here waits:
-// an executable graph that is destroyed while it runs is freed when it ends.
-namespace {
-struct BatchState {
-    int depth = 0;
-    bool open = false;                                  // the stream is being captured
-    cudaEvent_t last = nullptr;                         // behind the last batch
-    bool parted = false;                                // a first part of it has been submitted
-    uint64_t tag = 0, inner_at = 0;                     // ... and the launch count where the batch directly inside began
-    cudaStream_t stream = nullptr;
-    struct Exec { cudaGraphExec_t exec; uint64_t used; };
-    std::unordered_map<uint64_t, Exec> kept;            // by tag and number of nodes
-    std::unordered_map<uint64_t, Exec> shared;          // by kinds of nodes
-    uint64_t clock = 0, replaced = 0;                   // batches submitted; when an executable last made room for another
-};
-constexpr size_t BATCH_KEPT_MAX = 64;
-// The first pass inside a batch that makes this many launches is submitted at its end if the device has finished the batch before: a
-// step that is waited for would else run host and device one after the other (VGG at 100 images: 557 -> 474 us).  Below that the
-// second submission (6 us) costs a small network more than the device's head start gives.
-constexpr uint64_t BATCH_PART = 12;
-// An executable takes 125 us to make and 110 to destroy (14 launches): one in BATCH_TURN batches may go for another.
-constexpr uint64_t BATCH_STALE = 1024, BATCH_TURN = 64;
-constexpr size_t BATCH_SHARED_MAX = 32;
-BatchState &batch() { static BatchState b; return b; }
-
-// The nodes of a graph in order, if each follows the one before it; else nothing.
-std::vector<cudaGraphNode_t> chain_of(cudaGraph_t g) {
-    std::vector<cudaGraphNode_t> order;
-    size_t nodes = 0, edges = 0, roots = 1;
-    cudaGraphNode_t at = nullptr;
-    if (cudaGraphGetNodes(g, nullptr, &nodes) != cudaSuccess || cudaGraphGetEdges(g, nullptr, nullptr, &edges) != cudaSuccess ||
-        !nodes || edges != nodes - 1 || cudaGraphGetRootNodes(g, nullptr, &roots) != cudaSuccess || roots != 1 ||
-        cudaGraphGetRootNodes(g, &at, &roots) != cudaSuccess) {
-        cudaGetLastError();
-        return order;
-    }
-    std::vector<cudaGraphNode_t> from(edges), to(edges);
-    if (edges && cudaGraphGetEdges(g, from.data(), to.data(), &edges) != cudaSuccess) { cudaGetLastError(); return order; }
-    std::vector<std::pair<cudaGraphNode_t, cudaGraphNode_t>> next(edges);
-    for (size_t i = 0; i < edges; i++) next[i] = {from[i], to[i]};
-    std::sort(next.begin(), next.end());
-    while (at) {
-        order.push_back(at);
-        auto it = std::lower_bound(next.begin(), next.end(), std::make_pair(at, cudaGraphNode_t(nullptr)));
-        at = it != next.end() && it->first == at && order.size() < nodes ? it->second : nullptr;
-    }
-    if (order.size() != nodes) order.clear();           // something has two successors
-    return order;
-}
-
-// One node as a launch of its own.
-cudaError_t launch_node(cudaGraphNode_t node, cudaStream_t st) {
-    cudaGraphNodeType type;
-    cudaError_t e = cudaGraphNodeGetType(node, &type);
-    if (e != cudaSuccess || type == cudaGraphNodeTypeEmpty) return e;
-    if (type == cudaGraphNodeTypeKernel) {
-        cudaKernelNodeParams kp = {};
-        cudaKernelNodeAttrValue v = {};
-        if ((e = cudaGraphKernelNodeGetParams(node, &kp)) != cudaSuccess) return e;
-        if ((e = cudaGraphKernelNodeGetAttribute(node, cudaLaunchAttributeClusterDimension, &v)) != cudaSuccess) return e;
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
-        cfg.gridDim = kp.gridDim; cfg.blockDim = kp.blockDim; cfg.dynamicSmemBytes = kp.sharedMemBytes; cfg.stream = st;
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val = v;
-        cfg.attrs = attr; cfg.numAttrs = v.clusterDim.x > 1 ? 1 : 0;
-        return cudaLaunchKernelExC(&cfg, kp.func, kp.kernelParams);
-    }
-    if (type == cudaGraphNodeTypeMemset) {
-        cudaMemsetParams mp = {};
-        if ((e = cudaGraphMemsetNodeGetParams(node, &mp)) != cudaSuccess) return e;
-        return mp.height > 1 ? cudaMemset2DAsync(mp.dst, mp.pitch, (int)(mp.value & 255), mp.width * mp.elementSize, mp.height, st)
-                             : cudaMemsetAsync(mp.dst, (int)(mp.value & 255), mp.width * mp.elementSize, st);
-    }
-    cudaMemcpy3DParms cp = {};
-    if ((e = cudaGraphMemcpyNodeGetParams(node, &cp)) != cudaSuccess) return e;
-    return cudaMemcpy3DAsync(&cp, st);
-}
-// Whether launch_node can: kernels, copies, and fills with one byte.
-bool launches_alone(cudaGraphNode_t node) {
-    cudaGraphNodeType type;
-    if (cudaGraphNodeGetType(node, &type) != cudaSuccess) { cudaGetLastError(); return false; }
-    if (type != cudaGraphNodeTypeMemset) return type == cudaGraphNodeTypeKernel || type == cudaGraphNodeTypeMemcpy || type == cudaGraphNodeTypeEmpty;
-    cudaMemsetParams mp = {};
-    if (cudaGraphMemsetNodeGetParams(node, &mp) != cudaSuccess) { cudaGetLastError(); return false; }
-    const unsigned byte = mp.value & 255u;
-    return mp.value == (mp.elementSize == 4 ? byte * 0x01010101u : (mp.elementSize == 2 ? byte * 0x0101u : byte));
-}
-// Number and kinds of the nodes of a chain.
-uint64_t kinds_of(const std::vector<cudaGraphNode_t> &chain) {
-    uint64_t h = chain.size();
-    for (size_t i = 0; i < chain.size(); i++) {
-        cudaGraphNodeType type = cudaGraphNodeTypeKernel;
-        cudaGraphNodeGetType(chain[i], &type);
-        if (type != cudaGraphNodeTypeKernel) h = (h ^ (i * 16 + (uint64_t)type)) * 1099511628211ull;
-    }
-    return h;
-}
-}  // namespace
-
-// Hands over what an open batch has recorded.  `keep`: a recording of a whole batch, whose executable is worth keeping.
-static int batch_submit(bool keep) {
-    BatchState &b = batch();
-    if (!b.open) return SEERA_OK;
-    b.open = false;
-    cudaGraph_t g = nullptr;
-    if (int s = check_cuda(cudaStreamEndCapture(b.stream, &g), "batch: cudaStreamEndCapture")) { cudaGetLastError(); return s; }
-    cudaError_t e = cudaSuccess;
-    size_t n = 0;
-    e = cudaGraphGetNodes(g, nullptr, &n);
-    if (e == cudaSuccess && n) {
-        ++b.clock;
-        // The executable under `key`, brought up to date, or null.
-        auto updated = [&](std::unordered_map<uint64_t, BatchState::Exec> &m, uint64_t key) -> cudaGraphExec_t {
-            auto it = m.find(key);
-            if (it == m.end()) return nullptr;
-            cudaGraphExecUpdateResultInfo info;
-            if (cudaGraphExecUpdate(it->second.exec, g, &info) != cudaSuccess) {
-                cudaGetLastError();
-                cudaGraphExecDestroy(it->second.exec);
-                m.erase(it);
-                return nullptr;
-            }
-            it->second.used = b.clock;
-            return it->second.exec;
-        };
-        uint64_t key = b.tag ^ (0x9E3779B97F4A7C15ull * (uint64_t)n);
-        cudaGraphExec_t x = updated(b.kept, key);
-        const std::vector<cudaGraphNode_t> chain = x ? std::vector<cudaGraphNode_t>() : chain_of(g);
-        auto *into = &b.kept;
-        if (!x && keep && !chain.empty() && b.kept.size() >= BATCH_KEPT_MAX) {
-            auto old = b.kept.begin();
-            for (auto i = b.kept.begin(); i != b.kept.end(); ++i) if (i->second.used < old->second.used) old = i;
-            if (b.clock - old->second.used > BATCH_STALE && b.clock - b.replaced >= BATCH_TURN) {
-                b.replaced = b.clock;
-                cudaGraphExecDestroy(old->second.exec);
-                b.kept.erase(old);
-            } else {
-                key = kinds_of(chain);
-                x = updated(b.shared, key);
-                into = b.shared.size() < BATCH_SHARED_MAX ? &b.shared : nullptr;
-            }
-        }
-        if (x) {
-            e = cudaGraphLaunch(x, b.stream);
-        } else if (!chain.empty() && (!keep || !into) && std::all_of(chain.begin(), chain.end(), launches_alone)) {
-            for (size_t i = 0; i < chain.size() && e == cudaSuccess; i++) e = launch_node(chain[i], b.stream);
-        } else {
-            e = cudaGraphInstantiate(&x, g, 0);
-            if (e == cudaSuccess) e = cudaGraphLaunch(x, b.stream);
-            if (x && keep && into && !chain.empty()) (*into)[key] = BatchState::Exec{x, b.clock};
-            else if (x) cudaGraphExecDestroy(x);
-        }
-    }
-    cudaGraphDestroy(g);
-    if (e == cudaSuccess && (b.last || cudaEventCreateWithFlags(&b.last, cudaEventDisableTiming) == cudaSuccess)) e = cudaEventRecord(b.last, b.stream);
-    return e == cudaSuccess ? SEERA_OK : check_cuda(e, "batch");
-}
-int batch_flush() { return batch_submit(false); }
-
 // An optimizer update is being recorded into the open capture: its node is the one the stream's next work will depend on.
 void graph_note_optimizer(const OptLaunch &launch) {
     Pool &p = pool();
@@ -343,6 +173,31 @@ struct Spare {
 };
 std::vector<Spare> &spares() { static std::vector<Spare> v; return v; }
 }  // namespace
+// The nodes of a graph in order, if each follows the one before it; else nothing.
+static std::vector<cudaGraphNode_t> chain_of(cudaGraph_t g) {
+    std::vector<cudaGraphNode_t> order;
+    size_t nodes = 0, edges = 0, roots = 1;
+    cudaGraphNode_t at = nullptr;
+    if (cudaGraphGetNodes(g, nullptr, &nodes) != cudaSuccess || cudaGraphGetEdges(g, nullptr, nullptr, &edges) != cudaSuccess ||
+        !nodes || edges != nodes - 1 || cudaGraphGetRootNodes(g, nullptr, &roots) != cudaSuccess || roots != 1 ||
+        cudaGraphGetRootNodes(g, &at, &roots) != cudaSuccess) {
+        cudaGetLastError();
+        return order;
+    }
+    std::vector<cudaGraphNode_t> from(edges), to(edges);
+    if (edges && cudaGraphGetEdges(g, from.data(), to.data(), &edges) != cudaSuccess) { cudaGetLastError(); return order; }
+    std::vector<std::pair<cudaGraphNode_t, cudaGraphNode_t>> next(edges);
+    for (size_t i = 0; i < edges; i++) next[i] = {from[i], to[i]};
+    std::sort(next.begin(), next.end());
+    while (at) {
+        order.push_back(at);
+        auto it = std::lower_bound(next.begin(), next.end(), std::make_pair(at, cudaGraphNode_t(nullptr)));
+        at = it != next.end() && it->first == at && order.size() < nodes ? it->second : nullptr;
+    }
+    if (order.size() != nodes) order.clear();           // something has two successors
+    return order;
+}
+
 static void spares_trim(size_t keep) {
     auto &v = spares();
     while (v.size() > keep) {
@@ -605,10 +460,7 @@ int seera_pool_trim(void) {
         for (void *b : kv.second) { cudaFree(b); p.reserved -= kv.first; }
         kv.second.clear();
     }
-    for (auto *m : {&batch().kept, &batch().shared}) {
-        for (auto &kv : *m) cudaGraphExecDestroy(kv.second.exec);
-        m->clear();
-    }
+    batch_trim();
     spares_trim(0);
     pinned_trim();
     return SEERA_OK;
@@ -699,39 +551,6 @@ int seera_graph_set_scalars(void *graph, const float *values, int n) {
         if (int s = check_cuda(cudaGraphExecKernelNodeSetParams(g->exec, o.node, &kp), "cudaGraphExecKernelNodeSetParams")) return s;
     }
     return SEERA_OK;
-}
-
-static int batch_open(uint64_t tag) {
-    BatchState &b = batch();
-    if (cudaStreamBeginCapture(rt().stream, cudaStreamCaptureModeRelaxed) != cudaSuccess) { cudaGetLastError(); return SEERA_OK; }
-    b.open = true;
-    b.tag = tag;
-    b.stream = rt().stream;
-    return SEERA_OK;
-}
-int seera_batch_begin(uint64_t tag) {
-    SEERA_ENSURE();
-    BatchState &b = batch();
-    if (b.depth++ > 0) {
-        if (b.depth == 2) b.inner_at = rt().launches;
-        return SEERA_OK;
-    }
-    b.parted = false;
-    if (rt().capturing || prof().on || rt().stream == nullptr) return SEERA_OK;
-    cudaStreamCaptureStatus st;
-    if (cudaStreamIsCapturing(rt().stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) { cudaGetLastError(); return SEERA_OK; }
-    return batch_open(tag);
-}
-int seera_batches_kept(void) { return (int)(batch().kept.size() + batch().shared.size()); }
-int seera_batch_end(void) {
-    BatchState &b = batch();
-    if (b.depth == 0) return fail(SEERA_E_ARG, "batch_end: no batch is open");
-    if (--b.depth == 0) return batch_submit(true);
-    if (!b.open || b.parted || b.depth > 1 || rt().launches - b.inner_at < BATCH_PART) return SEERA_OK;
-    if (b.last && cudaEventQuery(b.last) != cudaSuccess) { cudaGetLastError(); return SEERA_OK; }
-    b.parted = true;
-    if (int s = batch_submit(true)) return s;
-    return batch_open(b.tag);
 }
 
 // Page-locked host blocks.  The driver takes milliseconds to pin and unpin a block (3 ms for 200 KB measured; a training loop of

@@ -705,13 +705,7 @@ int launch_tma_gemm(const TmaMaps &maps, TmaGemmParams p, const CS &cs, int ns, 
 #define SEERA_TMA_LAUNCH(NSV, PAIRV)                                                                                       \
     {                                                                                                                      \
         auto kern = tma_gemm_kernel<NSV, CS, PAIRV>;                                                                       \
-        static int smem_set[64];                     /* per instantiation and device: raise the limit once */              \
-        const int dev = rt().device & 63;                                                                                  \
-        e = cudaSuccess;                                                                                                   \
-        if (!smem_set[dev]) {                                                                                              \
-            e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 225 * 1024);                       \
-            if (e == cudaSuccess) smem_set[dev] = 1;                                                                       \
-        }                                                                                                                  \
+        e = allow_smem((const void *)kern, 225 * 1024);                                                                    \
         if (e == cudaSuccess) {                                                                                            \
             cudaLaunchConfig_t cfg = {};                                                                                   \
             cfg.gridDim = grid; cfg.blockDim = dim3(TG_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = st;             \

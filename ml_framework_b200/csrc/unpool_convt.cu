@@ -296,7 +296,7 @@ int seera_unpool2_convT_bias_act_fwd(const float *x, const float *w, const float
     const size_t smem = ((size_t)FSTAGES * FCH * FROWS * FPITCH + (size_t)Cin * 16) * sizeof(float);
     const int cap = rt().sm_count * 4;                    // resident blocks
     const int vec = (W & 3) == 0 && aligned16(x);
-    cudaError_t e = cudaFuncSetAttribute(unpool_convt_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem((const void *)unpool_convt_fwd_kernel, smem);
     if (e != cudaSuccess) return check_cuda(e, "unpool2_convT_fwd");
     profile_begin();
     unpool_convt_fwd_kernel<<<items < cap ? items : cap, 256, smem, rt().stream>>>(x, w, bias, y, Cin, H, W, act, segs, bands, items, vec,
@@ -325,7 +325,7 @@ int seera_unpool2_convT_act_bwd(const float *w, const float *x, const float *y, 
     if (!s) {
         profile_begin();
         const size_t smem = (size_t)BSTAGES * BSTAGE * sizeof(float);
-        cudaError_t e = cudaFuncSetAttribute(unpool_convt_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = allow_smem((const void *)unpool_convt_bwd_kernel, smem);
         if (e == cudaSuccess)
             unpool_convt_bwd_kernel<<<dim3((unsigned)blocks, (unsigned)chunks), 256, smem, rt().stream>>>(
                 x, w, dz, dx, partial, Cin, H, W, segs, bands, items, (W & 3) == 0 && aligned16(x) && aligned16(dz), fast_div(segs), fast_div(bands));

@@ -44,25 +44,25 @@ def _new(shape):
     return _wrap(_malloc(_numel(shape)), shape)
 
 
-# One submission for the launches of a phase (seera_batch_begin / _end): inside, the engine records its launches, and the end hands
-# them over as one graph - a third of the host time per launch and no gaps between them on the device.  A tag names what decides
-# which launches follow: the layers, the input's shape, the precision.  The first pass under a tag runs launch by launch, so that
-# whatever is set up on first use is set up outside a recording.  Only what is this module's own runs inside one: a caller's layer,
-# loss, optimizer or gradient function may launch, wait or record events on the stream by itself.
+# One submission for the launches of a phase (seera_batch_begin / _end): inside, the engine notes its launches down, and the end hands
+# them over as one graph - a fraction of the host time per launch and no gaps between them on the device.  A tag names the kind of pass:
+# the layers and the precision.  The first pass at a size runs launch by launch, which leaves no executable behind and lets the device
+# start at once.  Only what is this module's own runs inside a batch: a caller's layer, loss, optimizer or gradient function may launch,
+# wait or record events on the stream by itself.
 _batch_begin, _batch_end = getattr(sc, "batch_begin", None), getattr(sc, "batch_end", None)
-_tags_seen = set()
+_passes_seen = set()
 _inside = 0                          # batches open: what runs inside one has been looked over
 
 
-def _open_batch(tag):
+def _open_batch(tag, size):
     """True if a batch was opened; the caller then owes a _close_batch()."""
     global _inside
     if tag is None or _batch_begin is None:
         return False
-    if tag not in _tags_seen:
-        if len(_tags_seen) > 4096:
-            _tags_seen.clear()
-        _tags_seen.add(tag)
+    if not _inside and (tag, size) not in _passes_seen:
+        if len(_passes_seen) > 4096:
+            _passes_seen.clear()
+        _passes_seen.add((tag, size))
         return False
     _batch_begin(tag)
     _inside += 1
@@ -94,7 +94,7 @@ class Tensor:
     _takes_pooled = False            # its backward takes the gradient of a 2x2 max-pool of it in pooled form
     _copies = None                   # channels-last copies of the value, made by its producer for a convolution
     _rows = None                     # row-major copies of the value, made by its producer for a Dense layer
-    _tag = None                      # (batch tag, model) of the pass it came from
+    _pass = None                     # (batch tag, input shape, model) of the pass it came from
 
     def __init__(self, value, dtype="float32", is_leaf=False, device="cuda"):
         if isinstance(value, Tensor):
@@ -314,9 +314,9 @@ class autograd4nn:
     def backward(self):
         order, own = self._order()
         opened = False
-        if own and self.hook._tag is not None:
-            tag, model = self.hook._tag
-            opened = model._exchanges_nothing() and _open_batch(_make_tag(tag, "backward"))
+        if own and self.hook._pass is not None:
+            tag, size, model = self.hook._pass
+            opened = model._exchanges_nothing() and _open_batch(_make_tag(tag, "backward"), size)
         try:
             self._run(order)
         finally:
@@ -1100,7 +1100,8 @@ class Sequential:
                 raise TypeError("Input must be a Tensor or numpy array.")
             self.model[0].inputs = X
         tag = None if _inside else self._tag("forward")
-        opened = _open_batch(0 if _inside else tag)        # (inside a training step's: its first part ends with the forward)
+        size = None if tag is None else self.model[0].inputs.value.shape
+        opened = _open_batch(0 if _inside else tag, size)      # (inside a training step's: its first part ends with the forward)
         try:
             out = None
             for layer in self.model:
@@ -1109,7 +1110,7 @@ class Sequential:
             if opened:
                 _close_batch()
         if tag is not None:
-            out._tag = tag, self
+            out._pass = tag, size, self
         return out
 
     def _tag(self, *phase):
@@ -1118,7 +1119,7 @@ class Sequential:
         X = self.model[0].inputs
         if self._allreduce is not None or self._on_grad_ready is not None or X.__class__ is not Tensor or not self._own_passes():
             return None
-        return _make_tag(self._structure, X.value.shape, sc.get_precision(), FUSE_POOL, DENSE_EPILOGUE_COPIES, *phase)
+        return _make_tag(self._structure, sc.get_precision(), FUSE_POOL, DENSE_EPILOGUE_COPIES, *phase)
 
     def _exchanges_nothing(self):
         return self._allreduce is None and self._on_grad_ready is None
@@ -1211,7 +1212,7 @@ class Sequential:
                 yv = cuten._wrap(st["dy"].main_ptr, (m,) + y.shape[1:])
                 yv._owns_memory = False
             self.model[0].inputs = xb
-            opened = _own_step(Optimizer, Loss) and _open_batch(self._tag("fit", yv.shape, Optimizer.__class__.__name__))
+            opened = _own_step(Optimizer, Loss) and _open_batch(self._tag("fit", Optimizer.__class__.__name__), (xb.value.shape, yv.shape))
             try:
                 return _train_step(self, Optimizer, Loss, Tensor(yv, is_leaf=True))
             finally:
@@ -1407,7 +1408,7 @@ class Loss:
         # the gradient arrives as the all-ones seed of a scalar loss
         out = Tensor._of(loss, (logits,), lambda g: (_scale_gradients(dz), logits._accumulate(dz)))
         out._keep = (rows, yv)
-        out._tag = y_pred._tag
+        out._pass = y_pred._pass
         return out
 
     def _elementwise(self, kernel, y_pred, y, *extra):
@@ -1419,7 +1420,7 @@ class Loss:
                float(f32(1.0 / p.size)), *extra)
         out = Tensor._of(loss, (y_pred,), lambda g: (_scale_gradients(dp), y_pred._accumulate(dp)))
         out._keep = (part, yv)
-        out._tag = y_pred._tag
+        out._pass = y_pred._pass
         return out
 
     def mse(self, y_pred, y):
