@@ -66,6 +66,7 @@ namespace {
 struct OptNode {
     cudaGraphNode_t node;
     OptLaunch launch;
+    size_t at = 0;                                      // its place in a recording whose nodes follow one another
 };
 struct GraphRec {
     cudaGraph_t graph = nullptr;
@@ -75,7 +76,7 @@ struct GraphRec {
     uint64_t launches_at_begin = 0;
     bool collectives = false;                           // the recording holds launches of the data-parallel communicator
     std::vector<OptNode> optimizers;                    // recorded optimizer updates, whose scalars change from replay to replay
-    size_t chain = 0;                                   // number of nodes if each follows the one before it, else 0
+    uint64_t row = 0;                                   // hash of its kernels and grids if its nodes follow one another, else 0
 };
 static std::vector<GraphRec *> &live_graphs() { static std::vector<GraphRec *> v; return v; }
 struct Pool {
@@ -160,16 +161,17 @@ void graph_note_optimizer(const OptLaunch &launch) {
         cudaGetLastError();
 }
 
-// Executable graphs of recordings that have been destroyed, for the next recording of as many launches in a row: updating one takes
-// 8 us where making one takes 125 and destroying it 110 (14 launches; a short training run records its step once).  At most
-// SPARES_MAX; seera_pool_trim gives them back.  Nodes are named by the graph an executable was made from, which stays with it.
+// Executable graphs of recordings that have been destroyed, for the next recording of the same kernels and grids in a row (another would run
+// slower on them than on its own, see batch.cu): updating one takes 8 us where making one takes 125 and destroying it 110 (14 launches; a
+// short training run records its step once).  At most SPARES_MAX; seera_pool_trim gives them back.  Nodes are named by the graph an
+// executable was made from, which stays with it.
 namespace {
 constexpr size_t SPARES_MAX = 4;
 struct Spare {
     cudaGraph_t graph;
     cudaGraphExec_t exec;
     std::vector<OptNode> optimizers;
-    size_t chain;
+    uint64_t row;
 };
 std::vector<Spare> &spares() { static std::vector<Spare> v; return v; }
 }  // namespace
@@ -198,6 +200,25 @@ static std::vector<cudaGraphNode_t> chain_of(cudaGraph_t g) {
     return order;
 }
 
+// Notes what a recording is made of (GraphRec::row, OptNode::at).
+static void describe(GraphRec *g) {
+    const std::vector<cudaGraphNode_t> chain = chain_of(g->graph);
+    if (chain.empty()) return;
+    uint64_t h = 1469598103934665603ull;
+    auto mix = [&h](uint64_t v) { h = (h ^ v) * 1099511628211ull; h ^= h >> 32; };
+    for (size_t i = 0; i < chain.size(); i++) {
+        for (OptNode &o : g->optimizers) if (o.node == chain[i]) o.at = i;
+        cudaGraphNodeType type;
+        cudaKernelNodeParams kp = {};
+        if (cudaGraphNodeGetType(chain[i], &type) != cudaSuccess ||
+            (type == cudaGraphNodeTypeKernel && cudaGraphKernelNodeGetParams(chain[i], &kp) != cudaSuccess)) { cudaGetLastError(); return; }
+        mix((uint64_t)type);
+        mix((uint64_t)(uintptr_t)kp.func);
+        mix(((uint64_t)kp.gridDim.x << 32) ^ ((uint64_t)kp.gridDim.y << 16) ^ kp.gridDim.z);
+        mix(((uint64_t)kp.sharedMemBytes << 32) ^ ((uint64_t)kp.blockDim.x << 16) ^ (kp.blockDim.y << 8) ^ kp.blockDim.z);
+    }
+    g->row = h | 1;
+}
 static void spares_trim(size_t keep) {
     auto &v = spares();
     while (v.size() > keep) {
@@ -209,7 +230,10 @@ static void spares_trim(size_t keep) {
 static void take_spare(GraphRec *g) {
     auto &v = spares();
     for (size_t i = v.size(); i-- > 0;) {
-        if (v[i].chain != g->chain || v[i].optimizers.size() != g->optimizers.size()) continue;
+        if (v[i].row != g->row || v[i].optimizers.size() != g->optimizers.size()) continue;
+        bool same = true;
+        for (size_t k = 0; k < g->optimizers.size(); k++) same &= v[i].optimizers[k].at == g->optimizers[k].at;
+        if (!same) continue;
         Spare sp = v[i];
         v.erase(v.begin() + (long)i);
         cudaGraphExecUpdateResultInfo info;
@@ -227,9 +251,9 @@ static void take_spare(GraphRec *g) {
 }
 // The caller has waited for the graph's last launch.
 static void keep_spare(GraphRec *g) {
-    if (!g->exec || !g->graph || !g->chain) return;
+    if (!g->exec || !g->graph || !g->row) return;
     spares_trim(SPARES_MAX - 1);
-    spares().push_back({g->graph, g->exec, g->optimizers, g->chain});
+    spares().push_back({g->graph, g->exec, g->optimizers, g->row});
     g->graph = nullptr;
     g->exec = nullptr;
 }
@@ -495,8 +519,8 @@ void *seera_graph_end(void) {
     rt().launches = g->launches_at_begin;               // recorded, not executed
     cudaError_t e = cudaStreamEndCapture(rt().stream, &g->graph);
     if (e == cudaSuccess && !g->collectives) {
-        g->chain = chain_of(g->graph).size();
-        if (g->chain) take_spare(g);
+        describe(g);
+        if (g->row) take_spare(g);
     }
     if (e == cudaSuccess && !g->exec) e = cudaGraphInstantiate(&g->exec, g->graph, 0);
     if (e != cudaSuccess) {

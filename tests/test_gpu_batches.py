@@ -377,3 +377,27 @@ def test_launches_of_one_kernel_with_less_and_less_shared_memory(sc):
         sc.cuda_free(y)
     sc.cuda_free(x)
     sc.set_precision(0)
+
+
+def test_a_recording_keeps_its_update_apart_from_the_spares(sc):
+    """As many launches and updates as a destroyed recording had, the update elsewhere: its scalars go to the update."""
+    n = 1000
+    rs = np.random.RandomState(1)
+    a, b, w = (rs.standard_normal(n).astype(np.float32) for _ in range(3))
+    for first in (True, False, True, False):
+        da, db, dw = (sc.to_device_f32(x) for x in (a, b, w))
+        out, vel = sc.cuda_malloc_f32(n), sc.cuda_zeros_f(n)
+        sc.graph_begin()
+        if first:
+            sc.cuda_elemadd(da, db, out, n)
+        sc.cuda_sgd_step(dw, da, vel, n, 0.1, 0.0, 1.0)
+        if not first:
+            sc.cuda_elemadd(da, db, out, n)
+        g = sc.graph_end()
+        sc.graph_set_scalars(g, [0.5, 0.0, 1.0])
+        sc.graph_launch(g)
+        assert np.array_equal(sc.to_host_f32(out, (n,)), a + b)
+        assert np.allclose(sc.to_host_f32(dw, (n,)), w - 0.5 * a, rtol=1e-6, atol=1e-6)
+        sc.graph_destroy(g)
+        for p in (da, db, dw, out, vel):
+            sc.cuda_free(p)
