@@ -117,6 +117,7 @@ int         seera_get_precision(void);
  *   "tc_wait_ms" (1..60000, default 2000; also SEERA_TC_WAIT_MS): budget of every wait inside the TMA-fed tensor-core
  *       kernel, in milliseconds at ~2 GHz.  A wait that runs out makes the kernel record its code in the status word
  *       (seera_tc_device_status), let the copies already in flight land (bounded), free its TMEM and return.
+ *   "graph_test_lose_update" (0 / 1): TEST HOOK: the next recorded optimizer update cannot name its node and is an error.
  *   "tc_test_skip_load" (k-step index, -1 off): TEST HOOK for that path.  The next TMA-fed launch's first CTA leaves out
  *       the loads of that k-step, so the MMA issuer's wait for the stage runs out.  Nothing faults, traps or spins
  *       without a bound; the result of that one launch is garbage and the status word reads 2.  Clears itself.

@@ -16,6 +16,7 @@ struct Runtime {
     int precision = 0;                  // set from SEERA_PRECISION (default 3) when the runtime is created
     unsigned long long tc_wait_clocks = 4000000000ull;      // budget of a bounded wait inside a tensor-core kernel (~2 s)
     int tc_test_skip_load = -1;         // test hook ("tc_test_skip_load" option): see TmaGemmParams::skip_load
+    bool graph_test_lose_update = false;        // test hook ("graph_test_lose_update" option): the next recorded update cannot name its node
     bool dense_tma = true;              // Dense GEMMs in modes 1/2: TMA-fed kernel (false: in-kernel conversion kernel)
     int tile_n_cap2 = 128;              // widest accumulator tile with two operand copies per stage (bf16x3)
     int tile_n_cap3 = 128;              // ... with three (bf16x6)
@@ -139,7 +140,7 @@ struct OptLaunch {
     long long n; bool vec; int grid;
     float scalars[9]; int n_scalars;
 };
-void graph_note_optimizer(const OptLaunch &launch);
+int graph_note_optimizer(const OptLaunch &launch);
 // kernel, grid, block and argument pointers of the launch (the pointers point into `launch`)
 void optimizer_node_params(const OptLaunch &launch, cudaKernelNodeParams &kp, void **args);
 

@@ -59,6 +59,7 @@ int seera_set_option(const char *name, int value) {
         return SEERA_OK;
     }
     if (!strcmp(name, "tc_test_skip_load")) { rt().tc_test_skip_load = value; return SEERA_OK; }
+    if (!strcmp(name, "graph_test_lose_update")) { rt().graph_test_lose_update = value != 0; return SEERA_OK; }
     if (!strcmp(name, "pool_short_patch")) { rt().pool_short_patch = value != 0; return SEERA_OK; }
     if (!strcmp(name, "sm_reserve")) {
         if (value < 0 || value >= rt().sm_physical) return fail(SEERA_E_ARG, "set_option: sm_reserve must be in [0, %d)", rt().sm_physical);

@@ -744,7 +744,7 @@ int seera_adam_step(float *w, const float *g, float *m, float *v, int n, float l
     const int grid = stride_grid(vec ? (n + 3) / 4 : n);
     adam_kernel<<<grid, 256, 0, rt().stream>>>(w, g, m, v, n, vec, a);
     SEERA_LAUNCH_CHECK("adam_step");
-    if (rt().capturing) graph_note_optimizer({0, w, g, m, v, n, vec, grid, {lr, beta1, omb1, beta2, omb2, eps, c1, c2, grad_scale}, 9});
+    if (rt().capturing) return graph_note_optimizer({0, w, g, m, v, n, vec, grid, {lr, beta1, omb1, beta2, omb2, eps, c1, c2, grad_scale}, 9});
     return SEERA_OK;
 }
 
@@ -778,7 +778,7 @@ int seera_sgd_step(float *w, const float *g, float *vel, int n, float lr, float 
     const int grid = stride_grid(vec ? (n + 3) / 4 : n);
     sgd_kernel<<<grid, 256, 0, rt().stream>>>(w, g, vel, n, vec, lr, momentum, grad_scale);
     SEERA_LAUNCH_CHECK("sgd_step");
-    if (rt().capturing) graph_note_optimizer({1, w, g, vel, nullptr, n, vec, grid, {lr, momentum, grad_scale}, 3});
+    if (rt().capturing) return graph_note_optimizer({1, w, g, vel, nullptr, n, vec, grid, {lr, momentum, grad_scale}, 3});
     return SEERA_OK;
 }
 

@@ -76,6 +76,7 @@ struct GraphRec {
     uint64_t launches_at_begin = 0;
     bool collectives = false;                           // the recording holds launches of the data-parallel communicator
     std::vector<OptNode> optimizers;                    // recorded optimizer updates, whose scalars change from replay to replay
+    bool lost_update = false;                           // ... one of which is not among them
     uint64_t row = 0;                                   // hash of its kernels and grids if its nodes follow one another, else 0
 };
 static std::vector<GraphRec *> &live_graphs() { static std::vector<GraphRec *> v; return v; }
@@ -148,17 +149,24 @@ static void profile_collect() {
     p.recs.clear();
 }
 
-// An optimizer update is being recorded into the open capture: its node is the one the stream's next work will depend on.
-void graph_note_optimizer(const OptLaunch &launch) {
+// An optimizer update is being recorded into the open capture: its node is the one the stream's next work will depend on.  One whose node
+// cannot be named would keep the scalars that it was recorded with: an error, here and where scalars are set.
+int graph_note_optimizer(const OptLaunch &launch) {
     Pool &p = pool();
-    if (!p.capturing || !p.cur) return;
+    if (!p.capturing || !p.cur) return SEERA_OK;
     cudaStreamCaptureStatus st;
     const cudaGraphNode_t *deps = nullptr;
     size_t n = 0;
-    if (cudaStreamGetCaptureInfo_v2(rt().stream, &st, nullptr, nullptr, &deps, &n) == cudaSuccess && n == 1)
+    const cudaError_t e = cudaStreamGetCaptureInfo_v2(rt().stream, &st, nullptr, nullptr, &deps, &n);
+    if (rt().graph_test_lose_update) n = 2;
+    rt().graph_test_lose_update = false;                // one update only
+    if (e == cudaSuccess && n == 1) {
         p.cur->optimizers.push_back({deps[0], launch});
-    else
-        cudaGetLastError();
+        return SEERA_OK;
+    }
+    cudaGetLastError();
+    p.cur->lost_update = true;
+    return fail(SEERA_E_CUDA, "a recorded optimizer update has no node of its own (%zu dependencies): its scalars could not be replaced", n);
 }
 
 // Executable graphs of recordings that have been destroyed, for the next recording of the same kernels and grids in a row (another would run
@@ -566,6 +574,7 @@ int seera_is_capturing(void) { return pool().capturing ? 1 : 0; }
 int seera_graph_set_scalars(void *graph, const float *values, int n) {
     GraphRec *g = static_cast<GraphRec *>(graph);
     if (!g || !g->exec || !values) return fail(SEERA_E_ARG, "graph_set_scalars: not a captured graph");
+    if (g->lost_update) return fail(SEERA_E_ARG, "graph_set_scalars: the recording holds an update whose scalars cannot be replaced");
     for (OptNode &o : g->optimizers) {
         if (n != o.launch.n_scalars) return fail(SEERA_E_ARG, "graph_set_scalars: %d values for an update of %d", n, o.launch.n_scalars);
         memcpy(o.launch.scalars, values, (size_t)n * sizeof(float));

@@ -401,3 +401,31 @@ def test_a_recording_keeps_its_update_apart_from_the_spares(sc):
         sc.graph_destroy(g)
         for p in (da, db, dw, out, vel):
             sc.cuda_free(p)
+
+
+def test_a_recorded_update_that_cannot_be_found_again_is_an_error(sc):
+    """It would keep the scalars of the step it was recorded in."""
+    n = 100
+    d = [sc.cuda_ones_f(n) for _ in range(4)]
+    for lost in (True, False):
+        sc.set_option("graph_test_lose_update", int(lost))
+        sc.graph_begin()
+        try:
+            if lost:
+                with pytest.raises(RuntimeError, match="scalars"):
+                    sc.cuda_sgd_step(d[0], d[1], d[2], n, 0.5, 0.0, 1.0)
+            else:
+                sc.cuda_sgd_step(d[0], d[1], d[2], n, 0.5, 0.0, 1.0)
+        finally:
+            g = sc.graph_end()
+        if lost:
+            with pytest.raises(RuntimeError, match="scalars"):
+                sc.graph_set_scalars(g, [0.25, 0.0, 1.0])
+        else:
+            sc.graph_set_scalars(g, [0.25, 0.0, 1.0])
+            sc.graph_launch(g)
+            assert np.all(sc.to_host_f32(d[0], (n,)) == 0.75)
+        sc.graph_destroy(g)
+    sc.clear_status()
+    for p in d:
+        sc.cuda_free(p)
