@@ -218,23 +218,28 @@ class _PooledGrad:
         return dx
 
 
-class _Unpooled(cuten):
-    """The 2x2 nearest unpooling of `low` as a tensor whose memory is made when its address is asked for.  The transposed convolution that
-    reads it can work from `low` directly, and then it never is."""
-    low = None
+class _Formed(cuten):
+    """A tensor whose values are formed from another's when its address is asked for.  One that is left unformed by a recording is formed
+    anew each time it is asked for: every replay changes what it is formed from."""
+    source = None
+    stale = False                    # the values are those of an earlier replay, for all that is known here
 
     @classmethod
-    def of(cls, low):
-        N, C, H, W = low.shape
-        t = cls._wrap(None, (N, C, 2 * H, 2 * W))
-        t.low = low
+    def _of(cls, source, shape):
+        t = cls._wrap(None, shape)
+        t.source = source
+        t.stale = sc.is_capturing()
         return t
 
     @property
     def main_ptr(self):
         if self._ptr is None:
             self._ptr = _malloc(self.size)
-            sc.cuda_unpooling_fwd(self.low.main_ptr, self._ptr, *self.low.shape, 2, 2)
+            if not self.stale:
+                self._form()
+        if self.stale:
+            self.stale = not sc.is_capturing()           # inside the recording: from here on its replays form them
+            self._form()
         return self._ptr
 
     @main_ptr.setter
@@ -242,33 +247,37 @@ class _Unpooled(cuten):
         self._ptr = value
 
 
-class _Softmax(cuten):
-    """The row softmax of the logits `z` as a tensor whose values are made when its address is asked for.  The cross-entropy, which has to
-    form them anyway, writes them on its way (claim), and a training step then needs no pass for them."""
-    z = None
+class _Unpooled(_Formed):
+    """The 2x2 nearest unpooling of `source`.  The transposed convolution that reads it can work from the source directly, and then it
+    never is."""
+
+    @classmethod
+    def of(cls, low):
+        N, C, H, W = low.shape
+        return cls._of(low, (N, C, 2 * H, 2 * W))
+
+    def _form(self):
+        sc.cuda_unpooling_fwd(self.source.main_ptr, self._ptr, *self.source.shape, 2, 2)
+
+
+class _Softmax(_Formed):
+    """The row softmax of the logits `source`.  The cross-entropy, which has to form it anyway, writes it on its way (claim), and a training
+    step then needs no pass for it."""
 
     @classmethod
     def of(cls, z):
-        t = cls._wrap(None, z.shape)
-        t.z = z
-        return t
+        return cls._of(z, z.shape)
 
     def claim(self):
         """Address for a caller that writes the values itself."""
         if self._ptr is None:
             self._ptr = _malloc(self.size)
+        if self.stale:
+            self.stale = not sc.is_capturing()
         return self._ptr
 
-    @property
-    def main_ptr(self):
-        if self._ptr is None:
-            self._ptr = _malloc(self.size)
-            sc.cuda_softmax_fwd(self.z.main_ptr, self._ptr, *self.shape)
-        return self._ptr
-
-    @main_ptr.setter
-    def main_ptr(self, value):
-        self._ptr = value
+    def _form(self):
+        sc.cuda_softmax_fwd(self.source.main_ptr, self._ptr, *self.shape)
 
 
 class _KeptCopies:
@@ -664,7 +673,7 @@ class ConvTranspose2D(_ParamLayer):
         z = _new((N, Cout, Ho, Wo))
         if (xv.__class__ is _Unpooled and xv._ptr is None and H % 2 == 0 and Wd % 2 == 0
                 and sc.unpool2_convT_fusable(N, Cin, H // 2, Wd // 2, Cout, KH, KW, sh, sw, ph, pw)):
-            return self._forward_unpooled(x, xv.low, z, code)
+            return self._forward_unpooled(x, xv.source, z, code)
         need_dx = not x.is_leaf
         if _KEEPS:
             given = x._copies

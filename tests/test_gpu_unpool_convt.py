@@ -68,3 +68,46 @@ def test_the_unpooled_output_is_there_for_whoever_reads_it(monkeypatch):
     for a, b in zip(got[0][2], got[1][2]):
         assert rel_l2(a, b) < 1e-4
     sc.set_precision(0)
+
+
+def test_an_unpooling_left_out_of_a_recorded_step_is_read_as_of_the_last_replay():
+    from ml_framework_b200 import seera as S, seera_cuda as sc, train, workloads as wl
+    sc.init(0)
+    work = wl.WORKLOADS["c4"]()
+    tr = train.Trainer(work, seed=2, precision=train.policy_for(work))
+    X, Y = work.batch(4, 1)
+    x, y = S.Tensor(X, is_leaf=True), S.Tensor(Y, is_leaf=True)
+    for _ in range(2):
+        tr.step(x, y)
+    tr.capture(x, y)
+    layers = [(l, l.inpobj.outputs) for l in tr.model.model if isinstance(l, S.Unpool2D_Nearest)]
+    assert layers
+    for replay in range(3):
+        sc.upload_f32(x.value.main_ptr, work.batch(4, 10 + replay)[0])
+        tr.replay()
+        for l, low in layers:
+            a = low.value.to_host_f32()
+            assert np.array_equal(l.outputs.to_numpy(), a.repeat(2, axis=2).repeat(2, axis=3))
+    tr.release_graph()
+    sc.set_precision(0)
+
+
+def test_a_softmax_of_a_recorded_forward_is_read_as_of_the_last_replay():
+    from ml_framework_b200 import seera as S, seera_cuda as sc, train, workloads as wl
+    sc.init(0)
+    sc.set_precision(3)
+    work = wl.WORKLOADS["c1"]()
+    model = train.build_model(work, work.params(1))
+    x = S.Tensor(work.batch(5, 1)[0], is_leaf=True)
+    model.predict(x)
+    sc.graph_begin()
+    out = model.predict(x)
+    g = sc.graph_end()
+    for replay in range(3):
+        X = work.batch(5, 20 + replay)[0]
+        sc.upload_f32(x.value.main_ptr, X)
+        sc.graph_launch(g)
+        got = out.to_numpy()
+        assert np.array_equal(got, model.predict(X).to_numpy())
+    sc.graph_destroy(g)
+    sc.set_precision(0)

@@ -476,3 +476,30 @@ def test_batches_hold_nothing_of_the_callers(host, monkeypatch, foreign):
     for _ in range(3):
         trainer.step(X, Y)
     assert state["open"] == 0 and (state["opened"] > 0) == (foreign in ("nothing", "gradient", "loss", "optimizer"))        # the forward is one
+
+
+@pytest.mark.parametrize("kind", ["unpooling", "softmax"])
+@pytest.mark.parametrize("asked_inside", [False, True])
+def test_values_left_unformed_by_a_recording_follow_its_replays(host, monkeypatch, kind, asked_inside):
+    S, fake = host.seera, host.fake
+    rs = np.random.RandomState(3)
+    shape = (2, 3, 4, 5) if kind == "unpooling" else (4, 5)
+    source = host.cuTen.cuten(rs.standard_normal(shape).astype(np.float32))
+    form = (lambda a: a.repeat(2, axis=2).repeat(2, axis=3)) if kind == "unpooling" else (lambda a: co.softmax(a))
+    monkeypatch.setattr(fake, "is_capturing", lambda: True)
+    t = (S._Unpooled if kind == "unpooling" else S._Softmax).of(source)
+    if asked_inside:
+        t.main_ptr                                           # part of the recording: its replays form it
+    monkeypatch.setattr(fake, "is_capturing", lambda: False)
+    for replay in range(3):
+        a = rs.standard_normal(shape).astype(np.float32)
+        fake.upload_f32(source.main_ptr, a)
+        if asked_inside:
+            t._form()                                        # as the replay does
+        before = fake.launch_count()
+        assert np.array_equal(t.to_host_f32(), form(a))
+        assert t.main_ptr == t._ptr
+        formed = fake.CALLS.get("unpool_fwd" if kind == "unpooling" else "softmax", 0)
+        if asked_inside:
+            assert fake.launch_count() == before + 1         # the read alone
+    assert formed
