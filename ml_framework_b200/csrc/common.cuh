@@ -144,6 +144,10 @@ int graph_note_optimizer(const OptLaunch &launch);
 // kernel, grid, block and argument pointers of the launch (the pointers point into `launch`)
 void optimizer_node_params(const OptLaunch &launch, cudaKernelNodeParams &kp, void **args);
 
+// runtime.cu: which of the counters kept at zero a launch that finishes in its last block may use (fused.cu); -1: none.
+constexpr int FINISH_SLOTS = 256;
+int finish_slot();
+
 // Device float[2]: {dynamic factor of the fp16 gradient copies, its inverse}; both 1 until a loss head sets them (fused.cu).
 float *grad_scale_words();
 

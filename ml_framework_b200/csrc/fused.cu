@@ -10,8 +10,6 @@
 //   Adam / SGD              ~30 cuten operator launches per parameter tensor       (Seera.py:1038-1063, :992-1001)
 // Arithmetic follows the CPU engine, the parity oracle (engine/src/activation_ops.cpp:84-115,
 // Seera.py:1069-1084, :1006-1008).
-#include <atomic>
-
 #include "common.cuh"
 
 namespace seera {
@@ -204,18 +202,33 @@ __device__ __forceinline__ void grad_scale_finalize(float *w) {
 // infinities and NaNs do not steer the scale
 __device__ __forceinline__ float scale_entry(float g) { const float a = fabsf(g); return a < 3.0e38f ? a : 0.f; }
 
-// True in the block that finishes last; everything the others wrote before is then visible to it.  The counter (one of a
-// few that the launches use in turn) is back at zero afterwards.
-__device__ unsigned int g_finish_counters[64];
-__device__ __forceinline__ bool last_block_done(int counter) {
+// True in the block that finishes last; everything the others wrote before is then visible to it.  The counter is back at zero afterwards.
+__device__ __forceinline__ bool last_block_done(unsigned int *counter) {
     __shared__ int last;
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) last = atomicInc(&g_finish_counters[counter], gridDim.x - 1) == gridDim.x - 1;
+    if (threadIdx.x == 0) last = atomicInc(counter, gridDim.x - 1) == gridDim.x - 1;
     __syncthreads();
     if (last) __threadfence();
     return last != 0;
 }
+// No two launches that may run at the same time share a counter: the launches on a stream have one, every recorded launch has its own until
+// the recording is destroyed, and where there is none left, or in a caller's own capture, a launch takes a word from the pool and clears it
+// first.
+__device__ unsigned int g_finish_counters[FINISH_SLOTS];
+struct FinishCounter {
+    unsigned int *word = nullptr, *own = nullptr;
+    FinishCounter() {
+        static unsigned int *base = nullptr;
+        if (!base && cudaGetSymbolAddress((void **)&base, g_finish_counters) != cudaSuccess) { cudaGetLastError(); base = nullptr; }
+        const int slot = base ? finish_slot() : -1;
+        if (slot >= 0) { word = base + slot; return; }
+        word = own = (unsigned int *)scratch_alloc(sizeof(unsigned int));
+        if (own) cudaMemsetAsync(own, 0, sizeof(unsigned int), rt().stream);
+    }
+    ~FinishCounter() { if (own) scratch_free(own); }
+    FinishCounter(const FinishCounter &) = delete;
+};
 // The last block of a loss launch: the mean from what the blocks left in v[0..n), in a fixed order, and (scale != null) the dynamic
 // factor of the fp16 gradient copies from the largest entry.
 __device__ __forceinline__ void finish_loss(const float *v, int n, float factor, float *out, float *scale, float *sm) {
@@ -238,7 +251,6 @@ __device__ __forceinline__ void note_largest(float m, float *scale) {
     for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     if ((threadIdx.x & 31) == 0 && m > 0.f) atomicMax(reinterpret_cast<unsigned *>(scale) + 2, __float_as_uint(m));
 }
-inline int next_finish_counter() { static std::atomic<unsigned> k{0}; return (int)(++k & 63u); }
 // Where a loss launch in the present precision mode leaves the factor (null: the copies of this mode have none), and the note that
 // it has done so for gradient `dz`.
 inline float *loss_scale(const float *dz, long long n) {
@@ -252,7 +264,7 @@ inline float *loss_scale(const float *dz, long long n) {
 __global__ void __launch_bounds__(256) softmax_cce_kernel(const float *__restrict__ z, const float *__restrict__ yhot,
                                                           float *__restrict__ p, float *__restrict__ loss_rows,
                                                           float *__restrict__ dz, int N, int C, float eps, float inv_count,
-                                                          float *__restrict__ loss_mean, float *__restrict__ scale, int counter) {
+                                                          float *__restrict__ loss_mean, float *__restrict__ scale, unsigned int *counter) {
     __shared__ float sm[8];
     float largest = 0.f;
     int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -296,7 +308,7 @@ template <int L, int V>
 __global__ void __launch_bounds__(256) softmax_cce_row_kernel(const float *__restrict__ z, const float *__restrict__ yhot,
                                                               float *__restrict__ p, float *__restrict__ loss_rows,
                                                               float *__restrict__ dz, int N, int C, float eps, float inv_count,
-                                                              float *__restrict__ loss_mean, float *__restrict__ scale, int counter) {
+                                                              float *__restrict__ loss_mean, float *__restrict__ scale, unsigned int *counter) {
     __shared__ float sm[8];
     const int lane = threadIdx.x % L, per_block = 256 / L;
     const float hi = 1.0f - eps;
@@ -362,7 +374,7 @@ template <int KIND>
 __global__ void __launch_bounds__(256) elem_loss_kernel(const float *__restrict__ p, const float *__restrict__ y,
                                                         float *__restrict__ partials, float *__restrict__ dp,
                                                         long long n, float inv_count, float eps, float *__restrict__ loss_mean,
-                                                        float *__restrict__ scale, int counter, bool vec) {
+                                                        float *__restrict__ scale, unsigned int *counter, bool vec) {
     __shared__ float sm[8];
     float largest = 0.f;
     long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x, nthr = (long long)gridDim.x * blockDim.x;
@@ -670,9 +682,11 @@ int seera_softmax_cce_fwd_bwd(const float *z, const float *onehot, float *p, flo
     ProfBytes pb(16.0 * N * C, "softmax_cce");
     // at most two blocks per SM: every block pays for its turn at the finish counter
     const int per_block = C <= 16 ? 16 : 8, need = (N + per_block - 1) / per_block, grid = need < 2 * rt().sm_count ? need : 2 * rt().sm_count;
+    const FinishCounter counter;
+    if (!counter.word) return SEERA_E_OOM;
     auto launch = [&](auto kern) {
         kern<<<grid, 256, 0, rt().stream>>>(z, onehot, p, loss_rows, dz, N, C, eps, inv_count, loss_mean, loss_scale(dz, (long long)N * C),
-                                            next_finish_counter());
+                                            counter.word);
     };
     if (C <= 16) launch(softmax_cce_row_kernel<16, 1>);
     else if (C <= 32) launch(softmax_cce_row_kernel<32, 1>);
@@ -696,7 +710,9 @@ static int elem_loss(int kind, const float *p, const float *y, float *partials, 
     if (g > 2 * rt().sm_count) g = 2 * rt().sm_count;        // every block pays for its turn at the finish counter
     cudaStream_t st = rt().stream;
     float *scale = loss_scale(dp, size);
-    const int counter = next_finish_counter();
+    const FinishCounter finish;
+    if (!finish.word) return SEERA_E_OOM;
+    unsigned int *counter = finish.word;
     ProfBytes pb(12.0 * size, name);
     if (kind == 0) elem_loss_kernel<0><<<g, 256, 0, st>>>(p, y, partials, dp, size, inv_count, eps, loss_mean, scale, counter, vec);
     else if (kind == 1) elem_loss_kernel<1><<<g, 256, 0, st>>>(p, y, partials, dp, size, inv_count, eps, loss_mean, scale, counter, vec);

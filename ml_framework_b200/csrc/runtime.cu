@@ -76,6 +76,7 @@ struct GraphRec {
     uint64_t launches_at_begin = 0;
     bool collectives = false;                           // the recording holds launches of the data-parallel communicator
     std::vector<OptNode> optimizers;                    // recorded optimizer updates, whose scalars change from replay to replay
+    std::vector<int> finish_slots;                      // counters of the recorded launches that finish in their last block
     bool lost_update = false;                           // ... one of which is not among them
     uint64_t row = 0;                                   // hash of its kernels and grids if its nodes follow one another, else 0
 };
@@ -264,6 +265,39 @@ static void keep_spare(GraphRec *g) {
     spares().push_back({g->graph, g->exec, g->optimizers, g->row});
     g->graph = nullptr;
     g->exec = nullptr;
+}
+
+// Slot 0 serves the library's own stream, whose launches follow one another, the next ones a caller's stream each (streams have numbers that
+// are not given twice), and the rest are for recordings, which may be replayed beside all of them.
+namespace {
+constexpr int FINISH_STREAMS = 64;
+struct FinishSlots {
+    std::unordered_map<unsigned long long, int> streams;
+    std::vector<int> free;
+    FinishSlots() { for (int i = FINISH_SLOTS - 1; i >= FINISH_STREAMS; i--) free.push_back(i); }
+};
+FinishSlots &finish_slots() { static FinishSlots s; return s; }
+}  // namespace
+int finish_slot() {
+    Pool &p = pool();
+    FinishSlots &f = finish_slots();
+    if (p.capturing && p.cur) {
+        if (f.free.empty()) return -1;
+        p.cur->finish_slots.push_back(f.free.back());
+        f.free.pop_back();
+        return p.cur->finish_slots.back();
+    }
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(rt().stream, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) { cudaGetLastError(); return -1; }
+    if (rt().stream == rt().own_stream) return 0;
+    unsigned long long id = 0;
+    if (cudaStreamGetId(rt().stream, &id) != cudaSuccess) { cudaGetLastError(); return -1; }
+    auto it = f.streams.find(id);
+    if (it != f.streams.end()) return it->second;
+    if (f.streams.size() + 1 >= (size_t)FINISH_STREAMS) return -1;
+    const int slot = (int)f.streams.size() + 1;
+    f.streams[id] = slot;
+    return slot;
 }
 
 void *scratch_alloc(size_t bytes) { return seera_cuda_malloc(bytes); }
@@ -563,6 +597,7 @@ int seera_graph_destroy(void *graph) {
         p.owner.erase(b.first);
         if (!p.live.count(b.first)) p.free_lists[b.second].push_back(b.first);   // idle: back to the general pool
     }
+    for (int s : g->finish_slots) finish_slots().free.push_back(s);
     auto &lg = live_graphs();
     for (size_t i = 0; i < lg.size(); i++)
         if (lg[i] == g) { lg.erase(lg.begin() + (long)i); break; }

@@ -68,3 +68,99 @@ def test_the_predictions_are_there_for_whoever_reads_them(sc):
     pred = model.forward(x)
     S.Loss().categorical_cross_entropy(pred, S.Tensor(y, is_leaf=True))
     assert np.allclose(pred.to_numpy(), before, rtol=1e-6) and np.allclose(before.sum(1), 1, rtol=1e-5)
+
+
+def test_losses_on_two_streams_finish_each_by_itself():
+    """On the library's stream, on a caller's, and recorded and replayed on the caller's: more launches than there ever were counters."""
+    import torch
+    from ml_framework_b200 import seera_cuda as sc
+    sc.init(0)
+    sc.set_precision(3)
+    N, C, n = 60000, 10, 500000
+    rs = np.random.RandomState(4)
+    z, y = rs.standard_normal((N, C)).astype(np.float32), np.eye(C, dtype=np.float32)[rs.randint(0, C, N)]
+    a, b = rs.standard_normal(n).astype(np.float32), rs.standard_normal(n).astype(np.float32)
+    dz, dy, da, db = (sc.to_device_f32(v) for v in (z, y, a, b))
+    lp = z.astype(np.float64) - np.log(np.exp(z.astype(np.float64)).sum(1, keepdims=True))
+    want = (-(y * lp).sum(1).mean(), ((a.astype(np.float64) - b) ** 2).mean())
+    side = torch.cuda.Stream()
+
+    def buffers():
+        return ([sc.cuda_malloc_f32(k) for k in (N * C, N, 1, N * C)], [sc.cuda_malloc_f32(k) for k in (sc.mse_partials(n), 1, n)])
+
+    def losses(bufs):
+        (p, rows, loss, grad), (part, mse, dp) = bufs
+        sc.softmax_cce_fwd_bwd(dz, dy, p, rows, loss, grad, N, C, 1e-7, 1.0 / N)
+        sc.mse_fwd_bwd(da, db, part, mse, dp, n, 1.0 / n)
+    own, theirs, recorded = buffers(), buffers(), [buffers() for _ in range(2)]
+    sc.stream_synchronize()
+    graphs = []
+    for bufs in recorded:
+        sc.graph_begin()
+        losses(bufs)
+        graphs.append(sc.graph_end())
+    try:
+        for rep in range(100):
+            sc.set_stream(side.cuda_stream)
+            losses(theirs)
+            sc.graph_launch(graphs[0])
+            sc.set_stream(0)
+            losses(own)
+            sc.graph_launch(graphs[1])
+            if rep % 10 == 9:
+                torch.cuda.synchronize()
+                for bufs in [own, theirs] + recorded:
+                    got = [float(sc.to_host_f32(q, (1,))[0]) for q in (bufs[0][2], bufs[1][1])]
+                    assert np.allclose(got, want, rtol=1e-5), got
+                    sc.cuda_memset(bufs[0][2], 0, 4)
+                    sc.cuda_memset(bufs[1][1], 0, 4)
+                torch.cuda.synchronize()
+    finally:
+        sc.set_stream(0)
+        torch.cuda.synchronize()
+        for g in graphs:
+            sc.graph_destroy(g)
+        for bufs in [own, theirs] + recorded:
+            for q in bufs[0] + bufs[1]:
+                sc.cuda_free(q)
+        for q in (dz, dy, da, db):
+            sc.cuda_free(q)
+        sc.set_precision(0)
+
+
+def test_more_recorded_losses_than_counters():
+    """Beyond the counters that recordings hold a launch brings a word of its own; a destroyed recording gives its counters back.  The same
+    for callers' streams."""
+    from ml_framework_b200 import seera_cuda as sc
+    sc.init(0)
+    sc.set_precision(3)
+    n = 5000
+    a, b = np.linspace(-1, 1, n, dtype=np.float32), np.linspace(1, 3, n, dtype=np.float32)
+    da, db = sc.to_device_f32(a), sc.to_device_f32(b)
+    part, dp = sc.cuda_malloc_f32(sc.mse_partials(n)), sc.cuda_malloc_f32(n)
+    want = float(((a.astype(np.float64) - b) ** 2).mean())
+    for rep in range(3):
+        out = [sc.cuda_zeros_f(1) for _ in range(300)]
+        sc.graph_begin()
+        for q in out:
+            sc.mse_fwd_bwd(da, db, part, q, dp, n, 1.0 / n)
+        g = sc.graph_end()
+        for _ in range(2):
+            sc.graph_launch(g)
+        assert np.allclose([float(sc.to_host_f32(q, (1,))[0]) for q in out], want, rtol=1e-5)
+        sc.graph_destroy(g)
+        for q in out:
+            sc.cuda_free(q)
+    import torch
+    streams = [torch.cuda.Stream() for _ in range(32)]       # (torch has 32 a device and deals them out in turn)
+    loss = sc.cuda_zeros_f(1)
+    for rep in range(3):
+        for st in streams:
+            sc.set_stream(st.cuda_stream)
+            sc.cuda_memset(loss, 0, 4)
+            sc.mse_fwd_bwd(da, db, part, loss, dp, n, 1.0 / n)
+            assert np.allclose(sc.to_host_f32(loss, (1,)), want, rtol=1e-5)
+    sc.set_stream(0)
+    for q in (da, db, part, dp, loss):
+        sc.cuda_free(q)
+    sc.set_precision(0)
