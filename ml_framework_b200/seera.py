@@ -23,6 +23,7 @@ from __future__ import annotations
 
 import math
 import pickle
+import weakref
 
 import numpy as np
 
@@ -94,7 +95,7 @@ class Tensor:
     _takes_pooled = False            # its backward takes the gradient of a 2x2 max-pool of it in pooled form
     _copies = None                   # channels-last copies of the value, made by its producer for a convolution
     _rows = None                     # row-major copies of the value, made by its producer for a Dense layer
-    _pass = None                     # (batch tag, input shape, model) of the pass it came from
+    _pass = None                     # (batch tag, input shape, reference to the model) of the pass it came from
 
     def __init__(self, value, dtype="float32", is_leaf=False, device="cuda"):
         if isinstance(value, Tensor):
@@ -325,7 +326,8 @@ class autograd4nn:
         opened = False
         if own and self.hook._pass is not None:
             tag, size, model = self.hook._pass
-            opened = model._exchanges_nothing() and _open_batch(_make_tag(tag, "backward"), size)
+            model = model()
+            opened = model is not None and model._exchanges_nothing() and _open_batch(_make_tag(tag, "backward"), size)
         try:
             self._run(order)
         finally:
@@ -372,6 +374,7 @@ class autograd4nn:
 # ─────────────────────────────────────────────────────────────────────────────────────────────
 class Layer:
     # which layers read this one's output (set while a model is put together): a producer can then hand on more than its values
+    # (weak references and no `self` in a gradient function: a model that is dropped returns its memory at once, and the next one finds it)
     _pool_consumer = None
     _feeds_conv = _feeds_dense = _feeds_convT = _feeds_copies = False
     _fused = None                    # a pool that the layer folded into its own launch: (pooled, mask, copies)
@@ -478,15 +481,21 @@ class _ParamLayer(Layer):
         out._softmax_logits = node
         return out
 
-    def _deliver(self, x, W, b, dx, dw, db):
-        """Gradients of one backward call to the input and the parameters."""
-        b._accumulate(db)
-        W._accumulate(dw)
-        model = self._model
-        if model is not None and model._on_grad_ready is not None and W.grad is W._grad_slot and b.grad is b._grad_slot:
-            model._on_grad_ready(W)          # this layer's gradients sit in the arena: a bucket may go out
-        if dx is not None:
-            x._accumulate(dx)
+
+def _grads_in_arena(owner, W, b):
+    """Tells the model's hook that a layer's gradients sit in the arena: a bucket may go out."""
+    model = owner and owner()
+    if model is not None and model._on_grad_ready is not None and W.grad is W._grad_slot and b.grad is b._grad_slot:
+        model._on_grad_ready(W)
+
+
+def _deliver(owner, x, W, b, dx, dw, db):
+    """Gradients of one backward call to the input and the parameters."""
+    b._accumulate(db)
+    W._accumulate(dw)
+    _grads_in_arena(owner, W, b)
+    if dx is not None:
+        x._accumulate(dx)
 
 
 class Dense(_ParamLayer):
@@ -520,7 +529,7 @@ class Dense(_ParamLayer):
         want_out = DENSE_EPILOGUE_COPIES and self._feeds_dense and self.layeract != "softmax"
         ha, hw, ho = sc.matmul_bias_act_fwd_s(xv.main_ptr, wv.main_ptr, b.value.main_ptr, z._ptr, M, N, K, code, given.h if given else 0, want_out)
         kept_a, kept_w = _KeptRows(ha) if ha else None, _KeptRows(hw) if hw else None
-        need_dx = not x.is_leaf
+        need_dx, owner = not x.is_leaf, self._model
 
         def backward(g):
             # activation slope, bias gradient, dA and dB in one call; it reads the copies the forward call kept
@@ -532,7 +541,7 @@ class Dense(_ParamLayer):
             for k in (kept_a, kept_w, given):
                 if k:
                     k.release()
-            self._deliver(x, W, b, dx, dw, db)
+            _deliver(owner, x, W, b, dx, dw, db)
         self.outputs = out = self._output(x, z, backward)
         if want_out:
             out._rows = _KeptRows(ho)
@@ -579,7 +588,7 @@ class Conv2D(_ParamLayer):
         F, (KH, KW), (sh, sw), (ph, pw) = self.out_channels, self.kernel_size, self.stride, self.zero_padding
         OH, OW = (H + 2 * ph - KH) // sh + 1, (Wd + 2 * pw - KW) // sw + 1
         code = _ACT[self.layeract]
-        pool = self._pool_consumer
+        owner, pool = self._model, self._pool_consumer and self._pool_consumer()
         self._fused = None
         if FUSE_POOL and pool is not None and sc.conv2d_pool_fusable(N, C, H, Wd, F, KH, KW, sh, sw, ph, pw):
             # the pool is folded into this layer's epilogue: z stays a shape without memory
@@ -624,7 +633,7 @@ class Conv2D(_ParamLayer):
             for k in (kept, kept_w, given):
                 if k:
                     k.release()
-            self._deliver(x, W, b, dx, dw, db)
+            _deliver(owner, x, W, b, dx, dw, db)
         self.outputs = out = self._output(x, z, backward, takes_pooled=True)
         if hy:
             out._copies = _KeptCopies(hy)
@@ -674,7 +683,7 @@ class ConvTranspose2D(_ParamLayer):
         if (xv.__class__ is _Unpooled and xv._ptr is None and H % 2 == 0 and Wd % 2 == 0
                 and sc.unpool2_convT_fusable(N, Cin, H // 2, Wd // 2, Cout, KH, KW, sh, sw, ph, pw)):
             return self._forward_unpooled(x, xv.source, z, code)
-        need_dx = not x.is_leaf
+        need_dx, owner = not x.is_leaf, self._model
         if _KEEPS:
             given = x._copies
             h = sc.conv2DTranspose_bias_act_fwd_k(xv.main_ptr, wv.main_ptr, b.value.main_ptr, z._ptr, N, Cin, H, Wd, Cout, KH, KW, sh, sw, ph, pw,
@@ -691,7 +700,7 @@ class ConvTranspose2D(_ParamLayer):
                 for k in (kept, given):
                     if k:
                         k.release()
-                self._deliver(x, W, b, dx, dw, db)
+                _deliver(owner, x, W, b, dx, dw, db)
             self.outputs = self._output(x, z, backward)
             return self.outputs
         sc.conv2DTranspose_bias_act_fwd(xv.main_ptr, wv.main_ptr, b.value.main_ptr, z._ptr, N, Cin, H, Wd, Cout, KH, KW, sh, sw, ph, pw, code)
@@ -707,7 +716,7 @@ class ConvTranspose2D(_ParamLayer):
             dx = _new(shape) if need_dx else None
             sc.cuda_conv2DTranspose_bwd(wv._ptr, xv._ptr, dz.main_ptr, dx._ptr if need_dx else 0, dw._ptr, N, Cin, H, Wd, Cout, KH, KW,
                                        sh, sw, ph, pw)
-            self._deliver(x, W, b, dx, dw, db)
+            _deliver(owner, x, W, b, dx, dw, db)
         self.outputs = self._output(x, z, backward)
         return self.outputs
 
@@ -717,14 +726,14 @@ class ConvTranspose2D(_ParamLayer):
         N, Cin, H, Wd = low.shape
         sc.unpool2_convT_bias_act_fwd(low.main_ptr, W.value.main_ptr, b.value.main_ptr, z._ptr, N, Cin, H, Wd, code)
         source = x._parents[0]                    # what was unpooled: its gradient goes to it directly
-        need_dx = not source.is_leaf
+        need_dx, owner = not source.is_leaf, self._model
 
         def backward(g):
             db, dw = b._grad_target(), W._grad_target()
             dlow = _new(low.shape) if need_dx else None
             sc.unpool2_convT_act_bwd(W.value._ptr, low._ptr, z._ptr if code else 0, g.main_ptr, dlow._ptr if need_dx else 0, dw._ptr, db._ptr,
                                      N, Cin, H, Wd, code)
-            self._deliver(source, W, b, dlow, dw, db)
+            _deliver(owner, source, W, b, dlow, dw, db)
         self.outputs = self._output(x, z, backward)
         return self.outputs
 
@@ -786,7 +795,7 @@ class _BatchNorm(_ParamLayer):
         fwd, bwd = (sc.batchnorm_fwd_sync, sc.batchnorm_bwd_sync) if self.sync else (sc.batchnorm_fwd, sc.batchnorm_bwd)
         fwd(xv.main_ptr, g.value.main_ptr, b.value.main_ptr, self._rm.main_ptr, self._rv.main_ptr, y._ptr, mean._ptr, si._ptr, N, C, S,
             float(self.momentum), float(self.eps), bool(self.training))
-        need_dx = not x.is_leaf
+        need_dx, owner = not x.is_leaf, self._model
 
         def backward(dy):
             dg, db = g._grad_target(), b._grad_target()
@@ -794,9 +803,7 @@ class _BatchNorm(_ParamLayer):
             bwd(dy.main_ptr, xv._ptr, mean._ptr, si._ptr, g.value._ptr, dx._ptr, dg._ptr, db._ptr, N, C, S)
             g._accumulate(dg)
             b._accumulate(db)
-            model = self._model
-            if model is not None and model._on_grad_ready is not None and g.grad is g._grad_slot and b.grad is b._grad_slot:
-                model._on_grad_ready(g)
+            _grads_in_arena(owner, g, b)
             if need_dx:
                 x._accumulate(dx)
         self.outputs = out = Tensor._of(y, (x, g, b), backward)
@@ -869,7 +876,7 @@ class MaxPool2D(Layer):
             raise TypeError("Input must be a Layer instance.")
         self.inpobj = input_layer
         if (tuple(self.pool_size), self.stride, self.padding) == ((2, 2), (2, 2), (0, 0)):
-            input_layer._pool_consumer = self     # a Conv2D producer may fold this pool into its own launch
+            input_layer._pool_consumer = weakref.ref(self)     # a Conv2D producer may fold this pool into its own launch
         return self
 
     def forward(self):
@@ -1054,8 +1061,9 @@ class Sequential:
         self._modal = [l for l in self.model if hasattr(l, "training")]       # layers that behave differently in evaluation
         self._structure = hash(tuple((l.__class__.__name__,) + tuple(getattr(l, k, None) for k in _STRUCTURE) for l in self.model))
         self._build_arena()
+        self._ref = weakref.ref(self)
         for l in self.param_layers:
-            l._model = self
+            l._model = self._ref
 
     # one contiguous block each for parameters and gradients; slots are 64-float aligned
     def _build_arena(self):
@@ -1119,7 +1127,7 @@ class Sequential:
             if opened:
                 _close_batch()
         if tag is not None:
-            out._pass = tag, size, self
+            out._pass = tag, size, self._ref
         return out
 
     def _tag(self, *phase):

@@ -503,3 +503,37 @@ def test_values_left_unformed_by_a_recording_follow_its_replays(host, monkeypatc
         if asked_inside:
             assert fake.launch_count() == before + 1         # the read alone
     assert formed
+
+
+def test_a_dropped_model_gives_its_memory_back_at_once(host):
+    """Without waiting for the garbage collector: its blocks are there for the next model's first pass."""
+    import gc
+    S = host.seera
+
+    def alive():
+        return sum(isinstance(o, (host.cuTen.cuten, S.Tensor, S.Layer, S.Sequential)) for o in gc.get_objects())
+    layers = {
+        "image": lambda: [S.Input((1, 8, 8)), S.Conv2D(4, 1, (3, 3), "relu", stride=1, zero_padding=1), S.BatchNorm2d(4), S.MaxPool2D((2, 2), stride=2),
+                          S.Conv2D(4, 4, (3, 3), "relu", stride=1, zero_padding=1), S.MaxPool2D((2, 2), stride=2), S.Flatten(),
+                          S.Dense(16, 8, activation="relu"), S.BatchNorm1d(8), S.Dense(8, 3, activation="softmax")],
+        "autoencoder": lambda: [S.Input((1, 8, 8)), S.Conv2D(4, 1, (3, 3), "relu", stride=2, zero_padding=1), S.Unpool2D_Nearest((2, 2)),
+                                S.ConvTranspose2D(1, 4, (3, 3), "sigmoid", stride=1, zero_padding=1)]}
+    rs = np.random.RandomState(0)
+    X, Y = rs.uniform(0, 1, (6, 1, 8, 8)).astype(np.float32), np.eye(3, dtype=np.float32)[rs.randint(0, 3, 6)]
+    for name, make in layers.items():
+        lossf, y = (S.Loss().categorical_cross_entropy, Y) if name == "image" else (S.Loss().mse, X)
+        gc.collect()
+        gc.disable()
+        try:
+            before = alive()
+            for _ in range(2):
+                model = S.Sequential(make())
+                opt = S.Adam(model, lr=1e-3)
+                model.fit(X, y, opt, lossf, Epochs=2, batch_size=4, Loss_interval=100)
+                loss = lossf(model.forward(X), S.Tensor(y, is_leaf=True))
+                S.autograd4nn(loss)
+                model.predict(X)
+                del model, opt, loss
+                assert alive() == before, name
+        finally:
+            gc.enable()
