@@ -288,9 +288,9 @@ class _KeptCopies:
     def __init__(self, h=0):
         self.h = h
 
-    def release(self):
+    def release(self, free=sc.shadow_free):           # (held here: the module's names may be gone when the interpreter ends)
         if self.h:
-            sc.shadow_free(self.h)
+            free(self.h)
             self.h = 0
 
     __del__ = release
@@ -303,9 +303,9 @@ class _KeptRows:
     def __init__(self, h=0):
         self.h = h
 
-    def release(self):
+    def release(self, free=sc.rows_free):
         if self.h:
-            sc.rows_free(self.h)
+            free(self.h)
             self.h = 0
 
     __del__ = release

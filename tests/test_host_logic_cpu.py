@@ -537,3 +537,13 @@ def test_a_dropped_model_gives_its_memory_back_at_once(host):
                 assert alive() == before, name
         finally:
             gc.enable()
+
+
+def test_kept_copies_are_given_back_after_the_modules_names_have_gone(host, monkeypatch):
+    """As they are when the interpreter ends with a model in hand."""
+    S = host.seera
+    kept = [S._KeptCopies(1 << 20), S._KeptRows(1 << 20)]
+    monkeypatch.setattr(S, "sc", None)
+    for k in kept:
+        k.release()
+        assert k.h == 0
