@@ -14,6 +14,10 @@
 //               first maximum wins), pooled values, indices and the channels-last copies for the next convolution
 // Each position has a stage for its operand rows, the accumulator is double-buffered; the CTA is persistent.
 // The result is fp32-class in every mode: all copies are made whatever the mode's own number is.
+// Values that have no bf16 copies (infinities, NaNs, and what rounds to infinity) would leave NaNs behind, which the maximum passes over: a
+// producer that meets one makes all products of the window NaN, and the epilogue forms such a window again in fp32, in the order of
+// conv3x3_pool_kernel.  So it does with every window if it is a filter that holds such a value.  (Finite values whose result lies in the last
+// 2^-8 below fp32's largest may still overflow: the leading copies' product is that much larger at most.)
 #include "conv_first.cuh"
 #include "internal.h"
 #include "tma_gemm_kernel.cuh"
@@ -30,6 +34,8 @@ struct PoolTcGeom {
     int C, H, W, F, OHq, OWq, Pq, ph, pw, windows, tiles, bn, act;
     FastDiv by_Pq, by_OWq;
 };
+
+constexpr float PT_LARGEST = 3.38e38f;         // up to it a value has finite bf16 copies
 
 __device__ __forceinline__ uint32_t pt_offset(int row, int chunk) { return (uint32_t)row * 128u + (uint32_t)((chunk ^ (row & 7)) << 4); }
 // 16 columns of this warp's 32 lanes, requested
@@ -48,7 +54,7 @@ conv_pool_tc_kernel(const float *__restrict__ X, const float *__restrict__ Wt, c
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) unsigned long long bars[3 * PT_STAGES + 4];      // full, empty of even and of odd tiles, tfull[2], tempty[2]
     __shared__ uint32_t tmem_base_slot;
-    __shared__ int abort_flag;
+    __shared__ int abort_flag, filters_bad;
     constexpr int K = 9 * C, CHUNKS = (K + 15) / 16 * 2, SLICES = CHUNKS / 2;
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31, f_base = blockIdx.y * 64;
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -60,18 +66,24 @@ conv_pool_tc_kernel(const float *__restrict__ X, const float *__restrict__ Wt, c
 
     if (t == 0) {
         abort_flag = 0;
+        filters_bad = 0;
         for (int s = 0; s < PT_STAGES; s++) mbar_init(full0 + 8 * s, 4);
         for (int s = 0; s < 2 * PT_STAGES; s++) mbar_init(empty0 + 8 * s, 1);
         for (int b = 0; b < 2; b++) { mbar_init(tfull0 + 8 * b, 1); mbar_init(tempty0 + 8 * b, 4); }
         fence_mbar_init();
     }
+    __syncthreads();
     for (int e = t; e < g.bn; e += PT_THREADS) bk[e] = bias ? __ldg(bias + f_base + e) : 0.f;
     // filters: row f = first copy | second copy, and the third copy in the tile behind
     for (int e = t; e < g.bn * CHUNKS; e += PT_THREADS) {
         const int row = e / CHUNKS, kg = e - row * CHUNKS;
         float v[8];
 #pragma unroll
-        for (int i = 0; i < 8; i++) { const int k = kg * 8 + i; v[i] = k < K ? __ldg(Wt + (long long)(f_base + row) * K + k) : 0.f; }
+        for (int i = 0; i < 8; i++) {
+            const int k = kg * 8 + i;
+            v[i] = k < K ? __ldg(Wt + (long long)(f_base + row) * K + k) : 0.f;
+            if (!(fabsf(v[i]) <= PT_LARGEST)) filters_bad = 1;
+        }
         *reinterpret_cast<uint4 *>(b_base + pt_offset(row, kg)) = split_chunk(v);
         *reinterpret_cast<uint4 *>(b_base + pt_offset(row, kg + 4)) = split_chunk(v);
         *reinterpret_cast<uint4 *>(b_base + 64 * 128 + pt_offset(row, kg)) = split_chunk(v);
@@ -92,6 +104,7 @@ conv_pool_tc_kernel(const float *__restrict__ X, const float *__restrict__ Wt, c
             const int ih0 = 2 * qr - g.ph, iw0 = 2 * (rem - qr * g.OWq) - g.pw;
             const float *xn = X + (long long)n * C * plane + (long long)ih0 * g.W + iw0;
             float v[C][4][4];
+            bool bad = false;
 #pragma unroll
             for (int c = 0; c < C; c++)
 #pragma unroll
@@ -100,6 +113,7 @@ conv_pool_tc_kernel(const float *__restrict__ X, const float *__restrict__ Wt, c
                     for (int j = 0; j < 4; j++) {
                         const bool in = (unsigned)(ih0 + i) < (unsigned)g.H && (unsigned)(iw0 + j) < (unsigned)g.W;
                         v[c][i][j] = in ? __ldg(xn + c * plane + i * g.W + j) : 0.f;
+                        bad |= !(fabsf(v[c][i][j]) <= PT_LARGEST);
                     }
             bool gave_up = false;
 #pragma unroll
@@ -120,6 +134,7 @@ conv_pool_tc_kernel(const float *__restrict__ X, const float *__restrict__ Wt, c
                         const int k = kg * 8 + i, c = k / 9, r = (k % 9) / 3, q = k % 3;
                         u[i] = k < K ? v[c < C ? c : 0][(p >> 1) + r][(p & 1) + q] : 0.f;
                     }
+                    if (kg == 0 && bad) u[0] = __int_as_float(0x7fffffff);
                     *reinterpret_cast<uint4 *>(a + pt_offset(row, kg)) = split_chunk(u);
                     *reinterpret_cast<uint4 *>(a + pt_offset(row, kg + 4)) = split_chunk(u);
                     *reinterpret_cast<uint4 *>(a + PT_A_TILE + pt_offset(row, kg)) = split_chunk(u);
@@ -179,6 +194,7 @@ conv_pool_tc_kernel(const float *__restrict__ X, const float *__restrict__ Wt, c
             float *op = po.pooled + ((long long)n * g.F + f_base) * g.Pq + rem;
             int *om = po.mask + ((long long)n * g.F + f_base) * g.Pq + rem;
             const uint32_t at = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * 4 * g.bn);
+            bool again = filters_bad != 0;
             for (int f0 = 0; f0 < g.bn; f0 += 16) {
                 float z[4][16];
 #pragma unroll
@@ -209,7 +225,34 @@ conv_pool_tc_kernel(const float *__restrict__ X, const float *__restrict__ Wt, c
                     stage[lane * PT_ROW + f0 + f] = m;
                     if (live) { op[(unsigned)((f0 + f) * g.Pq)] = m; om[(unsigned)((f0 + f) * g.Pq)] = id; }
                 }
+                again |= z[0][0] != z[0][0];
             }
+            if (again) {                                  // the window in fp32 (not while z is held: the accumulator reads need its registers)
+                const int qr = g.by_OWq.div(rem), ih0 = 2 * qr - g.ph, iw0 = 2 * (rem - qr * g.OWq) - g.pw;
+                const float *xn = X + (long long)n * C * g.H * g.W, *wk = Wt + (long long)f_base * K;
+#pragma unroll 1
+                for (int f = 0; f < g.bn; f++, wk += K) {
+                    float m = -3.402823466e+38f;
+                    int id = 0;
+#pragma unroll 1
+                    for (int p = 0; p < 4; p++) {
+                        float x = 0.f;
+#pragma unroll 1
+                        for (int k = 0; k < K; k++) {
+                            const int c = k / 9, ih = ih0 + (p >> 1) + (k % 9) / 3, iw = iw0 + (p & 1) + k % 3;
+                            const bool in = (unsigned)ih < (unsigned)g.H && (unsigned)iw < (unsigned)g.W;
+                            x = fmaf(in ? __ldg(xn + ((long long)c * g.H + ih) * g.W + iw) : 0.f, __ldg(wk + k), x);
+                        }
+                        x += bk[f];
+                        if (ACT != SEERA_ACT_RELU) x = epilogue_act(x, ACT);
+                        if (x > m) { m = x; id = p; }
+                    }
+                    if (ACT == SEERA_ACT_RELU && !(m > 0.f)) { m = 0.f; id = 0; }
+                    stage[lane * PT_ROW + f] = m;
+                    if (live) { op[(unsigned)(f * g.Pq)] = m; om[(unsigned)(f * g.Pq)] = id; }
+                }
+            }
+            __syncwarp();
             if (po.copy[0]) {
                 __syncwarp();
                 const int per = g.bn >> 3, rows = min(32, g.windows - w0) * per;        // 8 filters each
