@@ -251,9 +251,11 @@ static int small_run(const SmallSource &src, const float *Wt, const float *bias,
 }
 
 bool conv_direct_applies(int NB, int C, int H, int W, int F, int R, int S, int sh, int sw, int ph, int pw, bool copies) {
-    // Not in the mode of a single bf16 product, whose results are those of rounded operands, nor in that of three copies: there the
-    // tensor-core kernel rounds as little as this one, and another order of the sums would move ties of the pools behind the layer (1e-3 of a
-    // first layer's gradient behind a batch normalisation) for 4 us of a step of 300.
+    // Not in the mode of a single bf16 product, whose results are those of rounded operands.  Not in mode 3 either, the default, with whose
+    // results runs are compared: a new order of the sums there moves ReLU and pool decisions of the layers behind (up to 4e-2 of a gradient two
+    // steps into a batch-norm network, in four of eight seeds), and is taken where it pays - conv_small and first_dw take a half to a
+    // fourth of what they replaced.  Here it is 16.3 -> 12.7 us of a step of 300 (3 -> 32 channels, 128 images of 32 x 32; 64 images of 4 x 20 x 20
+    // into 48: 10.6 -> 14.7), although against 64 bits this kernel is off by 1.0e-7 where the tensor-core form's six products are by 3.3e-7.
     if (rt().precision < 2 || rt().precision == 3 || !rt().conv_tma || R != 3 || S != 3 || sh != sw || sh < 1 || sh > 2 || ph < 0 || pw < 0 || ph > 2 || pw > 2) return false;
     const long long OH = ((long long)H + 2 * ph - 3) / sh + 1, OW = ((long long)W + 2 * pw - 3) / sw + 1;
     return NB >= 1 && C >= 1 && C <= 4 && F >= 1 && (size_t)(C * 9 + 1) * (F + 15) * sizeof(float) <= 64 * 1024 && (!copies || F % 8 == 0) &&
