@@ -460,6 +460,9 @@ int seera_bce_fwd_bwd(const float *p, const float *y, float *partials, float *lo
  * (seera_conv2d_act_bwd with a pooled gradient) calls it once per backward pass on the loss gradient.
  * No counterpart in the reference. */
 int seera_grad_scale_update(const float *g, long long n);
+/* The same for the gradient that the last loss entry (seera_softmax_cce_fwd_bwd, seera_mse_fwd_bwd, ...) wrote, as it wrote it: the loss
+ * launch has left the factor, and nothing is launched. */
+int seera_grad_scale_of_loss(const float *g, long long n);
 
 /* Adam (Seera.py:1069-1084) and SGD with momentum (Seera.py:1006-1008) in one pass, in place.
  * The caller passes the fp32-rounded scalars omb1 = 1-beta1, omb2 = 1-beta2, c1 = 1-beta1^t,

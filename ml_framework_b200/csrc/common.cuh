@@ -27,7 +27,7 @@ struct Runtime {
     int mma_issuers = 0;                // cap on the MMA-issuing threads of the TMA-fed GEMM kernel (0: none; 1 or 2)
     bool pair_tiles = false;            // TMA-fed GEMMs as clusters of two CTAs on 256-row tiles where the plan finds it pays
     bool conv_tma = true;               // convolutions in modes 1-3: TMA im2col kernel (false: in-kernel gather kernel)
-    // the loss gradient whose largest entry the loss head has already turned into the dynamic factor (grad_scale_update then has
+    // the loss gradient whose largest entry the loss head has already turned into the dynamic factor (grad_scale_of_loss then has
     // nothing left to do for it)
     const float *scaled_grad = nullptr;
     long long scaled_n = 0;

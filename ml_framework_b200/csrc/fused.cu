@@ -740,13 +740,20 @@ int seera_grad_scale_update(const float *g, long long n) {
     float *w = grad_scale_words();
     if (!w) return fail(SEERA_E_OOM, "grad_scale_update: no device memory for the scale words");
     if (n == 0) return SEERA_OK;
-    if (g == rt().scaled_grad && n == rt().scaled_n) { rt().scaled_grad = nullptr; return SEERA_OK; }     // the loss head has done it
     rt().scaled_grad = nullptr;                   // the factor is about to be another gradient's
     grad_amax_kernel<<<stride_grid(n), 256, 0, rt().stream>>>(g, n, reinterpret_cast<unsigned *>(w) + 2);
     SEERA_LAUNCH_CHECK("grad_scale_update(amax)");
     grad_scale_finalize_kernel<<<1, 32, 0, rt().stream>>>(w);
     SEERA_LAUNCH_CHECK("grad_scale_update");
     return SEERA_OK;
+}
+
+// For the gradient that a loss launch has just formed and nobody has written since: that launch has left the factor, unless another's has
+// come in between.
+int seera_grad_scale_of_loss(const float *g, long long n) {
+    SEERA_ENSURE();
+    if (g && g == rt().scaled_grad && n == rt().scaled_n) { rt().scaled_grad = nullptr; return SEERA_OK; }
+    return seera_grad_scale_update(g, n);
 }
 
 int seera_adam_step(float *w, const float *g, float *m, float *v, int n, float lr, float beta1, float omb1,

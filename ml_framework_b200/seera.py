@@ -1402,7 +1402,7 @@ def _scale_gradients(g):
     """In the fp16 precision modes the backward pass scales its gradient copies by a power of two taken from the largest
     entry of the loss gradient (fp16's exponent range is 2^-14 .. 2^16; a converging run's gradients leave it downwards)."""
     if sc.get_precision() in (4, 5):
-        sc.grad_scale_update(g.main_ptr, g.size)
+        sc.grad_scale_of_loss(g.main_ptr, g.size)           # (g is the loss's own: nobody has written it since)
 
 
 class Loss:

@@ -467,6 +467,9 @@ def mse_fwd_bwd(p, y, part, loss, dp, n, inv):
 def grad_scale_update(g, n): _count("grad_scale")
 
 
+grad_scale_of_loss = grad_scale_update
+
+
 def mae_fwd_bwd(p, y, part, loss, dp, n, inv):
     _count("mae")
     d = _view(p, n) - _view(y, n)

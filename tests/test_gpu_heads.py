@@ -164,3 +164,33 @@ def test_more_recorded_losses_than_counters():
     for q in (da, db, part, dp, loss):
         sc.cuda_free(q)
     sc.set_precision(0)
+
+
+@pytest.mark.parametrize("entry", ["convolution", "dense", "update"])
+def test_a_loss_gradient_that_was_written_since_has_a_factor_of_its_own(sc, entry):
+    """In the fp16 modes: scaled in place by a power of two that leaves fp16's range, at the address that the loss launch knew."""
+    N, C, H, F = 2, 16, 8, 32
+    rs = np.random.RandomState(2)
+    p, y = (rs.standard_normal(N * F * H * H).astype(np.float32) for _ in range(2))
+    x, w = rs.standard_normal((N, C, H, H)).astype(np.float32), rs.standard_normal((F, C, 3, 3)).astype(np.float32)
+    d = [sc.to_device_f32(a.ravel()) for a in (p, y, x, w)]
+    part, loss, dp, dx, dw = (sc.cuda_malloc_f32(n) for n in (sc.mse_partials(p.size), 1, p.size, max(x.size, p.size), max(w.size, F * F)))
+    sc.set_precision(4)
+    for factor in (1.0, 2.0 ** 20, 2.0 ** -30):
+        sc.mse_fwd_bwd(d[0], d[1], part, loss, dp, p.size, 1.0 / p.size)
+        sc.cuda_scaler_multiply_f(dp, factor, p.size)
+        g = sc.to_host_f32(dp, (p.size,)).astype(np.float64)
+        if entry == "dense":                                 # [N H H, F] @ [F, F]: dB = A^T g
+            M = N * H * H
+            sc.cuda_matmul_bwd(d[0], d[3], dp, dx, dw, M, F, F, 1)
+            got, want = sc.to_host_f32(dw, (F, F)), p.reshape(M, F).T.astype(np.float64) @ g.reshape(M, F)
+        else:
+            if entry == "update":
+                sc.grad_scale_update(dp, p.size)
+            sc.cuda_conv2d_bwd(d[3], d[2], dp, dx, dw, N, C, H, H, F, 3, 3, 1, 1, 1, 1)
+            import torch
+            got = sc.to_host_f32(dw, w.shape)
+            want = torch.nn.grad.conv2d_weight(torch.from_numpy(x).double(), w.shape, torch.from_numpy(g.reshape(N, F, H, H)), padding=1).numpy()
+        assert rel_l2(got, want) < 1e-3, factor              # weight gradients of this mode: one fp16 copy of each operand
+    for q in d + [part, loss, dp, dx, dw]:
+        sc.cuda_free(q)
