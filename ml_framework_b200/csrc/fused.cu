@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(256) softmax_vjp_kernel(const float *__restric
     }
 }
 
-// softmax -> clip -> log -> -y* -> sum(-1), and the gradient of inv_count * sum_rows w.r.t. z
+// ---- loss heads: values, gradient, mean and the factor of the fp16 gradient copies in one launch ---------------------------------
 // factor = 2^(-4 - e) with amax = m * 2^e, m in [0.5, 1): together with the static 2^12 of the gradient class the largest
 // entry of the loss gradient lands in [128, 256) - eight binades of headroom below fp16's maximum for gradients that grow
 // on the way down the network, twenty-one binades of normal range below it for those that shrink.
@@ -261,6 +261,7 @@ inline float *loss_scale(const float *dz, long long n) {
     return w;
 }
 
+// softmax -> clip -> log -> -y* -> sum(-1), and the gradient of inv_count * sum_rows w.r.t. z; a warp per row, for rows of any length
 __global__ void __launch_bounds__(256) softmax_cce_kernel(const float *__restrict__ z, const float *__restrict__ yhot,
                                                           float *__restrict__ p, float *__restrict__ loss_rows,
                                                           float *__restrict__ dz, int N, int C, float eps, float inv_count,
@@ -366,7 +367,6 @@ __global__ void __launch_bounds__(256) softmax_cce_row_kernel(const float *__res
     if (last_block_done(counter)) finish_loss(loss_rows, N, inv_count, loss_mean, scale, sm);
 }
 
-// Deterministic single-block sum of n floats times scale.
 // Element-wise losses with their gradient in the same pass.  KIND 0: (p-y)^2 (Seera.py:943-945); 1: |p-y| with the sign
 // convention of abs_fwd, 0 at 0 (Seera.py:947-949, engine/src/activation_ops.cpp:50-56); 2: binary cross-entropy
 // -y log(p+eps) - (1-y) log(1-p+eps) (Seera.py:951-953).  dp = dloss/dp * inv_count; per-block sums go to `partials`.

@@ -50,7 +50,7 @@ def _new(shape):
 # the layers and the precision.  The first pass at a size runs launch by launch, which leaves no executable behind and lets the device
 # start at once.  Only what is this module's own runs inside a batch: a caller's layer, loss, optimizer or gradient function may launch,
 # wait or record events on the stream by itself.
-_batch_begin, _batch_end = getattr(sc, "batch_begin", None), getattr(sc, "batch_end", None)
+_batch_begin, _batch_end = sc.batch_begin, sc.batch_end        # (_batch_begin None: every pass launch by launch)
 _passes_seen = set()
 _inside = 0                          # batches open: what runs inside one has been looked over
 
@@ -192,9 +192,7 @@ tensor = Tensor
 # layer's output in memory.
 FUSE_POOL = True
 # A 2x2 unpooling that feeds a ConvTranspose2D leaves its output unmade until somebody reads it (see _Unpooled).
-_LAZY_UNPOOL = hasattr(sc, "unpool2_convT_fusable")
-# The engine's forms that hand operand copies on from call to call (filters to the data gradient, outputs to the next convolution).
-_KEEPS = hasattr(sc, "conv2d_act_bwd_k")
+_LAZY_UNPOOL = True
 # A Dense layer that feeds another Dense layer can have its GEMM epilogue write the 16-bit copies of its output that the next
 # layer's GEMM reads (seera_matmul_bias_act_fwd_s, c_copies).  Off: at the sizes measured (4096 x 1024 outputs, one tile per
 # CTA) the two-byte stores lengthen an epilogue that nothing overlaps by more than the next layer's vectorised conversion
@@ -599,19 +597,13 @@ class Conv2D(_ParamLayer):
             pmask = _wrap(sc.cuda_malloc_i32(pooled.size), half, "int32")
             args = (xv.main_ptr, wv.main_ptr, b.value.main_ptr, pooled._ptr, pmask._ptr, N, C, H, Wd, F, KH, KW, ph, pw, sh, sw, code,
                     given.h if given else 0, pool._feeds_conv)
-            if _KEEPS:
-                h, hw, hp = sc.conv2d_bias_act_pool_fwd_k(*args)
-            else:
-                (h, hp), hw = sc.conv2d_bias_act_pool_fwd_s(*args), 0
+            h, hw, hp = sc.conv2d_bias_act_pool_fwd_k(*args)
             self._fused = (pooled, pmask, _KeptCopies(hp) if hp else None)
             hy = 0
         else:
             z = _new((N, F, OH, OW))
             args = (xv.main_ptr, wv.main_ptr, b.value.main_ptr, z._ptr, N, C, H, Wd, F, KH, KW, ph, pw, sh, sw, code, given.h if given else 0)
-            if _KEEPS:
-                h, hw, hy = sc.conv2d_bias_act_fwd_k(*args, self._feeds_copies)
-            else:
-                h, hw, hy = sc.conv2d_bias_act_fwd_s(*args), 0, 0
+            h, hw, hy = sc.conv2d_bias_act_fwd_k(*args, self._feeds_copies)
         kept, kept_w = _KeptCopies(h) if h else None, _KeptRows(hw) if hw else None
         need_dx = not x.is_leaf
 
@@ -626,10 +618,7 @@ class Conv2D(_ParamLayer):
             k = kept or given
             args = (wv._ptr, xv._ptr, z._ptr, gptr, gpptr, mptr, ypptr, dx._ptr if need_dx else 0, dw._ptr, db._ptr,
                     N, C, H, Wd, F, KH, KW, sh, sw, ph, pw, code, k.h if k else 0)
-            if _KEEPS:
-                sc.conv2d_act_bwd_k(*args, kept_w.h if kept_w else 0)
-            else:
-                sc.conv2d_act_bwd(*args)
+            sc.conv2d_act_bwd_k(*args, kept_w.h if kept_w else 0)
             for k in (kept, kept_w, given):
                 if k:
                     k.release()
@@ -684,38 +673,21 @@ class ConvTranspose2D(_ParamLayer):
                 and sc.unpool2_convT_fusable(N, Cin, H // 2, Wd // 2, Cout, KH, KW, sh, sw, ph, pw)):
             return self._forward_unpooled(x, xv.source, z, code)
         need_dx, owner = not x.is_leaf, self._model
-        if _KEEPS:
-            given = x._copies
-            h = sc.conv2DTranspose_bias_act_fwd_k(xv.main_ptr, wv.main_ptr, b.value.main_ptr, z._ptr, N, Cin, H, Wd, Cout, KH, KW, sh, sw, ph, pw,
-                                                  code, given.h if given else 0)
-            kept = _KeptCopies(h) if h else None
-
-            def backward(g):
-                # activation slope, bias gradient and both products in one call
-                db, dw = b._grad_target(), W._grad_target()
-                dx = _new(shape) if need_dx else None
-                k = kept or given
-                sc.conv2DTranspose_act_bwd_k(wv._ptr, xv._ptr, z._ptr, g.main_ptr, dx._ptr if need_dx else 0, dw._ptr, db._ptr, N, Cin, H, Wd, Cout,
-                                             KH, KW, sh, sw, ph, pw, code, k.h if k else 0)
-                for k in (kept, given):
-                    if k:
-                        k.release()
-                _deliver(owner, x, W, b, dx, dw, db)
-            self.outputs = self._output(x, z, backward)
-            return self.outputs
-        sc.conv2DTranspose_bias_act_fwd(xv.main_ptr, wv.main_ptr, b.value.main_ptr, z._ptr, N, Cin, H, Wd, Cout, KH, KW, sh, sw, ph, pw, code)
+        given = x._copies
+        h = sc.conv2DTranspose_bias_act_fwd_k(xv.main_ptr, wv.main_ptr, b.value.main_ptr, z._ptr, N, Cin, H, Wd, Cout, KH, KW, sh, sw, ph, pw,
+                                              code, given.h if given else 0)
+        kept = _KeptCopies(h) if h else None
 
         def backward(g):
+            # activation slope, bias gradient and both products in one call
             db, dw = b._grad_target(), W._grad_target()
-            dz = g
-            if code:
-                dz = _new(z.shape)
-                sc.act_bias_bwd(g.main_ptr, z._ptr, dz._ptr, db._ptr, z.size, Cout, Ho * Wo, code)
-            else:
-                sc.act_bias_bwd(g.main_ptr, 0, g.main_ptr, db._ptr, z.size, Cout, Ho * Wo, 0)
             dx = _new(shape) if need_dx else None
-            sc.cuda_conv2DTranspose_bwd(wv._ptr, xv._ptr, dz.main_ptr, dx._ptr if need_dx else 0, dw._ptr, N, Cin, H, Wd, Cout, KH, KW,
-                                       sh, sw, ph, pw)
+            k = kept or given
+            sc.conv2DTranspose_act_bwd_k(wv._ptr, xv._ptr, z._ptr, g.main_ptr, dx._ptr if need_dx else 0, dw._ptr, db._ptr, N, Cin, H, Wd, Cout,
+                                         KH, KW, sh, sw, ph, pw, code, k.h if k else 0)
+            for k in (kept, given):
+                if k:
+                    k.release()
             _deliver(owner, x, W, b, dx, dw, db)
         self.outputs = self._output(x, z, backward)
         return self.outputs
@@ -1009,7 +981,7 @@ class _RecordedStep:
     @staticmethod
     def fits(model, optimizer, lossf):
         """Steps whose every part is this module's own: what a caller's layer, loss or optimizer does on the host would not be repeated."""
-        return (hasattr(sc, "graph_set_scalars") and not sc.is_capturing() and not sc.profile_enabled()
+        return (not sc.is_capturing() and not sc.profile_enabled()
                 and model._exchanges_nothing() and _own_step(optimizer, lossf) and optimizer.model is model
                 and not optimizer.updates_by_bucket and model._own_passes())
 

@@ -109,7 +109,7 @@ class Trainer:
             raise RuntimeError("capture needs collectives that can be recorded (dp.attach_nccl); with other collectives use "
                                "capture_data_parallel")
         # the update's scalars travel with the recorded launch and are replaced in it before each replay
-        self.opt._scalars_in_graph = self._scalars_in_graph = not self.opt.updates_by_bucket and hasattr(sc, "graph_set_scalars")
+        self.opt._scalars_in_graph = self._scalars_in_graph = not self.opt.updates_by_bucket
         sc.graph_begin()
         try:
             loss = self.step(X, Y)

@@ -511,7 +511,7 @@ def test_a_dropped_model_gives_its_memory_back_at_once(host):
     S = host.seera
 
     def alive():
-        return sum(isinstance(o, (host.cuTen.cuten, S.Tensor, S.Layer, S.Sequential)) for o in gc.get_objects())
+        return sum(issubclass(type(o), (host.cuTen.cuten, S.Tensor, S.Layer, S.Sequential)) for o in gc.get_objects())
     layers = {
         "image": lambda: [S.Input((1, 8, 8)), S.Conv2D(4, 1, (3, 3), "relu", stride=1, zero_padding=1), S.BatchNorm2d(4), S.MaxPool2D((2, 2), stride=2),
                           S.Conv2D(4, 4, (3, 3), "relu", stride=1, zero_padding=1), S.MaxPool2D((2, 2), stride=2), S.Flatten(),
