@@ -159,8 +159,8 @@ int   seera_is_capturing(void);
  * is kept under `tag` (a name for the kind of pass) and given the arguments of the next such batch; a limited number is kept, and a
  * batch without one is launched call by call.  Calls that wait, read or write host memory, record events or use another stream first
  * submit what there is, and so does an allocation that the driver has to serve; the rest of the batch is then launched call by call, as
- * it is inside a seera_graph_begin recording and while the profile is on.  The stream is not captured: other threads may do what they
- * like, but what a caller enqueues on the stream by itself comes before the launches that are held back (seera_get_stream submits them).
+ * it is inside a seera_graph_begin recording, while the profile is on, and once another thread uses the stream through the library.  The
+ * stream is not captured: other threads may do what they like, but what a caller enqueues on the stream by itself comes before the launches that are held back (seera_get_stream submits them).
  * Batches nest: the outermost one counts, and the first long one inside it is submitted at its own end if the device waits for work. */
 int   seera_batch_begin(uint64_t tag);
 int   seera_batch_end(void);

@@ -72,8 +72,8 @@ struct Kept {
     }
 };
 struct State {
-    int depth = 0;
-    bool open = false;                                  // launches on `stream` are noted down
+    bool open = false;                                  // launches of the thread `owner` on `stream` are noted down
+    const int *owner = nullptr;
     bool parted = false;                                // a first part of the batch has been submitted
     uint64_t tag = 0, inner_at = 0;                     // ... and the launch count where the batch directly inside began
     cudaStream_t stream = nullptr;
@@ -92,6 +92,7 @@ constexpr uint64_t BATCH_STALE = 1024, BATCH_TURN = 64;
 // step that is waited for would else run host and device one after the other (VGG at 100 images: 557 -> 474 us).  Below that the
 // second submission (6 us) costs a small network more than the device's head start gives.
 constexpr uint64_t BATCH_PART = 12;
+thread_local int depth = 0;                             // batches that this thread has begun and not ended; its address names the thread
 State &st() { static State &s = *new State; return s; }          // not destroyed: the driver may be gone before
 
 const Layout &layout_of(const void *func) {
@@ -264,14 +265,16 @@ int submit(bool whole) {
 void open(uint64_t tag) {
     State &b = st();
     b.open = true;
+    b.owner = &depth;
     b.tag = tag;
     b.stream = rt().stream;
 }
-// Notes a launch down, or, where there is no memory for that, submits what there is and says no.
+// Notes a launch down, or, where there is no memory for that or another thread launches on the stream, submits what there is and says no.
 template <class Note>
 bool noted(cudaStream_t stream, Note note) {
     State &b = st();
     if (!b.open || stream != b.stream) return false;
+    if (b.owner != &depth) { submit(false); return false; }
     const size_t ops = b.row.ops.size();
     try {
         note();
@@ -338,10 +341,11 @@ cudaError_t __wrap_cudaMemcpyAsync(void *dst, const void *src, size_t bytes, cud
 int seera_batch_begin(uint64_t tag) {
     SEERA_ENSURE();
     State &b = st();
-    if (b.depth++ > 0) {
-        if (b.depth == 2) b.inner_at = rt().launches;
+    if (depth++ > 0) {
+        if (depth == 2) b.inner_at = rt().launches;
         return SEERA_OK;
     }
+    if (int s = submit(false)) return s;                // another thread's: the rest of it goes call by call
     b.parted = false;
     if (rt().capturing || seera_profile_enabled() || rt().stream == nullptr) return SEERA_OK;
     cudaStreamCaptureStatus status;
@@ -351,9 +355,11 @@ int seera_batch_begin(uint64_t tag) {
 }
 int seera_batch_end(void) {
     State &b = st();
-    if (b.depth == 0) return fail(SEERA_E_ARG, "batch_end: no batch is open");
-    if (--b.depth == 0) return submit(true);
-    if (!b.open || b.parted || b.depth > 1 || rt().launches - b.inner_at < BATCH_PART) return SEERA_OK;
+    if (depth == 0) return fail(SEERA_E_ARG, "batch_end: no batch is open");
+    --depth;
+    if (!b.open || b.owner != &depth) return SEERA_OK;
+    if (depth == 0) return submit(true);
+    if (b.parted || depth > 1 || rt().launches - b.inner_at < BATCH_PART) return SEERA_OK;
     if (b.last && cudaEventQuery(b.last) != cudaSuccess) { cudaGetLastError(); return SEERA_OK; }
     b.parted = true;
     if (int s = submit(true)) return s;

@@ -23,6 +23,7 @@ from __future__ import annotations
 
 import math
 import pickle
+import threading
 import weakref
 
 import numpy as np
@@ -52,27 +53,31 @@ def _new(shape):
 # wait or record events on the stream by itself.
 _batch_begin, _batch_end = sc.batch_begin, sc.batch_end        # (_batch_begin None: every pass launch by launch)
 _passes_seen = set()
-_inside = 0                          # batches open: what runs inside one has been looked over
+
+
+class _Inside(threading.local):
+    n = 0                            # batches that this thread has open: what runs inside one has been looked over
+
+
+_inside = _Inside()
 
 
 def _open_batch(tag, size):
     """True if a batch was opened; the caller then owes a _close_batch()."""
-    global _inside
     if tag is None or _batch_begin is None:
         return False
-    if not _inside and (tag, size) not in _passes_seen:
+    if not _inside.n and (tag, size) not in _passes_seen:
         if len(_passes_seen) > 4096:
             _passes_seen.clear()
         _passes_seen.add((tag, size))
         return False
     _batch_begin(tag)
-    _inside += 1
+    _inside.n += 1
     return True
 
 
 def _close_batch():
-    global _inside
-    _inside -= 1
+    _inside.n -= 1
     _batch_end()
 
 
@@ -1088,9 +1093,10 @@ class Sequential:
             if not isinstance(X, Tensor):
                 raise TypeError("Input must be a Tensor or numpy array.")
             self.model[0].inputs = X
-        tag = None if _inside else self._tag("forward")
+        inside = _inside.n
+        tag = None if inside else self._tag("forward")
         size = None if tag is None else self.model[0].inputs.value.shape
-        opened = _open_batch(0 if _inside else tag, size)      # (inside a training step's: its first part ends with the forward)
+        opened = _open_batch(0 if inside else tag, size)      # (inside a training step's: its first part ends with the forward)
         try:
             out = None
             for layer in self.model:

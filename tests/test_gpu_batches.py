@@ -429,3 +429,47 @@ def test_a_recorded_update_that_cannot_be_found_again_is_an_error(sc):
     sc.clear_status()
     for p in d:
         sc.cuda_free(p)
+
+
+def test_batches_of_two_threads(sc):
+    """Each thread's are its own: what one has ended is on the device whatever the other has open, and all calls keep their order."""
+    import threading
+    p, q = sc.cuda_ones_f(100), sc.cuda_ones_f(100)
+    sc.stream_synchronize()
+    turn, log = [threading.Event() for _ in range(6)], []
+
+    def other():
+        turn[0].wait(10)
+        sc.cuda_scaler_multiply_f(p, 10.0, 100)              # between the two of the first thread's batch, which goes on call by call
+        log.append(_device_now(p))
+        turn[1].set()
+        turn[2].wait(10)
+        sc.batch_begin(31)
+        sc.cuda_scaler_add_f(q, 1.0, 100)
+        turn[3].set()
+        turn[4].wait(10)
+        sc.cuda_scaler_multiply_f(q, 2.0, 100)
+        sc.batch_end()
+        turn[5].set()
+    t = threading.Thread(target=other)
+    t.start()
+    sc.batch_begin(30)
+    sc.cuda_scaler_add_f(p, 1.0, 100)
+    assert _device_now(p) == 1
+    turn[0].set()
+    turn[1].wait(10)
+    assert log == [20]
+    sc.cuda_scaler_add_f(p, 1.0, 100)
+    turn[2].set()
+    turn[3].wait(10)
+    sc.batch_end()
+    assert _device_now(p) == 21 and _device_now(q) == 1      # the other's is still open
+    turn[4].set()
+    turn[5].wait(10)
+    t.join()
+    assert _device_now(q) == 4
+    with pytest.raises(RuntimeError):
+        sc.batch_end()
+    sc.clear_status()
+    for x in (p, q):
+        sc.cuda_free(x)
