@@ -47,12 +47,10 @@ def _new(shape):
 
 
 # One submission for the launches of a phase (seera_batch_begin / _end): inside, the engine notes its launches down, and the end hands
-# them over as one graph - a fraction of the host time per launch and no gaps between them on the device.  A tag names the kind of pass:
-# the layers and the precision.  The first pass at a size runs launch by launch, which leaves no executable behind and lets the device
-# start at once.  Only what is this module's own runs inside a batch: a caller's layer, loss, optimizer or gradient function may launch,
-# wait or record events on the stream by itself.
+# them over as one graph - a fraction of the host time per launch and no gaps between them on the device.  A model's first pass at a size
+# runs launch by launch, which leaves no executable behind and lets the device start at once.  Only what is this module's own runs inside a
+# batch: a caller's layer, loss, optimizer or gradient function may launch, wait or record events on the stream by itself.
 _batch_begin, _batch_end = sc.batch_begin, sc.batch_end        # (_batch_begin None: every pass launch by launch)
-_passes_seen = set()
 
 
 class _Inside(threading.local):
@@ -62,16 +60,16 @@ class _Inside(threading.local):
 _inside = _Inside()
 
 
-def _open_batch(tag, size):
-    """True if a batch was opened; the caller then owes a _close_batch()."""
-    if tag is None or _batch_begin is None:
+def _open_batch(model, kind, size):
+    """True if a batch was opened, for a kind of pass that the model has made at this size before; the caller then owes a _close_batch()."""
+    if _batch_begin is None:
         return False
-    if not _inside.n and (tag, size) not in _passes_seen:
-        if len(_passes_seen) > 4096:
-            _passes_seen.clear()
-        _passes_seen.add((tag, size))
+    if (kind, size) not in model._passes:
+        if len(model._passes) > 4096:
+            model._passes.clear()
+        model._passes.add((kind, size))
         return False
-    _batch_begin(tag)
+    _batch_begin(kind)
     _inside.n += 1
     return True
 
@@ -81,8 +79,7 @@ def _close_batch():
     _batch_end()
 
 
-def _make_tag(*what):
-    return hash(what) & 0x7fffffffffffffff
+_FORWARD, _BACKWARD, _STEP = 1, 2, 3     # kinds of pass
 
 
 # ─────────────────────────────────────────────────────────────────────────────────────────────
@@ -100,7 +97,7 @@ class Tensor:
     _takes_pooled = False            # its backward takes the gradient of a 2x2 max-pool of it in pooled form
     _copies = None                   # channels-last copies of the value, made by its producer for a convolution
     _rows = None                     # row-major copies of the value, made by its producer for a Dense layer
-    _pass = None                     # (batch tag, input shape, reference to the model) of the pass it came from
+    _pass = None                     # (input shape, reference to the model) of the pass it came from
 
     def __init__(self, value, dtype="float32", is_leaf=False, device="cuda"):
         if isinstance(value, Tensor):
@@ -328,9 +325,9 @@ class autograd4nn:
         order, own = self._order()
         opened = False
         if own and self.hook._pass is not None:
-            tag, size, model = self.hook._pass
+            size, model = self.hook._pass
             model = model()
-            opened = model is not None and model._exchanges_nothing() and _open_batch(_make_tag(tag, "backward"), size)
+            opened = model is not None and model._exchanges_nothing() and _open_batch(model, _BACKWARD, size)
         try:
             self._run(order)
         finally:
@@ -957,11 +954,6 @@ _OWN_LAYERS = {c: c.forward for c in (Input, Dense, Conv2D, ConvTranspose2D, Bat
 # ─────────────────────────────────────────────────────────────────────────────────────────────
 # Sequential
 # ─────────────────────────────────────────────────────────────────────────────────────────────
-# what of a layer decides which launches it makes
-_STRUCTURE = ("in_units", "out_units", "layeract", "in_channels", "out_channels", "kernel_size", "stride", "zero_padding", "pool_size",
-              "padding", "size", "_num")
-
-
 def _train_step(model, optimizer, lossf, y):
     """One step on the model's current input: forward, loss, backward, update.  The loss."""
     loss = lossf(model.forward(), y)
@@ -1036,7 +1028,7 @@ class Sequential:
         self.model = [layers[0]] + [layer(layers[i]) for i, layer in enumerate(layers[1:])]
         self.world, self._allreduce, self._on_grad_ready = 1, None, None
         self._modal = [l for l in self.model if hasattr(l, "training")]       # layers that behave differently in evaluation
-        self._structure = hash(tuple((l.__class__.__name__,) + tuple(getattr(l, k, None) for k in _STRUCTURE) for l in self.model))
+        self._passes = set()                          # kinds and sizes of passes made (see _open_batch)
         self._build_arena()
         self._ref = weakref.ref(self)
         for l in self.param_layers:
@@ -1093,10 +1085,13 @@ class Sequential:
             if not isinstance(X, Tensor):
                 raise TypeError("Input must be a Tensor or numpy array.")
             self.model[0].inputs = X
-        inside = _inside.n
-        tag = None if inside else self._tag("forward")
-        size = None if tag is None else self.model[0].inputs.value.shape
-        opened = _open_batch(0 if inside else tag, size)      # (inside a training step's: its first part ends with the forward)
+        size = None
+        if _inside.n:                                 # part of a training step's, whose first part ends with the forward
+            _batch_begin(_STEP)
+            _inside.n += 1
+            opened = True
+        else:
+            opened = self._batchable() and _open_batch(self, _FORWARD, size := self.model[0].inputs.value.shape)
         try:
             out = None
             for layer in self.model:
@@ -1104,17 +1099,14 @@ class Sequential:
         finally:
             if opened:
                 _close_batch()
-        if tag is not None:
-            out._pass = tag, size, self._ref
+        if size is not None:
+            out._pass = size, self._ref
         return out
 
-    def _tag(self, *phase):
-        """Tag of a pass over the current input, or None where it does not run as one batch: with gradients exchanged between
-        ranks during backward, other streams take part in it."""
-        X = self.model[0].inputs
-        if self._allreduce is not None or self._on_grad_ready is not None or X.__class__ is not Tensor or not self._own_passes():
-            return None
-        return _make_tag(self._structure, sc.get_precision(), FUSE_POOL, DENSE_EPILOGUE_COPIES, *phase)
+    def _batchable(self):
+        """Whether a pass over the current input may run as one batch: with gradients exchanged between ranks during backward, other
+        streams take part in it."""
+        return (self._allreduce is None and self._on_grad_ready is None and self.model[0].inputs.__class__ is Tensor and self._own_passes())
 
     def _exchanges_nothing(self):
         return self._allreduce is None and self._on_grad_ready is None
@@ -1207,7 +1199,7 @@ class Sequential:
                 yv = cuten._wrap(st["dy"].main_ptr, (m,) + y.shape[1:])
                 yv._owns_memory = False
             self.model[0].inputs = xb
-            opened = _own_step(Optimizer, Loss) and _open_batch(self._tag("fit", Optimizer.__class__.__name__), (xb.value.shape, yv.shape))
+            opened = _own_step(Optimizer, Loss) and self._batchable() and _open_batch(self, _STEP, xb.value.shape)
             try:
                 return _train_step(self, Optimizer, Loss, Tensor(yv, is_leaf=True))
             finally:

@@ -87,7 +87,7 @@ class Trainer:
         self.opt.begin_step()
         self.model.model[0].inputs = X
         opened = (self.__class__ is Trainer and X._backward is None and S._own_step(self.opt, self.lossf)
-                  and S._open_batch(self.model._tag("step", self.precision, self.work.loss, self.work.opt["kind"]), X.value.shape))
+                  and self.model._batchable() and S._open_batch(self.model, S._STEP, X.value.shape))
         try:
             loss = self.forward_backward(X, Y)
             self.opt.step()
