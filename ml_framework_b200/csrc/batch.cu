@@ -311,6 +311,7 @@ extern "C" {
 // The library's own launches arrive here.
 cudaError_t __wrap_cudaLaunchKernel(const void *func, dim3 grid, dim3 block, void **args, size_t smem, cudaStream_t stream) {
     if (noted(stream, [&] { note_kernel(func, grid, block, args, smem, 1); })) return cudaSuccess;
+    if (rt().capturing) graph_note_launch(func, grid, block, smem);
     return __real_cudaLaunchKernel(func, grid, block, args, smem, stream);
 }
 cudaError_t __wrap_cudaLaunchKernelExC(const cudaLaunchConfig_t *config, const void *func, void **args) {
@@ -322,11 +323,13 @@ cudaError_t __wrap_cudaLaunchKernelExC(const cudaLaunchConfig_t *config, const v
     } else if (st().open && config->stream == st().stream) {
         submit(false);
     }
+    if (rt().capturing) graph_note_launch(func, config->gridDim, config->blockDim, config->dynamicSmemBytes);
     return __real_cudaLaunchKernelExC(config, func, args);
 }
 cudaError_t __wrap_cudaMemsetAsync(void *dst, int value, size_t bytes, cudaStream_t stream) {
     if (bytes && noted(stream, [&] { st().row.ops.push_back({Op::FILL, 1, (unsigned)value & 255u, dst, nullptr, {}, {}, bytes, 0, 0}); }))
         return cudaSuccess;
+    if (rt().capturing) graph_note_launch(nullptr, {}, {}, 1);
     return __real_cudaMemsetAsync(dst, value, bytes, stream);
 }
 cudaError_t __wrap_cudaMemcpyAsync(void *dst, const void *src, size_t bytes, cudaMemcpyKind kind, cudaStream_t stream) {
@@ -335,6 +338,7 @@ cudaError_t __wrap_cudaMemcpyAsync(void *dst, const void *src, size_t bytes, cud
     } else if (bytes && noted(stream, [&] { st().row.ops.push_back({Op::COPY, 1, 0, dst, src, {}, {}, bytes, 0, 0}); })) {
         return cudaSuccess;
     }
+    if (rt().capturing) graph_note_launch(nullptr, {}, {}, 2);
     return __real_cudaMemcpyAsync(dst, src, bytes, kind, stream);
 }
 

@@ -141,6 +141,7 @@ struct OptLaunch {
     float scalars[9]; int n_scalars;
 };
 int graph_note_optimizer(const OptLaunch &launch);
+void graph_note_launch(const void *func, dim3 grid, dim3 block, size_t smem);
 // kernel, grid, block and argument pointers of the launch (the pointers point into `launch`)
 void optimizer_node_params(const OptLaunch &launch, cudaKernelNodeParams &kp, void **args);
 

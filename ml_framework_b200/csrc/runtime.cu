@@ -66,7 +66,7 @@ namespace {
 struct OptNode {
     cudaGraphNode_t node;
     OptLaunch launch;
-    size_t at = 0;                                      // its place in a recording whose nodes follow one another
+    size_t at = 0;                                      // its place among the launches of the recording
 };
 struct GraphRec {
     cudaGraph_t graph = nullptr;
@@ -78,7 +78,9 @@ struct GraphRec {
     std::vector<OptNode> optimizers;                    // recorded optimizer updates, whose scalars change from replay to replay
     std::vector<int> finish_slots;                      // counters of the recorded launches that finish in their last block
     bool lost_update = false;                           // ... one of which is not among them
-    uint64_t row = 0;                                   // hash of its kernels and grids if its nodes follow one another, else 0
+    size_t noted = 0;                                   // launches recorded, and a hash of their kernels and grids
+    uint64_t hash = 1469598103934665603ull;
+    uint64_t row = 0;                                   // the hash if the nodes are those launches, one after the other; else 0
 };
 static std::vector<GraphRec *> &live_graphs() { static std::vector<GraphRec *> v; return v; }
 struct Pool {
@@ -162,7 +164,7 @@ int graph_note_optimizer(const OptLaunch &launch) {
     if (rt().graph_test_lose_update) n = 2;
     rt().graph_test_lose_update = false;                // one update only
     if (e == cudaSuccess && n == 1) {
-        p.cur->optimizers.push_back({deps[0], launch});
+        p.cur->optimizers.push_back({deps[0], launch, p.cur->noted - 1});
         return SEERA_OK;
     }
     cudaGetLastError();
@@ -184,49 +186,28 @@ struct Spare {
 };
 std::vector<Spare> &spares() { static std::vector<Spare> v; return v; }
 }  // namespace
-// The nodes of a graph in order, if each follows the one before it; else nothing.
-static std::vector<cudaGraphNode_t> chain_of(cudaGraph_t g) {
-    std::vector<cudaGraphNode_t> order;
-    size_t nodes = 0, edges = 0, roots = 1;
-    cudaGraphNode_t at = nullptr;
+// A launch, fill or copy goes into the open recording (batch.cu, which sees them all).
+void graph_note_launch(const void *func, dim3 grid, dim3 block, size_t smem) {
+    GraphRec *g = pool().cur;
+    if (!g) return;
+    auto mix = [g](uint64_t v) { g->hash = (g->hash ^ v) * 1099511628211ull; g->hash ^= g->hash >> 32; };
+    mix((uint64_t)(uintptr_t)func);
+    mix(((uint64_t)grid.x << 32) ^ ((uint64_t)grid.y << 16) ^ grid.z);
+    mix(((uint64_t)smem << 32) ^ ((uint64_t)block.x << 16) ^ (block.y << 8) ^ block.z);
+    g->noted++;
+}
+// The number of nodes of a graph if each follows the one before it, else 0.
+static size_t chain_length(cudaGraph_t g) {
+    size_t nodes = 0, edges = 0, roots = 0;
     if (cudaGraphGetNodes(g, nullptr, &nodes) != cudaSuccess || cudaGraphGetEdges(g, nullptr, nullptr, &edges) != cudaSuccess ||
-        !nodes || edges != nodes - 1 || cudaGraphGetRootNodes(g, nullptr, &roots) != cudaSuccess || roots != 1 ||
-        cudaGraphGetRootNodes(g, &at, &roots) != cudaSuccess) {
+        cudaGraphGetRootNodes(g, nullptr, &roots) != cudaSuccess || !nodes || roots != 1 || edges != nodes - 1) {
         cudaGetLastError();
-        return order;
+        return 0;
     }
     std::vector<cudaGraphNode_t> from(edges), to(edges);
-    if (edges && cudaGraphGetEdges(g, from.data(), to.data(), &edges) != cudaSuccess) { cudaGetLastError(); return order; }
-    std::vector<std::pair<cudaGraphNode_t, cudaGraphNode_t>> next(edges);
-    for (size_t i = 0; i < edges; i++) next[i] = {from[i], to[i]};
-    std::sort(next.begin(), next.end());
-    while (at) {
-        order.push_back(at);
-        auto it = std::lower_bound(next.begin(), next.end(), std::make_pair(at, cudaGraphNode_t(nullptr)));
-        at = it != next.end() && it->first == at && order.size() < nodes ? it->second : nullptr;
-    }
-    if (order.size() != nodes) order.clear();           // something has two successors
-    return order;
-}
-
-// Notes what a recording is made of (GraphRec::row, OptNode::at).
-static void describe(GraphRec *g) {
-    const std::vector<cudaGraphNode_t> chain = chain_of(g->graph);
-    if (chain.empty()) return;
-    uint64_t h = 1469598103934665603ull;
-    auto mix = [&h](uint64_t v) { h = (h ^ v) * 1099511628211ull; h ^= h >> 32; };
-    for (size_t i = 0; i < chain.size(); i++) {
-        for (OptNode &o : g->optimizers) if (o.node == chain[i]) o.at = i;
-        cudaGraphNodeType type;
-        cudaKernelNodeParams kp = {};
-        if (cudaGraphNodeGetType(chain[i], &type) != cudaSuccess ||
-            (type == cudaGraphNodeTypeKernel && cudaGraphKernelNodeGetParams(chain[i], &kp) != cudaSuccess)) { cudaGetLastError(); return; }
-        mix((uint64_t)type);
-        mix((uint64_t)(uintptr_t)kp.func);
-        mix(((uint64_t)kp.gridDim.x << 32) ^ ((uint64_t)kp.gridDim.y << 16) ^ kp.gridDim.z);
-        mix(((uint64_t)kp.sharedMemBytes << 32) ^ ((uint64_t)kp.blockDim.x << 16) ^ (kp.blockDim.y << 8) ^ kp.blockDim.z);
-    }
-    g->row = h | 1;
+    if (edges && cudaGraphGetEdges(g, from.data(), to.data(), &edges) != cudaSuccess) { cudaGetLastError(); return 0; }
+    std::sort(from.begin(), from.end());
+    return std::adjacent_find(from.begin(), from.end()) == from.end() ? nodes : 0;       // nothing has two successors
 }
 static void spares_trim(size_t keep) {
     auto &v = spares();
@@ -561,7 +542,7 @@ void *seera_graph_end(void) {
     rt().launches = g->launches_at_begin;               // recorded, not executed
     cudaError_t e = cudaStreamEndCapture(rt().stream, &g->graph);
     if (e == cudaSuccess && !g->collectives) {
-        describe(g);
+        if (chain_length(g->graph) == g->noted) g->row = g->hash | 1;
         if (g->row) take_spare(g);
     }
     if (e == cudaSuccess && !g->exec) e = cudaGraphInstantiate(&g->exec, g->graph, 0);
