@@ -159,11 +159,6 @@ void batch_trim();                          // gives back the executable graphs 
 // Lets a kernel be launched with up to `bytes` of dynamic shared memory.  The limit is the kernel's and not a launch's: it is only ever
 // raised, since a launch that has been noted down comes after this call.
 cudaError_t allow_smem(const void *kernel, size_t bytes);
-// RAII bracket over the launches of one entry (no-op inside a batch that is open already).
-struct Batch {
-    Batch(uint64_t tag) { seera_batch_begin(tag); }
-    ~Batch() { seera_batch_end(); }
-};
 
 // Pool-backed scratch for internal use (split-K partials, operand shadows).
 void graph_note_collective();              // runtime.cu: the open capture records a collective

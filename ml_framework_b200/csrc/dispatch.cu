@@ -15,7 +15,7 @@
 using namespace seera;
 
 // An entry of five and more launches submits them as one batch from its second call with the same shape on: launched one by one they leave
-// 2 us between kernels, and a small call is bound by launching them (2.75 us each on the host, 0.7 in a batch).  256 x 256 channels on 256 images
+// 2 us between kernels, and a small call is bound by launching them (2.75 us each on the host, 0.1 to 0.4 in a batch).  256 x 256 channels on 256 images
 // of 14 x 14, one bf16 pass: 158 -> 151 us; a small call 60 -> 39.  Inside a pass that is a batch or a recording already nothing changes.
 namespace {
 uint64_t entry_tag(std::initializer_list<long long> what) {

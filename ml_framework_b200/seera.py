@@ -1430,8 +1430,9 @@ _LOSSES = (Loss.categorical_cross_entropy, Loss.mse, Loss.mae, Loss.binary_cross
 # Optimizers: one fused launch over the whole parameter arena
 # ─────────────────────────────────────────────────────────────────────────────────────────────
 class _Optimizer:
-    """Keeps its step scalars in a small device buffer so that a captured step graph can be replayed: the
-    update kernel reads them at run time, `advance()` refreshes them before each replay."""
+    """The scalars of a step travel with the update's launch, and in a recorded step they are replaced in the graph before each replay
+    (graph_set_scalars).  Where the update is enqueued apart from them - bucket by bucket during backward, or behind a sum over the
+    ranks outside the recording - its kernel reads them from a small device buffer, which `advance()` refreshes."""
 
     def __init__(self, model):
         if not isinstance(model, Sequential):
