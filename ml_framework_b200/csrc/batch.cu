@@ -227,6 +227,34 @@ bool room() {
     return true;
 }
 
+// The executable for what has been noted down, with its arguments, or null.
+const Kept *executable(bool whole) {
+    State &b = st();
+    const uint64_t key = key_of(b.tag, b.row);
+    Kept *k = nullptr;
+    try {
+        auto it = b.kept.find(key);
+        if (it != b.kept.end()) {
+            k = it->second.get();
+            if (!bring_up(*k, b.row)) {
+                b.kept.erase(it);
+                return nullptr;
+            }
+        } else if (whole && !b.sighted.insert(key).second && room()) {
+            auto fresh = std::make_unique<Kept>();
+            if (!make(*fresh, b.row)) return nullptr;
+            k = fresh.get();
+            b.kept[key] = std::move(fresh);
+        }
+        if (b.sighted.size() > BATCH_SIGHTED_MAX) b.sighted.clear();
+    } catch (const std::bad_alloc &) {                   // no host memory for one: call by call
+        b.kept.clear();
+        return nullptr;
+    }
+    if (k) k->used = b.clock;
+    return k;
+}
+
 // Hands over what has been noted down.  `whole`: all of a batch, whose executable is worth keeping.
 int submit(bool whole) {
     State &b = st();
@@ -236,19 +264,8 @@ int submit(bool whole) {
     cudaError_t e = cudaSuccess;
     if (!row.ops.empty()) {
         ++b.clock;
-        const uint64_t key = key_of(b.tag, row);
-        auto it = b.kept.find(key);
-        Kept *k = it == b.kept.end() ? nullptr : it->second.get();
-        if (k && !bring_up(*k, row)) {
-            b.kept.erase(it);
-            k = nullptr;
-        } else if (!k && whole && !b.sighted.insert(key).second && room()) {
-            auto fresh = std::make_unique<Kept>();
-            if (make(*fresh, row)) k = (b.kept[key] = std::move(fresh)).get();
-        }
-        if (b.sighted.size() > BATCH_SIGHTED_MAX) b.sighted.clear();
+        const Kept *k = executable(whole);
         if (k) {
-            k->used = b.clock;
             e = cudaGraphLaunch(k->exec, b.stream);
         } else {
             for (size_t i = 0; i < row.ops.size() && e == cudaSuccess; i++) e = launch_alone(row.ops[i], row, b.stream);
