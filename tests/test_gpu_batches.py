@@ -255,7 +255,7 @@ def test_predictions_over_more_sizes_than_executables_are_kept(sc, monkeypatch):
     for batched in (False, True):
         monkeypatch.setattr(S, "_batch_begin", sc.batch_begin if batched else None)
         best = 1e9
-        for rep in range(4):
+        for rep in range(12):
             sc.stream_synchronize()
             t = time.perf_counter()
             out = [model.predict(x) for x in xs]
