@@ -159,7 +159,7 @@ struct StorePixelRows {    // m = (img, p): out[(img*Nch + n)*P + p]
 #pragma unroll
             for (int i = 0; i < 8; i++) o8[i] = n + i < Nch ? v[8 * c + i] : 0.f;
             const long long o = (long long)m * Cp + n;
-            store_split8_n(o8, ns, enc, cp[0] + o, cp[1] + o, cp[2] + o);
+            store_split8_rolled(o8, ns, enc, cp[0] + o, cp[1] + o, cp[2] + o);
         }
     }
 };

@@ -224,6 +224,36 @@ __device__ __forceinline__ void store_split8_n(float *v, int ns, const Enc &e, _
     else if (ns == 2) store_split8<2>(v, e, d0, d1, d2);
     else store_split8<3>(v, e, d0, d1, d2);
 }
+// The same as one body for each copy in turn, for code that runs once or twice per launch and waits for its own instructions.
+__device__ __forceinline__ void store_split8_rolled(float *v, int ns, const Enc &e, __nv_bfloat16 *d0, __nv_bfloat16 *d1, __nv_bfloat16 *d2) {
+    const float f = e.fmt ? enc_factor(e) : 1.f;
+#pragma unroll
+    for (int i = 0; i < 8; i++) v[i] *= f;
+#pragma unroll 1
+    for (int c = 0; c < ns; c++) {
+        __nv_bfloat16 *d = c == 0 ? d0 : (c == 1 ? d1 : d2);
+        *reinterpret_cast<uint4 *>(d) = e.fmt ? split_chunk_f16(v) : split_chunk(v);
+    }
+}
+// 4 consecutive values, 8-byte chunks; v is consumed.
+__device__ __forceinline__ void store_split4_n(float *v, int ns, const Enc &e, __nv_bfloat16 *d0, __nv_bfloat16 *d1, __nv_bfloat16 *d2) {
+    const float f = e.fmt ? enc_factor(e) : 1.f;
+#pragma unroll
+    for (int i = 0; i < 4; i++) v[i] *= f;
+#pragma unroll 1
+    for (int c = 0; c < ns; c++) {
+        __nv_bfloat16 *d = c == 0 ? d0 : (c == 1 ? d1 : d2);
+        uint2 h;
+        if (e.fmt) {
+            h.x = pack_f16x2_sat(v[0], v[1]); h.y = pack_f16x2_sat(v[2], v[3]);
+            v[0] -= f16_bits_to_float(h.x, 0); v[1] -= f16_bits_to_float(h.x, 1); v[2] -= f16_bits_to_float(h.y, 0); v[3] -= f16_bits_to_float(h.y, 1);
+        } else {
+            h.x = pack_bf16x2(v[0], v[1]); h.y = pack_bf16x2(v[2], v[3]);
+            v[0] -= bf16_bits_to_float(h.x, 0); v[1] -= bf16_bits_to_float(h.x, 1); v[2] -= bf16_bits_to_float(h.y, 0); v[3] -= bf16_bits_to_float(h.y, 1);
+        }
+        *reinterpret_cast<uint2 *>(d) = h;
+    }
+}
 // The same for one value (ns known at run time).
 __device__ __forceinline__ void store_split1(float v, int ns, const Enc &e, __nv_bfloat16 *d0, __nv_bfloat16 *d1, __nv_bfloat16 *d2) {
     unsigned short *u0 = reinterpret_cast<unsigned short *>(d0), *u1 = reinterpret_cast<unsigned short *>(d1),
