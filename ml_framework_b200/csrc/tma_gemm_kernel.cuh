@@ -242,6 +242,7 @@ struct TmaGemmParams {
     int pair;                // 1: launched as clusters of two CTAs sharing 256-row tiles (tcgen05 cta_group::2)
     int issuers;             // 1 or 2 threads issue the MMAs of a k-step (the K = 16 slices dealt round robin), each into its own
                              // accumulator; the epilogue adds the accumulators up
+    int joined;              // split products with B's first two copies side by side as one operand of 2 x bn columns (below)
     // convolution geometry for the im2col modes
     int OW, OHW;             // output width and pixels per image of the traversal
     int sw, sh, pw, ph;      // window stride and lower padding
@@ -273,13 +274,21 @@ constexpr int TG_THREADS = 384, TG_EPI_WARP0 = 4, TG_EPI_WARPS = 8;
 // then K split).  The operand ring keeps streaming across tile boundaries and the accumulator is double-buffered in
 // TMEM, so the epilogue of tile i overlaps the main loop of tile i+1.
 //
-// One thread can issue a tcgen05.mma only every 80-90 clocks, whatever the instruction's size (measured: 88 clocks per MMA at
-// N = 64 from one thread, the same MMAs from two threads at twice the rate), while a 128 x N x 16 instruction occupies the
-// tensor pipe for N / 2 clocks.  With N <= 128 a single issuing thread therefore leaves the pipe idle half of the time or more.
-// So two threads (lane 0 of warps 1 and 2) issue where the accumulators fit: they wait for the same stage, take the K = 16 slices
-// of the k-step alternately, each into an accumulator of its own (MMAs of different threads are not ordered among themselves), and each commits
-// to the stage's "empty" barrier and to the tile's "accumulator full" barrier, which count `issuers` arrivals.  TMEM holds
-// 2 buffers x issuers x bn columns (at most 512); the epilogue adds the accumulators of a buffer while it drains them.
+// What an MMA costs (a loop of MMAs alone, clocks per K = 16 slice of 128 rows): the larger of N / 2 on the tensor pipe and
+// 32 + N / 4 for its operands, which come from shared memory at 128 bytes a clock (4 KB of A, 32 N bytes of B): 40 / 48 / 64 / 128 at
+// N = 32 / 64 / 128 / 256.  One thread keeps up with that; commits cost nothing measurable.
+//
+// Split products (NS = 2: A0 B0 + A0 B1 + A1 B0; NS = 3: the six products down to 2^-16 of the first) therefore take B0 and B1, which
+// lie one after the other in a stage, as ONE operand of 2 x bn columns wherever that is at most 256 wide: A0 is read once for two
+// products, whose sums go to two accumulators side by side.  A slice of NS = 2 takes 64 + 48 clocks instead of 3 x 48 at
+// bn = 64 (88 for 120 at 32), one of NS = 3 2 x 64 + 2 x 48 instead of 288; at bn = 128 the tensor pipe bounds both forms, but the joined one
+// leaves a fifth of the reads of shared memory to the epilogue (131072 x 128 x 576 with the pool: 48.3 -> 47.5 us; NS = 3 at
+// bn = 64, 25600 x 64 x 1152: 34.3 -> 31.8).  Sums in two accumulators are also shorter chains: 1.92e-6 -> 1.02e-6 of error at NS = 3
+// against float64, 1.08e-6 -> 7.1e-7 at NS = 2 on fp16 (512 x 64 x 576).  The epilogue adds the two accumulators; TMEM holds 2 buffers x 2 x bn columns (at most 512).
+//
+// Products of one copy with N <= 128 are issued by two threads (lane 0 of warps 1 and 2), which take the K = 16 slices of a
+// k-step alternately, each into an accumulator of its own (MMAs of different threads are not ordered among themselves), and
+// commit to the stage's "empty" and the tile's "accumulator full" barriers, which count `issuers` arrivals.
 template <int NS, class CS, bool PAIR>
 __global__ void __launch_bounds__(TG_THREADS, 1)
 tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant__ CUtensorMap mapA1,
@@ -311,7 +320,9 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
     unsigned char *epi_smem = smem + (size_t)stages * stage_bytes;   // one EPI_WARP_SMEM per epilogue warp after the ring
     const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[8]), tfull0 = smem_u32(&bars[16]), tempty0 = smem_u32(&bars[18]);
     const int issuers = PAIR ? 1 : p.issuers;
-    const uint32_t tmem_cols = (uint32_t)(2 * issuers * bn < 32 ? 32 : 2 * issuers * bn);
+    const bool joined = !PAIR && NS >= 2 && p.joined;
+    const int nacc = joined ? 2 : issuers;                    // accumulators of a buffer, bn columns apart
+    const uint32_t tmem_cols = (uint32_t)(2 * nacc * bn < 32 ? 32 : 2 * nacc * bn);
 
     if (t == 0) {
         abort_flag = 0;
@@ -443,6 +454,7 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
         const int me = warp - 1;
         uint32_t idesc = umma_idesc_16bit(bn, p.a_fp16, p.b_fp16) | ((uint32_t)(a_mn ? 1 : 0) << 15) | ((uint32_t)p.b_mn << 16);
         if (PAIR) idesc = (idesc & ~(31u << 24)) | ((uint32_t)(TM >> 4) << 24);          // M = 256 over the two CTAs
+        const uint32_t idesc2 = umma_idesc_16bit(2 * bn, p.a_fp16, p.b_fp16) | ((uint32_t)(a_mn ? 1 : 0) << 15) | ((uint32_t)p.b_mn << 16);
         const uint32_t a_step = a_mn ? 2048u : 32u, b_step = p.b_mn ? 2048u : 32u;   // bytes per K=16 slice
         // split products kept: hi*hi | + hi*lo, lo*hi | + hi*lo2, lo2*hi, lo*lo
         constexpr int NPROD = NS == 1 ? 1 : (NS == 2 ? 3 : 6);
@@ -465,7 +477,7 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
             alive = mbar_wait(tempty0 + 8 * buf, (((uint32_t)local >> 1) & 1u) ^ 1u, abortp, p.status, 4, p.wait_clocks);
             if (!alive) break;
             tc_fence_after();
-            const uint32_t d_tmem = tmem_base + (uint32_t)((buf * issuers + me) * bn);
+            const uint32_t d_tmem = tmem_base + (uint32_t)((buf * nacc + me) * bn);
             uint32_t acc = 0;
             for (int kt = 0; kt < ktiles && alive; kt++) {
                 alive = mbar_wait(full0 + 8 * s, ph, abortp, p.status, 2, p.wait_clocks);
@@ -486,8 +498,22 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
                         else umma_bf16_add(d_tmem, da[pa[q]], db[pb[q]], idesc);
                     }
                 };
+                // the same with B0 and B1 as one operand: hi*(hi, lo) | lo*(hi, lo) and the two with a third copy, or lo*hi
+                auto slice_joined = [&](uint64_t dsa, uint64_t dsb, bool first) {
+                    umma_bf16(d_tmem, dsa, dsb, idesc2, first ? acc : 1u);
+                    if (NS == 2) {
+                        umma_bf16_add(d_tmem + (uint32_t)bn, dsa + a_copy16, dsb, idesc);
+                    } else {
+                        umma_bf16_add(d_tmem, dsa + a_copy16, dsb, idesc2);
+                        umma_bf16_add(d_tmem + (uint32_t)bn, dsa, dsb + 2u * b_copy16, idesc);
+                        umma_bf16_add(d_tmem + (uint32_t)bn, dsa + 2u * a_copy16, dsb, idesc);
+                    }
+                };
                 if (leader) {
-                if (issuers == 2) {
+                if (NS >= 2 && joined) {
+#pragma unroll
+                    for (int jj = 0; jj < TC_BK / 16; jj++) slice_joined(das + (uint32_t)jj * a_step16, dbs + (uint32_t)jj * b_step16, jj == 0);
+                } else if (issuers == 2) {
 #pragma unroll
                     for (int jj = 0; jj < TC_BK / 32; jj++) slice(das + (uint32_t)(2 * jj) * a_step16, dbs + (uint32_t)(2 * jj) * b_step16, jj == 0);
                 } else {
@@ -521,15 +547,15 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
                 __syncwarp();
                 if (lane == 0) { if (PAIR) mbar_arrive_cluster(tempty_at + 8 * buf); else mbar_arrive(tempty0 + 8 * buf); }
             };
-            const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * issuers * bn + c_first);
+            const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * nacc * bn + c_first);
             if (c_first >= bn)                                     // a 32-column tile has one chunk
                 release();
             else if (p.pool_on)
-                drain_accumulator_pooled(taddr, m0 + q * 32, n0, c_first, bn, 64, p.M, p.N, p.bias, p.act, p.pool, stage, out_scale, issuers,
+                drain_accumulator_pooled(taddr, m0 + q * 32, n0, c_first, bn, 64, p.M, p.N, p.bias, p.act, p.pool, stage, out_scale, nacc,
                                          (uint32_t)bn, release);
             else
                 drain_accumulator(taddr, m0 + q * 32, n0, c_first, bn, 64, p.M, p.N, cs, p.partial, (long long)z * p.M * p.N, stage, p.bias,
-                                  p.act, out_scale, issuers, (uint32_t)bn, release);
+                                  p.act, out_scale, nacc, (uint32_t)bn, release);
         }
     }
     tc_fence_before();
@@ -630,9 +656,10 @@ inline int tma_pick_bn(int N, int ns, int b_mn) {
 inline void tma_plan(TmaGemmParams &p, int ns, bool allow_split) {
     p.bn = tma_pick_bn(p.N, ns, p.b_mn);
     p.pair = 0;
-    // MMA-issuing threads: two where TMEM has room for their accumulators (2 buffers x issuers x bn <= 512 columns); one thread
-    // keeps up with 256-column instructions by itself
-    p.issuers = p.bn <= 128 ? 2 : 1;
+    // split products: one thread, B's first two copies as one operand; products of one copy: two threads where TMEM has room for
+    // their accumulators (2 buffers x issuers x bn <= 512 columns), one for 256-column instructions
+    p.joined = ns >= 2 && p.bn <= 128;
+    p.issuers = p.bn <= 128 && !p.joined ? 2 : 1;
     if (rt().mma_issuers && rt().mma_issuers < p.issuers) p.issuers = rt().mma_issuers;
     if (!rt().pair_tiles || ns > 2 || rt().sm_count < 4) return;
     int bn = p.bn;
@@ -642,13 +669,14 @@ inline void tma_plan(TmaGemmParams &p, int ns, bool allow_split) {
     if (!allow_split && pair_tiles < rt().sm_count / 2) return;
     p.bn = bn;
     p.pair = 1;
+    p.joined = 0;
 }
 
 // Launches the kernel on prepared tensor maps.  p.M, p.N, p.K (contraction length in elements), a_mode, b_mn, bn
 // and the geometry fields must be set; kchunk, stages, partial and status are filled here.
 template <class CS>
 int launch_tma_gemm(const TmaMaps &maps, TmaGemmParams p, const CS &cs, int ns, bool allow_split, double flops, const char *name) {
-    if (p.issuers != 2 || p.pair || 4 * p.bn > 512) p.issuers = 1;      // TMEM has 512 columns
+    if (p.issuers != 2 || p.pair || p.joined || 4 * p.bn > 512) p.issuers = 1;      // TMEM has 512 columns
     const int tm = p.pair ? 2 * TC_BM : TC_BM;
     size_t stage = (size_t)ns * (TC_BM * 128 + (size_t)(p.pair ? p.bn / 2 : p.bn) * 128);
     // 227 KB per CTA on sm_100a; keep 2 KB for the kernel's static shared memory and alignment slack

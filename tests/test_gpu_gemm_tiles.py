@@ -1,0 +1,71 @@
+"""Tiles of the TMA-fed products where they can go wrong: accumulator widths with the operand copies of B joined, ragged edges, every
+activation of the epilogues, windows of a pooled epilogue without one maximum.  Against float64."""
+import numpy as np
+import pytest
+
+from conftest import rel_l2
+
+pytestmark = pytest.mark.gpu
+
+#: bf16x3 leaves 2^-17 of a product out, bf16x6 and fp16x3 2^-22 or less; their sums run in 32 bits (see test_gpu_tensorcore.py).
+TOL = {1: 1e-2, 2: 2e-5, 3: 2e-6, 4: 1e-5}
+
+
+@pytest.fixture
+def sc():
+    from ml_framework_b200 import capi, seera_cuda as sc
+    sc.init(0)
+    sc.set_option("skinny_gemm", 0)
+    yield sc
+    sc.set_option("skinny_gemm", 1)
+    sc.set_precision(0)
+    assert capi.load().seera_tc_device_status() == 0
+
+
+def activated(z, act):
+    return [z, np.maximum(z, 0), 1 / (1 + np.exp(-z)), np.tanh(z)][act]
+
+
+@pytest.mark.parametrize("mode", [1, 2, 3, 4])
+@pytest.mark.parametrize("M,N,K", [(127, 17, 65), (129, 64, 192), (260, 65, 640), (33, 96, 130), (300, 131, 72), (128, 257, 448)])
+def test_widths_and_edges(sc, mode, M, N, K):
+    sc.set_precision(mode)
+    rs = np.random.RandomState(M + N + K)
+    a, w, b = (rs.standard_normal(s).astype(np.float32) for s in ((M, K), (K, N), (N,)))
+    g = (rs.standard_normal((M, N)) / 8).astype(np.float32)
+    act = (M + mode) % 4
+    w /= np.float32(np.sqrt(K))
+    ad, wd, bd, gd = (sc.to_device_f32(t.ravel()) for t in (a, w, b, g))
+    y, da, dw = (sc.cuda_malloc_f32(n) for n in (M * N, M * K, K * N))
+    sc.matmul_bias_act_fwd(ad, wd, bd, y, M, N, K, act)
+    ref = activated(a.astype(np.float64) @ w + b, act)
+    assert rel_l2(sc.to_host_f32(y, (M, N)), ref) < TOL[mode]
+    sc.cuda_matmul_bwd(ad, wd, gd, da, dw, M, N, K, 1)
+    assert rel_l2(sc.to_host_f32(da, (M, K)), g.astype(np.float64) @ w.T) < TOL[mode]
+    assert rel_l2(sc.to_host_f32(dw, (K, N)), a.T.astype(np.float64) @ g) < (1e-3 if mode == 4 else TOL[mode])      # one fp16 product there
+    for p in (ad, wd, bd, gd, y, da, dw):
+        sc.cuda_free(p)
+
+
+@pytest.mark.parametrize("act", [0, 1, 2, 3])
+@pytest.mark.parametrize("N,C,H,F", [(3, 16, 16, 40), (5, 72, 8, 33), (9, 24, 4, 130)])
+def test_pooled_epilogue(sc, act, N, C, H, F):
+    """The pool of the same layer's own output, bit for bit: values, and the first of equal maxima."""
+    sc.set_precision(3)
+    rs = np.random.RandomState(N + C + F + act)
+    x = rs.standard_normal((N, C, H, H)).astype(np.float32)
+    w = (rs.standard_normal((F, C, 3, 3)) / np.sqrt(9 * C)).astype(np.float32)
+    b = rs.standard_normal(F).astype(np.float32)
+    w[1], b[1] = 0, -0.5                                     # all equal
+    b[2] = np.inf
+    xd, wd, bd = (sc.to_device_f32(t.ravel()) for t in (x, w, b))
+    n = N * F * H * H // 4
+    out, mask, y = sc.cuda_malloc_f32(n), sc.cuda_malloc_i32(n), sc.cuda_malloc_f32(4 * n)
+    assert sc.conv2d_pool_fusable(N, C, H, H, F, 3, 3, 1, 1, 1, 1)
+    sc.shadow_free(sc.conv2d_bias_act_pool_fwd_s(xd, wd, bd, out, mask, N, C, H, H, F, 3, 3, 1, 1, 1, 1, act, 0, False)[0])
+    sc.shadow_free(sc.conv2d_bias_act_fwd_s(xd, wd, bd, y, N, C, H, H, F, 3, 3, 1, 1, 1, 1, act, 0))
+    full = sc.to_host_f32(y, (N, F, H // 2, 2, H // 2, 2)).transpose(0, 1, 2, 4, 3, 5).reshape(N, F, H // 2, H // 2, 4)
+    assert np.array_equal(sc.to_host_f32(out, full.shape[:-1]), full.max(-1))
+    assert np.array_equal(sc.to_host_i32(mask, full.shape[:-1]), full.argmax(-1))
+    for p in (xd, wd, bd, out, mask, y):
+        sc.cuda_free(p)
