@@ -334,13 +334,13 @@ cudaError_t __wrap_cudaLaunchKernel(const void *func, dim3 grid, dim3 block, voi
 cudaError_t __wrap_cudaLaunchKernelExC(const cudaLaunchConfig_t *config, const void *func, void **args) {
     const bool cluster = config->numAttrs == 1 && config->attrs[0].id == cudaLaunchAttributeClusterDimension &&
                          config->attrs[0].val.clusterDim.y == 1 && config->attrs[0].val.clusterDim.z == 1;
+    const unsigned c = cluster ? config->attrs[0].val.clusterDim.x : 1;
     if (config->numAttrs == 0 || cluster) {
-        const unsigned c = cluster ? config->attrs[0].val.clusterDim.x : 1;
         if (noted(config->stream, [&] { note_kernel(func, config->gridDim, config->blockDim, args, config->dynamicSmemBytes, c); })) return cudaSuccess;
     } else if (st().open && config->stream == st().stream) {
         submit(false);
     }
-    if (rt().capturing) graph_note_launch(func, config->gridDim, config->blockDim, config->dynamicSmemBytes);
+    if (rt().capturing) graph_note_launch(func, config->gridDim, config->blockDim, config->dynamicSmemBytes + ((size_t)c << 24));
     return __real_cudaLaunchKernelExC(config, func, args);
 }
 cudaError_t __wrap_cudaMemsetAsync(void *dst, int value, size_t bytes, cudaStream_t stream) {

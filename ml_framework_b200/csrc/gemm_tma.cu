@@ -112,6 +112,27 @@ const Shadow *rows_usable(const seera_rows *h, int ns, int rows, int cols, int c
         h->s.enc.dscale != want.dscale) return nullptr;
     return &h->s;
 }
+// One answer per device and size.  Asked of this kernel, whose blocks take a whole SM as all of these do.
+int clusters_at_once(int size) {
+    static std::atomic<int> known[9];
+    if (size < 2 || size > 8) return 0;
+    int n = known[size].load(std::memory_order_relaxed);
+    if (n) return n - 1;
+    auto kern = tma_gemm_kernel<1, StoreDense, false>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(rt().sm_count / size * size)); cfg.blockDim = dim3(TG_THREADS); cfg.dynamicSmemBytes = 200 * 1024;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)size; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    int got = 0;
+    if (allow_smem((const void *)kern, 225 * 1024) != cudaSuccess || cudaOccupancyMaxActiveClusters(&got, kern, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        got = 0;
+    }
+    known[size].store(got + 1, std::memory_order_relaxed);
+    return got;
+}
 static bool dense_keeps() { return rt().precision != 0 && rt().dense_tma; }
 
 }  // namespace seera

@@ -22,7 +22,7 @@ __device__ __forceinline__ void epi_put_row(float *stage, int lane, const float 
 // loop unrolled and both activation functions expanded per value that code was fetched from L2 for most of the time (ncu: 5 to 7
 // warps per issue in the no_instruction stall; a 128 x 128 pooled tile took 3.8 us).  So the loops over a chunk's pieces are
 // rolled, ReLU is a select, and the activations with a function call go through one rolled loop over the staging tile.  Dense products
-// of a few tiles gain most (100 x 256 x 1024 in six products 10.5 -> 7.2 us, 1000 x 1024 gradients in one 13.1 -> 9.6).
+// of a few tiles gain most (100 x 256 x 1024 in six products 10.5 -> 7.2 us, a 1024 x 256 x 512 weight gradient in one 12.5 -> 9.4).
 __device__ __forceinline__ float epilogue_act(float z, int act) {
     switch (act) {
         case 1: return z > 0.f ? z : 0.f;               // SEERA_ACT_RELU
@@ -153,6 +153,19 @@ __device__ __forceinline__ void put_chunk_columns(const float *v, float *row0, l
                 maybe_copy_out4(cs, row_base + r, n, x, 0);
             }
         }
+    }
+}
+
+// A chunk whose row and column origin are known only now (the functor's address is formed per chunk).
+template <class CS>
+__device__ __forceinline__ void put_chunk(float *v, int row_base, int n0, int M, int N, const CS &cs, float *stage, const float *bias, int act,
+                                          float scale) {
+    if (CS::kMContiguous) {
+        const int m = row_base + (threadIdx.x & 31);
+        put_chunk_rows(v, m < M ? cs.row(m) : nullptr, cs.nstride(), m, n0, N, cs, stage, bias, act, scale);
+    } else {
+        float *row0 = cs.row(row_base);
+        put_chunk_columns(v, row0, cs.row(row_base + 1) - row0, row_base, min(32, M - row_base), n0, N, cs, true, stage, bias, act, scale);
     }
 }
 

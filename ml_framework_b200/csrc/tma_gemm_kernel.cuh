@@ -3,6 +3,8 @@
 #pragma once
 #include <cuda.h>
 
+#include <atomic>
+
 #include "common.cuh"
 #include "contraction_functors.cuh"
 #include "tc_epilogue.cuh"
@@ -198,6 +200,9 @@ __device__ __forceinline__ void umma2_bf16(uint32_t d_tmem, uint64_t adesc, uint
                  "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
                  ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
+__device__ __forceinline__ void st_cluster_f4(uint32_t cluster_addr, float x, float y, float z, float w) {
+    asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(cluster_addr), "f"(x), "f"(y), "f"(z), "f"(w) : "memory");
+}
 // arrives on the barrier at this shared-memory offset in BOTH CTAs of the pair once the MMAs issued so far have finished
 __device__ __forceinline__ void umma2_commit_both(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
@@ -242,6 +247,7 @@ struct TmaGemmParams {
     int pair;                // 1: launched as clusters of two CTAs sharing 256-row tiles (tcgen05 cta_group::2)
     int issuers;             // 1 or 2 threads issue the MMAs of a k-step (the K = 16 slices dealt round robin), each into its own
                              // accumulator; the epilogue adds the accumulators up
+    int shared;              // CTAs of a cluster that share one tile, each with its part of the contraction (1: none)
     int joined;              // split products with B's first two copies side by side as one operand of 2 x bn columns (below)
     // convolution geometry for the im2col modes
     int OW, OHW;             // output width and pixels per image of the traversal
@@ -305,7 +311,10 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
     // PAIR: the two CTAs of a cluster work on one tile of 256 rows; `rank` 0 (the even CTA) issues its MMAs
     constexpr int TM = PAIR ? 2 * TC_BM : TC_BM;
     const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
-    const int worker = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x, nworkers = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
+    // a tile shared by the CTAs of a cluster: `part` is this CTA's share of its contraction (one tile per cluster)
+    const int shared = PAIR ? 1 : p.shared, part = shared > 1 ? (int)cluster_ctarank() : 0;
+    const int worker = PAIR ? (int)(blockIdx.x >> 1) : (shared > 1 ? (int)blockIdx.x / shared : (int)blockIdx.x);
+    const int nworkers = PAIR ? (int)(gridDim.x >> 1) : (shared > 1 ? (int)gridDim.x / shared : (int)gridDim.x);
     const int bh = PAIR ? bn >> 1 : bn;                       // columns of B this CTA stages
     const int mtiles = (p.M + TM - 1) / TM, ntiles = (p.N + bn - 1) / bn;
     const int total_tiles = mtiles * ntiles * p.splits;
@@ -344,7 +353,7 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
         z = p.by_ntiles.div(rest);
         int nt = rest - z * ntiles;
         m0 = mt * TM + (int)rank * TC_BM; n0 = nt * bn;         // this CTA's own 128 rows
-        kbeg = z * p.kchunk;
+        kbeg = (z + part) * p.kchunk;                           // (z is 0 where a cluster shares a tile)
         int kend = min(p.K, kbeg + p.kchunk);
         ktiles = (kend - kbeg + TC_BK - 1) / TC_BK;
     };
@@ -527,7 +536,7 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
             }
             if (alive && leader) { if (PAIR) umma2_commit_both(tfull0 + 8 * buf); else umma_commit(tfull0 + 8 * buf); }   // accumulator complete
         }
-    } else if (warp >= TG_EPI_WARP0) {
+    } else if (warp >= TG_EPI_WARP0 && shared == 1) {
         // ---------------- epilogue: warp w drains TMEM lane quarter w % 4, every second 32-column chunk ----------------
         const int q = warp & 3, c_first = ((warp - TG_EPI_WARP0) >> 2) * 32;
         float *stage = reinterpret_cast<float *>(epi_smem + (size_t)(warp - TG_EPI_WARP0) * EPI_WARP_SMEM);
@@ -556,6 +565,53 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
             else
                 drain_accumulator(taddr, m0 + q * 32, n0, c_first, bn, 64, p.M, p.N, cs, p.partial, (long long)z * p.M * p.N, stage, p.bias,
                                   p.act, out_scale, nacc, (uint32_t)bn, release);
+        }
+    }
+    if (!PAIR && shared > 1) {
+        // ---------------- a tile of a cluster: chunk ci (32 x 32) is added up and finished by CTA ci % shared ----------------
+        // Each CTA writes its sums of a chunk into the shared memory of that CTA, where the ring is done with.  What the tile's 64 KB
+        // cost between SMs is 2 us either way; reading the others' shares instead measured 0.3 to 1.5 us slower (and keeps every CTA
+        // until it has been read), bulk copies the same.
+        const bool epi = warp >= TG_EPI_WARP0;
+        const int ew = warp - TG_EPI_WARP0, cols = bn >> 5;
+        const bool done = epi && mbar_wait(tfull0, 0, abortp, p.status, 3, p.wait_clocks + (p.wait_clocks >> 2));
+        tc_fence_after();
+        cluster_sync_all();                                    // every CTA's ring is free
+        if (done) {
+            const int q = warp & 3;
+            const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16);
+#pragma unroll 1
+            for (int c = (ew >> 2) * 32; c < bn; c += 64) {
+                float v[32];
+                tmem_ld32_sum(taddr + (uint32_t)c, v, nacc, (uint32_t)bn);
+                const int ci = q * cols + (c >> 5), slot = ci / shared, owner = ci - slot * shared;
+                const uint32_t dst = mapa_rank(smem0 + (uint32_t)(((slot * shared + part) * 256 + lane) * 16), (uint32_t)owner);
+#pragma unroll
+                for (int k = 0; k < 8; k++) st_cluster_f4(dst + 512u * k, v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+            }
+        }
+        cluster_sync_all();                                    // every share is where it is added up, in the order of the shares
+        if (epi) {
+            float *stage = reinterpret_cast<float *>(epi_smem + (size_t)ew * EPI_WARP_SMEM);
+            const float out_scale = p.dinv ? p.out_scale * __ldg(p.dinv) : p.out_scale;
+            int m0, n0, kbeg, ktiles, z;
+            tile_origin(worker, m0, n0, kbeg, ktiles, z);
+#pragma unroll 1
+            for (int slot = ew, ci = slot * shared + part; ci < 4 * cols; slot += TG_EPI_WARPS, ci += TG_EPI_WARPS * shared) {
+                const float4 *src = reinterpret_cast<const float4 *>(smem) + slot * shared * 256 + lane;
+                float v[32];
+#pragma unroll
+                for (int k = 0; k < 32; k++) v[k] = 0.f;
+#pragma unroll 1
+                for (int r = 0; r < shared; r++, src += 256) {
+#pragma unroll
+                    for (int k = 0; k < 8; k++) { const float4 x = src[32 * k]; v[4 * k] += x.x; v[4 * k + 1] += x.y; v[4 * k + 2] += x.z; v[4 * k + 3] += x.w; }
+                }
+                const int q = ci / cols, row = m0 + q * 32, n = n0 + (ci - q * cols) * 32;
+                if (row >= p.M || n >= p.N) continue;
+                if (p.pool_on) put_chunk_pooled(v, row, n, p.M, p.N, p.bias, p.act, p.pool, stage, out_scale);
+                else put_chunk(v, row, n, p.M, p.N, cs, stage, p.bias, p.act, out_scale);
+            }
         }
     }
     tc_fence_before();
@@ -672,6 +728,9 @@ inline void tma_plan(TmaGemmParams &p, int ns, bool allow_split) {
     p.joined = 0;
 }
 
+// How many clusters of `size` CTAs of one SM each the chip holds at once (GPU processing clusters lose what is left over of their SMs).
+int clusters_at_once(int size);
+
 // Launches the kernel on prepared tensor maps.  p.M, p.N, p.K (contraction length in elements), a_mode, b_mn, bn
 // and the geometry fields must be set; kchunk, stages, partial and status are filled here.
 template <class CS>
@@ -685,32 +744,50 @@ int launch_tma_gemm(const TmaMaps &maps, TmaGemmParams p, const CS &cs, int ns, 
     if (stages < 2) return fail(SEERA_E_LIMIT, "%s: tile does not fit shared memory", name);
     size_t smem = stage * stages + TG_EPI_WARPS * EPI_WARP_SMEM + 1024;
     long long tiles = (long long)((p.M + tm - 1) / tm) * ((p.N + p.bn - 1) / p.bn);
-    // Split of the contraction: every (tile, split) item is one pass of a persistent CTA, so the launch takes
-    // ceil(items / SMs) rounds of ceil(ksteps / splits) k-steps each, plus a fixed cost per item (pipeline fill, the
-    // partial tile written out, worth about four k-steps).  A split also pays for the reduce launch (eight k-steps) and
-    // for moving the partial sums: splits x M x N floats written and read back, M x N written, priced at 5 TB/s against
-    // a k-step of about 0.25 us per product at N = 128 (small outputs stay in L2 and cost nothing; a 4096 x 4096 output
-    // split in two would cost more than the idle SMs it fills).  Take the split count with the smallest such estimate;
-    // ties go to fewer splits.
+    // How the contraction is shared out, by estimated time (microseconds past a launch's start; at 1.75 GHz, where the tensor pipe
+    // holds the clock).  A k-step takes what its MMAs take (see tma_gemm_kernel) or its loads at 80 bytes a clock.
+    //   one CTA a tile:     rounds of tiles over the SMs, each its k-steps and 1 us for the pipeline's fill and the tile's way out
+    //   a cluster a tile:   2 to 8 CTAs share the k-steps and add up through each other's shared memory, 2 us for that and 0.25 for
+    //                       each CTA; for as many tiles as clusters of that size fit on the chip at once
+    //   split with partial sums (allow_split): items of (tile, part) in rounds, a second launch of 3 us that adds the parts up, and
+    //                       the parts' way to L2 and back, 4 (2 parts + 1) M N bytes at 5 TB/s
+    // At least two k-steps for every CTA.  Ties go to fewer parts.  1600 x 256 x 2304 in six products (26 tiles,
+    // 38 us by one CTA each): 23.5 / 18.6 / 16.8 / 16.2 us by clusters of 2 / 3 / 4 / 5; 1000 x 1024 x 784 (64 tiles) 20.3 -> 15.1.  For 128 x
+    // 128 x 2304 (one tile, 37.5) clusters of 8 take 12.5 and a split of 18 with its reduction 7.5 + 4.2.
     int splits = 1;
+    p.shared = 1;
     const long long ksteps = (p.K + TC_BK - 1) / TC_BK;
-    if (allow_split) {
+    {
         const long long sms = p.pair ? rt().sm_count / 2 : rt().sm_count;      // workers: CTAs, or pairs of them
-        const double kstep_us = 0.25 * (ns == 1 ? 1 : (ns == 2 ? 3 : 6)) * p.bn / 128.0;
-        const double partial_ksteps = (double)p.M * p.N * 4.0 / 5e6 / kstep_us;      // one pass over M x N floats, in k-steps
-        long long maxs = ksteps / 2;                  // at least two k-steps per item
-        if (maxs > 256) maxs = 256;
-        long long best = -1;
-        for (long long sp = 1; sp <= maxs || sp == 1; sp++) {
-            long long per = (ksteps + sp - 1) / sp, eff = (ksteps + per - 1) / per;
-            long long rounds = (tiles * eff + sms - 1) / sms;
-            long long cost = rounds * (per + 4);
-            if (sp > 1) cost += 8 + (long long)((2.0 * eff + 1.0) * partial_ksteps);
-            if (best < 0 || cost < best) { best = cost; splits = (int)eff; }
+        auto mma = [](int n) { return n >= 128 ? n / 2 : 32 + n / 4; };
+        const int products = ns == 1 ? 1 : (ns == 2 ? 3 : 6);
+        const int slice = p.joined ? (ns == 2 ? mma(2 * p.bn) + mma(p.bn) : 2 * (mma(2 * p.bn) + mma(p.bn))) : products * mma(p.bn);
+        const double loads = (double)stage / 80., kstep_us = (4. * slice > loads ? 4. * slice : loads) / 1750.;
+        auto rounds_us = [&](long long items, long long per) { return (double)((items + sms - 1) / sms) * (per * kstep_us + 1.); };
+        double best = rounds_us(tiles, ksteps);
+        if (!p.pair) {
+            for (int c = 2; c <= 8 && 2 * c <= ksteps; c++) {
+                const size_t chunks = (size_t)p.bn / 8;
+                if ((chunks + c - 1) / c * c * 4096 > stages * stage) continue;        // every share of a CTA's chunks, where the ring was
+                const long long per = (ksteps + c - 1) / c;
+                if (tiles * c > sms || (c - 1) * per >= ksteps) continue;
+                const double t = per * kstep_us + 3. + 0.25 * c;
+                if (t < best && tiles <= clusters_at_once(c)) { best = t; p.shared = c; }
+            }
+        }
+        if (allow_split) {
+            const double pass_us = (double)p.M * p.N * 4. / 5e6;
+            const long long maxs = ksteps / 2 < 256 ? ksteps / 2 : 256;
+            for (long long sp = 2; sp <= maxs; sp++) {
+                const long long per = (ksteps + sp - 1) / sp, eff = (ksteps + per - 1) / per;
+                const double t = rounds_us(tiles * eff, per) + 3. + (2. * eff + 1.) * pass_us;
+                if (t < best) { best = t; splits = (int)eff; p.shared = 1; }
+            }
         }
     }
+    if (p.shared > 1) p.kchunk = (int)((ksteps + p.shared - 1) / p.shared) * TC_BK; else
     p.kchunk = (int)((ksteps + splits - 1) / splits) * TC_BK;
-    splits = (p.K + p.kchunk - 1) / p.kchunk;
+    splits = p.shared > 1 ? 1 : (p.K + p.kchunk - 1) / p.kchunk;
     p.splits = splits;
     p.stages = stages;
     p.by_mtiles = fast_div((p.M + tm - 1) / tm); p.by_ntiles = fast_div((p.N + p.bn - 1) / p.bn);
@@ -727,6 +804,8 @@ int launch_tma_gemm(const TmaMaps &maps, TmaGemmParams p, const CS &cs, int ns, 
     long long all_tiles = tiles * splits;
     const long long workers = p.pair ? rt().sm_count / 2 : rt().sm_count;
     dim3 grid((unsigned)((all_tiles < workers ? all_tiles : workers) * (p.pair ? 2 : 1)));     // persistent: one CTA per SM at most
+    if (p.shared > 1) grid.x = (unsigned)(tiles * p.shared);
+    const unsigned cluster = p.pair ? 2u : (unsigned)p.shared;
     cudaStream_t st = rt().stream;
     cudaError_t e;
     profile_begin();
@@ -739,8 +818,8 @@ int launch_tma_gemm(const TmaMaps &maps, TmaGemmParams p, const CS &cs, int ns, 
             cfg.gridDim = grid; cfg.blockDim = dim3(TG_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = st;             \
             cudaLaunchAttribute attr[1];                                                                                   \
             attr[0].id = cudaLaunchAttributeClusterDimension;                                                              \
-            attr[0].val.clusterDim.x = PAIRV ? 2 : 1; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;          \
-            cfg.attrs = attr; cfg.numAttrs = PAIRV ? 1 : 0;                                                                \
+            attr[0].val.clusterDim.x = cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;                \
+            cfg.attrs = attr; cfg.numAttrs = cluster > 1 ? 1 : 0;                                                          \
             e = cudaLaunchKernelEx(&cfg, kern, maps.a[0], maps.a[1], maps.a[2], maps.b[0], maps.b[1], maps.b[2], cs, p);   \
             if (e == cudaSuccess) e = cudaGetLastError();                                                                  \
         }                                                                                                                  \

@@ -8,7 +8,7 @@ from conftest import rel_l2
 pytestmark = pytest.mark.gpu
 
 #: bf16x3 leaves 2^-17 of a product out, bf16x6 and fp16x3 2^-22 or less; their sums run in 32 bits (see test_gpu_tensorcore.py).
-TOL = {1: 1e-2, 2: 2e-5, 3: 2e-6, 4: 1e-5}
+TOL = {1: 1e-2, 2: 2e-5, 3: 4e-6, 4: 1e-5}
 
 
 @pytest.fixture
@@ -27,7 +27,8 @@ def activated(z, act):
 
 
 @pytest.mark.parametrize("mode", [1, 2, 3, 4])
-@pytest.mark.parametrize("M,N,K", [(127, 17, 65), (129, 64, 192), (260, 65, 640), (33, 96, 130), (300, 131, 72), (128, 257, 448)])
+@pytest.mark.parametrize("M,N,K", [(127, 17, 65), (129, 64, 192), (260, 65, 640), (33, 96, 130), (300, 131, 72), (128, 257, 448),
+                                   (200, 33, 4100), (1, 300, 2304), (700, 130, 1000)])       # few tiles: clusters of every size share them
 def test_widths_and_edges(sc, mode, M, N, K):
     sc.set_precision(mode)
     rs = np.random.RandomState(M + N + K)
