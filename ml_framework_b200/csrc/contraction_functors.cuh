@@ -148,19 +148,14 @@ struct StorePixelRows {    // m = (img, p): out[(img*Nch + n)*P + p]
     }
     __device__ float *row(int m) const { int img = m / P, p = m - img * P; return out + (long long)img * Nch * P + p; }
     __device__ long long nstride() const { return P; }
-    // 32 consecutive channels of pixel m: a lane's own row, 64 contiguous bytes of each copy
-    __device__ void copy_row(int m, int n0, const float *v) const {
-        if (!cp[0]) return;
+    __device__ bool copies() const { return cp[0] != nullptr; }
+    // eight consecutive channels of pixel m; v is consumed
+    __device__ void copy8(int m, int n, float *v) const {
+        if (n >= Cp) return;
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
-            const int n = n0 + 8 * c;
-            if (n >= Cp) return;
-            float o8[8];
-#pragma unroll
-            for (int i = 0; i < 8; i++) o8[i] = n + i < Nch ? v[8 * c + i] : 0.f;
-            const long long o = (long long)m * Cp + n;
-            store_split8_rolled(o8, ns, enc, cp[0] + o, cp[1] + o, cp[2] + o);
-        }
+        for (int i = 0; i < 8; i++) if (n + i >= Nch) v[i] = 0.f;
+        const long long o = (long long)m * Cp + n;
+        store_split8_rolled(v, ns, enc, cp[0] + o, cp[1] + o, cp[2] + o);
     }
 };
 

@@ -13,10 +13,12 @@
 //     dW        dW[f][tap,c] = sum_pix dY_nhwc[pix, f] * X_nhwc[window(pix)+tap, c]         A = (tap,c) boxes by im2col,
 //                                                                                          B = dY columns, split over pixels
 // A transposed convolution is the same three kernels with the roles exchanged (its forward is a dX, its dX a
-// forward, its dW a dW with X and dY swapped).  Data gradients with stride > 1 go to the kernel that gathers in
-// its producer warps (contraction_tc.cu).  Outputs are written fp32 NCHW straight from TMEM (lanes run along
+// forward, its dW a dW with X and dY swapped).  Data gradients with stride > 1 are unit-stride products by output
+// phase.  Outputs are written fp32 NCHW straight from TMEM (lanes run along
 // pixels, so stores are coalesced).  Arithmetic follows engine/src/conv_ops.cpp:95-287.
+#include <algorithm>
 #include <cfloat>
+#include <vector>
 
 #include "internal.h"
 #include "tma_gemm_kernel.cuh"
@@ -255,13 +257,16 @@ __global__ void __launch_bounds__(256) shadow_weight_phase_kernel(const float *_
     }
 }
 
-// Output of one phase: row m = (img, i, j) of the phase grid is pixel (a + sh*i, b + sw*j) of the full-resolution tensor.
+// Output of one phase (a, b), which the kernel sets: row m = (img, i, j) of the phase grid is pixel (a + sh*i, b + sw*j) of the full-resolution tensor,
+// where that has such a pixel.
 struct StorePhaseRows {
     static constexpr bool kMContiguous = true;
-    float *out; int Nch, H, W, Hg, Wg, a, b, sh, sw;
+    static constexpr int kPhases = TMA_PHASES;
+    float *out; int Nch, H, W, sh, sw, a, b;
+    FastDiv by_pg, by_Wg;
     __device__ float *row(int m) const {
-        int pg = Hg * Wg, img = m / pg, rem = m - img * pg, i = rem / Wg, j = rem - i * Wg;
-        return out + (long long)img * Nch * H * W + (long long)(a + sh * i) * W + (b + sw * j);
+        const int img = by_pg.div(m), rem = m - img * by_pg.d, i = by_Wg.div(rem), h = a + sh * i, w = b + sw * (rem - i * by_Wg.d);
+        return h < H && w < W ? out + (long long)img * Nch * H * W + (long long)h * W + w : nullptr;
     }
     __device__ long long nstride() const { return (long long)H * W; }
     __device__ void operator()(int m, int n, float v) const { row(m)[n * nstride()] = v; }
@@ -293,7 +298,8 @@ static int tma_fprop(const NhwcShadow &x, const Shadow &wk, float *Y, int F, int
     p.K = p.taps * p.cchunks * 64;
     p.OW = OW; p.OHW = OH * OW; p.sw = sw; p.sh = sh; p.pw = pw; p.ph = ph;
     tma_plan(p, ns, false);
-    TmaMaps maps;
+    TmaMapSet<1> set;
+    TmaMaps &maps = set.of[0];
     for (int i = 0; i < 3; i++) {
         int j = i < ns ? i : 0;
         if (int s = make_map_im2col(&maps.a[i], x.p[j], x.NB, x.H, x.W, x.Cp, R, S, sh, sw, ph, pw, 64, TC_BM)) return s;
@@ -305,7 +311,7 @@ static int tma_fprop(const NhwcShadow &x, const Shadow &wk, float *Y, int F, int
         for (int i = 0; i < 3; i++) cs.cp[i] = ycopies->p[i];
         cs.Cp = ycopies->Cp; cs.ns = ns; cs.enc = ycopies->enc;
     }
-    return launch_tma_gemm(maps, p, cs, ns, false, flops, name);
+    return launch_tma_gemm(set, p, cs, ns, false, flops, name);
 }
 
 // Unit-stride data gradient from the forward's filter copies w[F][tap][Cp] as they are: the contraction runs over (tap, filter), so
@@ -321,13 +327,14 @@ static int tma_dgrad_kept(const NhwcShadow &dy, const Shadow &w, float *dX, int 
     p.K = p.taps * p.cchunks * 64;
     p.OW = W; p.OHW = H * W; p.sw = 1; p.sh = 1; p.pw = S - 1 - pw; p.ph = R - 1 - ph;
     tma_plan(p, ns, false);
-    TmaMaps maps;
+    TmaMapSet<1> set;
+    TmaMaps &maps = set.of[0];
     for (int i = 0; i < 3; i++) {
         int j = i < ns ? i : 0;
         if (int s = make_map_im2col(&maps.a[i], dy.p[j], dy.NB, dy.H, dy.W, dy.Cp, R, S, 1, 1, p.ph, p.pw, 64, TC_BM)) return s;
         if (int s = make_map_2d(&maps.b[i], w.p[j], w.rows, w.cols, w.ld, 64, 64)) return s;
     }
-    return launch_tma_gemm(maps, p, StorePixelRows{dX, C, H * W}, ns, false, 2.0 * p.M * (double)C * dy.C * R * S, name);
+    return launch_tma_gemm(set, p, StorePixelRows{dX, C, H * W}, ns, false, 2.0 * p.M * (double)C * dy.C * R * S, name);
 }
 
 // dW[Fo][C][R][S] = sum over output pixels of dY_nhwc[pix, f] * X_nhwc[window(pix)+tap, c]
@@ -342,14 +349,15 @@ static int tma_wgrad(const NhwcShadow &x, const NhwcShadow &dy, float *dW, int R
     p.K = x.NB * OH * OW;
     p.OW = OW; p.OHW = OH * OW; p.sw = sw; p.sh = sh; p.pw = pw; p.ph = ph;
     tma_plan(p, ns, true);
-    TmaMaps maps;
+    TmaMapSet<1> set;
+    TmaMaps &maps = set.of[0];
     for (int i = 0; i < 3; i++) {
         int j = i < ns ? i : 0;
         if (int s = make_map_im2col(&maps.a[i], x.p[j], x.NB, x.H, x.W, x.Cp, R, S, sh, sw, ph, pw, 64, 64)) return s;
         if (int s = make_map_2d(&maps.b[i], dy.p[j], dy.NB * OH * OW, dy.Cp, dy.Cp, 64, 64)) return s;
     }
     double flops = 2.0 * p.K * (double)F * x.C * R * S;
-    return launch_tma_gemm(maps, p, StoreWgrad{dW, x.C, R * S, p.cchunks * 64}, ns, true, flops, name);
+    return launch_tma_gemm(set, p, StoreWgrad{dW, x.C, R * S, p.cchunks * 64}, ns, true, flops, name);
 }
 
 // ---- strided data gradient by output phase ---------------------------------------------------------------------
@@ -357,8 +365,9 @@ static int tma_wgrad(const NhwcShadow &x, const NhwcShadow &dy, float *dW, int R
 //                   g[n, f, (h + ph - r)/sh, (w + pw - s)/sw] * Wt[o = c, i = f, r, s].
 // Output pixels with h % sh == a and w % sw == b see only the taps r = r0 + sh*t, s = s0 + sw*u (r0 = (a + ph) % sh,
 // s0 = (b + pw) % sw), and over the phase grid (i, j) = (h / sh, w / sw) the sum is a unit-stride convolution of g with
-// those taps: window corner (i + qa - (Ta-1), j + qb - (Ub-1)), qa = (a + ph - r0)/sh.  Each phase is one TMA
-// implicit-GEMM launch with its own window box and filter shadow, scattering into the full-resolution tensor.
+// those taps: window corner (i + qa - (Ta-1), j + qb - (Ub-1)), qa = (a + ph - r0)/sh.  Each phase is an implicit GEMM
+// with its own window box and filter copies, scattering into the full-resolution tensor; up to four share a launch (a
+// launch apiece: 43 us for 32 channels of 4 x 4 stride 2 from 64 at 16 x 16, 256 images, mode 4; 28.5 together).
 struct PhaseAxis { int r0, T, q, lower, upper, G; };
 static PhaseAxis phase_axis(int a, int pad, int stride, int K, int full, int gdim) {
     PhaseAxis x;
@@ -405,38 +414,56 @@ static int tma_dgrad_phases(const NhwcShadow &g, const float *Wt, long long so, 
     count_launch();
     cudaError_t ce = cudaGetLastError();
     if (ce != cudaSuccess) { free_shadow(all); return check_cuda(ce, "shadow_weight_phase"); }
-    for (int a = 0; a < sh; a++) {
-        PhaseAxis y = phase_axis(a, ph, sh, R, H, g.H);
-        if (!y.T || !y.G) continue;
+    // Up to TMA_PHASES phases share a launch, those with the most taps first.  They have to agree on the grid of their pixels: the larger
+    // one, the store leaving out what is beyond the tensor, where TMA can walk it for the smaller phases too.
+    struct Phase { int a, b, taps; PhaseAxis y, x; };
+    std::vector<Phase> list;
+    const int Gh = (H + sh - 1) / sh, Gw = (W + sw - 1) / sw;
+    bool even = true;
+    for (int a = 0; a < sh; a++)
         for (int b = 0; b < sw; b++) {
-            PhaseAxis x = phase_axis(b, pw, sw, S, W, g.W);
-            if (!x.T || !x.G) continue;
-            const int taps = y.T * x.T;
-            Shadow wk = all;
-            wk.cols = wk.ld = taps * Ip;
-            const long long first = (long long)Nch * phase_taps(a, b, R, S, sh, sw, ph, pw).first * Ip;
-            for (int i = 0; i < ns; i++) wk.p[i] = all.p[i] + first;
-
-            TmaGemmParams p{};
-            p.bias = bias; p.act = act;
-            p.a_mode = TMA_A_IM2COL; p.b_mn = 0;
-            p.a_fp16 = g.enc.fmt; p.b_fp16 = wk.enc.fmt; p.out_scale = 1.f / (g.enc.scale * wk.enc.scale); p.dinv = enc_dinv(g.enc, wk.enc);
-            p.M = g.NB * y.G * x.G; p.N = Nch;
-            p.cchunks = (g.Cp + 63) / 64; p.cpad = g.Cp; p.taps = taps; p.S = x.T;
-            p.K = p.taps * p.cchunks * 64;
-            p.OW = x.G; p.OHW = y.G * x.G; p.sw = 1; p.sh = 1; p.pw = -x.lower; p.ph = -y.lower;
-            tma_plan(p, ns, false);
-            TmaMaps maps;
-            int e = SEERA_OK;
-            for (int i = 0; i < 3 && !e; i++) {
-                int j = i < ns ? i : 0;
-                e = make_map_im2col_box(&maps.a[i], g.p[j], g.NB, g.H, g.W, g.Cp, 1, 1, x.lower, y.lower, x.upper, y.upper, 64, TC_BM);
-                if (!e) e = make_map_2d(&maps.b[i], wk.p[j], wk.rows, wk.cols, wk.ld, 64, p.pair ? p.bn / 2 : p.bn);
-            }
-            double flops = 2.0 * p.M * (double)Nch * g.C * taps;
-            if (!e) e = launch_tma_gemm(maps, p, StorePhaseRows{out, Nch, H, W, y.G, x.G, a, b, sh, sw}, ns, false, flops, name);
-            if (e) { free_shadow(all); return e; }
+            const PhaseAxis y = phase_axis(a, ph, sh, R, H, g.H), x = phase_axis(b, pw, sw, S, W, g.W);
+            if (!y.T || !y.G || !x.T || !x.G) continue;
+            list.push_back({a, b, y.T * x.T, y, x});
+            even = even && Gh - g.H + y.lower <= 0 && Gw - g.W + x.lower <= 0;
         }
+    std::stable_sort(list.begin(), list.end(), [](const Phase &l, const Phase &r) { return l.taps > r.taps; });
+    const size_t group = even ? TMA_PHASES : 1;
+    for (size_t first = 0; first < list.size(); first += group) {
+        const int n = (int)(list.size() - first < group ? list.size() - first : group);
+        TmaGemmParams p{};
+        p.bias = bias; p.act = act;
+        p.a_mode = TMA_A_IM2COL; p.b_mn = 0;
+        p.a_fp16 = g.enc.fmt; p.b_fp16 = all.enc.fmt; p.out_scale = 1.f / (g.enc.scale * all.enc.scale); p.dinv = enc_dinv(g.enc, all.enc);
+        const int GH = even ? Gh : list[first].y.G, GW = even ? Gw : list[first].x.G;
+        p.M = g.NB * GH * GW; p.N = Nch;
+        p.cchunks = (g.Cp + 63) / 64; p.cpad = g.Cp;
+        p.OW = GW; p.OHW = GH * GW; p.sw = 1; p.sh = 1;
+        tma_plan(p, ns, false);
+        p.pair = 0;
+        p.phases = n;
+        TmaMapSet<TMA_PHASES> set{};
+        const StorePhaseRows cs{out, Nch, H, W, sh, sw, 0, 0, fast_div(GH * GW), fast_div(GW)};
+        double flops = 0;
+        int e = SEERA_OK;
+        for (int k = 0; k < n; k++) {
+            const Phase &f = list[first + k];
+            Shadow wk = all;
+            wk.cols = wk.ld = f.taps * Ip;
+            const long long at = (long long)Nch * phase_taps(f.a, f.b, R, S, sh, sw, ph, pw).first * Ip;
+            for (int i = 0; i < ns; i++) wk.p[i] = all.p[i] + at;
+            p.phase[k] = TmaPhase{f.taps * p.cchunks * 64, f.x.T, -f.x.lower, -f.y.lower, f.a, f.b, fast_div(f.x.T)};
+            for (int i = 0; i < 3 && !e; i++) {
+                const int j = i < ns ? i : 0;
+                e = make_map_im2col_box(&set.of[k].a[i], g.p[j], g.NB, g.H, g.W, g.Cp, 1, 1, f.x.lower, f.y.lower, GW - g.W + f.x.lower,
+                                        GH - g.H + f.y.lower, 64, TC_BM);
+                if (!e) e = make_map_2d(&set.of[k].b[i], wk.p[j], wk.rows, wk.cols, wk.ld, 64, p.bn);
+            }
+            flops += 2.0 * g.NB * f.y.G * f.x.G * (double)Nch * g.C * f.taps;
+        }
+        p.K = p.phase[0].K;
+        if (!e) e = launch_tma_gemm(set, p, cs, ns, false, flops, name);
+        if (e) { free_shadow(all); return e; }
     }
     free_shadow(all);
     return SEERA_OK;

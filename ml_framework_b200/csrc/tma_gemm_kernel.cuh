@@ -4,6 +4,7 @@
 #include <cuda.h>
 
 #include <atomic>
+#include <type_traits>
 
 #include "common.cuh"
 #include "contraction_functors.cuh"
@@ -241,6 +242,15 @@ __device__ __forceinline__ uint64_t umma_desc_sw128_mn(uint32_t addr, uint32_t b
 //                 two boxes of 64 channels (MN-major).  B is then [pixels, N] read along its columns.
 enum { TMA_A_ROWS = 0, TMA_A_COLS = 1, TMA_A_IM2COL = 2, TMA_A_TAPS = 3 };
 
+// A launch of several output phases of a strided data gradient (functors with kPhases = 4): the same tiles for each phase, each with its own
+// maps, taps and window corner.
+constexpr int TMA_PHASES = 4;
+template <class CS, class = void> struct phases_of { static constexpr int value = 1; };
+template <class CS> struct phases_of<CS, std::void_t<decltype(CS::kPhases)>> { static constexpr int value = CS::kPhases; };
+struct TmaMaps { CUtensorMap a[3], b[3]; };
+template <int N> struct TmaMapSet { TmaMaps of[N]; };
+struct TmaPhase { int K, S, pw, ph, a, b; FastDiv by_S; };      // contraction, columns of taps, lower padding; the phase (a, b)
+
 struct TmaGemmParams {
     int M, N, K, kchunk, splits, bn, stages;
     int a_mode, b_mn;        // b_mn = 1: B read along its contiguous row index (MN-major)
@@ -256,6 +266,8 @@ struct TmaGemmParams {
     int cpad, cchunks;       // channel pitch of the weight rows / channels rounded up to 64, in chunks of 64
     int wflip;               // TMA_A_IM2COL with b_mn: B is [channel of A][tap][wflip columns], its taps in reverse order (a data
                              // gradient that reads the forward's filter copies as they are)
+    int phases;              // of a launch with several (0: none); the tiles of phase z follow those of phase z - 1
+    TmaPhase phase[TMA_PHASES];
     float *partial;
     int *status;
     unsigned long long wait_clocks;   // budget of every bounded wait in the kernel
@@ -297,9 +309,7 @@ constexpr int TG_THREADS = 384, TG_EPI_WARP0 = 4, TG_EPI_WARPS = 8;
 // commit to the stage's "empty" and the tile's "accumulator full" barriers, which count `issuers` arrivals.
 template <int NS, class CS, bool PAIR>
 __global__ void __launch_bounds__(TG_THREADS, 1)
-tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant__ CUtensorMap mapA1,
-                const __grid_constant__ CUtensorMap mapA2, const __grid_constant__ CUtensorMap mapB0,
-                const __grid_constant__ CUtensorMap mapB1, const __grid_constant__ CUtensorMap mapB2, CS cs, TmaGemmParams p) {
+tma_gemm_kernel(const __grid_constant__ TmaMapSet<phases_of<CS>::value> maps, CS cs, TmaGemmParams p) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) unsigned long long bars[2 * 8 + 4];      // full[8], empty[8], tfull[2], tempty[2]
     __shared__ uint32_t tmem_base_slot;
@@ -355,14 +365,13 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
         m0 = mt * TM + (int)rank * TC_BM; n0 = nt * bn;         // this CTA's own 128 rows
         kbeg = (z + part) * p.kchunk;                           // (z is 0 where a cluster shares a tile)
         int kend = min(p.K, kbeg + p.kchunk);
+        if (phases_of<CS>::value > 1) { kbeg = 0; kend = p.phase[z].K; }
         ktiles = (kend - kbeg + TC_BK - 1) / TC_BK;
     };
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
         const bool leader = elect_one();
-        const CUtensorMap *mA[3] = {&mapA0, &mapA1, &mapA2};
-        const CUtensorMap *mB[3] = {&mapB0, &mapB1, &mapB2};
         auto ld2d = [&](uint32_t dst, const CUtensorMap *m, int x, int y, uint32_t bar) {
             if (PAIR) tma2_load_2d(dst, m, x, y, bar); else tma_load_2d(dst, m, x, y, bar);
         };
@@ -378,11 +387,16 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
             tile_origin(id, m0, n0, kbeg, ktiles, z);
             const int nb0 = n0 + (int)rank * bh;               // this CTA's own columns of B
             // im2col, M = pixels: window corner of this tile's first output pixel
+            const TmaMaps &own = maps.of[phases_of<CS>::value > 1 ? z : 0];
+            const CUtensorMap *mA = own.a, *mB = own.b;
+            int S = p.S, pw = p.pw, phh = p.ph;
+            FastDiv by_S = p.by_S;
+            if (phases_of<CS>::value > 1) { S = p.phase[z].S; pw = p.phase[z].pw; phh = p.phase[z].ph; by_S = p.phase[z].by_S; }
             int pix_img = 0, pix_w = 0, pix_h = 0;
             if (p.a_mode == TMA_A_IM2COL) {
                 pix_img = p.by_OHW.div(m0);
                 int rem = m0 - pix_img * p.OHW, oh = p.by_OW.div(rem), ow = rem - oh * p.OW;
-                pix_w = ow * p.sw - p.pw; pix_h = oh * p.sh - p.ph;
+                pix_w = ow * p.sw - pw; pix_h = oh * p.sh - phh;
             }
             // im2col, M = (tap, channel): the two 64-channel boxes of this tile
             int box_c[2] = {0, 0}, box_s[2] = {0, 0}, box_r[2] = {0, 0};
@@ -416,16 +430,16 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
                 int bk = k0, bx = 0;                          // B's coordinate along the contraction, and where its columns begin
                 if (p.a_mode == TMA_A_ROWS) {
 #pragma unroll
-                    for (int i = 0; i < NS; i++) ld2d(a_tile(s, i), mA[i], k0, m0, bar);
+                    for (int i = 0; i < NS; i++) ld2d(a_tile(s, i), &mA[i], k0, m0, bar);
                 } else if (p.a_mode == TMA_A_COLS) {
 #pragma unroll
                     for (int i = 0; i < NS; i++)
-                        for (int b = 0; b < 2; b++) ld2d(a_tile(s, i) + b * 8192, mA[i], m0 + 64 * b, k0, bar);
+                        for (int b = 0; b < 2; b++) ld2d(a_tile(s, i) + b * 8192, &mA[i], m0 + 64 * b, k0, bar);
                 } else if (p.a_mode == TMA_A_IM2COL) {
                     int ktile = k0 >> 6, tap = p.by_cchunks.div(ktile), c0 = (ktile - tap * p.cchunks) * 64;
-                    int r = p.by_S.div(tap), sx = tap - r * p.S;
+                    int r = by_S.div(tap), sx = tap - r * S;
 #pragma unroll
-                    for (int i = 0; i < NS; i++) ldim(a_tile(s, i), mA[i], c0, pix_w, pix_h, pix_img, sx, r, bar);
+                    for (int i = 0; i < NS; i++) ldim(a_tile(s, i), &mA[i], c0, pix_w, pix_h, pix_img, sx, r, bar);
                     if (p.b_mn) { bk = c0; bx = (p.taps - 1 - tap) * p.wflip; }
                     else bk = tap * p.cpad + c0;
                 } else {
@@ -434,15 +448,15 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
 #pragma unroll
                     for (int i = 0; i < NS; i++)
                         for (int b = 0; b < 2; b++)
-                            if (box_ok[b]) ldim(a_tile(s, i) + b * 8192, mA[i], box_c[b], w, h, img, box_s[b], box_r[b], bar);
+                            if (box_ok[b]) ldim(a_tile(s, i) + b * 8192, &mA[i], box_c[b], w, h, img, box_s[b], box_r[b], bar);
                 }
                 if (p.b_mn) {
 #pragma unroll
                     for (int i = 0; i < NS; i++)
-                        for (int b = 0; b < bh / 64; b++) ld2d(b_tile(s, i) + b * 8192, mB[i], bx + nb0 + 64 * b, bk, bar);
+                        for (int b = 0; b < bh / 64; b++) ld2d(b_tile(s, i) + b * 8192, &mB[i], bx + nb0 + 64 * b, bk, bar);
                 } else {
 #pragma unroll
-                    for (int i = 0; i < NS; i++) ld2d(b_tile(s, i), mB[i], bk, nb0, bar);
+                    for (int i = 0; i < NS; i++) ld2d(b_tile(s, i), &mB[i], bk, nb0, bar);
                 }
                 }
                 if (++s == stages) { s = 0; ph ^= 1u; }
@@ -538,7 +552,7 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
         }
     } else if (warp >= TG_EPI_WARP0 && shared == 1) {
         // ---------------- epilogue: warp w drains TMEM lane quarter w % 4, every second 32-column chunk ----------------
-        const int q = warp & 3, c_first = ((warp - TG_EPI_WARP0) >> 2) * 32;
+        const int q = warp & 3, half = (warp - TG_EPI_WARP0) >> 2;
         float *stage = reinterpret_cast<float *>(epi_smem + (size_t)(warp - TG_EPI_WARP0) * EPI_WARP_SMEM);
         const float out_scale = p.dinv ? p.out_scale * __ldg(p.dinv) : p.out_scale;
         int local = 0;
@@ -546,7 +560,7 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
         for (int id = worker; id < total_tiles; id += nworkers, local++) {
             int m0, n0, kbeg, ktiles, z;
             tile_origin(id, m0, n0, kbeg, ktiles, z);
-            const int buf = local & 1;
+            const int buf = local & 1, c_first = bn == 32 ? (half ^ buf) * 32 : half * 32;     // one chunk a tile: the halves take tiles in turn
             // (a longer budget than the issuers', so that a stage that never fills is reported by the role that waits for it)
             if (!mbar_wait(tfull0 + 8 * buf, ((uint32_t)local >> 1) & 1u, abortp, p.status, 3, p.wait_clocks + (p.wait_clocks >> 2))) break;
             tc_fence_after();
@@ -557,7 +571,8 @@ tma_gemm_kernel(const __grid_constant__ CUtensorMap mapA0, const __grid_constant
                 if (lane == 0) { if (PAIR) mbar_arrive_cluster(tempty_at + 8 * buf); else mbar_arrive(tempty0 + 8 * buf); }
             };
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * nacc * bn + c_first);
-            if (c_first >= bn)                                     // a 32-column tile has one chunk
+            if constexpr (phases_of<CS>::value > 1) { cs.a = p.phase[z].a; cs.b = p.phase[z].b; }
+            if (c_first >= bn)
                 release();
             else if (p.pool_on)
                 drain_accumulator_pooled(taddr, m0 + q * 32, n0, c_first, bn, 64, p.M, p.N, p.bias, p.act, p.pool, stage, out_scale, nacc,
@@ -694,8 +709,6 @@ void launch_splitk_reduce(const TmaGemmParams &p, const CS &cs, int splits, cuda
 
 int *tc_status_word();
 
-struct TmaMaps { CUtensorMap a[3], b[3]; };
-
 inline int tma_pick_bn(int N, int ns, int b_mn) {
     int bn = N <= 32 ? 32 : (N <= 64 ? 64 : (N <= 128 ? 128 : 256));
     if (b_mn && bn < 64) bn = 64;
@@ -728,13 +741,24 @@ inline void tma_plan(TmaGemmParams &p, int ns, bool allow_split) {
     p.joined = 0;
 }
 
+// Estimated time of a k-step: its MMAs (see tma_gemm_kernel) or its loads at 80 bytes a clock, at the 1.75 GHz that the tensor pipe's
+// load leaves.
+inline double tma_kstep_us(int bn, int ns, int joined, size_t stage_bytes) {
+    auto mma = [](int n) { return n >= 128 ? n / 2 : 32 + n / 4; };
+    const int products = ns == 1 ? 1 : (ns == 2 ? 3 : 6);
+    const int slice = joined ? (ns == 2 ? mma(2 * bn) + mma(bn) : 2 * (mma(2 * bn) + mma(bn))) : products * mma(bn);
+    const double loads = (double)stage_bytes / 80.;
+    return (4. * slice > loads ? 4. * slice : loads) / 1750.;
+}
+
 // How many clusters of `size` CTAs of one SM each the chip holds at once (GPU processing clusters lose what is left over of their SMs).
 int clusters_at_once(int size);
 
 // Launches the kernel on prepared tensor maps.  p.M, p.N, p.K (contraction length in elements), a_mode, b_mn, bn
 // and the geometry fields must be set; kchunk, stages, partial and status are filled here.
 template <class CS>
-int launch_tma_gemm(const TmaMaps &maps, TmaGemmParams p, const CS &cs, int ns, bool allow_split, double flops, const char *name) {
+int launch_tma_gemm(const TmaMapSet<phases_of<CS>::value> &maps, TmaGemmParams p, const CS &cs, int ns, bool allow_split, double flops,
+                    const char *name) {
     if (p.issuers != 2 || p.pair || p.joined || 4 * p.bn > 512) p.issuers = 1;      // TMEM has 512 columns
     const int tm = p.pair ? 2 * TC_BM : TC_BM;
     size_t stage = (size_t)ns * (TC_BM * 128 + (size_t)(p.pair ? p.bn / 2 : p.bn) * 128);
@@ -744,8 +768,7 @@ int launch_tma_gemm(const TmaMaps &maps, TmaGemmParams p, const CS &cs, int ns, 
     if (stages < 2) return fail(SEERA_E_LIMIT, "%s: tile does not fit shared memory", name);
     size_t smem = stage * stages + TG_EPI_WARPS * EPI_WARP_SMEM + 1024;
     long long tiles = (long long)((p.M + tm - 1) / tm) * ((p.N + p.bn - 1) / p.bn);
-    // How the contraction is shared out, by estimated time (microseconds past a launch's start; at 1.75 GHz, where the tensor pipe
-    // holds the clock).  A k-step takes what its MMAs take (see tma_gemm_kernel) or its loads at 80 bytes a clock.
+    // How the contraction is shared out, by estimated time (microseconds past a launch's start).
     //   one CTA a tile:     rounds of tiles over the SMs, each its k-steps and 1 us for the pipeline's fill and the tile's way out
     //   a cluster a tile:   2 to 8 CTAs share the k-steps and add up through each other's shared memory, 2 us for that and 0.25 for
     //                       each CTA; for as many tiles as clusters of that size fit on the chip at once
@@ -757,12 +780,11 @@ int launch_tma_gemm(const TmaMaps &maps, TmaGemmParams p, const CS &cs, int ns, 
     int splits = 1;
     p.shared = 1;
     const long long ksteps = (p.K + TC_BK - 1) / TC_BK;
-    {
+    if (p.phases) {
+        splits = p.phases;
+    } else {
         const long long sms = p.pair ? rt().sm_count / 2 : rt().sm_count;      // workers: CTAs, or pairs of them
-        auto mma = [](int n) { return n >= 128 ? n / 2 : 32 + n / 4; };
-        const int products = ns == 1 ? 1 : (ns == 2 ? 3 : 6);
-        const int slice = p.joined ? (ns == 2 ? mma(2 * p.bn) + mma(p.bn) : 2 * (mma(2 * p.bn) + mma(p.bn))) : products * mma(p.bn);
-        const double loads = (double)stage / 80., kstep_us = (4. * slice > loads ? 4. * slice : loads) / 1750.;
+        const double kstep_us = tma_kstep_us(p.bn, ns, p.joined, stage);
         auto rounds_us = [&](long long items, long long per) { return (double)((items + sms - 1) / sms) * (per * kstep_us + 1.); };
         double best = rounds_us(tiles, ksteps);
         if (!p.pair) {
@@ -785,9 +807,9 @@ int launch_tma_gemm(const TmaMaps &maps, TmaGemmParams p, const CS &cs, int ns, 
             }
         }
     }
-    if (p.shared > 1) p.kchunk = (int)((ksteps + p.shared - 1) / p.shared) * TC_BK; else
-    p.kchunk = (int)((ksteps + splits - 1) / splits) * TC_BK;
-    splits = p.shared > 1 ? 1 : (p.K + p.kchunk - 1) / p.kchunk;
+    const int parts = p.shared > 1 ? p.shared : (p.phases ? 1 : splits);
+    p.kchunk = (int)((ksteps + parts - 1) / parts) * TC_BK;
+    if (!p.phases) splits = p.shared > 1 ? 1 : (p.K + p.kchunk - 1) / p.kchunk;
     p.splits = splits;
     p.stages = stages;
     p.by_mtiles = fast_div((p.M + tm - 1) / tm); p.by_ntiles = fast_div((p.N + p.bn - 1) / p.bn);
@@ -797,7 +819,7 @@ int launch_tma_gemm(const TmaMaps &maps, TmaGemmParams p, const CS &cs, int ns, 
     p.skip_load = rt().tc_test_skip_load;
     rt().tc_test_skip_load = -1;                 // one launch only
     p.partial = nullptr;
-    if (splits > 1) {
+    if (splits > 1 && !p.phases) {
         p.partial = (float *)scratch_alloc((size_t)splits * p.M * p.N * sizeof(float));
         if (!p.partial) return SEERA_E_OOM;
     }
@@ -820,7 +842,7 @@ int launch_tma_gemm(const TmaMaps &maps, TmaGemmParams p, const CS &cs, int ns, 
             attr[0].id = cudaLaunchAttributeClusterDimension;                                                              \
             attr[0].val.clusterDim.x = cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;                \
             cfg.attrs = attr; cfg.numAttrs = cluster > 1 ? 1 : 0;                                                          \
-            e = cudaLaunchKernelEx(&cfg, kern, maps.a[0], maps.a[1], maps.a[2], maps.b[0], maps.b[1], maps.b[2], cs, p);   \
+            e = cudaLaunchKernelEx(&cfg, kern, maps, cs, p);                                                               \
             if (e == cudaSuccess) e = cudaGetLastError();                                                                  \
         }                                                                                                                  \
     }
@@ -849,14 +871,15 @@ int run_tma_gemm(const Shadow &sa, int a_mn, const Shadow &sb, int b_mn, const C
     p.a_fp16 = sa.enc.fmt; p.b_fp16 = sb.enc.fmt; p.out_scale = 1.f / (sa.enc.scale * sb.enc.scale);
     p.dinv = enc_dinv(sa.enc, sb.enc);
     tma_plan(p, ns, allow_split);
-    TmaMaps maps;
+    TmaMapSet<1> set;
+    TmaMaps &maps = set.of[0];
     for (int i = 0; i < 3; i++) {
         int j = i < ns ? i : 0;
         // K-major: inner dimension = K (cols of the shadow), box 64 x rows-of-tile; MN-major: inner = M/N, box 64 x 64 k lines
         if (int s = make_map_2d(&maps.a[i], sa.p[j], sa.rows, sa.cols, sa.ld, 64, a_mn ? 64 : TC_BM)) return s;
         if (int s = make_map_2d(&maps.b[i], sb.p[j], sb.rows, sb.cols, sb.ld, 64, b_mn ? 64 : (p.pair ? p.bn / 2 : p.bn))) return s;
     }
-    return launch_tma_gemm(maps, p, cs, ns, allow_split, 2.0 * M * N * (double)K, name);
+    return launch_tma_gemm(set, p, cs, ns, allow_split, 2.0 * M * N * (double)K, name);
 }
 
 }  // namespace seera

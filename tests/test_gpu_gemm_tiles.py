@@ -70,3 +70,35 @@ def test_pooled_epilogue(sc, act, N, C, H, F):
     assert np.array_equal(sc.to_host_i32(mask, full.shape[:-1]), full.argmax(-1))
     for p in (xd, wd, bd, out, mask, y):
         sc.cuda_free(p)
+
+
+@pytest.mark.parametrize("mode", [1, 3, 4])
+@pytest.mark.parametrize("N,C,H,W,F,K,st,pad", [(3, 33, 9, 12, 40, 3, 2, 1),        # odd height: phases of different sizes
+                                                (2, 32, 16, 17, 72, 4, 2, 1), (3, 40, 10, 10, 24, 5, 3, 2),        # nine phases
+                                                (40, 32, 16, 16, 64, 3, 2, 1),      # tiles for every CTA, each warp half in turn
+                                                (2, 130, 8, 8, 70, 2, 2, 0), (2, 20, 12, 12, 16, 4, 4, 0)])          # sixteen
+def test_phases_of_a_strided_data_gradient(sc, mode, N, C, H, W, F, K, st, pad):
+    """Against float64; pixels that no window reaches are zero; a NaN stays with the pixels whose windows hold it."""
+    import torch
+    sc.set_precision(mode)
+    rs = np.random.RandomState(N + C + H + F)
+    OH, OW = (H + 2 * pad - K) // st + 1, (W + 2 * pad - K) // st + 1
+    w = (rs.standard_normal((F, C, K, K)) / np.sqrt(F * K)).astype(np.float32)
+    dy = rs.standard_normal((N, F, OH, OW)).astype(np.float32)
+    x, dx, dw = sc.to_device_f32(np.zeros(N * C * H * W, np.float32)), sc.cuda_malloc_f32(N * C * H * W), sc.cuda_malloc_f32(w.size)
+    wd = sc.to_device_f32(w.ravel())
+    for bad in (False, True):
+        if bad:
+            if mode == 4:
+                break                                    # its conversion saturates
+            dy[0, 3, OH // 2, OW // 2] = np.nan
+        g = sc.to_device_f32(dy.ravel())
+        sc.cuda_conv2d_bwd(wd, x, g, dx, dw, N, C, H, W, F, K, K, st, st, pad, pad)
+        ref = torch.nn.grad.conv2d_input((N, C, H, W), torch.from_numpy(w).double(), torch.from_numpy(dy).double(), st, pad).numpy()
+        got, ok = sc.to_host_f32(dx, ref.shape), ~np.isnan(ref)
+        assert np.array_equal(np.isnan(got), ~ok)
+        assert rel_l2(got[ok], ref[ok]) < TOL[mode]
+        assert not got[ref == 0].any()
+        sc.cuda_free(g)
+    for p in (x, dx, dw, wd):
+        sc.cuda_free(p)
