@@ -66,7 +66,8 @@ static int make_map_im2col_box(CUtensorMap *m, const void *base, int NB, int H, 
     cuuint32_t estr[4] = {1, (cuuint32_t)sw, (cuuint32_t)sh, 1};
     CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void *>(base), dims, strides, lower, upper,
                      (cuuint32_t)channels_per_pixel, (cuuint32_t)pixels_per_column, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                     CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                     channels_per_pixel == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS)
         return fail(SEERA_E_CUDA, "cuTensorMapEncodeIm2col failed (%d) for %dx%dx%dx%d window %dx%d stride %d,%d pad %d,%d", (int)r, NB, H, W,
                     Cp, R, S, sh, sw, ph, pw);
@@ -284,26 +285,32 @@ struct StoreWgrad {
     __device__ long long nstride() const { return (long long)C * taps; }
 };
 
+// Boxes of 32 channels where the tensor has no more (and more than one tap to pair): the contraction's length in k-steps of two taps.
+static void plan_channels(TmaGemmParams &p, int Cp, int taps, int S) {
+    p.narrow = Cp <= 32 && taps > 1;
+    p.cchunks = (Cp + 63) / 64; p.cpad = Cp; p.taps = taps; p.S = S;
+    p.K = p.narrow ? (taps + 1) / 2 * 64 : taps * p.cchunks * 64;
+}
 // Y[NB, F, OH, OW] = conv(X_nhwc, weights Wk[F][tap][Cp]) with window R x S, stride, lower padding.
 static int tma_fprop(const NhwcShadow &x, const Shadow &wk, float *Y, int F, int R, int S, int sh, int sw, int ph, int pw,
                      int OH, int OW, int ns, const char *name, const float *bias = nullptr, int act = 0, const PoolOut *pool = nullptr,
                      const NhwcShadow *ycopies = nullptr) {
     TmaGemmParams p{};
     p.bias = bias; p.act = act;
+    p.forward = 1;
     if (pool) { p.pool_on = 1; p.pool = *pool; pool_out_geometry(p.pool, OH * OW, OW, 0); }
     p.a_mode = TMA_A_IM2COL; p.b_mn = 0;
     p.a_fp16 = x.enc.fmt; p.b_fp16 = wk.enc.fmt; p.out_scale = 1.f / (x.enc.scale * wk.enc.scale); p.dinv = enc_dinv(x.enc, wk.enc);
     p.M = x.NB * OH * OW; p.N = F;
-    p.cchunks = (x.Cp + 63) / 64; p.cpad = x.Cp; p.taps = R * S; p.S = S;
-    p.K = p.taps * p.cchunks * 64;
+    plan_channels(p, x.Cp, R * S, S);
     p.OW = OW; p.OHW = OH * OW; p.sw = sw; p.sh = sh; p.pw = pw; p.ph = ph;
     tma_plan(p, ns, false);
     TmaMapSet<1> set;
     TmaMaps &maps = set.of[0];
     for (int i = 0; i < 3; i++) {
         int j = i < ns ? i : 0;
-        if (int s = make_map_im2col(&maps.a[i], x.p[j], x.NB, x.H, x.W, x.Cp, R, S, sh, sw, ph, pw, 64, TC_BM)) return s;
-        if (int s = make_map_2d(&maps.b[i], wk.p[j], wk.rows, wk.cols, wk.ld, 64, p.pair ? p.bn / 2 : p.bn)) return s;
+        if (int s = make_map_im2col(&maps.a[i], x.p[j], x.NB, x.H, x.W, x.Cp, R, S, sh, sw, ph, pw, p.narrow ? 32 : 64, TC_BM)) return s;
+        if (int s = make_map_2d(&maps.b[i], wk.p[j], wk.rows, wk.cols, wk.ld, p.narrow ? 32 : 64, p.pair ? p.bn / 2 : p.bn)) return s;
     }
     double flops = 2.0 * p.M * (double)F * x.C * R * S;
     StorePixelRows cs{Y, F, OH * OW};
@@ -322,17 +329,16 @@ static int tma_dgrad_kept(const NhwcShadow &dy, const Shadow &w, float *dX, int 
     p.a_mode = TMA_A_IM2COL; p.b_mn = 1;
     p.a_fp16 = dy.enc.fmt; p.b_fp16 = w.enc.fmt; p.out_scale = 1.f / (dy.enc.scale * w.enc.scale); p.dinv = enc_dinv(dy.enc, w.enc);
     p.M = dy.NB * H * W; p.N = C;
-    p.cchunks = (dy.Cp + 63) / 64; p.cpad = dy.Cp; p.taps = R * S; p.S = S;
+    plan_channels(p, dy.Cp, R * S, S);
     p.wflip = w.cols / (R * S);
-    p.K = p.taps * p.cchunks * 64;
     p.OW = W; p.OHW = H * W; p.sw = 1; p.sh = 1; p.pw = S - 1 - pw; p.ph = R - 1 - ph;
     tma_plan(p, ns, false);
     TmaMapSet<1> set;
     TmaMaps &maps = set.of[0];
     for (int i = 0; i < 3; i++) {
         int j = i < ns ? i : 0;
-        if (int s = make_map_im2col(&maps.a[i], dy.p[j], dy.NB, dy.H, dy.W, dy.Cp, R, S, 1, 1, p.ph, p.pw, 64, TC_BM)) return s;
-        if (int s = make_map_2d(&maps.b[i], w.p[j], w.rows, w.cols, w.ld, 64, 64)) return s;
+        if (int s = make_map_im2col(&maps.a[i], dy.p[j], dy.NB, dy.H, dy.W, dy.Cp, R, S, 1, 1, p.ph, p.pw, p.narrow ? 32 : 64, TC_BM)) return s;
+        if (int s = make_map_2d(&maps.b[i], w.p[j], w.rows, w.cols, w.ld, 64, p.narrow ? 32 : 64)) return s;
     }
     return launch_tma_gemm(set, p, StorePixelRows{dX, C, H * W}, ns, false, 2.0 * p.M * (double)C * dy.C * R * S, name);
 }
@@ -344,8 +350,9 @@ static int tma_wgrad(const NhwcShadow &x, const NhwcShadow &dy, float *dW, int R
     TmaGemmParams p{};
     p.a_mode = TMA_A_TAPS; p.b_mn = 1;
     p.a_fp16 = x.enc.fmt; p.b_fp16 = dy.enc.fmt; p.out_scale = 1.f / (x.enc.scale * dy.enc.scale); p.dinv = enc_dinv(x.enc, dy.enc);
-    p.cchunks = (x.Cp + 63) / 64; p.cpad = x.Cp; p.taps = R * S; p.S = S;
-    p.M = p.taps * p.cchunks * 64; p.N = F;
+    plan_channels(p, x.Cp, R * S, S);
+    const int pitch = p.narrow ? 32 : p.cchunks * 64;          // rows of a tap
+    p.M = p.taps * pitch; p.N = F;
     p.K = x.NB * OH * OW;
     p.OW = OW; p.OHW = OH * OW; p.sw = sw; p.sh = sh; p.pw = pw; p.ph = ph;
     tma_plan(p, ns, true);
@@ -353,11 +360,11 @@ static int tma_wgrad(const NhwcShadow &x, const NhwcShadow &dy, float *dW, int R
     TmaMaps &maps = set.of[0];
     for (int i = 0; i < 3; i++) {
         int j = i < ns ? i : 0;
-        if (int s = make_map_im2col(&maps.a[i], x.p[j], x.NB, x.H, x.W, x.Cp, R, S, sh, sw, ph, pw, 64, 64)) return s;
+        if (int s = make_map_im2col(&maps.a[i], x.p[j], x.NB, x.H, x.W, x.Cp, R, S, sh, sw, ph, pw, p.narrow ? 32 : 64, 64)) return s;
         if (int s = make_map_2d(&maps.b[i], dy.p[j], dy.NB * OH * OW, dy.Cp, dy.Cp, 64, 64)) return s;
     }
     double flops = 2.0 * p.K * (double)F * x.C * R * S;
-    return launch_tma_gemm(set, p, StoreWgrad{dW, x.C, R * S, p.cchunks * 64}, ns, true, flops, name);
+    return launch_tma_gemm(set, p, StoreWgrad{dW, x.C, R * S, pitch}, ns, true, flops, name);
 }
 
 // ---- strided data gradient by output phase ---------------------------------------------------------------------
@@ -391,7 +398,7 @@ static bool phases_supported(int H, int W, int GH, int GW, int R, int S, int sh,
     return true;
 }
 static int tma_dgrad_phases(const NhwcShadow &g, const float *Wt, long long so, long long si, float *out, int Nch, int H, int W,
-                            int R, int S, int sh, int sw, int ph, int pw, int ns, const char *name, const float *bias = nullptr,
+                            int R, int S, int sh, int sw, int ph, int pw, int ns, const char *name, bool forward, const float *bias = nullptr,
                             int act = 0) {
     cudaStream_t st = rt().stream;
     bool hole = false;
@@ -432,12 +439,12 @@ static int tma_dgrad_phases(const NhwcShadow &g, const float *Wt, long long so, 
     for (size_t first = 0; first < list.size(); first += group) {
         const int n = (int)(list.size() - first < group ? list.size() - first : group);
         TmaGemmParams p{};
-        p.bias = bias; p.act = act;
+        p.bias = bias; p.act = act; p.forward = forward;
         p.a_mode = TMA_A_IM2COL; p.b_mn = 0;
         p.a_fp16 = g.enc.fmt; p.b_fp16 = all.enc.fmt; p.out_scale = 1.f / (g.enc.scale * all.enc.scale); p.dinv = enc_dinv(g.enc, all.enc);
         const int GH = even ? Gh : list[first].y.G, GW = even ? Gw : list[first].x.G;
         p.M = g.NB * GH * GW; p.N = Nch;
-        p.cchunks = (g.Cp + 63) / 64; p.cpad = g.Cp;
+        plan_channels(p, g.Cp, list[first].taps, 1);           // (the most taps of the launch's phases)
         p.OW = GW; p.OHW = GH * GW; p.sw = 1; p.sh = 1;
         tma_plan(p, ns, false);
         p.pair = 0;
@@ -452,12 +459,12 @@ static int tma_dgrad_phases(const NhwcShadow &g, const float *Wt, long long so, 
             wk.cols = wk.ld = f.taps * Ip;
             const long long at = (long long)Nch * phase_taps(f.a, f.b, R, S, sh, sw, ph, pw).first * Ip;
             for (int i = 0; i < ns; i++) wk.p[i] = all.p[i] + at;
-            p.phase[k] = TmaPhase{f.taps * p.cchunks * 64, f.x.T, -f.x.lower, -f.y.lower, f.a, f.b, fast_div(f.x.T)};
+            p.phase[k] = TmaPhase{p.narrow ? (f.taps + 1) / 2 * 64 : f.taps * p.cchunks * 64, f.taps, f.x.T, -f.x.lower, -f.y.lower, f.a, f.b, fast_div(f.x.T)};
             for (int i = 0; i < 3 && !e; i++) {
                 const int j = i < ns ? i : 0;
                 e = make_map_im2col_box(&set.of[k].a[i], g.p[j], g.NB, g.H, g.W, g.Cp, 1, 1, f.x.lower, f.y.lower, GW - g.W + f.x.lower,
-                                        GH - g.H + f.y.lower, 64, TC_BM);
-                if (!e) e = make_map_2d(&set.of[k].b[i], wk.p[j], wk.rows, wk.cols, wk.ld, 64, p.bn);
+                                        GH - g.H + f.y.lower, p.narrow ? 32 : 64, TC_BM);
+                if (!e) e = make_map_2d(&set.of[k].b[i], wk.p[j], wk.rows, wk.cols, wk.ld, p.narrow ? 32 : 64, p.bn);
             }
             flops += 2.0 * g.NB * f.y.G * f.x.G * (double)Nch * g.C * f.taps;
         }
@@ -832,7 +839,7 @@ static int tma_conv2d_bwd_kept(const float *Wt, const float *X, const float *dY,
             else s = make_weight_shadow(Wt, C, F, R * S, R * S, (long long)C * R * S, 1, ns, wd);
             if (!s && !kept) s = tma_fprop(*dys, wd, dX, C, R, S, 1, 1, R - 1 - ph, S - 1 - pw, H, W, ns, "cuda_conv2d_bwd(dX)");
         } else if (phases) {
-            s = tma_dgrad_phases(*dys, Wt, R * S, (long long)C * R * S, dX, C, H, W, R, S, sh, sw, ph, pw, ns, "cuda_conv2d_bwd(dX)");
+            s = tma_dgrad_phases(*dys, Wt, R * S, (long long)C * R * S, dX, C, H, W, R, S, sh, sw, ph, pw, ns, "cuda_conv2d_bwd(dX)", false);
         } else {
             s = seera_tc_conv2d_bwd(Wt, X, dY, dX, nullptr, NB, C, H, W, F, R, S, sh, sw, ph, pw);
         }
@@ -1249,7 +1256,7 @@ static int convT_fwd_kept(const float *X, const float *Wt, const float *bias, fl
         if (!s) s = tma_fprop(xs, wd, out, Cout, KH, KW, 1, 1, KH - 1 - ph, KW - 1 - pw, Ho, Wo, ns, "cuda_conv2DTranpose_fwd", bias, act);
     } else if (!s) {
         s = tma_dgrad_phases(xs, Wt, taps, (long long)Cout * taps, out, Cout, Ho, Wo, KH, KW, sh, sw, ph, pw, ns, "cuda_conv2DTranpose_fwd",
-                             bias, act);
+                             true, bias, act);
     }
     if (!s && x_keep && !given) *x_keep = new seera_shadow{local, ns}; else free_nhwc(local);
     free_shadow(wd);

@@ -144,6 +144,10 @@ __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t addr) {
     d |= (uint64_t)2 << 61;                           // SWIZZLE_128B
     return d;
 }
+// The same for rows of 64 bytes (32 values) with the 64-byte swizzle: 8-row groups are 512 bytes apart.
+__device__ __forceinline__ uint64_t umma_desc_sw64(uint32_t addr) {
+    return (uint64_t)((addr & 0x3FFFFu) >> 4) | (uint64_t)1 << 16 | (uint64_t)(512 >> 4) << 32 | (uint64_t)1 << 46 | (uint64_t)4 << 61;
+}
 // Instruction descriptor: D fp32, A and B bf16, both K-major, M = 128, N = bn.
 __device__ __forceinline__ uint32_t umma_idesc_bf16(int bn) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);

@@ -102,3 +102,27 @@ def test_phases_of_a_strided_data_gradient(sc, mode, N, C, H, W, F, K, st, pad):
         sc.cuda_free(g)
     for p in (x, dx, dw, wd):
         sc.cuda_free(p)
+
+
+@pytest.mark.parametrize("mode", [1, 3, 4])
+@pytest.mark.parametrize("N,C,H,W,F,K,st,pad", [(3, 17, 12, 13, 33, 3, 1, 1), (2, 32, 9, 9, 24, 2, 1, 0), (4, 24, 16, 16, 130, 5, 2, 2), (40, 32, 16, 16, 64, 3, 2, 1),
+                                                (2, 8, 40, 40, 32, 7, 1, 3), (3, 31, 8, 8, 20, 1, 1, 0), (5, 40, 14, 14, 9, 3, 1, 1), (2, 32, 10, 9, 32, 4, 3, 2)])
+def test_layers_of_up_to_32_channels(sc, mode, N, C, H, W, F, K, st, pad):
+    """Two taps a k-step, an odd last one beside zeros; forward, both gradients and the transposed convolution, against float64."""
+    import torch
+    sc.set_precision(mode)
+    rs = np.random.RandomState(N + C + H + F)
+    OH, OW = (H + 2 * pad - K) // st + 1, (W + 2 * pad - K) // st + 1
+    x, w, dy = (rs.standard_normal(s).astype(np.float32) for s in ((N, C, H, W), (F, C, K, K), (N, F, OH, OW)))
+    xd, wd, gd = (sc.to_device_f32(t.ravel()) for t in (x, w, dy))
+    y, dx, dw = (sc.cuda_malloc_f32(t.size) for t in (dy, x, w))
+    sc.cuda_conv2d_fwd(xd, wd, y, N, C, H, W, F, K, K, pad, pad, st, st)
+    sc.cuda_conv2d_bwd(wd, xd, gd, dx, dw, N, C, H, W, F, K, K, st, st, pad, pad)
+    X, Wt = torch.from_numpy(x).double().requires_grad_(), torch.from_numpy(w).double().requires_grad_()
+    Y = torch.nn.functional.conv2d(X, Wt, stride=st, padding=pad)
+    Y.backward(torch.from_numpy(dy).double())
+    assert rel_l2(sc.to_host_f32(y, dy.shape), Y.detach().numpy()) < TOL[mode]
+    assert rel_l2(sc.to_host_f32(dx, x.shape), X.grad.numpy()) < TOL[mode]
+    assert rel_l2(sc.to_host_f32(dw, w.shape), Wt.grad.numpy()) < (1e-3 if mode == 4 else TOL[mode])      # one fp16 product there
+    for p in (xd, wd, gd, y, dx, dw):
+        sc.cuda_free(p)
