@@ -1,0 +1,33 @@
+"""Branches of the bandwidth-bound passes that their general tests do not reach: whole planes of batch normalisation by size, broadcast axes
+that merge or take 16-byte pieces."""
+import numpy as np
+import pytest
+
+import test_gpu_ops as ops
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("shape", [(200, 9, 2, 2), (33, 7, 4, 4), (5, 40, 32, 32), (3, 2, 36, 36), (130, 3, 8, 8), (700, 40)])
+def test_batchnorm_planes(shape):
+    ops.test_batchnorm_forward_and_backward(shape)
+
+
+@pytest.mark.parametrize("a,b", [((1, 1, 1000, 1024), (1, 1, 1, 1024)), ((1, 1, 129, 64), (1, 1, 129, 1)), ((3, 5, 7, 8), (1, 5, 1, 1)), ((1, 1, 1, 12), (6, 1, 5, 12)),
+                                 ((4, 1, 3, 16), (4, 6, 1, 16)), ((2, 3, 4, 5), (2, 3, 4, 5)), ((1, 1, 1, 1), (1, 1, 1, 1)), ((1, 1, 1, 1), (2, 2, 2, 4))])
+@pytest.mark.parametrize("shift", [0, 1])                    # an operand that is not 16-byte aligned
+def test_broadcast_axes(a, b, shift):
+    from ml_framework_b200 import seera_cuda as sc
+    sc.init(0)
+    rs = np.random.RandomState(sum(a) + sum(b))
+    x, y = rs.standard_normal(a).astype(np.float32), rs.standard_normal(b).astype(np.float32)
+    p, q = sc.to_device_f32(np.concatenate([np.zeros(shift, np.float32), x.ravel()])), sc.to_device_f32(y.ravel())
+    want = x + y
+    o = sc.cuda_malloc_f32(want.size)
+    for f, ref in ((sc.broadcast_add_4d, want), (sc.broadcast_mul_4d, x * y)):
+        f(p + 4 * shift, q, o, *a, *b)
+        assert np.array_equal(sc.to_host_f32(o, ref.shape), ref)
+        f(q, p + 4 * shift, o, *b, *a)
+        assert np.array_equal(sc.to_host_f32(o, ref.shape), ref)
+    for t in (p, q, o):
+        sc.cuda_free(t)
