@@ -31,3 +31,22 @@ def test_broadcast_axes(a, b, shift):
         assert np.array_equal(sc.to_host_f32(o, ref.shape), ref)
     for t in (p, q, o):
         sc.cuda_free(t)
+
+
+@pytest.mark.parametrize("M,K,N,shift", [(64, 784, 10, 0), (8, 33, 3, 0), (700, 1024, 10, 0), (700, 1024, 10, 1), (513, 1026, 16, 0), (1, 5, 1, 0), (300, 2050, 7, 0)])
+def test_both_gradients_of_a_narrow_product(M, K, N, shift):
+    """One launch for dA and dB; every pairing of their widths (16-byte rows of dA, 8-byte rows of A or not)."""
+    from conftest import rel_l2
+    from ml_framework_b200 import seera_cuda as sc
+    sc.init(0)
+    sc.set_precision(3)
+    rs = np.random.RandomState(M + K + N)
+    a, b, g = (rs.standard_normal(s).astype(np.float32) for s in ((M, K), (K, N), (M, N)))
+    ad, bd, gd = sc.to_device_f32(np.concatenate([np.zeros(shift, np.float32), a.ravel()])), sc.to_device_f32(b.ravel()), sc.to_device_f32(g.ravel())
+    da, db = sc.cuda_malloc_f32(M * K), sc.cuda_malloc_f32(K * N)
+    sc.cuda_matmul_bwd(ad + 4 * shift, bd, gd, da, db, M, N, K, 1)
+    assert rel_l2(sc.to_host_f32(da, (M, K)), g.astype(np.float64) @ b.T) < 1e-6
+    assert rel_l2(sc.to_host_f32(db, (K, N)), a.T.astype(np.float64) @ g) < 2e-6            # 32-bit sums over up to 700 rows
+    for p in (ad, bd, gd, da, db):
+        sc.cuda_free(p)
+    sc.set_precision(0)
