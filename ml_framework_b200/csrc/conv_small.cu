@@ -15,7 +15,7 @@
 // the tensor-core form is bound by the warps that gather and split patches.  1 -> 32 channels, stride 2, 256 images of 64 x 64 with copies
 // (67 MB): 35 -> 28 us, a third of it waiting for instructions (the straight-line code runs twice per warp); passing the outputs through
 // shared memory to shorten it gave 26 there and cost 2 us where no copies are made.
-#include "conv_first.cuh"
+#include "conv_dw_block.cuh"
 #include "contraction_functors.cuh"
 #include "internal.h"
 
@@ -53,12 +53,26 @@ struct SmallGeom {
     FastDiv by_bands, by_pitch, by_rows, by_cols, by_groups;
 };
 
+// What a launch works on; `grid` blocks walk `total` bands.
+struct SmallArgs {
+    SmallSource src;
+    const float *Wt, *bias;
+    float *Y;
+    SmallCopies cc;
+    SmallGeom g;
+    int total, reversed, act, grid;
+    size_t smem;
+};
 template <int FW, int ST>
-__global__ void __launch_bounds__(256, FW >= 8 ? 2 : 1) conv3x3_small_kernel(SmallSource src, const float *__restrict__ Wt,
-                                                                              const float *__restrict__ bias, float *__restrict__ Y,
-                                                                              SmallCopies cc, SmallGeom g, int total, int reversed, int act) {
+__device__ __forceinline__ void conv3x3_small_block(const SmallArgs &a, int block, float *sm) {
+    const SmallSource &src = a.src;
+    const float *__restrict__ Wt = a.Wt, *__restrict__ bias = a.bias;
+    float *__restrict__ Y = a.Y;
+    const SmallCopies &cc = a.cc;
+    const SmallGeom &g = a.g;
+    const int total = a.total, reversed = a.reversed, act = a.act;
     constexpr int PR = 3 + ST, PC = (PR + 1) / 2 * 2;     // rows of a patch, and columns read of it
-    extern __shared__ __align__(16) float sm[];          // [I][9][OP] weights, [OP] biases, [8][4 FW][32] sums (data gradient), [I][rows][pitch] band
+    // sm: [I][9][OP] weights, [OP] biases, [8][4 FW][32] sums (data gradient), [I][rows][pitch] band
     float *bk = sm + g.I * 9 * g.OP, *red = bk + g.OP, *band = red + (reversed ? 8 * 4 * FW * 32 : 0);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = g.I * 9 * g.OP;
     // Wt[o][i][t], or for the data gradient Wt[i][o][8 - t]
@@ -78,7 +92,7 @@ __global__ void __launch_bounds__(256, FW >= 8 ? 2 : 1) conv3x3_small_kernel(Sma
     const long long iplane = (long long)g.IH * g.IW, oplane = (long long)g.OH * g.OW;
     const bool pairs = (g.OW & 1) == 0 && (reinterpret_cast<uintptr_t>(Y) & 7) == 0;
 
-    for (int id = blockIdx.x; id < total; id += gridDim.x) {
+    for (int id = block; id < total; id += a.grid) {
         const int n = g.by_bands.div(id), q0 = (id - n * g.per_image) * g.window_rows, ih0 = 2 * ST * q0 - g.ph;
         if (src.mask) {                                   // every pixel from its window's gradient, index and output
             const int Wq = g.IW >> 1;
@@ -214,34 +228,83 @@ __global__ void __launch_bounds__(256, FW >= 8 ? 2 : 1) conv3x3_small_kernel(Sma
 }
 
 template <int FW, int ST>
-static int small_launch(const SmallSource &src, const float *Wt, const float *bias, float *Y, int NB, int I, int IH, int IW, int O, int OH, int OW,
-                        int ph, int pw, int reversed, int act, const SmallCopies &cc, const char *name) {
-    SmallGeom g{};
+__global__ void __launch_bounds__(256, FW >= 8 ? 2 : 1) conv3x3_small_kernel(const __grid_constant__ SmallArgs a) {
+    extern __shared__ __align__(16) float sm[];
+    conv3x3_small_block<FW, ST>(a, blockIdx.x, sm);
+}
+// Data and weight gradient of a layer in one launch: they depend on nothing of each other's, and one after the other each was a chain of
+// start, staging and end of 6 us on a chip with room for both (8 -> 16 channels, 64 images of 14 x 14: 6.9 + 6.1 -> 9.2 us, 30 images 13.1 -> 8.3).
+template <int FL, bool POOLED>
+__global__ void __launch_bounds__(256, 2) conv3x3_small_bwd_kernel(const __grid_constant__ SmallArgs a, const __grid_constant__ DwArgs d) {
+    extern __shared__ __align__(16) float sm[];
+    const int b = blockIdx.x, per = d.nblocks * d.chunks, wblocks = per * d.cgroups;
+    if (b < wblocks) {
+        const int bz = b / per, rest = b - bz * per, by = rest / d.nblocks;
+        first_dw_block<4, 1, FL, POOLED>(d, rest - by * d.nblocks, by, bz, sm);
+    } else {
+        conv3x3_small_block<4, 1>(a, b - wblocks, sm);
+    }
+}
+
+template <int FW, int ST>
+static SmallArgs small_args(const SmallSource &src, const float *Wt, const float *bias, float *Y, int NB, int I, int IH, int IW, int O, int OH, int OW,
+                            int ph, int pw, int reversed, int act, const SmallCopies &cc, int blocks) {
+    SmallArgs a{src, Wt, bias, Y, cc, {}, 0, reversed, act, 0, 0};
+    SmallGeom &g = a.g;
     g.I = I; g.IH = IH; g.IW = IW; g.O = O; g.OH = OH; g.OW = OW; g.ph = ph; g.pw = pw;
     const int wrows = (OH + 1) / 2, cols = (OW + 1) / 2;
     g.OP = (O + FW - 1) / FW * FW; g.groups = g.OP / FW;
     g.pitch = 2 * ST * cols + 2;
-    // bands of as many window rows as fit 24 KB (at least one), fewer while the blocks would not go round the SMs
+    // bands of as many window rows as fit 24 KB (at least one), fewer while there would not be `blocks` of them
     const size_t row = (size_t)I * g.pitch * sizeof(float);
     auto rows = [](int wr) { return 2 * ST * wr + 3 - ST; };
     int wr = 1;
     while (wr < wrows && rows(wr + 1) * row <= 24 * 1024) wr++;
-    while (wr > 1 && (long long)NB * ((wrows + wr - 1) / wr) < rt().sm_count) wr = (wr + 1) / 2;
+    while (wr > 1 && (long long)NB * ((wrows + wr - 1) / wr) < blocks) wr = (wr + 1) / 2;
     g.window_rows = wr; g.rows = rows(wr); g.per_image = (wrows + wr - 1) / wr;
     g.by_bands = fast_div(g.per_image); g.by_pitch = fast_div(g.pitch); g.by_rows = fast_div(g.rows);
     g.by_cols = fast_div(cols); g.by_groups = fast_div(g.groups);
-    const size_t smem = ((size_t)(I * 9 + 1) * g.OP + (reversed ? 8 * 4 * FW * 32 : 0)) * sizeof(float) + g.rows * row;
-    const int total = NB * g.per_image;
-    int grid = rt().sm_count * 4;
-    if (grid > total) grid = total;
+    a.smem = ((size_t)(I * 9 + 1) * g.OP + (reversed ? 8 * 4 * FW * 32 : 0)) * sizeof(float) + g.rows * row;
+    a.total = NB * g.per_image;
+    a.grid = rt().sm_count * 4;
+    if (a.grid > a.total) a.grid = a.total;
+    return a;
+}
+template <int FW, int ST>
+static int small_launch(const SmallSource &src, const float *Wt, const float *bias, float *Y, int NB, int I, int IH, int IW, int O, int OH, int OW,
+                        int ph, int pw, int reversed, int act, const SmallCopies &cc, const char *name) {
+    const SmallArgs a = small_args<FW, ST>(src, Wt, bias, Y, NB, I, IH, IW, O, OH, OW, ph, pw, reversed, act, cc, rt().sm_count);
     profile_begin();
-    cudaError_t e = allow_smem((const void *)conv3x3_small_kernel<FW, ST>, smem);
+    cudaError_t e = allow_smem((const void *)conv3x3_small_kernel<FW, ST>, a.smem);
     if (e == cudaSuccess) {
-        conv3x3_small_kernel<FW, ST><<<grid, 256, smem, rt().stream>>>(src, Wt, bias, Y, cc, g, total, reversed, act);
+        conv3x3_small_kernel<FW, ST><<<a.grid, 256, a.smem, rt().stream>>>(a);
         count_launch();
         e = cudaGetLastError();
     }
     profile_end(2.0 * NB * OH * OW * (double)O * I * 9, name);
+    return e == cudaSuccess ? SEERA_OK : check_cuda(e, name);
+}
+// Both gradients in one launch; its blocks are the two launches' together.
+template <int FL, bool POOLED>
+static int small_bwd_launch(const SmallArgs &a, const float *X, const DzSource &dz, float *dW, float *dbias, const FirstGeom &g, const char *name) {
+    DwArgs d = dw_args<4, 1, FL, POOLED>(X, dz, g);
+    d.partial = (float *)scratch_alloc(dw_partial_bytes<4>(d));
+    if (!d.partial) return SEERA_E_OOM;
+    const size_t smem = a.smem > d.smem ? a.smem : d.smem;
+    profile_begin();
+    cudaError_t e = allow_smem((const void *)conv3x3_small_bwd_kernel<FL, POOLED>, smem);
+    if (e == cudaSuccess) {
+        conv3x3_small_bwd_kernel<FL, POOLED><<<d.nblocks * d.chunks * d.cgroups + a.grid, 256, smem, rt().stream>>>(a, d);
+        count_launch();
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) {
+        using Sh = DwShape<4, 1, FL, POOLED>;
+        first_wgrad_reduce(d.partial, dW, dbias, g.F, g.K, Sh::K, Sh::KP, d.nblocks, rt().stream);
+        e = cudaGetLastError();
+    }
+    profile_end(4.0 * g.NB * g.OH * g.OW * (double)g.F * g.K, name);
+    scratch_free(d.partial);
     return e == cudaSuccess ? SEERA_OK : check_cuda(e, name);
 }
 // four output channels per warp: a small layer has too few 32-window tiles to fill the chip with more
@@ -293,6 +356,18 @@ int conv_small_bwd(const float *Wt, const float *X, const float *y, const float 
     const int OH = H + 2 * ph - 2, OW = W + 2 * pw - 2;
     const bool sloped = act != SEERA_ACT_NONE;
     int s = SEERA_OK;
+    if (dX && dW && C > 3) {                // (fewer channels have their own weight-gradient kernels)
+        const SmallSource src{gp ? gp : g, sloped ? (gp ? y_pooled : y) : nullptr, gp ? mask : nullptr, act};
+        // two thirds of a block per SM: the weight gradient's blocks fill the rest, and 354 blocks for 296 places took a second round
+        const SmallArgs a = small_args<4, 1>(src, Wt, nullptr, dX, NB, F, OH, OW, C, H, W, 2 - ph, 2 - pw, 1, SEERA_ACT_NONE, SmallCopies{},
+                                             rt().sm_count * 2 / 3);
+        const FirstGeom geo{NB, C, H, W, F, 3, 3, 1, 1, ph, pw, OH, OW, C * 9};
+        const DzSource dz{nullptr, g, gp, mask, y, act, y_pooled};
+        if (gp) return F <= 8 ? small_bwd_launch<8, true>(a, X, dz, dW, dbias, geo, name) : F <= 16 ? small_bwd_launch<16, true>(a, X, dz, dW, dbias, geo, name)
+                                                                                                   : small_bwd_launch<32, true>(a, X, dz, dW, dbias, geo, name);
+        return F <= 8 ? small_bwd_launch<8, false>(a, X, dz, dW, dbias, geo, name) : F <= 16 ? small_bwd_launch<16, false>(a, X, dz, dW, dbias, geo, name)
+                                                                                          : small_bwd_launch<32, false>(a, X, dz, dW, dbias, geo, name);
+    }
     if (dX) {
         const SmallSource src{gp ? gp : g, sloped ? (gp ? y_pooled : y) : nullptr, gp ? mask : nullptr, act};
         s = small_run(src, Wt, nullptr, dX, NB, F, OH, OW, C, H, W, 2 - ph, 2 - pw, 1, SEERA_ACT_NONE, name);
