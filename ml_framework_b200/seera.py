@@ -1017,6 +1017,8 @@ class _RecordedStep:
 
 
 class Sequential:
+    _whole = False                   # in predict: the pass forms a softmax output too, which a loss would form on its way
+
     def __init__(self, layers, device="cuda"):
         if not isinstance(layers, list):
             raise TypeError("Layers must be a list")
@@ -1096,6 +1098,8 @@ class Sequential:
             out = None
             for layer in self.model:
                 out = layer.forward()
+            if self._whole and out.value.__class__ is _Softmax:
+                out.value.main_ptr                    # formed with the pass: nothing behind it forms it on its way
         finally:
             if opened:
                 _close_batch()
@@ -1125,9 +1129,11 @@ class Sequential:
     def predict(self, X):
         """Forward in evaluation mode: BatchNorm layers normalise with their running statistics (Seera.py:690-700)."""
         self._set_mode(False)
+        self._whole = True
         try:
             return self.forward(X)
         finally:
+            self._whole = False
             self._set_mode(True)
 
     def _set_mode(self, training=True):
