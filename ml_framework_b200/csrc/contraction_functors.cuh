@@ -136,7 +136,7 @@ struct StoreDenseT {       // C[n*ld + m]
     __device__ long long nstride() const { return ld; }
 };
 struct StorePixelRows {    // m = (img, p): out[(img*Nch + n)*P + p]
-    static constexpr bool kMContiguous = true;
+    static constexpr bool kMContiguous = true, kNarrow = true;
     float *out; int Nch, P;
     // optional channels-last 16-bit copies of the same values, for the layer that reads them (pitch Cp, a multiple of 8)
     __nv_bfloat16 *cp[3] = {nullptr, nullptr, nullptr};

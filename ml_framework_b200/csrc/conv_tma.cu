@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(256) shadow_weight_phase_kernel(const float *_
 // Output of one phase (a, b), which the kernel sets: row m = (img, i, j) of the phase grid is pixel (a + sh*i, b + sw*j) of the full-resolution tensor,
 // where that has such a pixel.
 struct StorePhaseRows {
-    static constexpr bool kMContiguous = true;
+    static constexpr bool kMContiguous = true, kNarrow = true;
     static constexpr int kPhases = TMA_PHASES;
     float *out; int Nch, H, W, sh, sw, a, b;
     FastDiv by_pg, by_Wg;
@@ -275,7 +275,7 @@ struct StorePhaseRows {
 
 // dW element for accumulator row m = (tap, channel) and column n = output-side channel: dW[(n*C + c)*taps + tap]
 struct StoreWgrad {
-    static constexpr bool kMContiguous = true;
+    static constexpr bool kMContiguous = true, kNarrow = true;
     float *dW; int C, taps, c64;
     __device__ void operator()(int m, int n, float v) const {
         int tap = m / c64, c = m - tap * c64;

@@ -118,7 +118,7 @@ int clusters_at_once(int size) {
     if (size < 2 || size > 8) return 0;
     int n = known[size].load(std::memory_order_relaxed);
     if (n) return n - 1;
-    auto kern = tma_gemm_kernel<1, StoreDense, false>;
+    auto kern = tma_gemm_kernel<1, StoreDense, false, false>;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(rt().sm_count / size * size)); cfg.blockDim = dim3(TG_THREADS); cfg.dynamicSmemBytes = 200 * 1024;
     cudaLaunchAttribute attr[1];

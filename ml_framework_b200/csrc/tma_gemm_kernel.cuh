@@ -257,12 +257,17 @@ enum { TMA_A_ROWS = 0, TMA_A_COLS = 1, TMA_A_IM2COL = 2, TMA_A_TAPS = 3 };
 constexpr int TMA_PHASES = 4;
 template <class CS, class = void> struct phases_of { static constexpr int value = 1; };
 template <class CS> struct phases_of<CS, std::void_t<decltype(CS::kPhases)>> { static constexpr int value = CS::kPhases; };
+// Functors of the convolutions, whose products may take narrow boxes.
+template <class CS, class = void> struct narrow_of { static constexpr bool value = false; };
+template <class CS> struct narrow_of<CS, std::void_t<decltype(CS::kNarrow)>> { static constexpr bool value = true; };
 struct TmaMaps { CUtensorMap a[3], b[3]; };
 template <int N> struct TmaMapSet { TmaMaps of[N]; };
 struct TmaPhase { int K, taps, S, pw, ph, a, b; FastDiv by_S; };      // contraction, its taps and their columns, lower padding; the phase (a, b)
 
 struct TmaGemmParams {
     int M, N, K, kchunk, splits, bn, stages;
+    int first;               // tiles before this launch's (a product's last tiles, too few for a round, go to clusters)
+    int tiles;               // end of this launch's tiles
     int a_mode, b_mn;        // b_mn = 1: B read along its contiguous row index (MN-major)
     int pair;                // 1: launched as clusters of two CTAs sharing 256-row tiles (tcgen05 cta_group::2)
     int issuers;             // 1 or 2 threads issue the MMAs of a k-step (the K = 16 slices dealt round robin), each into its own
@@ -319,7 +324,8 @@ constexpr int TG_THREADS = 384, TG_EPI_WARP0 = 4, TG_EPI_WARPS = 8;
 // Products of one copy with N <= 128 are issued by two threads (lane 0 of warps 1 and 2), which take the K = 16 slices of a
 // k-step alternately, each into an accumulator of its own (MMAs of different threads are not ordered among themselves), and
 // commit to the stage's "empty" and the tile's "accumulator full" barriers, which count `issuers` arrivals.
-template <int NS, class CS, bool PAIR>
+// (NARROW apart from the rest: its branches in the producer and the issuer cost the others 5 % of a launch.)
+template <int NS, class CS, bool PAIR, bool NARROW>
 __global__ void __launch_bounds__(TG_THREADS, 1)
 tma_gemm_kernel(const __grid_constant__ TmaMapSet<phases_of<CS>::value> maps, CS cs, TmaGemmParams p) {
     extern __shared__ unsigned char smem_raw[];
@@ -335,11 +341,11 @@ tma_gemm_kernel(const __grid_constant__ TmaMapSet<phases_of<CS>::value> maps, CS
     const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
     // a tile shared by the CTAs of a cluster: `part` is this CTA's share of its contraction (one tile per cluster)
     const int shared = PAIR ? 1 : p.shared, part = shared > 1 ? (int)cluster_ctarank() : 0;
-    const int worker = PAIR ? (int)(blockIdx.x >> 1) : (shared > 1 ? (int)blockIdx.x / shared : (int)blockIdx.x);
+    const int worker = p.first + (PAIR ? (int)(blockIdx.x >> 1) : (shared > 1 ? (int)blockIdx.x / shared : (int)blockIdx.x));
     const int nworkers = PAIR ? (int)(gridDim.x >> 1) : (shared > 1 ? (int)gridDim.x / shared : (int)gridDim.x);
     const int bh = PAIR ? bn >> 1 : bn;                       // columns of B this CTA stages
     const int mtiles = (p.M + TM - 1) / TM, ntiles = (p.N + bn - 1) / bn;
-    const int total_tiles = mtiles * ntiles * p.splits;
+    const int total_tiles = p.tiles;
     const bool a_mn = p.a_mode == TMA_A_COLS || p.a_mode == TMA_A_TAPS;
 
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -414,7 +420,7 @@ tma_gemm_kernel(const __grid_constant__ TmaMapSet<phases_of<CS>::value> maps, CS
             int box_c[2] = {0, 0}, box_s[4] = {0, 0, 0, 0}, box_r[4] = {0, 0, 0, 0};
             bool box_ok[4] = {true, true, true, true};
             uint32_t tx_bytes = PAIR ? 2u * stage_bytes : stage_bytes;     // a pair counts both CTAs' bytes on the even CTA's barrier
-            if (p.a_mode == TMA_A_TAPS && p.narrow) {
+            if (NARROW && p.a_mode == TMA_A_TAPS) {
 #pragma unroll
                 for (int b = 0; b < 4; b++) {
                     const int tap = (m0 >> 5) + b;
@@ -455,7 +461,7 @@ tma_gemm_kernel(const __grid_constant__ TmaMapSet<phases_of<CS>::value> maps, CS
 #pragma unroll
                     for (int i = 0; i < NS; i++)
                         for (int b = 0; b < 2; b++) ld2d(a_tile(s, i) + b * 8192, &mA[i], m0 + 64 * b, k0, bar);
-                } else if (p.narrow) {
+                } else if (NARROW) {
                     if (p.a_mode == TMA_A_IM2COL) {
 #pragma unroll
                         for (int h = 0; h < 2; h++) {
@@ -496,7 +502,7 @@ tma_gemm_kernel(const __grid_constant__ TmaMapSet<phases_of<CS>::value> maps, CS
                         for (int b = 0; b < 2; b++)
                             if (box_ok[b]) ldim(a_tile(s, i) + b * 8192, &mA[i], box_c[b], w, h, img, box_s[b], box_r[b], bar);
                 }
-                if (p.narrow && p.a_mode == TMA_A_IM2COL) {
+                if (NARROW && p.a_mode == TMA_A_IM2COL) {
                     // above, beside A
                 } else if (p.b_mn) {
 #pragma unroll
@@ -527,7 +533,7 @@ tma_gemm_kernel(const __grid_constant__ TmaMapSet<phases_of<CS>::value> maps, CS
         if (PAIR) idesc = (idesc & ~(31u << 24)) | ((uint32_t)(TM >> 4) << 24);          // M = 256 over the two CTAs
         const uint32_t idesc2 = umma_idesc_16bit(2 * bn, p.a_fp16, p.b_fp16) | ((uint32_t)(a_mn ? 1 : 0) << 15) | ((uint32_t)p.b_mn << 16);
         // bytes from slice 0 to the next K = 16 slice and to the third
-        const bool a64 = p.narrow != 0, b64 = a64 && !p.b_mn;
+        const bool a64 = NARROW, b64 = NARROW && !p.b_mn;
         const uint32_t a_step = a_mn ? (a64 ? 1024u : 2048u) : 32u, b_step = p.b_mn ? 2048u : 32u;
         const uint32_t a_far = a64 && !a_mn ? 8192u : 2 * a_step, b_far = b64 ? (uint32_t)NS * (b_bytes >> 1) : 2 * b_step;
         // split products kept: hi*hi | + hi*lo, lo*hi | + hi*lo2, lo2*hi, lo*lo
@@ -541,6 +547,7 @@ tma_gemm_kernel(const __grid_constant__ TmaMapSet<phases_of<CS>::value> maps, CS
         // which never carries out of its 14 bits for addresses inside the CTA's shared memory
         const uint32_t a_step16 = a_step >> 4, b_step16 = b_step >> 4, a_copy16 = a_bytes >> 4, b_copy16 = b64 ? b_bytes >> 5 : b_bytes >> 4;
         const uint32_t a_far16 = a_far >> 4, b_far16 = b_far >> 4;
+        auto at = [](int jj, uint32_t step, uint32_t far) { return NARROW ? (uint32_t)(jj & 1) * step + (uint32_t)(jj >> 1) * far : (uint32_t)jj * step; };
         const uint64_t da0 = (a64 ? (a_mn ? umma_desc_sw64_mn(a_tile(0, 0), 4096) : umma_desc_sw64(a_tile(0, 0)))
                                   : (a_mn ? umma_desc_sw128_mn(a_tile(0, 0), 8192) : umma_desc_sw128(a_tile(0, 0)))) + (uint32_t)me * a_step16;
         const uint64_t db0 = (p.b_mn ? umma_desc_sw128_mn(b_tile(0, 0), 8192) : (b64 ? umma_desc_sw64(b_tile(0, 0)) : umma_desc_sw128(b_tile(0, 0)))) +
@@ -590,14 +597,14 @@ tma_gemm_kernel(const __grid_constant__ TmaMapSet<phases_of<CS>::value> maps, CS
                 if (NS >= 2 && joined) {
 #pragma unroll
                     for (int jj = 0; jj < TC_BK / 16; jj++)
-                        slice_joined(das + (jj & 1) * a_step16 + (jj >> 1) * a_far16, dbs + (jj & 1) * b_step16 + (jj >> 1) * b_far16, jj == 0);
+                        slice_joined(das + at(jj, a_step16, a_far16), dbs + at(jj, b_step16, b_far16), jj == 0);
                 } else if (issuers == 2) {
 #pragma unroll
-                    for (int jj = 0; jj < TC_BK / 32; jj++) slice(das + (uint32_t)jj * a_far16, dbs + (uint32_t)jj * b_far16, jj == 0);
+                    for (int jj = 0; jj < TC_BK / 32; jj++) slice(das + at(2 * jj, a_step16, a_far16), dbs + at(2 * jj, b_step16, b_far16), jj == 0);
                 } else {
 #pragma unroll
                     for (int jj = 0; jj < TC_BK / 16; jj++)
-                        slice(das + (jj & 1) * a_step16 + (jj >> 1) * a_far16, dbs + (jj & 1) * b_step16 + (jj >> 1) * b_far16, jj == 0);
+                        slice(das + at(jj, a_step16, a_far16), dbs + at(jj, b_step16, b_far16), jj == 0);
                 }
                 if (PAIR) umma2_commit_both(empty0 + 8 * s); else umma_commit(empty0 + 8 * s);
                 }
@@ -834,10 +841,13 @@ int launch_tma_gemm(const TmaMapSet<phases_of<CS>::value> &maps, TmaGemmParams p
     //                       each CTA; for as many tiles as clusters of that size fit on the chip at once
     //   split with partial sums (allow_split): items of (tile, part) in rounds, a second launch of 3 us that adds the parts up, and
     //                       the parts' way to L2 and back, 4 (2 parts + 1) M N bytes at 5 TB/s
+    // Where the tiles of a last round are few, that round goes to clusters too, as a launch of its own (6 us): 12432 x 256 x
+    // 2304 in six products (148 + 48 tiles) 75 -> 67 us.
     // At least two k-steps for every CTA.  Ties go to fewer parts.  1600 x 256 x 2304 in six products (26 tiles,
     // 38 us by one CTA each): 23.5 / 18.6 / 16.8 / 16.2 us by clusters of 2 / 3 / 4 / 5; 1000 x 1024 x 784 (64 tiles) 20.3 -> 15.1.  For 128 x
     // 128 x 2304 (one tile, 37.5) clusters of 8 take 12.5 and a split of 18 with its reduction 7.5 + 4.2.
-    int splits = 1;
+    int splits = 1, rest_shared = 0;               // rest_shared: CTAs a tile of the last round
+    long long rest = 0;                            // its tiles
     p.shared = 1;
     const long long ksteps = (p.K + TC_BK - 1) / TC_BK;
     if (p.phases) {
@@ -847,15 +857,24 @@ int launch_tma_gemm(const TmaMapSet<phases_of<CS>::value> &maps, TmaGemmParams p
         const double kstep_us = tma_kstep_us(p.bn, ns, p.joined, stage);
         auto rounds_us = [&](long long items, long long per) { return (double)((items + sms - 1) / sms) * (per * kstep_us + 1.); };
         double best = rounds_us(tiles, ksteps);
-        if (!p.pair) {
-            for (int c = 2; c <= 8 && 2 * c <= ksteps; c++) {
+        // the cluster size that finishes `n` tiles first, if that is before `t`
+        auto clusters = [&](long long n, double &t) {
+            int size = 0;
+            for (int c = 2; c <= 8 && 2 * c <= ksteps && !p.pair; c++) {
                 const size_t chunks = (size_t)p.bn / 8;
                 if ((chunks + c - 1) / c * c * 4096 > stages * stage) continue;        // every share of a CTA's chunks, where the ring was
                 const long long per = (ksteps + c - 1) / c;
-                if (tiles * c > sms || (c - 1) * per >= ksteps) continue;
-                const double t = per * kstep_us + 3. + 0.25 * c;
-                if (t < best && tiles <= clusters_at_once(c)) { best = t; p.shared = c; }
+                if (n * c > sms || (c - 1) * per >= ksteps) continue;
+                const double u = per * kstep_us + 3. + 0.25 * c;
+                if (u < t && n <= clusters_at_once(c)) { t = u; size = c; }
             }
+            return size;
+        };
+        if (const int c = clusters(tiles, best)) p.shared = c;
+        if (tiles > sms && tiles % sms) {
+            double last = rounds_us(1, ksteps) - 6.;
+            rest_shared = clusters(tiles % sms, last);
+            if (rest_shared) { rest = tiles % sms; best = rounds_us(tiles - rest, ksteps) + 6. + last; }
         }
         if (allow_split) {
             const double pass_us = (double)p.M * p.N * 4. / 5e6;
@@ -863,7 +882,7 @@ int launch_tma_gemm(const TmaMapSet<phases_of<CS>::value> &maps, TmaGemmParams p
             for (long long sp = 2; sp <= maxs; sp++) {
                 const long long per = (ksteps + sp - 1) / sp, eff = (ksteps + per - 1) / per;
                 const double t = rounds_us(tiles * eff, per) + 3. + (2. * eff + 1.) * pass_us;
-                if (t < best) { best = t; splits = (int)eff; p.shared = 1; }
+                if (t < best) { best = t; splits = (int)eff; p.shared = 1; rest = 0; }
             }
         }
     }
@@ -885,15 +904,17 @@ int launch_tma_gemm(const TmaMapSet<phases_of<CS>::value> &maps, TmaGemmParams p
     }
     long long all_tiles = tiles * splits;
     const long long workers = p.pair ? rt().sm_count / 2 : rt().sm_count;
-    dim3 grid((unsigned)((all_tiles < workers ? all_tiles : workers) * (p.pair ? 2 : 1)));     // persistent: one CTA per SM at most
+    p.first = 0;
+    p.tiles = (int)(all_tiles - rest);
+    dim3 grid((unsigned)((p.tiles < workers ? p.tiles : workers) * (p.pair ? 2 : 1)));     // persistent: one CTA per SM at most
     if (p.shared > 1) grid.x = (unsigned)(tiles * p.shared);
-    const unsigned cluster = p.pair ? 2u : (unsigned)p.shared;
+    unsigned cluster = p.pair ? 2u : (unsigned)p.shared;
     cudaStream_t st = rt().stream;
     cudaError_t e;
     profile_begin();
-#define SEERA_TMA_LAUNCH(NSV, PAIRV)                                                                                       \
+#define SEERA_TMA_LAUNCH(NSV, PAIRV, NARROWV)                                                                              \
     {                                                                                                                      \
-        auto kern = tma_gemm_kernel<NSV, CS, PAIRV>;                                                                       \
+        auto kern = tma_gemm_kernel<NSV, CS, PAIRV, NARROWV>;                                                              \
         e = allow_smem((const void *)kern, 225 * 1024);                                                                    \
         if (e == cudaSuccess) {                                                                                            \
             cudaLaunchConfig_t cfg = {};                                                                                   \
@@ -906,10 +927,20 @@ int launch_tma_gemm(const TmaMapSet<phases_of<CS>::value> &maps, TmaGemmParams p
             if (e == cudaSuccess) e = cudaGetLastError();                                                                  \
         }                                                                                                                  \
     }
-    if (p.pair) { if (ns == 1) SEERA_TMA_LAUNCH(1, true) else SEERA_TMA_LAUNCH(2, true) }
-    else if (ns == 1) SEERA_TMA_LAUNCH(1, false) else if (ns == 2) SEERA_TMA_LAUNCH(2, false) else SEERA_TMA_LAUNCH(3, false)
+    for (int turn = 0; turn < (rest ? 2 : 1); turn++) {
+        if (turn) {
+            if (e != cudaSuccess) break;
+            p.first = p.tiles; p.tiles = (int)all_tiles; p.shared = rest_shared; p.skip_load = -1;
+            p.kchunk = (int)((ksteps + rest_shared - 1) / rest_shared) * TC_BK;
+            grid.x = (unsigned)(rest * rest_shared); cluster = (unsigned)rest_shared;
+        }
+        constexpr bool N = narrow_of<CS>::value;
+        if (p.pair) { if (ns == 1) SEERA_TMA_LAUNCH(1, true, false) else SEERA_TMA_LAUNCH(2, true, false) }
+        else if (N && p.narrow) { if (ns == 1) SEERA_TMA_LAUNCH(1, false, N) else if (ns == 2) SEERA_TMA_LAUNCH(2, false, N) else SEERA_TMA_LAUNCH(3, false, N) }
+        else if (ns == 1) SEERA_TMA_LAUNCH(1, false, false) else if (ns == 2) SEERA_TMA_LAUNCH(2, false, false) else SEERA_TMA_LAUNCH(3, false, false)
+        count_launch();
+    }
 #undef SEERA_TMA_LAUNCH
-    count_launch();
     if (e == cudaSuccess && p.partial) {
         launch_splitk_reduce(p, cs, splits, st);
         e = cudaGetLastError();

@@ -126,3 +126,22 @@ def test_layers_of_up_to_32_channels(sc, mode, N, C, H, W, F, K, st, pad):
     assert rel_l2(sc.to_host_f32(dw, w.shape), Wt.grad.numpy()) < (1e-3 if mode == 4 else TOL[mode])      # one fp16 product there
     for p in (xd, wd, gd, y, dx, dw):
         sc.cuda_free(p)
+
+
+@pytest.mark.parametrize("mode", [3, 4])
+def test_last_round_in_clusters(sc, mode):
+    """148 tiles and a few more, with a long contraction: the last ones are shared by clusters, in a launch of their own."""
+    sc.set_precision(mode)
+    rs = np.random.RandomState(mode)
+    N, C, H, F = 605, 256, 4, 250                              # 9680 x 250 x 2304: 76 x 2 tiles
+    x, b = rs.standard_normal((N, C, H, H)).astype(np.float32), rs.standard_normal(F).astype(np.float32)
+    w = (rs.standard_normal((F, C, 3, 3)) / np.sqrt(9 * C)).astype(np.float32)
+    xd, wd, bd = (sc.to_device_f32(t.ravel()) for t in (x, w, b))
+    y = sc.cuda_malloc_f32(N * F * H * H)
+    sc.shadow_free(sc.conv2d_bias_act_fwd_s(xd, wd, bd, y, N, C, H, H, F, 3, 3, 1, 1, 1, 1, 1, 0))
+    import torch
+    dev = lambda t: torch.from_numpy(t).double().cuda()                          # noqa: E731
+    ref = (torch.nn.functional.conv2d(dev(x), dev(w), padding=1) + dev(b).view(1, -1, 1, 1)).relu().cpu().numpy()
+    assert rel_l2(sc.to_host_f32(y, ref.shape), ref) < TOL[mode]
+    for p in (xd, wd, bd, y):
+        sc.cuda_free(p)
