@@ -239,7 +239,7 @@ __device__ __forceinline__ uint64_t umma_desc_sw64_mn(uint32_t addr, uint32_t bo
            (uint64_t)4 << 61;
 }
 
-// How the producer thread forms the A tile of a stage:
+// How the producer forms the A tile of a stage:
 //   TMA_A_ROWS    2-D map of a row-major matrix [M, K], read along its rows (K-major)
 //   TMA_A_COLS    2-D map of a row-major matrix [K, M], read along its columns (MN-major, two 64-wide boxes)
 //   TMA_A_IM2COL  im2col map of an NHWC tensor; M = output pixels, K = (tap, channel): one tap x 64 channels
@@ -300,8 +300,8 @@ struct TmaGemmParams {
     FastDiv by_mtiles, by_ntiles, by_OHW, by_OW, by_S, by_cchunks;      // filled by launch_tma_gemm
 };
 
-// warp 0: TMA producer; warps 1-2: MMA issuers (the first p.issuers of them); warp 3 allocates TMEM; warps 4-11: epilogue, two warps
-// per TMEM lane quarter, which take its 32-column chunks alternately.  One warp per quarter drained a 128 x 128 tile in about the
+// warps 0 and 3: TMA producers of A and B; warps 1-2: MMA issuers (the first p.issuers of them); warp 3 allocates TMEM; warps 4-11:
+// epilogue, two warps per TMEM lane quarter, which take its 32-column chunks alternately.  One warp per quarter drained a 128 x 128 tile in about the
 // time of twice its main loop (VGG, 128 filters at 16 x 16: launch 80 us, main loop alone 37 us).
 constexpr int TG_THREADS = 384, TG_EPI_WARP0 = 4, TG_EPI_WARPS = 8;
 
@@ -387,8 +387,11 @@ tma_gemm_kernel(const __grid_constant__ TmaMapSet<phases_of<CS>::value> maps, CS
         ktiles = (kend - kbeg + TC_BK - 1) / TC_BK;
     };
 
-    if (warp == 0) {
-        // ---------------- TMA producer ----------------
+    if (warp == 0 || warp == 3) {
+        // ---------------- TMA producers: warp 0 loads A, warp 3 (once it has allocated TMEM) B ----------------
+        // What a producer issues per k-step bounds the launches of one copy per operand, and those whose columns are few: one warp for both
+        // operands that found its coordinates by division took 75 ns more a k-step for a dozen instructions
+        // (weight gradient 576 x 128 x 131072 31.5 -> 27.9 us, 2304 x 256 x 50176 48.5 -> 44.2, data gradient 131072 x 64 x 1152 56 -> 52.9).
         const bool leader = elect_one();
         auto ld2d = [&](uint32_t dst, const CUtensorMap *m, int x, int y, uint32_t bar) {
             if (PAIR) tma2_load_2d(dst, m, x, y, bar); else tma_load_2d(dst, m, x, y, bar);
@@ -396,135 +399,155 @@ tma_gemm_kernel(const __grid_constant__ TmaMapSet<phases_of<CS>::value> maps, CS
         auto ldim = [&](uint32_t dst, const CUtensorMap *m, int c, int w, int h, int n, int ow, int oh, uint32_t bar) {
             if (PAIR) tma2_load_im2col(dst, m, c, w, h, n, ow, oh, bar); else tma_load_im2col(dst, m, c, w, h, n, ow, oh, bar);
         };
-        int it = 0, issued_from = 0;
+        int it = 0;
         int s = 0;                                            // ring slot and its phase, carried across tiles
         uint32_t ph = 0;
         bool alive = true;
+        const int c64 = p.cchunks * 64;
         for (int id = worker; id < total_tiles && alive; id += nworkers) {
             int m0, n0, kbeg, ktiles, z;
             tile_origin(id, m0, n0, kbeg, ktiles, z);
-            const int nb0 = n0 + (int)rank * bh;               // this CTA's own columns of B
-            // im2col, M = pixels: window corner of this tile's first output pixel
             const TmaMaps &own = maps.of[phases_of<CS>::value > 1 ? z : 0];
-            const CUtensorMap *mA = own.a, *mB = own.b;
             int S = p.S, taps = p.taps, pw = p.pw, phh = p.ph;
             FastDiv by_S = p.by_S;
             if (phases_of<CS>::value > 1) { S = p.phase[z].S; taps = p.phase[z].taps; pw = p.phase[z].pw; phh = p.phase[z].ph; by_S = p.phase[z].by_S; }
-            int pix_img = 0, pix_w = 0, pix_h = 0;
+            // im2col, M = pixels: the tap and channel of the next k-step, counted on from the first one's
+            int tap = 0, c0 = 0, r = 0, sx = 0;
             if (p.a_mode == TMA_A_IM2COL) {
-                pix_img = p.by_OHW.div(m0);
-                int rem = m0 - pix_img * p.OHW, oh = p.by_OW.div(rem), ow = rem - oh * p.OW;
-                pix_w = ow * p.sw - pw; pix_h = oh * p.sh - phh;
+                const int ktile = kbeg >> 6;
+                tap = NARROW ? 2 * ktile : p.by_cchunks.div(ktile);
+                c0 = NARROW ? 0 : (ktile - tap * p.cchunks) * 64;
+                r = by_S.div(tap); sx = tap - r * S;
             }
-            // im2col, M = (tap, channel): the two 64-channel boxes of this tile
-            int box_c[2] = {0, 0}, box_s[4] = {0, 0, 0, 0}, box_r[4] = {0, 0, 0, 0};
-            bool box_ok[4] = {true, true, true, true};
-            uint32_t tx_bytes = PAIR ? 2u * stage_bytes : stage_bytes;     // a pair counts both CTAs' bytes on the even CTA's barrier
-            if (NARROW && p.a_mode == TMA_A_TAPS) {
+            auto next_tap = [&]() { tap++; if (++sx == S) { sx = 0; r++; } };
+            if (warp == 0) {
+                const CUtensorMap *mA = own.a;
+                // window corner of this tile's first output pixel
+                int pix_img = 0, pix_w = 0, pix_h = 0;
+                if (p.a_mode == TMA_A_IM2COL) {
+                    pix_img = p.by_OHW.div(m0);
+                    const int rem = m0 - pix_img * p.OHW, oh = p.by_OW.div(rem), ow = rem - oh * p.OW;
+                    pix_w = ow * p.sw - pw; pix_h = oh * p.sh - phh;
+                }
+                // im2col, M = (tap, channel): the boxes of this tile, and the first pixel of the next k-step
+                constexpr int BOXES = NARROW ? 4 : 2, BOX = TC_BM / BOXES;             // rows of a box: channels of one tap
+                int box_c[BOXES] = {}, box_s[BOXES] = {}, box_r[BOXES] = {}, img = 0, rem = 0;
+                bool box_ok[BOXES] = {};
+                uint32_t tx_bytes = PAIR ? 2u * stage_bytes : stage_bytes;     // a pair counts both CTAs' bytes on the even CTA's barrier
+                if (p.a_mode == TMA_A_TAPS) {
 #pragma unroll
-                for (int b = 0; b < 4; b++) {
-                    const int tap = (m0 >> 5) + b;
-                    box_ok[b] = tap < p.taps;
-                    box_r[b] = by_S.div(tap); box_s[b] = tap - box_r[b] * S;
-                    if (!box_ok[b]) tx_bytes -= (uint32_t)NS * 4096u;
-                }
-            } else if (p.a_mode == TMA_A_TAPS) {
-                int c64 = p.cchunks * 64;
-                for (int b = 0; b < 2; b++) {
-                    int mb = m0 + 64 * b, tap = p.by_cchunks.div(mb >> 6);
-                    box_ok[b] = tap < p.taps;
-                    box_c[b] = mb - tap * c64; box_r[b] = p.by_S.div(tap); box_s[b] = tap - box_r[b] * p.S;
-                    if (!box_ok[b]) tx_bytes -= (uint32_t)NS * 8192u;
-                }
-                if (PAIR && rank == 0) {                       // the peer's boxes beyond the last tap are not loaded either
-                    for (int b = 0; b < 2; b++) {
-                        int mb = m0 + TC_BM + 64 * b, tap = p.by_cchunks.div(mb >> 6);
-                        if (tap >= p.taps) tx_bytes -= (uint32_t)NS * 8192u;
+                    for (int b = 0; b < BOXES; b++) {
+                        const int mb = m0 + BOX * b, at = NARROW ? mb >> 5 : p.by_cchunks.div(mb >> 6);
+                        box_ok[b] = at < p.taps;
+                        box_c[b] = NARROW ? 0 : mb - at * c64; box_r[b] = p.by_S.div(at); box_s[b] = at - box_r[b] * p.S;
+                        if (!box_ok[b]) tx_bytes -= (uint32_t)NS * (uint32_t)(BOX * 128);
                     }
+                    if (PAIR && rank == 0) {                       // the peer's boxes beyond the last tap are not loaded either
+                        for (int b = 0; b < 2; b++) {
+                            const int mb = m0 + TC_BM + 64 * b, at = p.by_cchunks.div(mb >> 6);
+                            if (at >= p.taps) tx_bytes -= (uint32_t)NS * 8192u;
+                        }
+                    }
+                    img = p.by_OHW.div(kbeg); rem = kbeg - img * p.OHW;
                 }
-            }
-            for (int kt = 0; kt < ktiles; kt++, it++) {
-                if (!mbar_wait(empty0 + 8 * s, ph ^ 1u, abortp, p.status, 1, p.wait_clocks)) { alive = false; break; }
-                int k0 = kbeg + kt * TC_BK;
-                const uint32_t bar = PAIR ? mapa_rank(full0 + 8 * s, 0) : full0 + 8 * s;
-                if (p.skip_load >= 0 && blockIdx.x == 0 && it == p.skip_load) {      // test hook: this stage never fills
-                    if (++s == stages) { s = 0; ph ^= 1u; }
-                    continue;
-                }
-                if (leader) {
-                if (rank == 0) mbar_expect_tx(full0 + 8 * s, tx_bytes);
-                int bk = k0, bx = 0;                          // B's coordinate along the contraction, and where its columns begin
-                if (p.a_mode == TMA_A_ROWS) {
+                for (int kt = 0; kt < ktiles; kt++, it++) {
+                    if (!mbar_wait(empty0 + 8 * s, ph ^ 1u, abortp, p.status, 1, p.wait_clocks)) { alive = false; break; }
+                    const int k0 = kbeg + kt * TC_BK;
+                    const uint32_t bar = PAIR ? mapa_rank(full0 + 8 * s, 0) : full0 + 8 * s;
+                    const bool skip = p.skip_load >= 0 && blockIdx.x == 0 && it == p.skip_load;      // test hook: this stage never fills
+                    if (leader && !skip) {
+                        if (rank == 0) mbar_expect_tx(full0 + 8 * s, tx_bytes);
+                        if (p.a_mode == TMA_A_ROWS) {
 #pragma unroll
-                    for (int i = 0; i < NS; i++) ld2d(a_tile(s, i), &mA[i], k0, m0, bar);
-                } else if (p.a_mode == TMA_A_COLS) {
+                            for (int i = 0; i < NS; i++) ld2d(a_tile(s, i), &mA[i], k0, m0, bar);
+                        } else if (p.a_mode == TMA_A_COLS) {
 #pragma unroll
-                    for (int i = 0; i < NS; i++)
-                        for (int b = 0; b < 2; b++) ld2d(a_tile(s, i) + b * 8192, &mA[i], m0 + 64 * b, k0, bar);
-                } else if (NARROW) {
+                            for (int i = 0; i < NS; i++)
+                                for (int b = 0; b < 2; b++) ld2d(a_tile(s, i) + b * 8192, &mA[i], m0 + 64 * b, k0, bar);
+                        } else if (p.a_mode == TMA_A_IM2COL) {
+#pragma unroll
+                            for (int h = 0; h < (NARROW ? 2 : 1); h++) {
+                                const bool in = !NARROW || tap < taps;             // else: zeros, from beyond the channels
+#pragma unroll
+                                for (int i = 0; i < NS; i++)
+                                    ldim(a_tile(s, i) + h * 8192, &mA[i], in ? c0 : 32, pix_w, pix_h, pix_img, in ? sx : 0, in ? r : 0, bar);
+                                if (NARROW) next_tap();
+                            }
+                        } else {
+                            const int oh = p.by_OW.div(rem), ow = rem - oh * p.OW, w = ow * p.sw - p.pw, h = oh * p.sh - p.ph;
+#pragma unroll
+                            for (int i = 0; i < NS; i++)
+#pragma unroll
+                                for (int b = 0; b < BOXES; b++)
+                                    if (box_ok[b]) ldim(a_tile(s, i) + b * (BOX * 128), &mA[i], box_c[b], w, h, img, box_s[b], box_r[b], bar);
+                        }
+                    }
                     if (p.a_mode == TMA_A_IM2COL) {
+                        if (NARROW) { if (!leader || skip) { next_tap(); next_tap(); } }
+                        else if ((c0 += 64) == c64) { c0 = 0; next_tap(); }
+                    } else if (p.a_mode == TMA_A_TAPS) {
+                        if (p.OHW >= TC_BK) { if ((rem += TC_BK) >= p.OHW) { rem -= p.OHW; img++; } }
+                        else { img = p.by_OHW.div(k0 + TC_BK); rem = k0 + TC_BK - img * p.OHW; }
+                    }
+                    if (++s == stages) { s = 0; ph ^= 1u; }
+                }
+            } else {
+                const CUtensorMap *mB = own.b;
+                const int nb0 = n0 + (int)rank * bh;               // this CTA's own columns of B
+                for (int kt = 0; kt < ktiles; kt++, it++) {
+                    if (!mbar_wait(empty0 + 8 * s, ph ^ 1u, abortp, p.status, 1, p.wait_clocks)) { alive = false; break; }
+                    const uint32_t bar = PAIR ? mapa_rank(full0 + 8 * s, 0) : full0 + 8 * s;
+                    const bool skip = p.skip_load >= 0 && blockIdx.x == 0 && it == p.skip_load;
+                    if (leader && !skip) {
+                        if (NARROW && p.a_mode == TMA_A_IM2COL) {
 #pragma unroll
-                        for (int h = 0; h < 2; h++) {
-                            const int tap = (k0 >> 5) + h, r = by_S.div(tap), sx = tap - r * S;
-                            const bool in = tap < taps;             // else: zeros, from beyond the channels
+                            for (int h = 0; h < 2; h++) {
+                                const int at = tap + h;
+                                const bool in = at < taps;
 #pragma unroll
-                            for (int i = 0; i < NS; i++) {
-                                ldim(a_tile(s, i) + h * 8192, &mA[i], in ? 0 : 32, pix_w, pix_h, pix_img, in ? sx : 0, in ? r : 0, bar);
-                                if (p.b_mn) {
-                                    for (int b = 0; b < bh / 64; b++)
-                                        ld2d(b_tile(s, i) + b * 8192 + h * 4096, &mB[i], (in ? (taps - 1 - tap) * p.wflip : 0) + nb0 + 64 * b, in ? 0 : 32, bar);
-                                } else {
-                                    ld2d(b_tile(s, 0) + (uint32_t)(h * NS + i) * (b_bytes >> 1), &mB[i], tap * p.cpad, nb0, bar);
+                                for (int i = 0; i < NS; i++) {
+                                    if (p.b_mn) {
+                                        for (int b = 0; b < bh / 64; b++)
+                                            ld2d(b_tile(s, i) + b * 8192 + h * 4096, &mB[i], (in ? (taps - 1 - at) * p.wflip : 0) + nb0 + 64 * b, in ? 0 : 32, bar);
+                                    } else {
+                                        ld2d(b_tile(s, 0) + (uint32_t)(h * NS + i) * (b_bytes >> 1), &mB[i], at * p.cpad, nb0, bar);
+                                    }
                                 }
                             }
+                        } else {
+                            // B's coordinate along the contraction, and where its columns begin
+                            int bk = kbeg + kt * TC_BK, bx = 0;
+                            if (p.a_mode == TMA_A_IM2COL) {
+                                if (p.b_mn) { bk = c0; bx = (taps - 1 - tap) * p.wflip; }
+                                else bk = tap * p.cpad + c0;
+                            }
+                            if (p.b_mn) {
+#pragma unroll
+                                for (int i = 0; i < NS; i++)
+                                    for (int b = 0; b < bh / 64; b++) ld2d(b_tile(s, i) + b * 8192, &mB[i], bx + nb0 + 64 * b, bk, bar);
+                            } else {
+#pragma unroll
+                                for (int i = 0; i < NS; i++) ld2d(b_tile(s, i), &mB[i], bk, nb0, bar);
+                            }
                         }
-                    } else {
-                        int img = p.by_OHW.div(k0), rem = k0 - img * p.OHW, oh = p.by_OW.div(rem), ow = rem - oh * p.OW;
-                        int w = ow * p.sw - p.pw, h = oh * p.sh - p.ph;
-#pragma unroll
-                        for (int i = 0; i < NS; i++)
-#pragma unroll
-                            for (int b = 0; b < 4; b++)
-                                if (box_ok[b]) ldim(a_tile(s, i) + b * 4096, &mA[i], 0, w, h, img, box_s[b], box_r[b], bar);
                     }
-                } else if (p.a_mode == TMA_A_IM2COL) {
-                    int ktile = k0 >> 6, tap = p.by_cchunks.div(ktile), c0 = (ktile - tap * p.cchunks) * 64;
-                    int r = by_S.div(tap), sx = tap - r * S;
-#pragma unroll
-                    for (int i = 0; i < NS; i++) ldim(a_tile(s, i), &mA[i], c0, pix_w, pix_h, pix_img, sx, r, bar);
-                    if (p.b_mn) { bk = c0; bx = (p.taps - 1 - tap) * p.wflip; }
-                    else bk = tap * p.cpad + c0;
-                } else {
-                    int img = p.by_OHW.div(k0), rem = k0 - img * p.OHW, oh = p.by_OW.div(rem), ow = rem - oh * p.OW;
-                    int w = ow * p.sw - p.pw, h = oh * p.sh - p.ph;
-#pragma unroll
-                    for (int i = 0; i < NS; i++)
-                        for (int b = 0; b < 2; b++)
-                            if (box_ok[b]) ldim(a_tile(s, i) + b * 8192, &mA[i], box_c[b], w, h, img, box_s[b], box_r[b], bar);
+                    if (p.a_mode == TMA_A_IM2COL) {
+                        if (NARROW) tap += 2;
+                        else if ((c0 += 64) == c64) { c0 = 0; tap++; }
+                    }
+                    if (++s == stages) { s = 0; ph ^= 1u; }
                 }
-                if (NARROW && p.a_mode == TMA_A_IM2COL) {
-                    // above, beside A
-                } else if (p.b_mn) {
-#pragma unroll
-                    for (int i = 0; i < NS; i++)
-                        for (int b = 0; b < bh / 64; b++) ld2d(b_tile(s, i) + b * 8192, &mB[i], bx + nb0 + 64 * b, bk, bar);
-                } else {
-#pragma unroll
-                    for (int i = 0; i < NS; i++) ld2d(b_tile(s, i), &mB[i], bk, nb0, bar);
-                }
-                }
-                if (++s == stages) { s = 0; ph ^= 1u; }
             }
         }
         if (*abortp && rank == 0) {
             // give copies already in flight a bounded chance to land before the CTA's shared memory goes away
-            issued_from = it - stages < 0 ? 0 : it - stages;
-            for (int k = issued_from; k < it; k++) {
+            for (int k = it - stages < 0 ? 0 : it - stages; k < it; k++) {
                 unsigned long long t0 = clock64();
                 if (p.skip_load >= 0 && blockIdx.x == 0 && k == p.skip_load) continue;      // nothing was issued for it
                 while (!mbar_try_wait(full0 + 8 * (k % stages), (uint32_t)(k / stages) & 1u) && clock64() - t0 < p.wait_clocks) {}
             }
         }
+        __syncwarp();
     } else if (warp >= 1 && warp <= issuers && rank == 0) {
         // ---------------- MMA issuers (in the even CTA of a pair) ----------------
         const bool leader = elect_one();
