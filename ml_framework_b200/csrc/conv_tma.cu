@@ -446,9 +446,9 @@ static int tma_dgrad_phases(const NhwcShadow &g, const float *Wt, long long so, 
         p.M = g.NB * GH * GW; p.N = Nch;
         plan_channels(p, g.Cp, list[first].taps, 1);           // (the most taps of the launch's phases)
         p.OW = GW; p.OHW = GH * GW; p.sw = 1; p.sh = 1;
+        p.phases = n;
         tma_plan(p, ns, false);
         p.pair = 0;
-        p.phases = n;
         TmaMapSet<TMA_PHASES> set{};
         const StorePhaseRows cs{out, Nch, H, W, sh, sw, 0, 0, fast_div(GH * GW), fast_div(GW)};
         double flops = 0;

@@ -805,6 +805,90 @@ inline int tma_pick_bn(int N, int ns, int b_mn) {
     return bn;
 }
 
+// Estimated time of a k-step: its MMAs (see tma_gemm_kernel) or its loads, at the 1.75 GHz that the tensor pipe's load leaves.
+inline double tma_kstep_us(int bn, int ns, int joined, size_t stage_bytes) {
+    auto mma = [](int n) { return n >= 128 ? n / 2 : 32 + n / 4; };
+    const int products = ns == 1 ? 1 : (ns == 2 ? 3 : 6);
+    const int slice = joined ? (ns == 2 ? mma(2 * bn) + mma(bn) : 2 * (mma(2 * bn) + mma(bn))) : products * mma(bn);
+    const double loads = 180. + (double)stage_bytes / 140.;
+    return (4. * slice > loads ? 4. * slice : loads) / 1750.;
+}
+
+// How many clusters of `size` CTAs of one SM each the chip holds at once (GPU processing clusters lose what is left over of their SMs).
+int clusters_at_once(int size);
+
+// Shared memory of a launch: bytes of a stage, stages that fit beside the epilogue's staging (227 KB per CTA on sm_100a; 2 KB are kept
+// for the kernel's static shared memory and alignment slack).
+inline size_t tma_stage_bytes(const TmaGemmParams &p, int bn, int ns) { return (size_t)ns * (TC_BM * 128 + (size_t)(p.pair ? bn / 2 : bn) * 128); }
+inline int tma_stages(size_t stage) {
+    const int n = (int)((225 * 1024 - TG_EPI_WARPS * EPI_WARP_SMEM - 1024) / stage);
+    return n > 8 ? 8 : n;
+}
+
+// How a product's contraction is shared out at an accumulator width, by estimated time (microseconds past a launch's start).  A tile's way
+// out takes 1 us for 128 columns.
+//   one CTA a tile:     rounds of tiles over the SMs, each its k-steps and a tile's way out
+//   a cluster a tile:   2 to 8 CTAs share the k-steps and add up through each other's shared memory, 2 us for 128 columns and 0.25 for
+//                       each CTA; for as many tiles as clusters of that size fit on the chip at once
+//   split with partial sums (allow_split): items of (tile, part) in rounds, a second launch of 3 us that adds the parts up, and
+//                       the parts' way to L2 and back, 4 (2 parts + 1) M N bytes at 5 TB/s
+// Where the tiles of a last round are few, that round goes to clusters too, as a launch of its own (6 us): 12432 x 256 x
+// 2304 in six products (148 + 48 tiles) 75 -> 67 us.
+// At least two k-steps for every CTA.  Ties go to fewer parts.  1600 x 256 x 2304 in six products (26 tiles,
+// 38 us by one CTA each): 23.5 / 18.6 / 16.8 / 16.2 us by clusters of 2 / 3 / 4 / 5; 1000 x 1024 x 784 (64 tiles) 20.3 -> 15.1.  For 128 x
+// 128 x 2304 (one tile, 37.5) clusters of 8 take 12.5 and a split of 18 with its reduction 7.5 + 4.2.
+struct TmaShare {
+    double us = 0.;
+    int splits = 1, shared = 1;                    // parts in memory; CTAs a tile
+    long long rest = 0;                            // tiles of a last round in clusters of
+    int rest_shared = 0;
+};
+inline TmaShare tma_share(const TmaGemmParams &p, int bn, int joined, int ns, bool allow_split) {
+    TmaShare r;
+    const size_t stage = tma_stage_bytes(p, bn, ns);
+    const int stages = tma_stages(stage), tm = p.pair ? 2 * TC_BM : TC_BM;
+    const long long sms = p.pair ? rt().sm_count / 2 : rt().sm_count;      // workers: CTAs, or pairs of them
+    const long long tiles = (long long)((p.M + tm - 1) / tm) * ((p.N + bn - 1) / bn), ksteps = (p.K + TC_BK - 1) / TC_BK;
+    // Weight gradients of convolutions: their loads of A take 0.36 us a k-step and copy at any width, and their outputs lie a filter's taps
+    // apart, one sector each: 8 us for a tile of 128 columns by one CTA.
+    const bool taps = p.a_mode == TMA_A_TAPS;
+    const double mma_us = tma_kstep_us(bn, ns, joined, stage), kstep_us = taps && mma_us < 0.36 * ns ? 0.36 * ns : mma_us;
+    const double out_us = bn / 128., scatter_us = taps ? 8. * out_us : 0.;
+    auto rounds_us = [&](long long items, long long per, double scatter) {
+        return (double)((items + sms - 1) / sms) * (per * kstep_us + out_us + scatter);
+    };
+    // the cluster size that finishes `n` tiles first, if that is before `t`
+    auto clusters = [&](long long n, double &t) {
+        int size = 0;
+        for (int c = 2; c <= 8 && 2 * c <= ksteps && !p.pair; c++) {
+            const size_t chunks = (size_t)bn / 8;
+            if ((chunks + c - 1) / c * c * 4096 > stages * stage) continue;        // every share of a CTA's chunks, where the ring was
+            const long long per = (ksteps + c - 1) / c;
+            if (n * c > sms || (c - 1) * per >= ksteps) continue;
+            const double u = per * kstep_us + 1. + (2. + 0.25 * c) * out_us + scatter_us / c;
+            if (u < t && n <= clusters_at_once(c)) { t = u; size = c; }
+        }
+        return size;
+    };
+    r.us = rounds_us(tiles, ksteps, scatter_us);
+    if (const int c = clusters(tiles, r.us)) r.shared = c;
+    if (tiles > sms && tiles % sms) {
+        double last = rounds_us(1, ksteps, scatter_us) - 6.;
+        r.rest_shared = clusters(tiles % sms, last);
+        if (r.rest_shared) { r.rest = tiles % sms; r.us = rounds_us(tiles - r.rest, ksteps, scatter_us) + 6. + last; }
+    }
+    if (allow_split) {
+        const double pass_us = (double)p.M * p.N * 4. / 5e6, sum_us = 3. + (taps ? (double)p.M * p.N / (1750. * sms) : 0.);
+        const long long maxs = ksteps / 2 < 256 ? ksteps / 2 : 256;
+        for (long long sp = 2; sp <= maxs; sp++) {
+            const long long per = (ksteps + sp - 1) / sp, eff = (ksteps + per - 1) / per;
+            const double t = rounds_us(tiles * eff, per, 0.) + sum_us + (2. * eff + 1.) * pass_us;
+            if (t < r.us) { r.us = t; r.splits = (int)eff; r.shared = 1; r.rest = 0; }
+        }
+    }
+    return r;
+}
+
 // Chooses the accumulator width and whether the launch runs as CTA pairs; sets p.bn and p.pair from p.M, p.N, p.b_mn.
 // Pairs pay when the operand stream bounds the kernel (the split modes: per CTA and k-step 128 + N/2 operand rows instead of
 // 128 + N) and there are enough 256-row tiles to keep 74 pairs busy; a launch that may split its contraction always has.
@@ -817,7 +901,14 @@ inline void tma_plan(TmaGemmParams &p, int ns, bool allow_split) {
     // moves the ReLU and pool decisions that lie on a tie, and programs that follow a run from version to version see that (a network with
     // batch normalisation: 1e-3 to 1e-2 of a first-layer gradient in one of ten seeds).  It costs 1.5 us of 14 at 32768 x 64 x 288 and
     // nothing for Dense layers; at 128 columns the joined form is 3 % faster (198912 x 128 x 576: 126 -> 122 us).
-    p.joined = ns >= 2 && p.bn <= 128 && !(ns == 3 && p.forward && (p.a_mode != TMA_A_IM2COL || p.bn < 128));
+    auto joined = [&](int bn) { return ns >= 2 && bn <= 128 && !(ns == 3 && p.forward && (p.a_mode != TMA_A_IM2COL || bn < 128)); };
+    // Half the width gives twice the tiles, which is worth its extra loads of A where the wider ones leave SMs without work or a long way out
+    // of the accumulators: 1000 x 1024 x 1024 in one product, 256 columns 12.4, 128 columns 9.3 us; 3136 x 512 x 4608 20.9 against 24.2.
+    // Not where the order of the sums is kept.
+    if (!p.phases && !(ns == 3 && p.forward) && !rt().pair_tiles)
+        while (p.bn >= 128 && tma_share(p, p.bn / 2, joined(p.bn / 2), ns, allow_split).us + 0.5 < tma_share(p, p.bn, joined(p.bn), ns, allow_split).us)
+            p.bn /= 2;
+    p.joined = joined(p.bn);
     p.issuers = p.bn <= 128 && !p.joined ? 2 : 1;
     if (rt().mma_issuers && rt().mma_issuers < p.issuers) p.issuers = rt().mma_issuers;
     if (!rt().pair_tiles || ns > 2 || rt().sm_count < 4 || p.narrow) return;
@@ -831,19 +922,6 @@ inline void tma_plan(TmaGemmParams &p, int ns, bool allow_split) {
     p.joined = 0;
 }
 
-// Estimated time of a k-step: its MMAs (see tma_gemm_kernel) or its loads at 80 bytes a clock, at the 1.75 GHz that the tensor pipe's
-// load leaves.
-inline double tma_kstep_us(int bn, int ns, int joined, size_t stage_bytes) {
-    auto mma = [](int n) { return n >= 128 ? n / 2 : 32 + n / 4; };
-    const int products = ns == 1 ? 1 : (ns == 2 ? 3 : 6);
-    const int slice = joined ? (ns == 2 ? mma(2 * bn) + mma(bn) : 2 * (mma(2 * bn) + mma(bn))) : products * mma(bn);
-    const double loads = (double)stage_bytes / 80.;
-    return (4. * slice > loads ? 4. * slice : loads) / 1750.;
-}
-
-// How many clusters of `size` CTAs of one SM each the chip holds at once (GPU processing clusters lose what is left over of their SMs).
-int clusters_at_once(int size);
-
 // Launches the kernel on prepared tensor maps.  p.M, p.N, p.K (contraction length in elements), a_mode, b_mn, bn
 // and the geometry fields must be set; kchunk, stages, partial and status are filled here.
 template <class CS>
@@ -851,64 +929,15 @@ int launch_tma_gemm(const TmaMapSet<phases_of<CS>::value> &maps, TmaGemmParams p
                     const char *name) {
     if (p.issuers != 2 || p.pair || p.joined || 4 * p.bn > 512) p.issuers = 1;      // TMEM has 512 columns
     const int tm = p.pair ? 2 * TC_BM : TC_BM;
-    size_t stage = (size_t)ns * (TC_BM * 128 + (size_t)(p.pair ? p.bn / 2 : p.bn) * 128);
-    // 227 KB per CTA on sm_100a; keep 2 KB for the kernel's static shared memory and alignment slack
-    int stages = (int)((225 * 1024 - TG_EPI_WARPS * EPI_WARP_SMEM - 1024) / stage);
-    if (stages > 8) stages = 8;
+    const size_t stage = tma_stage_bytes(p, p.bn, ns);
+    const int stages = tma_stages(stage);
     if (stages < 2) return fail(SEERA_E_LIMIT, "%s: tile does not fit shared memory", name);
     size_t smem = stage * stages + TG_EPI_WARPS * EPI_WARP_SMEM + 1024;
-    long long tiles = (long long)((p.M + tm - 1) / tm) * ((p.N + p.bn - 1) / p.bn);
-    // How the contraction is shared out, by estimated time (microseconds past a launch's start).
-    //   one CTA a tile:     rounds of tiles over the SMs, each its k-steps and 1 us for the pipeline's fill and the tile's way out
-    //   a cluster a tile:   2 to 8 CTAs share the k-steps and add up through each other's shared memory, 2 us for that and 0.25 for
-    //                       each CTA; for as many tiles as clusters of that size fit on the chip at once
-    //   split with partial sums (allow_split): items of (tile, part) in rounds, a second launch of 3 us that adds the parts up, and
-    //                       the parts' way to L2 and back, 4 (2 parts + 1) M N bytes at 5 TB/s
-    // Where the tiles of a last round are few, that round goes to clusters too, as a launch of its own (6 us): 12432 x 256 x
-    // 2304 in six products (148 + 48 tiles) 75 -> 67 us.
-    // At least two k-steps for every CTA.  Ties go to fewer parts.  1600 x 256 x 2304 in six products (26 tiles,
-    // 38 us by one CTA each): 23.5 / 18.6 / 16.8 / 16.2 us by clusters of 2 / 3 / 4 / 5; 1000 x 1024 x 784 (64 tiles) 20.3 -> 15.1.  For 128 x
-    // 128 x 2304 (one tile, 37.5) clusters of 8 take 12.5 and a split of 18 with its reduction 7.5 + 4.2.
-    int splits = 1, rest_shared = 0;               // rest_shared: CTAs a tile of the last round
-    long long rest = 0;                            // its tiles
-    p.shared = 1;
-    const long long ksteps = (p.K + TC_BK - 1) / TC_BK;
-    if (p.phases) {
-        splits = p.phases;
-    } else {
-        const long long sms = p.pair ? rt().sm_count / 2 : rt().sm_count;      // workers: CTAs, or pairs of them
-        const double kstep_us = tma_kstep_us(p.bn, ns, p.joined, stage);
-        auto rounds_us = [&](long long items, long long per) { return (double)((items + sms - 1) / sms) * (per * kstep_us + 1.); };
-        double best = rounds_us(tiles, ksteps);
-        // the cluster size that finishes `n` tiles first, if that is before `t`
-        auto clusters = [&](long long n, double &t) {
-            int size = 0;
-            for (int c = 2; c <= 8 && 2 * c <= ksteps && !p.pair; c++) {
-                const size_t chunks = (size_t)p.bn / 8;
-                if ((chunks + c - 1) / c * c * 4096 > stages * stage) continue;        // every share of a CTA's chunks, where the ring was
-                const long long per = (ksteps + c - 1) / c;
-                if (n * c > sms || (c - 1) * per >= ksteps) continue;
-                const double u = per * kstep_us + 3. + 0.25 * c;
-                if (u < t && n <= clusters_at_once(c)) { t = u; size = c; }
-            }
-            return size;
-        };
-        if (const int c = clusters(tiles, best)) p.shared = c;
-        if (tiles > sms && tiles % sms) {
-            double last = rounds_us(1, ksteps) - 6.;
-            rest_shared = clusters(tiles % sms, last);
-            if (rest_shared) { rest = tiles % sms; best = rounds_us(tiles - rest, ksteps) + 6. + last; }
-        }
-        if (allow_split) {
-            const double pass_us = (double)p.M * p.N * 4. / 5e6;
-            const long long maxs = ksteps / 2 < 256 ? ksteps / 2 : 256;
-            for (long long sp = 2; sp <= maxs; sp++) {
-                const long long per = (ksteps + sp - 1) / sp, eff = (ksteps + per - 1) / per;
-                const double t = rounds_us(tiles * eff, per) + 3. + (2. * eff + 1.) * pass_us;
-                if (t < best) { best = t; splits = (int)eff; p.shared = 1; rest = 0; }
-            }
-        }
-    }
+    const long long tiles = (long long)((p.M + tm - 1) / tm) * ((p.N + p.bn - 1) / p.bn), ksteps = (p.K + TC_BK - 1) / TC_BK;
+    const TmaShare how = p.phases ? TmaShare{} : tma_share(p, p.bn, p.joined, ns, allow_split);
+    int splits = p.phases ? p.phases : how.splits;
+    const long long rest = how.rest;
+    p.shared = how.shared;
     const int parts = p.shared > 1 ? p.shared : (p.phases ? 1 : splits);
     p.kchunk = (int)((ksteps + parts - 1) / parts) * TC_BK;
     if (!p.phases) splits = p.shared > 1 ? 1 : (p.K + p.kchunk - 1) / p.kchunk;
@@ -953,9 +982,9 @@ int launch_tma_gemm(const TmaMapSet<phases_of<CS>::value> &maps, TmaGemmParams p
     for (int turn = 0; turn < (rest ? 2 : 1); turn++) {
         if (turn) {
             if (e != cudaSuccess) break;
-            p.first = p.tiles; p.tiles = (int)all_tiles; p.shared = rest_shared; p.skip_load = -1;
-            p.kchunk = (int)((ksteps + rest_shared - 1) / rest_shared) * TC_BK;
-            grid.x = (unsigned)(rest * rest_shared); cluster = (unsigned)rest_shared;
+            p.first = p.tiles; p.tiles = (int)all_tiles; p.shared = how.rest_shared; p.skip_load = -1;
+            p.kchunk = (int)((ksteps + how.rest_shared - 1) / how.rest_shared) * TC_BK;
+            grid.x = (unsigned)(rest * how.rest_shared); cluster = (unsigned)how.rest_shared;
         }
         constexpr bool N = narrow_of<CS>::value;
         if (p.pair) { if (ns == 1) SEERA_TMA_LAUNCH(1, true, false) else SEERA_TMA_LAUNCH(2, true, false) }
