@@ -882,6 +882,8 @@ inline TmaShare tma_share(const TmaGemmParams &p, int bn, int joined, int ns, bo
         const long long maxs = ksteps / 2 < 256 ? ksteps / 2 : 256;
         for (long long sp = 2; sp <= maxs; sp++) {
             const long long per = (ksteps + sp - 1) / sp, eff = (ksteps + per - 1) / per;
+            if (eff < sp) continue;                            // seen at eff already
+            if (sum_us + (2. * eff + 1.) * pass_us >= r.us) break;
             const double t = rounds_us(tiles * eff, per, 0.) + sum_us + (2. * eff + 1.) * pass_us;
             if (t < r.us) { r.us = t; r.splits = (int)eff; r.shared = 1; r.rest = 0; }
         }
@@ -904,8 +906,8 @@ inline void tma_plan(TmaGemmParams &p, int ns, bool allow_split) {
     auto joined = [&](int bn) { return ns >= 2 && bn <= 128 && !(ns == 3 && p.forward && (p.a_mode != TMA_A_IM2COL || bn < 128)); };
     // Half the width gives twice the tiles, which is worth its extra loads of A where the wider ones leave SMs without work or a long way out
     // of the accumulators: 1000 x 1024 x 1024 in one product, 256 columns 12.4, 128 columns 9.3 us; 3136 x 512 x 4608 20.9 against 24.2.
-    // Not where the order of the sums is kept.
-    if (!p.phases && !(ns == 3 && p.forward) && !rt().pair_tiles)
+    // (A width changes no order of sums by itself; convolutions in six products are joined at 128 columns and not below.)
+    if (!p.phases && !(ns == 3 && p.forward && p.a_mode == TMA_A_IM2COL) && !rt().pair_tiles)
         while (p.bn >= 128 && tma_share(p, p.bn / 2, joined(p.bn / 2), ns, allow_split).us + 0.5 < tma_share(p, p.bn, joined(p.bn), ns, allow_split).us)
             p.bn /= 2;
     p.joined = joined(p.bn);
