@@ -35,16 +35,20 @@ _bare = object.__new__
 
 # What an operator needs to know of its operands' shapes, formed once per shape: a dense layer of 1000 x 784 x 1024 composed from operators,
 # with its reductions, is bound by the host, and this is 69 -> 61 us of it.
-@functools.lru_cache(maxsize=1024)
-def _reduced(shape, dim):
+def _reduction(shape, dim):
     nd = len(shape)
     at = dim + nd if dim < 0 else dim
     if at < 0 or at >= nd:
         raise ValueError(f"[cuTen]: dim {at} out of range for shape {shape}")
-    out_shape = shape[:at] + shape[at + 1:] or (1,)
+    out_shape = tuple(d for i, d in enumerate(shape) if i != at) or (1,)
     dims = np.array(shape, dtype=np.int32)
     dims.setflags(write=False)
     return out_shape, _numel(out_shape), nd, at, dims
+
+
+_reduced = functools.lru_cache(maxsize=1024)(_reduction)         # for an axis that is an int: 1.0 would be known as 1, and an array by its identity
+
+
 
 
 @functools.lru_cache(maxsize=1024)
@@ -354,7 +358,7 @@ class cuten:
 
     # ---- single-axis reductions ----------------------------------------------------------------------------------
     def _reduce(self, kernel, dim):
-        out_shape, out_size, nd, dim, dimarr = _reduced(tuple(self.shape), dim)
+        out_shape, out_size, nd, dim, dimarr = (_reduced if dim.__class__ is int else _reduction)(tuple(self.shape), dim)
         p = seera_cuda.cuda_malloc_f32(out_size)
         kernel(self.main_ptr, p, nd, dim, dimarr)
         return cuten._wrap(p, out_shape)
@@ -372,7 +376,7 @@ class cuten:
         return self._reduce(seera_cuda.cuda_min_fwd, dim)
 
     def _argreduce(self, kernel, dim):
-        out_shape, out_size, nd, dim, dimarr = _reduced(tuple(self.shape), dim)
+        out_shape, out_size, nd, dim, dimarr = (_reduced if dim.__class__ is int else _reduction)(tuple(self.shape), dim)
         p = seera_cuda.cuda_malloc_i32(out_size)
         kernel(self.main_ptr, p, nd, dim, dimarr)
         return cuten._wrap(p, out_shape, "int32")

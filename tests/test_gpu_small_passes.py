@@ -50,3 +50,21 @@ def test_both_gradients_of_a_narrow_product(M, K, N, shift):
     for p in (ad, bd, gd, da, db):
         sc.cuda_free(p)
     sc.set_precision(0)
+
+
+def test_axes_of_a_reduction():
+    """What is kept of a shape per axis does not take an axis for another: arrays count as they stand, a float is refused."""
+    import torch
+
+    from ml_framework_b200.cuTen import cuten
+    x = np.arange(24, dtype=np.float32).reshape(2, 3, 4)
+    c, axis, t = cuten(x), np.array(1), torch.tensor(1)
+    for dim in (1, np.int64(1), axis, t, -2, True):
+        assert np.array_equal(c.sum(dim).to_host_f32(), x.sum(1))
+    axis[...], t[...] = 0, 0
+    for dim in (axis, t):
+        assert np.array_equal(c.sum(dim).to_host_f32(), x.sum(0))
+    with pytest.raises(TypeError):
+        c.sum(1.0)
+    with pytest.raises(ValueError):
+        c.sum(3)
