@@ -3,7 +3,7 @@
 // The reference runs this layer on the CPU only, even in its GPU path (Seera_init.py:870-921 forward,
 // Seera_Engine.py:381-415 backward, engine/src/batchnorm_ops.cpp:12-138 the arithmetic): every batch goes device -> host
 // -> device around it.  Here it is two bandwidth-bound passes over the tensor forward (statistics, normalise) and two backward
-// (sums of dout and dout * x_hat, dx), each with a C-thread finalise between them.
+// (sums of dout and dout * x_hat, dx), each with a finalise of a warp per channel between them.
 //
 // Statistics.  The reference takes the mean first and the variance from the differences to it (two passes over x).  Here every
 // thread walks its share of a channel ONCE, accumulating sum (x - K) and sum (x - K)^2 around the first value K it meets - a
@@ -15,7 +15,7 @@
 // order.  x_hat is not stored: the backward recomputes it from the layer input, the saved mean and 1/std (one multiply-add
 // against a second activation-sized buffer of traffic).
 //
-// Layout [N, C, S] with S = H*W (1 for the 1-D form).  S > 1: a block owns one channel and a stripe of images and reads
+// Layout [N, C, S] with S = H*W (1 for the 1-D form).  S > 1: a block of the statistics owns one channel and a stripe of images and reads
 // its planes contiguously.  S == 1: a block owns 32 adjacent channels x a stripe of rows, so warps read rows contiguously.
 #include "common.cuh"
 #include "tc_ptx.cuh"          // FastDiv

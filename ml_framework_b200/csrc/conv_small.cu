@@ -7,8 +7,8 @@
 // with its border of zeros, the filters as [input channel][tap][output channel], and a warp forms 32 blocks of 2 x 2 outputs for FW output channels:
 // per input channel 8 reads of its own 4 x 4 patch and 9 broadcasts of FW weights for 36 FW / 2 packed multiply-adds.  The data
 // gradient is the same convolution of dz with the taps reversed; dz - activation slope, and the routing through a 2x2 max-pool - is
-// formed while the band is staged.  The weight gradient goes to first_dw in groups of four input channels, and a layer with its pool to
-// conv_pool_simt.
+// formed while the band is staged.  The weight gradient is first_dw's in groups of four input channels, in the same launch, and a
+// layer with its pool goes to conv_pool_simt.
 //
 // The forward of a layer with up to four input channels (stride 1 or 2) takes the same kernel at any size: it is bound by its stores - the
 // output and, for the convolution that reads it, the channels-last copies - of which a lane with 16 filters writes whole sectors, where

@@ -11,8 +11,8 @@
 //     dB = A^T * dC    A MN-major, dC MN-major (contraction over the batch rows, split-K)
 // all read the same three shadows.
 //
-// Warp 0 of a CTA issues TMA loads into a ring of stages (mbarrier expect_tx), warps 1-2 issue the MMAs
-// (tcgen05.commit releases a stage), warp 3 owns TMEM, warps 4-11 drain the 128 x BN fp32 accumulator with
+// Warps 0 and 3 of a CTA issue the TMA loads of A and B into a ring of stages (mbarrier expect_tx), warps 1-2 issue the MMAs
+// (tcgen05.commit releases a stage), warp 3 owns TMEM too, warps 4-11 drain the 128 x BN fp32 accumulator with
 // tcgen05.ld and store it.  Every mbarrier wait is bounded; on expiry a status word is set and the
 // CTA still waits (bounded) for its copies in flight and frees TMEM before it exits.
 #include "internal.h"

@@ -321,7 +321,7 @@ constexpr int TG_THREADS = 384, TG_EPI_WARP0 = 4, TG_EPI_WARPS = 8;
 // bn = 64, 25600 x 64 x 1152: 34.3 -> 31.8).  Sums in two accumulators are also shorter chains: 1.92e-6 -> 1.02e-6 of error at NS = 3
 // against float64, 1.08e-6 -> 7.1e-7 at NS = 2 on fp16 (512 x 64 x 576).  The epilogue adds the two accumulators; TMEM holds 2 buffers x 2 x bn columns (at most 512).
 //
-// Products of one copy with N <= 128 are issued by two threads (lane 0 of warps 1 and 2), which take the K = 16 slices of a
+// Products of one copy with N <= 128, and the forward ones in six products that tma_plan names, are issued by two threads (lane 0 of warps 1 and 2), which take the K = 16 slices of a
 // k-step alternately, each into an accumulator of its own (MMAs of different threads are not ordered among themselves), and
 // commit to the stage's "empty" and the tile's "accumulator full" barriers, which count `issuers` arrivals.
 // (NARROW apart from the rest: its branches in the producer and the issuer cost the others 5 % of a launch.)
