@@ -349,7 +349,7 @@ def test_checkpoint_written_by_the_reference_loads_and_predicts(host, golden_dir
     assert rel_l2(m.predict(X[:fit_case.BATCH]).to_numpy(), gold["pred"]) < 1e-5
 
 
-@pytest.mark.skipif(not os.path.isdir(REFERENCE), reason="reference checkout not present")
+@pytest.mark.skipif(not os.path.isfile(os.path.join(REFERENCE, "Seera.py")), reason="reference checkout not present")
 def test_unmodified_reference_python_layer_runs_on_this_cuten(host, golden_dir):
     """Drop-in check of the tensor class: the reference's own Seera.py / Seera_init.py /
     Seera_Engine.py, device="cuda", over this package's cuTen and the stand-in binding."""
