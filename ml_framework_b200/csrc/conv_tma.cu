@@ -304,7 +304,7 @@ static int tma_fprop(const NhwcShadow &x, const Shadow &wk, float *Y, int F, int
     p.M = x.NB * OH * OW; p.N = F;
     plan_channels(p, x.Cp, R * S, S);
     p.OW = OW; p.OHW = OH * OW; p.sw = sw; p.sh = sh; p.pw = pw; p.ph = ph;
-    tma_plan(p, ns, false);
+    const TmaShare how = tma_plan(p, ns, false);
     TmaMapSet<1> set;
     TmaMaps &maps = set.of[0];
     for (int i = 0; i < 3; i++) {
@@ -318,7 +318,7 @@ static int tma_fprop(const NhwcShadow &x, const Shadow &wk, float *Y, int F, int
         for (int i = 0; i < 3; i++) cs.cp[i] = ycopies->p[i];
         cs.Cp = ycopies->Cp; cs.ns = ns; cs.enc = ycopies->enc;
     }
-    return launch_tma_gemm(set, p, cs, ns, false, flops, name);
+    return launch_tma_gemm(set, p, cs, ns, how, flops, name);
 }
 
 // Unit-stride data gradient from the forward's filter copies w[F][tap][Cp] as they are: the contraction runs over (tap, filter), so
@@ -332,7 +332,7 @@ static int tma_dgrad_kept(const NhwcShadow &dy, const Shadow &w, float *dX, int 
     plan_channels(p, dy.Cp, R * S, S);
     p.wflip = w.cols / (R * S);
     p.OW = W; p.OHW = H * W; p.sw = 1; p.sh = 1; p.pw = S - 1 - pw; p.ph = R - 1 - ph;
-    tma_plan(p, ns, false);
+    const TmaShare how = tma_plan(p, ns, false);
     TmaMapSet<1> set;
     TmaMaps &maps = set.of[0];
     for (int i = 0; i < 3; i++) {
@@ -340,7 +340,7 @@ static int tma_dgrad_kept(const NhwcShadow &dy, const Shadow &w, float *dX, int 
         if (int s = make_map_im2col(&maps.a[i], dy.p[j], dy.NB, dy.H, dy.W, dy.Cp, R, S, 1, 1, p.ph, p.pw, p.narrow ? 32 : 64, TC_BM)) return s;
         if (int s = make_map_2d(&maps.b[i], w.p[j], w.rows, w.cols, w.ld, 64, p.narrow ? 32 : 64)) return s;
     }
-    return launch_tma_gemm(set, p, StorePixelRows{dX, C, H * W}, ns, false, 2.0 * p.M * (double)C * dy.C * R * S, name);
+    return launch_tma_gemm(set, p, StorePixelRows{dX, C, H * W}, ns, how, 2.0 * p.M * (double)C * dy.C * R * S, name);
 }
 
 // dW[Fo][C][R][S] = sum over output pixels of dY_nhwc[pix, f] * X_nhwc[window(pix)+tap, c]
@@ -355,7 +355,7 @@ static int tma_wgrad(const NhwcShadow &x, const NhwcShadow &dy, float *dW, int R
     p.M = p.taps * pitch; p.N = F;
     p.K = x.NB * OH * OW;
     p.OW = OW; p.OHW = OH * OW; p.sw = sw; p.sh = sh; p.pw = pw; p.ph = ph;
-    tma_plan(p, ns, true);
+    const TmaShare how = tma_plan(p, ns, true);
     TmaMapSet<1> set;
     TmaMaps &maps = set.of[0];
     for (int i = 0; i < 3; i++) {
@@ -364,7 +364,7 @@ static int tma_wgrad(const NhwcShadow &x, const NhwcShadow &dy, float *dW, int R
         if (int s = make_map_2d(&maps.b[i], dy.p[j], dy.NB * OH * OW, dy.Cp, dy.Cp, 64, 64)) return s;
     }
     double flops = 2.0 * p.K * (double)F * x.C * R * S;
-    return launch_tma_gemm(set, p, StoreWgrad{dW, x.C, R * S, pitch}, ns, true, flops, name);
+    return launch_tma_gemm(set, p, StoreWgrad{dW, x.C, R * S, pitch}, ns, how, flops, name);
 }
 
 // ---- strided data gradient by output phase ---------------------------------------------------------------------
@@ -447,8 +447,7 @@ static int tma_dgrad_phases(const NhwcShadow &g, const float *Wt, long long so, 
         plan_channels(p, g.Cp, list[first].taps, 1);           // (the most taps of the launch's phases)
         p.OW = GW; p.OHW = GH * GW; p.sw = 1; p.sh = 1;
         p.phases = n;
-        tma_plan(p, ns, false);
-        p.pair = 0;
+        const TmaShare how = tma_plan(p, ns, false);
         TmaMapSet<TMA_PHASES> set{};
         const StorePhaseRows cs{out, Nch, H, W, sh, sw, 0, 0, fast_div(GH * GW), fast_div(GW)};
         double flops = 0;
@@ -469,7 +468,7 @@ static int tma_dgrad_phases(const NhwcShadow &g, const float *Wt, long long so, 
             flops += 2.0 * g.NB * f.y.G * f.x.G * (double)Nch * g.C * f.taps;
         }
         p.K = p.phase[0].K;
-        if (!e) e = launch_tma_gemm(set, p, cs, ns, false, flops, name);
+        if (!e) e = launch_tma_gemm(set, p, cs, ns, how, flops, name);
         if (e) { free_shadow(all); return e; }
     }
     free_shadow(all);

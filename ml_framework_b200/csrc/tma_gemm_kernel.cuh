@@ -843,28 +843,36 @@ struct TmaShare {
     long long rest = 0;                            // tiles of a last round in clusters of
     int rest_shared = 0;
 };
+// The counts of parts worth trying for `ksteps` k-steps: after `parts`, the next one whose longest part is shorter (0: none).  Those between
+// leave parts without work, or as long as before: 2048 k-steps have 81 such counts up to 256.
+inline int tma_next_parts(int ksteps, int parts) {
+    const int per = (ksteps + parts - 1) / parts;
+    return per > 1 ? (ksteps + per - 2) / (per - 1) : 0;
+}
 inline TmaShare tma_share(const TmaGemmParams &p, int bn, int joined, int ns, bool allow_split) {
     TmaShare r;
     const size_t stage = tma_stage_bytes(p, bn, ns);
     const int stages = tma_stages(stage), tm = p.pair ? 2 * TC_BM : TC_BM;
-    const long long sms = p.pair ? rt().sm_count / 2 : rt().sm_count;      // workers: CTAs, or pairs of them
-    const long long tiles = (long long)((p.M + tm - 1) / tm) * ((p.N + bn - 1) / bn), ksteps = (p.K + TC_BK - 1) / TC_BK;
+    const int sms = p.pair ? rt().sm_count / 2 : rt().sm_count, ksteps = (p.K - 1) / TC_BK + 1;      // workers: CTAs, or pairs of them
+    const long long tiles = (long long)((p.M - 1) / tm + 1) * ((p.N - 1) / bn + 1);
     // Weight gradients of convolutions: their loads of A take 0.36 us a k-step and copy at any width, and their outputs lie a filter's taps
     // apart, one sector each: 8 us for a tile of 128 columns by one CTA.
     const bool taps = p.a_mode == TMA_A_TAPS;
     const double mma_us = tma_kstep_us(bn, ns, joined, stage), kstep_us = taps && mma_us < 0.36 * ns ? 0.36 * ns : mma_us;
     const double out_us = bn / 128., scatter_us = taps ? 8. * out_us : 0.;
-    auto rounds_us = [&](long long items, long long per, double scatter) {
-        return (double)((items + sms - 1) / sms) * (per * kstep_us + out_us + scatter);
+    auto rounds_us = [&](long long items, int per, double scatter) {
+        const long long up = items + sms - 1;                     // (a 64-bit division takes several times a 32-bit one)
+        const double rounds = up < (1ll << 32) ? (double)((unsigned)up / (unsigned)sms) : (double)(up / sms);
+        return rounds * (per * kstep_us + out_us + scatter);
     };
     // the cluster size that finishes `n` tiles first, if that is before `t`
     auto clusters = [&](long long n, double &t) {
         int size = 0;
-        for (int c = 2; c <= 8 && 2 * c <= ksteps && !p.pair; c++) {
-            const size_t chunks = (size_t)bn / 8;
-            if ((chunks + c - 1) / c * c * 4096 > stages * stage) continue;        // every share of a CTA's chunks, where the ring was
-            const long long per = (ksteps + c - 1) / c;
-            if (n * c > sms || (c - 1) * per >= ksteps) continue;
+        for (int c = 2; c <= 8 && 2 * c <= ksteps && n * c <= sms && !p.pair; c++) {
+            const unsigned chunks = (unsigned)bn / 8;
+            if ((chunks + c - 1) / c * c * (size_t)4096 > stages * stage) continue;        // every share of a CTA's chunks, where the ring was
+            const int per = (ksteps + c - 1) / c;
+            if ((c - 1) * per >= ksteps) continue;
             const double u = per * kstep_us + 1. + (2. + 0.25 * c) * out_us + scatter_us / c;
             if (u < t && n <= clusters_at_once(c)) { t = u; size = c; }
         }
@@ -879,22 +887,25 @@ inline TmaShare tma_share(const TmaGemmParams &p, int bn, int joined, int ns, bo
     }
     if (allow_split) {
         const double pass_us = (double)p.M * p.N * 4. / 5e6, sum_us = 3. + (taps ? (double)p.M * p.N / (1750. * sms) : 0.);
-        const long long maxs = ksteps / 2 < 256 ? ksteps / 2 : 256;
-        for (long long sp = 2; sp <= maxs; sp++) {
-            const long long per = (ksteps + sp - 1) / sp, eff = (ksteps + per - 1) / per;
-            if (eff < sp) continue;                            // seen at eff already
-            if (sum_us + (2. * eff + 1.) * pass_us >= r.us) break;
-            const double t = rounds_us(tiles * eff, per, 0.) + sum_us + (2. * eff + 1.) * pass_us;
-            if (t < r.us) { r.us = t; r.splits = (int)eff; r.shared = 1; r.rest = 0; }
+        // no count takes less than the k-steps evenly over the SMs (a little off that, for the roundings on the way)
+        const double least_us = (double)tiles * ksteps / sms * kstep_us * (1. - 1e-6) + sum_us;
+        const int maxs = ksteps / 2 < 256 ? ksteps / 2 : 256;
+        for (int parts = 2; parts && parts <= maxs; parts = tma_next_parts(ksteps, parts)) {
+            const double way_us = (2. * parts + 1.) * pass_us;
+            if (least_us + way_us >= r.us) break;
+            const double t = rounds_us(tiles * parts, (ksteps + parts - 1) / parts, 0.) + sum_us + way_us;
+            if (t < r.us) { r.us = t; r.splits = parts; r.shared = 1; r.rest = 0; }
         }
     }
     return r;
 }
 
-// Chooses the accumulator width and whether the launch runs as CTA pairs; sets p.bn and p.pair from p.M, p.N, p.b_mn.
+// Chooses the accumulator width and whether the launch runs as CTA pairs; sets p.bn and p.pair from p.M, p.N, p.b_mn and returns how the
+// contraction is shared out, for launch_tma_gemm.  Every call of a program that runs eagerly pays for this, so each width is estimated once
+// (2.7 GHz Xeon, a plan: 576 x 128 x 131072 in one product 7.2 -> 1.0 us, the same x 25600 in six 5.3 -> 0.7, 1152 x 256 x 6400 in six 1.6 -> 0.2).
 // Pairs pay when the operand stream bounds the kernel (the split modes: per CTA and k-step 128 + N/2 operand rows instead of
 // 128 + N) and there are enough 256-row tiles to keep 74 pairs busy; a launch that may split its contraction always has.
-inline void tma_plan(TmaGemmParams &p, int ns, bool allow_split) {
+inline TmaShare tma_plan(TmaGemmParams &p, int ns, bool allow_split) {
     p.bn = tma_pick_bn(p.N, ns, p.b_mn);
     p.pair = 0;
     // split products: one thread, B's first two copies as one operand; the others: two threads where TMEM has room for
@@ -907,27 +918,37 @@ inline void tma_plan(TmaGemmParams &p, int ns, bool allow_split) {
     // Half the width gives twice the tiles, which is worth its extra loads of A where the wider ones leave SMs without work or a long way out
     // of the accumulators: 1000 x 1024 x 1024 in one product, 256 columns 12.4, 128 columns 9.3 us; 3136 x 512 x 4608 20.9 against 24.2.
     // (A width changes no order of sums by itself; convolutions in six products are joined at 128 columns and not below.)
-    if (!p.phases && !(ns == 3 && p.forward && p.a_mode == TMA_A_IM2COL) && !rt().pair_tiles)
-        while (p.bn >= 128 && tma_share(p, p.bn / 2, joined(p.bn / 2), ns, allow_split).us + 0.5 < tma_share(p, p.bn, joined(p.bn), ns, allow_split).us)
-            p.bn /= 2;
+    TmaShare how;
+    auto share = [&](int bn) { return p.phases ? TmaShare{} : tma_share(p, bn, joined(bn), ns, allow_split); };
+    if (!rt().pair_tiles) {
+        how = share(p.bn);
+        if (!p.phases && !(ns == 3 && p.forward && p.a_mode == TMA_A_IM2COL))
+            while (p.bn >= 128) {
+                const TmaShare half = share(p.bn / 2);
+                if (half.us + 0.5 >= how.us) break;
+                p.bn /= 2;
+                how = half;
+            }
+    }
     p.joined = joined(p.bn);
     p.issuers = p.bn <= 128 && !p.joined ? 2 : 1;
     if (rt().mma_issuers && rt().mma_issuers < p.issuers) p.issuers = rt().mma_issuers;
-    if (!rt().pair_tiles || ns > 2 || rt().sm_count < 4 || p.narrow) return;
+    if (!rt().pair_tiles) return how;
     int bn = p.bn;
     if (ns == 2 && p.N > 128) bn = 256;               // a pair stages half of B per CTA: 2 x (16 + 16) KB per stage, three stages
-    if (bn < 64 || (p.b_mn && bn < 128) || p.M < 2 * TC_BM) return;
     const long long pair_tiles = (long long)((p.M + 2 * TC_BM - 1) / (2 * TC_BM)) * ((p.N + bn - 1) / bn);
-    if (!allow_split && pair_tiles < rt().sm_count / 2) return;
+    if (ns > 2 || rt().sm_count < 4 || p.narrow || bn < 64 || (p.b_mn && bn < 128) || p.M < 2 * TC_BM ||
+        (!allow_split && pair_tiles < rt().sm_count / 2)) return share(p.bn);
     p.bn = bn;
-    p.pair = 1;
+    p.pair = !p.phases;                               // (phases share a launch of single CTAs)
     p.joined = 0;
+    return p.phases ? how : tma_share(p, p.bn, 0, ns, allow_split);
 }
 
 // Launches the kernel on prepared tensor maps.  p.M, p.N, p.K (contraction length in elements), a_mode, b_mn, bn
-// and the geometry fields must be set; kchunk, stages, partial and status are filled here.
+// and the geometry fields must be set; kchunk, stages, partial and status are filled here.  `how` is what tma_plan returned.
 template <class CS>
-int launch_tma_gemm(const TmaMapSet<phases_of<CS>::value> &maps, TmaGemmParams p, const CS &cs, int ns, bool allow_split, double flops,
+int launch_tma_gemm(const TmaMapSet<phases_of<CS>::value> &maps, TmaGemmParams p, const CS &cs, int ns, const TmaShare &how, double flops,
                     const char *name) {
     if (p.issuers != 2 || p.pair || p.joined || 4 * p.bn > 512) p.issuers = 1;      // TMEM has 512 columns
     const int tm = p.pair ? 2 * TC_BM : TC_BM;
@@ -936,7 +957,6 @@ int launch_tma_gemm(const TmaMapSet<phases_of<CS>::value> &maps, TmaGemmParams p
     if (stages < 2) return fail(SEERA_E_LIMIT, "%s: tile does not fit shared memory", name);
     size_t smem = stage * stages + TG_EPI_WARPS * EPI_WARP_SMEM + 1024;
     const long long tiles = (long long)((p.M + tm - 1) / tm) * ((p.N + p.bn - 1) / p.bn), ksteps = (p.K + TC_BK - 1) / TC_BK;
-    const TmaShare how = p.phases ? TmaShare{} : tma_share(p, p.bn, p.joined, ns, allow_split);
     int splits = p.phases ? p.phases : how.splits;
     const long long rest = how.rest;
     p.shared = how.shared;
@@ -1016,7 +1036,7 @@ int run_tma_gemm(const Shadow &sa, int a_mn, const Shadow &sb, int b_mn, const C
     p.forward = !a_mn && b_mn;                    // C = A B
     p.a_fp16 = sa.enc.fmt; p.b_fp16 = sb.enc.fmt; p.out_scale = 1.f / (sa.enc.scale * sb.enc.scale);
     p.dinv = enc_dinv(sa.enc, sb.enc);
-    tma_plan(p, ns, allow_split);
+    const TmaShare how = tma_plan(p, ns, allow_split);
     TmaMapSet<1> set;
     TmaMaps &maps = set.of[0];
     for (int i = 0; i < 3; i++) {
@@ -1025,7 +1045,7 @@ int run_tma_gemm(const Shadow &sa, int a_mn, const Shadow &sb, int b_mn, const C
         if (int s = make_map_2d(&maps.a[i], sa.p[j], sa.rows, sa.cols, sa.ld, 64, a_mn ? 64 : TC_BM)) return s;
         if (int s = make_map_2d(&maps.b[i], sb.p[j], sb.rows, sb.cols, sb.ld, 64, b_mn ? 64 : (p.pair ? p.bn / 2 : p.bn))) return s;
     }
-    return launch_tma_gemm(set, p, cs, ns, allow_split, 2.0 * M * N * (double)K, name);
+    return launch_tma_gemm(set, p, cs, ns, how, 2.0 * M * N * (double)K, name);
 }
 
 }  // namespace seera
