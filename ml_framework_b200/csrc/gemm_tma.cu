@@ -112,7 +112,8 @@ const Shadow *rows_usable(const seera_rows *h, int ns, int rows, int cols, int c
         h->s.enc.dscale != want.dscale) return nullptr;
     return &h->s;
 }
-// One answer per device and size.  Asked of this kernel, whose blocks take a whole SM as all of these do.
+// One answer per size (a process runs on one device), asked of this kernel, whose blocks take a whole SM as all of these do.  A query that
+// fails is no answer: the product at hand does without clusters, the next one asks again.
 int clusters_at_once(int size) {
     static std::atomic<int> known[9];
     if (size < 2 || size > 8) return 0;
@@ -128,7 +129,7 @@ int clusters_at_once(int size) {
     int got = 0;
     if (allow_smem((const void *)kern, 225 * 1024) != cudaSuccess || cudaOccupancyMaxActiveClusters(&got, kern, &cfg) != cudaSuccess) {
         cudaGetLastError();
-        got = 0;
+        return 0;
     }
     known[size].store(got + 1, std::memory_order_relaxed);
     return got;

@@ -13,11 +13,12 @@ PROGRAM = r"""
 #include <cstdio>
 #include <cstring>
 using namespace seera;
+static int failures = 0;
 extern "C" cudaError_t cudaFuncSetAttribute(const void *, cudaFuncAttribute, int) { return cudaSuccess; }
 extern "C" cudaError_t cudaOccupancyMaxActiveClusters(int *n, const void *, const cudaLaunchConfig_t *c) {
     static const int fit[9] = {0, 0, 74, 48, 36, 28, 22, 20, 16};
     *n = fit[c->attrs[0].val.clusterDim.x];
-    return cudaSuccess;
+    return failures-- > 0 ? cudaErrorUnknown : cudaSuccess;
 }
 template <class F> double least_us(F f) {
     double least = 1e9;
@@ -41,6 +42,10 @@ int main(int, char **argv) {
             }
             if (next) { printf("%d k-steps: %d at the end\n", ksteps, next); return 1; }
         }
+    } else if (!strcmp(argv[1], "clusters")) {
+        failures = 2;
+        for (int k = 0; k < 4; k++) printf("%d ", clusters_at_once(4));
+        printf("%d %d", clusters_at_once(8), clusters_at_once(4));
     } else if (!strcmp(argv[1], "cost")) {
         volatile unsigned long long by = 3;
         volatile unsigned long long out;
@@ -75,3 +80,7 @@ def test_a_plan_costs_few_divisions(program):
     times over every count."""
     cost = [float(v) for v in program("cost").stdout.split()]
     assert len(cost) == 3 and all(c < limit for c, limit in zip(cost, (600, 430, 130))), cost
+
+
+def test_a_failed_query_for_clusters_is_asked_again(program):
+    assert program("clusters").stdout.split() == ["0", "0", "36", "36", "16", "36"]
