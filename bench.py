@@ -387,15 +387,16 @@ def run_gpu(args, work):
         sc.stream_delay(int(min(100000, max(2000, 2000 * ms / args.steps))))
         tr.step(Xd, Yd)
         sc.stream_synchronize()
-    kinds = sc.profile_read_kinds()
     table = sc.profile_report()
     sc.profile_enable(0)
+    # contractions by kind: launches, milliseconds, operations (index 3 holds the bandwidth-bound passes, which have bytes instead)
+    kinds = [[sum(row[j] for row in table if row[1] == k) for j in (2, 3, 4)] if k != 3 else [0, 0, 0] for k in range(5)]
     if rank == 0 and sum(k[0] for k in kinds) and sum(k[1] for k in kinds) > 0:
         cnt, pms, pfl = (sum(k[j] for k in kinds) for j in range(3))
         ach = pfl / (pms / 1e3) / 1e12
         traffic, traffic_src = _traffic_from_profile(args.workload, args.precision)
         sub = {}
-        for name, (kn, kms, kfl) in zip(("forward", "dX", "dW"), kinds):
+        for name, (kn, kms, kfl) in zip(("forward", "dX", "dW", None, "dX+dW"), kinds):        # (the last: both in one launch)
             if kn and kms > 0:
                 t = kfl / (kms / 1e3) / 1e12
                 sub[name] = {"launches_per_step": kn / psteps, "ms_per_step": kms / psteps, "gflop_per_step": kfl / psteps / 1e9,
@@ -412,7 +413,7 @@ def run_gpu(args, work):
                 "launches_per_step": cnt / psteps, "ms_per_step_in_kernel": pms / psteps, "peak_source": peaks["src"] + " sustained bf16",
                 "share_of_step": (pms / psteps) / (ms / args.steps), "by_kind": sub,
                 "backward": None, "hbm_bound_passes": {"peak": peaks["hbm"], "unit": "GB/s", "peak_source": peaks["src"], "passes": hbm}}
-        bkn, bms, bfl = (kinds[1][j] + kinds[2][j] for j in range(3))
+        bkn, bms, bfl = (kinds[1][j] + kinds[2][j] + kinds[4][j] for j in range(3))
         if bkn and bms > 0:
             t = bfl / (bms / 1e3) / 1e12
             roof["backward"] = {"achieved": t, "frac": t / peaks["tensor"], "ms_per_step": bms / psteps}

@@ -61,10 +61,10 @@ int         seera_event_destroy(void *event);
  * stream.  Enabling starts an empty table.  seera_profile_read() waits for the events and returns the
  * contractions' count, summed device time and summed algorithmic FLOPs (2*M*N*K each), then clears the table.
  * seera_profile_read_kinds() gives the same three figures split by kind (index 0 forward products, 1 data
- * gradients dX / dA, 2 weight gradients dW / dB) and leaves the table alone.  seera_profile_report() writes one
- * line per tag, "tag<TAB>kind<TAB>launches<TAB>ms<TAB>work<NEWLINE>" (kind 0-2: work = FLOPs; kind 3: work =
- * algorithmic bytes of a bandwidth-bound pass), and leaves the table alone.  Nothing is recorded during a
- * stream capture.  No counterpart in the reference. */
+ * gradients dX / dA, 2 weight gradients dW / dB; launches that form both gradients are in neither) and leaves the
+ * table alone.  seera_profile_report() writes one line per tag, "tag<TAB>kind<TAB>launches<TAB>ms<TAB>work<NEWLINE>"
+ * (kind 0-2 and 4, both gradients in one launch: work = FLOPs; kind 3: work = algorithmic bytes of a bandwidth-bound
+ * pass), and leaves the table alone.  Nothing is recorded during a stream capture.  No counterpart in the reference. */
 int         seera_profile_enable(int on);
 int         seera_profile_enabled(void);
 int         seera_profile_read(uint64_t *launches, double *ms, double *flops);

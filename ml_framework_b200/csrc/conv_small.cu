@@ -286,7 +286,8 @@ static int small_launch(const SmallSource &src, const float *Wt, const float *bi
 }
 // Both gradients in one launch; its blocks are the two launches' together.
 template <int FL, bool POOLED>
-static int small_bwd_launch(const SmallArgs &a, const float *X, const DzSource &dz, float *dW, float *dbias, const FirstGeom &g, const char *name) {
+static int small_bwd_launch(const SmallArgs &a, const float *X, const DzSource &dz, float *dW, float *dbias, const FirstGeom &g) {
+    const char *name = "conv2d_small_bwd(dX+dW)";
     DwArgs d = dw_args<4, 1, FL, POOLED>(X, dz, g);
     d.partial = (float *)scratch_alloc(dw_partial_bytes<4>(d));
     if (!d.partial) return SEERA_E_OOM;
@@ -352,7 +353,7 @@ bool conv_small_bwd_applies(const float *y, const float *gp, const float *y_pool
     return !gp || act == SEERA_ACT_NONE || y_pooled;       // with the layer output alone a pooled gradient's slope would need a gather
 }
 int conv_small_bwd(const float *Wt, const float *X, const float *y, const float *g, const float *gp, const int *mask, const float *y_pooled,
-                   float *dX, float *dW, float *dbias, int NB, int C, int H, int W, int F, int ph, int pw, int act, const char *name) {
+                   float *dX, float *dW, float *dbias, int NB, int C, int H, int W, int F, int ph, int pw, int act) {
     const int OH = H + 2 * ph - 2, OW = W + 2 * pw - 2;
     const bool sloped = act != SEERA_ACT_NONE;
     int s = SEERA_OK;
@@ -363,18 +364,18 @@ int conv_small_bwd(const float *Wt, const float *X, const float *y, const float 
                                              rt().sm_count * 2 / 3);
         const FirstGeom geo{NB, C, H, W, F, 3, 3, 1, 1, ph, pw, OH, OW, C * 9};
         const DzSource dz{nullptr, g, gp, mask, y, act, y_pooled};
-        if (gp) return F <= 8 ? small_bwd_launch<8, true>(a, X, dz, dW, dbias, geo, name) : F <= 16 ? small_bwd_launch<16, true>(a, X, dz, dW, dbias, geo, name)
-                                                                                                   : small_bwd_launch<32, true>(a, X, dz, dW, dbias, geo, name);
-        return F <= 8 ? small_bwd_launch<8, false>(a, X, dz, dW, dbias, geo, name) : F <= 16 ? small_bwd_launch<16, false>(a, X, dz, dW, dbias, geo, name)
-                                                                                          : small_bwd_launch<32, false>(a, X, dz, dW, dbias, geo, name);
+        if (gp) return F <= 8 ? small_bwd_launch<8, true>(a, X, dz, dW, dbias, geo) : F <= 16 ? small_bwd_launch<16, true>(a, X, dz, dW, dbias, geo)
+                                                                                                   : small_bwd_launch<32, true>(a, X, dz, dW, dbias, geo);
+        return F <= 8 ? small_bwd_launch<8, false>(a, X, dz, dW, dbias, geo) : F <= 16 ? small_bwd_launch<16, false>(a, X, dz, dW, dbias, geo)
+                                                                                          : small_bwd_launch<32, false>(a, X, dz, dW, dbias, geo);
     }
     if (dX) {
         const SmallSource src{gp ? gp : g, sloped ? (gp ? y_pooled : y) : nullptr, gp ? mask : nullptr, act};
-        s = small_run(src, Wt, nullptr, dX, NB, F, OH, OW, C, H, W, 2 - ph, 2 - pw, 1, SEERA_ACT_NONE, name);
+        s = small_run(src, Wt, nullptr, dX, NB, F, OH, OW, C, H, W, 2 - ph, 2 - pw, 1, SEERA_ACT_NONE, "conv2d_small_bwd(dX)");
     }
     if (!s && dW) {
         FirstGeom geo{NB, C, H, W, F, 3, 3, 1, 1, ph, pw, OH, OW, C * 9};
-        s = first_dw(X, DzSource{nullptr, g, gp, mask, y, act, y_pooled}, dW, dbias, geo, name);
+        s = first_dw(X, DzSource{nullptr, g, gp, mask, y, act, y_pooled}, dW, dbias, geo, "conv2d_small_bwd(dW)");
     }
     return s;
 }

@@ -814,7 +814,7 @@ static int tma_conv2d_bwd_kept(const float *Wt, const float *X, const float *dY,
     SEERA_ENSURE();
     if (!conv_ok(NB, C, H, W, F, R, S, sh, sw, ph, pw) || !X || !Wt || (!dY && !dyk)) return fail(SEERA_E_ARG, "cuda_conv2d_bwd: bad argument");
     if (dY && !dyk && conv_small_applies(NB, C, H, W, F, R, S, sh, sw, ph, pw))
-        return conv_small_bwd(Wt, X, nullptr, dY, nullptr, nullptr, nullptr, dX, dW, nullptr, NB, C, H, W, F, ph, pw, SEERA_ACT_NONE, "cuda_conv2d_bwd");
+        return conv_small_bwd(Wt, X, nullptr, dY, nullptr, nullptr, nullptr, dX, dW, nullptr, NB, C, H, W, F, ph, pw, SEERA_ACT_NONE);
     int OH = (H + 2 * ph - R) / sh + 1, OW = (W + 2 * pw - S) / sw + 1;
     if (OH < 1 || OW < 1) return fail(SEERA_E_ARG, "cuda_conv2d_bwd: kernel larger than padded input");
     const bool first = conv_first_applies(C, R, S);
@@ -1175,7 +1175,7 @@ int seera_conv2d_act_bwd_k(const float *Wt, const float *X, const float *y, cons
     if (OH < 1 || OW < 1) return fail(SEERA_E_ARG, "conv2d_act_bwd: kernel larger than padded input");
     if (gp && ((OH & 1) || (OW & 1))) return fail(SEERA_E_ARG, "conv2d_act_bwd: pooled gradient needs even output height and width");
     if (dW && conv_small_applies(NB, C, H, W, F, R, S, sh, sw, ph, pw) && conv_small_bwd_applies(y, gp, y_pooled, act))
-        return conv_small_bwd(Wt, X, y, g, gp, pool_mask, gp ? y_pooled : nullptr, dX, dW, dbias, NB, C, H, W, F, ph, pw, act, "conv2d_act_bwd");
+        return conv_small_bwd(Wt, X, y, g, gp, pool_mask, gp ? y_pooled : nullptr, dX, dW, dbias, NB, C, H, W, F, ph, pw, act);
     const long long out_elems = (long long)NB * F * OH * OW;
     if (keeps_shadows(NB, C, H, W, F, R, S, sh, sw, ph, pw) &&
         (sh == 1 && sw == 1 ? true : phases_supported(H, W, OH, OW, R, S, sh, sw, ph, pw) || !dX)) {

@@ -444,7 +444,7 @@ int skinny_bwd(const float *A, const float *B, const float *dC, float *dA, float
         launch_sum_splits(partial, db_out, (K + 1) * N, splits, st, dbias, K * N);
         e = cudaGetLastError();
     }
-    profile_end((both ? 4.0 : 2.0) * rows * N * (double)K, want_b && !dA ? "cuda_matmul_bwd(dB)" : "cuda_matmul_bwd(dA)");
+    profile_end((both ? 4.0 : 2.0) * rows * N * (double)K, both ? "cuda_matmul_bwd(dA+dB)" : (dA ? "cuda_matmul_bwd(dA)" : "cuda_matmul_bwd(dB)"));
     if (partial) scratch_free(partial);
     if (tmp) scratch_free(tmp);
     return e == cudaSuccess ? SEERA_OK : check_cuda(e, "cuda_matmul_bwd");

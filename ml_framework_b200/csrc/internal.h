@@ -67,7 +67,7 @@ int conv_small_fwd(const float *X, const float *Wt, const float *bias, float *Y,
                    const char *name);
 bool conv_small_bwd_applies(const float *y, const float *gp, const float *y_pooled, int act);
 int conv_small_bwd(const float *Wt, const float *X, const float *y, const float *g, const float *gp, const int *mask, const float *y_pooled,
-                   float *dX, float *dW, float *dbias, int NB, int C, int H, int W, int F, int ph, int pw, int act, const char *name);
+                   float *dX, float *dW, float *dbias, int NB, int C, int H, int W, int F, int ph, int pw, int act);
 // Forward of a 3 x 3 convolution of stride 1 or 2 with at most four input channels, exact fp32 on the CUDA cores, with channels-last
 // copies of the output on request (conv_small.cu); bias and copies may be null.
 struct StorePixelRows;

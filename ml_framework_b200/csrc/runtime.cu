@@ -104,8 +104,8 @@ size_t round_size(size_t n) {
 
 // Per-launch profile (seera_profile_enable): launches bracketed by profile_begin / profile_end[_bytes] are timed with
 // events on the engine's stream and booked under a tag.  Contractions book FLOPs and a kind (0 forward, 1 data gradient,
-// 2 weight gradient, from the entry name's "(dX)" / "(dW)" suffix); bandwidth-bound passes book their algorithmic bytes
-// (kind 3).  Nothing is recorded while a graph is being captured.
+// 2 weight gradient, 4 both in one launch, from the entry name's "(dX)" / "(dW)" / "(dX+dW)" suffix); bandwidth-bound passes book
+// their algorithmic bytes (kind 3).  Nothing is recorded while a graph is being captured.
 struct ProfRec { cudaEvent_t a, b; double work; int kind; const char *tag; };
 struct ProfAgg { int kind = 0; uint64_t n = 0; double ms = 0, work = 0; };
 struct Prof { bool on = false; std::vector<ProfRec> recs; cudaEvent_t pending = nullptr; std::map<std::string, ProfAgg> table; };
@@ -118,13 +118,11 @@ void profile_begin() {
     cudaEventRecord(p.pending, rt().stream);
 }
 static int profile_kind(const char *name) {
-    if (!name) return 0;
-    size_t n = strlen(name);
-    if (n >= 4 && name[n - 1] == ')' && name[n - 4] == '(' && name[n - 3] == 'd') {
-        char c = name[n - 2];
-        return (c == 'X' || c == 'A') ? 1 : ((c == 'W' || c == 'B') ? 2 : 0);
-    }
-    return strcmp(name, "conv2d_act_bwd") == 0 ? 2 : 0;       // the short-patch layer backward forms only the weight gradient
+    const char *of = name ? strrchr(name, '(') : nullptr;
+    if (!of) return name && strcmp(name, "conv2d_act_bwd") == 0 ? 2 : 0;       // the short-patch layer backward forms only the weight gradient
+    if (!strcmp(of, "(dX)") || !strcmp(of, "(dA)")) return 1;
+    if (!strcmp(of, "(dW)") || !strcmp(of, "(dB)")) return 2;
+    return !strcmp(of, "(dX+dW)") || !strcmp(of, "(dA+dB)") ? 4 : 0;
 }
 static void profile_close(double work, int kind, const char *tag) {
     Prof &p = prof();
@@ -388,16 +386,21 @@ int seera_profile_enable(int on) {
     p.on = on != 0;
     return SEERA_OK;
 }
-int seera_profile_read_kinds(uint64_t *launches3, double *ms3, double *flops3) {
-    SEERA_ENSURE();
+// Sums over the kinds below `kinds` (5: all contractions), each kind in its own place or all of them in the first.
+static void profile_sum(int kinds, bool apart, uint64_t *n, double *ms, double *flops) {
     seera::profile_collect();
-    uint64_t n[3] = {0, 0, 0};
-    double t[3] = {0, 0, 0}, f[3] = {0, 0, 0};
     for (auto &kv : seera::prof().table) {
         const auto &g = kv.second;
-        if (g.kind > 2) continue;
-        n[g.kind] += g.n; t[g.kind] += g.ms; f[g.kind] += g.work;
+        if (g.kind == 3 || g.kind >= kinds) continue;
+        const int k = apart ? g.kind : 0;
+        n[k] += g.n; ms[k] += g.ms; flops[k] += g.work;
     }
+}
+int seera_profile_read_kinds(uint64_t *launches3, double *ms3, double *flops3) {
+    SEERA_ENSURE();
+    uint64_t n[3] = {0, 0, 0};
+    double t[3] = {0, 0, 0}, f[3] = {0, 0, 0};
+    profile_sum(3, true, n, t, f);
     for (int k = 0; k < 3; k++) {
         if (launches3) launches3[k] = n[k];
         if (ms3) ms3[k] = t[k];
@@ -406,12 +409,13 @@ int seera_profile_read_kinds(uint64_t *launches3, double *ms3, double *flops3) {
     return SEERA_OK;
 }
 int seera_profile_read(uint64_t *launches, double *ms, double *flops) {
-    uint64_t n[3];
-    double t[3], f[3];
-    if (int s = seera_profile_read_kinds(n, t, f)) return s;
-    if (launches) *launches = n[0] + n[1] + n[2];
-    if (ms) *ms = t[0] + t[1] + t[2];
-    if (flops) *flops = f[0] + f[1] + f[2];
+    SEERA_ENSURE();
+    uint64_t n = 0;
+    double t = 0, f = 0;
+    profile_sum(5, false, &n, &t, &f);
+    if (launches) *launches = n;
+    if (ms) *ms = t;
+    if (flops) *flops = f;
     seera::prof().table.clear();
     return SEERA_OK;
 }

@@ -194,3 +194,25 @@ def test_a_loss_gradient_that_was_written_since_has_a_factor_of_its_own(sc, entr
         assert rel_l2(got, want) < 1e-3, factor              # weight gradients of this mode: one fp16 copy of each operand
     for q in d + [part, loss, dp, dx, dw]:
         sc.cuda_free(q)
+
+
+def test_a_launch_of_both_gradients_is_booked_as_such(sc):
+    """Neither under the data gradients nor under the weight gradients: of a classifier head and of a small convolution."""
+    M, K, N = 600, 96, 10
+    images, C, F, H = 8, 8, 16, 14
+    a, b, g = (sc.cuda_zeros_f(n) for n in (M * K, K * N, M * N))
+    x, w, dy = (sc.cuda_zeros_f(n) for n in (images * C * H * H, F * C * 9, images * F * H * H))
+    out = {n: sc.cuda_zeros_f(n) for n in {M * K, K * N, images * C * H * H, F * C * 9}}
+    sc.profile_enable(1)
+    try:
+        sc.cuda_matmul_bwd(a, b, g, out[M * K], out[K * N], M, N, K, 1)
+        sc.cuda_conv2d_bwd(w, x, dy, out[images * C * H * H], out[F * C * 9], images, C, H, H, F, 3, 3, 1, 1, 1, 1)
+        table, kinds = sc.profile_report(), sc.profile_read_kinds()
+    finally:
+        sc.profile_enable(0)
+    assert sorted((tag, kind, n) for tag, kind, n, _, _ in table) == [("conv2d_small_bwd(dX+dW)", 4, 1), ("cuda_matmul_bwd(dA+dB)", 4, 1)]
+    work = {tag: flops for tag, _, _, _, flops in table}
+    assert work["cuda_matmul_bwd(dA+dB)"] == 4 * M * N * K and work["conv2d_small_bwd(dX+dW)"] == 4 * images * H * H * F * C * 9
+    assert [k[0] for k in kinds] == [0, 0, 0]
+    for p in (a, b, g, x, w, dy, *out.values()):
+        sc.cuda_free(p)
