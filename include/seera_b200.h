@@ -411,6 +411,10 @@ int seera_act_bias_bwd(const float *dy, const float *y, float *dz, float *dbias,
  * factor of the current backward pass (seera_grad_scale_update on the loss gradient). */
 int seera_matmul_bias_act_fwd_s(const float *A, const float *B, const float *bias, float *C, int M, int N, int K, int act,
                                 seera_rows_t *a_in, seera_rows_t **a_keep, seera_rows_t **w_keep, seera_rows_t **c_copies);
+/* A classifier head whose probabilities are wanted with its logits: C = A B + bias and P = softmax of C's rows in one launch, P the bits
+ * that seera_cuda_softmax_fwd makes of C.  *formed is 1; for other products than those of a few columns, which do not take the head
+ * kernels (mode 0 among them), it is 0 and nothing was written. */
+int seera_matmul_softmax_fwd(const float *A, const float *B, const float *bias, float *C, float *P, int M, int N, int K, int *formed);
 int seera_matmul_act_bwd(const float *A, const float *B, const float *y, const float *g, float *dA, float *dB,
                          float *dbias, int M, int N, int K, int act, seera_rows_t *a_keep, seera_rows_t *w_keep);
 /* seera_act_bias_bwd for callers that must not allocate.  No counterpart in the reference.

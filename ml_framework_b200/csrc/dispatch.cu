@@ -79,7 +79,7 @@ static bool skinny_ok(const void *a, const void *b, const void *c, int M, int N,
     return a && b && c && M >= 1 && Nbatch >= 1 && !seera::ensure_init() && seera::skinny_applies(M, N, K, Nbatch);
 }
 int seera_cuda_matmul(const float *A, const float *B, float *C, int M, int N, int K, int Nbatch) {
-    if (skinny_ok(A, B, C, M, N, K, Nbatch)) return seera::skinny_fwd(A, B, nullptr, C, M * Nbatch, N, K, SEERA_ACT_NONE, "cuda_matmul");
+    if (skinny_ok(A, B, C, M, N, K, Nbatch)) return seera::skinny_fwd(A, B, nullptr, C, nullptr, M * Nbatch, N, K, SEERA_ACT_NONE, "cuda_matmul");
     return rt().precision ? (rt().dense_tma ? seera_tma_matmul(A, B, C, M, N, K, Nbatch) : seera_tc_matmul(A, B, C, M, N, K, Nbatch)) : seera_simt_matmul(A, B, C, M, N, K, Nbatch);
 }
 int seera_cuda_matmul_bwd(const float *A, const float *B, const float *dC, float *dA, float *dB, int M, int N, int K, int Nbatch) {
@@ -115,9 +115,15 @@ static int bias_act_after(int s, float *y, const float *bias, long long size, in
     return seera_bias_act_fwd(y, bias, y, (int)size, channels, inner, act);
 }
 int seera_matmul_bias_act_fwd(const float *A, const float *B, const float *bias, float *C, int M, int N, int K, int act) {
-    if (skinny_ok(A, B, C, M, N, K, 1)) return seera::skinny_fwd(A, B, bias, C, M, N, K, act, "cuda_matmul");
+    if (skinny_ok(A, B, C, M, N, K, 1)) return seera::skinny_fwd(A, B, bias, C, nullptr, M, N, K, act, "cuda_matmul");
     if (rt().precision && rt().dense_tma) return seera_tma_matmul_bias_act(A, B, bias, C, M, N, K, 1, act);
     return bias_act_after(seera_cuda_matmul(A, B, C, M, N, K, 1), C, bias, (long long)M * N, N, 1, act);
+}
+int seera_matmul_softmax_fwd(const float *A, const float *B, const float *bias, float *C, float *P, int M, int N, int K, int *formed) {
+    SEERA_ENSURE();
+    if (!formed || !P) return fail(SEERA_E_ARG, "matmul_softmax_fwd: bad argument");
+    *formed = skinny_ok(A, B, C, M, N, K, 1);
+    return *formed ? seera::skinny_fwd(A, B, bias, C, P, M, N, K, SEERA_ACT_NONE, "cuda_matmul") : SEERA_OK;
 }
 int seera_conv2d_bias_act_fwd(const float *image, const float *kernel, const float *bias, float *out, int batchN, int C, int H, int W,
                               int F, int R, int S, int pad_h, int pad_w, int stride_h, int stride_w, int act) {

@@ -299,6 +299,11 @@ PYBIND11_MODULE(seera_cuda, m) {
         ck(seera_matmul_bias_act_fwd_s(P<const F>(a), P<const F>(b), P<const F>(bias), P<F>(c), M, N, K, act, P<seera_rows_t>(a_in), &ak, &wk,
                                        want_c_copies ? &cc : nullptr));
         return py::make_tuple(reinterpret_cast<uptr>(ak), reinterpret_cast<uptr>(wk), reinterpret_cast<uptr>(cc)); });
+    // a head's logits and probabilities in one launch; False where they need two (nothing was written)
+    m.def("matmul_softmax_fwd", [](uptr a, uptr b, uptr bias, uptr c, uptr p, int M, int N, int K) {
+        int formed = 0;
+        ck(seera_matmul_softmax_fwd(P<const F>(a), P<const F>(b), P<const F>(bias), P<F>(c), P<F>(p), M, N, K, &formed));
+        return formed != 0; });
     m.def("matmul_act_bwd", [](uptr a, uptr b, uptr y, uptr g, uptr da, uptr db, uptr dbias, int M, int N, int K, int act, uptr a_keep,
                                uptr w_keep) {
         ck(seera_matmul_act_bwd(P<const F>(a), P<const F>(b), P<const F>(y), P<const F>(g), P<F>(da), P<F>(db), P<F>(dbias), M, N, K, act,

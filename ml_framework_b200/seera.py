@@ -464,14 +464,15 @@ class _ParamLayer(Layer):
             sc.cuda_elemadd(t.value.main_ptr, neg.main_ptr, t.value.main_ptr, t.value.size)
 
     # shared by Dense, Conv2D, ConvTranspose2D
-    def _output(self, x, z, node_backward, takes_pooled=False):
-        """The layer's output Tensor around `z`, which holds act(contraction + bias), or the logits of a softmax."""
+    def _output(self, x, z, node_backward, takes_pooled=False, softmax=None):
+        """The layer's output Tensor around `z`, which holds act(contraction + bias), or the logits of a softmax (`softmax`, where its values
+        came with them)."""
         node = Tensor._of(z, (x, self.weights, self.bais), node_backward)
         if takes_pooled:
             node._takes_pooled = True
         if self.layeract != "softmax":
             return node
-        y = _Softmax.of(z)
+        y = softmax or _Softmax.of(z)
 
         def softmax_backward(g):
             dz = _new(y.shape)
@@ -496,6 +497,9 @@ def _deliver(owner, x, W, b, dx, dw, db):
     _grads_in_arena(owner, W, b)
     if dx is not None:
         x._accumulate(dx)
+
+
+_HEAD_COLUMNS = 16                   # the engine's head kernels hold whole rows of that many columns
 
 
 class Dense(_ParamLayer):
@@ -527,7 +531,15 @@ class Dense(_ParamLayer):
         code = _ACT.get(self.layeract, 0)                    # a softmax follows the product as a pass of its own
         given = x._rows                                      # copies written by the Dense layer before
         want_out = DENSE_EPILOGUE_COPIES and self._feeds_dense and self.layeract != "softmax"
-        ha, hw, ho = sc.matmul_bias_act_fwd_s(xv.main_ptr, wv.main_ptr, b.value.main_ptr, z._ptr, M, N, K, code, given.h if given else 0, want_out)
+        ha = hw = ho = 0
+        prob = None
+        model = self._model and self._model()
+        if model is not None and model._whole and self.layeract == "softmax" and N <= _HEAD_COLUMNS:
+            prob = _Softmax.of(z)                            # a prediction's, with its logits if one launch makes both
+            if not sc.matmul_softmax_fwd(xv.main_ptr, wv.main_ptr, b.value.main_ptr, z._ptr, prob.claim(), M, N, K):
+                prob = None
+        if prob is None:
+            ha, hw, ho = sc.matmul_bias_act_fwd_s(xv.main_ptr, wv.main_ptr, b.value.main_ptr, z._ptr, M, N, K, code, given.h if given else 0, want_out)
         kept_a, kept_w = _KeptRows(ha) if ha else None, _KeptRows(hw) if hw else None
         need_dx, owner = not x.is_leaf, self._model
 
@@ -542,7 +554,7 @@ class Dense(_ParamLayer):
                 if k:
                     k.release()
             _deliver(owner, x, W, b, dx, dw, db)
-        self.outputs = out = self._output(x, z, backward)
+        self.outputs = out = self._output(x, z, backward, softmax=prob)
         if want_out:
             out._rows = _KeptRows(ho)
         return out
@@ -1017,7 +1029,7 @@ class _RecordedStep:
 
 
 class Sequential:
-    _whole = False                   # in predict: the pass forms a softmax output too, which a loss would form on its way
+    _whole = False                   # in predict: a softmax that the last layer's launch can form is formed there
 
     def __init__(self, layers, device="cuda"):
         if not isinstance(layers, list):
@@ -1098,8 +1110,6 @@ class Sequential:
             out = None
             for layer in self.model:
                 out = layer.forward()
-            if self._whole and out.value.__class__ is _Softmax:
-                out.value.main_ptr                    # formed with the pass: nothing behind it forms it on its way
         finally:
             if opened:
                 _close_batch()

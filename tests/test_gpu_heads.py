@@ -70,6 +70,50 @@ def test_the_predictions_are_there_for_whoever_reads_them(sc):
     assert np.allclose(pred.to_numpy(), before, rtol=1e-6) and np.allclose(before.sum(1), 1, rtol=1e-5)
 
 
+#  rows: one, odd, both sizes of the kernel of few rows, the other one;  K: within a slice of the weights, over one
+@pytest.mark.parametrize("shape", [(1, 7, 1), (5, 40, 2), (37, 784, 10), (601, 96, 16), (1185, 1500, 3), (1187, 2100, 13), (1300, 64, 16)])
+def test_a_head_gives_its_probabilities_with_its_logits(sc, shape):
+    """The bits of the softmax launch, infinite and undefined logits among them."""
+    M, K, N = shape
+    rs = np.random.RandomState(sum(shape))
+    a, b, bias = (rs.standard_normal(s).astype(np.float32) for s in ((M, K), (K, N), (N,)))
+    a[M // 2, 0], a[M - 1, K // 2] = np.inf, np.nan
+    ad, bd, biasd = (sc.to_device_f32(t.ravel()) for t in (a, b, bias))
+    c, p, alone, q = (sc.cuda_malloc_f32(M * N + 1) for _ in range(4))
+    for out in (c, p, alone, q):
+        sc.upload_f32(out, np.full(M * N + 1, 7, np.float32))
+    before = sc.launch_count()
+    assert sc.matmul_softmax_fwd(ad, bd, biasd, c, p, M, N, K)
+    assert sc.launch_count() == before + 1
+    sc.matmul_bias_act_fwd(ad, bd, biasd, alone, M, N, K, 0)
+    sc.cuda_softmax_fwd(alone, q, M, N)
+    bits = [sc.to_host_f32(t, (M * N + 1,)).view(np.int32) for t in (c, alone, p, q)]
+    assert np.array_equal(bits[0], bits[1]) and np.array_equal(bits[2], bits[3])
+    sc.set_precision(0)
+    assert not sc.matmul_softmax_fwd(ad, bd, biasd, c, p, M, N, K)
+    for t in (ad, bd, biasd, c, p, alone, q):
+        sc.cuda_free(t)
+
+
+@pytest.mark.parametrize("classes,predicted", [(10, 1), (40, None)])
+def test_the_loss_of_a_prediction_takes_one_launch(sc, classes, predicted):
+    from ml_framework_b200 import seera as S
+    rs = np.random.RandomState(classes)
+    model, lossf = S.Sequential([S.Input((50,)), S.Dense(50, classes, "softmax")]), S.Loss().categorical_cross_entropy
+    x = S.Tensor(rs.standard_normal((64, 50)).astype(np.float32), is_leaf=True)
+    y = S.Tensor(np.eye(classes, dtype=np.float32)[rs.randint(0, classes, 64)], is_leaf=True)
+    for _ in range(3):                          # the first pass, and batched ones
+        counts = [sc.launch_count()]
+        pred = model.predict(x)
+        counts.append(sc.launch_count())
+        loss = lossf(pred, y)
+        counts.append(sc.launch_count())
+        assert predicted is None or counts[1] - counts[0] == predicted
+        assert counts[2] - counts[1] == 1
+        values = pred.to_numpy()
+        assert np.array_equal(values, model.predict(x).to_numpy()) and loss.item() > 0
+
+
 def test_losses_on_two_streams_finish_each_by_itself():
     """On the library's stream, on a caller's, and recorded and replayed on the caller's: more launches than there ever were counters."""
     import torch

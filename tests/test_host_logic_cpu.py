@@ -505,6 +505,22 @@ def test_values_left_unformed_by_a_recording_follow_its_replays(host, monkeypatc
     assert formed
 
 
+@pytest.mark.parametrize("classes", [3, 20])
+def test_the_loss_of_a_prediction_takes_no_more_launches_than_that_of_a_forward(host, classes):
+    S, fake = host.seera, host.fake
+    rs = np.random.RandomState(1)
+    X, Y = rs.standard_normal((6, 5)).astype(np.float32), S.Tensor(np.eye(classes, dtype=np.float32)[rs.randint(0, classes, 6)], is_leaf=True)
+    model, lossf = S.Sequential([S.Input((5,)), S.Dense(5, classes, "softmax")]), S.Loss().categorical_cross_entropy
+    X = S.Tensor(X, is_leaf=True)
+    used, losses = [], []
+    for call in (model.forward, model.predict):
+        fake.CALLS.clear()
+        losses.append(lossf(call(X), Y).item())
+        used.append({k: n for k, n in fake.CALLS.items() if "softmax" in k})
+    assert used == [{"softmax_cce": 1}] * 2 and losses[0] == losses[1]
+    assert np.array_equal(model.predict(X).to_numpy(), model.forward(X).to_numpy())
+
+
 def test_a_dropped_model_gives_its_memory_back_at_once(host):
     """Without waiting for the garbage collector: its blocks are there for the next model's first pass."""
     import gc
