@@ -103,8 +103,8 @@ int         seera_get_precision(void);
  *       (tcgen05 cta_group::2: each CTA stages its own 128 rows of A and half of B's columns, the even CTA issues the
  *       MMAs for both, completion of both CTAs' plain tensor copies is counted on its barrier; no multicast load).
  *       It cuts the operand bytes per CTA and k-step by a quarter to a third.  Bit-for-bit the same results; measured
- *       3-8 % SLOWER on every configuration here (C3 dgrad 51.3 -> 53.2 us, wgrad 41.2 -> 51.1 us), because these
- *       kernels are bound by the MMA issue rate at accumulator widths of 64-128 columns, not by the operand stream.
+ *       3-8 % SLOWER on every configuration here (C3 dgrad 51.3 -> 53.2 us, wgrad 41.2 -> 51.1 us): at accumulator widths
+ *       of 64-128 columns an MMA takes what its operands take out of shared memory, which a pair does not shorten.
  *   "wgrad_single" (default 1): in precision mode 4 a weight gradient (conv dW, Dense dB) is formed from the FIRST fp16
  *       copy of each operand alone - one product instead of three.  Its 2^-12 rounding stays inside that one tensor
  *       (nothing downstream in the backward pass reads dW); measured on the VGG configuration it moves no dW error

@@ -69,7 +69,7 @@ __device__ __forceinline__ BnMoments bn_merge_rows(const float *__restrict__ mom
             const float *p = moments + ((long long)(s0 + lane) * C + c) * 3;
             v = BnMoments{__ldg(p), __ldg(p + 1), __ldg(p + 2)};
         }
-        float n = lane == 0 ? t.n + v.n : v.n;                 // rows up to and with this one: whole numbers, exact
+        float n = lane == 0 ? t.n + v.n : v.n;                 // rows up to and with this one (exact up to 2^24 elements a channel)
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const float before = __shfl_up_sync(0xffffffffu, n, o);

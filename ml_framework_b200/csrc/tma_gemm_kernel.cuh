@@ -321,9 +321,9 @@ constexpr int TG_THREADS = 384, TG_EPI_WARP0 = 4, TG_EPI_WARPS = 8;
 // bn = 64, 25600 x 64 x 1152: 34.3 -> 31.8).  Sums in two accumulators are also shorter chains: 1.92e-6 -> 1.02e-6 of error at NS = 3
 // against float64, 1.08e-6 -> 7.1e-7 at NS = 2 on fp16 (512 x 64 x 576).  The epilogue adds the two accumulators; TMEM holds 2 buffers x 2 x bn columns (at most 512).
 //
-// Products of one copy with N <= 128, and the forward ones in six products that tma_plan names, are issued by two threads (lane 0 of warps 1 and 2), which take the K = 16 slices of a
-// k-step alternately, each into an accumulator of its own (MMAs of different threads are not ordered among themselves), and
-// commit to the stage's "empty" and the tile's "accumulator full" barriers, which count `issuers` arrivals.
+// Products of one copy with N <= 128, and the forward ones in six products that tma_plan names, are issued by two threads (lane 0 of
+// warps 1 and 2), which take the K = 16 slices of a k-step alternately, each into an accumulator of its own (MMAs of different threads are
+// not ordered among themselves), and commit to the stage's "empty" and the tile's "accumulator full" barriers, which count `issuers` arrivals.
 // (NARROW apart from the rest: its branches in the producer and the issuer cost the others 5 % of a launch.)
 template <int NS, class CS, bool PAIR, bool NARROW>
 __global__ void __launch_bounds__(TG_THREADS, 1)
@@ -591,8 +591,8 @@ tma_gemm_kernel(const __grid_constant__ TmaMapSet<phases_of<CS>::value> maps, CS
                 if (!alive) break;
                 tc_fence_after();
                 const uint64_t das = da0 + (uint32_t)s * stage16, dbs = db0 + (uint32_t)s * stage16;
-                // the K = 16 slices of this thread (da0 / db0 already point at its first one), fully unrolled either way: the
-                // issuing thread's own instruction stream is what limits the MMA rate
+                // the K = 16 slices of this thread (da0 / db0 already point at its first one), fully unrolled either way: one thread
+                // keeps up with the pipe only while an MMA costs it a few instructions
                 auto slice = [&](uint64_t dsa, uint64_t dsb, bool first) {
                     uint64_t da[NS], db[NS];
 #pragma unroll
@@ -913,7 +913,8 @@ inline TmaShare tma_plan(TmaGemmParams &p, int ns, bool allow_split) {
     // Outputs of a layer in six products keep the order of sums that two threads give, but for convolutions of 128 columns: another order
     // moves the ReLU and pool decisions that lie on a tie, and programs that follow a run from version to version see that (a network with
     // batch normalisation: 1e-3 to 1e-2 of a first-layer gradient in one of ten seeds).  It costs 1.5 us of 14 at 32768 x 64 x 288 and
-    // nothing for Dense layers; at 128 columns the joined form is 3 % faster (198912 x 128 x 576: 126 -> 122 us).
+    // nothing for Dense layers; at 128 columns the joined form is 3 % faster (198912 x 128 x 576: 126 -> 122 us).  Products of few tiles have
+    // another order all the same, where a cluster shares the contraction: there it halves the time.
     auto joined = [&](int bn) { return ns >= 2 && bn <= 128 && !(ns == 3 && p.forward && (p.a_mode != TMA_A_IM2COL || bn < 128)); };
     // Half the width gives twice the tiles, which is worth its extra loads of A where the wider ones leave SMs without work or a long way out
     // of the accumulators: 1000 x 1024 x 1024 in one product, 256 columns 12.4, 128 columns 9.3 us; 3136 x 512 x 4608 20.9 against 24.2.

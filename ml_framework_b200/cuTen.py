@@ -49,8 +49,6 @@ def _reduction(shape, dim):
 _reduced = functools.lru_cache(maxsize=1024)(_reduction)         # for an axis that is an int: 1.0 would be known as 1, and an array by its identity
 
 
-
-
 @functools.lru_cache(maxsize=1024)
 def _broadcast(a, b):
     """The output's shape and size, both operands' shapes as the engine takes them."""
