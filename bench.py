@@ -10,14 +10,15 @@ with every batch copied from pinned host memory and every loss read back.  Both 
 timed regions of K steps each; the spread is printed beside them.  `roofline` covers the contraction kernels
 (Dense / convolution forward, dX, dW, each with its own sub-record) and lists the bandwidth-bound passes with their
 algorithmic bytes against the HBM peak; all of it is timed live with CUDA events in a separate profiled pass.
-`cpu_baseline` is the reference's own CPU engine on this box's host cores on a bounded sample.
+`cpu_baseline` is the reference's own CPU engine, or the C restatement of it (its `kind` says which), on this box's host cores on a bounded sample.
 
 With N > 1 the batch is sharded: every rank trains `batch` samples per step (weak scaling; `--scaling strong` splits
 the configuration's batch over the ranks instead), the gradient arena is summed over the ranks by the engine's own
 NCCL data plane in buckets that overlap the rest of backward - inside the captured step graph - and the optimizer
 divides by the world size.  After the timed steps the ranks' weights are compared (`dp_check`).
-`--impl reference` times the reference CPU engine (oracle/_ref, else the C restatement) driven op for op as the
-reference's CPU path runs, with the thread layout stated in its line.
+`--impl reference` times the reference's own CPU engine (oracle/_ref) driven op for op as the reference's CPU path runs, with
+the thread layout stated in its line; without a build of it the line says that it is unavailable.  Nothing of this package's
+engine is loaded on that path.
 """
 import os
 
@@ -171,6 +172,11 @@ CPU_SAMPLE = {"c1": 64, "c2": 512, "c3": 32, "c4": 16}
 def run_reference(args, work):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
+        return
+    from oracle import ref_engine
+    if ref_engine.load() is None:
+        print(json.dumps({"impl": "reference", "unavailable": "oracle/_ref holds no build of the reference's CPU engine that loads here "
+                          "(make -C oracle ref REF=<checkout>)"}), flush=True)
         return
     sample = CPU_SAMPLE[args.workload]
     v, ms, kind, how = cpu_steps(work, sample, args.steps, args.warmup)
@@ -621,8 +627,8 @@ def main():
     ap.add_argument("--c5-batch", type=int, default=256)
     ap.add_argument("--impl", default="b200", choices=["b200", "reference"])
     ap.add_argument("--precision", default=None,
-                    help="0 fp32 CUDA cores | 1 bf16 | 2 bf16x3 | 3 bf16x6 | F/B per phase; default: 1 for c2 (a bf16 configuration), "
-                         "3/2 for the fp32 configurations")
+                    help="0 fp32 CUDA cores | 1 bf16 | 2 bf16x3 | 3 bf16x6 | 4 fp16x3 | 5 fp16 | F/B per phase; default: 4, for c2 (a 16-bit "
+                         "configuration) 4/5")
     ap.add_argument("--option", action="append", default=[], metavar="NAME=VALUE",
                     help="engine option for seera_set_option (repeatable), e.g. tile_n_cap3=128")
     ap.add_argument("--buckets", type=int, default=5, help="data parallel: target number of gradient buckets (all-reduces) per step")
@@ -648,14 +654,14 @@ def main():
             run_adjacent(args)
         return
     work = wl.WORKLOADS[args.workload]()
+    if args.impl == "reference":
+        run_reference(args, work)
+        return
     if args.precision is None:
         from ml_framework_b200.train import POLICY          # the policy the parity gates are checked at
         f, b = POLICY[work.precision]
         args.precision = str(f) if f == b else "%d/%d" % (f, b)
-    if args.impl == "reference":
-        run_reference(args, work)
-    else:
-        run_gpu(args, work)
+    run_gpu(args, work)
 
 
 if __name__ == "__main__":

@@ -163,3 +163,18 @@ def test_batchnorm_restatement_matches_the_reference_engine_and_numpy():
                 assert np.array_equal(rm, rm2) and np.array_equal(rv, rv2)
                 r = REF.batchnorm_backward(d, xh2, si2, g, M, len(shape) == 4)
                 assert all(np.array_equal(p, q) for p, q in zip((dx, dg, db), r))
+
+
+@pytest.mark.skipif(REF is not None, reason="the reference's engine is built")
+def test_the_bench_times_nothing_else_as_the_reference():
+    """Without a build of the reference's engine its arm says so, and this package's engine is not loaded for it either."""
+    import json
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    run = ("import runpy, sys; sys.argv = ['bench.py', '--impl', 'reference']; runpy.run_path('bench.py', run_name='__main__'); "
+           "print([l.split()[-1] for l in open('/proc/self/maps') if 'seera' in l.split()[-1]])")
+    out = subprocess.run([sys.executable, "-c", run], cwd=root, capture_output=True, text=True, check=True).stdout.splitlines()
+    line = json.loads(out[0])
+    assert line["impl"] == "reference" and line["unavailable"] and "value" not in line and out[1] == "[]"
