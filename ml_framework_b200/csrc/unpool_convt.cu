@@ -332,7 +332,7 @@ int seera_unpool2_convT_act_bwd(const float *w, const float *x, const float *y, 
         count_launch();
         launch_sum_splits(partial, dw, Cin * 9, blocks, rt().stream);
         if (e == cudaSuccess) e = cudaGetLastError();
-        profile_end(2.0 * N * 4 * H * W * (double)Cin * 9 * (dx ? 2 : 1), "unpool2_convT_bwd(dW)");
+        profile_end(2.0 * N * 4 * H * W * (double)Cin * 9 * (dx ? 2 : 1), dx ? "unpool2_convT_bwd(dX+dW)" : "unpool2_convT_bwd(dW)");
         if (e != cudaSuccess) s = check_cuda(e, "unpool2_convT_bwd");
     }
     if (partial) scratch_free(partial);

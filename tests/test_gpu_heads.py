@@ -241,22 +241,26 @@ def test_a_loss_gradient_that_was_written_since_has_a_factor_of_its_own(sc, entr
 
 
 def test_a_launch_of_both_gradients_is_booked_as_such(sc):
-    """Neither under the data gradients nor under the weight gradients: of a classifier head and of a small convolution."""
+    """Neither under the data gradients nor under the weight gradients: of a classifier head, of a small convolution, of an unpooled image."""
     M, K, N = 600, 96, 10
     images, C, F, H = 8, 8, 16, 14
     a, b, g = (sc.cuda_zeros_f(n) for n in (M * K, K * N, M * N))
     x, w, dy = (sc.cuda_zeros_f(n) for n in (images * C * H * H, F * C * 9, images * F * H * H))
+    low = images * C * H * H                             # an unpooled layer's input, twice the height and width in its output
+    u, du, yu, gu = (sc.cuda_zeros_f(n) for n in (low, low, 4 * images * H * H, 4 * images * H * H))
+    wu, dwu, dbu = (sc.cuda_zeros_f(n) for n in (C * 9, C * 9, 1))
     out = {n: sc.cuda_zeros_f(n) for n in {M * K, K * N, images * C * H * H, F * C * 9}}
     sc.profile_enable(1)
     try:
         sc.cuda_matmul_bwd(a, b, g, out[M * K], out[K * N], M, N, K, 1)
         sc.cuda_conv2d_bwd(w, x, dy, out[images * C * H * H], out[F * C * 9], images, C, H, H, F, 3, 3, 1, 1, 1, 1)
+        sc.unpool2_convT_act_bwd(wu, u, yu, gu, du, dwu, dbu, images, C, H, H, 2)
         table, kinds = sc.profile_report(), sc.profile_read_kinds()
     finally:
         sc.profile_enable(0)
-    assert sorted((tag, kind, n) for tag, kind, n, _, _ in table) == [("conv2d_small_bwd(dX+dW)", 4, 1), ("cuda_matmul_bwd(dA+dB)", 4, 1)]
-    work = {tag: flops for tag, _, _, _, flops in table}
-    assert work["cuda_matmul_bwd(dA+dB)"] == 4 * M * N * K and work["conv2d_small_bwd(dX+dW)"] == 4 * images * H * H * F * C * 9
+    assert {tag: (kind, n, work) for tag, kind, n, _, work in table if kind != 3} == {
+        "cuda_matmul_bwd(dA+dB)": (4, 1, 4 * M * N * K), "conv2d_small_bwd(dX+dW)": (4, 1, 4 * images * H * H * F * C * 9),
+        "unpool2_convT_bwd(dX+dW)": (4, 1, 16 * images * H * H * C * 9)}
     assert [k[0] for k in kinds] == [0, 0, 0]
-    for p in (a, b, g, x, w, dy, *out.values()):
+    for p in (a, b, g, x, w, dy, u, du, yu, gu, wu, dwu, dbu, *out.values()):
         sc.cuda_free(p)
